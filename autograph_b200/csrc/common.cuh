@@ -70,6 +70,8 @@ struct ag_device {
     size_t workspace_bytes = 0;
     void *staging = nullptr;        // second scratch block: operand re-layouts of the
     size_t staging_bytes = 0;       // tensor-core convolution (may be live next to workspace)
+    void *engine = nullptr;         // third block: k-slice sums and packed operands of the
+    size_t engine_bytes = 0;        // tensor-core engines (live next to the other two)
     std::vector<void *> retired;    // outgrown scratch blocks that captured graphs may still use
     int *status_dev = nullptr;      // device word: 0 = ok, else a timeout code
     int *status_host = nullptr;     // pinned mirror
@@ -102,6 +104,9 @@ class DeviceGuard {
 int workspace(ag_device *dev, size_t bytes, void **out);
 // The same for the second scratch block.
 int staging(ag_device *dev, size_t bytes, void **out);
+// The same for the tensor-core engines' block: a product may run on operands that lie in either of
+// the other two.
+int engine_scratch(ag_device *dev, size_t bytes, void **out);
 
 inline size_t dtype_size(ag_dtype t) {
     switch (t) {

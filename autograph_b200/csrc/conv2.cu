@@ -4,6 +4,7 @@
 #include "conv2_direct.cuh"
 #include "conv_tc.cuh"
 #include "gemm_simt_launch.cuh"
+#include "tcx_api.cuh"
 
 namespace ag {
 
@@ -301,6 +302,16 @@ int ag_conv2_forward(ag_device *dev, ag_dtype dtype, const void *x, int64_t bs, 
                                               (const __nv_bfloat16 *)bias, opt, fuse_relu != 0,
                                               false, (__nv_bfloat16 *)y);
     }
+    if (tcx::conv_worth(dtype, bs * g.oh * g.ow, oc, ic * g.fh * g.fw, opt)) {
+        if (dtype == AG_F32)
+            return tcx::conv_forward<float>(dev, (const float *)x, bs, ic, ih, iw, (const float *)w, oc,
+                                            (const float *)bias, opt, g.oh, g.ow, fuse_relu != 0,
+                                            (float *)y);
+        return tcx::conv_forward<__nv_bfloat16>(dev, (const __nv_bfloat16 *)x, bs, ic, ih, iw,
+                                                (const __nv_bfloat16 *)w, oc,
+                                                (const __nv_bfloat16 *)bias, opt, g.oh, g.ow,
+                                                fuse_relu != 0, (__nv_bfloat16 *)y);
+    }
     if (dtype == AG_F32)
         return conv2_forward_t<float>(dev, g, (const float *)x, (const float *)w, (int)oc,
                                       (const float *)bias, fuse_relu != 0, (float *)y);
@@ -401,6 +412,15 @@ int ag_conv2_backward_input(ag_device *dev, ag_dtype dtype, const void *w, int64
                                                      (const __nv_bfloat16 *)dy, bs, ih, iw, opt,
                                                      (__nv_bfloat16 *)dx);
     }
+    if (tcx::conv_worth(dtype, bs * ih * iw, ic, oc * g.fh * g.fw, opt) &&
+        bs * oc * g.oh * g.ow < (1ll << 31)) {
+        if (dtype == AG_F32)
+            return tcx::conv_backward_input<float>(dev, (const float *)w, oc, ic, (const float *)dy, bs,
+                                                   ih, iw, opt, g.oh, g.ow, (float *)dx);
+        return tcx::conv_backward_input<__nv_bfloat16>(dev, (const __nv_bfloat16 *)w, oc, ic,
+                                                       (const __nv_bfloat16 *)dy, bs, ih, iw, opt,
+                                                       g.oh, g.ow, (__nv_bfloat16 *)dx);
+    }
     if (dtype == AG_F32)
         return conv2_backward_input_t<float>(dev, g, (const float *)w, (int)oc, (const float *)dy,
                                              (float *)dx);
@@ -429,6 +449,16 @@ int ag_conv2_backward_weight(ag_device *dev, ag_dtype dtype, const void *x, int6
         return direct::backward_weight<__nv_bfloat16>(dev, (const __nv_bfloat16 *)x, bs, ic, ih, iw,
                                                       (const __nv_bfloat16 *)dy, oc, opt, beta,
                                                       (__nv_bfloat16 *)dw);
+    }
+    if (bs > 0 && tcx::conv_worth(dtype, ic * g.fh * g.fw, oc, bs * g.oh * g.ow, opt) &&
+        bs * oc * g.oh * g.ow < (1ll << 31)) {
+        if (dtype == AG_F32)
+            return tcx::conv_backward_weight<float>(dev, (const float *)x, bs, ic, ih, iw,
+                                                    (const float *)dy, oc, opt, g.oh, g.ow, beta,
+                                                    (float *)dw);
+        return tcx::conv_backward_weight<__nv_bfloat16>(dev, (const __nv_bfloat16 *)x, bs, ic, ih, iw,
+                                                        (const __nv_bfloat16 *)dy, oc, opt, g.oh, g.ow,
+                                                        beta, (__nv_bfloat16 *)dw);
     }
     if (dtype == AG_F32)
         return conv2_backward_weight_t<float>(dev, g, (const float *)x, (const float *)dy, (int)oc,

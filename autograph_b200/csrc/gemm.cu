@@ -3,6 +3,7 @@
 #include "dense_small.cuh"
 #include "gemm_simt_launch.cuh"
 #include "gemm_tc.cuh"
+#include "tcx_api.cuh"
 
 namespace ag {
 
@@ -85,6 +86,9 @@ extern "C" int ag_dense_forward(ag_device *dev, ag_dtype dtype, const void *x, i
             dev, (const __nv_bfloat16 *)x, (int)bs, (int)inputs, (const __nv_bfloat16 *)w,
             (int)outputs, (const __nv_bfloat16 *)bias, fuse_relu != 0, (__nv_bfloat16 *)y);
     }
+    if (dtype == AG_F32 && tcx::gemm_worth(dtype, bs, inputs, outputs))
+        return tcx::dense<float>(dev, (const float *)x, (int)bs, (int)inputs, (const float *)w,
+                                 (int)outputs, (const float *)bias, fuse_relu != 0, (float *)y);
     if (dtype == AG_F32)
         return dense_forward_simt<float>(dev, (const float *)x, (int)bs, (int)inputs,
                                          (const float *)w, (int)outputs, (const float *)bias,
@@ -104,6 +108,9 @@ extern "C" int ag_dense_forward(ag_device *dev, ag_dtype dtype, const void *x, i
         if (fuse_relu && !relu_fused) AG_TRY(ag_relu(dev, dtype, y, y, bs * outputs));
         return AG_OK;
     }
+    if (tcx::gemm_worth(dtype, bs, inputs, outputs))
+        return tcx::dense<__nv_bfloat16>(dev, px, (int)bs, (int)inputs, pw, (int)outputs,
+                                         (const __nv_bfloat16 *)bias, fuse_relu != 0, py);
     return dense_forward_simt<__nv_bfloat16>(dev, px, (int)bs, (int)inputs, pw, (int)outputs,
                                              (const __nv_bfloat16 *)bias, fuse_relu != 0, py);
 }
@@ -311,7 +318,13 @@ extern "C" int ag_gemm(ag_device *dev, ag_dtype dtype, int64_t m, int64_t k, int
             dev, (const __nv_bfloat16 *)a + off_a, (int)m, (int)k, (const __nv_bfloat16 *)b + off_b,
             (int)n, nullptr, false, (__nv_bfloat16 *)c + off_c);
     }
+    const bool tensor_core = tcx::gemm_worth(dtype, m, k, n);
     if (dtype == AG_F32) {
+        if (tensor_core)
+            return tcx::gemm_strided<float>(dev, (int)m, (int)k, (int)n, alpha,
+                                            (const float *)a + off_a, rsa, csa,
+                                            (const float *)b + off_b, rsb, csb, beta,
+                                            (float *)c + off_c, rsc, csc);
         return gemm_simt_dispatch<float>(dev, (int)m, (int)k, (int)n, alpha,
                                          (const float *)a + off_a, rsa, csa,
                                          (const float *)b + off_b, rsb, csb, beta,
@@ -323,6 +336,9 @@ extern "C" int ag_gemm(ag_device *dev, ag_dtype dtype, int64_t m, int64_t k, int
     if (tc::gemm_bf16_eligible(m, k, n, pa, rsa, csa, pb, rsb, csb, pc, rsc, csc))
         return tc::gemm_bf16(dev, (int)m, (int)k, (int)n, alpha, pa, rsa, csa, pb, rsb, csb, beta,
                              pc, rsc, csc);
+    if (tensor_core)
+        return tcx::gemm_strided<__nv_bfloat16>(dev, (int)m, (int)k, (int)n, alpha, pa, rsa, csa, pb,
+                                                rsb, csb, beta, pc, rsc, csc);
     return gemm_simt_dispatch<__nv_bfloat16>(dev, (int)m, (int)k, (int)n, alpha, pa, rsa, csa, pb,
                                              rsb, csb, beta, pc, rsc, csc);
 }

@@ -435,11 +435,13 @@ int gemm_bf16(ag_device *dev, int m, int k, int n, float alpha, const __nv_bfloa
     if (epi && epi->bias)
         AG_REQUIRE((reinterpret_cast<uintptr_t>(epi->bias) & 15) == 0, AG_ERR_INVALID, "bias not 16-byte aligned");
     // Few output tiles and a long k (a Dense layer with tens of thousands of inputs at a
-    // small batch): slices of k become work items so that the whole GPU is used.
+    // small batch): slices of k become work items so that the whole GPU is used.  A shorter k is
+    // worth the reduction's second launch only for a handful of tiles (200 x 3000 x 400 on four
+    // tiles: 28 -> 15.5 us; 512 x 1024 x 512 on eight: 11.3 us whole, 13.2 us in slices).
     const int out_tiles = (int)(ceil_div(m, BLOCK_M) * ceil_div(n, BLOCK_N));
     const int total_kb = (int)ceil_div(k, BLOCK_K);
     int splits = 1, kb_per_split = total_kb;
-    if (out_tiles * 4 <= dev->sm_count && total_kb >= 64) {
+    if (out_tiles * (total_kb >= 64 ? 4 : 32) <= dev->sm_count && total_kb >= 16) {
         splits = dev->sm_count / out_tiles;
         if (splits > total_kb / 4) splits = total_kb / 4;  // at least four k blocks per slice
         if (splits < 1) splits = 1;

@@ -1,0 +1,859 @@
+// Tensor-core tile engine with gathered operands: the counterpart of the SIMT engine in
+// gemm_simt.cuh for products that are worth a tensor core but that TMA cannot feed -- f32
+// operands, bf16 operands whose rows are not 16-byte aligned, and the implicit GEMMs of
+// convolutions with any padding / stride / dilation.
+//
+// One persistent CTA per SM walks 128 x BN output tiles (and k slices).  Warp roles:
+//   warps 0..7   producers: fetch 8 consecutive k of a row at a time with plain loads, split
+//                f32 values into bf16 planes, and write the 128-byte-swizzled K-major tiles
+//                tcgen05.mma reads
+//   EPI warps    read finished accumulators from tensor memory and store through an epilogue
+//   last warp    issues tcgen05.mma
+//
+// f32 products.  A f32 value is written as the sum of three bf16 values (hi, mid, lo: 8 + 8 + 8
+// bits, the remainders exact), and a product as the six partial products down to 2^-16 of the
+// leading one (Henry, Tang, Heinecke, "Leveraging the bfloat16 artificial intelligence datatype
+// for higher-precision computations", 2019); what is dropped is below 2^-25 of a product, half
+// an ulp of the f32 product.  The tensor core adds with truncation, so an accumulator is read
+// out after every 64 k and the 64-k sums are added in registers with round-to-nearest; within
+// 64 k the small partial products are accumulated first, which leaves four truncating additions
+// of full-size terms.  Uniform operands, relative 2-norm error against an f64 product: k = 128
+// 8e-8 (the FFMA kernel 1.1e-7), k = 1024 1.1e-7 (5.7e-7), k = 4096 1.7e-7 (1.2e-6).  An output
+// that comes out infinite or NaN is recomputed with FFMAs from the f32 operands (the split of
+// an infinity, or of a value that rounds up to one, is not usable).
+//
+// What bounds it: with BN = 128 a 64-k step is 16 MMAs that read (128 + N) x 32 bytes of shared
+// memory each, about 2600 cycles; the producers convert 16 k elements in the same time.
+#pragma once
+
+#include "common.cuh"
+#include "tc_ptx.cuh"
+
+namespace ag {
+namespace tcx {
+
+constexpr int BM = 128;
+constexpr int BK = 64;
+constexpr int PRODUCERS = 256;
+constexpr int ROW_BYTES = BK * 2;
+
+template <class T>
+struct Planes;
+template <>
+struct Planes<float> { static constexpr int N = 3; };
+template <>
+struct Planes<__nv_bfloat16> { static constexpr int N = 1; };
+
+// Eight consecutive k of one row, as fetched.
+template <class T>
+struct Vec8;
+template <>
+struct Vec8<float> { float v[8]; };
+template <>
+struct Vec8<__nv_bfloat16> { uint32_t v[8]; };  // one value per register until they are packed
+
+__device__ __forceinline__ void fetch(float &d, const float *p, bool ok) {
+    d = 0.f;
+    if (ok) d = __ldg(p);
+}
+__device__ __forceinline__ void fetch(uint32_t &d, const __nv_bfloat16 *p, bool ok) {
+    d = 0u;
+    if (ok) d = __ldg(reinterpret_cast<const unsigned short *>(p));
+}
+__device__ __forceinline__ void fetch8(Vec8<float> &d, const float *p) {
+    const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
+    const float4 b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
+    d.v[0] = a.x; d.v[1] = a.y; d.v[2] = a.z; d.v[3] = a.w;
+    d.v[4] = b.x; d.v[5] = b.y; d.v[6] = b.z; d.v[7] = b.w;
+}
+__device__ __forceinline__ void fetch8(Vec8<__nv_bfloat16> &d, const __nv_bfloat16 *p) {
+    const uint4 a = __ldg(reinterpret_cast<const uint4 *>(p));
+    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        d.v[2 * j] = w[j] & 0xffffu;
+        d.v[2 * j + 1] = w[j] >> 16;
+    }
+}
+
+// Bits whose upper halves are hi, mid and lo of an f32 value.  Rounding is half away from zero to 8
+// bits (the upper half of bits + 0x8000); both remainders are exact, of at most 16 and 8 bits.
+// A NaN must not wrap around, so an all-ones exponent becomes a NaN hi (its output is recomputed).
+__device__ __forceinline__ void split3(float v, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
+    uint32_t b = __float_as_uint(v);
+    b = (b & 0x7f800000u) == 0x7f800000u ? 0x7fc00000u : b + 0x8000u;
+    const float r = v - __uint_as_float(b & 0xffff0000u);
+    const uint32_t c = __float_as_uint(r) + 0x8000u;
+    hi = b;
+    mid = c;
+    lo = __float_as_uint(r - __uint_as_float(c & 0xffff0000u));
+}
+
+// Upper halves of two f32 words as one packed bf16 pair.
+__device__ __forceinline__ uint32_t upper_halves(uint32_t lo, uint32_t hi) {
+    return __byte_perm(lo, hi, 0x7632);
+}
+
+__device__ __forceinline__ void st_shared_v4(uint32_t dst, const uint32_t (&w)[4]) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                 "r"(w[3])
+                 : "memory");
+}
+
+// Writes eight k of one row into the tile's plane(s); dst = shared address of the 16-byte chunk
+// in plane 0, planes `plane_bytes` apart.
+__device__ __forceinline__ void put8(const Vec8<__nv_bfloat16> &x, uint32_t dst, uint32_t) {
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = __byte_perm(x.v[2 * j], x.v[2 * j + 1], 0x5410);
+    st_shared_v4(dst, w);
+}
+__device__ __forceinline__ void put8(const Vec8<float> &x, uint32_t dst, uint32_t plane_bytes) {
+    uint32_t h[4], m[4], l[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        uint32_t hb[2], mb[2], lb[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) split3(x.v[2 * j + i], hb[i], mb[i], lb[i]);
+        h[j] = upper_halves(hb[0], hb[1]);
+        m[j] = upper_halves(mb[0], mb[1]);
+        l[j] = upper_halves(lb[0], lb[1]);
+    }
+    st_shared_v4(dst, h);
+    st_shared_v4(dst + plane_bytes, m);
+    st_shared_v4(dst + 2 * plane_bytes, l);
+}
+
+// ---------------------------------------------------------------- operands
+// Concept (rows = the m or n index of the product):
+//   static constexpr bool kRowFast   memory is contiguous along the rows: a producer thread keeps
+//                                    one row (begin_row once per tile) and walks its k chunks;
+//                                    otherwise it keeps one k chunk (begin_chunk once per k
+//                                    step) and walks rows
+//   void load(const State &, table, int row, int k0, int k_end, Vec8<T> &) const
+//   float at(int row, int k) const   one element (the recomputation of a non-finite output)
+//   static constexpr int kTable      ints of shared memory prepared by init()
+
+// Strided matrix: element (row, k) at p[row * s_row + k * s_k].
+template <class T, bool ROW_FAST>
+struct Strided {
+    using value_type = T;
+    static constexpr bool kRowFast = ROW_FAST;
+    static constexpr int kTable = 0;
+    const T *p;
+    int64_t s_row, s_k;
+    int rows;
+    bool vec;  // s_k == 1, rows and base 16-byte aligned
+    struct State {};
+    __device__ __forceinline__ void init(int *, int, int) const {}
+    __device__ __forceinline__ void begin_row(State &, const int *, int) const {}
+    __device__ __forceinline__ void begin_chunk(State &, const int *, int, int) const {}
+    __device__ __forceinline__ void load(const State &, const int *, int row, int k0, int k_end,
+                                         Vec8<T> &d) const {
+        const T *q = p + (int64_t)row * s_row + (int64_t)k0 * s_k;
+        if (vec && row < rows && k0 + 8 <= k_end) {
+            fetch8(d, q);
+            return;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) fetch(d.v[j], q + j * s_k, row < rows && k0 + j < k_end);
+    }
+    __device__ __forceinline__ float at(int row, int k) const {
+        return to_f32(p[(int64_t)row * s_row + (int64_t)k * s_k]);
+    }
+};
+
+// Geometry of a convolution seen from a grid of positions [b][gh][gw]: position (b, y, x) and
+// filter tap (fi, fj) meet source element (sy, sx) of channel c of [b][channels][sh][sw].
+//   forward / weight gradient: sy = y * st_h - pad_h + fi * dil_h          (source = x)
+//   input gradient:            sy = (y + pad_h - fi * dil_h) / st_h, exact (source = dy)
+// In both cases the source address is separable, base(position) + offset(channel, tap): for the
+// input gradient (a - b) / s = floor(a / s) - floor(b / s) whenever s divides a - b.  Which taps
+// are valid at a position is a bit mask of at most 32 taps.
+struct ConvMap {
+    int channels, sh, sw;        // source planes
+    int gw, ghw;                 // position grid
+    int fh, fw, ff;
+    int st_h, st_w, pad_h, pad_w, dil_h, dil_w;
+    bool gradient;               // input-gradient form
+    bool always_valid;           // no tap of any position leaves the source
+    FastDiv div_ghw, div_gw, div_ff, div_fw, div_st_h, div_st_w;
+
+    __device__ __forceinline__ int tap_offset(int tap) const {
+        const int fi = (int)div_fw.div((uint32_t)tap), fj = tap - fi * fw;
+        if (gradient)
+            return -((int)div_st_h.div((uint32_t)(fi * dil_h)) * sw + (int)div_st_w.div((uint32_t)(fj * dil_w)));
+        return fi * dil_h * sw + fj * dil_w;
+    }
+    // Base address of a position and its tap mask.
+    __device__ __forceinline__ void position(int pos, int &base, uint32_t &mask) const {
+        uint32_t b, r, y, x;
+        div_ghw.divmod((uint32_t)pos, b, r);
+        div_gw.divmod(r, y, x);
+        const int image = (int)b * channels * sh * sw;
+        if (!gradient) {
+            const int y0 = (int)y * st_h - pad_h, x0 = (int)x * st_w - pad_w;
+            base = image + y0 * sw + x0;
+            if (always_valid) {
+                mask = 0xffffffffu;
+                return;
+            }
+            uint32_t cols = 0;
+            for (int fj = 0; fj < fw; ++fj)
+                if ((unsigned)(x0 + fj * dil_w) < (unsigned)sw) cols |= 1u << fj;
+            mask = 0;
+            for (int fi = 0; fi < fh; ++fi)
+                if ((unsigned)(y0 + fi * dil_h) < (unsigned)sh) mask |= cols << (fi * fw);
+        } else {
+            const int ty = (int)y + pad_h, tx = (int)x + pad_w;
+            base = image + (int)div_st_h.div((uint32_t)ty) * sw + (int)div_st_w.div((uint32_t)tx);
+            uint32_t cols = 0;
+            for (int fj = 0; fj < fw; ++fj) {
+                const int t = tx - fj * dil_w;
+                if (t < 0) break;
+                uint32_t q, rem;
+                div_st_w.divmod((uint32_t)t, q, rem);
+                if (rem == 0 && q < (uint32_t)sw) cols |= 1u << fj;
+            }
+            mask = 0;
+            for (int fi = 0; fi < fh; ++fi) {
+                const int t = ty - fi * dil_h;
+                if (t < 0) break;
+                uint32_t q, rem;
+                div_st_h.divmod((uint32_t)t, q, rem);
+                if (rem == 0 && q < (uint32_t)sh) mask |= cols << (fi * fw);
+            }
+        }
+    }
+};
+
+// Rows are positions, k = (channel, tap): the patch matrix of the forward pass and of the input
+// gradient.
+template <class T>
+struct ConvRows {
+    using value_type = T;
+    static constexpr bool kRowFast = true;
+    static constexpr int kTable = 32;
+    const T *src;
+    ConvMap g;
+    int rows;
+    struct State {
+        int base;
+        uint32_t mask;
+    };
+    __device__ __forceinline__ void init(int *table, int tid, int threads) const {
+        for (int t = tid; t < g.ff; t += threads) table[t] = g.tap_offset(t);
+    }
+    __device__ __forceinline__ void begin_row(State &s, const int *, int row) const {
+        s.base = 0;
+        s.mask = 0;
+        if (row < rows) g.position(row, s.base, s.mask);
+    }
+    __device__ __forceinline__ void begin_chunk(State &, const int *, int, int) const {}
+    __device__ __forceinline__ void load(const State &s, const int *table, int, int k0, int k_end,
+                                         Vec8<T> &d) const {
+        uint32_t c, tap;
+        g.div_ff.divmod((uint32_t)k0, c, tap);
+        const int plane = g.sh * g.sw;
+        int chan = s.base + (int)c * plane;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            fetch(d.v[j], src + (chan + table[tap]), k0 + j < k_end && ((s.mask >> tap) & 1u));
+            if (++tap == (uint32_t)g.ff) {
+                tap = 0;
+                chan += plane;
+            }
+        }
+    }
+    __device__ __forceinline__ float at(int row, int k) const {
+        int base;
+        uint32_t mask, c, tap;
+        g.position(row, base, mask);
+        g.div_ff.divmod((uint32_t)k, c, tap);
+        if (!((mask >> tap) & 1u)) return 0.f;
+        return to_f32(src[base + (int)c * g.sh * g.sw + g.tap_offset((int)tap)]);
+    }
+};
+
+// Rows are (channel, tap), k = positions: the transposed patch matrix of the weight gradient.
+template <class T>
+struct ConvCols {
+    using value_type = T;
+    static constexpr bool kRowFast = false;
+    static constexpr int kTable = 32;
+    const T *src;
+    ConvMap g;
+    int rows;
+    struct State {
+        int base[8];
+        uint32_t mask[8];
+    };
+    __device__ __forceinline__ void init(int *table, int tid, int threads) const {
+        for (int t = tid; t < g.ff; t += threads) table[t] = g.tap_offset(t);
+    }
+    __device__ __forceinline__ void begin_row(State &, const int *, int) const {}
+    __device__ __forceinline__ void begin_chunk(State &s, const int *, int k0, int k_end) const {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            s.base[j] = 0;
+            s.mask[j] = 0;
+            if (k0 + j < k_end) g.position(k0 + j, s.base[j], s.mask[j]);
+        }
+    }
+    __device__ __forceinline__ void load(const State &s, const int *table, int row, int, int,
+                                         Vec8<T> &d) const {
+        uint32_t c, tap;
+        g.div_ff.divmod((uint32_t)row, c, tap);
+        const bool ok = row < rows;
+        const T *q = src + (ok ? (int64_t)c * g.sh * g.sw + table[tap] : 0);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) fetch(d.v[j], q + s.base[j], ok && ((s.mask[j] >> tap) & 1u));
+    }
+    __device__ __forceinline__ float at(int row, int k) const {
+        int base;
+        uint32_t mask, c, tap;
+        g.position(k, base, mask);
+        g.div_ff.divmod((uint32_t)row, c, tap);
+        if (!((mask >> tap) & 1u)) return 0.f;
+        return to_f32(src[base + (int)c * g.sh * g.sw + g.tap_offset((int)tap)]);
+    }
+};
+
+// Rows are channels of an NCHW tensor, k = (image, position).
+template <class T>
+struct ChannelRows {
+    using value_type = T;
+    static constexpr bool kRowFast = false;
+    static constexpr int kTable = 0;
+    const T *src;
+    int rows, hw;
+    FastDiv div_hw;
+    bool vec;  // hw a multiple of 8 and the base 16-byte aligned
+    struct State {
+        int base[8];
+    };
+    __device__ __forceinline__ void init(int *, int, int) const {}
+    __device__ __forceinline__ void begin_row(State &, const int *, int) const {}
+    __device__ __forceinline__ void begin_chunk(State &s, const int *, int k0, int) const {
+        uint32_t b, r;
+        div_hw.divmod((uint32_t)k0, b, r);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            s.base[j] = (int)b * rows * hw + (int)r;
+            if (++r == (uint32_t)hw) {
+                r = 0;
+                ++b;
+            }
+        }
+    }
+    __device__ __forceinline__ void load(const State &s, const int *, int row, int k0, int k_end,
+                                         Vec8<T> &d) const {
+        if (vec && row < rows && k0 + 8 <= k_end) {
+            fetch8(d, src + (s.base[0] + row * hw));
+            return;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            fetch(d.v[j], src + (s.base[j] + row * hw), row < rows && k0 + j < k_end);
+    }
+    __device__ __forceinline__ float at(int row, int k) const {
+        uint32_t b, r;
+        div_hw.divmod((uint32_t)k, b, r);
+        return to_f32(src[((int64_t)b * rows + row) * hw + r]);
+    }
+};
+
+// Rows are input channels, k = (output channel, tap): w[k / ff][row][k % ff].
+template <class T>
+struct WeightRows {
+    using value_type = T;
+    static constexpr bool kRowFast = false;
+    static constexpr int kTable = 0;
+    const T *w;
+    int rows, ff;
+    FastDiv div_ff;
+    struct State {};
+    __device__ __forceinline__ void init(int *, int, int) const {}
+    __device__ __forceinline__ void begin_row(State &, const int *, int) const {}
+    __device__ __forceinline__ void begin_chunk(State &, const int *, int, int) const {}
+    __device__ __forceinline__ void load(const State &, const int *, int row, int k0, int k_end,
+                                         Vec8<T> &d) const {
+        uint32_t co, tap;
+        div_ff.divmod((uint32_t)k0, co, tap);
+        int at = ((int)co * rows + row) * ff + (int)tap;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            fetch(d.v[j], w + at, row < rows && k0 + j < k_end);
+            ++at;
+            if (++tap == (uint32_t)ff) {
+                tap = 0;
+                at += (rows - 1) * ff;
+            }
+        }
+    }
+    __device__ __forceinline__ float at(int row, int k) const {
+        uint32_t co, tap;
+        div_ff.divmod((uint32_t)k, co, tap);
+        return to_f32(w[((int64_t)co * rows + row) * ff + tap]);
+    }
+};
+
+// ---------------------------------------------------------------- epilogues
+// Concept: State begin(int row); void store(const State &, int row, int col, float acc).
+// A warp holds 32 consecutive rows of one column at a time, so the tensor written should be
+// contiguous along the rows.
+
+// C = alpha * acc + beta * C, element (row, col) at c[row * s_row + col * s_col].
+template <class T>
+struct StridedOut {
+    T *c;
+    int64_t s_row, s_col;
+    float alpha, beta;
+    struct State { T *q; };
+    __device__ __forceinline__ State begin(int row) const { return State{c + (int64_t)row * s_row}; }
+    __device__ __forceinline__ void store(const State &s, int, int col, float acc) const {
+        T *q = s.q + (int64_t)col * s_col;
+        float v = alpha * acc;
+        if (beta != 0.f) v += beta * to_f32(*q);
+        *q = from_f32<T>(v);
+    }
+};
+
+// y[col][row] = relu?(round(round(acc) + bias[row])): a Dense layer with rows = outputs.
+template <class T>
+struct DenseOut {
+    T *c;
+    int64_t s_col;
+    const T *bias;
+    bool relu;
+    struct State { T *q; float b; };
+    __device__ __forceinline__ State begin(int row) const {
+        return State{c + row, bias != nullptr ? to_f32(bias[row]) : 0.f};
+    }
+    __device__ __forceinline__ void store(const State &s, int, int col, float acc) const {
+        float v = to_f32(from_f32<T>(acc));
+        if (bias != nullptr) v = to_f32(from_f32<T>(__fadd_rn(v, s.b)));
+        if (relu) v = (v >= 0.f) ? v : 0.f;
+        s.q[(int64_t)col * s_col] = from_f32<T>(v);
+    }
+};
+
+// Rows are (image, position), columns channels of an NCHW tensor; optional bias and relu with
+// the roundings of the separate operators.
+template <class T>
+struct NchwOut {
+    T *y;
+    const T *bias;
+    int channels, hw;
+    FastDiv div_hw;
+    bool relu;
+    struct State { T *q; };
+    __device__ __forceinline__ State begin(int row) const {
+        uint32_t b, r;
+        div_hw.divmod((uint32_t)row, b, r);
+        return State{y + ((int64_t)b * channels * hw + r)};
+    }
+    __device__ __forceinline__ void store(const State &s, int, int col, float acc) const {
+        float v = to_f32(from_f32<T>(acc));
+        if (bias != nullptr) v = to_f32(from_f32<T>(v + to_f32(bias[col])));
+        if (relu) v = (v >= 0.f) ? v : 0.f;
+        s.q[(int64_t)col * hw] = from_f32<T>(v);
+    }
+};
+
+// ------------------------------------------------------------------- kernel
+template <class T, int BN_>
+struct Cfg {
+    static constexpr int PL = Planes<T>::N;
+    static constexpr int BN = BN_;
+    static constexpr int EPI_WARPS = BN >= 64 ? 8 : 4;
+    static constexpr int COLS = BN * 4 / EPI_WARPS;              // columns per epilogue warp
+    static constexpr int THREADS = PRODUCERS + EPI_WARPS * 32 + 32;
+    static constexpr int A_PLANE = BM * ROW_BYTES, B_PLANE = BN * ROW_BYTES;
+    static constexpr int STAGE = PL * (A_PLANE + B_PLANE);
+    static constexpr int STAGES = PL == 3 ? (BN > 64 ? 2 : 3) : 4;
+    static constexpr int ACC_COLS = PL == 3 ? 2 * BN : BN;       // f32: leading block + corrections
+    static constexpr int TMEM = 2 * ACC_COLS < 64 ? 64 : 2 * ACC_COLS;
+    static constexpr int SMEM = STAGES * STAGE + 1024 + 512;
+    static_assert(TMEM <= 512 && (TMEM & (TMEM - 1)) == 0, "tensor memory columns");
+    static_assert(COLS % 16 == 0, "epilogue warps read 16 columns at a time");
+};
+
+struct Params {
+    int M, N, K;
+    int tiles_m, tiles_n, splits, k_split;  // k_split: k per slice, a multiple of BK
+    float *partial;                         // splits > 1: [splits][N][M] f32 sums
+    int *status;
+};
+
+// 32 lanes x 16 columns.
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+          "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+
+// Exact-f32 recomputation of an output whose split sum is not finite.
+template <class AOp, class BOp>
+__device__ __noinline__ float recompute(const AOp &A, const BOp &B, int row, int col, int k0, int k1) {
+    float s = 0.f;
+    for (int k = k0; k < k1; ++k) s = fmaf(A.at(row, k), B.at(col, k), s);
+    return s;
+}
+
+template <class T, int BN, class AOp, class BOp, class Epi>
+__global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
+    gemm_tcx_kernel(const __grid_constant__ AOp A, const __grid_constant__ BOp B,
+                    const __grid_constant__ Epi E, const Params p) {
+    using C = Cfg<T, BN>;
+    constexpr int PL = C::PL, STAGES = C::STAGES;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                                ~uintptr_t(1023));
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + STAGES * C::STAGE);
+    uint64_t *full_bar = bars, *empty_bar = bars + STAGES;
+    uint64_t *acc_full = bars + 2 * STAGES, *acc_empty = bars + 2 * STAGES + 2;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    int *table_a = reinterpret_cast<int *>(tmem_slot + 2), *table_b = table_a + 32;
+
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    constexpr int MMA_WARP = PRODUCERS / 32 + C::EPI_WARPS;
+
+    if (tid == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            tc::mbar_init(tc::smem_u32(&full_bar[s]), PRODUCERS / 32);
+            tc::mbar_init(tc::smem_u32(&empty_bar[s]), 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            tc::mbar_init(tc::smem_u32(&acc_full[s]), 1);
+            tc::mbar_init(tc::smem_u32(&acc_empty[s]), C::EPI_WARPS);
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == MMA_WARP) {
+        tc::tmem_alloc(tc::smem_u32(tmem_slot), C::TMEM);
+        tc::tmem_relinquish();
+    }
+    if (AOp::kTable) A.init(table_a, tid, C::THREADS);
+    if (BOp::kTable) B.init(table_b, tid, C::THREADS);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    const int tiles = p.tiles_m * p.tiles_n;
+    const int num_work = tiles * p.splits;
+
+    if (warp < PRODUCERS / 32) {
+        // ------------------------------------------------------------------ producers
+        constexpr int A_PER = BM * 8 / PRODUCERS;                       // row chunks per thread
+        constexpr int B_PER = BN * 8 / PRODUCERS < 1 ? 1 : BN * 8 / PRODUCERS;
+        int stage = 0;
+        uint32_t phase = 0;
+        for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
+            const int tile = w % tiles, z = w / tiles;
+            const int m0 = (tile % p.tiles_m) * BM, n0 = (tile / p.tiles_m) * BN;
+            const int k_begin = z * p.k_split, k_end = min(p.K, k_begin + p.k_split);
+            // slot i of a thread: row-fast operands keep the row, the others the chunk
+            const int ar = AOp::kRowFast ? (tid & (BM - 1)) : (tid >> 3);
+            const int ac = AOp::kRowFast ? tid / BM : (tid & 7);
+            const int br = BOp::kRowFast ? (tid & (BN - 1)) : (tid >> 3);
+            const int bc = BOp::kRowFast ? tid / BN : (tid & 7);
+            typename AOp::State sa;
+            typename BOp::State sb;
+            if (AOp::kRowFast) A.begin_row(sa, table_a, m0 + ar);
+            if (BOp::kRowFast) B.begin_row(sb, table_b, n0 + br);
+            bool ok = true;
+            for (int k0 = k_begin; k0 < k_end; k0 += BK) {
+                Vec8<T> va[A_PER], vb[B_PER];
+                if (!AOp::kRowFast) A.begin_chunk(sa, table_a, k0 + ac * 8, k_end);
+#pragma unroll
+                for (int i = 0; i < A_PER; ++i) {
+                    const int row = AOp::kRowFast ? ar : ar + i * (PRODUCERS / 8);
+                    const int ch = AOp::kRowFast ? ac + i * (PRODUCERS / BM) : ac;
+                    A.load(sa, table_a, m0 + row, k0 + ch * 8, k_end, va[i]);
+                }
+                if (!BOp::kRowFast) B.begin_chunk(sb, table_b, k0 + bc * 8, k_end);
+#pragma unroll
+                for (int i = 0; i < B_PER; ++i) {
+                    const int row = BOp::kRowFast ? br : br + i * (PRODUCERS / 8);
+                    const int ch = BOp::kRowFast ? bc + i * (PRODUCERS / BN) : bc;
+                    B.load(sb, table_b, n0 + row, k0 + ch * 8, k_end, vb[i]);
+                }
+                if (!tc::mbar_wait(tc::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag)) {
+                    if (lane == 0) atomicExch(p.status, 181);
+                    ok = false;
+                    break;
+                }
+                const uint32_t a_base = tc::smem_u32(smem + stage * C::STAGE);
+                const uint32_t b_base = a_base + PL * C::A_PLANE;
+#pragma unroll
+                for (int i = 0; i < A_PER; ++i) {
+                    const int row = AOp::kRowFast ? ar : ar + i * (PRODUCERS / 8);
+                    const int ch = AOp::kRowFast ? ac + i * (PRODUCERS / BM) : ac;
+                    put8(va[i], a_base + row * ROW_BYTES + ((ch ^ (row & 7)) << 4), C::A_PLANE);
+                }
+#pragma unroll
+                for (int i = 0; i < B_PER; ++i) {
+                    const int row = BOp::kRowFast ? br : br + i * (PRODUCERS / 8);
+                    const int ch = BOp::kRowFast ? bc + i * (PRODUCERS / BN) : bc;
+                    put8(vb[i], b_base + row * ROW_BYTES + ((ch ^ (row & 7)) << 4), C::B_PLANE);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(tc::smem_u32(&full_bar[stage]));
+                if (++stage == STAGES) {
+                    stage = 0;
+                    phase ^= 1;
+                }
+            }
+            if (!ok) break;
+        }
+    } else if (warp == MMA_WARP) {
+        // ------------------------------------------------------------------ MMA issue
+        if (lane == 0) {
+            constexpr uint32_t idesc1 = tc::make_idesc(false, false, BM, BN);
+            constexpr uint32_t idesc2 = tc::make_idesc(false, false, BM, PL == 3 ? 2 * BN : BN);
+            int stage = 0, acc = 0;
+            uint32_t phase = 0, acc_phase = 0;
+            bool ok = true;
+            for (int w = blockIdx.x; ok && w < num_work; w += gridDim.x) {
+                const int k_begin = (w / tiles) * p.k_split, k_end = min(p.K, k_begin + p.k_split);
+                for (int k0 = k_begin; k0 < k_end; k0 += BK) {
+                    if (PL == 3 || k0 == k_begin) {
+                        if (!tc::mbar_wait(tc::smem_u32(&acc_empty[acc]), acc_phase ^ 1, abort_flag)) {
+                            atomicExch(p.status, 182);
+                            ok = false;
+                            break;
+                        }
+                    }
+                    if (!tc::mbar_wait(tc::smem_u32(&full_bar[stage]), phase, abort_flag)) {
+                        atomicExch(p.status, 183);
+                        ok = false;
+                        break;
+                    }
+                    tc::tc_fence_after();
+                    const uint32_t d = tmem + acc * C::ACC_COLS;
+                    const uint32_t a_base = tc::smem_u32(smem + stage * C::STAGE);
+                    const uint32_t b_base = a_base + PL * C::A_PLANE;
+                    if (PL == 1) {
+#pragma unroll
+                        for (int k = 0; k < BK / 16; ++k)
+                            tc::umma_bf16(d, tc::make_smem_desc(a_base + k * 32, 0, 1024),
+                                          tc::make_smem_desc(b_base + k * 32, 0, 1024), idesc1,
+                                          (k0 > k_begin || k > 0) ? 1u : 0u);
+                    } else {
+                        // corrections first: column block 0 collects hi.mid, mid.hi, lo.hi, block 1
+                        // hi.lo and mid.mid; then the leading products into block 0
+#pragma unroll
+                        for (int k = 0; k < BK / 16; ++k) {
+                            const uint64_t a_hi = tc::make_smem_desc(a_base + k * 32, 0, 1024);
+                            const uint64_t a_mid = tc::make_smem_desc(a_base + C::A_PLANE + k * 32, 0, 1024);
+                            const uint64_t a_lo = tc::make_smem_desc(a_base + 2 * C::A_PLANE + k * 32, 0, 1024);
+                            const uint64_t b_hi = tc::make_smem_desc(b_base + k * 32, 0, 1024);
+                            const uint64_t b_mid = tc::make_smem_desc(b_base + C::B_PLANE + k * 32, 0, 1024);
+                            tc::umma_bf16(d, a_hi, b_mid, idesc2, k > 0 ? 1u : 0u);   // b_mid, b_lo
+                            tc::umma_bf16(d, a_mid, b_hi, idesc2, 1u);                // b_hi, b_mid
+                            tc::umma_bf16(d, a_lo, b_hi, idesc1, 1u);
+                        }
+#pragma unroll
+                        for (int k = 0; k < BK / 16; ++k)
+                            tc::umma_bf16(d, tc::make_smem_desc(a_base + k * 32, 0, 1024),
+                                          tc::make_smem_desc(b_base + k * 32, 0, 1024), idesc1, 1u);
+                    }
+                    tc::umma_commit(tc::smem_u32(&empty_bar[stage]));
+                    if (++stage == STAGES) {
+                        stage = 0;
+                        phase ^= 1;
+                    }
+                    if (PL == 3 || k0 + BK >= k_end) {
+                        tc::umma_commit(tc::smem_u32(&acc_full[acc]));
+                        if (++acc == 2) {
+                            acc = 0;
+                            acc_phase ^= 1;
+                        }
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------------------------------------------ epilogue
+        const int e = warp - PRODUCERS / 32;
+        const int quarter = warp % 4;
+        const int col_base = (e / 4) * C::COLS;
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        bool ok = true;
+        for (int w = blockIdx.x; ok && w < num_work; w += gridDim.x) {
+            const int tile = w % tiles, z = w / tiles;
+            const int m0 = (tile % p.tiles_m) * BM, n0 = (tile / p.tiles_m) * BN;
+            const int k_begin = z * p.k_split, k_end = min(p.K, k_begin + p.k_split);
+            const int steps = PL == 3 ? (k_end - k_begin + BK - 1) / BK : 1;
+            float sum[C::COLS];
+#pragma unroll
+            for (int j = 0; j < C::COLS; ++j) sum[j] = 0.f;
+            for (int s = 0; s < steps; ++s) {
+                if (!tc::mbar_wait(tc::smem_u32(&acc_full[acc]), acc_phase, abort_flag)) {
+                    if (lane == 0) atomicExch(p.status, 184);
+                    ok = false;
+                    break;
+                }
+                tc::tc_fence_after();
+                const uint32_t t = tmem + acc * C::ACC_COLS + col_base + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll
+                for (int c = 0; c < C::COLS; c += 16) {
+                    uint32_t r0[16], r1[16];
+                    tmem_ld_32x16(t + c, r0);
+                    if (PL == 3) tmem_ld_32x16(t + BN + c, r1);
+                    tc::tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        float v = __uint_as_float(r0[j]);
+                        if (PL == 3) v = sum[c + j] + (v + __uint_as_float(r1[j]));
+                        sum[c + j] = v;
+                    }
+                }
+                tc::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(tc::smem_u32(&acc_empty[acc]));
+                if (++acc == 2) {
+                    acc = 0;
+                    acc_phase ^= 1;
+                }
+            }
+            if (!ok) break;
+            const int row = m0 + quarter * 32 + lane;
+            const int col0 = n0 + col_base;
+            const bool in = row < p.M;
+            // a sum that is not finite makes the row's columns take the exact path
+            float finite = 0.f;
+            if (PL == 3) {
+#pragma unroll
+                for (int j = 0; j < C::COLS; ++j) finite = fmaf(sum[j], 0.f, finite);
+            }
+            if (in && !(finite == 0.f)) {
+                const typename Epi::State st = E.begin(row);
+#pragma unroll 1
+                for (int col = col0; col < min(p.N, col0 + C::COLS); ++col) {
+                    const float v = recompute(A, B, row, col, k_begin, k_end);
+                    if (p.splits > 1)
+                        p.partial[((int64_t)z * p.N + col) * p.M + row] = v;
+                    else
+                        E.store(st, row, col, v);
+                }
+            } else if (in && p.splits > 1) {
+                float *q = p.partial + (int64_t)z * p.M * p.N + row;
+#pragma unroll
+                for (int j = 0; j < C::COLS; ++j)
+                    if (col0 + j < p.N) q[(int64_t)(col0 + j) * p.M] = sum[j];
+            } else if (in) {
+                const typename Epi::State st = E.begin(row);
+#pragma unroll
+                for (int j = 0; j < C::COLS; ++j)
+                    if (col0 + j < p.N) E.store(st, row, col0 + j, sum[j]);
+            }
+            __syncwarp();  // the next tensor-memory load is a warp-wide instruction
+        }
+    }
+
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == MMA_WARP) {
+        tc::tc_fence_after();
+        if (*abort_flag) {   // let MMAs in flight finish before their tensor memory is given back
+            const uint64_t t0 = tc::global_timer_ns();
+            while (tc::global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+        }
+        tc::tmem_dealloc(tmem, C::TMEM);
+    }
+}
+
+// out = epilogue(sum over slices in slice order).
+template <class Epi>
+__global__ void __launch_bounds__(256)
+    reduce_splits_kernel(const float *partial, int splits, int M, int N, FastDiv div_m, Epi E) {
+    const int64_t plane = (int64_t)M * N;
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= plane) return;
+    const float *q = partial + i;
+    float s = 0.f;
+    int z = 0;
+    for (; z + 4 <= splits; z += 4) {
+        const float a = q[(int64_t)z * plane], b = q[(int64_t)(z + 1) * plane],
+                    c = q[(int64_t)(z + 2) * plane], d = q[(int64_t)(z + 3) * plane];
+        s = s + a;
+        s = s + b;
+        s = s + c;
+        s = s + d;
+    }
+    for (; z < splits; ++z) s += q[(int64_t)z * plane];
+    const int col = (int)(i / M), row = (int)(i - (int64_t)col * M);
+    E.store(E.begin(row), row, col, s);
+}
+
+// --------------------------------------------------------------------- host
+template <class T, int BN, class AOp, class BOp, class Epi>
+int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
+    using C = Cfg<T, BN>;
+    p.tiles_m = (int)ceil_div(p.M, BM);
+    p.tiles_n = (int)ceil_div(p.N, BN);
+    const int64_t tiles = (int64_t)p.tiles_m * p.tiles_n;
+    // Slices of k fill the SMs that whole tiles leave idle; at least two k steps each.
+    const int steps = (int)ceil_div(p.K, BK);
+    int splits = 1;
+    if (tiles * 2 <= dev->sm_count && steps >= 4) {
+        splits = (int)(dev->sm_count / tiles);
+        if (splits > steps / 2) splits = steps / 2;
+    }
+    const int per = (int)ceil_div(steps, splits);
+    p.k_split = per * BK;
+    p.splits = (int)ceil_div(steps, per);
+    p.status = dev->status_dev;
+    p.partial = nullptr;
+    if (p.splits > 1) {
+        void *ws = nullptr;
+        AG_TRY(engine_scratch(dev, sizeof(float) * (size_t)p.splits * p.M * p.N, &ws));
+        p.partial = (float *)ws;
+    }
+    auto kernel = gemm_tcx_kernel<T, BN, AOp, BOp, Epi>;
+    static bool configured_on[64] = {};
+    bool &configured = configured_on[dev->ordinal & 63];
+    if (!configured) {
+        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+        configured = true;
+    }
+    const int64_t work = tiles * p.splits;
+    const int grid = (int)(work < dev->sm_count ? work : dev->sm_count);
+    kernel<<<grid, C::THREADS, C::SMEM, dev->stream>>>(A, B, E, p);
+    AG_CHECK_LAUNCH();
+    if (p.splits > 1) {
+        reduce_splits_kernel<Epi><<<(unsigned)ceil_div((int64_t)p.M * p.N, 256), 256, 0, dev->stream>>>(
+            p.partial, p.splits, p.M, p.N, FastDiv((uint32_t)p.M), E);
+        AG_CHECK_LAUNCH();
+    }
+    return AG_OK;
+}
+
+// Tile width: the narrowest that holds all columns, else 128 columns when the tiles fill the GPU.
+template <class T, class AOp, class BOp, class Epi>
+int gemm(ag_device *dev, int M, int N, int K, const AOp &A, const BOp &B, const Epi &E) {
+    Params p = {};
+    p.M = M;
+    p.N = N;
+    p.K = K;
+    if (N <= 32) return launch<T, 32>(dev, A, B, E, p);
+    const int64_t tiles = ceil_div(M, BM) * ceil_div(N, 128);
+    if (N <= 64 || tiles * 2 <= dev->sm_count) return launch<T, 64>(dev, A, B, E, p);
+    return launch<T, 128>(dev, A, B, E, p);
+}
+
+}  // namespace tcx
+}  // namespace ag

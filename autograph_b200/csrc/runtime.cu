@@ -56,6 +56,13 @@ int staging(ag_device *dev, size_t bytes, void **out) {
     return AG_OK;
 }
 
+int engine_scratch(ag_device *dev, size_t bytes, void **out) {
+    if (bytes > dev->engine_bytes)
+        AG_TRY(grow_block(dev, &dev->engine, &dev->engine_bytes, bytes, size_t(8) << 20));
+    *out = dev->engine;
+    return AG_OK;
+}
+
 static int device_init(int ordinal, cudaStream_t stream, bool owns, ag_device **out) {
     AG_REQUIRE(out != nullptr, AG_ERR_INVALID, "out is null");
     int count = 0;
@@ -153,6 +160,7 @@ int ag_device_destroy(ag_device *dev) {
     if (dev->stream) cudaStreamSynchronize(dev->stream);
     if (dev->workspace) cudaFree(dev->workspace);
     if (dev->staging) cudaFree(dev->staging);
+    if (dev->engine) cudaFree(dev->engine);
     for (void *p : dev->retired) cudaFree(p);
     if (dev->status_dev) cudaFree(dev->status_dev);
     if (dev->scalar_dev) cudaFree(dev->scalar_dev);

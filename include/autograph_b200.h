@@ -118,7 +118,9 @@ AG_API int ag_fill_zero(ag_device *dev, void *dptr, size_t bytes);
  * transposed view; never a copy).  bf16 inputs are multiplied and accumulated
  * in f32 and the result is rounded once (linalg.rs:244).  beta == 0 never
  * reads C.  Large-k, small-output products are split along k with f32 partial
- * sums and a fixed reduction order (deterministic). */
+ * sums and a fixed reduction order (deterministic).  f32 products of 3e7 and more multiply-adds
+ * run on the tensor cores with every operand split into three bf16 values that add up to it
+ * (f32-accurate: the error against an f64 product is below that of a chain of f32 FMAs). */
 AG_API int ag_gemm(ag_device *dev, ag_dtype dtype, int64_t m, int64_t k, int64_t n, float alpha,
                    const void *a, int64_t off_a, int64_t rsa, int64_t csa,
                    const void *b, int64_t off_b, int64_t rsb, int64_t csb,
@@ -243,7 +245,8 @@ AG_API int ag_conv2_relu_max_pool2_forward_keep(ag_device *dev, ag_dtype dtype, 
  * autograph_backend.rs:129-146) -- as ONE kernel that keeps every activation in shared memory.
  * x [bs, ic, ih, iw]; dense arguments as in ag_dense_chain_forward (dims[0] must equal the
  * flattened size of the last stage); y [bs, dims[n_dense]].  Equals the layer-by-layer calls bit
- * for bit.  Only networks that fit the kernel are taken (default convolution options, one 5x5 or
+ * for bit while every dense layer has at most 512 inputs and bs * inputs * outputs is at most
+ * 1.7e8 (beyond, ag_dense_forward adds in another order and the results agree to rounding).  Only networks that fit the kernel are taken (default convolution options, one 5x5 or
  * 3x3 filter size, 2x2 pools, <= 16 input and <= 64 output channels per stage, dense layers with
  * <= 2048 inputs and <= 256 outputs, 8 images of every activation within one CTA's shared
  * memory); any other network returns AG_ERR_UNSUPPORTED without touching y, and the caller runs

@@ -1,0 +1,144 @@
+"""GPU: the tensor-core engines for operands TMA cannot read as they are (f32 split into bf16
+planes, unaligned bf16, convolutions with any options) against float64."""
+import numpy as np
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _views(a, b, layout):
+    return (a.T if layout[0] == "t" else a), (b.T if layout[1] == "t" else b)
+
+
+def _f32_bound(av, bv, k):
+    """Per-element bound, S = sum |a||b|: in every 64-k block four additions of full-size terms and
+    twenty of terms 2^-8 of that truncate to 24 bits (below 5 * 2^-23 S), the partial products left
+    out are below 2^-24 S, and the k / 64 block sums are added with a rounding of 2^-24 each; k
+    slices add at most as many roundings again."""
+    s = av.double().abs() @ bv.double().abs()
+    return s * (5 * 2.0 ** -23 + 2.0 ** -24 + 2 * (k / 64 + 1) * 2.0 ** -24)
+
+
+@pytest.mark.parametrize("layout", ["nn", "nt", "tn", "tt"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [
+    # gathered engine: one 32 / 64 / 128 column tile with ragged edges, k not a multiple of 8 or 64
+    (2049, 513, 31), (4001, 165, 63), (257, 1030, 129), (1300, 333, 1301),
+    # k slices, the last one short
+    (130, 8003, 33),
+    # packed engine: slices of k, whole tiles, tiles of a partial wave cut in two
+    (1000, 5001, 130), (1537, 1601, 1703), (2560, 321, 2050),
+])
+def test_product_vs_f64(dev, dtype, layout, shape):
+    m, k, n = shape
+    gen = torch.Generator(device=dev.torch_device).manual_seed(m + k + n)
+    mk = lambda r, c: (torch.rand((r, c), generator=gen, device=dev.torch_device) * 2 - 1).to(dtype)
+    a = mk(*((m, k) if layout[0] == "n" else (k, m)))
+    b = mk(*((k, n) if layout[1] == "n" else (n, k)))
+    av, bv = _views(a, b, layout)
+    c = dev.dot(av, bv)
+    assert torch.equal(c, dev.dot(av, bv))
+    ref = av.double() @ bv.double()
+    err = (c.double() - ref).abs()
+    bound = _f32_bound(av, bv, k)
+    if dtype == torch.bfloat16:
+        bound = ref.abs() * 2.0 ** -8 + bound * 64   # one bf16 store; truncating sums over all k
+    assert (err <= bound).all()
+    # alpha, beta and a view of C, exact on small integers
+    ai, bi = (torch.randint(-2, 3, t.shape, generator=gen, device=dev.torch_device).to(dtype) for t in (a, b))
+    c0 = torch.randint(-4, 5, (m, n + 3), generator=gen, device=dev.torch_device).to(dtype)
+    want = c0.double()
+    want[:, 1:n + 1] = 0.5 * (_views(ai, bi, layout)[0].double() @ _views(ai, bi, layout)[1].double()) + 2 * want[:, 1:n + 1]
+    dev.gemm(0.5, *_views(ai, bi, layout), 2.0, c0[:, 1:n + 1])
+    assert torch.equal(c0, want.to(dtype))
+    dev.wait()
+
+
+@pytest.mark.parametrize("shape", [(700, 300, 200), (1100, 700, 1300)])
+def test_f32_special_values(dev, shape):
+    """Infinities, NaNs and values that round up to infinity in bf16 give what f32 gives; the rest
+    of the product is not disturbed."""
+    m, k, n = shape
+    rng = np.random.default_rng(3)
+    a = rng.integers(-3, 4, (m, k)).astype(np.float32)
+    b = rng.integers(1, 4, (k, n)).astype(np.float32)
+    a[3, 5], a[7, 9], a[11, 2], b[4, 6] = np.inf, np.nan, np.finfo(np.float32).max, -np.inf
+    a[11, :] = np.where(np.arange(k) == 2, a[11, 2], 0)
+    b[2, :] = np.where(np.arange(n) % 2, 1.0, 2.0)     # 2 * max overflows, 1 * max does not
+    with np.errstate(all="ignore"):
+        want = (a.astype(np.float64) @ b.astype(np.float64)).astype(np.float32)
+    got = dev.dot(dev.tensor(a), dev.tensor(b)).cpu().numpy()
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(got[~np.isnan(got)], want[~np.isnan(want)])
+
+
+CONVS = [
+    # bs, ic, ih, iw, oc, f, padding, stride, dilation
+    (9, 5, 31, 27, 33, 3, 1, 1, 1), (6, 16, 32, 32, 70, 3, 1, 2, 1), (5, 24, 29, 30, 130, 5, 2, 1, 1),
+    (4, 33, 23, 41, 7, 3, 2, 2, 2), (7, 6, 40, 17, 96, (5, 3), (2, 0), (3, 1), (1, 2)),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("case", CONVS)
+def test_convolution_vs_f64(dev, dtype, case):
+    bs, ic, ih, iw, oc, f, pad, st, dil = case
+    pair = lambda v: v if isinstance(v, tuple) else (v, v)
+    f = pair(f)
+    kw = dict(padding=pair(pad), stride=pair(st), dilation=pair(dil))
+    gen = torch.Generator(device=dev.torch_device).manual_seed(ic * oc)
+    rnd = lambda s: torch.randn(s, generator=gen, device=dev.torch_device).to(dtype)
+    x, w = rnd((bs, ic, ih, iw)), rnd((oc, ic) + f)
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    y = F.conv2d(xd, wd, **kw)
+    dy = rnd(tuple(y.shape))
+    dx, dw = torch.autograd.grad(y, (xd, wd), dy.double())
+    xa, wa = x.double().abs().requires_grad_(), w.double().abs().requires_grad_()
+    ya = F.conv2d(xa, wa, **kw)
+    dxa, dwa = torch.autograd.grad(ya, (xa, wa), dy.double().abs())
+    got = (dev.conv2_forward(x, w, **kw), dev.conv2_backward_input(w, dy, (ih, iw), **kw),
+           dev.conv2_backward_weight(x, dy, f, **kw))
+    ks = (ic * f[0] * f[1], oc * f[0] * f[1], bs * y.shape[2] * y.shape[3])
+    for g, ref, s, k in zip(got, (y, dx, dw), (ya, dxa, dwa), ks):
+        bound = s * (5 * 2.0 ** -23 + 2.0 ** -24 + 2 * (k / 64 + 1) * 2.0 ** -24)   # as in _f32_bound
+        if dtype == torch.bfloat16:
+            bound = ref.abs() * 2.0 ** -8 + bound * 64
+        assert ((g.double() - ref).abs() <= bound).all()
+    dw2 = dev.conv2_backward_weight(x, dy, f, beta=1.0, dw=torch.ones_like(w), **kw)
+    assert ((dw2.double() - dw - 1).abs() <= (bound * 1.01 + (dw.abs() + 1) * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23))).all()
+    # the fused bias + relu equals the separate calls bit for bit
+    b = rnd((oc,))
+    assert torch.equal(dev.conv2_forward(x, w, bias=b, relu=True, **kw), dev.relu(dev.bias_add(got[0].clone(), b)))
+    dev.wait()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(777, 333, 129), (5001, 260, 131), (1500, 1001, 900)])
+def test_dense_epilogue(dev, dtype, shape):
+    """Bias and relu in either engine's epilogue equal the product and the separate calls."""
+    bs, ins, outs = shape
+    gen = torch.Generator(device=dev.torch_device).manual_seed(bs)
+    rnd = lambda s: (torch.rand(s, generator=gen, device=dev.torch_device) - 0.5).to(dtype)
+    x, w, b = rnd((bs, ins)), rnd((ins, outs)), rnd((outs,))
+    assert torch.equal(dev.dense_forward(x, w, bias=b, relu=True),
+                       dev.relu(dev.bias_add(dev.dot(x, w), b), inplace=True))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(1, 40, 33), (3, 512, 256), (75, 129, 64), (149, 17, 200), (600, 84, 10),
+                                   (1200, 300, 100), (7, 8, 32)])
+def test_small_products(dev, dtype, shape):
+    """Every split of rows over CTAs of the latency-oriented kernel, ragged in all dimensions."""
+    m, k, n = shape
+    gen = torch.Generator(device=dev.torch_device).manual_seed(m)
+    rnd = lambda s: (torch.rand(s, generator=gen, device=dev.torch_device) * 2 - 1).to(dtype)
+    x, w, b = rnd((m, k)), rnd((k, n)), rnd((n,))
+    ref = x.double() @ w.double()
+    bound = x.double().abs() @ w.double().abs() * (k + 2) * 2.0 ** -24   # any order of k f32 roundings
+    if dtype == torch.bfloat16:
+        bound = bound + ref.abs() * 2.0 ** -8
+    c = dev.dot(x, w)
+    assert ((c.double() - ref).abs() <= bound).all()
+    assert torch.equal(dev.dense_forward(x, w, bias=b, relu=True), dev.relu(dev.bias_add(c, b)))
