@@ -212,7 +212,7 @@ static size_t make_plan(Plan *pl, int64_t bs, int64_t ic, int64_t ih, int64_t iw
     }
     if (c * h * w != layers[0].inputs) return 0;
     for (int i = 0; i < n_dense; ++i) {
-        if (!dense_small::eligible(ROWS, layers[i].inputs, layers[i].outputs)) return 0;
+        if (!dense_small::fits_one_kernel(layers[i].inputs, layers[i].outputs)) return 0;
         if (i > 0 && layers[i].inputs != layers[i - 1].outputs) return 0;
     }
     dense_small::plan_chain(&pl->chain, (int)bs, n_dense, layers);

@@ -463,7 +463,7 @@ inline size_t make_plan(Plan *pl, ag_dtype dtype, int64_t bs, int64_t ic, int64_
     }
     if (n_dense < 1 || n_dense > dense_small::kMaxChain || layers[0].inputs != kFlat) return 0;
     for (int i = 0; i < n_dense; ++i) {
-        if (!dense_small::eligible(ROWS, layers[i].inputs, layers[i].outputs)) return 0;
+        if (!dense_small::fits_one_kernel(layers[i].inputs, layers[i].outputs)) return 0;
         if (i > 0 && layers[i].inputs != layers[i - 1].outputs) return 0;
     }
     const size_t es = dtype_size(dtype);

@@ -1,70 +1,148 @@
-// Latency-oriented kernel for small dense products (m up to a few thousand
+// Latency-oriented kernels for small dense products (m up to a few thousand
 // rows, n <= 256 outputs): y[m,n] = x[m,k] . w[k,n] (+ bias) (relu), row-major.
 //
 // At these sizes a shared-memory-tiled GEMM runs two warps per SM through a
 // chain of load -> barrier -> multiply steps and is bound by memory and
-// instruction-fetch latency.  Here a CTA owns 8 rows of x (staged once in
-// shared memory, transposed so that the 8 row values of one k are two 16-byte
-// loads) and up to 1024 threads split the work as (output column, k slice):
-// each thread streams its weights straight from L2 with coalesced loads and
-// keeps 8 accumulators.  The k slices are then summed in a fixed order, so the
-// result is deterministic.  The code is small on purpose.
+// instruction-fetch latency.  Here the threads of a CTA split the work as
+// (output column, k slice): each streams its weights straight from L2 with
+// coalesced loads and keeps one accumulator per row; the k slices are then
+// summed in a fixed order, so the result is deterministic.  How k is sliced
+// depends on (k, n) alone and every kernel that runs such a layer -- a single
+// product, a chain of layers, a whole network -- adds in that order, so their
+// bits agree.
 #include "dense_small.cuh"
 #include "dense_small_device.cuh"
 
 namespace ag {
 namespace dense_small {
 
+// One layer of the chain's code on 8 rows per CTA: layers with at most 16 outputs, and batches
+// large enough to fill the GPU at 8 rows per CTA.
 template <class T>
 __global__ void __launch_bounds__(1024)
-    dense_small_kernel(const T *__restrict__ x, const T *__restrict__ w,
-                       const T *__restrict__ bias, T *__restrict__ y, int M, int K, int N, int np,
-                       int slices, int kchunk, int relu) {
+    dense_rows_kernel(const T *__restrict__ x, T *__restrict__ y, int M, const ChainStep st) {
     extern __shared__ __align__(16) float smem[];
-    float *xs = smem;                          // [K][ROWS]
-    float *red = smem + (size_t)K * ROWS;      // [slices][ROWS][np]
+    float *xs = smem;                             // [K][ROWS]
+    float *red = smem + (size_t)st.K * ROWS;      // [slices][ROWS][np]
     const int m0 = blockIdx.x * ROWS;
     const int rows = min(ROWS, M - m0);
-
-    for (int i = threadIdx.x; i < ROWS * K; i += blockDim.x) {
-        const int r = i / K, k = i - r * K;    // coalesced along k
-        xs[k * ROWS + r] = (r < rows) ? to_f32(x[(int64_t)(m0 + r) * K + k]) : 0.f;
+    for (int i = threadIdx.x; i < ROWS * st.K; i += blockDim.x) {
+        const int r = i / st.K, k = i - r * st.K;    // coalesced along k
+        xs[k * ROWS + r] = (r < rows) ? to_f32(x[(int64_t)(m0 + r) * st.K + k]) : 0.f;
     }
     __syncthreads();
-
-    // one layer of the chain code: the same sums in the same order as inside every fused kernel
-    ChainStep st;
-    st.w = w; st.bias = bias;
-    st.K = K; st.N = N; st.np = np; st.slices = slices; st.kchunk = kchunk; st.relu = relu;
-    st.pre = nullptr; st.act = nullptr;
-    st.transposed = 0; st.gate = nullptr;
-    chain_layer<T>(st, w, xs, nullptr, red, m0, rows, true, y);
+    chain_layer<T>(st, reinterpret_cast<const T *>(st.w), xs, nullptr, red, m0, rows, true, y);
 }
 
+// R rows x 32 columns per CTA, a warp per k slice.  Latency bound (a CTA streams kchunk weights
+// per thread from L2), so a small batch is spread over rows and columns until every SM has a
+// CTA instead of running 8 rows and all columns on each of a few.
+template <class T, int R>
+__global__ void __launch_bounds__(512)
+    dense_small_kernel(const T *__restrict__ x, T *__restrict__ y, int M, const ChainStep st) {
+    extern __shared__ __align__(16) float smem[];
+    float *xs = smem;                          // [K][R]
+    float *red = smem + (size_t)st.K * R;      // [slices][R][32]
+    const T *w = reinterpret_cast<const T *>(st.w), *bias = reinterpret_cast<const T *>(st.bias);
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+    const int m0 = blockIdx.x * R, n = blockIdx.y * 32 + lane;
+    const int k0 = slice * st.kchunk, k1 = min(st.K, k0 + st.kchunk);
+    const bool live = n < st.N;
+    // the first weights are on their way while x is staged
+    constexpr int AHEAD = 16;
+    float wv[AHEAD];
+    const T *wp = w + (int64_t)k0 * st.N + n;
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j) wv[j] = live && k0 + j < k1 ? to_f32(wp[(int64_t)j * st.N]) : 0.f;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        for (int k = threadIdx.x; k < st.K; k += blockDim.x)
+            xs[k * R + r] = m0 + r < M ? to_f32(x[(int64_t)(m0 + r) * st.K + k]) : 0.f;
+    __syncthreads();
+    float acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = 0.f;
+    for (int k = k0; k < k1; k += AHEAD) {
+        float cur[AHEAD];
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j) cur[j] = wv[j];
+        wp += (int64_t)AHEAD * st.N;
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j)
+            wv[j] = live && k + AHEAD + j < k1 ? to_f32(wp[(int64_t)j * st.N]) : 0.f;
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j) {
+            if (k + j < k1) {
+                const float *xk = xs + (k + j) * R;
+#pragma unroll
+                for (int r = 0; r < R; ++r) acc[r] = fmaf(xk[r], cur[j], acc[r]);
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) red[(slice * R + r) * 32 + lane] = acc[r];
+    __syncthreads();
+    for (int i = threadIdx.x; i < R * 32; i += blockDim.x) {
+        const int r = i / 32, c = blockIdx.y * 32 + (i & 31);
+        if (c >= st.N || m0 + r >= M) continue;
+        float s = 0.f;
+        for (int sl = 0; sl < st.slices; ++sl) s += red[sl * R * 32 + i];
+        float v = to_f32(from_f32<T>(s));
+        if (bias != nullptr) v = to_f32(from_f32<T>(__fadd_rn(v, to_f32(bias[c]))));
+        if (st.relu) v = (v >= 0.f) ? v : 0.f;
+        y[(int64_t)(m0 + r) * st.N + c] = from_f32<T>(v);
+    }
+}
+
+// Up to 512 inputs and 1.7e8 multiply-adds: beyond either the tensor-core engines are faster
+// (602 x 861 x 163 f32: 21 us here, 13 us there; 32 x 2048 x 32: 30 and 5 us).  The limit on the
+// multiply-adds keeps LeNet5's layers here up to the batch at which the one-kernel network is
+// split (5120 x 256 x 128), because the two have to give the same bits.
 bool eligible(int64_t m, int64_t k, int64_t n) {
-    return m > 0 && m <= 4096 && n > 0 && n <= 256 && k > 0 && k <= 2048;
+    return m > 0 && m <= 4096 && n > 0 && n <= 256 && k > 0 && k <= 512 && m * k * n <= 170000000;
+}
+
+bool fits_one_kernel(int64_t k, int64_t n) { return n > 0 && n <= 256 && k > 0 && k <= 2048; }
+
+template <class T, int R>
+static int launch_small(ag_device *dev, const T *x, T *y, int m, const ChainStep &st) {
+    const size_t smem = ((size_t)st.K + (size_t)st.slices * 32) * R * sizeof(float);
+    dense_small_kernel<T, R><<<dim3((unsigned)ceil_div(m, R), (unsigned)(st.np / 32)), 32 * st.slices, smem,
+                               dev->stream>>>(x, y, m, st);
+    AG_CHECK_LAUNCH();
+    return AG_OK;
 }
 
 template <class T>
 int forward(ag_device *dev, const T *x, int m, int k, const T *w, int n, const T *bias, bool relu,
             T *y) {
-    const int np = ((n + 31) / 32) * 32;
-    int slices = 1024 / np;
-    if (slices > 16) slices = 16;
-    if (slices > k / 8) slices = k / 8;
-    if (slices < 1) slices = 1;
-    const int kchunk = (k + slices - 1) / slices;
-    slices = (k + kchunk - 1) / kchunk;
-    const int threads = np * slices;
-    const size_t smem = ((size_t)k * ROWS + (size_t)slices * ROWS * np) * sizeof(float);
-    auto kernel = dense_small_kernel<T>;
-    if (smem > 48 * 1024)
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
-    kernel<<<(unsigned)ceil_div(m, ROWS), threads, smem, dev->stream>>>(x, w, bias, y, m, k, n, np,
-                                                                         slices, kchunk, relu ? 1 : 0);
-    AG_CHECK_LAUNCH();
-    return AG_OK;
+    ChainStep st = {};
+    st.w = w; st.bias = bias;
+    st.K = k; st.N = n; st.relu = relu ? 1 : 0;
+    plan_step(k, n, &st.np, &st.slices, &st.kchunk);
+    // Rows x columns against k: with many outputs the 8-row form's wider tiles win, with a long k the
+    // spread form's larger number of loads in flight (f32 100 x 256 x 128: 7.9 us on 8 rows per CTA,
+    // 4.2 us spread; 256^3 13.1 and 10.1; 384 x 145 x 135 5.9 and 6.8; bf16 256^3 13.1 and 13.9).
+    const bool narrow = narrow_step(st);
+    if (narrow || (int64_t)m * st.np > (sizeof(T) == 4 ? 256 : 128) * (int64_t)k) {
+        const int threads = narrow ? (ROWS * n * 4 < 512 ? (ROWS * n * 4 + 31) / 32 * 32 : 512) : st.np * st.slices;
+        const size_t smem = ((size_t)k * ROWS + (narrow ? 0 : (size_t)st.slices * ROWS * st.np)) * sizeof(float);
+        static bool configured_on[64] = {};
+        if (smem > 48 * 1024 && !configured_on[dev->ordinal & 63]) {
+            AG_CUDA_TRY(cudaFuncSetAttribute(dense_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             80 * 1024));
+            configured_on[dev->ordinal & 63] = true;
+        }
+        dense_rows_kernel<T><<<(unsigned)ceil_div(m, ROWS), threads, smem, dev->stream>>>(x, y, m, st);
+        AG_CHECK_LAUNCH();
+        return AG_OK;
+    }
+    // the most rows per CTA (weights read once for them) that still give every SM eight warps;
+    // shared memory stays below 48 KB with 512 inputs
+    const int64_t warps = (int64_t)(st.np / 32) * st.slices;
+    if (ceil_div(m, 4) * warps >= 8 * dev->sm_count) return launch_small<T, 4>(dev, x, y, m, st);
+    if (ceil_div(m, 2) * warps >= 8 * dev->sm_count) return launch_small<T, 2>(dev, x, y, m, st);
+    return launch_small<T, 1>(dev, x, y, m, st);
 }
 
 // ---------------------------------------------------------------- layer chain

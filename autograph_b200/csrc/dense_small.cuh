@@ -10,6 +10,8 @@ namespace dense_small {
 // True when the latency-oriented kernel should take y[m,n] = x[m,k] . w[k,n]
 // (all row-major contiguous): few rows, narrow output, moderate k.
 bool eligible(int64_t m, int64_t k, int64_t n);
+// The widest layer that the one-kernel networks (conv_chain.cu) take.
+bool fits_one_kernel(int64_t k, int64_t n);
 
 template <class T>
 int forward(ag_device *dev, const T *x, int m, int k, const T *w, int n, const T *bias, bool relu,

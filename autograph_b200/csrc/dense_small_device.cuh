@@ -163,7 +163,7 @@ __device__ __forceinline__ float load1_as(const __nv_bfloat16 *p) {
 // (p0 + p1) + (p2 + p3) by two shuffles -- no scratch, one barrier.  The order does not depend
 // on the CTA size, and every kernel that runs such a layer comes through here, so the bits are
 // the same everywhere.
-__device__ __forceinline__ bool narrow_step(const ChainStep &st) {
+__host__ __device__ __forceinline__ bool narrow_step(const ChainStep &st) {
     return !st.transposed && st.gate == nullptr && st.N <= 16 && st.K <= 1024;
 }
 
