@@ -4,7 +4,7 @@
 // convolutions with any padding / stride / dilation.
 //
 // One persistent CTA per SM walks 128 x BN output tiles (and k slices).  Warp roles:
-//   warps 0..7   producers: fetch 8 consecutive k of a row at a time with plain loads, split
+//   first warps  producers: fetch 8 consecutive k of a row at a time with plain loads, split
 //                f32 values into bf16 planes, and write the 128-byte-swizzled K-major tiles
 //                tcgen05.mma reads
 //   EPI warps    read finished accumulators from tensor memory and store through an epilogue
@@ -34,7 +34,6 @@ namespace tcx {
 
 constexpr int BM = 128;
 constexpr int BK = 64;
-constexpr int PRODUCERS = 256;
 constexpr int ROW_BYTES = BK * 2;
 
 template <class T>
@@ -78,15 +77,14 @@ __device__ __forceinline__ void fetch8(Vec8<__nv_bfloat16> &d, const __nv_bfloat
 
 // Bits whose upper halves are hi, mid and lo of an f32 value.  Rounding is half away from zero to 8
 // bits (the upper half of bits + 0x8000); both remainders are exact, of at most 16 and 8 bits.
-// A NaN must not wrap around, so an all-ones exponent becomes a NaN hi (its output is recomputed).
+// A NaN or an infinity, or a value whose hi rounds up to one, ends in a NaN: NaN - x and
+// inf - inf give the NaN 0x7fffffff, whose upper half stays a NaN in lo (only the additions of
+// 0x8000 can wrap one around).  Its outputs are NaN and are recomputed.
 __device__ __forceinline__ void split3(float v, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
-    uint32_t b = __float_as_uint(v);
-    b = (b & 0x7f800000u) == 0x7f800000u ? 0x7fc00000u : b + 0x8000u;
-    const float r = v - __uint_as_float(b & 0xffff0000u);
-    const uint32_t c = __float_as_uint(r) + 0x8000u;
-    hi = b;
-    mid = c;
-    lo = __float_as_uint(r - __uint_as_float(c & 0xffff0000u));
+    hi = __float_as_uint(v) + 0x8000u;
+    const float r = v - __uint_as_float(hi & 0xffff0000u);
+    mid = __float_as_uint(r) + 0x8000u;
+    lo = __float_as_uint(r - __uint_as_float(mid & 0xffff0000u));
 }
 
 // Upper halves of two f32 words as one packed bf16 pair.
@@ -125,38 +123,70 @@ __device__ __forceinline__ void put8(const Vec8<float> &x, uint32_t dst, uint32_
 }
 
 // ---------------------------------------------------------------- operands
-// Concept (rows = the m or n index of the product):
-//   static constexpr bool kRowFast   memory is contiguous along the rows: a producer thread keeps
-//                                    one row (begin_row once per tile) and walks its k chunks;
-//                                    otherwise it keeps one k chunk (begin_chunk once per k
-//                                    step) and walks rows
-//   void load(const State &, table, int row, int k0, int k_end, Vec8<T> &) const
-//   float at(int row, int k) const   one element (the recomputation of a non-finite output)
+// rows = the m or n index of the product.  How a producer warp walks an operand, and with it the
+// tile's layout in shared memory, follows the memory:
+enum Walk {
+    kVecK,    // rows contiguous along k and 16-byte aligned: a thread fetches 8 k with vector loads,
+              // eight threads a row; K-major tile
+    kByRow,   // contiguous along the rows: a thread keeps one row and fetches 8 k one by one, a warp
+              // 32 neighbouring rows; K-major tile
+    kByK,     // contiguous along k, no alignment: a thread keeps one k and fetches 8 rows one by one,
+              // a warp 32 neighbouring k; MN-major tile
+};
+// Concept:
+//   static constexpr Walk kWalk
 //   static constexpr int kTable      ints of shared memory prepared by init()
+//   void begin(State &, table, int i, int end)   kByRow: row i once per tile; kByK: k = i once per
+//                                    64-k step (end: rows, or the k slice's end)
+//   void load(const State &, table, int row, int k, int k_end, Vec8<T> &) const
+//                                    kVecK, kByRow: k .. k + 7 of `row`; kByK: row .. row + 7 at
+//                                    the state's k
+//   float at(int row, int k) const   one element (the recomputation of a non-finite output)
+// Rows beyond `rows` are zero or not staged at all: they only reach output rows or columns that
+// are not stored.
 
 // Strided matrix: element (row, k) at p[row * s_row + k * s_k].
-template <class T, bool ROW_FAST>
+template <class T, Walk WALK>
 struct Strided {
-    using value_type = T;
-    static constexpr bool kRowFast = ROW_FAST;
+    static constexpr Walk kWalk = WALK;
     static constexpr int kTable = 0;
     const T *p;
     int64_t s_row, s_k;
     int rows;
-    bool vec;  // s_k == 1, rows and base 16-byte aligned
-    struct State {};
+    struct State { int k, ok; };
     __device__ __forceinline__ void init(int *, int, int) const {}
-    __device__ __forceinline__ void begin_row(State &, const int *, int) const {}
-    __device__ __forceinline__ void begin_chunk(State &, const int *, int, int) const {}
-    __device__ __forceinline__ void load(const State &, const int *, int row, int k0, int k_end,
+    __device__ __forceinline__ void begin(State &s, const int *, int i, int end) const {
+        s.k = i;
+        s.ok = i < end;
+    }
+    __device__ __forceinline__ void load(const State &s, const int *, int row, int k, int k_end,
                                          Vec8<T> &d) const {
-        const T *q = p + (int64_t)row * s_row + (int64_t)k0 * s_k;
-        if (vec && row < rows && k0 + 8 <= k_end) {
-            fetch8(d, q);
+        if (WALK == kByK) {
+            const T *q = p + (int64_t)row * s_row + (int64_t)s.k * s_k;
+            if (row + 8 <= rows) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j, q += s_row) fetch(d.v[j], q, s.ok);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j, q += s_row) fetch(d.v[j], q, s.ok && row + j < rows);
+            }
             return;
         }
+        const T *q = p + (int64_t)row * s_row + (int64_t)k * s_k;
+        if (WALK == kVecK) {
+            if (k + 8 <= k_end) {
+                fetch8(d, q);
+            } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) fetch(d.v[j], q + j * s_k, row < rows && k0 + j < k_end);
+                for (int j = 0; j < 8; ++j) fetch(d.v[j], q + j, k + j < k_end);
+            }
+        } else if (k + 8 <= k_end) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j, q += s_k) fetch(d.v[j], q, true);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j, q += s_k) fetch(d.v[j], q, k + j < k_end);
+        }
     }
     __device__ __forceinline__ float at(int row, int k) const {
         return to_f32(p[(int64_t)row * s_row + (int64_t)k * s_k]);
@@ -177,7 +207,8 @@ struct ConvMap {
     int st_h, st_w, pad_h, pad_w, dil_h, dil_w;
     bool gradient;               // input-gradient form
     bool always_valid;           // no tap of any position leaves the source
-    FastDiv div_ghw, div_gw, div_ff, div_fw, div_st_h, div_st_w;
+    FastDiv div_ghw, div_gw, div_fw, div_st_h, div_st_w, div_cp;
+    int cp;                      // channels rounded up to 8
 
     __device__ __forceinline__ int tap_offset(int tap) const {
         const int fi = (int)div_fw.div((uint32_t)tap), fj = tap - fi * fw;
@@ -185,54 +216,61 @@ struct ConvMap {
             return -((int)div_st_h.div((uint32_t)(fi * dil_h)) * sw + (int)div_st_w.div((uint32_t)(fj * dil_w)));
         return fi * dil_h * sw + fj * dil_w;
     }
-    // Base address of a position and its tap mask.
-    __device__ __forceinline__ void position(int pos, int &base, uint32_t &mask) const {
-        uint32_t b, r, y, x;
-        div_ghw.divmod((uint32_t)pos, b, r);
-        div_gw.divmod(r, y, x);
-        const int image = (int)b * channels * sh * sw;
-        if (!gradient) {
-            const int y0 = (int)y * st_h - pad_h, x0 = (int)x * st_w - pad_w;
-            base = image + y0 * sw + x0;
-            if (always_valid) {
-                mask = 0xffffffffu;
-                return;
-            }
-            uint32_t cols = 0;
-            for (int fj = 0; fj < fw; ++fj)
-                if ((unsigned)(x0 + fj * dil_w) < (unsigned)sw) cols |= 1u << fj;
-            mask = 0;
-            for (int fi = 0; fi < fh; ++fi)
-                if ((unsigned)(y0 + fi * dil_h) < (unsigned)sh) mask |= cols << (fi * fw);
-        } else {
-            const int ty = (int)y + pad_h, tx = (int)x + pad_w;
-            base = image + (int)div_st_h.div((uint32_t)ty) * sw + (int)div_st_w.div((uint32_t)tx);
-            uint32_t cols = 0;
-            for (int fj = 0; fj < fw; ++fj) {
-                const int t = tx - fj * dil_w;
+    // Taps of one filter row valid at grid column x, and the rows' bits (bit fi * fw) at grid row y.
+    __device__ __forceinline__ uint32_t columns(int x) const {
+        uint32_t cols = 0;
+        for (int fj = 0; fj < fw; ++fj) {
+            if (!gradient) {
+                if ((unsigned)(x * st_w - pad_w + fj * dil_w) < (unsigned)sw) cols |= 1u << fj;
+            } else {
+                const int t = x + pad_w - fj * dil_w;
                 if (t < 0) break;
                 uint32_t q, rem;
                 div_st_w.divmod((uint32_t)t, q, rem);
                 if (rem == 0 && q < (uint32_t)sw) cols |= 1u << fj;
             }
-            mask = 0;
-            for (int fi = 0; fi < fh; ++fi) {
-                const int t = ty - fi * dil_h;
+        }
+        return cols;
+    }
+    __device__ __forceinline__ uint32_t row_bits(int y) const {
+        uint32_t bits = 0;
+        for (int fi = 0; fi < fh; ++fi) {
+            if (!gradient) {
+                if ((unsigned)(y * st_h - pad_h + fi * dil_h) < (unsigned)sh) bits |= 1u << (fi * fw);
+            } else {
+                const int t = y + pad_h - fi * dil_h;
                 if (t < 0) break;
                 uint32_t q, rem;
                 div_st_h.divmod((uint32_t)t, q, rem);
-                if (rem == 0 && q < (uint32_t)sh) mask |= cols << (fi * fw);
+                if (rem == 0 && q < (uint32_t)sh) bits |= 1u << (fi * fw);
             }
         }
+        return bits;
+    }
+    __device__ __forceinline__ int base_of(int b, int y, int x) const {
+        const int image = b * channels * sh * sw;
+        if (!gradient) return image + (y * st_h - pad_h) * sw + x * st_w - pad_w;
+        return image + (int)div_st_h.div((uint32_t)(y + pad_h)) * sw + (int)div_st_w.div((uint32_t)(x + pad_w));
+    }
+    // Base address of a position and its tap mask (columns < 2^fw, so the product has no carries).
+    __device__ __forceinline__ void position(int pos, int &base, uint32_t &mask) const {
+        uint32_t b, r, y, x;
+        div_ghw.divmod((uint32_t)pos, b, r);
+        div_gw.divmod(r, y, x);
+        base = base_of((int)b, (int)y, (int)x);
+        mask = always_valid ? 0xffffffffu : row_bits((int)y) * columns((int)x);
     }
 };
 
-// Rows are positions, k = (channel, tap): the patch matrix of the forward pass and of the input
+// The patch index runs tap-major over channels padded to a multiple of 8, so that eight neighbouring
+// indices share a tap: its check and offset are made once and the addresses step by whole planes (4
+// instructions per element, where a channel-major order takes 16).
+//
+// Rows are positions, k = (tap, channel): the patch matrix of the forward pass and of the input
 // gradient.
 template <class T>
 struct ConvRows {
-    using value_type = T;
-    static constexpr bool kRowFast = true;
+    static constexpr Walk kWalk = kByRow;
     static constexpr int kTable = 32;
     const T *src;
     ConvMap g;
@@ -244,77 +282,77 @@ struct ConvRows {
     __device__ __forceinline__ void init(int *table, int tid, int threads) const {
         for (int t = tid; t < g.ff; t += threads) table[t] = g.tap_offset(t);
     }
-    __device__ __forceinline__ void begin_row(State &s, const int *, int row) const {
+    __device__ __forceinline__ void begin(State &s, const int *, int row, int end) const {
         s.base = 0;
         s.mask = 0;
-        if (row < rows) g.position(row, s.base, s.mask);
+        if (row < end) g.position(row, s.base, s.mask);
     }
-    __device__ __forceinline__ void begin_chunk(State &, const int *, int, int) const {}
-    __device__ __forceinline__ void load(const State &s, const int *table, int, int k0, int k_end,
+    __device__ __forceinline__ void load(const State &s, const int *table, int, int k, int k_end,
                                          Vec8<T> &d) const {
-        uint32_t c, tap;
-        g.div_ff.divmod((uint32_t)k0, c, tap);
+        uint32_t tap, c;
+        g.div_cp.divmod((uint32_t)k, tap, c);
         const int plane = g.sh * g.sw;
-        int chan = s.base + (int)c * plane;
+        const bool ok = k < k_end && ((s.mask >> tap) & 1u);
+        const T *q = src + (ok ? s.base + table[tap] + (int)c * plane : 0);
+        if (c + 8 <= (uint32_t)g.channels) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            fetch(d.v[j], src + (chan + table[tap]), k0 + j < k_end && ((s.mask >> tap) & 1u));
-            if (++tap == (uint32_t)g.ff) {
-                tap = 0;
-                chan += plane;
-            }
+            for (int j = 0; j < 8; ++j, q += plane) fetch(d.v[j], q, ok);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j, q += plane) fetch(d.v[j], q, ok && (int)c + j < g.channels);
         }
     }
     __device__ __forceinline__ float at(int row, int k) const {
         int base;
         uint32_t mask, c, tap;
         g.position(row, base, mask);
-        g.div_ff.divmod((uint32_t)k, c, tap);
-        if (!((mask >> tap) & 1u)) return 0.f;
+        g.div_cp.divmod((uint32_t)k, tap, c);
+        if (!((mask >> tap) & 1u) || (int)c >= g.channels) return 0.f;
         return to_f32(src[base + (int)c * g.sh * g.sw + g.tap_offset((int)tap)]);
     }
 };
 
-// Rows are (channel, tap), k = positions: the transposed patch matrix of the weight gradient.
+// Rows are (tap, channel), k = positions: the transposed patch matrix of the weight gradient.
 template <class T>
 struct ConvCols {
-    using value_type = T;
-    static constexpr bool kRowFast = false;
+    static constexpr Walk kWalk = kByK;
     static constexpr int kTable = 32;
     const T *src;
     ConvMap g;
     int rows;
     struct State {
-        int base[8];
-        uint32_t mask[8];
+        int base;
+        uint32_t mask;
     };
     __device__ __forceinline__ void init(int *table, int tid, int threads) const {
         for (int t = tid; t < g.ff; t += threads) table[t] = g.tap_offset(t);
     }
-    __device__ __forceinline__ void begin_row(State &, const int *, int) const {}
-    __device__ __forceinline__ void begin_chunk(State &s, const int *, int k0, int k_end) const {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            s.base[j] = 0;
-            s.mask[j] = 0;
-            if (k0 + j < k_end) g.position(k0 + j, s.base[j], s.mask[j]);
-        }
+    __device__ __forceinline__ void begin(State &s, const int *, int k, int end) const {
+        s.base = 0;
+        s.mask = 0;
+        if (k < end) g.position(k, s.base, s.mask);
     }
     __device__ __forceinline__ void load(const State &s, const int *table, int row, int, int,
                                          Vec8<T> &d) const {
-        uint32_t c, tap;
-        g.div_ff.divmod((uint32_t)row, c, tap);
-        const bool ok = row < rows;
-        const T *q = src + (ok ? (int64_t)c * g.sh * g.sw + table[tap] : 0);
+        uint32_t tap, c;
+        g.div_cp.divmod((uint32_t)row, tap, c);
+        const int plane = g.sh * g.sw;
+        const bool ok = (s.mask >> tap) & 1u;
+        const T *q = src + (ok ? s.base + table[tap] + (int)c * plane : 0);
+        if (c + 8 <= (uint32_t)g.channels) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) fetch(d.v[j], q + s.base[j], ok && ((s.mask[j] >> tap) & 1u));
+            for (int j = 0; j < 8; ++j, q += plane) fetch(d.v[j], q, ok);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j, q += plane) fetch(d.v[j], q, ok && (int)c + j < g.channels);
+        }
     }
     __device__ __forceinline__ float at(int row, int k) const {
         int base;
         uint32_t mask, c, tap;
         g.position(k, base, mask);
-        g.div_ff.divmod((uint32_t)row, c, tap);
-        if (!((mask >> tap) & 1u)) return 0.f;
+        g.div_cp.divmod((uint32_t)row, tap, c);
+        if (!((mask >> tap) & 1u) || (int)c >= g.channels) return 0.f;
         return to_f32(src[base + (int)c * g.sh * g.sw + g.tap_offset((int)tap)]);
     }
 };
@@ -322,79 +360,33 @@ struct ConvCols {
 // Rows are channels of an NCHW tensor, k = (image, position).
 template <class T>
 struct ChannelRows {
-    using value_type = T;
-    static constexpr bool kRowFast = false;
+    static constexpr Walk kWalk = kByK;
     static constexpr int kTable = 0;
     const T *src;
     int rows, hw;
     FastDiv div_hw;
-    bool vec;  // hw a multiple of 8 and the base 16-byte aligned
-    struct State {
-        int base[8];
-    };
+    struct State { int base, ok; };
     __device__ __forceinline__ void init(int *, int, int) const {}
-    __device__ __forceinline__ void begin_row(State &, const int *, int) const {}
-    __device__ __forceinline__ void begin_chunk(State &s, const int *, int k0, int) const {
+    __device__ __forceinline__ void begin(State &s, const int *, int k, int end) const {
         uint32_t b, r;
-        div_hw.divmod((uint32_t)k0, b, r);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            s.base[j] = (int)b * rows * hw + (int)r;
-            if (++r == (uint32_t)hw) {
-                r = 0;
-                ++b;
-            }
-        }
+        div_hw.divmod((uint32_t)k, b, r);
+        s.base = (int)b * rows * hw + (int)r;
+        s.ok = k < end;
     }
-    __device__ __forceinline__ void load(const State &s, const int *, int row, int k0, int k_end,
-                                         Vec8<T> &d) const {
-        if (vec && row < rows && k0 + 8 <= k_end) {
-            fetch8(d, src + (s.base[0] + row * hw));
-            return;
-        }
+    __device__ __forceinline__ void load(const State &s, const int *, int row, int, int, Vec8<T> &d) const {
+        const T *q = src + (s.ok ? s.base + row * hw : 0);
+        if (row + 8 <= rows) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            fetch(d.v[j], src + (s.base[j] + row * hw), row < rows && k0 + j < k_end);
+            for (int j = 0; j < 8; ++j, q += hw) fetch(d.v[j], q, s.ok);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j, q += hw) fetch(d.v[j], q, s.ok && row + j < rows);
+        }
     }
     __device__ __forceinline__ float at(int row, int k) const {
         uint32_t b, r;
         div_hw.divmod((uint32_t)k, b, r);
         return to_f32(src[((int64_t)b * rows + row) * hw + r]);
-    }
-};
-
-// Rows are input channels, k = (output channel, tap): w[k / ff][row][k % ff].
-template <class T>
-struct WeightRows {
-    using value_type = T;
-    static constexpr bool kRowFast = false;
-    static constexpr int kTable = 0;
-    const T *w;
-    int rows, ff;
-    FastDiv div_ff;
-    struct State {};
-    __device__ __forceinline__ void init(int *, int, int) const {}
-    __device__ __forceinline__ void begin_row(State &, const int *, int) const {}
-    __device__ __forceinline__ void begin_chunk(State &, const int *, int, int) const {}
-    __device__ __forceinline__ void load(const State &, const int *, int row, int k0, int k_end,
-                                         Vec8<T> &d) const {
-        uint32_t co, tap;
-        div_ff.divmod((uint32_t)k0, co, tap);
-        int at = ((int)co * rows + row) * ff + (int)tap;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            fetch(d.v[j], w + at, row < rows && k0 + j < k_end);
-            ++at;
-            if (++tap == (uint32_t)ff) {
-                tap = 0;
-                at += (rows - 1) * ff;
-            }
-        }
-    }
-    __device__ __forceinline__ float at(int row, int k) const {
-        uint32_t co, tap;
-        div_ff.divmod((uint32_t)k, co, tap);
-        return to_f32(w[((int64_t)co * rows + row) * ff + tap]);
     }
 };
 
@@ -461,6 +453,27 @@ struct NchwOut {
     }
 };
 
+// Rows are (tap, padded channel), columns output channels: dw[col][channel][tap] = beta * dw + acc.
+template <class T>
+struct FilterOut {
+    T *dw;
+    int channels, ff;
+    FastDiv div_cp;
+    int cp;
+    float beta;
+    struct State { T *q; };
+    __device__ __forceinline__ State begin(int row) const {
+        uint32_t tap, c;
+        div_cp.divmod((uint32_t)row, tap, c);
+        return State{(int)c < channels ? dw + ((int)c * ff + (int)tap) : nullptr};
+    }
+    __device__ __forceinline__ void store(const State &s, int, int col, float acc) const {
+        if (s.q == nullptr) return;
+        T *q = s.q + (int64_t)col * channels * ff;
+        *q = from_f32<T>(beta != 0.f ? acc + beta * to_f32(*q) : acc);
+    }
+};
+
 // ------------------------------------------------------------------- kernel
 template <class T, int BN_>
 struct Cfg {
@@ -468,6 +481,9 @@ struct Cfg {
     static constexpr int BN = BN_;
     static constexpr int EPI_WARPS = BN >= 64 ? 8 : 4;
     static constexpr int COLS = BN * 4 / EPI_WARPS;              // columns per epilogue warp
+    // Sixteen producer warps hide more of the loads' latency; the 128-column epilogue
+    // leaves registers for eight.
+    static constexpr int PRODUCERS = BN == 128 ? 256 : 512;
     static constexpr int THREADS = PRODUCERS + EPI_WARPS * 32 + 32;
     static constexpr int A_PLANE = BM * ROW_BYTES, B_PLANE = BN * ROW_BYTES;
     static constexpr int STAGE = PL * (A_PLANE + B_PLANE);
@@ -484,6 +500,34 @@ struct Params {
     int tiles_m, tiles_n, splits, k_split;  // k_split: k per slice, a multiple of BK
     float *partial;                         // splits > 1: [splits][N][M] f32 sums
     int *status;
+};
+
+// Which 16-byte chunks of an R x 64 operand tile a producer thread fills.  K-major tiles hold rows of
+// 128 bytes (64 k), MN-major tiles 64-row atoms of 8 KiB with 128 bytes (64 rows) per k; both with
+// the 128-byte swizzle.
+template <Walk WALK, int R, int PRODUCERS>
+struct Slots {
+    int a, b;      // kByRow: row, chunk; kVecK: row, chunk; kByK: k, group of 8 rows
+    bool mine;
+    __device__ __forceinline__ explicit Slots(int tid) {
+        a = WALK == kByRow ? (tid & (R - 1)) : WALK == kVecK ? (tid >> 3) : (tid & 63);
+        b = WALK == kByRow ? tid / R : WALK == kVecK ? (tid & 7) : (tid >> 6);
+        mine = R * 8 >= PRODUCERS || tid < R * 8;
+    }
+    __device__ __forceinline__ int row(int i) const {
+        return WALK == kByRow ? a : WALK == kVecK ? a + i * (PRODUCERS / 8) : (b + i * (PRODUCERS / 64)) * 8;
+    }
+    __device__ __forceinline__ int k(int i) const {
+        return WALK == kByRow ? (b + i * (PRODUCERS / R)) * 8 : WALK == kVecK ? b * 8 : a;
+    }
+    __device__ __forceinline__ uint32_t offset(int i) const {
+        if (WALK == kByK) {
+            const int g = b + i * (PRODUCERS / 64);
+            return (g >> 3) * 8192 + a * 128 + (((g & 7) ^ (a & 7)) << 4);
+        }
+        const int r = row(i), ch = k(i) >> 3;
+        return r * ROW_BYTES + ((ch ^ (r & 7)) << 4);
+    }
 };
 
 // 32 lanes x 16 columns.
@@ -511,7 +555,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
     gemm_tcx_kernel(const __grid_constant__ AOp A, const __grid_constant__ BOp B,
                     const __grid_constant__ Epi E, const Params p) {
     using C = Cfg<T, BN>;
-    constexpr int PL = C::PL, STAGES = C::STAGES;
+    constexpr int PL = C::PL, STAGES = C::STAGES, PRODUCERS = C::PRODUCERS;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                 ~uintptr_t(1023));
@@ -537,6 +581,16 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    // The last tile's B rows beyond N are never staged: they start as zeros, so that the columns
+    // nobody stores do not look like sums to recompute.
+    if (PL == 3 && p.N % BN != 0) {
+        for (uint32_t i = tid; i < STAGES * PL * C::B_PLANE / 16; i += C::THREADS) {
+            const uint32_t st = i / (PL * C::B_PLANE / 16), off = i % (PL * C::B_PLANE / 16);
+            const uint32_t zero[4] = {0, 0, 0, 0};
+            st_shared_v4(tc::smem_u32(smem + st * C::STAGE + PL * C::A_PLANE) + off * 16, zero);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
     if (warp == MMA_WARP) {
         tc::tmem_alloc(tc::smem_u32(tmem_slot), C::TMEM);
         tc::tmem_relinquish();
@@ -561,32 +615,25 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
             const int tile = w % tiles, z = w / tiles;
             const int m0 = (tile % p.tiles_m) * BM, n0 = (tile / p.tiles_m) * BN;
             const int k_begin = z * p.k_split, k_end = min(p.K, k_begin + p.k_split);
-            // slot i of a thread: row-fast operands keep the row, the others the chunk
-            const int ar = AOp::kRowFast ? (tid & (BM - 1)) : (tid >> 3);
-            const int ac = AOp::kRowFast ? tid / BM : (tid & 7);
-            const int br = BOp::kRowFast ? (tid & (BN - 1)) : (tid >> 3);
-            const int bc = BOp::kRowFast ? tid / BN : (tid & 7);
+            const Slots<AOp::kWalk, BM, PRODUCERS> la(tid);
+            const Slots<BOp::kWalk, BN, PRODUCERS> lb(tid);
             typename AOp::State sa;
             typename BOp::State sb;
-            if (AOp::kRowFast) A.begin_row(sa, table_a, m0 + ar);
-            if (BOp::kRowFast) B.begin_row(sb, table_b, n0 + br);
+            if (AOp::kWalk == kByRow) A.begin(sa, table_a, m0 + la.row(0), p.M);
+            if (BOp::kWalk == kByRow) B.begin(sb, table_b, n0 + lb.row(0), p.N);
             bool ok = true;
             for (int k0 = k_begin; k0 < k_end; k0 += BK) {
                 Vec8<T> va[A_PER], vb[B_PER];
-                if (!AOp::kRowFast) A.begin_chunk(sa, table_a, k0 + ac * 8, k_end);
+                if (AOp::kWalk == kByK) A.begin(sa, table_a, k0 + la.k(0), k_end);
 #pragma unroll
-                for (int i = 0; i < A_PER; ++i) {
-                    const int row = AOp::kRowFast ? ar : ar + i * (PRODUCERS / 8);
-                    const int ch = AOp::kRowFast ? ac + i * (PRODUCERS / BM) : ac;
-                    A.load(sa, table_a, m0 + row, k0 + ch * 8, k_end, va[i]);
-                }
-                if (!BOp::kRowFast) B.begin_chunk(sb, table_b, k0 + bc * 8, k_end);
+                for (int i = 0; i < A_PER; ++i)
+                    if (m0 + la.row(i) < p.M)
+                        A.load(sa, table_a, m0 + la.row(i), k0 + la.k(i), k_end, va[i]);
+                if (BOp::kWalk == kByK) B.begin(sb, table_b, k0 + lb.k(0), k_end);
 #pragma unroll
-                for (int i = 0; i < B_PER; ++i) {
-                    const int row = BOp::kRowFast ? br : br + i * (PRODUCERS / 8);
-                    const int ch = BOp::kRowFast ? bc + i * (PRODUCERS / BN) : bc;
-                    B.load(sb, table_b, n0 + row, k0 + ch * 8, k_end, vb[i]);
-                }
+                for (int i = 0; i < B_PER; ++i)
+                    if (lb.mine && n0 + lb.row(i) < p.N)
+                        B.load(sb, table_b, n0 + lb.row(i), k0 + lb.k(i), k_end, vb[i]);
                 if (!tc::mbar_wait(tc::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag)) {
                     if (lane == 0) atomicExch(p.status, 181);
                     ok = false;
@@ -595,17 +642,11 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
                 const uint32_t a_base = tc::smem_u32(smem + stage * C::STAGE);
                 const uint32_t b_base = a_base + PL * C::A_PLANE;
 #pragma unroll
-                for (int i = 0; i < A_PER; ++i) {
-                    const int row = AOp::kRowFast ? ar : ar + i * (PRODUCERS / 8);
-                    const int ch = AOp::kRowFast ? ac + i * (PRODUCERS / BM) : ac;
-                    put8(va[i], a_base + row * ROW_BYTES + ((ch ^ (row & 7)) << 4), C::A_PLANE);
-                }
+                for (int i = 0; i < A_PER; ++i)
+                    if (m0 + la.row(i) < p.M) put8(va[i], a_base + la.offset(i), C::A_PLANE);
 #pragma unroll
-                for (int i = 0; i < B_PER; ++i) {
-                    const int row = BOp::kRowFast ? br : br + i * (PRODUCERS / 8);
-                    const int ch = BOp::kRowFast ? bc + i * (PRODUCERS / BN) : bc;
-                    put8(vb[i], b_base + row * ROW_BYTES + ((ch ^ (row & 7)) << 4), C::B_PLANE);
-                }
+                for (int i = 0; i < B_PER; ++i)
+                    if (lb.mine && n0 + lb.row(i) < p.N) put8(vb[i], b_base + lb.offset(i), C::B_PLANE);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(tc::smem_u32(&full_bar[stage]));
@@ -619,8 +660,12 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
     } else if (warp == MMA_WARP) {
         // ------------------------------------------------------------------ MMA issue
         if (lane == 0) {
-            constexpr uint32_t idesc1 = tc::make_idesc(false, false, BM, BN);
-            constexpr uint32_t idesc2 = tc::make_idesc(false, false, BM, PL == 3 ? 2 * BN : BN);
+            constexpr bool A_MN = AOp::kWalk == kByK, B_MN = BOp::kWalk == kByK;
+            constexpr uint32_t idesc1 = tc::make_idesc(A_MN, B_MN, BM, BN);
+            constexpr uint32_t idesc2 = tc::make_idesc(A_MN, B_MN, BM, PL == 3 ? 2 * BN : BN);
+            // 16 k further on, and the stride between 64-row atoms
+            constexpr uint32_t a_step = A_MN ? 2048 : 32, b_step = B_MN ? 2048 : 32;
+            constexpr uint32_t a_lbo = A_MN ? 8192 : 0, b_lbo = B_MN ? 8192 : 0;
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
@@ -643,30 +688,27 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
                     const uint32_t d = tmem + acc * C::ACC_COLS;
                     const uint32_t a_base = tc::smem_u32(smem + stage * C::STAGE);
                     const uint32_t b_base = a_base + PL * C::A_PLANE;
+                    auto da = [&](int plane, int k) {
+                        return tc::make_smem_desc(a_base + plane * C::A_PLANE + k * a_step, a_lbo, 1024);
+                    };
+                    auto db = [&](int plane, int k) {
+                        return tc::make_smem_desc(b_base + plane * C::B_PLANE + k * b_step, b_lbo, 1024);
+                    };
                     if (PL == 1) {
 #pragma unroll
                         for (int k = 0; k < BK / 16; ++k)
-                            tc::umma_bf16(d, tc::make_smem_desc(a_base + k * 32, 0, 1024),
-                                          tc::make_smem_desc(b_base + k * 32, 0, 1024), idesc1,
-                                          (k0 > k_begin || k > 0) ? 1u : 0u);
+                            tc::umma_bf16(d, da(0, k), db(0, k), idesc1, (k0 > k_begin || k > 0) ? 1u : 0u);
                     } else {
                         // corrections first: column block 0 collects hi.mid, mid.hi, lo.hi, block 1
                         // hi.lo and mid.mid; then the leading products into block 0
 #pragma unroll
                         for (int k = 0; k < BK / 16; ++k) {
-                            const uint64_t a_hi = tc::make_smem_desc(a_base + k * 32, 0, 1024);
-                            const uint64_t a_mid = tc::make_smem_desc(a_base + C::A_PLANE + k * 32, 0, 1024);
-                            const uint64_t a_lo = tc::make_smem_desc(a_base + 2 * C::A_PLANE + k * 32, 0, 1024);
-                            const uint64_t b_hi = tc::make_smem_desc(b_base + k * 32, 0, 1024);
-                            const uint64_t b_mid = tc::make_smem_desc(b_base + C::B_PLANE + k * 32, 0, 1024);
-                            tc::umma_bf16(d, a_hi, b_mid, idesc2, k > 0 ? 1u : 0u);   // b_mid, b_lo
-                            tc::umma_bf16(d, a_mid, b_hi, idesc2, 1u);                // b_hi, b_mid
-                            tc::umma_bf16(d, a_lo, b_hi, idesc1, 1u);
+                            tc::umma_bf16(d, da(0, k), db(1, k), idesc2, k > 0 ? 1u : 0u);   // b_mid, b_lo
+                            tc::umma_bf16(d, da(1, k), db(0, k), idesc2, 1u);                // b_hi, b_mid
+                            tc::umma_bf16(d, da(2, k), db(0, k), idesc1, 1u);
                         }
 #pragma unroll
-                        for (int k = 0; k < BK / 16; ++k)
-                            tc::umma_bf16(d, tc::make_smem_desc(a_base + k * 32, 0, 1024),
-                                          tc::make_smem_desc(b_base + k * 32, 0, 1024), idesc1, 1u);
+                        for (int k = 0; k < BK / 16; ++k) tc::umma_bf16(d, da(0, k), db(0, k), idesc1, 1u);
                     }
                     tc::umma_commit(tc::smem_u32(&empty_bar[stage]));
                     if (++stage == STAGES) {
@@ -843,13 +885,16 @@ int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
 }
 
 // Tile width: the narrowest that holds all columns, else 128 columns when the tiles fill the GPU.
+// MN-major B tiles are whole 64-row atoms.
 template <class T, class AOp, class BOp, class Epi>
 int gemm(ag_device *dev, int M, int N, int K, const AOp &A, const BOp &B, const Epi &E) {
     Params p = {};
     p.M = M;
     p.N = N;
     p.K = K;
-    if (N <= 32) return launch<T, 32>(dev, A, B, E, p);
+    if constexpr (BOp::kWalk != kByK) {
+        if (N <= 32) return launch<T, 32>(dev, A, B, E, p);
+    }
     const int64_t tiles = ceil_div(M, BM) * ceil_div(N, 128);
     if (N <= 64 || tiles * 2 <= dev->sm_count) return launch<T, 64>(dev, A, B, E, p);
     return launch<T, 128>(dev, A, B, E, p);

@@ -14,22 +14,26 @@ static bool rows_aligned(const T *p, int64_t s_row, int64_t s_k) {
            (reinterpret_cast<uintptr_t>(p) & 15) == 0;
 }
 
-template <class T, bool RF>
-static Strided<T, RF> strided(const T *p, int64_t s_row, int64_t s_k, int rows) {
-    return Strided<T, RF>{p, s_row, s_k, rows, rows_aligned(p, s_row, s_k)};
+template <Walk WALK, class T>
+static Strided<T, WALK> strided(const T *p, int64_t s_row, int64_t s_k, int rows) {
+    return Strided<T, WALK>{p, s_row, s_k, rows};
 }
 
+// Calls f with the operand in the walk that its memory asks for.
+template <class T, class F>
+static int with_operand(const T *p, int64_t s_row, int64_t s_k, int rows, F f) {
+    if (rows_aligned(p, s_row, s_k)) return f(strided<kVecK>(p, s_row, s_k, rows));
+    if (s_k == 1) return f(strided<kByK>(p, s_row, s_k, rows));
+    return f(strided<kByRow>(p, s_row, s_k, rows));
+}
+
+// rows of the kernel's tile: the m index of (p, q) below.
 template <class T>
 static int run(ag_device *dev, int M, int N, int K, const T *p, int64_t p_row, int64_t p_k, const T *q,
                int64_t q_row, int64_t q_k, const StridedOut<T> &E) {
-    const bool pf = p_k != 1, qf = q_k != 1;
-    if (pf && qf)
-        return gemm<T>(dev, M, N, K, strided<T, true>(p, p_row, p_k, M), strided<T, true>(q, q_row, q_k, N), E);
-    if (pf)
-        return gemm<T>(dev, M, N, K, strided<T, true>(p, p_row, p_k, M), strided<T, false>(q, q_row, q_k, N), E);
-    if (qf)
-        return gemm<T>(dev, M, N, K, strided<T, false>(p, p_row, p_k, M), strided<T, true>(q, q_row, q_k, N), E);
-    return gemm<T>(dev, M, N, K, strided<T, false>(p, p_row, p_k, M), strided<T, false>(q, q_row, q_k, N), E);
+    return with_operand(p, p_row, p_k, M, [&](const auto &A) {
+        return with_operand(q, q_row, q_k, N, [&](const auto &B) { return gemm<T>(dev, M, N, K, A, B, E); });
+    });
 }
 
 template <class T>
@@ -56,8 +60,10 @@ int dense(ag_device *dev, const T *x, int bs, int inputs, const T *w, int output
     if (packed_worth(bs, inputs, outputs))
         return packed::gemm<T>(dev, outputs, bs, inputs, w, 1, outputs, x, inputs, 1, 1.f, 0.f, y, outputs,
                                bias, relu);
-    return gemm<T>(dev, outputs, bs, inputs, strided<T, true>(w, 1, outputs, outputs),
-                   strided<T, false>(x, inputs, 1, bs), DenseOut<T>{y, outputs, bias, relu});
+    const DenseOut<T> E{y, outputs, bias, relu};
+    return with_operand(x, (int64_t)inputs, (int64_t)1, bs, [&](const auto &B) {
+        return gemm<T>(dev, outputs, bs, inputs, strided<kByRow>(w, 1, outputs, outputs), B, E);
+    });
 }
 
 }  // namespace tcx
