@@ -302,7 +302,7 @@ int ag_conv2_forward(ag_device *dev, ag_dtype dtype, const void *x, int64_t bs, 
                                               (const __nv_bfloat16 *)bias, opt, fuse_relu != 0,
                                               false, (__nv_bfloat16 *)y);
     }
-    if (tcx::conv_worth(dtype, bs * g.oh * g.ow, oc, ic * g.fh * g.fw, opt)) {
+    if (tcx::conv_worth(dtype, ic * g.fh * g.fw, oc, bs * g.oh * g.ow, opt)) {
         if (dtype == AG_F32)
             return tcx::conv_forward<float>(dev, (const float *)x, bs, ic, ih, iw, (const float *)w, oc,
                                             (const float *)bias, opt, g.oh, g.ow, fuse_relu != 0,
@@ -412,7 +412,7 @@ int ag_conv2_backward_input(ag_device *dev, ag_dtype dtype, const void *w, int64
                                                      (const __nv_bfloat16 *)dy, bs, ih, iw, opt,
                                                      (__nv_bfloat16 *)dx);
     }
-    if (tcx::conv_worth(dtype, bs * ih * iw, ic, oc * g.fh * g.fw, opt) &&
+    if (tcx::conv_input_worth(oc * g.fh * g.fw, ic, bs * ih * iw, opt) &&
         bs * oc * g.oh * g.ow < (1ll << 31)) {
         if (dtype == AG_F32)
             return tcx::conv_backward_input<float>(dev, (const float *)w, oc, ic, (const float *)dy, bs,
@@ -450,7 +450,7 @@ int ag_conv2_backward_weight(ag_device *dev, ag_dtype dtype, const void *x, int6
                                                       (const __nv_bfloat16 *)dy, oc, opt, beta,
                                                       (__nv_bfloat16 *)dw);
     }
-    if (bs > 0 && tcx::conv_worth(dtype, ic * g.fh * g.fw, oc, bs * g.oh * g.ow, opt) &&
+    if (bs > 0 && tcx::conv_weight_worth(dtype, ic * g.fh * g.fw, oc, bs * g.oh * g.ow, opt) &&
         bs * oc * g.oh * g.ow < (1ll << 31)) {
         if (dtype == AG_F32)
             return tcx::conv_backward_weight<float>(dev, (const float *)x, bs, ic, ih, iw,

@@ -32,9 +32,27 @@ bool packed_worth(int64_t m, int64_t k, int64_t n) {
     return m >= 128 && n >= 128 && k >= 64 && (double)m * (double)n * (double)k >= 2.5e8;
 }
 
-bool conv_worth(ag_dtype dtype, int64_t rows, int64_t cols, int64_t k, const ag_conv2_options *o) {
+// channels x taps and columns of the product, its depth.  Few channels are padded to eight and few
+// columns to 32: 1 -> 16 5x5 forward 42 us here and 16 us on the SIMT engine, 3 -> 16 3x3 20 and 10,
+// 3 -> 64 28 and 28, 16 -> 16 (8 x 12 x 12) 11 and 21.
+bool conv_worth(ag_dtype dtype, int64_t patch, int64_t cols, int64_t positions, const ag_conv2_options *o) {
     (void)dtype;
-    return enabled() && o->filter[0] * o->filter[1] <= 32 && rows >= 16 && cols >= 4 && k >= 16;
+    return enabled() && o->filter[0] * o->filter[1] <= 32 && patch * cols >= 1024 &&
+           positions * patch * cols >= 2000000;
+}
+
+// The input gradient, whose engine has a form for few columns (1 <- 16 5x5: 177 us on the SIMT engine).
+bool conv_input_worth(int64_t patch, int64_t cols, int64_t positions, const ag_conv2_options *o) {
+    return enabled() && o->filter[0] * o->filter[1] <= 32 && patch * cols >= 140 &&
+           positions * patch * cols >= 2000000;
+}
+
+// The weight gradient: 3 -> 16 3x3 f32 24 us here and 27, 1 -> 16 5x5 52 and 40 (bf16 38 and 60); small
+// ones (2.7e6 multiply-adds) 11 and 10.
+bool conv_weight_worth(ag_dtype dtype, int64_t patch, int64_t oc, int64_t positions, const ag_conv2_options *o) {
+    if (!enabled() || o->filter[0] * o->filter[1] > 32) return false;
+    const int64_t macs = positions * patch * oc;
+    return dtype == AG_F32 ? patch * oc >= 420 && macs >= 4000000 : patch * oc >= 128 && macs >= 2000000;
 }
 
 template int gemm_strided<float>(ag_device *, int, int, int, float, const float *, int64_t, int64_t,

@@ -25,8 +25,12 @@ template <class T>
 int dense(ag_device *dev, const T *x, int bs, int inputs, const T *w, int outputs, const T *bias,
           bool relu, T *y);
 
-// Convolutions (any padding / stride / dilation, at most 32 taps), NCHW.
-bool conv_worth(ag_dtype dtype, int64_t rows, int64_t cols, int64_t k, const ag_conv2_options *o);
+// Convolutions (any padding / stride / dilation, at most 32 taps), NCHW.  Sizes as a product: patch =
+// channels x taps (of the source that is gathered), cols, positions.
+bool conv_worth(ag_dtype dtype, int64_t patch, int64_t cols, int64_t positions, const ag_conv2_options *o);
+bool conv_input_worth(int64_t patch, int64_t cols, int64_t positions, const ag_conv2_options *o);
+bool conv_weight_worth(ag_dtype dtype, int64_t patch, int64_t oc, int64_t positions,
+                       const ag_conv2_options *o);
 template <class T>
 int conv_forward(ag_device *dev, const T *x, int64_t bs, int64_t ic, int64_t ih, int64_t iw,
                  const T *w, int64_t oc, const T *bias, const ag_conv2_options *o, int64_t oh,
