@@ -8,6 +8,10 @@ LeNet5-style model object) so that tests and benchmarks read like the
 reference's own.  PyTorch is used only to hold device memory, streams and for
 ``torch.distributed``.
 
+The per-step calls go through a small CPython extension (``csrc/python/front.c``) that
+reads the tensors and calls the library directly; the methods below are the same calls in
+Python and ctypes, which it hands anything but the plain case to.
+
 There is no CPU fallback: if the library is missing, importing this package
 fails; if there is no B200, creating a :class:`Device` fails.
 """
@@ -20,6 +24,18 @@ import numpy as np
 
 from . import _capi
 from ._capi import AgError, lib, lib_path  # noqa: F401
+
+try:
+    from . import _front
+    _DeviceBase, _ModelBase = _front.DeviceBase, _front.ModelBase
+except ImportError:   # not built yet (the build imports this package): creating a Device fails
+    _front = None
+
+    class _DeviceBase:
+        pass
+
+    class _ModelBase:
+        pass
 
 __all__ = ["AgError", "Device", "Model", "lib", "lib_path", "LENET5_SPEC", "WIDE_STACK_SPEC"]
 
@@ -50,6 +66,24 @@ def _ptr(t) -> ctypes.c_void_p:
     return ctypes.c_void_p(t.data_ptr() if t is not None else 0)
 
 
+_front_bound = False
+
+
+def _bind_front():
+    """Gives the extension the library's functions and the Python form of every method."""
+    global _front_bound
+    if _front is None:
+        raise ImportError("autograph_b200._front is missing: build it with "
+                          "`python -m autograph_b200.build`")
+    if not _front_bound:
+        handle = lib()
+        _front.bind({n: ctypes.cast(getattr(handle, n), ctypes.c_void_p).value for n in _front.FUNCTIONS},
+                    _torch(), _capi.check)
+        for name in _front.METHODS:
+            _front.set_fallback(name, getattr(_PyDevice, name, None) or getattr(_PyModel, name))
+        _front_bound = True
+
+
 def _conv_options(filter, padding=(0, 0), stride=(1, 1), dilation=(1, 1)):
     o = _capi.ConvOptions()
     o.filter[0], o.filter[1] = filter
@@ -66,7 +100,7 @@ def kernel_launch_count() -> int:
     return n.value
 
 
-class Device:
+class _PyDevice:
     """≙ ``Device::builder().index(i).build()``.  Work is submitted to a CUDA
     stream: by default a torch stream created here, which also becomes torch's
     current stream for the GPU, so that torch allocations, copies and events are
@@ -88,9 +122,12 @@ class Device:
         _capi.check(lib().ag_device_create_on_stream(index, ctypes.c_void_p(self.stream.cuda_stream),
                                                      ctypes.byref(handle)))
         self._h = handle
+        _bind_front()
+        self._bind(handle.value, self._stream_ptr, index, self.torch_device)
 
     def close(self):
         if getattr(self, "_h", None):
+            self._bind(0, 0, self.index, self.torch_device)
             lib().ag_device_destroy(self._h)
             self._h = None
 
@@ -119,6 +156,7 @@ class Device:
     def set_guards(self, on: bool):
         self._guarded = [] if on else None
         self._guard_mark = 0
+        self._set_guarded(bool(on))
 
     def _out(self, shape, dtype):
         """Output buffer of an operator (guarded and poisoned when guards are on)."""
@@ -645,6 +683,10 @@ class Device:
         return w, v
 
 
+class Device(_DeviceBase, _PyDevice):
+    __doc__ = _PyDevice.__doc__
+
+
 # Layer specs shared with the oracle's composition (kind, a, b, c, d, bias).
 LENET5_SPEC = [
     ("conv", 1, 6, (5, 5), False), ("relu",), ("pool", (2, 2)),
@@ -687,7 +729,7 @@ def _c_specs(spec):
     return arr
 
 
-class Model:
+class _PyModel:
     """≙ ``LeNet5Classifier`` of the reference's bench crate: a chain of layers with
     resident parameters, ``infer`` and ``train`` steps."""
 
@@ -709,9 +751,11 @@ class Model:
             _capi.check(lib().ag_model_parameter_len(self._h, i, ctypes.byref(ln)))
             self.parameter_lens.append(ln.value)
         self.out_features = [l for l in self.spec if l[0] == "dense"][-1][2]
+        self._bind(h.value, _dtype_code(self.dtype), device.index, self.out_features)
 
     def close(self):
         if getattr(self, "_h", None):
+            self._bind(0, 0, 0, 0)
             lib().ag_model_destroy(self._h)
             self._h = None
 
@@ -877,3 +921,7 @@ class Model:
 
     def apply_update(self, lr):
         _capi.check(lib().ag_model_apply_update(self._h, ctypes.c_float(lr)))
+
+
+class Model(_ModelBase, _PyModel):
+    __doc__ = _PyModel.__doc__

@@ -1,4 +1,5 @@
-"""Builds libautograph_b200.so (the C-ABI library) with nvcc for sm_100a.
+"""Builds libautograph_b200.so (the C-ABI library) with nvcc for sm_100a, and the CPython extension
+that calls it from the Python front end with the C compiler.
 
 Usage: ``python -m autograph_b200.build [--force] [--verbose]``.
 Objects go to ``autograph_b200/_build``; the shared library is written next to
@@ -10,6 +11,7 @@ import hashlib
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -63,6 +65,8 @@ def _compile(src: Path, digest: str, force: bool, verbose: bool) -> Path:
 
 def build(force: bool = False, verbose: bool = False) -> Path:
     BUILD.mkdir(exist_ok=True)
+    if not os.environ.get("AG_LIB_OUT"):
+        build_front(force)
     digest = _headers_digest()
     srcs = sources()
     with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as pool:
@@ -74,6 +78,24 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stderr[-4000:]}")
     return LIB
+
+
+def build_front(force: bool = False) -> Path:
+    """The native half of the Python front end (csrc/python/front.c), a CPython extension next to
+    the library."""
+    src = CSRC / "python" / "front.c"
+    out = HERE / ("_front" + sysconfig.get_config_var("EXT_SUFFIX"))
+    stamp = BUILD / "front.stamp"
+    cmd = [os.environ.get("CC", "gcc"), "-O2", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden",
+           "-I" + sysconfig.get_paths()["include"], str(src), "-o", str(out)]
+    header = HERE.parent / "include" / "autograph_b200.h"
+    key = hashlib.sha256(src.read_bytes() + header.read_bytes() + " ".join(cmd).encode()).hexdigest()
+    if force or not out.exists() or not stamp.exists() or stamp.read_text() != key:
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError(f"{cmd[0]} failed for {src.name}:\n{res.stderr[-4000:]}")
+        stamp.write_text(key)
+    return out
 
 
 if __name__ == "__main__":
