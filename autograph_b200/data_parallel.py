@@ -9,6 +9,7 @@ step; because the loss gradient is scaled by the *local* batch size
 """
 from __future__ import annotations
 
+import atexit
 import ctypes
 import os
 
@@ -37,7 +38,16 @@ def init_process_group(backend: str, timeout_s: float | None = None):
         os.environ.setdefault("MASTER_PORT", "29500")
         kw = {} if timeout_s is None else {"timeout": datetime.timedelta(seconds=timeout_s)}
         dist.init_process_group(backend=backend, **kw)
+        # A process that ends with its group alive after a failed collective may abort in the
+        # group's worker thread (seen with gloo): take it down first.
+        atexit.register(_close_process_group)
     return dist
+
+
+def _close_process_group():
+    import torch.distributed as dist
+    if dist.is_initialized() and dist.get_backend() == "gloo":
+        dist.destroy_process_group()
 
 
 def allreduce_gradients(bucket, world: int):
