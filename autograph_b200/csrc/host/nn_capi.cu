@@ -8,6 +8,7 @@
 
 #include "../comm.cuh"
 #include "../common.cuh"
+#include "../lenet_train.cuh"
 #include "nn.hpp"
 #include "conv_stages.hpp"
 
@@ -87,6 +88,8 @@ struct ag_model {
     cudaEvent_t fork_event = nullptr, join_event[2] = {nullptr, nullptr};
     int slices = 0;  // 0: chosen from the batch size
     bool whole_network = true;  // try the one-kernel form of the network at inference
+    bool fused_train = false;   // training steps take the fused LeNet5 kernels
+    ::ag::lenet_train::Net train_net;
     // Pipelined host inference (ag_model_infer_enqueue / _wait): two slots, each with a device
     // copy of its batch; the copy engine fills one slot on its own stream while the network runs
     // on the other.
@@ -201,6 +204,32 @@ void fill_uniform(ag_model *m, Tensor &dst, float a, Rng &rng) {
 
 int64_t round_up(int64_t v, int64_t to) { return (v + to - 1) / to * to; }
 
+// Whether the model is LeNet5 (autograph_backend.rs:129-146), whose training steps have kernels of
+// their own (lenet_train.cu); AG_FUSE_NET=0 keeps the layers separate, as it does at inference.
+void plan_fused_train(ag_model *m) {
+    size_t at = 0;
+    auto next = [&]() -> Layer * { return at < m->layers.size() ? m->layers[at++].get() : nullptr; };
+    auto relu = [&]() { return dynamic_cast<Relu *>(next()) != nullptr; };
+    auto stage = [&](int64_t ic, int64_t oc) {
+        auto *c = dynamic_cast<Conv2 *>(next());
+        if (!c || c->has_bias || !c->options.is_default() || c->weight.value.shape() != Shape{oc, ic, 5, 5} || !relu())
+            return false;
+        auto *p = dynamic_cast<MaxPool2 *>(next());
+        return p && p->filter[0] == 2 && p->filter[1] == 2 && p->stride[0] == 2 && p->stride[1] == 2;
+    };
+    Dense *last = nullptr;
+    auto dense = [&](int64_t k, int64_t n) {
+        last = dynamic_cast<Dense *>(next());
+        return last && !last->tied && last->weight.value.shape() == Shape{k, n};
+    };
+    if (!m->whole_network || !stage(1, 6) || !stage(6, 16) || !dynamic_cast<Flatten *>(next())) return;
+    if (!dense(256, 128) || last->has_bias || !relu() || !dense(128, 84) || last->has_bias || !relu() ||
+        !dense(84, 10) || at != m->layers.size())
+        return;
+    for (int i = 0; i < 6; ++i) m->train_net.off[i] = i < 5 || last->has_bias ? m->offsets[i] : -1;
+    m->fused_train = true;
+}
+
 void build_model(ag_model *m, const ag_layer_spec *specs, int n, uint64_t seed) {
     struct Pending {
         Parameter *p;
@@ -278,6 +307,7 @@ void build_model(ag_model *m, const ag_layer_spec *specs, int n, uint64_t seed) 
         fill_uniform(m, p->value, pending[i].a, rng);
         m->params.push_back(p);
     }
+    plan_fused_train(m);
 }
 
 // ≙ the derived Forward: input.forward(&self.f0)?...forward(&self.fN) (autograph_derive/src/lib.rs:291-340)
@@ -897,6 +927,61 @@ void apply_update(ag_model *m, float lr) {
     for (Parameter *p : m->params) p->node.reset();  // ≙ take_grad consumed the gradient
 }
 
+void ensure_loss_buffers(ag_model *m) {
+    if (m->loss_dev.defined()) return;
+    m->loss_dev = Tensor::zeros(m->pool, {1}, AG_F32);
+    void *hp = nullptr;
+    check(ag_host_alloc(sizeof(float), &hp));
+    m->loss_pinned = (float *)hp;
+}
+
+// A LeNet5 training step as two or three launches that read the images and labels where they are
+// (device memory or pinned host memory) and leave the loss in pinned host memory: with so few
+// launches a graph of them, and the copies to fixed addresses that it needs, cost more than they
+// save.  Returns false when the model, the image size or the buffers are not theirs.
+bool train_step_fused(ag_model *m, const void *x, const uint8_t *t, int64_t bs, int64_t c, int64_t h, int64_t w,
+                      float lr, float *loss_host, bool with_update, bool from_device) {
+    if (!m->fused_train || bs <= 0 || bs >= (1 << 24) || c != 1 || h != 28 || w != 28) return false;
+    Tensor xt, tt;  // device copies of pageable host buffers
+    if (!from_device) {
+        const void *xd = pinned_device_pointer(x), *td = pinned_device_pointer(t);
+        if (!xd) {
+            xt = Tensor::from_host(m->pool, {bs, c, h, w}, m->dtype, x);
+            xd = xt.data();
+        }
+        if (!td) {
+            tt = Tensor::from_host(m->pool, {bs}, AG_U8, t);
+            td = tt.data();
+        }
+        x = xd;
+        t = (const uint8_t *)td;
+    }
+    if (reinterpret_cast<uintptr_t>(x) % 16 != 0) {
+        // the kernel's loads are 16 bytes wide: a view that starts elsewhere is copied first
+        Tensor copy = Tensor::uninit(m->pool, {bs, c, h, w}, m->dtype);
+        if (cudaMemcpyAsync(copy.data(), x, copy.nbytes(), cudaMemcpyDefault,
+                            (cudaStream_t)ag_device_stream(m->dev)) != cudaSuccess)
+            throw Error(AG_ERR_CUDA, "input copy failed");
+        xt = copy;
+        x = xt.data();
+    }
+    ensure_loss_buffers(m);
+    // a gradient scale other than 1 is applied between the gradients and the update
+    const bool in_kernel = with_update && m->grad_scale == 1.f;
+    const ::ag::lenet_train::Sgd sgd = {in_kernel, m->use_momentum, lr, m->momentum};
+    check(::ag::lenet_train::step(m->dev, m->dtype, m->train_net, x, t, bs, m->values.data(), m->grads.data(),
+                                  m->velocity.data(), sgd, (float *)pinned_device_pointer(m->loss_pinned)));
+    for (Parameter *p : m->params) p->node.reset();
+    if (with_update && !in_kernel) apply_update(m, lr);
+    m->loss_in_flight = loss_host == nullptr;
+    if (loss_host) {
+        if (cudaStreamSynchronize((cudaStream_t)ag_device_stream(m->dev)) != cudaSuccess)
+            throw Error(AG_ERR_CUDA, "cudaStreamSynchronize failed");
+        *loss_host = *m->loss_pinned;
+    }
+    return true;
+}
+
 // One training step from pinned host buffers, replayed from a CUDA graph from the second
 // call with the same shape and optimizer scalars on.  Returns false when the step has to
 // run eagerly (pageable host memory, graphs disabled, capture failed).
@@ -905,6 +990,7 @@ bool train_step_graph(ag_model *m, const void *x_host, const uint8_t *t_host, in
                       bool from_device = false) {
     // x_host / t_host are device pointers when from_device is set (the data-parallel path:
     // forward and backward only, the caller all-reduces the gradient bucket and updates).
+    if (train_step_fused(m, x_host, t_host, bs, c, h, w, lr, loss_host, with_update, from_device)) return true;
     if (!m->graphs_enabled || bs <= 0) return false;
     if (!from_device && (!is_pinned_host(x_host) || !is_pinned_host(t_host))) return false;
     const cudaMemcpyKind kin = from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
@@ -953,12 +1039,7 @@ bool train_step_graph(ag_model *m, const void *x_host, const uint8_t *t_host, in
         e->x_stage = Tensor::uninit(m->pool, {bs, c, h, w}, m->dtype);
         e->t_stage = Tensor::uninit(m->pool, {bs}, AG_U8);
     }
-    if (!m->loss_dev.defined()) {
-        m->loss_dev = Tensor::zeros(m->pool, {1}, AG_F32);
-        void *hp = nullptr;
-        check(ag_host_alloc(sizeof(float), &hp));
-        m->loss_pinned = (float *)hp;
-    }
+    ensure_loss_buffers(m);
     auto cuda_ok = [](cudaError_t err, const char *what) {
         if (err != cudaSuccess)
             throw Error(AG_ERR_CUDA, std::string(what) + " failed: " + cudaGetErrorString(err));
