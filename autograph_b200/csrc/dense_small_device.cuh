@@ -397,6 +397,133 @@ __device__ __forceinline__ void chain_layer(const ChainStep &st, const T *w, con
     }
 }
 
+// Forward layers whose sizes are known at compile time, weights in shared memory, for the first R
+// of the ROWS rows: the k slices, and with them every sum, are chain_layer's.  A thread has C
+// columns x RT rows of one slice, all 512 threads at once; two sums per fma.rn.f32x2.  Run-time
+// sizes cost chain_layer more than the products do: 256 -> 128 -> 84 -> 10 on 7 rows took 4.0 + 2.7 +
+// 1.3 us there, whatever the number of rows.
+template <int K, int N>
+struct SlicePlan {   // plan_step's split
+    static constexpr int np = (N + 31) / 32 * 32;
+    static constexpr int s0 = 1024 / np > 16 ? 16 : 1024 / np, s1 = s0 > K / 8 ? K / 8 : s0, s2 = s1 < 1 ? 1 : s1;
+    static constexpr int kchunk = (K + s2 - 1) / s2, slices = (K + kchunk - 1) / kchunk;
+};
+
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void fma2(uint64_t &acc, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+template <class T, int K, int N, int R>
+__device__ __forceinline__ void sliced_layer(const ChainStep &st, const T *w, const float *xa, float *xb,
+                                             float *red) {
+    using P = SlicePlan<K, N>;
+    constexpr int RT = R < 4 ? R : 4, HALVES = R / RT, C = HALVES == 2 ? 4 : 2, COLS = N / C;
+    static_assert(N % C == 0 && COLS * HALVES * P::slices <= 512, "one item per thread");
+    const int q = threadIdx.x;
+    if (q < COLS * HALVES * P::slices) {
+        const int half = q % HALVES, n = q / HALVES % COLS * C, slice = q / (HALVES * COLS), k0 = slice * P::kchunk;
+        const T *wp = w + k0 * N + n;
+        const float *xp = xa + k0 * ROWS + RT * half;
+        // RT >= 2: pairs of rows; RT == 1: pairs of columns
+        uint64_t acc[RT > 1 ? C : 1][RT > 1 ? RT / 2 : C / 2] = {};
+#pragma unroll
+        for (int k = 0; k < P::kchunk; ++k) {
+            if (K % P::kchunk != 0 && k0 + k >= K) break;
+            float wv[C];
+            if constexpr (C == 4)
+                load4_w_as<true>(wp + k * N, wv);
+            else
+                load2_as<true>(wp + k * N, wv[0], wv[1]);
+            if constexpr (RT == 1) {
+                const float v = xp[k * ROWS];
+                fma2(acc[0][0], pack2(v, v), pack2(wv[0], wv[1]));
+            } else {
+                uint64_t v[RT / 2];
+                if constexpr (RT == 4) {
+                    const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(xp + k * ROWS);
+                    v[0] = t.x;
+                    v[1] = t.y;
+                } else {
+                    v[0] = *reinterpret_cast<const uint64_t *>(xp + k * ROWS);
+                }
+#pragma unroll
+                for (int c = 0; c < C; ++c)
+#pragma unroll
+                    for (int r = 0; r < RT / 2; ++r) fma2(acc[c][r], v[r], pack2(wv[c], wv[c]));
+            }
+        }
+        float v[RT][C];
+#pragma unroll
+        for (int i = 0; i < (RT > 1 ? C : 1); ++i)
+#pragma unroll
+            for (int j = 0; j < (RT > 1 ? RT / 2 : C / 2); ++j) {
+                float lo, hi;
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[i][j]));
+                if constexpr (RT > 1) {
+                    v[2 * j][i] = lo;
+                    v[2 * j + 1][i] = hi;
+                } else {
+                    v[0][2 * j] = lo;
+                    v[0][2 * j + 1] = hi;
+                }
+            }
+#pragma unroll
+        for (int r = 0; r < RT; ++r) {
+            float *dst = red + (slice * R + RT * half + r) * P::np + n;
+            if constexpr (C == 4)
+                *reinterpret_cast<float4 *>(dst) = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
+            else
+                *reinterpret_cast<float2 *>(dst) = make_float2(v[r][0], v[r][1]);
+        }
+    }
+    __syncthreads();
+    const T *bias = reinterpret_cast<const T *>(st.bias);
+    for (int i = threadIdx.x; i < R * P::np; i += 512) {
+        const int r = i / P::np, c = i % P::np;
+        if (c >= N) continue;
+        float part[P::slices], s = 0.f;
+#pragma unroll
+        for (int sl = 0; sl < P::slices; ++sl) part[sl] = red[(sl * R + r) * P::np + c];
+#pragma unroll
+        for (int sl = 0; sl < P::slices; ++sl) s += part[sl];
+        float v = to_f32(from_f32<T>(s));
+        if (bias != nullptr) v = to_f32(from_f32<T>(__fadd_rn(v, to_f32(bias[c]))));
+        if (st.relu) v = (v >= 0.f) ? v : 0.f;
+        xb[c * ROWS + r] = v;
+    }
+    __syncthreads();
+}
+
+// narrow_layer for a last layer of known sizes.
+template <class T, int K, int N>
+__device__ __forceinline__ void narrow_last_layer(const ChainStep &st, const T *w, const float *xa, int m0,
+                                                  int rows, T *__restrict__ y) {
+    static_assert(N <= 16 && K <= 1024 && ROWS * N * 4 <= 512, "a narrow layer, one item per thread");
+    const int q = threadIdx.x & 3, r = threadIdx.x / 4 / N, c = threadIdx.x / 4 % N;
+    if (threadIdx.x >= ((rows * N * 4 + 31) & ~31)) return;
+    const T *bias = reinterpret_cast<const T *>(st.bias);
+    const bool live = r < rows;
+    const float bv = live && bias != nullptr && q == 0 ? to_f32(bias[c]) : 0.f;
+    const float *xp = xa + q * ROWS + (live ? r : 0);
+    const T *wp = w + q * N + c;
+    float p = 0.f;
+#pragma unroll
+    for (int k = 0; k < K; k += 4)
+        if (K % 4 == 0 || k + q < K) p = fmaf(xp[k * ROWS], load1_as<true>(wp + k * N), p);
+    p += __shfl_xor_sync(0xffffffffu, p, 1);
+    p += __shfl_xor_sync(0xffffffffu, p, 2);
+    if (!live || q != 0) return;
+    float v = to_f32(from_f32<T>(p));
+    if (bias != nullptr) v = to_f32(from_f32<T>(__fadd_rn(v, bv)));
+    if (st.relu) v = (v >= 0.f) ? v : 0.f;
+    y[(int64_t)(m0 + r) * N + c] = from_f32<T>(v);
+}
+
 // Runs every layer of the chain for the ROWS rows whose first-layer input is in
 // xa as [k][ROWS] (f32).  xb is the second activation buffer, red the
 // [slices][ROWS][np] scratch.  The plan's (column, k slice) pairs are spread over

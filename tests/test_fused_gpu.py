@@ -269,3 +269,24 @@ def test_fused_errors(dev):
         dev.conv2_relu_max_pool2(x, w, pool=(3, 3))       # conv output 2x2 < window
     with pytest.raises(ag.AgError, match="a_cols != b_rows"):
         dev.dense_forward(dev.empty((2, 3), torch.float32), dev.empty((4, 5), torch.float32))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("bs", [1, 2, 149, 297, 445, 700, 1036])
+def test_lenet5_head_equals_separate_calls(dev, dtype, bs):
+    """The sizes compiled into the kernel (256 -> 128 -> 84 -> 10), at every number of images per CTA:
+    the bits of the layer-by-layer calls."""
+    rng = np.random.default_rng(bs)
+    shapes = [(6, 1, 5, 5), (16, 6, 5, 5), (256, 128), (128, 84), (84, 10), (128,), (84,), (10,)]
+    P = [dev.tensor(_prep(rng.uniform(-1, 1, s) * 0.3, dtype), dtype) for s in shapes]
+    x = dev.tensor(_prep(rng.uniform(0, 1, (bs, 1, 28, 28)), dtype), dtype)
+    stages = [(P[0], None, True, (2, 2)), (P[1], None, True, (2, 2))]
+    for biases in ([None, None, P[7]], P[5:]):
+        fused = dev.conv_dense_chain_forward(x, stages, P[2:5], biases, [True, True, False])
+        v = x
+        for wt, b, relu, pool in stages:
+            v = dev.max_pool2(dev.conv2_forward(v, wt, bias=b, relu=relu), pool)
+        v = v.reshape(bs, -1)
+        for wd, b, r in zip(P[2:5], biases, [True, True, False]):
+            v = dev.dense_forward(v, wd, bias=b, relu=r)
+        assert torch.equal(fused, v)
