@@ -16,6 +16,7 @@
 #include "conv2_direct.cuh"
 #include "conv2_direct_device.cuh"
 #include "conv_chain.cuh"
+#include "lenet_tiles.cuh"
 #include "dense_small_device.cuh"
 
 #include <cstdlib>
@@ -294,6 +295,22 @@ int forward(ag_device *dev, const T *x, const uint8_t *x8, float alpha, int64_t 
         const char *e = getenv("AG_CHAIN_GENERIC");
         return e && e[0] == '1';
     }();
+    if constexpr (sizeof(T) == 2) {
+        // Large bf16 batches of LeNet5 itself: tiles of 128 images on the tensor cores.
+        lenet::Plan lp;
+        if (!generic_only && x8 == nullptr && lenet_tiles::takes(dev, x, y, bs) &&
+            lenet::make_plan(&lp, AG_BF16, bs, ic, ih, iw, n_conv, stages, n_dense, layers) != 0 && lp.lenet5 &&
+            layers[0].relu && layers[1].relu && !layers[2].relu) {
+            lenet_tiles::Weights w;
+            w.conv1 = stages[0].w;
+            w.conv2 = stages[1].w;
+            for (int i = 0; i < 3; ++i) {
+                w.dense[i] = layers[i].w;
+                w.bias[i] = layers[i].bias;
+            }
+            return lenet_tiles::forward(dev, x, bs, w, y);
+        }
+    }
     // Large batches of a LeNet5-geometry network: the kernel stops after the flatten and the
     // dense layers run as products over the whole batch (ag_dense_forward: tensor cores for
     // bf16, the SIMT tile engine for f32).  Inside the one-kernel form every CTA streams all

@@ -1,0 +1,607 @@
+// LeNet5 inference in bf16 on the tensor cores: a CTA takes tiles of 128 images from pixels to logits.
+//
+// Every layer is a product whose 128 rows are the tile's images; what an image's row holds is a window of its
+// activations, and the weights are laid out as the banded matrix that maps a window to a block of
+// outputs:
+//   conv1: 8 columns of 6 rows (48 values) -> 4 x 2 outputs x 6 channels (N = 48), three k steps that are each
+//          8 columns of a row pair; six blocks make a pooled row;
+//   conv2: 8 columns x 6 channels of 5 rows (240 values) -> 4 outputs of one row x 8 channels (N = 32);
+//   dense: the usual matrices.
+// About half of the multiplied weights are structural zeros, which the tensor cores (4096 multiply-adds a
+// clock) do not mind: the FFMA form spends 11 us on 7 images per SM, this one about as long on 128.
+//
+// Pixels come through shared memory (the window of a k step is 32 contiguous bytes of an image's row).
+// From conv1's output on, the activations live in tensor memory only, where the accumulators' readers
+// (a thread per image) put them as the next product's A operand, packed in pairs:
+//   columns [0, 128)   accumulators: two buffers of 64 for the convolutions, one of 128 for the dense layers
+//   columns [128, 416) six rows of conv1's pooled output: 24 columns for pixels 0..7, 24 for pixels 4..11
+//   columns [416, 512) pooled rows 0..2 of conv2's output (row 3 goes where conv1's rows were)
+// Warps 0-3 load pixels, 4-11 (two sets of four, one per accumulator buffer) turn accumulators into the
+// next operand, warp 12 issues.  The issuing thread is chosen by elect.sync: behind a lane test every
+// tcgen05.mma takes 46-93 cycles to issue (measured), here about 10.
+//
+// 0 x infinity is not 0: a tile with a pixel or an activation that is not finite is marked and its
+// images are computed again by plain loops at the end.
+//
+// 65,536 images: 790 us as convolutions on the FP32 pipe and dense products over the batch.
+#include <cuda_bf16.h>
+#include <cstdlib>
+
+#include "lenet_tiles.cuh"
+#include "tc_ptx.cuh"
+
+namespace ag {
+namespace lenet_tiles {
+
+typedef __nv_bfloat16 bf16;
+
+constexpr int kImages = 128, kThreads = 13 * 32;
+constexpr int kPix = 784, kPairs = 14, kRows = 12;     // row pairs of an image, pooled rows after conv1
+constexpr int D1 = 128, D2 = 84, D3 = 10, D2P = 96, D3P = 16;
+
+// The weights as shared memory holds them: K-major rows of 64 values (128 bytes, swizzled), a block of rows
+// per 64 k.
+constexpr int B1_BYTES = 48 * 128, B2_CHUNK = 64 * 128, B2_BYTES = 4 * B2_CHUNK;
+constexpr int W1_CHUNK = D1 * 128, W1_BYTES = 4 * W1_CHUNK, W2_CHUNK = D2P * 128, W2_BYTES = 2 * W2_CHUNK;
+constexpr int W3_CHUNK = D3P * 128, W3_BYTES = 2 * W3_CHUNK;
+constexpr int B1_OFF = 0, B2_OFF = B1_OFF + B1_BYTES, W1_OFF = B2_OFF + B2_BYTES, W2_OFF = W1_OFF + W1_BYTES;
+constexpr int W3_OFF = W2_OFF + W2_BYTES, kBlob = W3_OFF + W3_BYTES;
+// Pixels: four row pairs, two to a group of three 128-byte-row blocks (pair i of a group: slots 6 i .. 6 i + 5 of
+// 32 bytes).
+constexpr int IN_OFF = kBlob, IN_BLOCK = kImages * 128, IN_GROUP = 3 * IN_BLOCK;
+constexpr int BAR_OFF = IN_OFF + 2 * IN_GROUP, kSmem = BAR_OFF + 256;
+static_assert(kSmem <= 227 * 1024 && kBlob % 1024 == 0, "shared memory");
+
+constexpr uint32_t MID = 128, FLAT = 416;              // tensor memory columns
+
+enum Bar { W_FULL = 0, IN_FULL = 3, IN_EMPTY = 7, ACC_FULL = 11, ACC_EMPTY = 13, MID_FULL = 15, D_FULL = 21, A_READY = 22,
+           kBars = 23 };
+
+struct Args {
+    const bf16 *x;
+    bf16 *y;
+    int bs;
+    const unsigned char *blob;
+    int *bad;                        // per tile: computed again by plain loops
+    Weights w;
+    int *status;
+};
+
+// ------------------------------------------------------------------------------ weights
+// A value of row n, column k of a block of `rows` rows per 64 k.
+__device__ __forceinline__ int place(int chunk_bytes, int n, int k) {
+    return (k >> 6) * chunk_bytes + n * 128 + ((((k >> 3) & 7) ^ (n & 7)) << 4) + (k & 7) * 2;
+}
+
+__global__ void __launch_bounds__(256) pack_kernel(const Weights w, unsigned char *__restrict__ blob, int *bad, int tiles) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < tiles) bad[i] = 0;
+    if (i >= kBlob / 2) return;
+    const bf16 *c1 = (const bf16 *)w.conv1, *c2 = (const bf16 *)w.conv2;
+    int at, j = i;
+    bf16 v = __float2bfloat16(0.f);
+    if (j < B1_BYTES / 2) {
+        // n = (pooled column, channel, dy, dx), k = (row pair, row, column)
+        const int n = j >> 6, k = j & 63, cell = n & 3, dy = cell >> 1, dx = cell & 1, oc = (n >> 2) % 6, px = (n >> 2) / 6;
+        const int fi = (k >> 3) - dy, fj = (k & 7) - 2 * px - dx;
+        if (k < 48 && fi >= 0 && fi < 5 && fj >= 0 && fj < 5) v = c1[(oc * 5 + fi) * 5 + fj];
+        at = B1_OFF + place(B1_BYTES, n, k);
+    } else if ((j -= B1_BYTES / 2) < B2_BYTES / 2) {
+        // n = (channel half, pooled column, channel, dx), k = (filter row, column, input channel)
+        const int n = j >> 8, k = j & 255, dx = n & 1, oc = (n >> 5) * 8 + ((n >> 1) & 7), px = (n >> 4) & 1;
+        const int fi = k / 48, r = k - fi * 48, ci = r % 6, fj = r / 6 - 2 * px - dx;
+        if (fi < 5 && fj >= 0 && fj < 5) v = c2[((oc * 6 + ci) * 5 + fi) * 5 + fj];
+        at = B2_OFF + place(B2_CHUNK, n, k);
+    } else if ((j -= B2_BYTES / 2) < W1_BYTES / 2) {
+        // k = (pooled row, column half, channel half, column, channel), as conv2's output is stored
+        const int n = j >> 8, k = j & 255, q = k >> 6, h = (k >> 5) & 1, half = (k >> 4) & 1, px = 2 * h + ((k >> 3) & 1);
+        const int oc = half * 8 + (k & 7);
+        v = ((const bf16 *)w.dense[0])[(oc * 16 + q * 4 + px) * D1 + n];
+        at = W1_OFF + place(W1_CHUNK, n, k);
+    } else if ((j -= W1_BYTES / 2) < W2_BYTES / 2) {
+        const int n = j >> 7, k = j & 127;
+        if (n < D2) v = ((const bf16 *)w.dense[1])[k * D2 + n];
+        at = W2_OFF + place(W2_CHUNK, n, k);
+    } else {
+        j -= W2_BYTES / 2;
+        const int n = j >> 7, k = j & 127;
+        if (n < D3 && k < D2) v = ((const bf16 *)w.dense[2])[k * D3 + n];
+        at = W3_OFF + place(W3_CHUNK, n, k);
+    }
+    *reinterpret_cast<bf16 *>(blob + at) = v;
+}
+
+// ----------------------------------------------------------------------------------- PTX
+__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "}\n" ::"r"(d),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void ld16(uint32_t t, uint32_t *r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(t)
+                 : "memory");
+}
+__device__ __forceinline__ void st2(uint32_t t, const uint32_t *r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(t), "r"(r[0]), "r"(r[1]) : "memory");
+}
+__device__ __forceinline__ void st8(uint32_t t, const uint32_t *r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(t), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// Relu and maximum of a pool window, before the rounding that the layer stores with: rounding keeps
+// order, so the result is the same.
+__device__ __forceinline__ float pool4(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    return fmaxf(fmaxf(fmaxf(__uint_as_float(a), __uint_as_float(b)), fmaxf(__uint_as_float(c), __uint_as_float(d))), 0.f);
+}
+__device__ __forceinline__ uint32_t pack(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+__device__ __forceinline__ bool not_finite(uint32_t w) {
+    return (w & 0x7f80u) == 0x7f80u || (w & 0x7f800000u) == 0x7f800000u;
+}
+
+// ------------------------------------------------------------------- images by plain loops
+__device__ float relu_pool(const float *v) {
+    float m = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float r = __bfloat162float(__float2bfloat16(v[i]));
+        if (r > m) m = r;
+    }
+    return m;
+}
+__device__ __noinline__ void plain_image(const Args &a, int b, float *s) {
+    float *x = s, *p1 = x + kPix, *f = p1 + 864, *h1 = f + 256, *h2 = h1 + D1;
+    const int tid = threadIdx.x;
+    const bf16 *c1 = (const bf16 *)a.w.conv1, *c2 = (const bf16 *)a.w.conv2;
+    __syncthreads();
+    for (int i = tid; i < kPix; i += kThreads) x[i] = __bfloat162float(a.x[(int64_t)b * kPix + i]);
+    __syncthreads();
+    for (int i = tid; i < 864; i += kThreads) {
+        const int c = i / 144, r = i % 144, y = r / 12 * 2, xx = r % 12 * 2;
+        float v[4];
+        for (int cell = 0; cell < 4; ++cell) {
+            float sum = 0.f;
+            for (int t = 0; t < 25; ++t)
+                sum = fmaf(x[(y + cell / 2 + t / 5) * 28 + xx + cell % 2 + t % 5], __bfloat162float(c1[c * 25 + t]), sum);
+            v[cell] = sum;
+        }
+        p1[i] = relu_pool(v);
+    }
+    __syncthreads();
+    for (int i = tid; i < 256; i += kThreads) {
+        const int c = i / 16, y = i % 16 / 4 * 2, xx = i % 4 * 2;
+        float v[4];
+        for (int cell = 0; cell < 4; ++cell) {
+            float sum = 0.f;
+            for (int t = 0; t < 150; ++t)
+                sum = fmaf(p1[t / 25 * 144 + (y + cell / 2 + t % 25 / 5) * 12 + xx + cell % 2 + t % 5],
+                           __bfloat162float(c2[c * 150 + t]), sum);
+            v[cell] = sum;
+        }
+        f[i] = relu_pool(v);
+    }
+    const float *in = f;
+    for (int l = 0; l < 3; ++l) {
+        __syncthreads();
+        const int K = l == 0 ? 256 : l == 1 ? D1 : D2, N = l == 0 ? D1 : l == 1 ? D2 : D3;
+        const bf16 *w = (const bf16 *)a.w.dense[l], *bias = (const bf16 *)a.w.bias[l];
+        for (int n = tid; n < N; n += kThreads) {
+            float sum = 0.f;
+            for (int k = 0; k < K; ++k) sum = fmaf(in[k], __bfloat162float(w[k * N + n]), sum);
+            float v = __bfloat162float(__float2bfloat16(sum));
+            if (bias) v = __bfloat162float(__float2bfloat16(v + __bfloat162float(bias[n])));
+            if (l == 2)
+                a.y[(int64_t)b * D3 + n] = __float2bfloat16(v);
+            else
+                (l == 0 ? h1 : h2)[n] = v >= 0.f ? v : 0.f;
+        }
+        in = l == 0 ? h1 : h2;
+    }
+}
+
+// --------------------------------------------------------------------------------- kernel
+__global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant__ Args a) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    const uint32_t base = tc::smem_u32(smem);
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    int *abort_flag = reinterpret_cast<int *>(smem + BAR_OFF + kBars * 8), *tmem_at = abort_flag + 1;
+    const auto bar = [&](int i) { return base + BAR_OFF + 8 * (uint32_t)i; };
+    const int tiles = (a.bs + kImages - 1) / kImages;
+
+    if (threadIdx.x == 0) {
+        *abort_flag = (base & 1023u) != 0;   // the swizzled layouts start on 1024-byte boundaries
+        for (int i = 0; i < kBars; ++i) {
+            const bool warps4 = (i >= IN_FULL && i < IN_EMPTY) || (i >= ACC_EMPTY && i < MID_FULL);
+            const bool warps8 = (i >= MID_FULL && i < D_FULL) || i == A_READY;
+            tc::mbar_init(bar(i), warps4 ? 4 : warps8 ? 8 : 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 12) {
+        tc::tmem_alloc(tc::smem_u32(tmem_at), 512);
+        tc::tmem_relinquish();
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = *reinterpret_cast<volatile int *>(tmem_at);
+    const bool start = *reinterpret_cast<volatile int *>(abort_flag) == 0;
+    if (!start && threadIdx.x == 0) atomicCAS(a.status, 0, 175);
+    // Waits of warp-wide code: the lanes agree on the outcome, since it decides what the warp runs next.
+    const auto wait = [&](int i, uint32_t parity) {
+        return __all_sync(0xffffffffu, tc::mbar_wait(bar(i), parity, abort_flag)) != 0;
+    };
+    const auto arrive = [&](int i) {
+        if (lane == 0) tc::mbar_arrive(bar(i));
+    };
+
+    bool ok = start;
+    if (warp < 4) {
+        // ------------------------------------------------------------------------- pixels
+        const int img = threadIdx.x;
+        uint4 v[7];
+        const auto load = [&](int tile, int pair) {
+            const int b = tile * kImages + img;
+#pragma unroll
+            for (int i = 0; i < 7; ++i)
+                v[i] = b < a.bs ? __ldg(reinterpret_cast<const uint4 *>(a.x + (int64_t)b * kPix + pair * 56) + i)
+                                : make_uint4(0, 0, 0, 0);
+        };
+        if (ok) load(blockIdx.x, 0);
+        uint32_t g = 0;
+        for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
+            bool bad = false;
+            for (int pair = 0; pair < kPairs; ++pair, ++g) {
+                const uint32_t slot = g & 3;
+                if (!(ok = wait(IN_EMPTY + slot, ((g >> 2) & 1) ^ 1))) break;
+                uint32_t w[28];
+#pragma unroll
+                for (int i = 0; i < 7; ++i) {
+                    w[4 * i] = v[i].x; w[4 * i + 1] = v[i].y; w[4 * i + 2] = v[i].z; w[4 * i + 3] = v[i].w;
+                }
+                const bool more = pair + 1 < kPairs;
+                if (more || tile + (int)gridDim.x < tiles) load(more ? tile : tile + gridDim.x, more ? pair + 1 : 0);
+                const uint32_t row = IN_OFF + (slot >> 1) * IN_GROUP + img * 128;
+#pragma unroll
+                for (int b = 0; b < 6; ++b) {
+                    const uint32_t s = (slot & 1) * 6 + b, block = s >> 2, piece = (s & 3) * 2;
+#pragma unroll
+                    for (int r = 0; r < 2; ++r)
+                        *reinterpret_cast<uint4 *>(smem + row + block * IN_BLOCK + (((piece + r) ^ (img & 7)) << 4)) =
+                            make_uint4(w[14 * r + 2 * b], w[14 * r + 2 * b + 1], w[14 * r + 2 * b + 2], w[14 * r + 2 * b + 3]);
+                }
+#pragma unroll
+                for (int i = 0; i < 28; ++i) bad |= not_finite(w[i]);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                arrive(IN_FULL + slot);
+            }
+            if (bad) a.bad[tile] = 1;
+        }
+    } else if (warp < 12) {
+        // ---------------------------------------------------------- accumulators -> operands
+        const int set = (warp - 4) >> 2;
+        const uint32_t t = tmem + ((uint32_t)(warp & 3) << 21);   // lanes 32 * (warp % 4) ..
+        const uint32_t acc = t + 64 * set;
+        uint32_t jobs = 0, dense = 0;
+        for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
+            uint32_t held[8], top = 0;
+            for (int p = 0; ok && p < kRows; ++p) {
+                const uint32_t mid = t + MID + 48 * (p % 6);
+#pragma unroll 1
+                for (int b = set; b < 6; b += 2, ++jobs) {
+                    if (!(ok = wait(ACC_FULL + set, jobs & 1))) break;
+                    tc::tc_fence_after();
+                    uint32_t r[48], o[6];
+                    ld16(acc, r);
+                    ld16(acc + 16, r + 16);
+                    ld16(acc + 32, r + 32);
+                    tc::tmem_ld_wait();
+                    tc::tc_fence_before();
+                    __syncwarp();
+                    arrive(ACC_EMPTY + set);
+#pragma unroll
+                    for (int i = 0; i < 6; ++i) {
+                        o[i] = pack(pool4(r[8 * i], r[8 * i + 1], r[8 * i + 2], r[8 * i + 3]),
+                                    pool4(r[8 * i + 4], r[8 * i + 5], r[8 * i + 6], r[8 * i + 7]));
+                        top = max(top, max(o[i] & 0x7fff0000u, o[i] << 16));
+                    }
+#pragma unroll
+                    for (int i = 0; i < 6; i += 2) {
+                        if (b < 4) st2(mid + 6 * b + i, o + i);
+                        if (b >= 2) st2(mid + 24 + 6 * (b - 2) + i, o + i);
+                    }
+                }
+                if (!ok) break;
+                st_wait();
+                tc::tc_fence_before();
+                __syncwarp();
+                arrive(MID_FULL + p % 6);
+                if (p < 5 || (p & 1) == 0) continue;
+                // conv2's pooled row q: channel half `set` of both column halves
+                const int q = (p - 5) >> 1;
+#pragma unroll 1
+                for (int h = 0; h < 2; ++h, ++jobs) {
+                    if (!(ok = wait(ACC_FULL + set, jobs & 1))) break;
+                    tc::tc_fence_after();
+                    uint32_t r[64], o[8];
+#pragma unroll
+                    for (int i = 0; i < 64; i += 16) ld16(acc + i, r + i);
+                    tc::tmem_ld_wait();
+                    tc::tc_fence_before();
+                    __syncwarp();
+                    arrive(ACC_EMPTY + set);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        o[i] = pack(pool4(r[4 * i], r[4 * i + 1], r[32 + 4 * i], r[32 + 4 * i + 1]),
+                                    pool4(r[4 * i + 2], r[4 * i + 3], r[32 + 4 * i + 2], r[32 + 4 * i + 3]));
+                    if (q < 3) {
+                        st8(t + FLAT + 32 * q + 16 * h + 8 * set, o);
+                    } else if (h == 0) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) held[i] = o[i];
+                    } else {
+                        // conv1's rows are free where conv2 read pixels 0..7: its left half is complete
+                        st8(t + MID + 8 * set, held);
+                        st8(t + MID + 48 + 8 * set, o);
+                    }
+                }
+            }
+            if (!ok) break;
+            if (top >= 0x7f800000u) a.bad[tile] = 1;
+            st_wait();
+            tc::tc_fence_before();
+            __syncwarp();
+            arrive(A_READY);
+            // ---- dense layers: half of the columns each
+            const int b = tile * kImages + (warp & 3) * 32 + lane;
+            const auto dense_value = [&](uint32_t r, const bf16 *bias, int n, int N) {
+                float v = __bfloat162float(__float2bfloat16(__uint_as_float(r)));
+                if (bias != nullptr && n < N) v = __bfloat162float(__float2bfloat16(v + __bfloat162float(bias[n])));
+                return v;
+            };
+            if (!(ok = wait(D_FULL, dense++ & 1))) break;
+            tc::tc_fence_after();
+            {
+                const bf16 *bias = (const bf16 *)a.w.bias[0];
+                uint32_t r[64], o[32];
+#pragma unroll
+                for (int i = 0; i < 64; i += 16) ld16(acc + i, r + i);
+                tc::tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                    o[i] = pack(fmaxf(dense_value(r[2 * i], bias, 64 * set + 2 * i, D1), 0.f),
+                                fmaxf(dense_value(r[2 * i + 1], bias, 64 * set + 2 * i + 1, D1), 0.f));
+#pragma unroll
+                for (int i = 0; i < 32; i += 8) st8(t + FLAT + 32 * set + i, o + i);
+            }
+            st_wait();
+            tc::tc_fence_before();
+            __syncwarp();
+            arrive(A_READY);
+            if (!(ok = wait(D_FULL, dense++ & 1))) break;
+            tc::tc_fence_after();
+            {
+                const bf16 *bias = (const bf16 *)a.w.bias[1];
+                uint32_t r[48], o[24];
+#pragma unroll
+                for (int i = 0; i < 48; i += 16) ld16(t + 48 * set + i, r + i);
+                tc::tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 24; ++i)
+                    o[i] = pack(fmaxf(dense_value(r[2 * i], bias, 48 * set + 2 * i, D2), 0.f),
+                                fmaxf(dense_value(r[2 * i + 1], bias, 48 * set + 2 * i + 1, D2), 0.f));
+#pragma unroll
+                for (int i = 0; i < 24; i += 8) st8(t + MID + 24 * set + i, o + i);
+            }
+            st_wait();
+            tc::tc_fence_before();
+            __syncwarp();
+            arrive(A_READY);
+            if (!(ok = wait(D_FULL, dense++ & 1))) break;
+            tc::tc_fence_after();
+            if (set == 0) {
+                const bf16 *bias = (const bf16 *)a.w.bias[2];
+                uint32_t r[16];
+                ld16(t, r);
+                tc::tmem_ld_wait();
+                if (b < a.bs) {
+                    uint32_t *y = reinterpret_cast<uint32_t *>(a.y + (int64_t)b * D3);
+#pragma unroll
+                    for (int i = 0; i < 5; ++i)
+                        y[i] = pack(dense_value(r[2 * i], bias, 2 * i, D3), dense_value(r[2 * i + 1], bias, 2 * i + 1, D3));
+                }
+            }
+            tc::tc_fence_before();
+            __syncwarp();
+            arrive(A_READY);
+        }
+    } else {
+        // ---------------------------------------------------------------------- tensor cores
+        const bool leader = tc::elect_one();
+        if (ok && leader) {
+            const int off[3] = {B1_OFF, B2_OFF, W1_OFF}, bytes[3] = {B1_BYTES, B2_BYTES, kBlob - W1_OFF};
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                tc::mbar_arrive_expect_tx(bar(W_FULL + i), (uint32_t)bytes[i]);
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                             ::"r"(base + off[i]), "l"(a.blob + off[i]), "r"((uint32_t)bytes[i]), "r"(bar(W_FULL + i))
+                             : "memory");
+            }
+        }
+        __syncwarp();
+        const auto commit = [&](int i) {
+            if (tc::elect_one()) tc::umma_commit(bar(i));
+            __syncwarp();
+        };
+        const auto desc = [&](uint32_t at) { return tc::make_smem_desc(base + at, 0, 1024); };
+        constexpr uint32_t id48 = tc::make_idesc(false, false, 128, 48), id32 = tc::make_idesc(false, false, 128, 32);
+        constexpr uint32_t id128 = tc::make_idesc(false, false, 128, D1), id96 = tc::make_idesc(false, false, 128, D2P);
+        constexpr uint32_t id16 = tc::make_idesc(false, false, 128, D3P);
+        uint32_t g = 0, jobs[2] = {0, 0}, mids = 0, ready = 0;
+        bool first = true;
+        for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
+            if (first) ok = wait(W_FULL, 0);
+            for (int p = 0; ok && p < kRows; ++p) {
+                // row p reads row pairs p, p + 1, p + 2
+                for (int i = p == 0 ? 0 : 2; ok && i < 3; ++i) ok = wait(IN_FULL + ((g + p + i) & 3), ((g + p + i) >> 2) & 1);
+                if (!ok) break;
+                tc::tc_fence_after();
+#pragma unroll
+                for (int b = 0; b < 6; ++b) {
+                    if (!(ok = wait(ACC_EMPTY + (b & 1), (jobs[b & 1]++ & 1) ^ 1))) break;
+                    tc::tc_fence_after();
+                    if (tc::elect_one()) {
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) {
+                            const uint32_t slot = (g + p + i) & 3, s = (slot & 1) * 6 + b;
+                            tc::umma_bf16(tmem + 64 * (b & 1),
+                                          desc(IN_OFF + (slot >> 1) * IN_GROUP + (s >> 2) * IN_BLOCK + (s & 3) * 32),
+                                          desc(B1_OFF + 32 * i), id48, i > 0);
+                        }
+                        tc::umma_commit(bar(ACC_FULL + (b & 1)));
+                    }
+                    __syncwarp();
+                }
+                if (!ok) break;
+                commit(IN_EMPTY + ((g + p) & 3));
+                if (p == kRows - 1) {
+                    commit(IN_EMPTY + ((g + p + 1) & 3));
+                    commit(IN_EMPTY + ((g + p + 2) & 3));
+                }
+                if (p < 5 || (p & 1) == 0) continue;
+                if (first && p == 5 && !(ok = wait(W_FULL + 1, 0))) break;
+                const int q = (p - 5) >> 1;
+                // each of the six row slots is filled twice per tile
+                for (int row = q == 0 ? 0 : p - 1; ok && row <= p; ++row) ok = wait(MID_FULL + row % 6, (mids + row / 6) & 1);
+                if (!ok) break;
+                tc::tc_fence_after();
+#pragma unroll 1
+                for (int job = 0; job < 4; ++job) {
+                    const int h = job >> 1, half = job & 1;
+                    if (!(ok = wait(ACC_EMPTY + half, (jobs[half]++ & 1) ^ 1))) break;
+                    tc::tc_fence_after();
+                    if (tc::elect_one()) {
+#pragma unroll 1
+                        for (int dy = 0; dy < 2; ++dy) {
+                            int slot = (2 * q + dy) % 6;
+#pragma unroll
+                            for (int fi = 0; fi < 5; ++fi) {
+#pragma unroll
+                                for (int i = 0; i < 3; ++i) {
+                                    const int s = 3 * fi + i;
+                                    umma_ts(tmem + 64 * half + 32 * dy, tmem + MID + 48 * slot + 24 * h + 8 * i,
+                                            desc(B2_OFF + (s >> 2) * B2_CHUNK + half * 4096 + (s & 3) * 32), id32, s > 0);
+                                }
+                                slot = slot == 5 ? 0 : slot + 1;
+                            }
+                        }
+                        tc::umma_commit(bar(ACC_FULL + half));
+                    }
+                    __syncwarp();
+                }
+            }
+            if (!ok) break;
+            g += kPairs;
+            mids += 2;
+            if (first && !(ok = wait(W_FULL + 2, 0))) break;
+            first = false;
+            // the accumulators are free when the flattened rows are complete
+            if (!(ok = wait(A_READY, ready++ & 1))) break;
+            tc::tc_fence_after();
+            if (tc::elect_one()) {
+#pragma unroll
+                for (int s = 0; s < 16; ++s) {
+                    const uint32_t at = s < 12 ? FLAT + 8 * s : MID + 48 * ((s - 12) >> 1) + 8 * (s & 1);
+                    umma_ts(tmem, tmem + at, desc(W1_OFF + (s >> 2) * W1_CHUNK + (s & 3) * 32), id128, s > 0);
+                }
+                tc::umma_commit(bar(D_FULL));
+            }
+            __syncwarp();
+            if (!(ok = wait(A_READY, ready++ & 1))) break;
+            tc::tc_fence_after();
+            if (tc::elect_one()) {
+#pragma unroll
+                for (int s = 0; s < 8; ++s)
+                    umma_ts(tmem, tmem + FLAT + 8 * s, desc(W2_OFF + (s >> 2) * W2_CHUNK + (s & 3) * 32), id96, s > 0);
+                tc::umma_commit(bar(D_FULL));
+            }
+            __syncwarp();
+            if (!(ok = wait(A_READY, ready++ & 1))) break;
+            tc::tc_fence_after();
+            if (tc::elect_one()) {
+#pragma unroll
+                for (int s = 0; s < 6; ++s)
+                    umma_ts(tmem, tmem + MID + 8 * s, desc(W3_OFF + (s >> 2) * W3_CHUNK + (s & 3) * 32), id16, s > 0);
+                tc::umma_commit(bar(D_FULL));
+            }
+            __syncwarp();
+            ok = wait(A_READY, ready++ & 1);
+            tc::tc_fence_after();
+        }
+        if (start && !ok) {   // a bounded wait for the weight copies in flight
+            int none = 0;
+            for (int i = 0; i < 3; ++i) tc::mbar_wait_for(bar(W_FULL + i), 0, &none, 100000000ull);
+        }
+    }
+    if (!ok && start && lane == 0) atomicCAS(a.status, 0, 176);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    if (warp == 12) tc::tmem_dealloc(tmem, 512);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        if (*reinterpret_cast<volatile int *>(a.bad + tile) == 0) continue;
+        for (int b = tile * kImages; b < min(a.bs, (tile + 1) * kImages); ++b)
+            plain_image(a, b, reinterpret_cast<float *>(smem));
+    }
+}
+
+// ----------------------------------------------------------------------------------- host
+bool takes(const ag_device *dev, const void *x, const void *y, int64_t bs) {
+    // From about half a tile per SM on.  Below, the FFMA kernel gives the bits of the layers run one by
+    // one, which callers compare; a single wave of tiles takes as long as 1000 images there.
+    if (bs < (int64_t)kImages / 2 * dev->sm_count || bs >= (1 << 30)) return false;
+    const char *e = getenv("AG_LENET_TILES");   // 0: off, for comparisons
+    return !(e && e[0] == '0') && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(y) & 3) == 0;
+}
+
+int forward(ag_device *dev, const void *x, int64_t bs, const Weights &w, void *y) {
+    const int tiles = (int)ceil_div(bs, (int64_t)kImages);
+    void *ws = nullptr;
+    AG_TRY(workspace(dev, kBlob + (size_t)tiles * sizeof(int), &ws));
+    Args a;
+    a.x = (const bf16 *)x;
+    a.y = (bf16 *)y;
+    a.bs = (int)bs;
+    a.blob = (const unsigned char *)ws;
+    a.bad = (int *)((char *)ws + kBlob);
+    a.w = w;
+    a.status = dev->status_dev;
+    const int threads = tiles > kBlob / 2 ? tiles : kBlob / 2;
+    pack_kernel<<<(unsigned)ceil_div(threads, 256), 256, 0, dev->stream>>>(w, (unsigned char *)ws, a.bad, tiles);
+    AG_CHECK_LAUNCH();
+    static bool configured[64] = {};
+    if (dev->ordinal >= 64 || !configured[dev->ordinal]) {
+        AG_CUDA_TRY(cudaFuncSetAttribute(tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        if (dev->ordinal < 64) configured[dev->ordinal] = true;
+    }
+    tile_kernel<<<(unsigned)(tiles < dev->sm_count ? tiles : dev->sm_count), kThreads, kSmem, dev->stream>>>(a);
+    AG_CHECK_LAUNCH();
+    return AG_OK;
+}
+
+}  // namespace lenet_tiles
+}  // namespace ag

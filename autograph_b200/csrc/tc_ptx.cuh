@@ -108,6 +108,21 @@ __device__ __forceinline__ void tc_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
+// One thread of a converged warp.  tcgen05.mma issues in about 10 cycles from a branch on this and in 46 to
+// 93 from a branch on the lane number, where the operands' uniform registers are filled per instruction
+// (both measured); it matters wherever N is below 192.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n"
+        ".reg .pred q;\n"
+        "elect.sync _|q, 0xffffffff;\n"
+        "selp.b32 %0, 1, 0, q;\n"
+        "}\n"
+        : "=r"(p));
+    return p != 0;
+}
+
 // D[tmem] (+)= A[smem] . B[smem]; one thread issues for the whole CTA.
 __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                           uint32_t idesc, uint32_t accumulate) {
