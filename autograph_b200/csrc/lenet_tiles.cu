@@ -13,12 +13,15 @@
 // Pixels come through shared memory (the window of a k step is 32 contiguous bytes of an image's row).
 // From conv1's output on, the activations live in tensor memory only, where the accumulators' readers
 // (a thread per image) put them as the next product's A operand, packed in pairs:
-//   columns [0, 128)   accumulators: two buffers of 64 for the convolutions, one of 128 for the dense layers
-//   columns [128, 416) six rows of conv1's pooled output: 24 columns for pixels 0..7, 24 for pixels 4..11
-//   columns [416, 512) pooled rows 0..2 of conv2's output (row 3 goes where conv1's rows were)
-// Warps 0-3 load pixels, 4-11 (two sets of four, one per accumulator buffer) turn accumulators into the
-// next operand, warp 12 issues.  The issuing thread is chosen by elect.sync: behind a lane test every
-// tcgen05.mma takes 46-93 cycles to issue (measured), here about 10.
+//   columns [0, 192)   accumulators: for each of the two sets of readers two buffers of 48 (conv1) or one of 64
+//                      (conv2); 128 for the dense layers
+//   columns [192, 480) six rows of conv1's pooled output: 24 columns for pixels 0..7, 24 for pixels 4..11
+//   columns [480, 512) pooled row 0 of conv2's output; rows 1 to 3 wait in registers until conv2 has read
+//                      the last of conv1's rows, and take their place
+// Warps 0-3 load pixels (two row pairs ahead), 4-11 (two sets of four) turn accumulators into the next
+// operand, warp 12 issues.  The issuing thread is chosen by elect.sync and what varies between its operands
+// is made warp-uniform first: behind a lane test, or with operands from ordinary registers, a
+// tcgen05.mma takes 46-93 cycles to issue (measured), here about 10; the products themselves take 16 to 64.
 //
 // 0 x infinity is not 0: a tile with a pixel or an activation that is not finite is marked and its
 // images are computed again by plain loops at the end.
@@ -26,6 +29,7 @@
 // 65,536 images: 790 us as convolutions on the FP32 pipe and dense products over the batch.
 #include <cuda_bf16.h>
 #include <cstdlib>
+#include <type_traits>
 
 #include "lenet_tiles.cuh"
 #include "tc_ptx.cuh"
@@ -46,16 +50,21 @@ constexpr int W1_CHUNK = D1 * 128, W1_BYTES = 4 * W1_CHUNK, W2_CHUNK = D2P * 128
 constexpr int W3_CHUNK = D3P * 128, W3_BYTES = 2 * W3_CHUNK;
 constexpr int B1_OFF = 0, B2_OFF = B1_OFF + B1_BYTES, W1_OFF = B2_OFF + B2_BYTES, W2_OFF = W1_OFF + W1_BYTES;
 constexpr int W3_OFF = W2_OFF + W2_BYTES, kBlob = W3_OFF + W3_BYTES;
-// Pixels: four row pairs, two to a group of three 128-byte-row blocks (pair i of a group: slots 6 i .. 6 i + 5 of
-// 32 bytes).
+// Pixels: four row pairs, two to a group of three blocks of 128-byte rows.  Windows 0..3 of pair i of a group are
+// the four 32-byte pieces of block i, windows 4 and 5 half i of block 2.
 constexpr int IN_OFF = kBlob, IN_BLOCK = kImages * 128, IN_GROUP = 3 * IN_BLOCK;
 constexpr int BAR_OFF = IN_OFF + 2 * IN_GROUP, kSmem = BAR_OFF + 256;
 static_assert(kSmem <= 227 * 1024 && kBlob % 1024 == 0, "shared memory");
 
-constexpr uint32_t MID = 128, FLAT = 416;              // tensor memory columns
+constexpr uint32_t MID = 192, FLAT = 480;              // tensor memory columns
 
-enum Bar { W_FULL = 0, IN_FULL = 3, IN_EMPTY = 7, ACC_FULL = 11, ACC_EMPTY = 13, MID_FULL = 15, D_FULL = 21, A_READY = 22,
-           kBars = 23 };
+// Where the k step i of the dense layers that follows pooled row 0 lies: three to a slot of conv1's rows.
+__host__ __device__ constexpr uint32_t late_columns(int i) { return MID + 48 * (i / 3) + 8 * (i % 3); }
+// The first hidden layer (64 columns): slots 4 and 5, which hold none of those; the second (48): slot 0.
+constexpr uint32_t HIDDEN = MID + 48 * 4;
+
+enum Bar { W_FULL = 0, IN_FULL = 3, IN_EMPTY = 7, ACC_FULL = 11, ACC_EMPTY = 15, MID_FULL = 19, D_FULL = 25, A_READY = 26,
+           kBars = 27 };
 
 struct Args {
     const bf16 *x;
@@ -112,14 +121,36 @@ __global__ void __launch_bounds__(256) pack_kernel(const Weights w, unsigned cha
 }
 
 // ----------------------------------------------------------------------------------- PTX
-__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// The same value in every lane, known as such to the compiler.
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
+// Matrix descriptors are built from their low word (address >> 4) where they are used; the high word is
+// the same for all: 1024 bytes between eight-row groups, version 1, 128-byte swizzle.
+constexpr uint32_t kDescHigh = 64u | 1u << 14 | 2u << 29;
+
+__device__ __forceinline__ void umma_ss(uint32_t d, uint32_t a_low, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n"
         ".reg .pred p;\n"
+        ".reg .b64 da, db;\n"
+        "mov.b64 da, {%1, %5};\n"
+        "mov.b64 db, {%2, %5};\n"
         "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
         "}\n" ::"r"(d),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "n"(kDescHigh)
+        : "memory");
+}
+__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a_tmem, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        ".reg .b64 db;\n"
+        "mov.b64 db, {%2, %5};\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n"
+        "}\n" ::"r"(d),
+        "r"(a_tmem), "r"(b_low), "r"(idesc), "r"(accumulate), "n"(kDescHigh)
         : "memory");
 }
 __device__ __forceinline__ void ld16(uint32_t t, uint32_t *r) {
@@ -237,7 +268,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
-    const uint32_t tmem = *reinterpret_cast<volatile int *>(tmem_at);
+    const uint32_t tmem = uniform(*reinterpret_cast<volatile uint32_t *>(tmem_at));
     const bool start = *reinterpret_cast<volatile int *>(abort_flag) == 0;
     if (!start && threadIdx.x == 0) atomicCAS(a.status, 0, 175);
     // Waits of warp-wide code: the lanes agree on the outcome, since it decides what the warp runs next.
@@ -252,42 +283,54 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
     if (warp < 4) {
         // ------------------------------------------------------------------------- pixels
         const int img = threadIdx.x;
-        uint4 v[7];
-        const auto load = [&](int tile, int pair) {
-            const int b = tile * kImages + img;
+        uint4 v[2][7];
+        // row pair `pair` of this CTA's i-th tile (pairs count on into the next tiles)
+        const auto load = [&](int i, int pair, uint4 (&dst)[7]) {
+            if (pair >= kPairs) {
+                pair -= kPairs;
+                ++i;
+            }
+            const int64_t b = ((int64_t)blockIdx.x + (int64_t)i * gridDim.x) * kImages + img;
 #pragma unroll
-            for (int i = 0; i < 7; ++i)
-                v[i] = b < a.bs ? __ldg(reinterpret_cast<const uint4 *>(a.x + (int64_t)b * kPix + pair * 56) + i)
-                                : make_uint4(0, 0, 0, 0);
+            for (int q = 0; q < 7; ++q)
+                dst[q] = b < a.bs ? __ldg(reinterpret_cast<const uint4 *>(a.x + b * kPix + pair * 56) + q)
+                                  : make_uint4(0, 0, 0, 0);
         };
-        if (ok) load(blockIdx.x, 0);
+        if (ok) {
+            load(0, 0, v[0]);
+            load(0, 1, v[1]);
+        }
         uint32_t g = 0;
-        for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
+        int i = 0;
+        for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x, ++i) {
             bool bad = false;
-            for (int pair = 0; pair < kPairs; ++pair, ++g) {
-                const uint32_t slot = g & 3;
-                if (!(ok = wait(IN_EMPTY + slot, ((g >> 2) & 1) ^ 1))) break;
-                uint32_t w[28];
+            for (int pair = 0; ok && pair < kPairs; pair += 2) {
 #pragma unroll
-                for (int i = 0; i < 7; ++i) {
-                    w[4 * i] = v[i].x; w[4 * i + 1] = v[i].y; w[4 * i + 2] = v[i].z; w[4 * i + 3] = v[i].w;
+                for (int half = 0; half < 2; ++half, ++g) {
+                    const uint32_t slot = g & 3;   // its low bit is `half`
+                    if (!(ok = wait(IN_EMPTY + slot, ((g >> 2) & 1) ^ 1))) break;
+                    uint32_t w[28];
+#pragma unroll
+                    for (int q = 0; q < 7; ++q) {
+                        w[4 * q] = v[half][q].x; w[4 * q + 1] = v[half][q].y;
+                        w[4 * q + 2] = v[half][q].z; w[4 * q + 3] = v[half][q].w;
+                    }
+                    load(i, pair + half + 2, v[half]);
+                    const uint32_t group = IN_OFF + (slot >> 1) * IN_GROUP + img * 128;
+#pragma unroll
+                    for (int b = 0; b < 6; ++b) {
+                        const uint32_t block = b < 4 ? half : 2, piece = b < 4 ? 2 * b : 4 * half + 2 * (b - 4);
+#pragma unroll
+                        for (int r = 0; r < 2; ++r)
+                            *reinterpret_cast<uint4 *>(smem + group + block * IN_BLOCK + (((piece + r) ^ (img & 7)) << 4)) =
+                                make_uint4(w[14 * r + 2 * b], w[14 * r + 2 * b + 1], w[14 * r + 2 * b + 2], w[14 * r + 2 * b + 3]);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 28; ++q) bad |= not_finite(w[q]);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    arrive(IN_FULL + slot);
                 }
-                const bool more = pair + 1 < kPairs;
-                if (more || tile + (int)gridDim.x < tiles) load(more ? tile : tile + gridDim.x, more ? pair + 1 : 0);
-                const uint32_t row = IN_OFF + (slot >> 1) * IN_GROUP + img * 128;
-#pragma unroll
-                for (int b = 0; b < 6; ++b) {
-                    const uint32_t s = (slot & 1) * 6 + b, block = s >> 2, piece = (s & 3) * 2;
-#pragma unroll
-                    for (int r = 0; r < 2; ++r)
-                        *reinterpret_cast<uint4 *>(smem + row + block * IN_BLOCK + (((piece + r) ^ (img & 7)) << 4)) =
-                            make_uint4(w[14 * r + 2 * b], w[14 * r + 2 * b + 1], w[14 * r + 2 * b + 2], w[14 * r + 2 * b + 3]);
-                }
-#pragma unroll
-                for (int i = 0; i < 28; ++i) bad |= not_finite(w[i]);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                arrive(IN_FULL + slot);
             }
             if (bad) a.bad[tile] = 1;
         }
@@ -295,24 +338,55 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
         // ---------------------------------------------------------- accumulators -> operands
         const int set = (warp - 4) >> 2;
         const uint32_t t = tmem + ((uint32_t)(warp & 3) << 21);   // lanes 32 * (warp % 4) ..
-        const uint32_t acc = t + 64 * set;
-        uint32_t jobs = 0, dense = 0;
+        const uint32_t acc = t + 96 * set;
+        uint32_t phase[2] = {0, 0}, dense = 0;
         for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
-            uint32_t held[8], top = 0;
-            for (int p = 0; ok && p < kRows; ++p) {
-                const uint32_t mid = t + MID + 48 * (p % 6);
-#pragma unroll 1
-                for (int b = set; b < 6; b += 2, ++jobs) {
-                    if (!(ok = wait(ACC_FULL + set, jobs & 1))) break;
+            uint32_t held[5][8], top = 0;   // pooled rows 1 and 2, left half of row 3
+            // conv2's pooled row Q: channel half `set` of both column halves
+            const auto pooled_row = [&](auto row) {
+                constexpr int Q = decltype(row)::value;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (!(ok = wait(ACC_FULL + 2 * set, phase[0]))) return;
+                    phase[0] ^= 1;
                     tc::tc_fence_after();
-                    uint32_t r[48], o[6];
-                    ld16(acc, r);
-                    ld16(acc + 16, r + 16);
-                    ld16(acc + 32, r + 32);
+                    uint32_t r[64], now[8];
+                    uint32_t *o = Q == 0 || (Q == 3 && h == 1) ? now : held[2 * (Q - 1) + h];
+#pragma unroll
+                    for (int i = 0; i < 64; i += 16) ld16(acc + i, r + i);
                     tc::tmem_ld_wait();
                     tc::tc_fence_before();
                     __syncwarp();
-                    arrive(ACC_EMPTY + set);
+                    arrive(ACC_EMPTY + 2 * set);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        o[i] = pack(pool4(r[4 * i], r[4 * i + 1], r[32 + 4 * i], r[32 + 4 * i + 1]),
+                                    pool4(r[4 * i + 2], r[4 * i + 3], r[32 + 4 * i + 2], r[32 + 4 * i + 3]));
+                    if (Q == 0) st8(t + FLAT + 16 * h + 8 * set, o);
+                    if (Q == 3 && h == 1) {
+                        // conv2's left halves are complete: the columns of pixels 0..7 are free
+#pragma unroll
+                        for (int c = 0; c < 5; ++c) st8(t + late_columns(2 * c + set), held[c]);
+                        st8(t + late_columns(10 + set), o);
+                    }
+                }
+            };
+            for (int p = 0; ok && p < kRows; ++p) {
+                const uint32_t mid = t + MID + 48 * (p % 6);
+                // conv1's blocks of this set; its buffers alternate
+#pragma unroll 1
+                for (int b = set; b < 6; b += 2) {
+                    const int k = (p + (b >> 1)) & 1;
+                    if (!(ok = wait(ACC_FULL + 2 * set + k, k ? phase[1] : phase[0]))) break;
+                    (k ? phase[1] : phase[0]) ^= 1;
+                    tc::tc_fence_after();
+                    uint32_t r[48], o[6];
+#pragma unroll
+                    for (int i = 0; i < 48; i += 16) ld16(acc + 48 * k + i, r + i);
+                    tc::tmem_ld_wait();
+                    tc::tc_fence_before();
+                    __syncwarp();
+                    arrive(ACC_EMPTY + 2 * set + k);
 #pragma unroll
                     for (int i = 0; i < 6; ++i) {
                         o[i] = pack(pool4(r[8 * i], r[8 * i + 1], r[8 * i + 2], r[8 * i + 3]),
@@ -331,34 +405,14 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                 __syncwarp();
                 arrive(MID_FULL + p % 6);
                 if (p < 5 || (p & 1) == 0) continue;
-                // conv2's pooled row q: channel half `set` of both column halves
-                const int q = (p - 5) >> 1;
-#pragma unroll 1
-                for (int h = 0; h < 2; ++h, ++jobs) {
-                    if (!(ok = wait(ACC_FULL + set, jobs & 1))) break;
-                    tc::tc_fence_after();
-                    uint32_t r[64], o[8];
-#pragma unroll
-                    for (int i = 0; i < 64; i += 16) ld16(acc + i, r + i);
-                    tc::tmem_ld_wait();
-                    tc::tc_fence_before();
-                    __syncwarp();
-                    arrive(ACC_EMPTY + set);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        o[i] = pack(pool4(r[4 * i], r[4 * i + 1], r[32 + 4 * i], r[32 + 4 * i + 1]),
-                                    pool4(r[4 * i + 2], r[4 * i + 3], r[32 + 4 * i + 2], r[32 + 4 * i + 3]));
-                    if (q < 3) {
-                        st8(t + FLAT + 32 * q + 16 * h + 8 * set, o);
-                    } else if (h == 0) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) held[i] = o[i];
-                    } else {
-                        // conv1's rows are free where conv2 read pixels 0..7: its left half is complete
-                        st8(t + MID + 8 * set, held);
-                        st8(t + MID + 48 + 8 * set, o);
-                    }
-                }
+                if (p == 5)
+                    pooled_row(std::integral_constant<int, 0>());
+                else if (p == 7)
+                    pooled_row(std::integral_constant<int, 1>());
+                else if (p == 9)
+                    pooled_row(std::integral_constant<int, 2>());
+                else
+                    pooled_row(std::integral_constant<int, 3>());
             }
             if (!ok) break;
             if (top >= 0x7f800000u) a.bad[tile] = 1;
@@ -379,14 +433,14 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                 const bf16 *bias = (const bf16 *)a.w.bias[0];
                 uint32_t r[64], o[32];
 #pragma unroll
-                for (int i = 0; i < 64; i += 16) ld16(acc + i, r + i);
+                for (int i = 0; i < 64; i += 16) ld16(t + 64 * set + i, r + i);
                 tc::tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 32; ++i)
                     o[i] = pack(fmaxf(dense_value(r[2 * i], bias, 64 * set + 2 * i, D1), 0.f),
                                 fmaxf(dense_value(r[2 * i + 1], bias, 64 * set + 2 * i + 1, D1), 0.f));
 #pragma unroll
-                for (int i = 0; i < 32; i += 8) st8(t + FLAT + 32 * set + i, o + i);
+                for (int i = 0; i < 32; i += 8) st8(t + HIDDEN + 32 * set + i, o + i);
             }
             st_wait();
             tc::tc_fence_before();
@@ -447,11 +501,13 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
             if (tc::elect_one()) tc::umma_commit(bar(i));
             __syncwarp();
         };
-        const auto desc = [&](uint32_t at) { return tc::make_smem_desc(base + at, 0, 1024); };
+        const auto low = [&](uint32_t at) { return uniform((base + at) >> 4); };
         constexpr uint32_t id48 = tc::make_idesc(false, false, 128, 48), id32 = tc::make_idesc(false, false, 128, 32);
         constexpr uint32_t id128 = tc::make_idesc(false, false, 128, D1), id96 = tc::make_idesc(false, false, 128, D2P);
         constexpr uint32_t id16 = tc::make_idesc(false, false, 128, D3P);
-        uint32_t g = 0, jobs[2] = {0, 0}, mids = 0, ready = 0;
+        const uint32_t b1 = low(B1_OFF), b2 = low(B2_OFF), w1 = low(W1_OFF), w2 = low(W2_OFF), w3 = low(W3_OFF);
+        uint32_t g = 0, mids = 0, ready = 0;
+        uint32_t free_phase[4] = {1, 1, 1, 1};   // of ACC_EMPTY
         bool first = true;
         for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
             if (first) ok = wait(W_FULL, 0);
@@ -459,20 +515,25 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                 // row p reads row pairs p, p + 1, p + 2
                 for (int i = p == 0 ? 0 : 2; ok && i < 3; ++i) ok = wait(IN_FULL + ((g + p + i) & 3), ((g + p + i) >> 2) & 1);
                 if (!ok) break;
-                tc::tc_fence_after();
+                uint32_t left[3], right[3];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    const uint32_t slot = (g + p + i) & 3;
+                    left[i] = low(IN_OFF + (slot >> 1) * IN_GROUP + (slot & 1) * IN_BLOCK);
+                    right[i] = low(IN_OFF + (slot >> 1) * IN_GROUP + 2 * IN_BLOCK + (slot & 1) * 64);
+                }
 #pragma unroll
                 for (int b = 0; b < 6; ++b) {
-                    if (!(ok = wait(ACC_EMPTY + (b & 1), (jobs[b & 1]++ & 1) ^ 1))) break;
+                    const int k = (p + (b >> 1)) & 1, at = 2 * (b & 1) + k;
+                    if (!(ok = wait(ACC_EMPTY + at, k ? free_phase[2 * (b & 1) + 1] : free_phase[2 * (b & 1)]))) break;
+                    (k ? free_phase[2 * (b & 1) + 1] : free_phase[2 * (b & 1)]) ^= 1;
                     tc::tc_fence_after();
+                    const uint32_t d = uniform(tmem + 48 * (uint32_t)k);
                     if (tc::elect_one()) {
 #pragma unroll
-                        for (int i = 0; i < 3; ++i) {
-                            const uint32_t slot = (g + p + i) & 3, s = (slot & 1) * 6 + b;
-                            tc::umma_bf16(tmem + 64 * (b & 1),
-                                          desc(IN_OFF + (slot >> 1) * IN_GROUP + (s >> 2) * IN_BLOCK + (s & 3) * 32),
-                                          desc(B1_OFF + 32 * i), id48, i > 0);
-                        }
-                        tc::umma_commit(bar(ACC_FULL + (b & 1)));
+                        for (int i = 0; i < 3; ++i)
+                            umma_ss(d + 96 * (b & 1), b < 4 ? left[i] + 2 * b : right[i] + 2 * (b - 4), b1 + 2 * i, id48, i > 0);
+                        tc::umma_commit(bar(ACC_FULL + at));
                     }
                     __syncwarp();
                 }
@@ -488,28 +549,27 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                 // each of the six row slots is filled twice per tile
                 for (int row = q == 0 ? 0 : p - 1; ok && row <= p; ++row) ok = wait(MID_FULL + row % 6, (mids + row / 6) & 1);
                 if (!ok) break;
-                tc::tc_fence_after();
+                uint32_t rows[6];
+#pragma unroll
+                for (int i = 0; i < 6; ++i) rows[i] = uniform(tmem + MID + 48 * ((2 * q + i) % 6));
 #pragma unroll 1
                 for (int job = 0; job < 4; ++job) {
                     const int h = job >> 1, half = job & 1;
-                    if (!(ok = wait(ACC_EMPTY + half, (jobs[half]++ & 1) ^ 1))) break;
+                    // the set's one large buffer covers its second small one too
+                    if (!(ok = wait(ACC_EMPTY + 2 * half, half ? free_phase[2] : free_phase[0]))) break;
+                    if (!(ok = wait(ACC_EMPTY + 2 * half + 1, half ? free_phase[3] : free_phase[1]))) break;
+                    (half ? free_phase[2] : free_phase[0]) ^= 1;
                     tc::tc_fence_after();
+                    const uint32_t d = uniform(tmem + 96 * (uint32_t)half), b = uniform(b2 + 256 * (uint32_t)half);
+                    const uint32_t left_or_right = uniform(24 * (uint32_t)h);
                     if (tc::elect_one()) {
-#pragma unroll 1
-                        for (int dy = 0; dy < 2; ++dy) {
-                            int slot = (2 * q + dy) % 6;
 #pragma unroll
-                            for (int fi = 0; fi < 5; ++fi) {
+                        for (int dy = 0; dy < 2; ++dy)
 #pragma unroll
-                                for (int i = 0; i < 3; ++i) {
-                                    const int s = 3 * fi + i;
-                                    umma_ts(tmem + 64 * half + 32 * dy, tmem + MID + 48 * slot + 24 * h + 8 * i,
-                                            desc(B2_OFF + (s >> 2) * B2_CHUNK + half * 4096 + (s & 3) * 32), id32, s > 0);
-                                }
-                                slot = slot == 5 ? 0 : slot + 1;
-                            }
-                        }
-                        tc::umma_commit(bar(ACC_FULL + half));
+                            for (int s = 0; s < 15; ++s)
+                                umma_ts(d + 32 * dy, rows[dy + s / 3] + left_or_right + 8 * (s % 3),
+                                        b + (s >> 2) * (B2_CHUNK / 16) + 2 * (s & 3), id32, s > 0);
+                        tc::umma_commit(bar(ACC_FULL + 2 * half));
                     }
                     __syncwarp();
                 }
@@ -524,10 +584,9 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
             tc::tc_fence_after();
             if (tc::elect_one()) {
 #pragma unroll
-                for (int s = 0; s < 16; ++s) {
-                    const uint32_t at = s < 12 ? FLAT + 8 * s : MID + 48 * ((s - 12) >> 1) + 8 * (s & 1);
-                    umma_ts(tmem, tmem + at, desc(W1_OFF + (s >> 2) * W1_CHUNK + (s & 3) * 32), id128, s > 0);
-                }
+                for (int s = 0; s < 16; ++s)
+                    umma_ts(tmem, tmem + (s < 4 ? FLAT + 8 * s : late_columns(s - 4)), w1 + (s >> 2) * (W1_CHUNK / 16) + 2 * (s & 3),
+                            id128, s > 0);
                 tc::umma_commit(bar(D_FULL));
             }
             __syncwarp();
@@ -536,7 +595,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
             if (tc::elect_one()) {
 #pragma unroll
                 for (int s = 0; s < 8; ++s)
-                    umma_ts(tmem, tmem + FLAT + 8 * s, desc(W2_OFF + (s >> 2) * W2_CHUNK + (s & 3) * 32), id96, s > 0);
+                    umma_ts(tmem, tmem + HIDDEN + 8 * s, w2 + (s >> 2) * (W2_CHUNK / 16) + 2 * (s & 3), id96, s > 0);
                 tc::umma_commit(bar(D_FULL));
             }
             __syncwarp();
@@ -545,7 +604,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
             if (tc::elect_one()) {
 #pragma unroll
                 for (int s = 0; s < 6; ++s)
-                    umma_ts(tmem, tmem + MID + 8 * s, desc(W3_OFF + (s >> 2) * W3_CHUNK + (s & 3) * 32), id16, s > 0);
+                    umma_ts(tmem, tmem + MID + 8 * s, w3 + (s >> 2) * (W3_CHUNK / 16) + 2 * (s & 3), id16, s > 0);
                 tc::umma_commit(bar(D_FULL));
             }
             __syncwarp();
