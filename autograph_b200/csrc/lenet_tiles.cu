@@ -13,15 +13,17 @@
 // Pixels come through shared memory (the window of a k step is 32 contiguous bytes of an image's row).
 // From conv1's output on, the activations live in tensor memory only, where the accumulators' readers
 // (a thread per image) put them as the next product's A operand, packed in pairs:
-//   columns [0, 192)   accumulators: for each of the two sets of readers two buffers of 48 (conv1) or one of 64
-//                      (conv2); 128 for the dense layers
+//   columns [0, 192)   accumulators: four buffers of 48 (conv1), two of 64 at the same places as two of those
+//                      each (conv2), 128 for the dense layers
 //   columns [192, 480) six rows of conv1's pooled output: 24 columns for pixels 0..7, 24 for pixels 4..11
 //   columns [480, 512) pooled row 0 of conv2's output; rows 1 to 3 wait in registers until conv2 has read
 //                      the last of conv1's rows, and take their place
-// Warps 0-3 load pixels (two row pairs ahead), 4-11 (two sets of four) turn accumulators into the next
-// operand, warp 12 issues.  The issuing thread is chosen by elect.sync and what varies between its operands
-// is made warp-uniform first: behind a lane test, or with operands from ordinary registers, a
-// tcgen05.mma takes 46-93 cycles to issue (measured), here about 10; the products themselves take 16 to 64.
+// Warps 0-3 load pixels (two row pairs ahead), 4-19 (four sets, one per small buffer) turn accumulators into
+// the next operand, warp 20 issues.  Reading accumulators is a chain of latencies (wait, load, maximum, pack,
+// store), so warps count: with two sets a tile took 33 us.  The issuing thread is chosen by elect.sync and
+// what varies between its operands is made warp-uniform first: behind a lane test, or with operands from
+// ordinary registers, a tcgen05.mma takes 46-93 cycles to issue (measured), here about 10; the products
+// themselves take 16 to 64.
 //
 // 0 x infinity is not 0: a tile with a pixel or an activation that is not finite is marked and its
 // images are computed again by plain loops at the end.
@@ -39,7 +41,7 @@ namespace lenet_tiles {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int kImages = 128, kThreads = 13 * 32;
+constexpr int kImages = 128, kSets = 4, kIssuer = 4 + 4 * kSets, kThreads = 32 * (kIssuer + 1);
 constexpr int kPix = 784, kPairs = 14, kRows = 12;     // row pairs of an image, pooled rows after conv1
 constexpr int D1 = 128, D2 = 84, D3 = 10, D2P = 96, D3P = 16;
 
@@ -163,6 +165,17 @@ __device__ __forceinline__ void ld16(uint32_t t, uint32_t *r) {
 __device__ __forceinline__ void st2(uint32_t t, const uint32_t *r) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(t), "r"(r[0]), "r"(r[1]) : "memory");
 }
+__device__ __forceinline__ void ld8(uint32_t t, uint32_t *r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(t)
+                 : "memory");
+}
+__device__ __forceinline__ void st4(uint32_t t, const uint32_t *r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(t), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3])
+                 : "memory");
+}
 __device__ __forceinline__ void st8(uint32_t t, const uint32_t *r) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(t), "r"(r[0]),
                  "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
@@ -256,12 +269,12 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
         *abort_flag = (base & 1023u) != 0;   // the swizzled layouts start on 1024-byte boundaries
         for (int i = 0; i < kBars; ++i) {
             const bool warps4 = (i >= IN_FULL && i < IN_EMPTY) || (i >= ACC_EMPTY && i < MID_FULL);
-            const bool warps8 = (i >= MID_FULL && i < D_FULL) || i == A_READY;
-            tc::mbar_init(bar(i), warps4 ? 4 : warps8 ? 8 : 1);
+            const bool readers = (i >= MID_FULL && i < D_FULL) || i == A_READY;
+            tc::mbar_init(bar(i), warps4 ? 4 : readers ? 4 * kSets : 1);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 12) {
+    if (warp == kIssuer) {
         tc::tmem_alloc(tc::smem_u32(tmem_at), 512);
         tc::tmem_relinquish();
     }
@@ -309,13 +322,10 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                 for (int half = 0; half < 2; ++half, ++g) {
                     const uint32_t slot = g & 3;   // its low bit is `half`
                     if (!(ok = wait(IN_EMPTY + slot, ((g >> 2) & 1) ^ 1))) break;
-                    uint32_t w[28];
-#pragma unroll
-                    for (int q = 0; q < 7; ++q) {
-                        w[4 * q] = v[half][q].x; w[4 * q + 1] = v[half][q].y;
-                        w[4 * q + 2] = v[half][q].z; w[4 * q + 3] = v[half][q].w;
-                    }
-                    load(i, pair + half + 2, v[half]);
+                    const auto w = [&](int n) {
+                        const uint4 &q = v[half][n >> 2];
+                        return (n & 3) == 0 ? q.x : (n & 3) == 1 ? q.y : (n & 3) == 2 ? q.z : q.w;
+                    };
                     const uint32_t group = IN_OFF + (slot >> 1) * IN_GROUP + img * 128;
 #pragma unroll
                     for (int b = 0; b < 6; ++b) {
@@ -323,10 +333,11 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
 #pragma unroll
                         for (int r = 0; r < 2; ++r)
                             *reinterpret_cast<uint4 *>(smem + group + block * IN_BLOCK + (((piece + r) ^ (img & 7)) << 4)) =
-                                make_uint4(w[14 * r + 2 * b], w[14 * r + 2 * b + 1], w[14 * r + 2 * b + 2], w[14 * r + 2 * b + 3]);
+                                make_uint4(w(14 * r + 2 * b), w(14 * r + 2 * b + 1), w(14 * r + 2 * b + 2), w(14 * r + 2 * b + 3));
                     }
 #pragma unroll
-                    for (int q = 0; q < 28; ++q) bad |= not_finite(w[q]);
+                    for (int q = 0; q < 28; ++q) bad |= not_finite(w(q));
+                    load(i, pair + half + 2, v[half]);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
                     arrive(IN_FULL + slot);
@@ -334,69 +345,74 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
             }
             if (bad) a.bad[tile] = 1;
         }
-    } else if (warp < 12) {
+    } else if (warp < kIssuer) {
         // ---------------------------------------------------------- accumulators -> operands
         const int set = (warp - 4) >> 2;
         const uint32_t t = tmem + ((uint32_t)(warp & 3) << 21);   // lanes 32 * (warp % 4) ..
-        const uint32_t acc = t + 96 * set;
-        uint32_t phase[2] = {0, 0}, dense = 0;
+        const uint32_t acc = t + 48 * set;
+        uint32_t phase = 0, dense = 0;
         for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
-            uint32_t held[5][8], top = 0;   // pooled rows 1 and 2, left half of row 3
-            // conv2's pooled row Q: channel half `set` of both column halves
+            uint32_t held[5][4];   // conv2's pooled rows 1 and 2, left half of row 3
+            __nv_bfloat162 top = __floats2bfloat162_rn(0.f, 0.f);
+            // conv2's pooled row Q: sets 0 and 1 have channels 0..7, 2 and 3 the others, each set one column
+            // of each half
             const auto pooled_row = [&](auto row) {
                 constexpr int Q = decltype(row)::value;
+                const uint32_t from = t + 96 * (set >> 1) + 16 * (set & 1), word = 4 * (set & 1);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    if (!(ok = wait(ACC_FULL + 2 * set, phase[0]))) return;
-                    phase[0] ^= 1;
+                    if (!(ok = wait(ACC_FULL + set, phase))) return;
+                    phase ^= 1;
                     tc::tc_fence_after();
-                    uint32_t r[64], now[8];
+                    uint32_t r[32], now[4];
                     uint32_t *o = Q == 0 || (Q == 3 && h == 1) ? now : held[2 * (Q - 1) + h];
-#pragma unroll
-                    for (int i = 0; i < 64; i += 16) ld16(acc + i, r + i);
+                    ld16(from, r);
+                    ld16(from + 32, r + 16);
                     tc::tmem_ld_wait();
                     tc::tc_fence_before();
                     __syncwarp();
-                    arrive(ACC_EMPTY + 2 * set);
+                    arrive(ACC_EMPTY + set);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        o[i] = pack(pool4(r[4 * i], r[4 * i + 1], r[32 + 4 * i], r[32 + 4 * i + 1]),
-                                    pool4(r[4 * i + 2], r[4 * i + 3], r[32 + 4 * i + 2], r[32 + 4 * i + 3]));
-                    if (Q == 0) st8(t + FLAT + 16 * h + 8 * set, o);
+                    for (int i = 0; i < 4; ++i)
+                        o[i] = pack(pool4(r[4 * i], r[4 * i + 1], r[16 + 4 * i], r[16 + 4 * i + 1]),
+                                    pool4(r[4 * i + 2], r[4 * i + 3], r[16 + 4 * i + 2], r[16 + 4 * i + 3]));
+                    if (Q == 0) st4(t + FLAT + 16 * h + 8 * (set >> 1) + word, o);
                     if (Q == 3 && h == 1) {
                         // conv2's left halves are complete: the columns of pixels 0..7 are free
 #pragma unroll
-                        for (int c = 0; c < 5; ++c) st8(t + late_columns(2 * c + set), held[c]);
-                        st8(t + late_columns(10 + set), o);
+                        for (int c = 0; c < 5; ++c) st4(t + late_columns(2 * c + (set >> 1)) + word, held[c]);
+                        st4(t + late_columns(10 + (set >> 1)) + word, o);
                     }
                 }
             };
             for (int p = 0; ok && p < kRows; ++p) {
                 const uint32_t mid = t + MID + 48 * (p % 6);
-                // conv1's blocks of this set; its buffers alternate
+                // conv1's blocks go round the sets
 #pragma unroll 1
-                for (int b = set; b < 6; b += 2) {
-                    const int k = (p + (b >> 1)) & 1;
-                    if (!(ok = wait(ACC_FULL + 2 * set + k, k ? phase[1] : phase[0]))) break;
-                    (k ? phase[1] : phase[0]) ^= 1;
+                for (int b = (set - 6 * p) & 3; b < 6; b += 4) {
+                    if (!(ok = wait(ACC_FULL + set, phase))) break;
+                    phase ^= 1;
                     tc::tc_fence_after();
                     uint32_t r[48], o[6];
 #pragma unroll
-                    for (int i = 0; i < 48; i += 16) ld16(acc + 48 * k + i, r + i);
+                    for (int i = 0; i < 48; i += 16) ld16(acc + i, r + i);
                     tc::tmem_ld_wait();
                     tc::tc_fence_before();
                     __syncwarp();
-                    arrive(ACC_EMPTY + 2 * set + k);
+                    arrive(ACC_EMPTY + set);
 #pragma unroll
                     for (int i = 0; i < 6; ++i) {
                         o[i] = pack(pool4(r[8 * i], r[8 * i + 1], r[8 * i + 2], r[8 * i + 3]),
                                     pool4(r[8 * i + 4], r[8 * i + 5], r[8 * i + 6], r[8 * i + 7]));
-                        top = max(top, max(o[i] & 0x7fff0000u, o[i] << 16));
+                        top = __hmax2(top, *reinterpret_cast<const __nv_bfloat162 *>(&o[i]));
                     }
-#pragma unroll
-                    for (int i = 0; i < 6; i += 2) {
-                        if (b < 4) st2(mid + 6 * b + i, o + i);
-                        if (b >= 2) st2(mid + 24 + 6 * (b - 2) + i, o + i);
+                    if (b < 4) {
+                        st4(mid + 6 * b, o);
+                        st2(mid + 6 * b + 4, o + 4);
+                    }
+                    if (b >= 2) {
+                        st4(mid + 24 + 6 * (b - 2), o);
+                        st2(mid + 24 + 6 * (b - 2) + 4, o + 4);
                     }
                 }
                 if (!ok) break;
@@ -404,23 +420,22 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                 tc::tc_fence_before();
                 __syncwarp();
                 arrive(MID_FULL + p % 6);
-                if (p < 5 || (p & 1) == 0) continue;
                 if (p == 5)
                     pooled_row(std::integral_constant<int, 0>());
                 else if (p == 7)
                     pooled_row(std::integral_constant<int, 1>());
                 else if (p == 9)
                     pooled_row(std::integral_constant<int, 2>());
-                else
+                else if (p == 11)
                     pooled_row(std::integral_constant<int, 3>());
             }
             if (!ok) break;
-            if (top >= 0x7f800000u) a.bad[tile] = 1;
+            if (not_finite(*reinterpret_cast<const uint32_t *>(&top))) a.bad[tile] = 1;
             st_wait();
             tc::tc_fence_before();
             __syncwarp();
             arrive(A_READY);
-            // ---- dense layers: half of the columns each
+            // ---- dense layers: a quarter of the columns each
             const int b = tile * kImages + (warp & 3) * 32 + lane;
             const auto dense_value = [&](uint32_t r, const bf16 *bias, int n, int N) {
                 float v = __bfloat162float(__float2bfloat16(__uint_as_float(r)));
@@ -431,16 +446,16 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
             tc::tc_fence_after();
             {
                 const bf16 *bias = (const bf16 *)a.w.bias[0];
-                uint32_t r[64], o[32];
-#pragma unroll
-                for (int i = 0; i < 64; i += 16) ld16(t + 64 * set + i, r + i);
+                uint32_t r[32], o[16];
+                ld16(t + 32 * set, r);
+                ld16(t + 32 * set + 16, r + 16);
                 tc::tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    o[i] = pack(fmaxf(dense_value(r[2 * i], bias, 64 * set + 2 * i, D1), 0.f),
-                                fmaxf(dense_value(r[2 * i + 1], bias, 64 * set + 2 * i + 1, D1), 0.f));
-#pragma unroll
-                for (int i = 0; i < 32; i += 8) st8(t + HIDDEN + 32 * set + i, o + i);
+                for (int i = 0; i < 16; ++i)
+                    o[i] = pack(fmaxf(dense_value(r[2 * i], bias, 32 * set + 2 * i, D1), 0.f),
+                                fmaxf(dense_value(r[2 * i + 1], bias, 32 * set + 2 * i + 1, D1), 0.f));
+                st8(t + HIDDEN + 16 * set, o);
+                st8(t + HIDDEN + 16 * set + 8, o + 8);
             }
             st_wait();
             tc::tc_fence_before();
@@ -450,16 +465,16 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
             tc::tc_fence_after();
             {
                 const bf16 *bias = (const bf16 *)a.w.bias[1];
-                uint32_t r[48], o[24];
+                uint32_t r[24], o[12];
 #pragma unroll
-                for (int i = 0; i < 48; i += 16) ld16(t + 48 * set + i, r + i);
+                for (int i = 0; i < 24; i += 8) ld8(t + 24 * set + i, r + i);
                 tc::tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 24; ++i)
-                    o[i] = pack(fmaxf(dense_value(r[2 * i], bias, 48 * set + 2 * i, D2), 0.f),
-                                fmaxf(dense_value(r[2 * i + 1], bias, 48 * set + 2 * i + 1, D2), 0.f));
+                for (int i = 0; i < 12; ++i)
+                    o[i] = pack(fmaxf(dense_value(r[2 * i], bias, 24 * set + 2 * i, D2), 0.f),
+                                fmaxf(dense_value(r[2 * i + 1], bias, 24 * set + 2 * i + 1, D2), 0.f));
 #pragma unroll
-                for (int i = 0; i < 24; i += 8) st8(t + MID + 24 * set + i, o + i);
+                for (int i = 0; i < 12; i += 4) st4(t + MID + 12 * set + i, o + i);
             }
             st_wait();
             tc::tc_fence_before();
@@ -507,7 +522,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
         constexpr uint32_t id16 = tc::make_idesc(false, false, 128, D3P);
         const uint32_t b1 = low(B1_OFF), b2 = low(B2_OFF), w1 = low(W1_OFF), w2 = low(W2_OFF), w3 = low(W3_OFF);
         uint32_t g = 0, mids = 0, ready = 0;
-        uint32_t free_phase[4] = {1, 1, 1, 1};   // of ACC_EMPTY
+        uint32_t free_phase = 15;   // of ACC_EMPTY, a bit each
         bool first = true;
         for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
             if (first) ok = wait(W_FULL, 0);
@@ -524,16 +539,16 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                 }
 #pragma unroll
                 for (int b = 0; b < 6; ++b) {
-                    const int k = (p + (b >> 1)) & 1, at = 2 * (b & 1) + k;
-                    if (!(ok = wait(ACC_EMPTY + at, k ? free_phase[2 * (b & 1) + 1] : free_phase[2 * (b & 1)]))) break;
-                    (k ? free_phase[2 * (b & 1) + 1] : free_phase[2 * (b & 1)]) ^= 1;
+                    const uint32_t k = (6 * p + b) & 3;
+                    if (!(ok = wait(ACC_EMPTY + k, ((free_phase >> k) & 1)))) break;
+                    free_phase ^= 1u << k;
                     tc::tc_fence_after();
-                    const uint32_t d = uniform(tmem + 48 * (uint32_t)k);
+                    const uint32_t d = uniform(tmem + 48 * k);
                     if (tc::elect_one()) {
 #pragma unroll
                         for (int i = 0; i < 3; ++i)
-                            umma_ss(d + 96 * (b & 1), b < 4 ? left[i] + 2 * b : right[i] + 2 * (b - 4), b1 + 2 * i, id48, i > 0);
-                        tc::umma_commit(bar(ACC_FULL + at));
+                            umma_ss(d, b < 4 ? left[i] + 2 * b : right[i] + 2 * (b - 4), b1 + 2 * i, id48, i > 0);
+                        tc::umma_commit(bar(ACC_FULL + k));
                     }
                     __syncwarp();
                 }
@@ -555,10 +570,10 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
 #pragma unroll 1
                 for (int job = 0; job < 4; ++job) {
                     const int h = job >> 1, half = job & 1;
-                    // the set's one large buffer covers its second small one too
-                    if (!(ok = wait(ACC_EMPTY + 2 * half, half ? free_phase[2] : free_phase[0]))) break;
-                    if (!(ok = wait(ACC_EMPTY + 2 * half + 1, half ? free_phase[3] : free_phase[1]))) break;
-                    (half ? free_phase[2] : free_phase[0]) ^= 1;
+                    // a large buffer is two small ones, read by both sets
+                    if (!(ok = wait(ACC_EMPTY + 2 * half, (free_phase >> (2 * half)) & 1))) break;
+                    if (!(ok = wait(ACC_EMPTY + 2 * half + 1, (free_phase >> (2 * half + 1)) & 1))) break;
+                    free_phase ^= 3u << (2 * half);
                     tc::tc_fence_after();
                     const uint32_t d = uniform(tmem + 96 * (uint32_t)half), b = uniform(b2 + 256 * (uint32_t)half);
                     const uint32_t left_or_right = uniform(24 * (uint32_t)h);
@@ -570,6 +585,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                                 umma_ts(d + 32 * dy, rows[dy + s / 3] + left_or_right + 8 * (s % 3),
                                         b + (s >> 2) * (B2_CHUNK / 16) + 2 * (s & 3), id32, s > 0);
                         tc::umma_commit(bar(ACC_FULL + 2 * half));
+                        tc::umma_commit(bar(ACC_FULL + 2 * half + 1));
                     }
                     __syncwarp();
                 }
@@ -620,7 +636,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
-    if (warp == 12) tc::tmem_dealloc(tmem, 512);
+    if (warp == kIssuer) tc::tmem_dealloc(tmem, 512);
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         if (*reinterpret_cast<volatile int *>(a.bad + tile) == 0) continue;
         for (int b = tile * kImages; b < min(a.bs, (tile + 1) * kImages); ++b)
