@@ -500,8 +500,12 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
         }
     } else {
         // ---------------------------------------------------------------------- tensor cores
-        const bool leader = tc::elect_one();
-        if (ok && leader) {
+        // One thread does all of it, so a wait leads straight to the next issue.  Rows go in pairs: which
+        // buffer a block gets is then known at compile time.
+        const uint32_t b1 = (base + B1_OFF) >> 4, b2 = (base + B2_OFF) >> 4, w1 = (base + W1_OFF) >> 4;
+        const uint32_t w2 = (base + W2_OFF) >> 4, w3 = (base + W3_OFF) >> 4;
+        if (ok && tc::elect_one()) {
+            const auto wait1 = [&](int i, uint32_t parity) { return tc::mbar_wait(bar(i), parity, abort_flag); };
             const int off[3] = {B1_OFF, B2_OFF, W1_OFF}, bytes[3] = {B1_BYTES, B2_BYTES, kBlob - W1_OFF};
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
@@ -510,127 +514,111 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                              ::"r"(base + off[i]), "l"(a.blob + off[i]), "r"((uint32_t)bytes[i]), "r"(bar(W_FULL + i))
                              : "memory");
             }
-        }
-        __syncwarp();
-        const auto commit = [&](int i) {
-            if (tc::elect_one()) tc::umma_commit(bar(i));
-            __syncwarp();
-        };
-        const auto low = [&](uint32_t at) { return uniform((base + at) >> 4); };
-        constexpr uint32_t id48 = tc::make_idesc(false, false, 128, 48), id32 = tc::make_idesc(false, false, 128, 32);
-        constexpr uint32_t id128 = tc::make_idesc(false, false, 128, D1), id96 = tc::make_idesc(false, false, 128, D2P);
-        constexpr uint32_t id16 = tc::make_idesc(false, false, 128, D3P);
-        const uint32_t b1 = low(B1_OFF), b2 = low(B2_OFF), w1 = low(W1_OFF), w2 = low(W2_OFF), w3 = low(W3_OFF);
-        uint32_t g = 0, mids = 0, ready = 0;
-        uint32_t free_phase = 15;   // of ACC_EMPTY, a bit each
-        bool first = true;
-        for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
-            if (first) ok = wait(W_FULL, 0);
-            for (int p = 0; ok && p < kRows; ++p) {
-                // row p reads row pairs p, p + 1, p + 2
-                for (int i = p == 0 ? 0 : 2; ok && i < 3; ++i) ok = wait(IN_FULL + ((g + p + i) & 3), ((g + p + i) >> 2) & 1);
-                if (!ok) break;
-                uint32_t left[3], right[3];
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    const uint32_t slot = (g + p + i) & 3;
-                    left[i] = low(IN_OFF + (slot >> 1) * IN_GROUP + (slot & 1) * IN_BLOCK);
-                    right[i] = low(IN_OFF + (slot >> 1) * IN_GROUP + 2 * IN_BLOCK + (slot & 1) * 64);
-                }
-#pragma unroll
-                for (int b = 0; b < 6; ++b) {
-                    const uint32_t k = (6 * p + b) & 3;
-                    if (!(ok = wait(ACC_EMPTY + k, ((free_phase >> k) & 1)))) break;
-                    free_phase ^= 1u << k;
-                    tc::tc_fence_after();
-                    const uint32_t d = uniform(tmem + 48 * k);
-                    if (tc::elect_one()) {
-#pragma unroll
-                        for (int i = 0; i < 3; ++i)
-                            umma_ss(d, b < 4 ? left[i] + 2 * b : right[i] + 2 * (b - 4), b1 + 2 * i, id48, i > 0);
-                        tc::umma_commit(bar(ACC_FULL + k));
-                    }
-                    __syncwarp();
-                }
-                if (!ok) break;
-                commit(IN_EMPTY + ((g + p) & 3));
-                if (p == kRows - 1) {
-                    commit(IN_EMPTY + ((g + p + 1) & 3));
-                    commit(IN_EMPTY + ((g + p + 2) & 3));
-                }
-                if (p < 5 || (p & 1) == 0) continue;
-                if (first && p == 5 && !(ok = wait(W_FULL + 1, 0))) break;
-                const int q = (p - 5) >> 1;
-                // each of the six row slots is filled twice per tile
-                for (int row = q == 0 ? 0 : p - 1; ok && row <= p; ++row) ok = wait(MID_FULL + row % 6, (mids + row / 6) & 1);
-                if (!ok) break;
-                uint32_t rows[6];
-#pragma unroll
-                for (int i = 0; i < 6; ++i) rows[i] = uniform(tmem + MID + 48 * ((2 * q + i) % 6));
+            constexpr uint32_t id48 = tc::make_idesc(false, false, 128, 48), id32 = tc::make_idesc(false, false, 128, 32);
+            constexpr uint32_t id128 = tc::make_idesc(false, false, 128, D1), id96 = tc::make_idesc(false, false, 128, D2P);
+            constexpr uint32_t id16 = tc::make_idesc(false, false, 128, D3P);
+            uint32_t g = 0, mids = 0, ready = 0;
+            uint32_t free_phase = 15;   // of ACC_EMPTY, a bit each
+            bool first = true;
+            for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
+                if (first) ok = wait1(W_FULL, 0);
 #pragma unroll 1
-                for (int job = 0; job < 4; ++job) {
-                    const int h = job >> 1, half = job & 1;
-                    // a large buffer is two small ones, read by both sets
-                    if (!(ok = wait(ACC_EMPTY + 2 * half, (free_phase >> (2 * half)) & 1))) break;
-                    if (!(ok = wait(ACC_EMPTY + 2 * half + 1, (free_phase >> (2 * half + 1)) & 1))) break;
-                    free_phase ^= 3u << (2 * half);
-                    tc::tc_fence_after();
-                    const uint32_t d = uniform(tmem + 96 * (uint32_t)half), b = uniform(b2 + 256 * (uint32_t)half);
-                    const uint32_t left_or_right = uniform(24 * (uint32_t)h);
-                    if (tc::elect_one()) {
+                for (int p2 = 0; ok && p2 < kRows; p2 += 2) {
 #pragma unroll
-                        for (int dy = 0; dy < 2; ++dy)
+                    for (int odd = 0; odd < 2; ++odd) {
+                        const int p = p2 + odd;
+                        // row p reads row pairs p, p + 1, p + 2
+                        if (p2 == 0 && odd == 0) ok = wait1(IN_FULL + (g & 3), (g >> 2) & 1) && wait1(IN_FULL + ((g + 1) & 3), ((g + 1) >> 2) & 1);
+                        ok = ok && wait1(IN_FULL + ((g + p + 2) & 3), ((g + p + 2) >> 2) & 1);
+                        if (!ok) break;
+                        uint32_t left[3], right[3];
 #pragma unroll
-                            for (int s = 0; s < 15; ++s)
-                                umma_ts(d + 32 * dy, rows[dy + s / 3] + left_or_right + 8 * (s % 3),
-                                        b + (s >> 2) * (B2_CHUNK / 16) + 2 * (s & 3), id32, s > 0);
-                        tc::umma_commit(bar(ACC_FULL + 2 * half));
-                        tc::umma_commit(bar(ACC_FULL + 2 * half + 1));
+                        for (int i = 0; i < 3; ++i) {
+                            const uint32_t slot = (g + p + i) & 3;
+                            left[i] = (base + IN_OFF + (slot >> 1) * IN_GROUP + (slot & 1) * IN_BLOCK) >> 4;
+                            right[i] = (base + IN_OFF + (slot >> 1) * IN_GROUP + 2 * IN_BLOCK + (slot & 1) * 64) >> 4;
+                        }
+#pragma unroll
+                        for (int b = 0; b < 6; ++b) {
+                            const int k = (6 * odd + b) & 3;
+                            if (!(ok = wait1(ACC_EMPTY + k, (free_phase >> k) & 1))) break;
+                            free_phase ^= 1u << k;
+                            tc::tc_fence_after();
+#pragma unroll
+                            for (int i = 0; i < 3; ++i)
+                                umma_ss(tmem + 48 * k, b < 4 ? left[i] + 2 * b : right[i] + 2 * (b - 4), b1 + 2 * i, id48, i > 0);
+                            tc::umma_commit(bar(ACC_FULL + k));
+                        }
+                        if (!ok) break;
+                        tc::umma_commit(bar(IN_EMPTY + ((g + p) & 3)));
                     }
-                    __syncwarp();
+                    if (!ok || p2 < 4) continue;
+                    const int q = (p2 - 4) >> 1;
+                    if (p2 == 10) {
+                        tc::umma_commit(bar(IN_EMPTY + ((g + 12) & 3)));
+                        tc::umma_commit(bar(IN_EMPTY + ((g + 13) & 3)));
+                    }
+                    if (first && q == 0 && !(ok = wait1(W_FULL + 1, 0))) break;
+                    // each of the six row slots is filled twice per tile
+                    for (int row = q == 0 ? 0 : p2; ok && row <= p2 + 1; ++row) ok = wait1(MID_FULL + row % 6, (mids + row / 6) & 1);
+                    if (!ok) break;
+                    uint32_t rows[6];
+#pragma unroll
+                    for (int i = 0; i < 6; ++i) rows[i] = tmem + MID + 48 * ((2 * q + i) % 6);
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int half = 0; half < 2; ++half) {
+                            // a large buffer is two small ones, read by both sets
+                            if (!(ok = ok && wait1(ACC_EMPTY + 2 * half, (free_phase >> (2 * half)) & 1))) break;
+                            if (!(ok = wait1(ACC_EMPTY + 2 * half + 1, (free_phase >> (2 * half + 1)) & 1))) break;
+                            free_phase ^= 3u << (2 * half);
+                            tc::tc_fence_after();
+#pragma unroll
+                            for (int dy = 0; dy < 2; ++dy)
+#pragma unroll
+                                for (int s = 0; s < 15; ++s)
+                                    umma_ts(tmem + 96 * half + 32 * dy, rows[dy + s / 3] + 24 * h + 8 * (s % 3),
+                                            b2 + 256 * half + (s >> 2) * (B2_CHUNK / 16) + 2 * (s & 3), id32, s > 0);
+                            tc::umma_commit(bar(ACC_FULL + 2 * half));
+                            tc::umma_commit(bar(ACC_FULL + 2 * half + 1));
+                        }
                 }
-            }
-            if (!ok) break;
-            g += kPairs;
-            mids += 2;
-            if (first && !(ok = wait(W_FULL + 2, 0))) break;
-            first = false;
-            // the accumulators are free when the flattened rows are complete
-            if (!(ok = wait(A_READY, ready++ & 1))) break;
-            tc::tc_fence_after();
-            if (tc::elect_one()) {
+                if (!ok) break;
+                g += kPairs;
+                mids += 2;
+                if (first && !(ok = wait1(W_FULL + 2, 0))) break;
+                first = false;
+                // the accumulators are free when the flattened rows are complete
+                if (!(ok = wait1(A_READY, ready++ & 1))) break;
+                tc::tc_fence_after();
 #pragma unroll
                 for (int s = 0; s < 16; ++s)
                     umma_ts(tmem, tmem + (s < 4 ? FLAT + 8 * s : late_columns(s - 4)), w1 + (s >> 2) * (W1_CHUNK / 16) + 2 * (s & 3),
                             id128, s > 0);
                 tc::umma_commit(bar(D_FULL));
-            }
-            __syncwarp();
-            if (!(ok = wait(A_READY, ready++ & 1))) break;
-            tc::tc_fence_after();
-            if (tc::elect_one()) {
+                if (!(ok = wait1(A_READY, ready++ & 1))) break;
+                tc::tc_fence_after();
 #pragma unroll
                 for (int s = 0; s < 8; ++s)
                     umma_ts(tmem, tmem + HIDDEN + 8 * s, w2 + (s >> 2) * (W2_CHUNK / 16) + 2 * (s & 3), id96, s > 0);
                 tc::umma_commit(bar(D_FULL));
-            }
-            __syncwarp();
-            if (!(ok = wait(A_READY, ready++ & 1))) break;
-            tc::tc_fence_after();
-            if (tc::elect_one()) {
+                if (!(ok = wait1(A_READY, ready++ & 1))) break;
+                tc::tc_fence_after();
 #pragma unroll
                 for (int s = 0; s < 6; ++s)
                     umma_ts(tmem, tmem + MID + 8 * s, w3 + (s >> 2) * (W3_CHUNK / 16) + 2 * (s & 3), id16, s > 0);
                 tc::umma_commit(bar(D_FULL));
+                ok = wait1(A_READY, ready++ & 1);
+                tc::tc_fence_after();
             }
-            __syncwarp();
-            ok = wait(A_READY, ready++ & 1);
-            tc::tc_fence_after();
+            if (!ok) {   // a bounded wait for the weight copies in flight
+                int none = 0;
+                for (int i = 0; i < 3; ++i) tc::mbar_wait_for(bar(W_FULL + i), 0, &none, 100000000ull);
+                atomicCAS(a.status, 0, 176);
+            }
         }
-        if (start && !ok) {   // a bounded wait for the weight copies in flight
-            int none = 0;
-            for (int i = 0; i < 3; ++i) tc::mbar_wait_for(bar(W_FULL + i), 0, &none, 100000000ull);
-        }
+        __syncwarp();
     }
     if (!ok && start && lane == 0) atomicCAS(a.status, 0, 176);
     tc::tc_fence_before();
