@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         __syncwarp();
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = make_idesc(false, false, BLOCK_M, BLOCK_N);
             int stage = 0;
             uint32_t phase = 0;

@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             // the filter bank, once
             const uint32_t wbar = smem_u32(w_full_bar);
             mbar_arrive_expect_tx(wbar, (uint32_t)(w_tiles * W_TILE_BYTES));
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         __syncwarp();
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = make_idesc(false, false, HB_M, BLOCK_N);
             int stage = 0;
             uint32_t phase = 0;

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             const int per_image = p.chunks_y * p.chunks_x;
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
         __syncwarp();
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             // The x tiles of the taps of a filter row lie one after the other in the stage and
             // their accumulators one after the other in TMEM, so several taps are ONE operand
             // of up to 256 columns: one tcgen05.mma per k step covers them all, which moves

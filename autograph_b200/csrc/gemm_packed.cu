@@ -186,7 +186,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     const uint32_t tmem_acc[2] = {tmem_slot[0], tmem_slot[1]};
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -229,7 +229,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (leader && lane == 0) {
+        if (leader && elect_one()) {
             constexpr uint32_t lbo = PL * ATOM;
             const uint32_t a_plane = A_MN ? ATOM : HALF_BYTES;
             const uint32_t a_step = A_MN ? 16 * 128 : 32, b_step = B_MN ? 16 * 128 : 32;

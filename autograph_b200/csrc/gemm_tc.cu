@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         __syncwarp();
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = make_idesc(A_MN, B_MN, BLOCK_M, BLOCK_N);
             const uint32_t a_lbo = A_MN ? (uint32_t)ATOM_BYTES : p.lbo_k;
             const uint32_t b_lbo = B_MN ? (uint32_t)ATOM_BYTES : p.lbo_k;

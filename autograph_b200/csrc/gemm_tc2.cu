@@ -187,7 +187,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer (both CTAs)
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -237,7 +237,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
         __syncwarp();
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer (leader only)
-        if (leader && lane == 0) {
+        if (leader && elect_one()) {
             const uint32_t a_lbo = A_MN ? (uint32_t)ATOM_BYTES : 0u;
             const uint32_t b_lbo = B_MN ? (uint32_t)ATOM_BYTES : 0u;
             const uint32_t a_kstep = A_MN ? UMMA_K * 128 : UMMA_K * 2;

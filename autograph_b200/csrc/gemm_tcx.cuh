@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
         }
     } else if (warp == MMA_WARP) {
         // ------------------------------------------------------------------ MMA issue
-        if (lane == 0) {
+        if (tc::elect_one()) {
             constexpr bool A_MN = AOp::kWalk == kByK, B_MN = BOp::kWalk == kByK;
             constexpr uint32_t idesc1 = tc::make_idesc(A_MN, B_MN, BM, BN);
             constexpr uint32_t idesc2 = tc::make_idesc(A_MN, B_MN, BM, PL == 3 ? 2 * BN : BN);
