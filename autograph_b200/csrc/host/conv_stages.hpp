@@ -1,4 +1,4 @@
-// A run of Conv2 -> Relu -> MaxPool2 (2 x 2, stride 2) stages of a gradient-recording bf16 pass,
+// A run of Conv2 -> Relu -> MaxPool2 (2 x 2, stride 2) stages of a bf16 pass, gradients recorded or not,
 // kept channels-last from the first convolution's input to the last pool's output.
 //
 // The tensor-core convolution kernels work on channels-last data; run layer by layer, every
@@ -51,9 +51,9 @@ inline bool conv_stages_enabled() {
 }
 
 // Fills `d` when the stage (conv on an input of [bs, ic, ih, iw], Relu, 2 x 2 pool) can be part of
-// a channels-last run.  needs_dx: the gradient at the stage's input is wanted.
+// a channels-last run.  recording: gradients will be wanted; needs_dx: the stage's input's among them.
 inline bool plan_stage(Conv2 &conv, const MaxPool2 &mp, ag_dtype dtype, int64_t bs, int64_t ic,
-                       int64_t ih, int64_t iw, bool needs_dx, StageDesc *d) {
+                       int64_t ih, int64_t iw, bool recording, bool needs_dx, StageDesc *d) {
     if (dtype != AG_BF16 || !::ag::convtc::tc_conv_enabled()) return false;
     if (mp.filter[0] != 2 || mp.filter[1] != 2 || mp.stride[0] != 2 || mp.stride[1] != 2) return false;
     const Tensor &w = conv.weight.value;
@@ -84,7 +84,7 @@ inline bool plan_stage(Conv2 &conv, const MaxPool2 &mp, ag_dtype dtype, int64_t 
     for (int i = 0; i < 2; ++i) { ko.padding[i] = 0; ko.stride[i] = 1; ko.dilation[i] = 1; }
     using namespace ::ag::convtc;
     if (!eligible_forward(bs, d->k_ic, d->k_ih, d->k_iw, d->oc, &ko)) return false;
-    if (!eligible_backward_weight(bs, d->k_ic, d->k_ih, d->k_iw, d->oc, &ko)) return false;
+    if (recording && !eligible_backward_weight(bs, d->k_ic, d->k_ih, d->k_iw, d->oc, &ko)) return false;
     if (needs_dx && !eligible_backward_input(bs, d->k_ic, d->k_ih, d->k_iw, d->oc, &ko)) return false;
     return true;
 }
@@ -95,6 +95,7 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
     ag_device *dev = nullptr;
     int64_t bs = 0;
     bool input_grad = false;
+    bool keep = true;                 // forward's tensors stay for the backward pass
     std::vector<StageDesc> st;
     std::vector<Tensor> act, pre;     // per stage: the kernels' input and the convolution's output
     std::vector<Tensor> dpre;         // per stage: gradient at the convolution's output (maybe framed)
@@ -131,8 +132,19 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
     }
 
     // x: the run's input, NCHW.  Returns the last pool's output, NCHW.
-    Tensor forward(const Tensor &x) {
+    Tensor forward(const Tensor &input) {
         ::ag::DeviceGuard guard(dev);
+        Tensor x = input;
+        cudaPointerAttributes where;
+        if (cudaPointerGetAttributes(&where, input.data()) != cudaSuccess) {
+            cudaGetLastError();
+        } else if (where.type == cudaMemoryTypeHost) {
+            // pinned host images: the patch kernel reads a pixel up to nine times, so they cross PCIe first
+            x = make(input.shape());
+            if (cudaMemcpyAsync(x.data(), input.data(), input.nbytes(), cudaMemcpyHostToDevice,
+                                (cudaStream_t)ag_device_stream(dev)) != cudaSuccess)
+                throw Error(AG_ERR_CUDA, "input copy failed");
+        }
         Tensor pooled;
         for (size_t s = 0; s < st.size(); ++s) {
             const StageDesc &d = st[s];
@@ -158,8 +170,10 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
                 d.conv->has_bias ? cptr(d.conv->bias.value) : nullptr, false, ptr(wk), ptr(p)));
             Tensor y = make({bs, d.ph, d.pw, d.ocp});
             check(::ag::nhwc::relu_pool(dev, cptr(p), bs, d.oh, d.ow, d.ocp, ptr(y)));
-            act.push_back(a);
-            pre.push_back(p);
+            if (keep) {
+                act.push_back(a);
+                pre.push_back(p);
+            }
             pooled = y;
         }
         const StageDesc &l = st.back();

@@ -495,18 +495,11 @@ Variable forward_chain(ag_model *m, Variable v, void *out_ptr = nullptr) {
         Layer *l = m->layers[i].get();
         auto *relu1 = i + 1 < n ? dynamic_cast<Relu *>(m->layers[i + 1].get()) : nullptr;
         if (auto *conv = dynamic_cast<Conv2 *>(l)) {
-            if (!conv->records_gradient(v) && relu1) {
-                auto *mp = i + 2 < n ? dynamic_cast<MaxPool2 *>(m->layers[i + 2].get()) : nullptr;
-                const bool pool_ok = mp && mp->stride[0] == mp->filter[0] &&
-                                     mp->stride[1] == mp->filter[1];
-                v = conv->forward_fused(m->pool, v, true, pool_ok ? mp->filter : nullptr);
-                i += pool_ok ? 2 : 1;
-                continue;
-            }
-            // Recording gradients in bf16 with shapes the tensor-core kernels take: this and the
-            // following Conv2 -> Relu -> MaxPool2 stages run as one channels-last node.
-            if (conv->records_gradient(v) && relu1 && conv_stages_enabled() && v.value.ndim() == 4 &&
-                v.value.is_standard_layout() && v.value.dtype() == AG_BF16) {
+            // bf16 with shapes the tensor-core kernels take: this and the following Conv2 -> Relu ->
+            // MaxPool2 stages run channels-last, as one node when gradients are recorded.
+            const bool recording = conv->records_gradient(v);
+            if (relu1 && conv_stages_enabled() && v.value.ndim() == 4 && v.value.is_standard_layout() &&
+                v.value.dtype() == AG_BF16) {
                 auto run = std::make_shared<StageRun>();
                 int64_t c = v.value.dim(1), h = v.value.dim(2), w = v.value.dim(3);
                 size_t j = i;
@@ -515,9 +508,9 @@ Variable forward_chain(ag_model *m, Variable v, void *out_ptr = nullptr) {
                     auto *rj = dynamic_cast<Relu *>(m->layers[j + 1].get());
                     auto *pj = dynamic_cast<MaxPool2 *>(m->layers[j + 2].get());
                     StageDesc d;
-                    const bool needs_dx = j > i || (bool)v.node;
-                    if (!cj || !rj || !pj || !cj->weight.to_variable().node ||
-                        !plan_stage(*cj, *pj, v.value.dtype(), v.value.dim(0), c, h, w, needs_dx, &d))
+                    const bool needs_dx = recording && (j > i || (bool)v.node);
+                    if (!cj || !rj || !pj || (bool)cj->weight.to_variable().node != recording ||
+                        !plan_stage(*cj, *pj, v.value.dtype(), v.value.dim(0), c, h, w, recording, needs_dx, &d))
                         break;
                     run->st.push_back(d);
                     c = d.oc; h = d.ph; w = d.pw;
@@ -528,10 +521,19 @@ Variable forward_chain(ag_model *m, Variable v, void *out_ptr = nullptr) {
                     run->dev = m->dev;
                     run->bs = v.value.dim(0);
                     run->input_grad = (bool)v.node;
-                    v = conv_stage_run_forward(m->pool, run, v);
+                    run->keep = recording;
+                    v = recording ? conv_stage_run_forward(m->pool, run, v) : Variable{run->forward(v.value), nullptr};
                     i = j - 1;
                     continue;
                 }
+            }
+            if (!recording && relu1) {
+                auto *mp = i + 2 < n ? dynamic_cast<MaxPool2 *>(m->layers[i + 2].get()) : nullptr;
+                const bool pool_ok = mp && mp->stride[0] == mp->filter[0] &&
+                                     mp->stride[1] == mp->filter[1];
+                v = conv->forward_fused(m->pool, v, true, pool_ok ? mp->filter : nullptr);
+                i += pool_ok ? 2 : 1;
+                continue;
             }
             // Recording gradients, Relu and an even 2x2 pool next: one forward call that keeps
             // the convolution's output for the backward edges.
