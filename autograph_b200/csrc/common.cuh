@@ -56,6 +56,9 @@ uint64_t launch_count();
 
 }  // namespace ag
 
+// Tiles whose k slices may be added by the CTA that finishes last.
+constexpr int kTileCounters = 1024;
+
 // ---- device object ---------------------------------------------------------
 // One per (GPU, stream).  Owns a scratch workspace that kernels such as the
 // split-k GEMM use for partial sums, a device status word that bounded device
@@ -73,6 +76,7 @@ struct ag_device {
     void *engine = nullptr;         // third block: k-slice sums and packed operands of the
     size_t engine_bytes = 0;        // tensor-core engines (live next to the other two)
     std::vector<void *> retired;    // outgrown scratch blocks that captured graphs may still use
+    int *tile_counters = nullptr;   // kTileCounters zeros: arrivals at a tile, back to zero after each launch
     int *status_dev = nullptr;      // device word: 0 = ok, else a timeout code
     int *status_host = nullptr;     // pinned mirror
     float *scalar_dev = nullptr;    // small device buffer for loss / accuracy sums (64 B)

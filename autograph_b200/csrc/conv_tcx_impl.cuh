@@ -58,13 +58,25 @@ static int patches_times_filters(ag_device *dev, const T *src, const ConvMap &ma
     return gemm<T>(dev, M, N, K, ConvRows<T>{src, map, M}, strided<kVecK>((const T *)packed, K, 1, N), E);
 }
 
+// Whether a convolution's patches are better indexed by (channel, tap) than by (tap, channel padded to
+// eight): the padding costs more than the table look-ups (6 channels: 8 / 6 of 4 instructions
+// per element against 6).
+static bool few_channels(const ConvMap &g) {
+    return g.cp * 10 > g.channels * 14 && g.channels * g.ff <= kFewPatch && (int64_t)g.channels * g.sh * g.sw < (1 << 26);
+}
+
 template <class T>
 int conv_forward(ag_device *dev, const T *x, int64_t bs, int64_t ic, int64_t ih, int64_t iw,
                  const T *w, int64_t oc, const T *bias, const ag_conv2_options *o, int64_t oh,
                  int64_t ow, bool relu, T *y) {
     const int M = (int)(bs * oh * ow), N = (int)oc, ff = o->filter[0] * o->filter[1];
     NchwOut<T> E{y, bias, N, (int)(oh * ow), FastDiv((uint32_t)(oh * ow)), relu};
-    return patches_times_filters<T>(dev, x, conv_map(ic, ih, iw, oh, ow, o, false), M, w, N, (int)ic * ff, ff, E);
+    const ConvMap map = conv_map(ic, ih, iw, oh, ow, o, false);
+    if (few_channels(map)) {
+        const int patch = (int)ic * ff;
+        return gemm<T>(dev, M, N, patch, FewRows<T>{x, map, M, patch}, strided<kByRow>(w, patch, 1, N), E);
+    }
+    return patches_times_filters<T>(dev, x, map, M, w, N, (int)ic * ff, ff, E);
 }
 
 // dx from the products with every tap: col[c * ff + tap][position of dy] -> dx[b][c][y][x].
@@ -137,7 +149,13 @@ int conv_backward_weight(ag_device *dev, const T *x, int64_t bs, int64_t ic, int
                          const T *dy, int64_t oc, const ag_conv2_options *o, int64_t oh, int64_t ow,
                          float beta, T *dw) {
     const ConvMap map = conv_map(ic, ih, iw, oh, ow, o, false);
-    const int M = map.ff * map.cp, N = (int)oc, K = (int)(bs * oh * ow), hw = (int)(oh * ow);
+    const int N = (int)oc, K = (int)(bs * oh * ow), hw = (int)(oh * ow);
+    if (few_channels(map)) {
+        const int patch = (int)ic * map.ff;
+        return gemm<T>(dev, patch, N, K, FewCols<T>{{x, map, 0, patch}}, ChannelRows<T>{dy, N, hw, FastDiv((uint32_t)hw)},
+                       StridedOut<T>{dw, 1, patch, 1.f, beta});
+    }
+    const int M = map.ff * map.cp;
     return gemm<T>(dev, M, N, K, ConvCols<T>{x, map, M}, ChannelRows<T>{dy, N, hw, FastDiv((uint32_t)hw)},
                    FilterOut<T>{dw, map.channels, map.ff, map.div_cp, map.cp, beta});
 }

@@ -357,6 +357,64 @@ struct ConvCols {
     }
 };
 
+// Few channels: padding them to eight would multiply the patch (1 channel: by eight).  The patch index is
+// the filter bank's own (channel, tap) order instead, so the filters need no repacking; a table holds
+// each index's offset and tap, and an element costs 6 instructions.
+constexpr int kFewPatch = 160;           // longest patch
+template <class T>
+struct FewRows {                         // as ConvRows
+    static constexpr Walk kWalk = kByRow;
+    static constexpr int kTable = kFewPatch;
+    const T *src;
+    ConvMap g;
+    int rows, patch;                     // patch = channels * taps
+    struct State {
+        int base;
+        uint32_t mask;
+    };
+    __device__ __forceinline__ int entry(int k) const {
+        const int c = k / g.ff, tap = k - c * g.ff;
+        return ((c * g.sh * g.sw + g.tap_offset(tap)) << 5) | tap;
+    }
+    __device__ __forceinline__ void init(int *table, int tid, int threads) const {
+        for (int k = tid; k < patch; k += threads) table[k] = entry(k);
+    }
+    __device__ __forceinline__ void begin(State &s, const int *, int row, int end) const {
+        s.base = 0;
+        s.mask = 0;
+        if (row < end) g.position(row, s.base, s.mask);
+    }
+    __device__ __forceinline__ void one(const State &s, const int *table, int k, bool in, decltype(Vec8<T>().v[0]) &d) const {
+        const int e = in ? table[k] : 0;
+        const bool ok = in && ((s.mask >> (e & 31)) & 1u);
+        fetch(d, src + (ok ? s.base + (e >> 5) : 0), ok);
+    }
+    __device__ __forceinline__ void load(const State &s, const int *table, int, int k, int k_end, Vec8<T> &d) const {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) one(s, table, k + j, k + j < k_end, d.v[j]);
+    }
+    __device__ __forceinline__ float at(int row, int k) const {
+        State s;
+        begin(s, nullptr, row, row + 1);
+        const int e = entry(k);
+        return (s.mask >> (e & 31)) & 1u ? to_f32(src[s.base + (e >> 5)]) : 0.f;
+    }
+};
+template <class T>
+struct FewCols {                         // as ConvCols: rows are (channel, tap), k = positions
+    static constexpr Walk kWalk = kByK;
+    static constexpr int kTable = kFewPatch;
+    FewRows<T> f;                        // f.rows is not used
+    using State = typename FewRows<T>::State;
+    __device__ __forceinline__ void init(int *table, int tid, int threads) const { f.init(table, tid, threads); }
+    __device__ __forceinline__ void begin(State &s, const int *table, int k, int end) const { f.begin(s, table, k, end); }
+    __device__ __forceinline__ void load(const State &s, const int *table, int row, int, int, Vec8<T> &d) const {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f.one(s, table, row + j, row + j < f.patch, d.v[j]);
+    }
+    __device__ __forceinline__ float at(int row, int k) const { return f.at(k, row); }
+};
+
 // Rows are channels of an NCHW tensor, k = (image, position).
 template <class T>
 struct ChannelRows {
@@ -490,7 +548,8 @@ struct Cfg {
     static constexpr int STAGES = PL == 3 ? (BN > 64 ? 2 : 3) : 4;
     static constexpr int ACC_COLS = PL == 3 ? 2 * BN : BN;       // f32: leading block + corrections
     static constexpr int TMEM = 2 * ACC_COLS < 64 ? 64 : 2 * ACC_COLS;
-    static constexpr int SMEM = STAGES * STAGE + 1024 + 512;
+    static constexpr int SMEM = STAGES * STAGE + 1024 + 256 + 2 * kFewPatch * (int)sizeof(int);
+    static_assert(SMEM <= 227 * 1024, "shared memory");
     static_assert(TMEM <= 512 && (TMEM & (TMEM - 1)) == 0, "tensor memory columns");
     static_assert(COLS % 16 == 0, "epilogue warps read 16 columns at a time");
 };
@@ -499,6 +558,7 @@ struct Params {
     int M, N, K;
     int tiles_m, tiles_n, splits, k_split;  // k_split: k per slice, a multiple of BK
     float *partial;                         // splits > 1: [splits][N][M] f32 sums
+    int *arrivals;                          // not null: the CTA of a tile that finishes last adds its slices
     int *status;
 };
 
@@ -550,6 +610,37 @@ __device__ __noinline__ float recompute(const AOp &A, const BOp &B, int row, int
     return s;
 }
 
+// One tile's slices added in slice order, as reduce_splits_kernel adds them, and stored: four columns and
+// four slices at a time, because a single SM pulls them out of L2.
+template <int THREADS, class Epi>
+__device__ __forceinline__ void reduce_tile(const Params &p, const Epi &E, int m0, int n0, int bn, int tid) {
+    constexpr int LANES = THREADS / BM;        // threads beyond LANES * BM idle
+    const int row = m0 + tid % BM, n1 = min(p.N, n0 + bn);
+    if (tid >= LANES * BM || row >= p.M) return;
+    const typename Epi::State st = E.begin(row);
+    const int64_t plane = (int64_t)p.M * p.N;
+    for (int col = n0 + tid / BM * 4; col < n1; col += LANES * 4) {
+        const float *q = p.partial + (int64_t)col * p.M + row;
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int z = 0; z < p.splits; z += 4) {
+            float v[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    v[i][j] = z + i < p.splits && col + j < n1 ? __ldcg(q + (z + i) * plane + (int64_t)j * p.M) : 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (z + i < p.splits) s[j] += v[i][j];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (col + j < n1) E.store(st, row, col + j, s[j]);
+    }
+}
+
 template <class T, int BN, class AOp, class BOp, class Epi>
 __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
     gemm_tcx_kernel(const __grid_constant__ AOp A, const __grid_constant__ BOp B,
@@ -564,7 +655,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
     uint64_t *acc_full = bars + 2 * STAGES, *acc_empty = bars + 2 * STAGES + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    int *table_a = reinterpret_cast<int *>(tmem_slot + 2), *table_b = table_a + 32;
+    int *table_a = reinterpret_cast<int *>(tmem_slot + 2), *table_b = table_a + kFewPatch;
 
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     constexpr int MMA_WARP = PRODUCERS / 32 + C::EPI_WARPS;
@@ -816,6 +907,22 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
         }
         tc::tmem_dealloc(tmem, C::TMEM);
     }
+    if (p.arrivals != nullptr) {
+        // every CTA has had one slice of one tile (grid = tiles * splits)
+        const int tile = blockIdx.x % tiles;
+        int *last = table_a;
+        if (tid == 0) {
+            __threadfence();   // the slice's sums, stored by the epilogue warps before the barrier
+            const int n = atomicAdd(p.arrivals + tile, 1);
+            *last = n == p.splits - 1;
+            if (n == p.splits - 1) p.arrivals[tile] = 0;   // for the next launch
+        }
+        __syncthreads();
+        if (*last) {
+            __threadfence();
+            reduce_tile<C::THREADS>(p, E, (tile % p.tiles_m) * BM, (tile / p.tiles_m) * BN, BN, tid);
+        }
+    }
 }
 
 // out = epilogue(sum over slices in slice order).
@@ -860,10 +967,17 @@ int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
     p.splits = (int)ceil_div(steps, per);
     p.status = dev->status_dev;
     p.partial = nullptr;
+    p.arrivals = nullptr;
     if (p.splits > 1) {
         void *ws = nullptr;
         AG_TRY(engine_scratch(dev, sizeof(float) * (size_t)p.splits * p.M * p.N, &ws));
         p.partial = (float *)ws;
+        // Up to eight slices the tile's last CTA adds them (two rounds of loads, at most 256 KB from L2: 2 us):
+        // a separate kernel costs its launch on the host (4 us) and 3 us on the device.  More slices
+        // would be a chain of round trips (3 -> 64 3x3 weight gradient, 37 slices: 24 us against 13).
+        if (p.splits <= 8 && tiles <= kTileCounters &&
+            (int64_t)p.splits * (p.M < BM ? p.M : BM) * (p.N < BN ? p.N : BN) <= 65536)
+            p.arrivals = dev->tile_counters;
     }
     auto kernel = gemm_tcx_kernel<T, BN, AOp, BOp, Epi>;
     static bool configured_on[64] = {};
@@ -876,7 +990,7 @@ int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
     const int grid = (int)(work < dev->sm_count ? work : dev->sm_count);
     kernel<<<grid, C::THREADS, C::SMEM, dev->stream>>>(A, B, E, p);
     AG_CHECK_LAUNCH();
-    if (p.splits > 1) {
+    if (p.splits > 1 && p.arrivals == nullptr) {
         reduce_splits_kernel<Epi><<<(unsigned)ceil_div((int64_t)p.M * p.N, 256), 256, 0, dev->stream>>>(
             p.partial, p.splits, p.M, p.N, FastDiv((uint32_t)p.M), E);
         AG_CHECK_LAUNCH();

@@ -89,6 +89,8 @@ static int device_init(int ordinal, cudaStream_t stream, bool owns, ag_device **
         dev->stream = stream;
     }
     cudaError_t e = cudaMalloc(&dev->status_dev, 64);
+    if (e == cudaSuccess) e = cudaMalloc(&dev->tile_counters, kTileCounters * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemsetAsync(dev->tile_counters, 0, kTileCounters * sizeof(int), dev->stream);
     if (e == cudaSuccess) e = cudaMalloc(&dev->scalar_dev, 64);
     if (e == cudaSuccess) e = cudaMallocHost(&dev->status_host, 64);
     if (e == cudaSuccess) e = cudaMallocHost(&dev->scalar_host, 64);
@@ -163,6 +165,7 @@ int ag_device_destroy(ag_device *dev) {
     if (dev->engine) cudaFree(dev->engine);
     for (void *p : dev->retired) cudaFree(p);
     if (dev->status_dev) cudaFree(dev->status_dev);
+    if (dev->tile_counters) cudaFree(dev->tile_counters);
     if (dev->scalar_dev) cudaFree(dev->scalar_dev);
     if (dev->status_host) cudaFreeHost(dev->status_host);
     if (dev->scalar_host) cudaFreeHost(dev->scalar_host);
@@ -179,6 +182,8 @@ int ag_device_wait(ag_device *dev) {
     if (*dev->status_host != 0) {
         int code = *dev->status_host;
         cudaMemsetAsync(dev->status_dev, 0, sizeof(int), dev->stream);
+        // a kernel that gave up may have left arrivals behind
+        cudaMemsetAsync(dev->tile_counters, 0, kTileCounters * sizeof(int), dev->stream);
         return fail(AG_ERR_DEVICE_TIMEOUT, "a bounded device-side wait gave up (code %d)", code);
     }
     return AG_OK;
