@@ -449,7 +449,9 @@ struct ChannelRows {
 };
 
 // ---------------------------------------------------------------- epilogues
-// Concept: State begin(int row); void store(const State &, int row, int col, float acc).
+// Concept: State begin(int row, int col); void store(State &, int col, float acc), which stores at the
+// state's position and moves it to the next column: with a 64-bit address per element from
+// scratch the stores were a third of the kernel's instructions at 48 k.
 // A warp holds 32 consecutive rows of one column at a time, so the tensor written should be
 // contiguous along the rows.
 
@@ -460,12 +462,14 @@ struct StridedOut {
     int64_t s_row, s_col;
     float alpha, beta;
     struct State { T *q; };
-    __device__ __forceinline__ State begin(int row) const { return State{c + (int64_t)row * s_row}; }
-    __device__ __forceinline__ void store(const State &s, int, int col, float acc) const {
-        T *q = s.q + (int64_t)col * s_col;
+    __device__ __forceinline__ State begin(int row, int col) const {
+        return State{c + (int64_t)row * s_row + (int64_t)col * s_col};
+    }
+    __device__ __forceinline__ void store(State &s, int, float acc) const {
         float v = alpha * acc;
-        if (beta != 0.f) v += beta * to_f32(*q);
-        *q = from_f32<T>(v);
+        if (beta != 0.f) v += beta * to_f32(*s.q);
+        *s.q = from_f32<T>(v);
+        s.q += s_col;
     }
 };
 
@@ -477,14 +481,15 @@ struct DenseOut {
     const T *bias;
     bool relu;
     struct State { T *q; float b; };
-    __device__ __forceinline__ State begin(int row) const {
-        return State{c + row, bias != nullptr ? to_f32(bias[row]) : 0.f};
+    __device__ __forceinline__ State begin(int row, int col) const {
+        return State{c + row + (int64_t)col * s_col, bias != nullptr ? to_f32(bias[row]) : 0.f};
     }
-    __device__ __forceinline__ void store(const State &s, int, int col, float acc) const {
+    __device__ __forceinline__ void store(State &s, int, float acc) const {
         float v = to_f32(from_f32<T>(acc));
         if (bias != nullptr) v = to_f32(from_f32<T>(__fadd_rn(v, s.b)));
         if (relu) v = (v >= 0.f) ? v : 0.f;
-        s.q[(int64_t)col * s_col] = from_f32<T>(v);
+        *s.q = from_f32<T>(v);
+        s.q += s_col;
     }
 };
 
@@ -498,16 +503,17 @@ struct NchwOut {
     FastDiv div_hw;
     bool relu;
     struct State { T *q; };
-    __device__ __forceinline__ State begin(int row) const {
+    __device__ __forceinline__ State begin(int row, int col) const {
         uint32_t b, r;
         div_hw.divmod((uint32_t)row, b, r);
-        return State{y + ((int64_t)b * channels * hw + r)};
+        return State{y + ((int64_t)b * channels + col) * hw + r};
     }
-    __device__ __forceinline__ void store(const State &s, int, int col, float acc) const {
+    __device__ __forceinline__ void store(State &s, int col, float acc) const {
         float v = to_f32(from_f32<T>(acc));
         if (bias != nullptr) v = to_f32(from_f32<T>(v + to_f32(bias[col])));
         if (relu) v = (v >= 0.f) ? v : 0.f;
-        s.q[(int64_t)col * hw] = from_f32<T>(v);
+        *s.q = from_f32<T>(v);
+        s.q += hw;
     }
 };
 
@@ -519,16 +525,15 @@ struct FilterOut {
     FastDiv div_cp;
     int cp;
     float beta;
-    struct State { T *q; };
-    __device__ __forceinline__ State begin(int row) const {
+    struct State { T *q; bool padding; };
+    __device__ __forceinline__ State begin(int row, int col) const {
         uint32_t tap, c;
         div_cp.divmod((uint32_t)row, tap, c);
-        return State{(int)c < channels ? dw + ((int)c * ff + (int)tap) : nullptr};
+        return State{dw + ((int64_t)col * channels + (int)c) * ff + (int)tap, (int)c >= channels};
     }
-    __device__ __forceinline__ void store(const State &s, int, int col, float acc) const {
-        if (s.q == nullptr) return;
-        T *q = s.q + (int64_t)col * channels * ff;
-        *q = from_f32<T>(beta != 0.f ? acc + beta * to_f32(*q) : acc);
+    __device__ __forceinline__ void store(State &s, int, float acc) const {
+        if (!s.padding) *s.q = from_f32<T>(beta != 0.f ? acc + beta * to_f32(*s.q) : acc);
+        s.q += channels * ff;
     }
 };
 
@@ -617,7 +622,6 @@ __device__ __forceinline__ void reduce_tile(const Params &p, const Epi &E, int m
     constexpr int LANES = THREADS / BM;        // threads beyond LANES * BM idle
     const int row = m0 + tid % BM, n1 = min(p.N, n0 + bn);
     if (tid >= LANES * BM || row >= p.M) return;
-    const typename Epi::State st = E.begin(row);
     const int64_t plane = (int64_t)p.M * p.N;
     for (int col = n0 + tid / BM * 4; col < n1; col += LANES * 4) {
         const float *q = p.partial + (int64_t)col * p.M + row;
@@ -635,9 +639,10 @@ __device__ __forceinline__ void reduce_tile(const Params &p, const Epi &E, int m
                 for (int j = 0; j < 4; ++j)
                     if (z + i < p.splits) s[j] += v[i][j];
         }
+        typename Epi::State st = E.begin(row, col);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (col + j < n1) E.store(st, row, col + j, s[j]);
+            if (col + j < n1) E.store(st, col + j, s[j]);
     }
 }
 
@@ -715,15 +720,16 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
             bool ok = true;
             for (int k0 = k_begin; k0 < k_end; k0 += BK) {
                 Vec8<T> va[A_PER], vb[B_PER];
+                const int k_stop = k0 + BK <= k_end ? BK : (k_end - k0 + 15) & ~15;   // what the MMAs will read
                 if (AOp::kWalk == kByK) A.begin(sa, table_a, k0 + la.k(0), k_end);
 #pragma unroll
                 for (int i = 0; i < A_PER; ++i)
-                    if (m0 + la.row(i) < p.M)
+                    if (m0 + la.row(i) < p.M && la.k(i) < k_stop)
                         A.load(sa, table_a, m0 + la.row(i), k0 + la.k(i), k_end, va[i]);
                 if (BOp::kWalk == kByK) B.begin(sb, table_b, k0 + lb.k(0), k_end);
 #pragma unroll
                 for (int i = 0; i < B_PER; ++i)
-                    if (lb.mine && n0 + lb.row(i) < p.N)
+                    if (lb.mine && n0 + lb.row(i) < p.N && lb.k(i) < k_stop)
                         B.load(sb, table_b, n0 + lb.row(i), k0 + lb.k(i), k_end, vb[i]);
                 if (!tc::mbar_wait(tc::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag)) {
                     if (lane == 0) atomicExch(p.status, 181);
@@ -734,10 +740,10 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
                 const uint32_t b_base = a_base + PL * C::A_PLANE;
 #pragma unroll
                 for (int i = 0; i < A_PER; ++i)
-                    if (m0 + la.row(i) < p.M) put8(va[i], a_base + la.offset(i), C::A_PLANE);
+                    if (m0 + la.row(i) < p.M && la.k(i) < k_stop) put8(va[i], a_base + la.offset(i), C::A_PLANE);
 #pragma unroll
                 for (int i = 0; i < B_PER; ++i)
-                    if (lb.mine && n0 + lb.row(i) < p.N) put8(vb[i], b_base + lb.offset(i), C::B_PLANE);
+                    if (lb.mine && n0 + lb.row(i) < p.N && lb.k(i) < k_stop) put8(vb[i], b_base + lb.offset(i), C::B_PLANE);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(tc::smem_u32(&full_bar[stage]));
@@ -785,21 +791,24 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
                     auto db = [&](int plane, int k) {
                         return tc::make_smem_desc(b_base + plane * C::B_PLANE + k * b_step, b_lbo, 1024);
                     };
+                    const int k_steps = k0 + BK <= k_end ? BK / 16 : (k_end - k0 + 15) / 16;   // a short last step
                     if (PL == 1) {
 #pragma unroll
                         for (int k = 0; k < BK / 16; ++k)
-                            tc::umma_bf16(d, da(0, k), db(0, k), idesc1, (k0 > k_begin || k > 0) ? 1u : 0u);
+                            if (k < k_steps) tc::umma_bf16(d, da(0, k), db(0, k), idesc1, (k0 > k_begin || k > 0) ? 1u : 0u);
                     } else {
                         // corrections first: column block 0 collects hi.mid, mid.hi, lo.hi, block 1
                         // hi.lo and mid.mid; then the leading products into block 0
 #pragma unroll
                         for (int k = 0; k < BK / 16; ++k) {
+                            if (k >= k_steps) break;
                             tc::umma_bf16(d, da(0, k), db(1, k), idesc2, k > 0 ? 1u : 0u);   // b_mid, b_lo
                             tc::umma_bf16(d, da(1, k), db(0, k), idesc2, 1u);                // b_hi, b_mid
                             tc::umma_bf16(d, da(2, k), db(0, k), idesc1, 1u);
                         }
 #pragma unroll
-                        for (int k = 0; k < BK / 16; ++k) tc::umma_bf16(d, da(0, k), db(0, k), idesc1, 1u);
+                        for (int k = 0; k < BK / 16; ++k)
+                            if (k < k_steps) tc::umma_bf16(d, da(0, k), db(0, k), idesc1, 1u);
                     }
                     tc::umma_commit(tc::smem_u32(&empty_bar[stage]));
                     if (++stage == STAGES) {
@@ -873,25 +882,25 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
                 for (int j = 0; j < C::COLS; ++j) finite = fmaf(sum[j], 0.f, finite);
             }
             if (in && !(finite == 0.f)) {
-                const typename Epi::State st = E.begin(row);
+                typename Epi::State st = E.begin(row, col0);
 #pragma unroll 1
                 for (int col = col0; col < min(p.N, col0 + C::COLS); ++col) {
                     const float v = recompute(A, B, row, col, k_begin, k_end);
                     if (p.splits > 1)
                         p.partial[((int64_t)z * p.N + col) * p.M + row] = v;
                     else
-                        E.store(st, row, col, v);
+                        E.store(st, col, v);
                 }
             } else if (in && p.splits > 1) {
-                float *q = p.partial + (int64_t)z * p.M * p.N + row;
+                float *q = p.partial + ((int64_t)z * p.N + col0) * p.M + row;
 #pragma unroll
-                for (int j = 0; j < C::COLS; ++j)
-                    if (col0 + j < p.N) q[(int64_t)(col0 + j) * p.M] = sum[j];
+                for (int j = 0; j < C::COLS; ++j, q += p.M)
+                    if (col0 + j < p.N) *q = sum[j];
             } else if (in) {
-                const typename Epi::State st = E.begin(row);
+                typename Epi::State st = E.begin(row, col0);
 #pragma unroll
                 for (int j = 0; j < C::COLS; ++j)
-                    if (col0 + j < p.N) E.store(st, row, col0 + j, sum[j]);
+                    if (col0 + j < p.N) E.store(st, col0 + j, sum[j]);
             }
             __syncwarp();  // the next tensor-memory load is a warp-wide instruction
         }
@@ -945,7 +954,8 @@ __global__ void __launch_bounds__(256)
     }
     for (; z < splits; ++z) s += q[(int64_t)z * plane];
     const int col = (int)(i / M), row = (int)(i - (int64_t)col * M);
-    E.store(E.begin(row), row, col, s);
+    typename Epi::State st = E.begin(row, col);
+    E.store(st, col, s);
 }
 
 // --------------------------------------------------------------------- host
