@@ -20,9 +20,13 @@ static bool enabled() {
 // 100 x 256 x 128 8 and 8, 390 x 145 x 135 9 and 18.  A call here costs about 9 us in f32 (slices of
 // k, two kernels) whatever the size, so the line is drawn at the multiply-adds the SIMT kernels do
 // in that time.
+// Few rows: 1 to 8 x 25088 x 512 18 us and 68 (bf16 13 and 97), 12 x 100 x 20000 9 and 27.  Few columns: 20000 x 200 x
+// 12 25 and 14, 5000 x 2000 x 12 51 and 98.  k below a tile's step: 25088 x 24 x 512 39 and 27.
 bool gemm_worth(ag_dtype dtype, int64_t m, int64_t k, int64_t n) {
-    if (!enabled() || m < 16 || n < 16 || k < 32) return false;
-    return (double)m * (double)n * (double)k >= (dtype == AG_F32 ? 3e7 : 4e6);
+    if (!enabled() || k < 32) return false;
+    const double macs = (double)m * (double)n * (double)k;
+    if (m < 16 || n < 16) return macs >= 1e7 && k >= (n < 16 ? 1024 : 64);
+    return macs >= (dtype == AG_F32 ? 3e7 : 4e6);
 }
 
 // Against the gathered engine: 1000 x 5000 x 130 f32 33 us packed and 48 us gathered, 1024^3 29 and
@@ -32,27 +36,31 @@ bool packed_worth(int64_t m, int64_t k, int64_t n) {
     return m >= 128 && n >= 128 && k >= 64 && (double)m * (double)n * (double)k >= 2.5e8;
 }
 
-// channels x taps and columns of the product, its depth.  Few channels are padded to eight and few
-// columns to 32: 1 -> 16 5x5 forward 42 us here and 16 us on the SIMT engine, 3 -> 16 3x3 20 and 10,
-// 3 -> 64 28 and 28, 16 -> 16 (8 x 12 x 12) 11 and 21.
+// patch = channels x taps.  Against the SIMT engine, us here and there (f32 unless said):
+//   1024 and more: here.  Below, by what the SIMT tiles are good at:
+//   96 columns x 9 (203 x 41 x 41 / 2): 35 and 31, bf16 35 and 52;  32 x 9 (254 x 55 x 55): 124 and 148;
+//   32 x 25 (64 x 24 x 24): 10 and 16;  6 x 144 (8 x 40 x 40): 9.4 and 32, bf16 8.3 and 46;
+//   16 x 27 (233 x 48 x 48): 77 and 59;  6 x 9 (116 x 35 x 35): 20 and 8;
+//   1.8e6 multiply-adds (32 x 27, 21 x 10 x 10): 7 and 4.
 bool conv_worth(ag_dtype dtype, int64_t patch, int64_t cols, int64_t positions, const ag_conv2_options *o) {
-    (void)dtype;
-    return enabled() && o->filter[0] * o->filter[1] <= 32 && patch * cols >= 1024 &&
-           positions * patch * cols >= 2000000;
-}
-
-// The input gradient, whose engine has a form for few columns (1 <- 16 5x5: 177 us on the SIMT engine).
-bool conv_input_worth(int64_t patch, int64_t cols, int64_t positions, const ag_conv2_options *o) {
-    return enabled() && o->filter[0] * o->filter[1] <= 32 && patch * cols >= 140 &&
-           positions * patch * cols >= 2000000;
-}
-
-// The weight gradient: 3 -> 16 3x3 f32 24 us here and 27, 1 -> 16 5x5 52 and 40 (bf16 38 and 60); small
-// ones (2.7e6 multiply-adds) 11 and 10.
-bool conv_weight_worth(ag_dtype dtype, int64_t patch, int64_t oc, int64_t positions, const ag_conv2_options *o) {
     if (!enabled() || o->filter[0] * o->filter[1] > 32) return false;
-    const int64_t macs = positions * patch * oc;
-    return dtype == AG_F32 ? patch * oc >= 420 && macs >= 4000000 : patch * oc >= 128 && macs >= 2000000;
+    const int64_t macs = positions * patch * cols;
+    if (patch * cols >= 1024) return macs >= 2000000;
+    if (macs < 3000000) return false;
+    if (dtype == AG_F32) return cols < 32 ? patch >= 96 : cols <= 64 && patch * cols >= 256;
+    return cols < 32 ? patch >= 64 : patch * cols >= 256;
+}
+
+// The input gradient, whose engine has a form for few columns (SIMT engine: 1 <- 16 5x5 177 us, 3 <- 32 3x3 on
+// 21 x 10 x 10 60 us here 10, 1 <- 6 3x3 on 116 x 37 x 37 51 us here 24).
+bool conv_input_worth(int64_t patch, int64_t cols, int64_t positions, const ag_conv2_options *o) {
+    return enabled() && o->filter[0] * o->filter[1] <= 32 && positions * patch * cols >= 1000000;
+}
+
+// The weight gradient: 1 -> 32 3x3 (254 x 55 x 55) 148 us here and 276, 6 -> 6 3x3 (84 x 60 x 60) 57 and 170; small ones
+// (1.1e6 multiply-adds) 11 and 12.
+bool conv_weight_worth(ag_dtype, int64_t patch, int64_t oc, int64_t positions, const ag_conv2_options *o) {
+    return enabled() && o->filter[0] * o->filter[1] <= 32 && positions * patch * oc >= 1000000;
 }
 
 template int gemm_strided<float>(ag_device *, int, int, int, float, const float *, int64_t, int64_t,
