@@ -285,6 +285,14 @@ static int launch_lenet(ag_device *dev, const T *x, const uint8_t *x8, float alp
     return AG_OK;
 }
 
+int64_t split_batch() {
+    static const int64_t v = [] {
+        const char *e = getenv("AG_CHAIN_SPLIT_BATCH");
+        return e ? (int64_t)atoll(e) : (int64_t)5120;
+    }();
+    return v;
+}
+
 template <class T>
 int forward(ag_device *dev, const T *x, const uint8_t *x8, float alpha, int64_t bs, int64_t ic,
             int64_t ih, int64_t iw, int n_conv, const ag_conv_stage *stages, int n_dense,
@@ -315,11 +323,7 @@ int forward(ag_device *dev, const T *x, const uint8_t *x8, float alpha, int64_t 
     // dense layers run as products over the whole batch (ag_dense_forward: tensor cores for
     // bf16, the SIMT tile engine for f32).  Inside the one-kernel form every CTA streams all
     // dense weights for its 7 images; over the whole batch they are read once per 128-row tile.
-    static const int64_t split_batch = [] {
-        const char *e = getenv("AG_CHAIN_SPLIT_BATCH");
-        return e ? (int64_t)atoll(e) : (int64_t)5120;
-    }();
-    if (!generic_only && split_batch > 0 && bs >= split_batch) {
+    if (!generic_only && split_batch() > 0 && bs >= split_batch()) {
         const ag_dtype dtype = sizeof(T) == 4 ? AG_F32 : AG_BF16;
         int64_t widest = layers[0].inputs;
         for (int i = 0; i < n_dense; ++i) widest = layers[i].outputs > widest ? layers[i].outputs : widest;

@@ -17,6 +17,10 @@ constexpr int kMaxConv = 2;
 bool eligible(int64_t bs, int64_t ic, int64_t ih, int64_t iw, int n_conv,
               const ag_conv_stage *stages, int n_dense, const dense_small::ChainLayer *layers);
 
+// From this batch size on a network of LeNet5's geometry runs its dense layers as products over the whole
+// batch (0: never; AG_CHAIN_SPLIT_BATCH).
+int64_t split_batch();
+
 // Reads x, or (x8 != null) u8 images that are scaled by alpha while they are staged.
 template <class T>
 int forward(ag_device *dev, const T *x, const uint8_t *x8, float alpha, int64_t bs, int64_t ic,

@@ -8,6 +8,7 @@
 
 #include "../comm.cuh"
 #include "../common.cuh"
+#include "../conv_chain.cuh"
 #include "../lenet_train.cuh"
 #include "nn.hpp"
 #include "conv_stages.hpp"
@@ -799,6 +800,18 @@ void run_inference(ag_model *m, GraphEntry *g, bool host, const void *x, void *o
     if (m->whole_network && g->bs > 0 && (!host || m->zero_copy_enabled)) {
         void *x_dev = host ? pinned_device_pointer(x) : const_cast<void *>(x);
         void *out_dev = host ? pinned_device_pointer(out) : out;
+        // Batches whose dense layers run over the whole batch are copied to the device first: the kernels
+        // of that form read the images too irregularly for PCIe (8000 f32 images: 1300 us read in place,
+        // 710 copied; below, 4500 images take 350 either way and smaller batches less in place).
+        Tensor stage;
+        if (host && x_dev && out_dev && m->fused_train && ::ag::conv_chain::split_batch() > 0 &&
+            g->bs >= ::ag::conv_chain::split_batch()) {
+            stage = Tensor::uninit(m->pool, {g->bs, g->c, g->h, g->w}, m->dtype);
+            if (cudaMemcpyAsync(stage.data(), x, stage.nbytes(), cudaMemcpyHostToDevice,
+                                (cudaStream_t)ag_device_stream(m->dev)) != cudaSuccess)
+                throw Error(AG_ERR_CUDA, "input copy failed");
+            x_dev = stage.data();
+        }
         if (x_dev && out_dev) {
             Tensor xt = Tensor::external(m->dev, x_dev, {g->bs, g->c, g->h, g->w}, m->dtype);
             Variable y = forward_chain(m, Variable{xt, nullptr}, out_dev);
