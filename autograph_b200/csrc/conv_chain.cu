@@ -257,6 +257,7 @@ static int launch_lenet(ag_device *dev, const T *x, const uint8_t *x8, float alp
     int64_t group = ceil_div(bs, (int64_t)dev->sm_count);
     lp.group = (int)(group < 1 ? 1 : (group > lenet::kGroup ? lenet::kGroup : group));
     lp.status = dev->status_dev;
+    if (flat_out == nullptr) lp.done = take_signal(dev);
     auto kernel = lenet::lenet_chain_kernel<T>;
     static bool attr_set[64] = {};
     if (dev->ordinal >= 64 || !attr_set[dev->ordinal]) {

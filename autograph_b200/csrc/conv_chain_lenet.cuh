@@ -73,14 +73,8 @@ struct Plan {
     // When set, the kernel stops after the flatten and writes the activations [bs, 256] here
     // (the dense layers then run as separate products over the whole batch).
     void *flat_out;
+    Done done;                        // of the form that runs the dense layers
 };
-
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-        "l"(src), "r"(bytes), "r"(bar)
-        : "memory");
-}
 
 template <class T>
 __device__ __forceinline__ float round_t(float v) {
@@ -287,7 +281,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (bytes) {
             tc::mbar_arrive_expect_tx(bar0, bytes);
             for (int l = 0; l < pl.early; ++l)
-                bulk_g2s(tc::smem_u32(smem + pl.w_smem[l]), pl.chain.s[l].w, (uint32_t)pl.w_bytes[l], bar0);
+                tc::bulk_load(tc::smem_u32(smem + pl.w_smem[l]), pl.chain.s[l].w, (uint32_t)pl.w_bytes[l], bar0);
         }
     }
 
@@ -403,21 +397,18 @@ __global__ void __launch_bounds__(kThreads, 1)
             tc::mbar_arrive_expect_tx(bar1, bytes);
             for (int l = pl.early; l < pl.chain.n_layers; ++l)
                 if (pl.w_smem[l] >= 0)
-                    bulk_g2s(tc::smem_u32(smem + pl.w_smem[l]), pl.chain.s[l].w, (uint32_t)pl.w_bytes[l],
+                    tc::bulk_load(tc::smem_u32(smem + pl.w_smem[l]), pl.chain.s[l].w, (uint32_t)pl.w_bytes[l],
                              bar1);
         }
     }
 
     // ---- dense chain
     if (pl.lenet5) {
-        if (nimg > 4)
-            lenet5_head<T, 8>(pl, smem, b0, nimg, bar0, bar1, &s_abort, y);
-        else if (nimg > 2)
-            lenet5_head<T, 4>(pl, smem, b0, nimg, bar0, bar1, &s_abort, y);
-        else if (nimg == 2)
-            lenet5_head<T, 2>(pl, smem, b0, nimg, bar0, bar1, &s_abort, y);
-        else
-            lenet5_head<T, 1>(pl, smem, b0, nimg, bar0, bar1, &s_abort, y);
+        const bool ok = nimg > 4    ? lenet5_head<T, 8>(pl, smem, b0, nimg, bar0, bar1, &s_abort, y)
+                        : nimg > 2  ? lenet5_head<T, 4>(pl, smem, b0, nimg, bar0, bar1, &s_abort, y)
+                        : nimg == 2 ? lenet5_head<T, 2>(pl, smem, b0, nimg, bar0, bar1, &s_abort, y)
+                                    : lenet5_head<T, 1>(pl, smem, b0, nimg, bar0, bar1, &s_abort, y);
+        if (ok) signal_done(pl.done);
         return;
     }
     float *red = smem + pl.red_off;
@@ -449,6 +440,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         xb = t;
     }
     AG_STAMP(7);
+    signal_done(pl.done);
 }
 
 // Fills the plan for a network of this geometry; returns the dynamic shared memory in bytes,

@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             tc::mbar_arrive_expect_tx(bar_w, bytes);
             for (int l = 0; l < pl.chain.n_layers; ++l)
                 if (pl.w_smem[l] >= 0)
-                    bulk_g2s(tc::smem_u32(smem + pl.w_smem[l]), pl.chain.s[l].w, (uint32_t)pl.w_bytes[l], bar_w);
+                    tc::bulk_load(tc::smem_u32(smem + pl.w_smem[l]), pl.chain.s[l].w, (uint32_t)pl.w_bytes[l], bar_w);
         }
     }
     if (warp == 0) {   // tensor memory for the eight accumulators

@@ -792,7 +792,8 @@ bool run_zero_copy(ag_model *m, GraphEntry *g, const void *x, void *out) {
 // One inference pass x -> out.  `host` selects host pointers (x and out in host
 // memory: H2D, chain, D2H) or device pointers (D2D, chain, D2D).  The first call for
 // a shape runs eagerly; the second captures the pass; later calls replay it.
-void run_inference(ag_model *m, GraphEntry *g, bool host, const void *x, void *out) {
+// armed (the caller will wait): set when wait_signal has a word to poll.
+void run_inference(ag_model *m, GraphEntry *g, bool host, const void *x, void *out, bool *armed = nullptr) {
     g->last_use = ++m->tick;
     // A network that runs as one kernel needs neither staging copies nor a graph: the
     // kernel reads the caller's images and writes the caller's logits (device memory, or
@@ -814,6 +815,7 @@ void run_inference(ag_model *m, GraphEntry *g, bool host, const void *x, void *o
         }
         if (x_dev && out_dev) {
             Tensor xt = Tensor::external(m->dev, x_dev, {g->bs, g->c, g->h, g->w}, m->dtype);
+            if (armed && m->fused_train) *armed = ::ag::arm_signal(m->dev);
             Variable y = forward_chain(m, Variable{xt, nullptr}, out_dev);
             if (y.value.data() != out_dev) {
                 // not a one-kernel network after all (remembered): hand this result over
@@ -1149,9 +1151,9 @@ bool train_step_graph(ag_model *m, const void *x_host, const uint8_t *t_host, in
 // u8 host images -> logits on the host (blocking); see ag_model_infer_u8.
 void infer_u8(ag_model *m, const uint8_t *x_host, int64_t bs, int64_t c, int64_t h, int64_t w,
               float alpha, void *logits_host) {
-    cudaStream_t stream = (cudaStream_t)ag_device_stream(m->dev);
+    bool armed = false;
     auto sync = [&]() {
-        cudaError_t e = cudaStreamSynchronize(stream);
+        cudaError_t e = ::ag::wait_signal(m->dev, armed);
         if (e != cudaSuccess)
             throw Error(AG_ERR_CUDA, std::string("cudaStreamSynchronize failed: ") + cudaGetErrorString(e));
     };
@@ -1163,6 +1165,7 @@ void infer_u8(ag_model *m, const uint8_t *x_host, int64_t bs, int64_t c, int64_t
     if (m->whole_network && m->zero_copy_enabled && x_dev && out_dev) {
         U8Images u8{(const uint8_t *)x_dev, alpha};
         Tensor shape_only = Tensor::external(m->dev, x_dev, {bs, c, h, w}, m->dtype);
+        armed = m->fused_train && ::ag::arm_signal(m->dev);
         Variable y;
         if (forward_whole_network(m, Variable{shape_only, nullptr}, &y, out_dev, &u8)) {
             sync();
@@ -1309,8 +1312,9 @@ int ag_model_infer(ag_model *model, const void *x_host, int64_t bs, int64_t c, i
         if (bs < 0 || c <= 0 || h <= 0 || w <= 0) throw Error(AG_ERR_SHAPE, "bad input shape");
         if (!x_host && bs > 0) throw Error(AG_ERR_INVALID, "input pointer is null");
         GraphEntry *g = find_graph(model, bs, c, h, w);
-        run_inference(model, g, true, x_host, logits_host);
-        cudaError_t e = cudaStreamSynchronize((cudaStream_t)ag_device_stream(model->dev));
+        bool armed = false;
+        run_inference(model, g, true, x_host, logits_host, &armed);
+        cudaError_t e = ::ag::wait_signal(model->dev, armed);
         if (e != cudaSuccess)
             throw Error(AG_ERR_CUDA, std::string("cudaStreamSynchronize failed: ") + cudaGetErrorString(e));
     })

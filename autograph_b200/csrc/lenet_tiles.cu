@@ -510,9 +510,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
                 tc::mbar_arrive_expect_tx(bar(W_FULL + i), (uint32_t)bytes[i]);
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                             ::"r"(base + off[i]), "l"(a.blob + off[i]), "r"((uint32_t)bytes[i]), "r"(bar(W_FULL + i))
-                             : "memory");
+                tc::bulk_load(base + off[i], a.blob + off[i], (uint32_t)bytes[i], bar(W_FULL + i));
             }
             constexpr uint32_t id48 = tc::make_idesc(false, false, 128, 48), id32 = tc::make_idesc(false, false, 128, 32);
             constexpr uint32_t id128 = tc::make_idesc(false, false, 128, D1), id96 = tc::make_idesc(false, false, 128, D2P);

@@ -167,9 +167,7 @@ __global__ void __launch_bounds__(kThreads, 1) lenet_train_kernel(const Args a) 
         const void *src[3] = {a.d1, a.d2, a.d3};
         const uint32_t dst[3] = {tc::smem_u32(dw1), tc::smem_u32(dw2), tc::smem_u32(dw3)}, n[3] = {n1, n2, n3};
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"(dst[i]), "l"(src[i]), "r"(n[i]), "r"(bar) : "memory");
+        for (int i = 0; i < 3; ++i) tc::bulk_load(dst[i], src[i], n[i], bar);
     }
     // a thread's piece of the group's images (G * 196 pieces of four pixels)
     auto fetch = [&](int grp, float4 (&v)[(G * 196 + kThreads - 1) / kThreads]) {
@@ -706,7 +704,7 @@ constexpr int kChunk = 64, kPitch = 36;
 // Blocks [0, 47 * splits): a 32 x 32 tile of a dense weight gradient over a part of the batch;
 // then 80 blocks for the convolution gradients and one for the loss.
 template <class T>
-__global__ void __launch_bounds__(256) lenet_finish_kernel(const Finish f) {
+__global__ void __launch_bounds__(256) lenet_finish_kernel(const __grid_constant__ Finish f) {
     __shared__ __align__(16) float As[2][kChunk][kPitch], Bs[2][kChunk][kPitch];
     const int tid = threadIdx.x;
     int blk = blockIdx.x;
@@ -822,7 +820,7 @@ __global__ void __launch_bounds__(256) lenet_finish_kernel(const Finish f) {
 
 // The parts of the dense gradients, added in order.
 template <class T>
-__global__ void __launch_bounds__(256) lenet_reduce_kernel(const Finish f) {
+__global__ void __launch_bounds__(256) lenet_reduce_kernel(const __grid_constant__ Finish f) {
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= kDense - (f.off[5] < 0 ? D3 : 0)) return;
     float s = 0.f;

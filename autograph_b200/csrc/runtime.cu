@@ -2,6 +2,9 @@
 #include <atomic>
 #include <cstring>
 
+#include <atomic>
+#include <chrono>
+
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
@@ -56,6 +59,22 @@ int staging(ag_device *dev, size_t bytes, void **out) {
     return AG_OK;
 }
 
+cudaError_t wait_signal(ag_device *dev, bool armed) {
+    const bool taken = armed && dev->signal == 0;
+    dev->signal = 0;
+    if (taken) {
+        const auto t0 = std::chrono::steady_clock::now();
+        for (uint32_t i = 1;; ++i) {
+            if (*dev->done_host == dev->done_seq) {
+                std::atomic_thread_fence(std::memory_order_acquire);
+                return cudaSuccess;
+            }
+            if ((i & 1023u) == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(20)) break;
+        }
+    }
+    return cudaStreamSynchronize(dev->stream);
+}
+
 int engine_scratch(ag_device *dev, size_t bytes, void **out) {
     if (bytes > dev->engine_bytes)
         AG_TRY(grow_block(dev, &dev->engine, &dev->engine_bytes, bytes, size_t(8) << 20));
@@ -94,6 +113,13 @@ static int device_init(int ordinal, cudaStream_t stream, bool owns, ag_device **
     if (e == cudaSuccess) e = cudaMalloc(&dev->scalar_dev, 64);
     if (e == cudaSuccess) e = cudaMallocHost(&dev->status_host, 64);
     if (e == cudaSuccess) e = cudaMallocHost(&dev->scalar_host, 64);
+    void *done = nullptr;
+    if (e == cudaSuccess) e = cudaHostAlloc(&done, 64, cudaHostAllocMapped);
+    if (e == cudaSuccess) {
+        dev->done_host = (volatile uint32_t *)done;
+        *dev->done_host = 0;
+        e = cudaHostGetDevicePointer((void **)&dev->done_dev, done, 0);
+    }
     if (e == cudaSuccess) e = cudaMemsetAsync(dev->status_dev, 0, 64, dev->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(dev->scalar_dev, 0, 64, dev->stream);
     if (e != cudaSuccess) {
@@ -169,6 +195,7 @@ int ag_device_destroy(ag_device *dev) {
     if (dev->scalar_dev) cudaFree(dev->scalar_dev);
     if (dev->status_host) cudaFreeHost(dev->status_host);
     if (dev->scalar_host) cudaFreeHost(dev->scalar_host);
+    if (dev->done_host) cudaFreeHost((void *)dev->done_host);
     if (dev->owns_stream && dev->stream) cudaStreamDestroy(dev->stream);
     delete dev;
     return AG_OK;
