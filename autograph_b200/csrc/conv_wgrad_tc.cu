@@ -240,7 +240,14 @@ __global__ void wgrad_reduce_kernel(const float *__restrict__ partial, int split
     const float *src = partial + ((int64_t)oc * taps + tap) * Cp + ci;
     float s = 0.f;
     if (live)
-        for (int z = threadIdx.y; z < splits; z += 8) s += src[(int64_t)z * plane];
+        for (int z = threadIdx.y; z < splits; z += 48) {   // six loads in flight (one at a time: 7.3 us for 148 planes)
+            float v[6];
+#pragma unroll
+            for (int j = 0; j < 6; ++j) v[j] = z + 8 * j < splits ? src[(int64_t)(z + 8 * j) * plane] : 0.f;
+#pragma unroll
+            for (int j = 0; j < 6; ++j)
+                if (z + 8 * j < splits) s += v[j];
+        }
     part[threadIdx.y][threadIdx.x] = s;
     __syncthreads();
     if (threadIdx.y != 0 || !live) return;

@@ -98,6 +98,7 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
     bool keep = true;                 // forward's tensors stay for the backward pass
     std::vector<StageDesc> st;
     std::vector<Tensor> act, pre;     // per stage: the kernels' input and the convolution's output
+    std::vector<Tensor> code;         // per stage: where each pool window's gradient goes
     std::vector<Tensor> dpre;         // per stage: gradient at the convolution's output (maybe framed)
     std::vector<char> have, framed;
 
@@ -169,8 +170,11 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
                 dev, c, cptr(a), ::ag::convtc::nhwc_wants_frame(c), cptr(wv), d.oc, d.k_ic,
                 d.conv->has_bias ? cptr(d.conv->bias.value) : nullptr, false, ptr(wk), ptr(p)));
             Tensor y = make({bs, d.ph, d.pw, d.ocp});
-            check(::ag::nhwc::relu_pool(dev, cptr(p), bs, d.oh, d.ow, d.ocp, ptr(y)));
+            Tensor codes = keep ? Tensor::uninit(*pool, {bs, d.ph, d.pw, d.ocp / 2}, AG_U8) : Tensor{};
+            check(::ag::nhwc::relu_pool(dev, cptr(p), bs, d.oh, d.ow, d.ocp, ptr(y),
+                                        keep ? (uint32_t *)codes.data() : nullptr));
             if (keep) {
+                code.push_back(codes);
                 act.push_back(a);
                 pre.push_back(p);
             }
@@ -233,7 +237,7 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
             dpre[s] = make({bs, d.oh, d.ow, d.ocp});
         }
         const View v = interior(s);
-        check(::ag::nhwc::relu_pool_backward(dev, cptr(pre[s]), cptr(dpool), bs, d.oh, d.ow, d.ocp, v.p,
+        check(::ag::nhwc::relu_pool_backward(dev, cptr(pre[s]), (const uint32_t *)code[s].data(), cptr(dpool), bs, d.oh, d.ow, d.ocp, v.p,
                                             v.row_pitch, v.image_pitch));
         have[s] = 1;
     }

@@ -62,8 +62,72 @@ __global__ void im2col_channels_kernel(const __nv_bfloat16 *__restrict__ x, __nv
     }
 }
 
+// The same for the channel pitch of a 64-channel tensor, with the rows a CTA reads staged in shared memory
+// and nothing divided per store: the kernel above spends 43 us on 256 x 3 x 64 x 64, 19 us of it stores, in
+// index arithmetic and two-byte loads that touch 30 cache lines a warp.
+template <int FH, int FW>
+__global__ void __launch_bounds__(256)
+    im2col_rows_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ out, int ic, int ih, int iw, int oh,
+                       int ow, int rows) {
+    extern __shared__ __align__(16) unsigned short staged[];   // [ic][rows + FH - 1][iw]
+    constexpr int taps = FH * FW, groups = 8;
+    const int64_t b = blockIdx.y;
+    const int y0 = blockIdx.x * rows, ny = min(rows, oh - y0), have = ny + FH - 1, run = have * iw;
+    const unsigned short *img = reinterpret_cast<const unsigned short *>(x) + (b * ic * ih + y0) * iw;
+    if (iw % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+        for (int i = threadIdx.x; i < ic * (run / 8); i += 256) {
+            const int c = i / (run / 8), r = i - c * (run / 8);
+            reinterpret_cast<uint4 *>(staged)[i] = __ldg(reinterpret_cast<const uint4 *>(img + (int64_t)c * ih * iw) + r);
+        }
+    } else {
+        for (int c = 0; c < ic; ++c)
+            for (int i = threadIdx.x; i < run; i += 256) staged[c * run + i] = __ldg(img + (int64_t)c * ih * iw + i);
+    }
+    // a thread keeps its channel group: eight offsets, and the words that hold channels at all
+    const int g = threadIdx.x % groups, k = ic * taps;
+    int off[8];
+    uint32_t keep[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int c = g * 8 + e, ci = c / taps, r = c - ci * taps;
+        off[e] = c < k ? ci * run + r / FW * iw + r % FW : 0;
+        if (c < k) keep[e >> 1] |= 0xffffu << ((e & 1) * 16);
+    }
+    __syncthreads();
+    uint4 *q = reinterpret_cast<uint4 *>(out) + (b * oh + y0) * (int64_t)ow * groups + threadIdx.x;
+    int ry = threadIdx.x / groups / ow, ox = threadIdx.x / groups - ry * ow;
+    while (ry < ny) {
+        uint4 o = make_uint4(0u, 0u, 0u, 0u);
+        if (g * 8 < k) {
+            const unsigned short *px = staged + ry * iw + ox;
+            uint32_t v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = px[off[e]];
+            o = make_uint4(__byte_perm(v[0], v[1], 0x5410) & keep[0], __byte_perm(v[2], v[3], 0x5410) & keep[1],
+                           __byte_perm(v[4], v[5], 0x5410) & keep[2], __byte_perm(v[6], v[7], 0x5410) & keep[3]);
+        }
+        *q = o;
+        q += 256;
+        for (ox += 256 / groups; ox >= ow; ox -= ow) ++ry;
+    }
+}
+
+template <int FH, int FW>
+bool launch_im2col_rows(ag_device *dev, const __nv_bfloat16 *x, __nv_bfloat16 *out, int64_t bs, int64_t ic, int64_t ih,
+                        int64_t iw, int64_t oh, int64_t ow, int64_t cp) {
+    if (cp != 64) return false;
+    for (int rows = 16; rows >= 1; rows /= 2) {   // what fits in shared memory without opting in to more
+        const int64_t bytes = ic * (rows + FH - 1) * iw * 2;
+        if (bytes > 40 * 1024) continue;
+        im2col_rows_kernel<FH, FW><<<dim3((unsigned)ceil_div(oh, rows), (unsigned)bs), 256, (size_t)bytes, dev->stream>>>(
+            x, out, (int)ic, (int)ih, (int)iw, (int)oh, (int)ow, rows);
+        return true;
+    }
+    return false;
+}
+
 __global__ void relu_pool_kernel(const __nv_bfloat16 *__restrict__ pre, __nv_bfloat16 *__restrict__ y,
-                                 int ih, int iw, int ph, int pw, int cp, int64_t total) {
+                                 uint32_t *__restrict__ codes, int ih, int iw, int ph, int pw, int cp, int64_t total) {
     const int groups = cp / 8;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -74,34 +138,38 @@ __global__ void relu_pool_kernel(const __nv_bfloat16 *__restrict__ pre, __nv_bfl
         const int py = (int)(t % ph);
         const int64_t b = t / ph;
         const __nv_bfloat16 *p = pre + ((b * ih + 2 * py) * (int64_t)iw + 2 * px) * cp + g * 8;
-        Vec8 a0, a1, b0, b1, o;
-        a0.raw = *reinterpret_cast<const uint4 *>(p);
-        a1.raw = *reinterpret_cast<const uint4 *>(p + cp);
-        b0.raw = *reinterpret_cast<const uint4 *>(p + (int64_t)iw * cp);
-        b1.raw = *reinterpret_cast<const uint4 *>(p + (int64_t)iw * cp + cp);
+        const uint4 raw[4] = {*reinterpret_cast<const uint4 *>(p), *reinterpret_cast<const uint4 *>(p + cp),
+                              *reinterpret_cast<const uint4 *>(p + (int64_t)iw * cp),
+                              *reinterpret_cast<const uint4 *>(p + (int64_t)iw * cp + cp)};   // (0,0), (0,1), (1,0), (1,1)
+        // two channels per instruction: one at a time the arithmetic takes longer than the memory
+        uint32_t code = 0, o[4];
+        const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            float m[2];
+            __nv_bfloat162 v[4];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int e = 2 * j + h;
-                float v0 = a0.get(e), v1 = a1.get(e), v2 = b0.get(e), v3 = b1.get(e);
-                v0 = v0 >= 0.f ? v0 : 0.f; v1 = v1 >= 0.f ? v1 : 0.f;
-                v2 = v2 >= 0.f ? v2 : 0.f; v3 = v3 >= 0.f ? v3 : 0.f;
-                float mm = v0;   // window order (0,0),(0,1),(1,0),(1,1)
-                if (v1 > mm) mm = v1;
-                if (v2 > mm) mm = v2;
-                if (v3 > mm) mm = v3;
-                m[h] = mm;
+            for (int c = 0; c < 4; ++c) {
+                const uint32_t w = (&raw[c].x)[j];
+                v[c] = __hmax2(*reinterpret_cast<const __nv_bfloat162 *>(&w), zero);   // Relu; a NaN gives 0
             }
-            o.set_pair(j, m[0], m[1]);
+            const __nv_bfloat162 m = __hmax2(__hmax2(v[0], v[1]), __hmax2(v[2], v[3]));
+            o[j] = *reinterpret_cast<const uint32_t *>(&m);
+            // the first cell that holds the maximum, and whether the Relu passes its gradient: it does
+            // for a positive maximum; a zero one is cell 0's, whose sign decides
+            const uint32_t e0 = __heq2_mask(v[0], m), e1 = __heq2_mask(v[1], m), e2 = __heq2_mask(v[2], m);
+            const uint32_t first = (&raw[0].x)[j];
+            const uint32_t pass = __hgt2_mask(m, zero) | __hge2_mask(*reinterpret_cast<const __nv_bfloat162 *>(&first), zero);
+            const uint32_t bit1 = ~e0 & ~e1, bit0 = ~e0 & (e1 | ~e2);
+            const uint32_t w = (bit0 & 0x00010001u) | (bit1 & 0x00020002u) | (pass & 0x00040004u);
+            code |= ((w | (w >> 12)) & 0xffu) << (8 * j);
         }
-        reinterpret_cast<uint4 *>(y)[i] = o.raw;
+        if (codes != nullptr) codes[i] = code;
+        reinterpret_cast<uint4 *>(y)[i] = make_uint4(o[0], o[1], o[2], o[3]);
     }
 }
 
 // One thread per (image, window position of the grid that covers every cell, channel group).
-__global__ void relu_pool_backward_kernel(const __nv_bfloat16 *__restrict__ pre,
+__global__ void relu_pool_backward_kernel(const __nv_bfloat16 *__restrict__ pre, const uint32_t *__restrict__ codes,
                                           const __nv_bfloat16 *__restrict__ dy, __nv_bfloat16 *__restrict__ out,
                                           int ih, int iw, int ph, int pw, int cp, int64_t row_pitch,
                                           int64_t image_pitch, int64_t total) {
@@ -119,50 +187,40 @@ __global__ void relu_pool_backward_kernel(const __nv_bfloat16 *__restrict__ pre,
         const bool has_r1 = y0 + 1 < ih, has_c1 = x0 + 1 < iw;
         const __nv_bfloat16 *p = pre + ((b * ih + y0) * (int64_t)iw + x0) * cp + g * 8;
         __nv_bfloat16 *q = out + b * image_pitch + y0 * row_pitch + (int64_t)x0 * cp + g * 8;
+        if (wy < ph && wx < pw) {   // a whole window
+            const int64_t at = ((b * ph + wy) * (int64_t)pw + wx) * groups + g;
+            const uint32_t code = __ldg(codes + at);
+            const uint4 gr = __ldg(reinterpret_cast<const uint4 *>(dy) + at);
+            const uint32_t gw[4] = {gr.x, gr.y, gr.z, gr.w};
+            uint32_t w[4][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                // 0 + dy: the gradient's bits but for a negative zero
+                const uint32_t lo = (gw[j] & 0xffffu) == 0x8000u ? 0u : gw[j] & 0xffffu;
+                const uint32_t hi = (gw[j] >> 16) == 0x8000u ? 0u : gw[j] & 0xffff0000u;
+                const uint32_t cl = (code >> (8 * j)) & 15u, ch = (code >> (8 * j + 4)) & 15u;
+#pragma unroll
+                for (uint32_t c = 0; c < 4; ++c) w[c][j] = (cl == (c | 4u) ? lo : 0u) | (ch == (c | 4u) ? hi : 0u);
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                *reinterpret_cast<uint4 *>(q + (c >> 1) * row_pitch + (c & 1) * cp) = make_uint4(w[c][0], w[c][1], w[c][2], w[c][3]);
+            continue;
+        }
+        // cells no window covers keep the Relu's output
         Vec8 v[4], o[4];
         const uint4 zero = make_uint4(0, 0, 0, 0);
         v[0].raw = *reinterpret_cast<const uint4 *>(p);
         v[1].raw = has_c1 ? *reinterpret_cast<const uint4 *>(p + cp) : zero;
         v[2].raw = has_r1 ? *reinterpret_cast<const uint4 *>(p + (int64_t)iw * cp) : zero;
         v[3].raw = (has_r1 && has_c1) ? *reinterpret_cast<const uint4 *>(p + (int64_t)iw * cp + cp) : zero;
-        if (wy < ph && wx < pw) {   // a whole window
-            Vec8 gr;
-            gr.raw = *reinterpret_cast<const uint4 *>(dy + ((b * ph + wy) * (int64_t)pw + wx) * cp + g * 8);
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                float r[4][2];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int e = 2 * j + h;
-                    float a[4];
-                    bool pass[4];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const float x = v[c].get(e);
-                        pass[c] = x >= 0.f;          // Relu's gate
-                        a[c] = pass[c] ? x : 0.f;    // Relu's output, which the pool saw
-                    }
-                    float m = a[0];
-                    int am = 0;
-                    if (a[1] > m) { m = a[1]; am = 1; }
-                    if (a[2] > m) { m = a[2]; am = 2; }
-                    if (a[3] > m) { m = a[3]; am = 3; }
-                    const float gv = __fadd_rn(0.f, gr.get(e));
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) r[c][h] = (am == c && pass[c]) ? gv : 0.f;
-                }
-#pragma unroll
-                for (int c = 0; c < 4; ++c) o[c].set_pair(j, r[c][0], r[c][1]);
+                const float x0v = v[c].get(2 * j), x1v = v[c].get(2 * j + 1);
+                o[c].set_pair(j, x0v >= 0.f ? x0v : 0.f, x1v >= 0.f ? x1v : 0.f);
             }
-        } else {                    // cells no window covers keep the Relu's output
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float x0v = v[c].get(2 * j), x1v = v[c].get(2 * j + 1);
-                    o[c].set_pair(j, x0v >= 0.f ? x0v : 0.f, x1v >= 0.f ? x1v : 0.f);
-                }
-        }
         *reinterpret_cast<uint4 *>(q) = o[0].raw;
         if (has_c1) *reinterpret_cast<uint4 *>(q + cp) = o[1].raw;
         if (has_r1) *reinterpret_cast<uint4 *>(q + row_pitch) = o[2].raw;
@@ -221,6 +279,11 @@ int im2col_channels(ag_device *dev, const __nv_bfloat16 *x, int64_t bs, int64_t 
                "im2col_channels: image too large");
     AG_REQUIRE(256 % (cp / 8) == 0, AG_ERR_UNSUPPORTED, "im2col_channels: channel pitch must be 64, 128 or 256");
     if (bs == 0) return AG_OK;
+    if ((fh == 3 && fw == 3 && launch_im2col_rows<3, 3>(dev, x, out, bs, ic, ih, iw, oh, ow, cp)) ||
+        (fh == 5 && fw == 5 && launch_im2col_rows<5, 5>(dev, x, out, bs, ic, ih, iw, oh, ow, cp))) {
+        AG_CHECK_LAUNCH();
+        return AG_OK;
+    }
     // eight pixels per thread, so that the offsets a thread computes up front are used eight times
     const int64_t want = ceil_div(per_image, 256 * 8);
     const dim3 grid((unsigned)(want > 4096 ? 4096 : want), (unsigned)bs);
@@ -238,20 +301,20 @@ int im2col_channels(ag_device *dev, const __nv_bfloat16 *x, int64_t bs, int64_t 
 }
 
 int relu_pool(ag_device *dev, const __nv_bfloat16 *pre, int64_t bs, int64_t ih, int64_t iw, int64_t cp,
-              __nv_bfloat16 *y) {
+              __nv_bfloat16 *y, uint32_t *codes) {
     AG_REQUIRE(cp % 8 == 0 && aligned16(pre) && aligned16(y), AG_ERR_INVALID,
                "relu_pool: bad channel pitch or alignment");
     AG_REQUIRE(ih >= 2 && iw >= 2, AG_ERR_SHAPE, "relu_pool: window larger than input");
     const int64_t ph = ih / 2, pw = iw / 2;
     const int64_t total = bs * ph * pw * (cp / 8);
     if (total == 0) return AG_OK;
-    relu_pool_kernel<<<grid_for(dev, total), 256, 0, dev->stream>>>(pre, y, (int)ih, (int)iw, (int)ph,
+    relu_pool_kernel<<<grid_for(dev, total), 256, 0, dev->stream>>>(pre, y, codes, (int)ih, (int)iw, (int)ph,
                                                                    (int)pw, (int)cp, total);
     AG_CHECK_LAUNCH();
     return AG_OK;
 }
 
-int relu_pool_backward(ag_device *dev, const __nv_bfloat16 *pre, const __nv_bfloat16 *dy, int64_t bs,
+int relu_pool_backward(ag_device *dev, const __nv_bfloat16 *pre, const uint32_t *codes, const __nv_bfloat16 *dy, int64_t bs,
                        int64_t ih, int64_t iw, int64_t cp, __nv_bfloat16 *out, int64_t out_row_pitch,
                        int64_t out_image_pitch) {
     AG_REQUIRE(cp % 8 == 0 && out_row_pitch % 8 == 0 && out_image_pitch % 8 == 0 && aligned16(pre) &&
@@ -261,7 +324,7 @@ int relu_pool_backward(ag_device *dev, const __nv_bfloat16 *pre, const __nv_bflo
     const int64_t total = bs * ((ih + 1) / 2) * ((iw + 1) / 2) * (cp / 8);
     if (total == 0) return AG_OK;
     relu_pool_backward_kernel<<<grid_for(dev, total), 256, 0, dev->stream>>>(
-        pre, dy, out, (int)ih, (int)iw, (int)(ih / 2), (int)(iw / 2), (int)cp, out_row_pitch,
+        pre, codes, dy, out, (int)ih, (int)iw, (int)(ih / 2), (int)(iw / 2), (int)cp, out_row_pitch,
         out_image_pitch, total);
     AG_CHECK_LAUNCH();
     return AG_OK;
