@@ -19,7 +19,7 @@
 //   columns [480, 512) pooled row 0 of conv2's output; rows 1 to 3 wait in registers until conv2 has read
 //                      the last of conv1's rows, and take their place
 // Warps 0-3 load pixels (two row pairs ahead), 4-19 (four sets, one per small buffer) turn accumulators into
-// the next operand, warp 20 issues.  Reading accumulators is a chain of latencies (wait, load, maximum, pack,
+// the next operand, 20 and 21 issue.  Reading accumulators is a chain of latencies (wait, load, maximum, pack,
 // store), so warps count: with two sets a tile took 33 us.  The issuing thread is chosen by elect.sync and
 // what varies between its operands is made warp-uniform first: behind a lane test, or with operands from
 // ordinary registers, a tcgen05.mma takes 46-93 cycles to issue (measured), here about 10; the products
@@ -41,7 +41,7 @@ namespace lenet_tiles {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int kImages = 128, kSets = 4, kIssuer = 4 + 4 * kSets, kThreads = 32 * (kIssuer + 1);
+constexpr int kImages = 128, kSets = 4, kIssuer = 4 + 4 * kSets, kThreads = 32 * (kIssuer + 2);
 constexpr int kPix = 784, kPairs = 14, kRows = 12;     // row pairs of an image, pooled rows after conv1
 constexpr int D1 = 128, D2 = 84, D3 = 10, D2P = 96, D3P = 16;
 
@@ -66,7 +66,7 @@ __host__ __device__ constexpr uint32_t late_columns(int i) { return MID + 48 * (
 constexpr uint32_t HIDDEN = MID + 48 * 4;
 
 enum Bar { W_FULL = 0, IN_FULL = 3, IN_EMPTY = 7, ACC_FULL = 11, ACC_EMPTY = 15, MID_FULL = 19, D_FULL = 25, A_READY = 26,
-           kBars = 27 };
+           ROW_DONE = 27, TILE_DONE = 28, kBars = 29 };
 
 struct Args {
     const bf16 *x;
@@ -270,7 +270,8 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
         for (int i = 0; i < kBars; ++i) {
             const bool warps4 = (i >= IN_FULL && i < IN_EMPTY) || (i >= ACC_EMPTY && i < MID_FULL);
             const bool readers = (i >= MID_FULL && i < D_FULL) || i == A_READY;
-            tc::mbar_init(bar(i), warps4 ? 4 : readers ? 4 * kSets : 1);
+            const bool issuers = (i >= IN_EMPTY && i < ACC_FULL) || i == ROW_DONE;
+            tc::mbar_init(bar(i), warps4 ? 4 : readers ? 4 * kSets : issuers ? 2 : 1);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
         const int set = (warp - 4) >> 2;
         const uint32_t t = tmem + ((uint32_t)(warp & 3) << 21);   // lanes 32 * (warp % 4) ..
         const uint32_t acc = t + 48 * set;
-        uint32_t phase = 0, dense = 0;
+        uint32_t phase = 0, dense = 0, rows_done = 0;
         for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
             uint32_t held[5][4];   // conv2's pooled rows 1 and 2, left half of row 3
             __nv_bfloat162 top = __floats2bfloat162_rn(0.f, 0.f);
@@ -378,7 +379,9 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                                     pool4(r[4 * i + 2], r[4 * i + 3], r[16 + 4 * i + 2], r[16 + 4 * i + 3]));
                     if (Q == 0) st4(t + FLAT + 16 * h + 8 * (set >> 1) + word, o);
                     if (Q == 3 && h == 1) {
-                        // conv2's left halves are complete: the columns of pixels 0..7 are free
+                        // conv2 has read the last of conv1's rows
+                        if (!(ok = wait(ROW_DONE, rows_done++ & 1))) return;
+                        tc::tc_fence_after();
 #pragma unroll
                         for (int c = 0; c < 5; ++c) st4(t + late_columns(2 * c + (set >> 1)) + word, held[c]);
                         st4(t + late_columns(10 + (set >> 1)) + word, o);
@@ -387,6 +390,11 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
             };
             for (int p = 0; ok && p < kRows; ++p) {
                 const uint32_t mid = t + MID + 48 * (p % 6);
+                // conv2's last pooled row has read the slots of this row and the next
+                if (p >= 6 && (p & 1) == 0) {
+                    if (!(ok = wait(ROW_DONE, rows_done++ & 1))) break;
+                    tc::tc_fence_after();
+                }
                 // conv1's blocks go round the sets
 #pragma unroll 1
                 for (int b = (set - 6 * p) & 3; b < 6; b += 4) {
@@ -500,15 +508,17 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
         }
     } else {
         // ---------------------------------------------------------------------- tensor cores
-        // One thread does all of it, so a wait leads straight to the next issue.  Rows go in pairs: which
-        // buffer a block gets is then known at compile time.
+        // One thread of each of two warps, so a wait leads straight to the next issue: `side` 0 fills the buffers
+        // of sets 0 and 1 and issues the dense layers, side 1 those of sets 2 and 3.  With one thread for
+        // all, the 300 cycles from a wait to its commit, 72 times a tile, bound conv1 (28 us a tile).
+        const int side = warp - kIssuer;
         const uint32_t b1 = (base + B1_OFF) >> 4, b2 = (base + B2_OFF) >> 4, w1 = (base + W1_OFF) >> 4;
         const uint32_t w2 = (base + W2_OFF) >> 4, w3 = (base + W3_OFF) >> 4;
         if (ok && tc::elect_one()) {
             const auto wait1 = [&](int i, uint32_t parity) { return tc::mbar_wait(bar(i), parity, abort_flag); };
             const int off[3] = {B1_OFF, B2_OFF, W1_OFF}, bytes[3] = {B1_BYTES, B2_BYTES, kBlob - W1_OFF};
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
+            for (int i = 0; i < 3 && side == 0; ++i) {
                 tc::mbar_arrive_expect_tx(bar(W_FULL + i), (uint32_t)bytes[i]);
                 tc::bulk_load(base + off[i], a.blob + off[i], (uint32_t)bytes[i], bar(W_FULL + i));
             }
@@ -516,7 +526,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
             constexpr uint32_t id128 = tc::make_idesc(false, false, 128, D1), id96 = tc::make_idesc(false, false, 128, D2P);
             constexpr uint32_t id16 = tc::make_idesc(false, false, 128, D3P);
             uint32_t g = 0, mids = 0, ready = 0;
-            uint32_t free_phase = 15;   // of ACC_EMPTY, a bit each
+            uint32_t free_phase = 3;   // of this side's two ACC_EMPTY, a bit each
             bool first = true;
             for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
                 if (first) ok = wait1(W_FULL, 0);
@@ -536,16 +546,20 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                             left[i] = (base + IN_OFF + (slot >> 1) * IN_GROUP + (slot & 1) * IN_BLOCK) >> 4;
                             right[i] = (base + IN_OFF + (slot >> 1) * IN_GROUP + 2 * IN_BLOCK + (slot & 1) * 64) >> 4;
                         }
+                        // blocks go round the four buffers, so this side has 0, 1, 4, 5 of one row of a pair
+                        // and 2, 3 of the other
 #pragma unroll
-                        for (int b = 0; b < 6; ++b) {
-                            const int k = (6 * odd + b) & 3;
-                            if (!(ok = wait1(ACC_EMPTY + k, (free_phase >> k) & 1))) break;
+                        for (int j = 0; j < 4; ++j) {
+                            if (j >= 2 && odd != side) break;
+                            const int b = odd == side ? (j < 2 ? j : j + 2) : 2 + j, k = j & 1;
+                            if (!(ok = wait1(ACC_EMPTY + 2 * side + k, (free_phase >> k) & 1))) break;
                             free_phase ^= 1u << k;
                             tc::tc_fence_after();
+                            const uint32_t d = tmem + 96 * side + 48 * k;
 #pragma unroll
                             for (int i = 0; i < 3; ++i)
-                                umma_ss(tmem + 48 * k, b < 4 ? left[i] + 2 * b : right[i] + 2 * (b - 4), b1 + 2 * i, id48, i > 0);
-                            tc::umma_commit(bar(ACC_FULL + k));
+                                umma_ss(d, b < 4 ? left[i] + 2 * b : right[i] + 2 * (b - 4), b1 + 2 * i, id48, i > 0);
+                            tc::umma_commit(bar(ACC_FULL + 2 * side + k));
                         }
                         if (!ok) break;
                         tc::umma_commit(bar(IN_EMPTY + ((g + p) & 3)));
@@ -564,29 +578,34 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
 #pragma unroll
                     for (int i = 0; i < 6; ++i) rows[i] = tmem + MID + 48 * ((2 * q + i) % 6);
 #pragma unroll 1
-                    for (int h = 0; h < 2; ++h)
+                    for (int h = 0; h < 2; ++h) {
+                        // a large buffer is two small ones, read by both sets
+                        if (!(ok = wait1(ACC_EMPTY + 2 * side, free_phase & 1))) break;
+                        if (!(ok = wait1(ACC_EMPTY + 2 * side + 1, free_phase >> 1))) break;
+                        free_phase ^= 3u;
+                        tc::tc_fence_after();
+                        const uint32_t d = tmem + 96 * side, w = b2 + 256 * side;
 #pragma unroll
-                        for (int half = 0; half < 2; ++half) {
-                            // a large buffer is two small ones, read by both sets
-                            if (!(ok = ok && wait1(ACC_EMPTY + 2 * half, (free_phase >> (2 * half)) & 1))) break;
-                            if (!(ok = wait1(ACC_EMPTY + 2 * half + 1, (free_phase >> (2 * half + 1)) & 1))) break;
-                            free_phase ^= 3u << (2 * half);
-                            tc::tc_fence_after();
+                        for (int dy = 0; dy < 2; ++dy)
 #pragma unroll
-                            for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-                                for (int s = 0; s < 15; ++s)
-                                    umma_ts(tmem + 96 * half + 32 * dy, rows[dy + s / 3] + 24 * h + 8 * (s % 3),
-                                            b2 + 256 * half + (s >> 2) * (B2_CHUNK / 16) + 2 * (s & 3), id32, s > 0);
-                            tc::umma_commit(bar(ACC_FULL + 2 * half));
-                            tc::umma_commit(bar(ACC_FULL + 2 * half + 1));
-                        }
+                            for (int s = 0; s < 15; ++s)
+                                umma_ts(d + 32 * dy, rows[dy + s / 3] + 24 * h + 8 * (s % 3),
+                                        w + (s >> 2) * (B2_CHUNK / 16) + 2 * (s & 3), id32, s > 0);
+                        tc::umma_commit(bar(ACC_FULL + 2 * side));
+                        tc::umma_commit(bar(ACC_FULL + 2 * side + 1));
+                    }
+                    if (ok) tc::umma_commit(bar(ROW_DONE));
                 }
                 if (!ok) break;
                 g += kPairs;
                 mids += 2;
                 if (first && !(ok = wait1(W_FULL + 2, 0))) break;
                 first = false;
+                if (side == 1) {   // side 0 issues the dense layers
+                    ok = wait1(TILE_DONE, ready++ & 1);
+                    tc::tc_fence_after();
+                    continue;
+                }
                 // the accumulators are free when the flattened rows are complete
                 if (!(ok = wait1(A_READY, ready++ & 1))) break;
                 tc::tc_fence_after();
@@ -609,6 +628,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                 tc::umma_commit(bar(D_FULL));
                 ok = wait1(A_READY, ready++ & 1);
                 tc::tc_fence_after();
+                if (ok) tc::mbar_arrive(bar(TILE_DONE));
             }
             if (!ok) {   // a bounded wait for the weight copies in flight
                 int none = 0;
