@@ -157,6 +157,8 @@ __global__ void __launch_bounds__(kThreads, 1) lenet_train_kernel(const Args a) 
     const uint32_t bar = tc::smem_u32(smem + S::bar);
     const T *x = reinterpret_cast<const T *>(a.x);
     const int ngroups = (a.bs + G - 1) / G;
+    // The second launch may take the SMs this one leaves free now; it waits there for this one's end.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     if (tid == kThreads - 1) {   // the dense weights start their way into shared memory
         s_abort = 0;
@@ -706,6 +708,8 @@ constexpr int kChunk = 64, kPitch = 36;
 template <class T>
 __global__ void __launch_bounds__(256) lenet_finish_kernel(const __grid_constant__ Finish f) {
     __shared__ __align__(16) float As[2][kChunk][kPitch], Bs[2][kChunk][kPitch];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int tid = threadIdx.x;
     int blk = blockIdx.x;
     if (blk >= kTiles * f.splits) {
@@ -716,8 +720,16 @@ __global__ void __launch_bounds__(256) lenet_finish_kernel(const __grid_constant
             const int lane = tid & 31, grp = tid >> 5, i = blk * 32 + lane;
             float s = 0.f;
             if (i < 2550) {
-#pragma unroll 4
-                for (int z = grp; z < f.planes; z += 8) s += f.conv_planes[(int64_t)z * kPlane + i];
+                // sixteen loads in flight: 148 planes in two rounds
+                for (int z = grp; z < f.planes; z += 128) {
+                    float v[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        v[j] = z + 8 * j < f.planes ? f.conv_planes[(int64_t)(z + 8 * j) * kPlane + i] : 0.f;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (z + 8 * j < f.planes) s += v[j];
+                }
             }
             part[grp * 32 + lane] = s;
             __syncthreads();
@@ -753,25 +765,30 @@ __global__ void __launch_bounds__(256) lenet_finish_kernel(const __grid_constant
     const int kg = tid >> 6, t = tid & 63, tx = t & 7, ty = t >> 3;
     const bool bias = layer == 2 && f.off[5] >= 0 && m0 == 0 && tid < 32;
     float acc[4][4] = {}, bsum = 0.f;
-    float ra[kChunk / 8], rb[kChunk / 8];
-    auto load = [&](int kc) {
+    // two chunks ahead: a batch of up to 128 images costs one trip to memory
+    float ra[2][kChunk / 8], rb[2][kChunk / 8];
+    auto load = [&](int kc, float (&va)[kChunk / 8], float (&vb)[kChunk / 8]) {
 #pragma unroll
         for (int i = 0; i < kChunk / 8; ++i) {
             const int r = kc + i * 8 + kb;
-            ra[i] = r < r1 && m0 + mn < rows ? to_f32(in[(int64_t)r * rows + m0 + mn]) : 0.f;
-            rb[i] = r < r1 && n0 + mn < cols ? to_f32(g[(int64_t)r * cols + n0 + mn]) : 0.f;
+            va[i] = r < r1 && m0 + mn < rows ? to_f32(in[(int64_t)r * rows + m0 + mn]) : 0.f;
+            vb[i] = r < r1 && n0 + mn < cols ? to_f32(g[(int64_t)r * cols + n0 + mn]) : 0.f;
         }
     };
-    load(r0);
-    int buf = 0;
-    for (int kc = r0; kc < r1; kc += kChunk, buf ^= 1) {
+    load(r0, ra[0], rb[0]);
+    load(r0 + kChunk, ra[1], rb[1]);
+    for (int kc0 = r0; kc0 < r1; kc0 += 2 * kChunk)
+#pragma unroll
+    for (int buf = 0; buf < 2; ++buf) {
+        const int kc = kc0 + buf * kChunk;
+        if (kc >= r1) break;
 #pragma unroll
         for (int i = 0; i < kChunk / 8; ++i) {
-            As[buf][i * 8 + kb][mn] = ra[i];
-            Bs[buf][i * 8 + kb][mn] = rb[i];
+            As[buf][i * 8 + kb][mn] = ra[buf][i];
+            Bs[buf][i * 8 + kb][mn] = rb[buf][i];
         }
         __syncthreads();
-        if (kc + kChunk < r1) load(kc + kChunk);
+        if (kc + 2 * kChunk < r1) load(kc + 2 * kChunk, ra[buf], rb[buf]);
         // four groups of 64 threads, a quarter of the chunk each, 4 x 4 outputs per thread
 #pragma unroll 8
         for (int k = kg * (kChunk / 4); k < (kg + 1) * (kChunk / 4); ++k) {
@@ -821,6 +838,7 @@ __global__ void __launch_bounds__(256) lenet_finish_kernel(const __grid_constant
 // The parts of the dense gradients, added in order.
 template <class T>
 __global__ void __launch_bounds__(256) lenet_reduce_kernel(const __grid_constant__ Finish f) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= kDense - (f.off[5] < 0 ? D3 : 0)) return;
     float s = 0.f;
@@ -843,6 +861,23 @@ static int launch_pass(ag_device *dev, const Args &a, int ctas) {
         configured = true;
     }
     kernel<<<ctas, kThreads, bytes, dev->stream>>>(a);
+    AG_CHECK_LAUNCH();
+    return AG_OK;
+}
+
+// A launch whose CTAs may be placed before the previous kernel ends (both wait for it themselves): at 100
+// images the step is a chain of launches, each of which started 2 us after the last.
+static int launch_after(ag_device *dev, void (*kernel)(const Finish), int ctas, const Finish &f) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(256);
+    cfg.stream = dev->stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    AG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, f));
     AG_CHECK_LAUNCH();
     return AG_OK;
 }
@@ -902,12 +937,8 @@ static int step_typed(ag_device *dev, const Net &net, const void *x, const uint8
     f.conv_planes = a.planes;
     f.row_loss = a.row_loss;
     f.loss = loss;
-    lenet_finish_kernel<T><<<(unsigned)(kTiles * f.splits + kConvBlocks + 1), 256, 0, dev->stream>>>(f);
-    AG_CHECK_LAUNCH();
-    if (f.splits > 1) {
-        lenet_reduce_kernel<T><<<(unsigned)ceil_div(kDense, 256), 256, 0, dev->stream>>>(f);
-        AG_CHECK_LAUNCH();
-    }
+    AG_TRY(launch_after(dev, lenet_finish_kernel<T>, kTiles * f.splits + kConvBlocks + 1, f));
+    if (f.splits > 1) AG_TRY(launch_after(dev, lenet_reduce_kernel<T>, (int)ceil_div(kDense, 256), f));
     return AG_OK;
 }
 
