@@ -49,6 +49,11 @@ template <class T>
 static int patches_times_filters(ag_device *dev, const T *src, const ConvMap &map, int M, const T *w, int N,
                                  int s_row, int s_c, const NchwOut<T> &E) {
     const int K = map.ff * map.cp, total = N * K;
+    // One wave of tiles and up to 18 k steps of an input gradient, whose neighbouring rows are neighbouring
+    // filters: read in place at the copy's device time, without its launch (forward, 5 x 64 x 22 x 22 -> 128:
+    // 27 us in place, 19 copied; input gradient 21.7 and 21.5; 50 steps of 128 channels 5x5 190 and 87).
+    if (s_row < s_c && K <= 18 * BK && ceil_div(M, BM) * ceil_div(N, 64) <= dev->sm_count)
+        return gemm<T>(dev, M, N, K, ConvRows<T>{src, map, M}, FilterRows<T>{w, s_row, s_c, map.channels, map.div_cp}, E);
     void *ws = nullptr;
     AG_TRY(staging(dev, (size_t)total * sizeof(T), &ws));
     T *packed = (T *)ws;

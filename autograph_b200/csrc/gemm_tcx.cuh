@@ -357,6 +357,33 @@ struct ConvCols {
     }
 };
 
+// A filter bank in the order of ConvRows' k, read where it lies: element (row, (tap, channel)) at
+// w[row * s_row + channel * s_c + tap], zero for the padding channels.  Eight strided loads per chunk where the
+// repacked copy is one vector, but no launch to make the copy.
+template <class T>
+struct FilterRows {
+    static constexpr Walk kWalk = kByRow;
+    static constexpr int kTable = 0;
+    const T *w;
+    int s_row, s_c, channels;
+    FastDiv div_cp;
+    struct State { const T *q; };
+    __device__ __forceinline__ void init(int *, int, int) const {}
+    __device__ __forceinline__ void begin(State &s, const int *, int row, int) const { s.q = w + (int64_t)row * s_row; }
+    __device__ __forceinline__ void load(const State &s, const int *, int, int k, int k_end, Vec8<T> &d) const {
+        uint32_t tap, c;
+        div_cp.divmod((uint32_t)k, tap, c);
+        const T *q = s.q + (int)c * s_c + (int)tap;
+#pragma unroll
+        for (int j = 0; j < 8; ++j, q += s_c) fetch(d.v[j], q, k < k_end && (int)c + j < channels);
+    }
+    __device__ __forceinline__ float at(int row, int k) const {
+        uint32_t tap, c;
+        div_cp.divmod((uint32_t)k, tap, c);
+        return (int)c < channels ? to_f32(w[(int64_t)row * s_row + (int)c * s_c + (int)tap]) : 0.f;
+    }
+};
+
 // Few channels: padding them to eight would multiply the patch (1 channel: by eight).  The patch index is
 // the filter bank's own (channel, tap) order instead, so the filters need no repacking; a table holds
 // each index's offset and tap, and an element costs 6 instructions.

@@ -524,8 +524,10 @@ __global__ void bias_grad_cols_vec_kernel(const T *__restrict__ x, float *__rest
 template <class T>
 __global__ void bias_grad_inner_kernel(const T *__restrict__ x, float *__restrict__ partial,
                                        int64_t rows, int64_t cols, int64_t inner,
-                                       int64_t rows_per_chunk) {
+                                       int64_t rows_per_chunk, int *__restrict__ arrivals, T *__restrict__ y,
+                                       float beta) {
     __shared__ float part[256];
+    __shared__ bool last;
     const int64_t c = blockIdx.x;
     const int64_t r0 = (int64_t)blockIdx.y * rows_per_chunk;
     const int64_t r1 = min(rows, r0 + rows_per_chunk);
@@ -541,6 +543,25 @@ __global__ void bias_grad_inner_kernel(const T *__restrict__ x, float *__restric
         __syncthreads();
     }
     if (threadIdx.x == 0) partial[(int64_t)blockIdx.y * cols + c] = part[0];
+    if (arrivals == nullptr) return;
+    // the column's last chunk adds them all, chunk k in thread k % 256, then by the tree above
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(arrivals + c, 1) == (int)gridDim.y - 1;
+        if (last) arrivals[c] = 0;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    s = 0.f;
+    for (int k = threadIdx.x; k < (int)gridDim.y; k += 256) s += __ldcg(partial + (int64_t)k * cols + c);
+    part[threadIdx.x] = s;
+    __syncthreads();
+    for (int off = 128; off > 0; off >>= 1) {
+        if ((int)threadIdx.x < off) part[threadIdx.x] += part[threadIdx.x + off];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) y[c] = from_f32<T>(beta != 0.f ? __fadd_rn(part[0], __fmul_rn(beta, to_f32(y[c]))) : part[0]);
 }
 
 // Block of 32 x 8 threads: 32 consecutive columns, the chunk rows dealt round-robin to the eight
@@ -596,9 +617,16 @@ static int bias_grad_run(ag_device *dev, const T *x, int64_t rows, int64_t cols,
     else if (inner == 1)
         bias_grad_cols_kernel<T><<<grid, 256, 0, dev->stream>>>(x, (float *)ws, rows, cols,
                                                                 rows_per_chunk, nullptr, 0.f);
-    else
+    else {
+        // one launch when every column has a counter
+        int *arrivals = cols < kTileCounters ? dev->tile_counters : nullptr;
         bias_grad_inner_kernel<T><<<grid, 256, 0, dev->stream>>>(x, (float *)ws, rows, cols, inner,
-                                                                 rows_per_chunk);
+                                                                 rows_per_chunk, arrivals, y, beta);
+        if (arrivals != nullptr) {
+            AG_CHECK_LAUNCH();
+            return AG_OK;
+        }
+    }
     AG_CHECK_LAUNCH();
     bias_grad_final_kernel<T><<<(unsigned)ceil_div(cols, 32), dim3(32, 8), 0, dev->stream>>>(
         (const float *)ws, y, cols, (int)chunks, beta);
