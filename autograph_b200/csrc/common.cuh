@@ -90,6 +90,28 @@ struct ag_device {
 
 namespace ag {
 
+// Programmatic dependent launch.  A kernel launched with launch_dependent may be placed on SMs that its
+// predecessor in the stream has left and set itself up there; after dependency_wait everything the
+// predecessor wrote is visible.  Every thread that touches global memory comes through that wait first.
+__device__ __forceinline__ void let_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+int launch_dependent(ag_device *dev, void (*kernel)(P...), dim3 grid, int threads, size_t smem, const A &...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = dev->stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    AG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
+    AG_CHECK_LAUNCH();
+    return AG_OK;
+}
+
 // How a kernel tells a waiting host thread that it is done: its last CTA writes `seq` to a word of pinned
 // memory, which the host polls.  cudaStreamSynchronize returns 3 us later (launch and wait 10.5 us, with
 // the word 7.4), a sixth of a small inference call.

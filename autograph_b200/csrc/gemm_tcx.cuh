@@ -724,6 +724,8 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    let_dependents_launch();
+    dependency_wait();
 
     const int tiles = p.tiles_m * p.tiles_n;
     const int num_work = tiles * p.splits;
@@ -1025,8 +1027,7 @@ int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
     }
     const int64_t work = tiles * p.splits;
     const int grid = (int)(work < dev->sm_count ? work : dev->sm_count);
-    kernel<<<grid, C::THREADS, C::SMEM, dev->stream>>>(A, B, E, p);
-    AG_CHECK_LAUNCH();
+    AG_TRY(launch_dependent(dev, kernel, dim3((unsigned)grid), C::THREADS, C::SMEM, A, B, E, p));
     if (p.splits > 1 && p.arrivals == nullptr) {
         reduce_splits_kernel<Epi><<<(unsigned)ceil_div((int64_t)p.M * p.N, 256), 256, 0, dev->stream>>>(
             p.partial, p.splits, p.M, p.N, FastDiv((uint32_t)p.M), E);
