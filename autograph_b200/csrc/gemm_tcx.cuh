@@ -485,6 +485,7 @@ struct ChannelRows {
 // C = alpha * acc + beta * C, element (row, col) at c[row * s_row + col * s_col].
 template <class T>
 struct StridedOut {
+    static constexpr bool kLastCtaAdds = false;   // who adds k slices, see launch()
     T *c;
     int64_t s_row, s_col;
     float alpha, beta;
@@ -503,6 +504,7 @@ struct StridedOut {
 // y[col][row] = relu?(round(round(acc) + bias[row])): a Dense layer with rows = outputs.
 template <class T>
 struct DenseOut {
+    static constexpr bool kLastCtaAdds = false;
     T *c;
     int64_t s_col;
     const T *bias;
@@ -524,6 +526,7 @@ struct DenseOut {
 // the roundings of the separate operators.
 template <class T>
 struct NchwOut {
+    static constexpr bool kLastCtaAdds = true;
     T *y;
     const T *bias;
     int channels, hw;
@@ -547,6 +550,7 @@ struct NchwOut {
 // Rows are (tap, padded channel), columns output channels: dw[col][channel][tap] = beta * dw + acc.
 template <class T>
 struct FilterOut {
+    static constexpr bool kLastCtaAdds = true;
     T *dw;
     int channels, ff;
     FastDiv div_cp;
@@ -945,7 +949,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
         }
         tc::tmem_dealloc(tmem, C::TMEM);
     }
-    if (p.arrivals != nullptr) {
+    if (Epi::kLastCtaAdds && p.arrivals != nullptr) {
         // every CTA has had one slice of one tile (grid = tiles * splits)
         const int tile = blockIdx.x % tiles;
         int *last = table_a;
@@ -953,11 +957,13 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
             __threadfence();   // the slice's sums, stored by the epilogue warps before the barrier
             const int n = atomicAdd(p.arrivals + tile, 1);
             *last = n == p.splits - 1;
-            if (n == p.splits - 1) p.arrivals[tile] = 0;   // for the next launch
+            if (n == p.splits - 1) {
+                p.arrivals[tile] = 0;   // for the next launch
+                __threadfence();        // the other slices, for the whole CTA after the barrier
+            }
         }
         __syncthreads();
         if (*last) {
-            __threadfence();
             reduce_tile<C::THREADS>(p, E, (tile % p.tiles_m) * BM, (tile / p.tiles_m) * BN, BN, tid);
         }
     }
@@ -967,6 +973,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
 template <class Epi>
 __global__ void __launch_bounds__(256)
     reduce_splits_kernel(const float *partial, int splits, int M, int N, FastDiv div_m, Epi E) {
+    dependency_wait();
     const int64_t plane = (int64_t)M * N;
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (i >= plane) return;
@@ -1011,10 +1018,11 @@ int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
         void *ws = nullptr;
         AG_TRY(engine_scratch(dev, sizeof(float) * (size_t)p.splits * p.M * p.N, &ws));
         p.partial = (float *)ws;
-        // Up to eight slices the tile's last CTA adds them (two rounds of loads, at most 256 KB from L2: 2 us):
-        // a separate kernel costs its launch on the host (4 us) and 3 us on the device.  More slices
-        // would be a chain of round trips (3 -> 64 3x3 weight gradient, 37 slices: 24 us against 13).
-        if (p.splits <= 8 && tiles <= kTileCounters &&
+        // Convolutions of up to eight slices: the tile's last CTA adds them.  That takes 3 us more on the device
+        // than the separate kernel (512^3 f32 13.8 us against 9.9), whose launch costs 4 us on the host; a pass
+        // over a small convolution's edges is ten launches that the device waits for, a product by itself
+        // is not.  More slices would be a chain of round trips (37 slices: 24 us against 13).
+        if (Epi::kLastCtaAdds && p.splits <= 8 && tiles <= kTileCounters &&
             (int64_t)p.splits * (p.M < BM ? p.M : BM) * (p.N < BN ? p.N : BN) <= 65536)
             p.arrivals = dev->tile_counters;
     }
@@ -1029,9 +1037,8 @@ int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
     const int grid = (int)(work < dev->sm_count ? work : dev->sm_count);
     AG_TRY(launch_dependent(dev, kernel, dim3((unsigned)grid), C::THREADS, C::SMEM, A, B, E, p));
     if (p.splits > 1 && p.arrivals == nullptr) {
-        reduce_splits_kernel<Epi><<<(unsigned)ceil_div((int64_t)p.M * p.N, 256), 256, 0, dev->stream>>>(
-            p.partial, p.splits, p.M, p.N, FastDiv((uint32_t)p.M), E);
-        AG_CHECK_LAUNCH();
+        AG_TRY(launch_dependent(dev, reduce_splits_kernel<Epi>, dim3((unsigned)ceil_div((int64_t)p.M * p.N, 256)), 256, 0,
+                                (const float *)p.partial, p.splits, p.M, p.N, FastDiv((uint32_t)p.M), E));
     }
     return AG_OK;
 }

@@ -548,11 +548,13 @@ __global__ void bias_grad_inner_kernel(const T *__restrict__ x, float *__restric
     if (threadIdx.x == 0) {
         __threadfence();
         last = atomicAdd(arrivals + c, 1) == (int)gridDim.y - 1;
-        if (last) arrivals[c] = 0;
+        if (last) {
+            arrivals[c] = 0;
+            __threadfence();
+        }
     }
     __syncthreads();
     if (!last) return;
-    __threadfence();
     s = 0.f;
     for (int k = threadIdx.x; k < (int)gridDim.y; k += 256) s += __ldcg(partial + (int64_t)k * cols + c);
     part[threadIdx.x] = s;
