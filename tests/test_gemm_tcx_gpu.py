@@ -142,3 +142,19 @@ def test_small_products(dev, dtype, shape):
     c = dev.dot(x, w)
     assert ((c.double() - ref).abs() <= bound).all()
     assert torch.equal(dev.dense_forward(x, w, bias=b, relu=True), dev.relu(dev.bias_add(c, b)))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(1, 25003, 515), (15, 700, 1201), (4999, 1030, 3)])
+def test_few_rows_or_columns(dev, dtype, shape):
+    """Long products with fewer rows or columns than an MMA tile has."""
+    m, k, n = shape
+    gen = torch.Generator(device=dev.torch_device).manual_seed(k)
+    rnd = lambda s: (torch.rand(s, generator=gen, device=dev.torch_device) * 2 - 1).to(dtype)
+    a, b = rnd((m, k)), rnd((k, n))
+    ref = a.double() @ b.double()
+    bound = _f32_bound(a, b, k)
+    if dtype == torch.bfloat16:
+        bound = ref.abs() * 2.0 ** -8 + bound * 64   # as in test_product_vs_f64
+    assert ((dev.dot(a, b).double() - ref).abs() <= bound).all()
+    dev.wait()
