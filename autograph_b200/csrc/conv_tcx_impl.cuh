@@ -19,6 +19,9 @@ static ConvMap conv_map(int64_t channels, int64_t sh, int64_t sw, int64_t gh, in
     g.dil_h = o->dilation[0]; g.dil_w = o->dilation[1];
     g.gradient = gradient;
     g.always_valid = !gradient && g.pad_h == 0 && g.pad_w == 0;  // gh, gw come from the output rule
+    g.ranges = (g.dil_h == 1 || g.fh == 1) && (g.dil_w == 1 || g.fw == 1) && (!gradient || (g.st_h == 1 && g.st_w == 1));
+    g.row_ones = 0;
+    for (int fi = 0; fi < g.fh; ++fi) g.row_ones |= 1u << (fi * g.fw & 31);
     g.div_ghw = FastDiv((uint32_t)g.ghw);
     g.div_gw = FastDiv((uint32_t)g.gw);
     g.div_fw = FastDiv((uint32_t)g.fw);
