@@ -21,19 +21,23 @@ static bool enabled() {
 // k, two kernels) whatever the size, so the line is drawn at the multiply-adds the SIMT kernels do
 // in that time.
 // Few rows: 1 to 8 x 25088 x 512 18 us and 68 (bf16 13 and 97), 12 x 100 x 20000 9 and 27.  Few columns: 20000 x 200 x
-// 12 25 and 14, 5000 x 2000 x 12 51 and 98.  k below a tile's step: 25088 x 24 x 512 39 and 27.
+// 12 25 and 14, 5000 x 2000 x 12 51 and 98.  k below a tile's step: 25088 x 24 x 512 39 and 27,
+// f32 1264 x 32 x 4896 22 and 17, 892 x 39 x 7961 24 and 25.
 bool gemm_worth(ag_dtype dtype, int64_t m, int64_t k, int64_t n) {
-    if (!enabled() || k < 32) return false;
+    if (!enabled() || k < (dtype == AG_F32 ? 40 : 32)) return false;
     const double macs = (double)m * (double)n * (double)k;
     if (m < 16 || n < 16) return macs >= 1e7 && k >= (n < 16 ? 1024 : 64);
     return macs >= (dtype == AG_F32 ? 3e7 : 4e6);
 }
 
-// Against the gathered engine: 1000 x 5000 x 130 f32 33 us packed and 48 us gathered, 1024^3 29 and
-// 34 (tn 48), 777 x 1009 x 333 21 and 24, 150 x 8000 x 200 (2.4e8 multiply-adds) 23 and 18.  The
-// copy pass and its launch are what a small product cannot amortise.
+// Against the gathered engine, m x k x n, us packed and gathered: f32 305 x 369 x 2296 29 and 15, 2592 x 2080 x 128 41
+// and 24, 3568 x 1344 x 528 72 and 58, 1040 x 3440 x 544 58 and 88, 5728 x 608 x 1200 81 and 100; bf16 1037 x 438 x
+// 1885 39 and 27, 4313 x 791 x 1252 41 and 71.  The copy pass, its launch and 256 x 256 tiles want 1.8e9
+// multiply-adds, more of them when k is short, because a tile is then mostly its epilogue (over 317 drawn
+// products this line is 1.4% above always taking the faster engine).
 bool packed_worth(int64_t m, int64_t k, int64_t n) {
-    return m >= 128 && n >= 128 && k >= 64 && (double)m * (double)n * (double)k >= 2.5e8;
+    const double macs = (double)m * (double)n * (double)k;
+    return m >= 128 && n >= 128 && k >= 64 && macs >= 1.8e9 && macs * (double)k >= 1.2e12;
 }
 
 // patch = channels x taps.  Against the SIMT engine, us here and there (f32 unless said):

@@ -30,6 +30,7 @@ def _f32_bound(av, bv, k):
     (130, 8003, 33),
     # packed engine: slices of k, whole tiles, tiles of a partial wave cut in two
     (1000, 5001, 130), (1537, 1601, 1703), (2560, 321, 2050),
+    (1000, 20001, 130), (2560, 641, 2050),
 ])
 def test_product_vs_f64(dev, dtype, layout, shape):
     m, k, n = shape
@@ -56,7 +57,7 @@ def test_product_vs_f64(dev, dtype, layout, shape):
     dev.wait()
 
 
-@pytest.mark.parametrize("shape", [(700, 300, 200), (1100, 700, 1300)])
+@pytest.mark.parametrize("shape", [(700, 300, 200), (1100, 700, 1300), (1100, 1500, 1300)])
 def test_f32_special_values(dev, shape):
     """Infinities, NaNs and values that round up to infinity in bf16 give what f32 gives; the rest
     of the product is not disturbed."""
@@ -115,7 +116,7 @@ def test_convolution_vs_f64(dev, dtype, case):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("shape", [(777, 333, 129), (5001, 260, 131), (1500, 1001, 900)])
+@pytest.mark.parametrize("shape", [(777, 333, 129), (5001, 260, 131), (1500, 1001, 900), (1500, 1601, 900)])
 def test_dense_epilogue(dev, dtype, shape):
     """Bias and relu in either engine's epilogue equal the product and the separate calls."""
     bs, ins, outs = shape
