@@ -66,6 +66,17 @@ static int dense_forward_simt(ag_device *dev, const T *x, int bs, int inputs, co
 
 using namespace ag;
 
+// Aligned bf16 products that the TMA kernels are better at than the gathered engine, whose k slices and smaller tiles fill
+// the chip where those have a handful of tiles.  m x k x n, us with TMA and gathered: 160 x 416 x 432 12.5 and 8.3, 208 x
+// 1328 x 144 17 and 8.4, 1408 x 608 x 192 12.5 and 10.1, 6928 x 64 x 432 10.4 and 12.1, 384 x 2864 x 336 16.6 and 11.2, 176 x
+// 3680 x 1088 27 and 16, 960 x 224 x 2608 11 and 22, 496 x 4832 x 416 21 and 24.
+static bool tma_worth(int64_t m, int64_t k, int64_t n) {
+    const double macs = (double)m * (double)n * (double)k;
+    if (!tcx::gemm_worth(AG_BF16, m, k, n)) return true;
+    if (k >= 1024 && ag::ceil_div(m, 128) * ag::ceil_div(n, 128) <= 24) return macs >= 8e8;
+    return macs >= 1.5e8;
+}
+
 extern "C" int ag_dense_forward(ag_device *dev, ag_dtype dtype, const void *x, int64_t bs,
                                 int64_t inputs, const void *w, int64_t outputs, const void *bias,
                                 int fuse_relu, void *y) {
@@ -95,7 +106,8 @@ extern "C" int ag_dense_forward(ag_device *dev, ag_dtype dtype, const void *x, i
                                          fuse_relu != 0, (float *)y);
     const __nv_bfloat16 *px = (const __nv_bfloat16 *)x, *pw = (const __nv_bfloat16 *)w;
     __nv_bfloat16 *py = (__nv_bfloat16 *)y;
-    if (tc::gemm_bf16_eligible(bs, inputs, outputs, px, inputs, 1, pw, outputs, 1, py, outputs, 1)) {
+    if (tma_worth(bs, inputs, outputs) &&
+        tc::gemm_bf16_eligible(bs, inputs, outputs, px, inputs, 1, pw, outputs, 1, py, outputs, 1)) {
         // Large products go to the tensor cores with bias and relu in the kernel's epilogue
         // (a bias that is not 16-byte aligned is added by a separate pass).
         const __nv_bfloat16 *pb = (const __nv_bfloat16 *)bias;
@@ -333,7 +345,7 @@ extern "C" int ag_gemm(ag_device *dev, ag_dtype dtype, int64_t m, int64_t k, int
     const __nv_bfloat16 *pa = (const __nv_bfloat16 *)a + off_a;
     const __nv_bfloat16 *pb = (const __nv_bfloat16 *)b + off_b;
     __nv_bfloat16 *pc = (__nv_bfloat16 *)c + off_c;
-    if (tc::gemm_bf16_eligible(m, k, n, pa, rsa, csa, pb, rsb, csb, pc, rsc, csc))
+    if (tma_worth(m, k, n) && tc::gemm_bf16_eligible(m, k, n, pa, rsa, csa, pb, rsb, csb, pc, rsc, csc))
         return tc::gemm_bf16(dev, (int)m, (int)k, (int)n, alpha, pa, rsa, csa, pb, rsb, csb, beta,
                              pc, rsc, csc);
     if (tensor_core)

@@ -146,9 +146,10 @@ def test_small_products(dev, dtype, shape):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("shape", [(1, 25003, 515), (15, 700, 1201), (4999, 1030, 3)])
+@pytest.mark.parametrize("shape", [(1, 25003, 515), (15, 700, 1201), (4999, 1030, 3),
+                                   (208, 1328, 144), (384, 2864, 336), (160, 416, 432)])
 def test_few_rows_or_columns(dev, dtype, shape):
-    """Long products with fewer rows or columns than an MMA tile has."""
+    """Long products with fewer rows or columns than an MMA tile has; aligned ones of a few tiles."""
     m, k, n = shape
     gen = torch.Generator(device=dev.torch_device).manual_seed(k)
     rnd = lambda s: (torch.rand(s, generator=gen, device=dev.torch_device) * 2 - 1).to(dtype)
