@@ -23,10 +23,13 @@ static bool enabled() {
 // Few rows: 1 to 8 x 25088 x 512 18 us and 68 (bf16 13 and 97), 12 x 100 x 20000 9 and 27.  Few columns: 20000 x 200 x
 // 12 25 and 14, 5000 x 2000 x 12 51 and 98.  k below a tile's step: 25088 x 24 x 512 39 and 27,
 // f32 1264 x 32 x 4896 22 and 17, 892 x 39 x 7961 24 and 25.
+// Beyond k = 128, where the SIMT kernels have no form that stages all of k at once, slices of k win much earlier: f32 16 x
+// 1056 x 1088 12.5 and 8.7, 32 x 800 x 64 10.2 and 8.4; bf16 88 x 211 x 97 23 and 8.3, 16 x 496 x 144 17 and 8.3.
 bool gemm_worth(ag_dtype dtype, int64_t m, int64_t k, int64_t n) {
     if (!enabled() || k < (dtype == AG_F32 ? 40 : 32)) return false;
     const double macs = (double)m * (double)n * (double)k;
     if (m < 16 || n < 16) return macs >= 1e7 && k >= (n < 16 ? 1024 : 64);
+    if (k > 128) return macs >= (dtype == AG_F32 ? 2e6 : 1e6);
     return macs >= (dtype == AG_F32 ? 3e7 : 4e6);
 }
 

@@ -147,7 +147,8 @@ def test_small_products(dev, dtype, shape):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape", [(1, 25003, 515), (15, 700, 1201), (4999, 1030, 3),
-                                   (208, 1328, 144), (384, 2864, 336), (160, 416, 432)])
+                                   (208, 1328, 144), (384, 2864, 336), (160, 416, 432),
+                                   (17, 333, 401), (40, 1436, 36)])
 def test_few_rows_or_columns(dev, dtype, shape):
     """Long products with fewer rows or columns than an MMA tile has; aligned ones of a few tiles."""
     m, k, n = shape
