@@ -29,7 +29,7 @@ bool gemm_worth(ag_dtype dtype, int64_t m, int64_t k, int64_t n) {
     if (!enabled() || k < (dtype == AG_F32 ? 40 : 32)) return false;
     const double macs = (double)m * (double)n * (double)k;
     if (m < 16 || n < 16) return macs >= 1e7 && k >= (n < 16 ? 1024 : 64);
-    if (k > 128) return macs >= (dtype == AG_F32 ? 2e6 : 1e6);
+    if (k > 128) return macs >= (dtype == AG_F32 ? 2e6 : 3e5);
     return macs >= (dtype == AG_F32 ? 3e7 : 4e6);
 }
 
