@@ -6,8 +6,8 @@
 // Roles per CTA (320 threads): warp 0 = TMA producer of the CTA's own halves, warp 1 = MMA
 // issuer (leader) and tensor-memory allocation, warps 2..9 = epilogue, each 32 rows x 128
 // columns.  An f32 product reads the accumulator out after every 64 k and adds the 64-k sums
-// in registers (the arithmetic, and why, is described in gemm_tcx.cuh); a bf16 product once per
-// tile.
+// in registers (the arithmetic, and why, is described in gemm_tcx.cuh; so is what happens to sums that
+// are not finite); a bf16 product once per tile.
 //
 // The tile's rows run along the contiguous index of C (a row-major C is computed as
 // C^T = B^T . A^T), so a warp's store is 32 consecutive elements and needs no alignment.
@@ -38,7 +38,8 @@ template <int PL>
 struct Cfg {
     static constexpr int STAGE = 2 * PL * HALF_BYTES;      // A half + B half of this CTA
     static constexpr int STAGES = PL == 3 ? 2 : 6;
-    static constexpr int SMEM = STAGES * STAGE + 1024 + 256;
+    static constexpr int SMEM = STAGES * STAGE + 1024 + 256 + (PL == 3 ? tcx::kMarks : 0);
+    static_assert(THREADS / 32 * tcx::kRedoFloats * 4 <= STAGES * STAGE, "the stages hold redo_block's buffers");
 };
 
 template <class T>
@@ -49,11 +50,12 @@ struct Params {
     T *C;
     // Items [0, t_full) are whole tiles, the tiles after them cut in tail_split pieces along n.
     int t_full, tail_split, num_work, group_m;
+    int work0, work1;         // this launch's share of them
     int splits, kb_split;     // slices of k (whole tiles only) and 64-k steps per slice
     float *partial;           // splits > 1: [splits][N][M] f32 sums
     const T *bias;            // per row, with relu the Dense layer's epilogue
     int relu;
-    // the operands as the caller gave them (recomputation of non-finite outputs)
+    // the operands as the caller gave them (redo_block)
     const T *p, *q;
     int64_t p_row, p_k, q_row, q_k;
     int *status;
@@ -94,15 +96,6 @@ __device__ __forceinline__ Work decode(int w, const Params<T> &p) {
 }
 
 template <class T>
-__device__ __noinline__ float recompute(const Params<T> &p, int row, int col, int k0, int k1) {
-    float s = 0.f;
-    const T *a = p.p + (int64_t)row * p.p_row, *b = p.q + (int64_t)col * p.q_row;
-    for (int k = k0; k < min(p.K, k1); ++k)
-        s = fmaf(to_f32(a[(int64_t)k * p.p_k]), to_f32(b[(int64_t)k * p.q_k]), s);
-    return s;
-}
-
-template <class T>
 __device__ __forceinline__ void store_out(const Params<T> &p, int row, int col, float acc) {
     T *q = p.C + row + (int64_t)col * p.ldc;
     float v = p.alpha * acc;
@@ -111,6 +104,50 @@ __device__ __forceinline__ void store_out(const Params<T> &p, int row, int col, 
     T o = from_f32<T>(v);
     if (p.relu && !(to_f32(o) >= 0.f)) o = from_f32<T>(0.f);
     *q = o;
+}
+
+// An operand as redo_block reads it.
+template <class T>
+struct Given {
+    const T *p;
+    int64_t s_row, s_k;
+    __device__ __forceinline__ float at(int row, int k) const { return to_f32(p[row * s_row + k * s_k]); }
+};
+
+// The blocks that this CTA's epilogue warps left out (gemm_tcx.cuh), dealt to its warps.
+template <bool A_MN, bool B_MN, class T>
+__device__ __noinline__ void redo_marked(const Params<T> &p, const unsigned *marks, float *buf, int rank) {
+    constexpr int WARPS = THREADS / 32;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const Given<T> A{p.p, p.p_row, p.p_k}, B{p.q, p.q_row, p.q_k};
+    int turn = 0;
+    for (int w = p.work0 + (int)(blockIdx.x >> 1), i = 0; w < p.work1; w += gridDim.x >> 1, ++i) {
+        const unsigned mark = marks[i / 4] >> (i % 4 * 8) & 255u;
+        if (mark == 0) continue;
+        const Work wk = decode(w, p);
+        const int width = wk.n_width / 2;
+        for (int block = 0; block < EPI_WARPS * width / 32; ++block) {
+            const int e = block % EPI_WARPS;   // warp 2 + e
+            const int row0 = wk.m_blk * TILE + rank * 128 + (2 + e) % 4 * 32;
+            const int col0 = wk.n_blk * TILE + wk.n_off + e / 4 * width + block / EPI_WARPS * 32;
+            if ((mark >> e & 1u) == 0 || row0 >= p.M || col0 >= p.N || turn++ % WARPS != warp) continue;
+            float acc[4][8];
+            tcx::redo_block<A_MN, B_MN>(A, B, row0, p.M, col0, p.N, wk.kb0 * BK, min(p.K, wk.kb1 * BK), buf, acc);
+            for (int r = 0; r < 4; ++r) {
+                const int row = row0 + lane / 4 * 4 + r;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const int col = col0 + lane % 4 * 8 + c;
+                    if (row >= p.M || col >= p.N) break;
+                    const float v = r == 0 ? acc[0][c] : r == 1 ? acc[1][c] : r == 2 ? acc[2][c] : acc[3][c];
+                    if (p.splits > 1)
+                        p.partial[((int64_t)wk.z * p.N + col) * p.M + row] = v;
+                    else
+                        store_out(p, row, col, v);
+                }
+            }
+        }
+    }
 }
 
 // Shared-memory layout of one operand half in a stage (rows = 128, or 64 for a tail piece of B):
@@ -134,11 +171,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     uint64_t *acc_empty = bars + 2 * STAGES + 2;       // [2] leader only
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);  // [2]
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 2);
+    volatile int *redo = reinterpret_cast<volatile int *>(tmem_slot + 3);                // any mark
+    unsigned *marks = tmem_slot + 4;   // bit e of byte i: epilogue warp e left its block of the pair's i-th item out
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const uint32_t rank = cluster_ctarank();
     const bool leader = rank == 0;
-    const int pair_id = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+    const int work0 = p.work0 + (int)(blockIdx.x >> 1), num_pairs = gridDim.x >> 1;
 
     if (threadIdx.x == 0) {
         prefetch_tmap(&tmap_a);
@@ -154,9 +193,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         }
         tmem_slot[0] = tmem_slot[1] = 0xffffffffu;
         *abort_flag = 0;
+        *redo = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    if (PL == 3 && threadIdx.x < tcx::kMarks / 4) marks[threadIdx.x] = 0;
     __syncthreads();
     // Tensor memory in two 256-column steps; after the first the pair compares addresses (as in
     // gemm_tc2.cu) and stops before anything could block on them if they differ.
@@ -190,7 +231,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int w = pair_id; ok && w < p.num_work; w += num_pairs) {
+            for (int w = work0; ok && w < p.work1; w += num_pairs) {
                 const Work wk = decode(w, p);
                 const int half_n = wk.n_width / 2;
                 const int m0 = wk.m_blk * TILE + (int)rank * 128;
@@ -236,7 +277,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
-            for (int w = pair_id; ok && w < p.num_work; w += num_pairs) {
+            for (int w = work0; ok && w < p.work1; w += num_pairs) {
                 const Work wk = decode(w, p);
                 const uint32_t idesc = make_idesc(A_MN, B_MN, TILE, wk.n_width);
                 const uint32_t b_plane = B_MN ? ATOM : wk.n_width / 2 * BK * 2;
@@ -299,7 +340,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         int acc = 0;
         uint32_t acc_phase = 0;
         bool ok = true;
-        for (int w = pair_id; ok && w < p.num_work; w += num_pairs) {
+        for (int w = work0; ok && w < p.work1; w += num_pairs) {
             const Work wk = decode(w, p);
             const int width = wk.n_width / 2;   // columns of this warp: 128, or 64 of a tail piece
             float sum[128];
@@ -338,24 +379,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             if (!ok) break;
             const int row = wk.m_blk * TILE + (int)rank * 128 + quarter * 32 + lane;
             const int col0 = wk.n_blk * TILE + wk.n_off + half * width;
-            float finite = 0.f;
+            bool redo_it = false;
             if (PL == 3) {
+                float finite = 0.f;
 #pragma unroll
                 for (int c = 0; c < 128; c += 32)
                     if (c < width)
 #pragma unroll
                         for (int j = 0; j < 32; ++j) finite = fmaf(sum[c + j], 0.f, finite);
+                redo_it = __any_sync(0xffffffffu, row < p.M && !(finite == 0.f));
+                if (redo_it && lane == 0) {
+                    const int i = (w - work0) / num_pairs;
+                    atomicOr(marks + i / 4, 1u << (i % 4 * 8 + warp - 2));
+                    *redo = 1;
+                }
             }
             float *part = p.splits > 1 ? p.partial + (int64_t)wk.z * p.M * p.N + row : nullptr;
-            if (row < p.M && !(finite == 0.f)) {
-#pragma unroll 1
-                for (int col = col0; col < min(p.N, col0 + width); ++col) {
-                    const float v = recompute(p, row, col, wk.kb0 * BK, wk.kb1 * BK);
-                    if (part != nullptr)
-                        part[(int64_t)col * p.M] = v;
-                    else
-                        store_out(p, row, col, v);
-                }
+            if (redo_it) {
             } else if (row < p.M) {
 #pragma unroll
                 for (int c = 0; c < 128; c += 32)
@@ -387,6 +427,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         tmem_dealloc2(tmem_acc[0], 256);
         tmem_dealloc2(tmem_acc[1], 256);
     }
+    // the pair's MMAs, which read both CTAs' stages, are done
+    if (PL == 3 && *redo && !*abort_flag)
+        redo_marked<A_MN, B_MN>(p, marks, reinterpret_cast<float *>(smem) + warp * tcx::kRedoFloats, (int)rank);
 }
 
 // C from the f32 sums of the slices, added in slice order.
@@ -456,7 +499,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const PackJob<T> j0, const Pa
 // ---------------------------------------------------------------------- host
 template <int PL, bool A_MN, bool B_MN, class T>
 static int launch(ag_device *dev, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tt,
-                  const Params<T> &p) {
+                  Params<T> p) {
     auto kernel = gemm_packed_kernel<PL, A_MN, B_MN, T>;
     static bool configured_on[64] = {};
     bool &configured = configured_on[dev->ordinal & 63];
@@ -465,9 +508,14 @@ static int launch(ag_device *dev, const CUtensorMap &ta, const CUtensorMap &tb, 
                                          Cfg<PL>::SMEM));
         configured = true;
     }
-    const int pairs = p.num_work < dev->sm_count / 2 ? p.num_work : dev->sm_count / 2;
-    kernel<<<2 * pairs, THREADS, Cfg<PL>::SMEM, dev->stream>>>(ta, tb, tt, p);
-    AG_CHECK_LAUNCH();
+    const int most = tcx::kMarks * (dev->sm_count / 2);   // one launch for up to 5e9 outputs
+    for (p.work0 = 0; p.work0 < p.num_work; p.work0 = p.work1) {
+        const int left = p.num_work - p.work0, n = left < most ? left : most;
+        p.work1 = p.work0 + n;
+        const int pairs = n < dev->sm_count / 2 ? n : dev->sm_count / 2;
+        kernel<<<2 * pairs, THREADS, Cfg<PL>::SMEM, dev->stream>>>(ta, tb, tt, p);
+        AG_CHECK_LAUNCH();
+    }
     return AG_OK;
 }
 

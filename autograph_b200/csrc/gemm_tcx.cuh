@@ -18,9 +18,10 @@
 // out after every 64 k and the 64-k sums are added in registers with round-to-nearest; within
 // 64 k the small partial products are accumulated first, which leaves four truncating additions
 // of full-size terms.  Uniform operands, relative 2-norm error against an f64 product: k = 128
-// 8e-8 (the FFMA kernel 1.1e-7), k = 1024 1.1e-7 (5.7e-7), k = 4096 1.7e-7 (1.2e-6).  An output
-// that comes out infinite or NaN is recomputed with FFMAs from the f32 operands (the split of
-// an infinity, or of a value that rounds up to one, is not usable).
+// 8e-8 (the FFMA kernel 1.1e-7), k = 1024 1.1e-7 (5.7e-7), k = 4096 1.7e-7 (1.2e-6).  The split of
+// an infinity, or of a value that rounds up to one, is not usable: blocks of outputs with a sum
+// that is infinite or NaN are left out and computed with FFMAs from the f32 operands when the
+// CTA's tiles are done (redo_block).
 //
 // What bounds it: with BN = 128 a 64-k step is 16 MMAs that read (128 + N) x 32 bytes of shared
 // memory each, about 2600 cycles; the producers convert 16 k elements in the same time.
@@ -589,6 +590,11 @@ struct FilterOut {
 };
 
 // ------------------------------------------------------------------- kernel
+// Tiles of one CTA in one launch whose blocks of outputs can be marked, a byte each.
+constexpr int kMarks = 1024;
+// Shared memory of redo_block: 16 k of 32 rows and 32 columns.
+constexpr int kRedoK = 16, kRedoPitch = 36, kRedoFloats = 2 * kRedoK * kRedoPitch;
+
 template <class T, int BN_>
 struct Cfg {
     static constexpr int PL = Planes<T>::N;
@@ -604,15 +610,18 @@ struct Cfg {
     static constexpr int STAGES = PL == 3 ? (BN > 64 ? 2 : 3) : 4;
     static constexpr int ACC_COLS = PL == 3 ? 2 * BN : BN;       // f32: leading block + corrections
     static constexpr int TMEM = 2 * ACC_COLS < 64 ? 64 : 2 * ACC_COLS;
-    static constexpr int SMEM = STAGES * STAGE + 1024 + 256 + 2 * kFewPatch * (int)sizeof(int);
+    static constexpr int SMEM = STAGES * STAGE + 1024 + 256 + 2 * kFewPatch * (int)sizeof(int) + (PL == 3 ? kMarks : 0);
     static_assert(SMEM <= 227 * 1024, "shared memory");
     static_assert(TMEM <= 512 && (TMEM & (TMEM - 1)) == 0, "tensor memory columns");
-    static_assert(COLS % 16 == 0, "epilogue warps read 16 columns at a time");
+    static_assert(COLS % 32 == 0 && EPI_WARPS <= 8, "blocks of 32 columns, a mark bit per epilogue warp");
+    static_assert(PRODUCERS % 128 == 0, "epilogue warp e reads rows e % 4 * 32 ..");
+    static_assert(THREADS / 32 * kRedoFloats * 4 <= STAGES * STAGE || PL == 1, "the stages hold redo_block's buffers");
 };
 
 struct Params {
     int M, N, K;
     int tiles_m, tiles_n, splits, k_split;  // k_split: k per slice, a multiple of BK
+    int work0, work1;                       // this launch's share of the tiles x slices
     float *partial;                         // splits > 1: [splits][N][M] f32 sums
     int *arrivals;                          // not null: the CTA of a tile that finishes last adds its slices
     int *status;
@@ -662,12 +671,61 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
         : "memory");
 }
 
-// Exact-f32 recomputation of an output whose split sum is not finite.
-template <class AOp, class BOp>
-__device__ __noinline__ float recompute(const AOp &A, const BOp &B, int row, int col, int k0, int k1) {
-    float s = 0.f;
-    for (int k = k0; k < k1; ++k) s = fmaf(A.at(row, k), B.at(col, k), s);
-    return s;
+// The 32 x 32 outputs at (row0, col0) from the operands as they were given: sums of k0 .. k1 in order, one
+// warp.  A lane has rows row0 + lane / 4 * 4 .. + 3 and columns col0 + lane % 4 * 8 .. + 7.  `buf` is the warp's
+// (kRedoFloats); ROWS_A, ROWS_B: neighbouring lanes fetch neighbouring rows of the operand, else
+// neighbouring k.  4096^3 f32, 0.59 ms: with a NaN in one row of A 2.3 ms (a chain of FMAs per lane in
+// the epilogue, which the pipeline's bounded waits had to outlast: 31 to 42 ms), with NaNs everywhere 0.7 ms.
+template <bool ROWS_A, bool ROWS_B, class AOp, class BOp>
+__device__ __forceinline__ void redo_block(const AOp &A, const BOp &B, int row0, int M, int col0, int N, int k0, int k1,
+                                        float *buf, float (&acc)[4][8]) {
+    const int lane = threadIdx.x & 31, ty = lane >> 2, tx = lane & 3;
+    float *sa = buf, *sb = buf + kRedoK * kRedoPitch;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int k = k0; k < k1; k += kRedoK) {
+        __syncwarp();
+#pragma unroll 1
+        for (int i0 = 0; i0 < kRedoK; i0 += 8) {   // sixteen loads in flight
+            float va[8], vb[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int ra = ROWS_A ? lane : 2 * (i0 + i) + (lane >> 4), ka = ROWS_A ? i0 + i : lane & 15;
+                const int rb = ROWS_B ? lane : 2 * (i0 + i) + (lane >> 4), kb = ROWS_B ? i0 + i : lane & 15;
+                va[i] = row0 + ra < M && k + ka < k1 ? A.at(row0 + ra, k + ka) : 0.f;
+                vb[i] = col0 + rb < N && k + kb < k1 ? B.at(col0 + rb, k + kb) : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                sa[(ROWS_A ? i0 + i : lane & 15) * kRedoPitch + (ROWS_A ? lane : 2 * (i0 + i) + (lane >> 4))] = va[i];
+                sb[(ROWS_B ? i0 + i : lane & 15) * kRedoPitch + (ROWS_B ? lane : 2 * (i0 + i) + (lane >> 4))] = vb[i];
+            }
+        }
+        __syncwarp();
+        const int ks = min(kRedoK, k1 - k);
+        for (int i = 0; i < ks; ++i) {
+            const float4 a = *reinterpret_cast<const float4 *>(sa + i * kRedoPitch + 4 * ty);
+            const float4 b0 = *reinterpret_cast<const float4 *>(sb + i * kRedoPitch + 8 * tx);
+            const float4 b1 = *reinterpret_cast<const float4 *>(sb + i * kRedoPitch + 8 * tx + 4);
+            const float av[4] = {a.x, a.y, a.z, a.w}, bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 8; ++c) acc[r][c] = fmaf(av[r], bv[c], acc[r][c]);
+        }
+        // a sum that is a NaN stays one: a block of them is done
+        if (__all_sync(0xffffffffu, isnan(acc[0][0]) || row0 + 4 * ty >= M || col0 + 8 * tx >= N)) {
+            bool all = true;
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    all = all && (isnan(acc[r][c]) || row0 + 4 * ty + r >= M || col0 + 8 * tx + c >= N);
+            if (__all_sync(0xffffffffu, all)) return;
+        }
+    }
 }
 
 // One tile's slices added in slice order, as reduce_splits_kernel adds them, and stored: four columns and
@@ -701,10 +759,46 @@ __device__ __forceinline__ void reduce_tile(const Params &p, const Epi &E, int m
     }
 }
 
+// The marked blocks of this CTA's tiles, dealt to its warps.
+template <class C, class AOp, class BOp, class Epi>
+__device__ __noinline__ void redo_marked(const AOp &A, const BOp &B, const Epi &E, const Params &p,
+                                         const unsigned *marks, float *buf) {
+    constexpr int WARPS = C::THREADS / 32, BLOCKS = C::EPI_WARPS * C::COLS / 32;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, tiles = p.tiles_m * p.tiles_n;
+    int turn = 0;
+    for (int w = p.work0 + blockIdx.x, i = 0; w < p.work1; w += gridDim.x, ++i) {
+        const unsigned mark = marks[i / 4] >> (i % 4 * 8) & 255u;
+        const int tile = w % tiles, z = w / tiles;
+        const int k_begin = z * p.k_split, k_end = min(p.K, k_begin + p.k_split);
+        for (int block = 0; mark != 0 && block < BLOCKS; ++block) {
+            const int e = block % C::EPI_WARPS;
+            const int row0 = (tile % p.tiles_m) * BM + e % 4 * 32;
+            const int col0 = (tile / p.tiles_m) * C::BN + e / 4 * C::COLS + block / C::EPI_WARPS * 32;
+            if ((mark >> e & 1u) == 0 || row0 >= p.M || col0 >= p.N || turn++ % WARPS != warp) continue;
+            float acc[4][8];
+            redo_block<AOp::kWalk == kByRow, BOp::kWalk == kByRow>(A, B, row0, p.M, col0, p.N, k_begin, k_end, buf, acc);
+            const int row = row0 + lane / 4 * 4, col = col0 + lane % 4 * 8;
+            for (int r = 0; r < 4; ++r) {
+                if (row + r >= p.M || col >= p.N) break;
+                typename Epi::State st = E.begin(row + r, col);
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    if (col + c >= p.N) break;
+                    const float v = r == 0 ? acc[0][c] : r == 1 ? acc[1][c] : r == 2 ? acc[2][c] : acc[3][c];
+                    if (p.splits > 1)
+                        p.partial[((int64_t)z * p.N + col + c) * p.M + row + r] = v;
+                    else
+                        E.store(st, col + c, v);
+                }
+            }
+        }
+    }
+}
+
 template <class T, int BN, class AOp, class BOp, class Epi>
 __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
     gemm_tcx_kernel(const __grid_constant__ AOp A, const __grid_constant__ BOp B,
-                    const __grid_constant__ Epi E, const Params p) {
+                    const __grid_constant__ Epi E, const __grid_constant__ Params p) {
     using C = Cfg<T, BN>;
     constexpr int PL = C::PL, STAGES = C::STAGES, PRODUCERS = C::PRODUCERS;
     extern __shared__ uint8_t smem_raw[];
@@ -715,7 +809,10 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
     uint64_t *acc_full = bars + 2 * STAGES, *acc_empty = bars + 2 * STAGES + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    int *table_a = reinterpret_cast<int *>(tmem_slot + 2), *table_b = table_a + kFewPatch;
+    volatile int *redo = reinterpret_cast<volatile int *>(tmem_slot + 2);   // any mark
+    int *table_a = reinterpret_cast<int *>(tmem_slot + 4), *table_b = table_a + kFewPatch;
+    // bit e of byte i: epilogue warp e left its block of this CTA's i-th tile out
+    unsigned *marks = reinterpret_cast<unsigned *>(table_b + kFewPatch);
 
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     constexpr int MMA_WARP = PRODUCERS / 32 + C::EPI_WARPS;
@@ -733,7 +830,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // The last tile's B rows beyond N are never staged: they start as zeros, so that the columns
-    // nobody stores do not look like sums to recompute.
+    // nobody stores do not look like sums to compute again.
     if (PL == 3 && p.N % BN != 0) {
         for (uint32_t i = tid; i < STAGES * PL * C::B_PLANE / 16; i += C::THREADS) {
             const uint32_t st = i / (PL * C::B_PLANE / 16), off = i % (PL * C::B_PLANE / 16);
@@ -741,6 +838,10 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
             st_shared_v4(tc::smem_u32(smem + st * C::STAGE + PL * C::A_PLANE) + off * 16, zero);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (PL == 3) {
+        if (tid == 0) *redo = 0;
+        if (tid < kMarks / 4) marks[tid] = 0;
     }
     if (warp == MMA_WARP) {
         tc::tmem_alloc(tc::smem_u32(tmem_slot), C::TMEM);
@@ -756,7 +857,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
     dependency_wait();
 
     const int tiles = p.tiles_m * p.tiles_n;
-    const int num_work = tiles * p.splits;
+    const int num_work = p.work1, work0 = p.work0 + blockIdx.x;
 
     if (warp < PRODUCERS / 32) {
         // ------------------------------------------------------------------ producers
@@ -764,7 +865,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
         constexpr int B_PER = BN * 8 / PRODUCERS < 1 ? 1 : BN * 8 / PRODUCERS;
         int stage = 0;
         uint32_t phase = 0;
-        for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
+        for (int w = work0; w < num_work; w += gridDim.x) {
             const int tile = w % tiles, z = w / tiles;
             const int m0 = (tile % p.tiles_m) * BM, n0 = (tile / p.tiles_m) * BN;
             const int k_begin = z * p.k_split, k_end = min(p.K, k_begin + p.k_split);
@@ -823,7 +924,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             bool ok = true;
-            for (int w = blockIdx.x; ok && w < num_work; w += gridDim.x) {
+            for (int w = work0; ok && w < num_work; w += gridDim.x) {
                 const int k_begin = (w / tiles) * p.k_split, k_end = min(p.K, k_begin + p.k_split);
                 for (int k0 = k_begin; k0 < k_end; k0 += BK) {
                     if (PL == 3 || k0 == k_begin) {
@@ -891,7 +992,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
         int acc = 0;
         uint32_t acc_phase = 0;
         bool ok = true;
-        for (int w = blockIdx.x; ok && w < num_work; w += gridDim.x) {
+        for (int w = work0; ok && w < num_work; w += gridDim.x) {
             const int tile = w % tiles, z = w / tiles;
             const int m0 = (tile % p.tiles_m) * BM, n0 = (tile / p.tiles_m) * BN;
             const int k_begin = z * p.k_split, k_end = min(p.K, k_begin + p.k_split);
@@ -932,22 +1033,20 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
             const int row = m0 + quarter * 32 + lane;
             const int col0 = n0 + col_base;
             const bool in = row < p.M;
-            // a sum that is not finite makes the row's columns take the exact path
-            float finite = 0.f;
+            // a sum that is not finite: the warp's block is left for redo_block
+            bool redo_it = false;
             if (PL == 3) {
+                float finite = 0.f;
 #pragma unroll
                 for (int j = 0; j < C::COLS; ++j) finite = fmaf(sum[j], 0.f, finite);
-            }
-            if (in && !(finite == 0.f)) {
-                typename Epi::State st = E.begin(row, col0);
-#pragma unroll 1
-                for (int col = col0; col < min(p.N, col0 + C::COLS); ++col) {
-                    const float v = recompute(A, B, row, col, k_begin, k_end);
-                    if (p.splits > 1)
-                        p.partial[((int64_t)z * p.N + col) * p.M + row] = v;
-                    else
-                        E.store(st, col, v);
+                redo_it = __any_sync(0xffffffffu, in && !(finite == 0.f));
+                if (redo_it && lane == 0) {
+                    const int i = (w - work0) / gridDim.x;
+                    atomicOr(marks + i / 4, 1u << (i % 4 * 8 + e));
+                    *redo = 1;
                 }
+            }
+            if (redo_it) {
             } else if (in && p.splits > 1) {
                 float *q = p.partial + ((int64_t)z * p.N + col0) * p.M + row;
 #pragma unroll
@@ -972,6 +1071,10 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
             while (tc::global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
         }
         tc::tmem_dealloc(tmem, C::TMEM);
+    }
+    if (PL == 3 && *redo && !*abort_flag) {
+        redo_marked<C, AOp, BOp, Epi>(A, B, E, p, marks, reinterpret_cast<float *>(smem) + warp * kRedoFloats);
+        __syncthreads();
     }
     if (Epi::kLastCtaAdds && p.arrivals != nullptr) {
         // every CTA has had one slice of one tile (grid = tiles * splits)
@@ -1057,9 +1160,14 @@ int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
         AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
         configured = true;
     }
-    const int64_t work = tiles * p.splits;
-    const int grid = (int)(work < dev->sm_count ? work : dev->sm_count);
-    AG_TRY(launch_dependent(dev, kernel, dim3((unsigned)grid), C::THREADS, C::SMEM, A, B, E, p));
+    const int64_t work = tiles * p.splits, most = (int64_t)kMarks * dev->sm_count;
+    for (int64_t w = 0; w < work; w += most) {   // one launch, but for f32 outputs of 2.4e9 values and more
+        p.work0 = (int)w;
+        p.work1 = (int)(C::PL == 1 || work - w < most ? work : w + most);
+        const int grid = (int)(work - w < dev->sm_count ? work - w : dev->sm_count);
+        AG_TRY(launch_dependent(dev, kernel, dim3((unsigned)grid), C::THREADS, C::SMEM, A, B, E, p));
+        if (C::PL == 1) break;
+    }
     if (p.splits > 1 && p.arrivals == nullptr) {
         AG_TRY(launch_dependent(dev, reduce_splits_kernel<Epi>, dim3((unsigned)ceil_div((int64_t)p.M * p.N, 256)), 256, 0,
                                 (const float *)p.partial, p.splits, p.M, p.N, FastDiv((uint32_t)p.M), E));

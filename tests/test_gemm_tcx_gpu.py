@@ -161,3 +161,60 @@ def test_few_rows_or_columns(dev, dtype, shape):
         bound = ref.abs() * 2.0 ** -8 + bound * 64   # as in test_product_vs_f64
     assert ((dev.dot(a, b).double() - ref).abs() <= bound).all()
     dev.wait()
+
+
+def _same_specials(got, want):
+    """want in float64 of small integers: finite values equal, infinities and NaNs in their places."""
+    want = want.to(torch.float32)
+    nan = torch.isnan(want)
+    assert torch.equal(torch.isnan(got), nan)
+    assert torch.equal(got[~nan], want[~nan])
+
+
+@pytest.mark.parametrize("layout", ["nn", "nt", "tn", "tt"])
+@pytest.mark.parametrize("shape", [
+    # gathered engine: several tiles per CTA; slices of k.  Packed: several tiles per pair, some cut in two; slices of k
+    (2561, 100, 2049), (130, 8003, 33), (3300, 1501, 3333), (1000, 20001, 130),
+])
+def test_f32_not_finite_blocks(dev, layout, shape):
+    """Sums that are not finite leave the pipeline of tiles alone: their blocks are computed after it, with
+    C's old values read once."""
+    m, k, n = shape
+    gen = torch.Generator(device=dev.torch_device).manual_seed(m)
+    ints = lambda r, c: torch.randint(-2, 3, (r, c), generator=gen, device=dev.torch_device).float()
+    a, b = ints(m, k), ints(k, n)
+    a[5, 7], a[m // 2, k - 1], a[m - 1, 0] = float("inf"), float("nan"), torch.finfo(torch.float32).max
+    b[k // 3, n - 1] = float("-inf")
+    b[0].clamp_(-1, 1)   # no overflow with the largest value
+    strided = lambda t, l: t if l == "n" else t.t().contiguous().t()
+    av, bv = strided(a, layout[0]), strided(b, layout[1])
+    want = a.double() @ b.double()
+    _same_specials(dev.dot(av, bv), want)
+    c = ints(m, n + 1)
+    want2 = 2 * want + 3 * c[:, 1:].double()
+    dev.gemm(2.0, av, bv, 3.0, c[:, 1:])
+    _same_specials(c[:, 1:], want2)
+    # every output at once
+    av[:, k // 2] = float("nan")
+    assert torch.isnan(dev.dot(av, bv)).all()
+    dev.wait()
+
+
+def test_f32_not_finite_weight_gradient(dev):
+    """180 tiles of 23,328 positions each on 148 SMs, without slices."""
+    bs, ic, hw, oc = 8, 512, 56, 640
+    gen = torch.Generator(device=dev.torch_device).manual_seed(1)
+    ints = lambda *s: torch.randint(-2, 3, s, generator=gen, device=dev.torch_device).float()
+    x, dy = ints(bs, ic, hw, hw), ints(bs, oc, hw - 2, hw - 2)
+
+    def want():
+        d = dy.double().transpose(0, 1).reshape(oc, -1)
+        taps = [d @ x[:, :, i:i + hw - 2, j:j + hw - 2].double().transpose(0, 1).reshape(ic, -1).t()
+                for i in range(3) for j in range(3)]
+        return torch.stack(taps, 2).view(oc, ic, 3, 3)
+
+    x[3, 100, 20, 20], x[0, 511, 55, 55], dy[1, 639, 0, 0] = float("nan"), float("inf"), float("-inf")
+    _same_specials(dev.conv2_backward_weight(x, dy, (3, 3)), want())
+    x.fill_(float("nan"))
+    assert torch.isnan(dev.conv2_backward_weight(x, dy, (3, 3))).all()
+    dev.wait()
