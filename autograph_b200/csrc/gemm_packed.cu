@@ -298,26 +298,37 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                     const uint32_t d = tmem_acc[acc];
                     const uint32_t a_base = smem_u32(smem + stage * STAGE);
                     const uint32_t b_base = a_base + PL * HALF_BYTES;
+                    auto desc_a = [&](int plane, int k) {
+                        return make_smem_desc(a_base + plane * a_plane + k * a_step, A_MN ? lbo : 0, 1024);
+                    };
+                    auto desc_b = [&](int plane, int k) {
+                        return make_smem_desc(b_base + plane * b_plane + k * b_step, B_MN ? lbo : 0, 1024);
+                    };
                     auto mma = [&](int pa, int pb, int k, bool add) {
-                        umma2_bf16(d, make_smem_desc(a_base + pa * a_plane + k * a_step, A_MN ? lbo : 0, 1024),
-                                   make_smem_desc(b_base + pb * b_plane + k * b_step, B_MN ? lbo : 0, 1024),
-                                   idesc, add ? 1u : 0u);
+                        umma2_bf16(d, desc_a(pa, k), desc_b(pb, k), idesc, add ? 1u : 0u);
                     };
                     if (PL == 1) {
 #pragma unroll
                         for (int k = 0; k < BK / 16; ++k) mma(0, 0, k, kb > wk.kb0 || k > 0);
                     } else {
-                        // the small partial products first, the leading ones last
+                        // the smallest partial products first, the leading ones last; the first of each
+                        // size takes 2^8 off the scale of what was added before
 #pragma unroll
                         for (int k = 0; k < BK / 16; ++k) {
                             mma(0, 2, k, k > 0);
                             mma(2, 0, k, true);
                             mma(1, 1, k, true);
+                        }
+                        umma2_bf16_shift8(d, desc_a(0, 0), desc_b(1, 0), idesc);
+                        mma(1, 0, 0, true);
+#pragma unroll
+                        for (int k = 1; k < BK / 16; ++k) {
                             mma(0, 1, k, true);
                             mma(1, 0, k, true);
                         }
+                        umma2_bf16_shift8(d, desc_a(0, 0), desc_b(0, 0), idesc);
 #pragma unroll
-                        for (int k = 0; k < BK / 16; ++k) mma(0, 0, k, true);
+                        for (int k = 1; k < BK / 16; ++k) mma(0, 0, k, true);
                     }
                     umma2_commit_multicast(smem_u32(&empty_bar[stage]), 3);
                     if (++stage == STAGES) {

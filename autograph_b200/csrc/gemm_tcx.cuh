@@ -10,11 +10,14 @@
 //   EPI warps    read finished accumulators from tensor memory and store through an epilogue
 //   last warp    issues tcgen05.mma
 //
-// f32 products.  A f32 value is written as the sum of three bf16 values (hi, mid, lo: 8 + 8 + 8
+// f32 products.  A f32 value is written as hi + 2^-8 mid + 2^-16 lo of three bf16 values (8 + 8 + 8
 // bits, the remainders exact), and a product as the six partial products down to 2^-16 of the
 // leading one (Henry, Tang, Heinecke, "Leveraging the bfloat16 artificial intelligence datatype
-// for higher-precision computations", 2019); what is dropped is below 2^-25 of a product, half
-// an ulp of the f32 product.  The tensor core adds with truncation, so an accumulator is read
+// for higher-precision computations", 2019); what is dropped is below 2^-24 of a product, an ulp
+// at most.  mid and lo are held scaled up, because bf16 ends at 2^-133: unscaled, a value below 2^-109
+// lost bits (1e-36 times 1e30 kept 15 of 24), scaled, every f32 value down to 2^-149 is exact (what is
+// dropped of a product with a subnormal one is below 2^-149 of the other operand).  The scales come off between groups of partial products of one size, by the shift of the accumulator
+// that tcgen05.mma can do.  The tensor core adds with truncation, so an accumulator is read
 // out after every 64 k and the 64-k sums are added in registers with round-to-nearest; within
 // 64 k the small partial products are accumulated first, which leaves four truncating additions
 // of full-size terms.  Uniform operands, relative 2-norm error against an f64 product: k = 128
@@ -76,16 +79,17 @@ __device__ __forceinline__ void fetch8(Vec8<__nv_bfloat16> &d, const __nv_bfloat
     }
 }
 
-// Bits whose upper halves are hi, mid and lo of an f32 value.  Rounding is half away from zero to 8
-// bits (the upper half of bits + 0x8000); both remainders are exact, of at most 16 and 8 bits.
+// Bits whose upper halves are hi, mid and lo of an f32 value (hi + 2^-8 mid + 2^-16 lo).  Rounding is half
+// away from zero to 8 bits (the upper half of bits + 0x8000); both remainders are exact, of at most 16
+// and 8 bits, and stay so times 2^8: each is at most 2^-8 of the value it is left from.
 // A NaN or an infinity, or a value whose hi rounds up to one, ends in a NaN: NaN - x and
 // inf - inf give the NaN 0x7fffffff, whose upper half stays a NaN in lo (only the additions of
 // 0x8000 can wrap one around).  Its outputs are NaN and are recomputed.
 __device__ __forceinline__ void split3(float v, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
     hi = __float_as_uint(v) + 0x8000u;
-    const float r = v - __uint_as_float(hi & 0xffff0000u);
+    const float r = (v - __uint_as_float(hi & 0xffff0000u)) * 256.f;
     mid = __float_as_uint(r) + 0x8000u;
-    lo = __float_as_uint(r - __uint_as_float(mid & 0xffff0000u));
+    lo = __float_as_uint((r - __uint_as_float(mid & 0xffff0000u)) * 256.f);
 }
 
 // Upper halves of two f32 words as one packed bf16 pair.
@@ -955,17 +959,19 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
                         for (int k = 0; k < BK / 16; ++k)
                             if (k < k_steps) tc::umma_bf16(d, da(0, k), db(0, k), idesc1, (k0 > k_begin || k > 0) ? 1u : 0u);
                     } else {
-                        // corrections first: column block 0 collects hi.mid, mid.hi, lo.hi, block 1
-                        // hi.lo and mid.mid; then the leading products into block 0
+                        // corrections first: column block 0 collects hi.mid and mid.hi (scale 2^8), block 1
+                        // hi.lo, mid.mid and lo.hi (scale 2^16); then the leading products into block 0,
+                        // whose scale the first of them takes off
 #pragma unroll
                         for (int k = 0; k < BK / 16; ++k) {
                             if (k >= k_steps) break;
                             tc::umma_bf16(d, da(0, k), db(1, k), idesc2, k > 0 ? 1u : 0u);   // b_mid, b_lo
                             tc::umma_bf16(d, da(1, k), db(0, k), idesc2, 1u);                // b_hi, b_mid
-                            tc::umma_bf16(d, da(2, k), db(0, k), idesc1, 1u);
+                            tc::umma_bf16(d + BN, da(2, k), db(0, k), idesc1, 1u);
                         }
+                        tc::umma_bf16_shift8(d, da(0, 0), db(0, 0), idesc1);
 #pragma unroll
-                        for (int k = 0; k < BK / 16; ++k)
+                        for (int k = 1; k < BK / 16; ++k)
                             if (k < k_steps) tc::umma_bf16(d, da(0, k), db(0, k), idesc1, 1u);
                     }
                     tc::umma_commit(tc::smem_u32(&empty_bar[stage]));
@@ -1017,7 +1023,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         float v = __uint_as_float(r0[j]);
-                        if (PL == 3) v = sum[c + j] + (v + __uint_as_float(r1[j]));
+                        if (PL == 3) v = sum[c + j] + fmaf(__uint_as_float(r1[j]), 0x1p-16f, v);
                         sum[c + j] = v;
                     }
                 }

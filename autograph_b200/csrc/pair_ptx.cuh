@@ -73,6 +73,17 @@ __device__ __forceinline__ void umma2_bf16(uint32_t d_tmem, uint64_t a_desc, uin
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// D = D * 2^-8 + A . B.
+__device__ __forceinline__ void umma2_bf16_shift8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, 1, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p, 8;\n"
+        "}\n" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc)
+        : "memory");
+}
 // One arrival on the barrier at the same offset in every CTA of `mask`, once all
 // tcgen05 operations issued so far by this thread have completed.
 __device__ __forceinline__ void umma2_commit_multicast(uint32_t bar, uint16_t mask) {

@@ -118,9 +118,12 @@ AG_API int ag_fill_zero(ag_device *dev, void *dptr, size_t bytes);
  * transposed view; never a copy).  bf16 inputs are multiplied and accumulated
  * in f32 and the result is rounded once (linalg.rs:244).  beta == 0 never
  * reads C.  Large-k, small-output products are split along k with f32 partial
- * sums and a fixed reduction order (deterministic).  f32 products of 3e7 and more multiply-adds
- * run on the tensor cores with every operand split into three bf16 values that add up to it
- * (f32-accurate: the error against an f64 product is below that of a chain of f32 FMAs). */
+ * sums and a fixed reduction order (deterministic).  Larger f32 products (from 2e6 multiply-adds when
+ * k is above 128, 3e7 below, 1e7 with fewer than 16 rows or columns) run on the tensor cores with every
+ * operand split into three scaled bf16 values that add up to it.  They are f32-accurate: the error
+ * against an f64 product is below that of a chain of f32 FMAs, over the whole range of normal f32
+ * operands; a subnormal operand counts with an error of up to 2^-149.  Outputs that are infinite or
+ * NaN are those of f32 FMAs. */
 AG_API int ag_gemm(ag_device *dev, ag_dtype dtype, int64_t m, int64_t k, int64_t n, float alpha,
                    const void *a, int64_t off_a, int64_t rsa, int64_t csa,
                    const void *b, int64_t off_b, int64_t rsb, int64_t csb,

@@ -218,3 +218,27 @@ def test_f32_not_finite_weight_gradient(dev):
     x.fill_(float("nan"))
     assert torch.isnan(dev.conv2_backward_weight(x, dy, (3, 3))).all()
     dev.wait()
+
+
+@pytest.mark.parametrize("shape", [(700, 300, 200), (2561, 100, 2049), (1000, 5001, 130), (2560, 641, 2050)])
+@pytest.mark.parametrize("layout", ["nn", "tn"])
+@pytest.mark.parametrize("tiny", [-100, -112, -120, -126, -135, -145])
+def test_f32_small_magnitudes(dev, shape, layout, tiny):
+    """Operands down to f32's smallest normal number keep all their bits when the other operand brings the
+    product back into range, whichever of the two is small; subnormal ones and sums count with an error of
+    one unit of 2^-149 (the products left out are below 2^-24 of a product only while the first eight bits
+    of an operand are a bf16 number)."""
+    m, k, n = shape
+    gen = torch.Generator(device=dev.torch_device).manual_seed(m)
+    rnd = lambda r, c, e: torch.ldexp(torch.rand((r, c), generator=gen, device=dev.torch_device) * 2 - 1,
+                                      torch.tensor(float(e), device=dev.torch_device))
+    strided = lambda t, l: t if l == "n" else t.t().contiguous().t()
+    for ea, eb in ((tiny, 100), (100, tiny)):
+        a, b = strided(rnd(m, k, ea), layout[0]), strided(rnd(k, n, eb), layout[1])
+        if tiny == -112:   # among ordinary values too
+            a[::3], b[:, ::5] = torch.ldexp(a[::3], torch.tensor(-20.0, device=dev.torch_device)), 2.0 ** -10
+        assert a.abs().max() > 0 and b.abs().max() > 0
+        err = (dev.dot(a, b).double() - a.double() @ b.double()).abs()
+        units = a.double().abs().sum(1, keepdim=True) + b.double().abs().sum(0, keepdim=True) + k
+        assert (err <= _f32_bound(a, b, k) + units * 2.0 ** -149).all()
+    dev.wait()
