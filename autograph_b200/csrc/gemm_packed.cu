@@ -6,8 +6,8 @@
 // Roles per CTA (320 threads): warp 0 = TMA producer of the CTA's own halves, warp 1 = MMA
 // issuer (leader) and tensor-memory allocation, warps 2..9 = epilogue, each 32 rows x 128
 // columns.  An f32 product reads the accumulator out after every 64 k and adds the 64-k sums
-// in registers (the arithmetic, and why, is described in gemm_tcx.cuh; so is what happens to sums that
-// are not finite); a bf16 product once per tile.
+// in registers, a bf16 product after every 1024 (the arithmetic, and why, is described in gemm_tcx.cuh; so is
+// what happens to sums that are not finite).
 //
 // The tile's rows run along the contiguous index of C (a row-major C is computed as
 // C^T = B^T . A^T), so a warp's store is 32 consecutive elements and needs no alignment.
@@ -281,8 +281,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                 const Work wk = decode(w, p);
                 const uint32_t idesc = make_idesc(A_MN, B_MN, TILE, wk.n_width);
                 const uint32_t b_plane = B_MN ? ATOM : wk.n_width / 2 * BK * 2;
+                int taken = 0;   // steps in this accumulator
                 for (int kb = wk.kb0; kb < wk.kb1; ++kb) {
-                    if (PL == 3 || kb == wk.kb0) {
+                    if (taken == 0) {
                         if (!mbar_wait(smem_u32(&acc_empty[acc]), acc_phase ^ 1, abort_flag)) {
                             atomicExch(p.status, 192);
                             ok = false;
@@ -309,7 +310,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                     };
                     if (PL == 1) {
 #pragma unroll
-                        for (int k = 0; k < BK / 16; ++k) mma(0, 0, k, kb > wk.kb0 || k > 0);
+                        for (int k = 0; k < BK / 16; ++k) mma(0, 0, k, taken > 0 || k > 0);
                     } else {
                         // the smallest partial products first, the leading ones last; the first of each
                         // size takes 2^8 off the scale of what was added before
@@ -335,7 +336,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                         stage = 0;
                         phase ^= 1;
                     }
-                    if (PL == 3 || kb + 1 == wk.kb1) {
+                    if (++taken == tcx::kAccSteps<PL> || kb + 1 == wk.kb1) {
+                        taken = 0;
                         umma2_commit_multicast(smem_u32(&acc_full[acc]), 3);
                         if (++acc == 2) {
                             acc = 0;
@@ -355,7 +357,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             const Work wk = decode(w, p);
             const int width = wk.n_width / 2;   // columns of this warp: 128, or 64 of a tail piece
             float sum[128];
-            const int steps = PL == 3 ? wk.kb1 - wk.kb0 : 1;
+            const int steps = (wk.kb1 - wk.kb0 + tcx::kAccSteps<PL> - 1) / tcx::kAccSteps<PL>;
             for (int s = 0; s < steps; ++s) {
                 if (!mbar_wait(smem_u32(&acc_full[acc]), acc_phase, abort_flag)) {
                     if (lane == 0) atomicExch(p.status, 194);

@@ -20,8 +20,10 @@
 // that tcgen05.mma can do.  The tensor core adds with truncation, so an accumulator is read
 // out after every 64 k and the 64-k sums are added in registers with round-to-nearest; within
 // 64 k the small partial products are accumulated first, which leaves four truncating additions
-// of full-size terms.  Uniform operands, relative 2-norm error against an f64 product: k = 128
-// 8e-8 (the FFMA kernel 1.1e-7), k = 1024 1.1e-7 (5.7e-7), k = 4096 1.7e-7 (1.2e-6).  The split of
+// of full-size terms.  A bf16 accumulator takes 1024 k, 64 truncating additions: over all of a long k
+// those add up (positive operands, k = 100,001: 6e-4 of a value, always towards zero; read out like
+// this 2e-7, in the same time).  Uniform f32 operands, relative 2-norm error against an f64 product:
+// k = 128 8e-8 (the FFMA kernel 1.1e-7), k = 1024 1.1e-7 (5.7e-7), k = 4096 1.7e-7 (1.2e-6).  The split of
 // an infinity, or of a value that rounds up to one, is not usable: blocks of outputs with a sum
 // that is infinite or NaN are left out and computed with FFMAs from the f32 operands when the
 // CTA's tiles are done (redo_block).
@@ -39,6 +41,10 @@ namespace tcx {
 constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int ROW_BYTES = BK * 2;
+
+// 64-k steps that one accumulator takes before it is read out and added in registers.
+template <int PL>
+constexpr int kAccSteps = PL == 3 ? 1 : 16;
 
 template <class T>
 struct Planes;
@@ -930,8 +936,9 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
             bool ok = true;
             for (int w = work0; ok && w < num_work; w += gridDim.x) {
                 const int k_begin = (w / tiles) * p.k_split, k_end = min(p.K, k_begin + p.k_split);
+                int taken = 0;   // steps in this accumulator
                 for (int k0 = k_begin; k0 < k_end; k0 += BK) {
-                    if (PL == 3 || k0 == k_begin) {
+                    if (taken == 0) {
                         if (!tc::mbar_wait(tc::smem_u32(&acc_empty[acc]), acc_phase ^ 1, abort_flag)) {
                             atomicExch(p.status, 182);
                             ok = false;
@@ -957,7 +964,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
                     if (PL == 1) {
 #pragma unroll
                         for (int k = 0; k < BK / 16; ++k)
-                            if (k < k_steps) tc::umma_bf16(d, da(0, k), db(0, k), idesc1, (k0 > k_begin || k > 0) ? 1u : 0u);
+                            if (k < k_steps) tc::umma_bf16(d, da(0, k), db(0, k), idesc1, (taken > 0 || k > 0) ? 1u : 0u);
                     } else {
                         // corrections first: column block 0 collects hi.mid and mid.hi (scale 2^8), block 1
                         // hi.lo, mid.mid and lo.hi (scale 2^16); then the leading products into block 0,
@@ -979,7 +986,8 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
                         stage = 0;
                         phase ^= 1;
                     }
-                    if (PL == 3 || k0 + BK >= k_end) {
+                    if (++taken == kAccSteps<PL> || k0 + BK >= k_end) {
+                        taken = 0;
                         tc::umma_commit(tc::smem_u32(&acc_full[acc]));
                         if (++acc == 2) {
                             acc = 0;
@@ -1002,7 +1010,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
             const int tile = w % tiles, z = w / tiles;
             const int m0 = (tile % p.tiles_m) * BM, n0 = (tile / p.tiles_m) * BN;
             const int k_begin = z * p.k_split, k_end = min(p.K, k_begin + p.k_split);
-            const int steps = PL == 3 ? (k_end - k_begin + BK - 1) / BK : 1;
+            const int steps = (k_end - k_begin + kAccSteps<PL> * BK - 1) / (kAccSteps<PL> * BK);
             float sum[C::COLS];
 #pragma unroll
             for (int j = 0; j < C::COLS; ++j) sum[j] = 0.f;
@@ -1023,8 +1031,8 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         float v = __uint_as_float(r0[j]);
-                        if (PL == 3) v = sum[c + j] + fmaf(__uint_as_float(r1[j]), 0x1p-16f, v);
-                        sum[c + j] = v;
+                        if (PL == 3) v = fmaf(__uint_as_float(r1[j]), 0x1p-16f, v);
+                        sum[c + j] += v;
                     }
                 }
                 tc::tc_fence_before();

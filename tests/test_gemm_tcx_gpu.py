@@ -21,6 +21,12 @@ def _f32_bound(av, bv, k):
     return s * (5 * 2.0 ** -23 + 2.0 ** -24 + 2 * (k / 64 + 1) * 2.0 ** -24)
 
 
+def _bf16_bound(s, ref, k):
+    """S = sum |a||b| again: in every 1024-k block 64 additions that truncate to 24 bits (2 more for those
+    within one instruction), the block sums and k slices added with a rounding each, one bf16 store."""
+    return ref.abs() * 2.0 ** -8 + s * (66 * 2.0 ** -23 + 2 * (k / 1024 + 1) * 2.0 ** -24)
+
+
 @pytest.mark.parametrize("layout", ["nn", "nt", "tn", "tt"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape", [
@@ -45,7 +51,7 @@ def test_product_vs_f64(dev, dtype, layout, shape):
     err = (c.double() - ref).abs()
     bound = _f32_bound(av, bv, k)
     if dtype == torch.bfloat16:
-        bound = ref.abs() * 2.0 ** -8 + bound * 64   # one bf16 store; truncating sums over all k
+        bound = _bf16_bound(av.double().abs() @ bv.double().abs(), ref, k)
     assert (err <= bound).all()
     # alpha, beta and a view of C, exact on small integers
     ai, bi = (torch.randint(-2, 3, t.shape, generator=gen, device=dev.torch_device).to(dtype) for t in (a, b))
@@ -105,7 +111,7 @@ def test_convolution_vs_f64(dev, dtype, case):
     for g, ref, s, k in zip(got, (y, dx, dw), (ya, dxa, dwa), ks):
         bound = s * (5 * 2.0 ** -23 + 2.0 ** -24 + 2 * (k / 64 + 1) * 2.0 ** -24)   # as in _f32_bound
         if dtype == torch.bfloat16:
-            bound = ref.abs() * 2.0 ** -8 + bound * 64
+            bound = _bf16_bound(s, ref, k)
         assert ((g.double() - ref).abs() <= bound).all()
     dw2 = dev.conv2_backward_weight(x, dy, f, beta=1.0, dw=torch.ones_like(w), **kw)
     assert ((dw2.double() - dw - 1).abs() <= (bound * 1.01 + (dw.abs() + 1) * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23))).all()
@@ -158,7 +164,7 @@ def test_few_rows_or_columns(dev, dtype, shape):
     ref = a.double() @ b.double()
     bound = _f32_bound(a, b, k)
     if dtype == torch.bfloat16:
-        bound = ref.abs() * 2.0 ** -8 + bound * 64   # as in test_product_vs_f64
+        bound = _bf16_bound(a.double().abs() @ b.double().abs(), ref, k)
     assert ((dev.dot(a, b).double() - ref).abs() <= bound).all()
     dev.wait()
 
@@ -241,4 +247,36 @@ def test_f32_small_magnitudes(dev, shape, layout, tiny):
         err = (dev.dot(a, b).double() - a.double() @ b.double()).abs()
         units = a.double().abs().sum(1, keepdim=True) + b.double().abs().sum(0, keepdim=True) + k
         assert (err <= _f32_bound(a, b, k) + units * 2.0 ** -149).all()
+    dev.wait()
+
+
+def _mean_signed(got, ref):
+    return float(((got.double() - ref) / ref).mean())
+
+
+@pytest.mark.parametrize("shape", [(1601, 100001, 1603), (1601, 3001, 1603), (130, 100001, 67)])
+def test_bf16_long_positive_sums(dev, shape):
+    """Sums of one sign over a long k: the truncating additions of an accumulator (64, half an ulp of 2^-23
+    each on average) leave no more than 4e-6 towards zero; the rest of the limit is what the stores' roundings,
+    whose spacing the sums' spread does not average out, show with FP32 arithmetic (2e-5)."""
+    m, k, n = shape
+    gen = torch.Generator(device=dev.torch_device).manual_seed(k)
+    rnd = lambda r, c: torch.rand((r, c), generator=gen, device=dev.torch_device)
+    a, b = (rnd(m, k) * (1 + rnd(m, 1))).bfloat16(), rnd(k, n).bfloat16()
+    assert abs(_mean_signed(dev.dot(a, b), a.double() @ b.double())) <= 4e-5
+    dev.wait()
+
+
+def test_bf16_long_positive_weight_gradient(dev):
+    """135 tiles of 147,456 positions each, without slices."""
+    bs, ic, o, oc = 64, 128, 48, 640
+    gen = torch.Generator(device=dev.torch_device).manual_seed(7)
+    rnd = lambda *s: torch.rand(s, generator=gen, device=dev.torch_device)
+    x, dy = rnd(bs, ic, 2 * o + 1, 2 * o + 1).bfloat16(), (rnd(bs, oc, o, o) * (1 + rnd(1, oc, 1, 1))).bfloat16()
+    dw = dev.conv2_backward_weight(x, dy, (3, 3), stride=(2, 2))
+    d = dy.double().transpose(0, 1).reshape(oc, -1)
+    for i in range(3):
+        for j in range(3):
+            tap = x[:, :, i:i + 2 * o - 1:2, j:j + 2 * o - 1:2].double().transpose(0, 1).reshape(ic, -1)
+            assert abs(_mean_signed(dw[:, :, i, j], d @ tap.t())) <= 4e-5
     dev.wait()
