@@ -27,6 +27,7 @@ namespace packed {
 
 using namespace tc;
 using namespace tc::pair;
+using tcx::Planes;
 
 constexpr int TILE = 256;      // per pair, both ways
 constexpr int BK = 64;
@@ -541,27 +542,60 @@ static int packed_map(CUtensorMap *map, const __nv_bfloat16 *base, int inner, in
     return make_tmap_bf16(map, base, 3, dims, strides, box);
 }
 
+// One operand's copy; returns the bytes of its planes.
+template <class T>
+static int64_t plan(PackJob<T> *j, const T *src, int rows, int k, int64_t s_row, int64_t s_k) {
+    const bool mn = s_k != 1;
+    j->src = src;
+    j->inner = mn ? rows : k;
+    j->outer = mn ? k : rows;
+    j->stride = mn ? s_k : s_row;
+    j->pitch = (j->inner + 7) / 8 * 8;
+    j->plane = (int64_t)j->pitch * j->outer;
+    j->div_words = FastDiv((uint32_t)(j->pitch / 2));
+    return (j->plane * Planes<T>::N * 2 + 1023) / 1024 * 1024;
+}
+
+// Planes of one launch.  Larger products are cut into blocks of rows and columns, whose operands are
+// copied in turn: 24,576^3 f32 (7.2 GB of planes) runs in two blocks at the rate of 16,384^3 in one (129 ms, 34 ms).
+constexpr int64_t kMostPlanes = 4ll << 30;
+
+template <class T>
+static int64_t planes(int M, int N, int K, int64_t p_k, int64_t q_k) {
+    PackJob<T> j;
+    return plan<T>(&j, nullptr, M, K, 1, p_k) + plan<T>(&j, nullptr, N, K, 1, q_k);
+}
+
+template <class T>
+bool reserve(ag_device *dev, int M, int N, int K, int64_t p_k, int64_t q_k) {
+    const int64_t all = planes<T>(M, N, K, p_k, q_k);
+    // the smallest blocks there are
+    if (planes<T>(M < 2 * TILE ? M : 2 * TILE - 1, N < 2 * TILE ? N : 2 * TILE - 1, K, p_k, q_k) > kMostPlanes) return false;
+    // and at most one tile per pair of f32 sums of slices
+    const int64_t bytes = (all < kMostPlanes ? all : kMostPlanes) + (int64_t)sizeof(float) * TILE * TILE * (dev->sm_count / 2);
+    void *ws;
+    return engine_scratch(dev, (size_t)bytes, &ws) == AG_OK;
+}
+
 template <class T>
 int gemm(ag_device *dev, int M, int N, int K, const T *p, int64_t p_row, int64_t p_k, const T *q,
          int64_t q_row, int64_t q_k, float alpha, float beta, T *c, int64_t ldc, const T *bias,
          bool relu) {
-    constexpr int PL = sizeof(T) == 4 ? 3 : 1;
+    if (planes<T>(M, N, K, p_k, q_k) > kMostPlanes) {
+        const int longer = M >= N ? M : N, h = (int)ceil_div(longer / 2, TILE) * TILE;
+        if (M >= N) {
+            AG_TRY(gemm<T>(dev, h, N, K, p, p_row, p_k, q, q_row, q_k, alpha, beta, c, ldc, bias, relu));
+            return gemm<T>(dev, M - h, N, K, p + h * p_row, p_row, p_k, q, q_row, q_k, alpha, beta, c + h, ldc,
+                           bias != nullptr ? bias + h : nullptr, relu);
+        }
+        AG_TRY(gemm<T>(dev, M, h, K, p, p_row, p_k, q, q_row, q_k, alpha, beta, c, ldc, bias, relu));
+        return gemm<T>(dev, M, N - h, K, p, p_row, p_k, q + h * q_row, q_row, q_k, alpha, beta, c + h * ldc, ldc, bias, relu);
+    }
+    constexpr int PL = Planes<T>::N;
     const bool a_mn = p_k != 1, b_mn = q_k != 1;
     PackJob<T> ja, jb;
-    auto plan = [](PackJob<T> *j, const T *src, bool mn, int rows, int k, int64_t s_row, int64_t s_k) {
-        j->src = src;
-        j->inner = mn ? rows : k;
-        j->outer = mn ? k : rows;
-        j->stride = mn ? s_k : s_row;
-        j->pitch = (j->inner + 7) / 8 * 8;
-        j->plane = (int64_t)j->pitch * j->outer;
-        j->div_words = FastDiv((uint32_t)(j->pitch / 2));
-        return (j->plane * PL * 2 + 1023) / 1024 * 1024;
-    };
-    const int64_t a_bytes = plan(&ja, p, a_mn, M, K, p_row, p_k);
-    const int64_t b_bytes = plan(&jb, q, b_mn, N, K, q_row, q_k);
+    const int64_t a_bytes = plan<T>(&ja, p, M, K, p_row, p_k), b_bytes = plan<T>(&jb, q, N, K, q_row, q_k);
     const int64_t words = (ja.plane > jb.plane ? ja.plane : jb.plane) / 2;
-    AG_REQUIRE(words < (1ll << 31) - (1 << 22), AG_ERR_LIMIT, "operand beyond 2^32 elements");
 
     Params<T> a;
     a.M = M; a.N = N; a.K = K;
@@ -629,6 +663,8 @@ int gemm(ag_device *dev, int M, int N, int K, const T *p, int64_t p_row, int64_t
     return AG_OK;
 }
 
+template bool reserve<float>(ag_device *, int, int, int, int64_t, int64_t);
+template bool reserve<__nv_bfloat16>(ag_device *, int, int, int, int64_t, int64_t);
 template int gemm<float>(ag_device *, int, int, int, const float *, int64_t, int64_t, const float *,
                          int64_t, int64_t, float, float, float *, int64_t, const float *, bool);
 template int gemm<__nv_bfloat16>(ag_device *, int, int, int, const __nv_bfloat16 *, int64_t, int64_t,

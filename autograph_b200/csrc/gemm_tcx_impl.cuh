@@ -44,9 +44,9 @@ int gemm_strided(ag_device *dev, int m, int k, int n, float alpha, const T *a, i
     // so a row-major C is computed as C^T = B^T . A^T.
     const bool a_ok = rsa == 1 || csa == 1, b_ok = rsb == 1 || csb == 1;
     if (a_ok && b_ok && packed_worth(m, k, n)) {
-        if (csc == 1)
+        if (csc == 1 && packed::reserve<T>(dev, n, m, k, rsb, csa))
             return packed::gemm<T>(dev, n, m, k, b, csb, rsb, a, rsa, csa, alpha, beta, c, rsc, nullptr, false);
-        if (rsc == 1)
+        if (csc != 1 && rsc == 1 && packed::reserve<T>(dev, m, n, k, csa, rsb))
             return packed::gemm<T>(dev, m, n, k, a, rsa, csa, b, csb, rsb, alpha, beta, c, csc, nullptr, false);
     }
     if (csc == 1 && rsc != 1)
@@ -57,7 +57,7 @@ int gemm_strided(ag_device *dev, int m, int k, int n, float alpha, const T *a, i
 template <class T>
 int dense(ag_device *dev, const T *x, int bs, int inputs, const T *w, int outputs, const T *bias,
           bool relu, T *y) {
-    if (packed_worth(bs, inputs, outputs))
+    if (packed_worth(bs, inputs, outputs) && packed::reserve<T>(dev, outputs, bs, inputs, outputs, 1))
         return packed::gemm<T>(dev, outputs, bs, inputs, w, 1, outputs, x, inputs, 1, 1.f, 0.f, y, outputs,
                                bias, relu);
     const DenseOut<T> E{y, outputs, bias, relu};

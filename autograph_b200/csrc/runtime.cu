@@ -38,7 +38,17 @@ static int grow_block(ag_device *dev, void **block, size_t *have, size_t bytes, 
     size_t want = *have ? *have * 2 : floor;
     if (want < bytes) want = bytes + bytes / 4;
     void *fresh = nullptr;
-    AG_CUDA_TRY(cudaMalloc(&fresh, want));
+    // A caller may be capturing the stream: the allocation itself is not part of the graph.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    AG_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+    cudaError_t e = cudaMalloc(&fresh, want);
+    if (e == cudaErrorMemoryAllocation && want > bytes) {
+        cudaGetLastError();
+        want = bytes;
+        e = cudaMalloc(&fresh, want);
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    AG_CUDA_TRY(e);
     if (*block) dev->retired.push_back(*block);
     *block = fresh;
     *have = want;
