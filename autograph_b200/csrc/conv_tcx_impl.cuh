@@ -38,10 +38,10 @@ static ConvMap conv_map(int64_t channels, int64_t sh, int64_t sw, int64_t gh, in
 template <class T>
 __global__ void repack_kernel(const T *w, T *out, int total, int channels, int cp, int s_row, int s_c,
                               FastDiv div_k, FastDiv div_cp) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= total) return;
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= (uint32_t)total) return;
     uint32_t row, k, tap, c;
-    div_k.divmod((uint32_t)i, row, k);
+    div_k.divmod(i, row, k);
     div_cp.divmod(k, tap, c);
     out[i] = (int)c < channels ? w[(int)row * s_row + (int)c * s_c + (int)tap] : from_f32<T>(0.f);
 }
@@ -68,9 +68,11 @@ static int patches_times_filters(ag_device *dev, const T *src, const ConvMap &ma
 
 // Whether a convolution's patches are better indexed by (channel, tap) than by (tap, channel padded to
 // eight): the padding costs more than the table look-ups (6 channels: 8 / 6 of 4 instructions
-// per element against 6).
+// per element against 6).  The table packs an offset of at most 26 bits and a sign with the tap; a tap that
+// meets the image from far into the padding is at an offset beyond the channel's plane.
 static bool few_channels(const ConvMap &g) {
-    return g.cp * 10 > g.channels * 14 && g.channels * g.ff <= kFewPatch && (int64_t)g.channels * g.sh * g.sw < (1 << 26);
+    const int64_t furthest = (int64_t)g.channels * g.sh * g.sw + (int64_t)(g.fh - 1) * g.dil_h * g.sw + (int64_t)(g.fw - 1) * g.dil_w;
+    return g.cp * 10 > g.channels * 14 && g.channels * g.ff <= kFewPatch && furthest < (1 << 26);
 }
 
 template <class T>
@@ -92,10 +94,10 @@ template <class T>
 __global__ void __launch_bounds__(256)
     taps_to_image_kernel(const float *col, T *dx, ConvMap g, int grid_hw, int64_t positions,
                          int total, FastDiv div_hw, FastDiv div_w, FastDiv div_c) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= total) return;
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= (uint32_t)total) return;
     uint32_t plane, r, y, x, b, c;
-    div_hw.divmod((uint32_t)i, plane, r);
+    div_hw.divmod(i, plane, r);
     div_w.divmod(r, y, x);
     div_c.divmod(plane, b, c);
     const float *q = col + (int64_t)c * g.ff * positions + (int64_t)b * grid_hw;

@@ -7,6 +7,9 @@
 namespace ag {
 namespace tcx {
 
+// The slices' ends are ints and round k up.
+constexpr int64_t kMostK = 1ll << 30;
+
 static bool enabled() {
     static const bool v = []() {
         const char *e = getenv("AG_TCX");
@@ -26,7 +29,7 @@ static bool enabled() {
 // Beyond k = 128, where the SIMT kernels have no form that stages all of k at once, slices of k win much earlier: f32 16 x
 // 1056 x 1088 12.5 and 8.7, 32 x 800 x 64 10.2 and 8.4; bf16 88 x 211 x 97 23 and 8.3, 16 x 496 x 144 17 and 8.3.
 bool gemm_worth(ag_dtype dtype, int64_t m, int64_t k, int64_t n) {
-    if (!enabled() || k < (dtype == AG_F32 ? 40 : 32)) return false;
+    if (!enabled() || k >= kMostK || k < (dtype == AG_F32 ? 40 : 32)) return false;
     const double macs = (double)m * (double)n * (double)k;
     if (m < 16 || n < 16) return macs >= 1e7 && k >= (n < 16 ? 1024 : 64);
     if (k > 128) return macs >= (dtype == AG_F32 ? 2e6 : 3e5);
@@ -43,6 +46,9 @@ bool packed_worth(int64_t m, int64_t k, int64_t n) {
     return m >= 128 && n >= 128 && k >= 64 && macs >= 1.8e9 && macs * (double)k >= 1.2e12;
 }
 
+// The filters are also counted with their channels padded to eight, in an int (repack_kernel).
+static bool filters_fit(int64_t patch, int64_t cols, int64_t taps) { return (patch + 7 * taps) * cols < (1ll << 31); }
+
 // patch = channels x taps.  Against the SIMT engine, us here and there (f32 unless said):
 //   1024 and more: here.  Below, by what the SIMT tiles are good at:
 //   96 columns x 9 (203 x 41 x 41 / 2): 35 and 31, bf16 35 and 52;  32 x 9 (254 x 55 x 55): 124 and 148;
@@ -50,7 +56,8 @@ bool packed_worth(int64_t m, int64_t k, int64_t n) {
 //   16 x 27 (233 x 48 x 48): 77 and 59;  6 x 9 (116 x 35 x 35): 20 and 8;
 //   1.8e6 multiply-adds (32 x 27, 21 x 10 x 10): 7 and 4.
 bool conv_worth(ag_dtype dtype, int64_t patch, int64_t cols, int64_t positions, const ag_conv2_options *o) {
-    if (!enabled() || o->filter[0] * o->filter[1] > 32) return false;
+    const int64_t taps = (int64_t)o->filter[0] * o->filter[1];
+    if (!enabled() || taps > 32 || !filters_fit(patch, cols, taps)) return false;
     const int64_t macs = positions * patch * cols;
     if (patch * cols >= 1024) return macs >= 2000000;
     if (macs < 3000000) return false;
@@ -61,13 +68,14 @@ bool conv_worth(ag_dtype dtype, int64_t patch, int64_t cols, int64_t positions, 
 // The input gradient, whose engine has a form for few columns (SIMT engine: 1 <- 16 5x5 177 us, 3 <- 32 3x3 on
 // 21 x 10 x 10 60 us here 10, 1 <- 6 3x3 on 116 x 37 x 37 51 us here 24).
 bool conv_input_worth(int64_t patch, int64_t cols, int64_t positions, const ag_conv2_options *o) {
-    return enabled() && o->filter[0] * o->filter[1] <= 32 && positions * patch * cols >= 1000000;
+    const int64_t taps = (int64_t)o->filter[0] * o->filter[1];
+    return enabled() && taps <= 32 && filters_fit(patch, cols, taps) && positions * patch * cols >= 1000000;
 }
 
 // The weight gradient: 1 -> 32 3x3 (254 x 55 x 55) 148 us here and 276, 6 -> 6 3x3 (84 x 60 x 60) 57 and 170; small ones
 // (1.1e6 multiply-adds) 11 and 12.
 bool conv_weight_worth(ag_dtype, int64_t patch, int64_t oc, int64_t positions, const ag_conv2_options *o) {
-    return enabled() && o->filter[0] * o->filter[1] <= 32 && positions * patch * oc >= 1000000;
+    return enabled() && (int64_t)o->filter[0] * o->filter[1] <= 32 && positions < kMostK && positions * patch * oc >= 1000000;
 }
 
 template int gemm_strided<float>(ag_device *, int, int, int, float, const float *, int64_t, int64_t,
