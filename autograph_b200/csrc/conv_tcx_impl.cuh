@@ -55,10 +55,11 @@ static int patches_times_filters(ag_device *dev, const T *src, const ConvMap &ma
     // One wave of tiles and up to 18 k steps of an input gradient, whose neighbouring rows are neighbouring
     // filters: read in place at the copy's device time, without its launch (forward, 5 x 64 x 22 x 22 -> 128:
     // 27 us in place, 19 copied; input gradient 21.7 and 21.5; 50 steps of 128 channels 5x5 190 and 87).
-    if (s_row < s_c && K <= 18 * BK && ceil_div(M, BM) * ceil_div(N, 64) <= dev->sm_count)
-        return gemm<T>(dev, M, N, K, ConvRows<T>{src, map, M}, FilterRows<T>{w, s_row, s_c, map.channels, map.div_cp}, E);
+    // So are they where there is no room for the copy.
     void *ws = nullptr;
-    AG_TRY(staging(dev, (size_t)total * sizeof(T), &ws));
+    if ((s_row < s_c && K <= 18 * BK && ceil_div(M, BM) * ceil_div(N, 64) <= dev->sm_count) ||
+        staging(dev, (size_t)total * sizeof(T), &ws) != AG_OK)
+        return gemm<T>(dev, M, N, K, ConvRows<T>{src, map, M}, FilterRows<T>{w, s_row, s_c, map.channels, map.div_cp}, E);
     T *packed = (T *)ws;
     repack_kernel<T><<<(unsigned)ceil_div(total, 256), 256, 0, dev->stream>>>(
         w, packed, total, map.channels, map.cp, s_row, s_c, FastDiv((uint32_t)K), map.div_cp);
@@ -88,6 +89,8 @@ int conv_forward(ag_device *dev, const T *x, int64_t bs, int64_t ic, int64_t ih,
     }
     return patches_times_filters<T>(dev, x, map, M, w, N, (int)ic * ff, ff, E);
 }
+
+constexpr int64_t kTapSums = 1ll << 28;   // f32 values
 
 // dx from the products with every tap: col[c * ff + tap][position of dy] -> dx[b][c][y][x].
 template <class T>
@@ -134,20 +137,25 @@ int conv_backward_input(ag_device *dev, const T *w, int64_t oc, int64_t ic, cons
     const int taps_n = N * ff;
     const double by_patches = 1.7 * (double)ceil_div((int64_t)ff * map.cp, 64);
     const double by_taps = 1.7 * (double)(ceil_div(oc, 64) * ceil_div(taps_n, 128)) + 0.03 * taps_n;
-    const int64_t positions = bs * oh * ow;
-    if (taps_n <= 128 && 1.3 * by_taps < by_patches && positions * taps_n < (1ll << 31)) {
-        void *ws = nullptr;
-        AG_TRY(staging(dev, sizeof(float) * (size_t)(positions * taps_n), &ws));
+    // As many images at a time as have 1 GiB of sums per tap; without room for those, by patches.
+    const int64_t image = oh * ow * taps_n, at_once = image < kTapSums ? kTapSums / image : 1;
+    const int64_t images = at_once < bs ? at_once : bs;
+    void *ws = nullptr;
+    if (taps_n <= 128 && 1.3 * by_taps < by_patches && image < (1ll << 31) &&
+        staging(dev, sizeof(float) * (size_t)(images * image), &ws) == AG_OK) {
         float *col = (float *)ws;
         ag_conv2_options point = {{1, 1}, {0, 0}, {1, 1}, {1, 1}};
-        AG_TRY(gemm<T>(dev, (int)positions, taps_n, (int)oc,
-                       ConvRows<T>{dy, conv_map(oc, oh, ow, oh, ow, &point, false), (int)positions},
-                       strided<kByRow>(w, 1, taps_n, taps_n), StridedOut<float>{col, 1, positions, 1.f, 0.f}));
-        const int total = (int)(bs * ic * ih * iw);
-        taps_to_image_kernel<T><<<(unsigned)ceil_div(total, 256), 256, 0, dev->stream>>>(
-            col, dx, map, (int)(oh * ow), positions, total, FastDiv((uint32_t)(ih * iw)),
-            FastDiv((uint32_t)iw), FastDiv((uint32_t)ic));
-        AG_CHECK_LAUNCH();
+        for (int64_t b = 0; b < bs; b += images) {
+            const int64_t n = images < bs - b ? images : bs - b, positions = n * oh * ow;
+            AG_TRY(gemm<T>(dev, (int)positions, taps_n, (int)oc,
+                           ConvRows<T>{dy + b * oc * oh * ow, conv_map(oc, oh, ow, oh, ow, &point, false), (int)positions},
+                           strided<kByRow>(w, 1, taps_n, taps_n), StridedOut<float>{col, 1, positions, 1.f, 0.f}));
+            const int total = (int)(n * ic * ih * iw);
+            taps_to_image_kernel<T><<<(unsigned)ceil_div(total, 256), 256, 0, dev->stream>>>(
+                col, dx + b * ic * ih * iw, map, (int)(oh * ow), positions, total, FastDiv((uint32_t)(ih * iw)),
+                FastDiv((uint32_t)iw), FastDiv((uint32_t)ic));
+            AG_CHECK_LAUNCH();
+        }
         return AG_OK;
     }
     NchwOut<T> E{dx, nullptr, N, (int)(ih * iw), FastDiv((uint32_t)(ih * iw)), false};

@@ -1,6 +1,10 @@
-"""GPU: convolutions whose index arithmetic is near the ends of 32 bits."""
+"""GPU: convolutions whose index arithmetic is near the ends of 32 bits, and scratch that is bounded or not to be
+had."""
 import pytest
 import torch
+import torch.nn.functional as F
+
+import autograph_b200 as ag
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +44,50 @@ def test_filters_beyond_2_31_elements(dev):
     for i in (0, 1, oc // 2, 58254, 58255, oc - 1):   # 2^31 lies in row 58,254
         assert torch.equal(dw[i], x.view(-1) * dy[0, i, 0, 0])
     dev.wait()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_input_gradient_in_batch_slices(dev, dtype):
+    """Sums per tap beyond 1 GiB are made for some of the images at a time, the last slice short."""
+    bs, ic, oc, hw = 2271, 6, 64, 50   # 2157 images and 114
+    gen = torch.Generator(device=dev.torch_device).manual_seed(3)
+    ints = lambda *s: torch.randint(-2, 3, s, generator=gen, device=dev.torch_device).to(dtype)
+    w, dy = ints(oc, ic, 3, 3), ints(bs, oc, hw - 2, hw - 2)
+    dx = dev.conv2_backward_input(w, dy, (hw, hw))
+    at = torch.tensor([0, 1000, 2156, 2157, 2270], device=dev.torch_device)
+    want = F.conv_transpose2d(dy[at].double(), w.double())
+    assert torch.equal(dx[at], want.to(dtype))   # sums of 576 products of at most 4 in absolute value
+    assert torch.equal(dx[2200:], dev.conv2_backward_input(w, dy[2200:], (hw, hw)))
+    dev.wait()
+
+
+@pytest.mark.parametrize("channels", [(6, 128), (512, 512)])
+def test_no_room_for_scratch(dev, channels):
+    """With no memory for the sums per tap (few input channels) or for the copy of the filters the other forms
+    run."""
+    ic, oc = channels
+    bs, hw = (512, 40) if ic == 6 else (64, 32)
+    gen = torch.Generator(device=dev.torch_device).manual_seed(4)
+    ints = lambda *s: torch.randint(-2, 3, s, generator=gen, device=dev.torch_device).float()
+    x, w = ints(bs, ic, hw, hw), ints(oc, ic, 3, 3)
+    dy = ints(bs, oc, hw - 2, hw - 2)
+
+    def run(d):
+        return d.conv2_forward(x, w), d.conv2_backward_input(w, dy, (hw, hw))
+
+    want = run(dev)   # and the kernels are loaded
+    dev.wait()
+    fresh = ag.Device(0)
+    torch.cuda.set_stream(fresh.stream)
+    room = [torch.empty_like(t) for t in want]
+    torch.cuda.synchronize()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - (40 << 20 if ic == 6 else 6 << 20), dtype=torch.uint8,
+                      device=dev.torch_device)
+    del room   # the outputs' memory
+    got = run(fresh)
+    fresh.wait()
+    del hog
+    torch.cuda.empty_cache()
+    assert all(torch.equal(g, t) for g, t in zip(got, want))
+    fresh.close()
+    torch.cuda.set_stream(dev.stream)
