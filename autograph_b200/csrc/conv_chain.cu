@@ -12,7 +12,8 @@
 //
 // The arithmetic is that of the stand-alone kernels (conv2_direct_device.cuh,
 // dense_small_device.cuh), including the rounding to the tensor type at every
-// layer boundary, so the result equals the layer-by-layer calls bit for bit.
+// layer boundary, so the result equals the layer-by-layer calls bit for bit while they run on those
+// kernels (see ag_conv_dense_chain_forward).
 #include "conv2_direct.cuh"
 #include "conv2_direct_device.cuh"
 #include "conv_chain.cuh"
@@ -289,7 +290,7 @@ static int launch_lenet(ag_device *dev, const T *x, const uint8_t *x8, float alp
 int64_t split_batch() {
     static const int64_t v = [] {
         const char *e = getenv("AG_CHAIN_SPLIT_BATCH");
-        return e ? (int64_t)atoll(e) : (int64_t)5120;
+        return e ? (int64_t)atoll(e) : dense_small::kMostRows + 1;
     }();
     return v;
 }
@@ -320,10 +321,11 @@ int forward(ag_device *dev, const T *x, const uint8_t *x8, float alpha, int64_t 
             return lenet_tiles::forward(dev, x, bs, w, y);
         }
     }
-    // Large batches of a LeNet5-geometry network: the kernel stops after the flatten and the
-    // dense layers run as products over the whole batch (ag_dense_forward: tensor cores for
-    // bf16, the SIMT tile engine for f32).  Inside the one-kernel form every CTA streams all
-    // dense weights for its 7 images; over the whole batch they are read once per 128-row tile.
+    // Batches of a LeNet5-geometry network beyond those whose dense layers ag_dense_forward adds like this
+    // kernel: it stops after the flatten and the dense layers run as products over the whole batch
+    // (ag_dense_forward: the tensor cores).  Inside the one-kernel form every CTA streams all dense weights
+    // for its 7 images; over the whole batch they are read once per 128-row tile (4097 images f32 72 us as
+    // one kernel, 78 split, bf16 76 and 78; 4600 88 and 88, 92 and 89; 5119 88 and 91, 92 and 99).
     if (!generic_only && split_batch() > 0 && bs >= split_batch()) {
         const ag_dtype dtype = sizeof(T) == 4 ? AG_F32 : AG_BF16;
         int64_t widest = layers[0].inputs;

@@ -96,10 +96,9 @@ __global__ void __launch_bounds__(512)
 
 // Up to 512 inputs and 1.7e8 multiply-adds: beyond either the tensor-core engines are faster
 // (602 x 861 x 163 f32: 21 us here, 13 us there; 32 x 2048 x 32: 30 and 5 us).  The limit on the
-// multiply-adds keeps LeNet5's layers here up to the batch at which the one-kernel network is
-// split (5120 x 256 x 128), because the two have to give the same bits.
+// multiply-adds keeps LeNet5's layers here up to kMostRows images (1.34e8).
 bool eligible(int64_t m, int64_t k, int64_t n) {
-    return m > 0 && m <= 4096 && n > 0 && n <= 256 && k > 0 && k <= 512 && m * k * n <= 170000000;
+    return m > 0 && m <= kMostRows && n > 0 && n <= 256 && k > 0 && k <= 512 && m * k * n <= 170000000;
 }
 
 bool fits_one_kernel(int64_t k, int64_t n) { return n > 0 && n <= 256 && k > 0 && k <= 2048; }

@@ -7,6 +7,11 @@
 namespace ag {
 namespace dense_small {
 
+// Rows beyond which the latency-oriented kernel never takes a product, and at which the one-kernel LeNet5 (conv_chain.cu)
+// hands its dense layers over: with one line for both, the network gives the bits of the separate layers on
+// either side of it.
+constexpr int64_t kMostRows = 4096;
+
 // True when the latency-oriented kernel should take y[m,n] = x[m,k] . w[k,n]
 // (all row-major contiguous): few rows, narrow output, moderate k.
 bool eligible(int64_t m, int64_t k, int64_t n);

@@ -248,8 +248,11 @@ AG_API int ag_conv2_relu_max_pool2_forward_keep(ag_device *dev, ag_dtype dtype, 
  * autograph_backend.rs:129-146) -- as ONE kernel that keeps every activation in shared memory.
  * x [bs, ic, ih, iw]; dense arguments as in ag_dense_chain_forward (dims[0] must equal the
  * flattened size of the last stage); y [bs, dims[n_dense]].  Equals the layer-by-layer calls bit
- * for bit while every dense layer has at most 512 inputs and bs * inputs * outputs is at most
- * 1.7e8 (beyond, ag_dense_forward adds in another order and the results agree to rounding).  Only networks that fit the kernel are taken (default convolution options, one 5x5 or
+ * for bit while they run on the kernels that add in the same order: up to 4096 images, fewer than
+ * 32 output channels in every stage, at most 512 inputs in every dense layer and bs * inputs *
+ * outputs up to 1.7e8; for the stages of LeNet5 (1 -> 6 -> 16 channels, 5x5, 28 x 28 images) also
+ * beyond, in f32 at any batch, in bf16 up to 63 images per SM.  Elsewhere the results agree to
+ * rounding.  Only networks that fit the kernel are taken (default convolution options, one 5x5 or
  * 3x3 filter size, 2x2 pools, <= 16 input and <= 64 output channels per stage, dense layers with
  * <= 2048 inputs and <= 256 outputs, 8 images of every activation within one CTA's shared
  * memory); any other network returns AG_ERR_UNSUPPORTED without touching y, and the caller runs

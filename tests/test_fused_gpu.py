@@ -290,3 +290,11 @@ def test_lenet5_head_equals_separate_calls(dev, dtype, bs):
         for wd, b, r in zip(P[2:5], biases, [True, True, False]):
             v = dev.dense_forward(v, wd, bias=b, relu=r)
         assert torch.equal(fused, v)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("bs", [4096, 4097, 5119, 5120])
+def test_lenet5_at_the_split_equals_separate_calls(dev, dtype, bs):
+    """Either side of the batch at which the network's dense layers become products over the batch, which is
+    where the separate calls change kernels too."""
+    test_lenet5_head_equals_separate_calls(dev, dtype, bs)
