@@ -67,14 +67,15 @@ static int dense_forward_simt(ag_device *dev, const T *x, int bs, int inputs, co
 using namespace ag;
 
 // Aligned bf16 products that the TMA kernels are better at than the gathered engine, whose k slices and smaller tiles fill
-// the chip where those have a handful of tiles.  m x k x n, us with TMA and gathered: 160 x 416 x 432 12.5 and 8.3, 208 x
-// 1328 x 144 17 and 8.4, 1408 x 608 x 192 12.5 and 10.1, 6928 x 64 x 432 10.4 and 12.1, 384 x 2864 x 336 16.6 and 11.2, 176 x
-// 3680 x 1088 27 and 16, 960 x 224 x 2608 11 and 22, 496 x 4832 x 416 21 and 24.
+// the chip where those have a handful of tiles.  m x k x n, us with TMA and gathered: 160 x 416 x 432 12.4 and 8.2, 208 x
+// 1328 x 144 16.6 and 8.6, 1408 x 608 x 192 12.4 and 9.6, 176 x 560 x 1648 12.4 and 8.8, 6928 x 64 x 432 10.4 and 12.7, 384 x
+// 2864 x 336 16.5 and 11.4, 176 x 3680 x 1088 26 and 16, 960 x 224 x 2608 11.0 and 19.2, 496 x 4832 x 416 20.8 and 21.3.
+// Over 320 drawn products of 4e7 to 3e9 multiply-adds these lines are 0.6 % above always taking the faster one.
 static bool tma_worth(int64_t m, int64_t k, int64_t n) {
     const double macs = (double)m * (double)n * (double)k;
     if (!tcx::gemm_worth(AG_BF16, m, k, n)) return true;
-    if (k >= 1024 && ag::ceil_div(m, 128) * ag::ceil_div(n, 128) <= 24) return macs >= 8e8;
-    return macs >= 1.5e8;
+    if (k >= 1024 && ag::ceil_div(m, 128) * ag::ceil_div(n, 128) <= 32) return macs >= 1e9;
+    return macs >= (k < 160 ? 1.5e8 : 2.5e8);
 }
 
 extern "C" int ag_dense_forward(ag_device *dev, ag_dtype dtype, const void *x, int64_t bs,

@@ -18,11 +18,11 @@ static bool enabled() {
     return v;
 }
 
-// Against the SIMT engine (B200, device time): f32 390 x 145 x 135 13 us here and 8 us there,
-// 300 x 100 x 2000 9.7 and 10.8, 602 x 861 x 163 13 and 32, 1024^3 34 and 83; bf16
-// 100 x 256 x 128 8 and 8, 390 x 145 x 135 9 and 18.  A call here costs about 9 us in f32 (slices of
-// k, two kernels) whatever the size, so the line is drawn at the multiply-adds the SIMT kernels do
-// in that time.
+// Against the SIMT engine, m x k x n, us here and there (row-major operands back to back): f32 464 x 16 x 416 7.7 and
+// 5.2, 112 x 64 x 2528 7.0 and 6.3, 928 x 2336 x 16 14.0 and 16.5, 300 x 100 x 2000 8.0 and 12.4, 602 x 861 x 163 11.7 and
+// 37, 1024^3 34 and 83; bf16 672 x 112 x 96 6.3 and 6.4, 96 x 3120 x 48 7.7 and 16.8, 208 x 624 x 96 7.2 and 14.7.  A
+// short k is one launch here, and both engines take 5 to 8 us up to some 1e7 multiply-adds, most of it the launch: the
+// lines lie where the SIMT kernels begin to take longer.
 // Few rows: 1 to 8 x 25088 x 512 18 us and 68 (bf16 13 and 97), 12 x 100 x 20000 9 and 27.  Few columns: 20000 x 200 x
 // 12 25 and 14, 5000 x 2000 x 12 51 and 98.  k below a tile's step: 25088 x 24 x 512 39 and 27,
 // f32 1264 x 32 x 4896 22 and 17, 892 x 39 x 7961 24 and 25.
@@ -36,14 +36,17 @@ bool gemm_worth(ag_dtype dtype, int64_t m, int64_t k, int64_t n) {
     return macs >= (dtype == AG_F32 ? 3e7 : 4e6);
 }
 
-// Against the gathered engine, m x k x n, us packed and gathered: f32 305 x 369 x 2296 29 and 15, 2592 x 2080 x 128 41
-// and 24, 3568 x 1344 x 528 72 and 58, 1040 x 3440 x 544 58 and 88, 5728 x 608 x 1200 81 and 100; bf16 1037 x 438 x
-// 1885 39 and 27, 4313 x 791 x 1252 41 and 71.  The copy pass, its launch and 256 x 256 tiles want 1.8e9
-// multiply-adds, more of them when k is short, because a tile is then mostly its epilogue (over 317 drawn
-// products this line is 1.4% above always taking the faster engine).
+// Against the gathered engine, m x k x n, us packed and gathered: f32 305 x 369 x 2296 29 and 15, 2592 x 2080 x 128 39
+// and 25, 1024 x 1872 x 560 37 and 50, 3568 x 1344 x 528 64 and 60, 1040 x 3440 x 544 52 and 87, 5728 x 608 x 1200 74 and
+// 104; bf16 1037 x 438 x 1885 39 and 27, 4313 x 791 x 1252 41 and 71.  The copy pass and its launch want some 8e8
+// multiply-adds, counted by how much of its 256 x 256 tiles the output fills (528 columns are 69 % of three tiles), and more
+// of them when k is short, because a tile is then mostly its epilogue.  Over 470 drawn products of 3e8 to 1e10 multiply-adds
+// this line is 1.2 % above always taking the faster engine, without the fill and from 1.8e9 on it was 3.2 %; 3568 x 1344 x
+// 528 is still on the wrong side of it.
 bool packed_worth(int64_t m, int64_t k, int64_t n) {
-    const double macs = (double)m * (double)n * (double)k;
-    return m >= 128 && n >= 128 && k >= 64 && macs >= 1.8e9 && macs * (double)k >= 1.2e12;
+    const double fill = ((double)m / (256.0 * ceil_div(m, 256))) * ((double)n / (256.0 * ceil_div(n, 256)));
+    const double macs = (double)m * (double)n * (double)k * fill;
+    return m >= 128 && n >= 128 && k >= 64 && macs >= 8e8 && macs * (double)k >= 6e11;
 }
 
 // The filters are also counted with their channels padded to eight, in an int (repack_kernel).
