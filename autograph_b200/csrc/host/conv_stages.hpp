@@ -97,7 +97,7 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
     bool input_grad = false;
     bool keep = true;                 // forward's tensors stay for the backward pass
     std::vector<StageDesc> st;
-    std::vector<Tensor> act, pre;     // per stage: the kernels' input and the convolution's output
+    std::vector<Tensor> act, pre;     // per stage: the kernels' input, and the convolution's output if it is odd
     std::vector<Tensor> code;         // per stage: where each pool window's gradient goes
     std::vector<Tensor> dpre;         // per stage: gradient at the convolution's output (maybe framed)
     std::vector<char> have, framed;
@@ -176,7 +176,8 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
             if (keep) {
                 code.push_back(codes);
                 act.push_back(a);
-                pre.push_back(p);
+                // the backward pass reads it only where an odd plane has cells that no window covers
+                pre.push_back(d.oh % 2 != 0 || d.ow % 2 != 0 ? p : Tensor{});
             }
             pooled = y;
         }
@@ -237,7 +238,8 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
             dpre[s] = make({bs, d.oh, d.ow, d.ocp});
         }
         const View v = interior(s);
-        check(::ag::nhwc::relu_pool_backward(dev, cptr(pre[s]), (const uint32_t *)code[s].data(), cptr(dpool), bs, d.oh, d.ow, d.ocp, v.p,
+        check(::ag::nhwc::relu_pool_backward(dev, pre[s].defined() ? cptr(pre[s]) : nullptr, (const uint32_t *)code[s].data(),
+                                            cptr(dpool), bs, d.oh, d.ow, d.ocp, v.p,
                                             v.row_pitch, v.image_pitch));
         have[s] = 1;
     }

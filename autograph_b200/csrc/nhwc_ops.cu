@@ -321,6 +321,7 @@ int relu_pool_backward(ag_device *dev, const __nv_bfloat16 *pre, const uint32_t 
                    aligned16(dy) && aligned16(out),
                AG_ERR_INVALID, "relu_pool_backward: bad pitch or alignment");
     AG_REQUIRE(ih >= 2 && iw >= 2, AG_ERR_SHAPE, "relu_pool_backward: window larger than input");
+    AG_REQUIRE(pre != nullptr || (ih % 2 == 0 && iw % 2 == 0), AG_ERR_INVALID, "relu_pool_backward: odd planes need pre");
     const int64_t total = bs * ((ih + 1) / 2) * ((iw + 1) / 2) * (cp / 8);
     if (total == 0) return AG_OK;
     relu_pool_backward_kernel<<<grid_for(dev, total), 256, 0, dev->stream>>>(
