@@ -65,17 +65,6 @@ __device__ __forceinline__ uint64_t make_desc_sw32(uint32_t addr) {
     return d;
 }
 
-__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
-
 __global__ void __launch_bounds__(kThreads, 1)
     lenet_chain_tc_kernel(const __nv_bfloat16 *__restrict__ x, const uint8_t *__restrict__ x8, float alpha,
                           __nv_bfloat16 *__restrict__ y, const Plan pl) {
@@ -270,7 +259,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             tc::tc_fence_after();
             uint32_t r[16];
-            tmem_ld_32x16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(t * 16), r);
+            tc::tmem_ld_32x16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(t * 16), r);
             tc::tmem_ld_wait();
             uint32_t o[8];
 #pragma unroll

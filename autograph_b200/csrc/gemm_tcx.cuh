@@ -669,18 +669,6 @@ struct Slots {
     }
 };
 
-// 32 lanes x 16 columns.
-__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
-
 // The 32 x 32 outputs at (row0, col0) from the operands as they were given: sums of k0 .. k1 in order, one
 // warp.  A lane has rows row0 + lane / 4 * 4 .. + 3 and columns col0 + lane % 4 * 8 .. + 7.  `buf` is the warp's
 // (kRedoFloats); ROWS_A, ROWS_B: neighbouring lanes fetch neighbouring rows of the operand, else
@@ -1025,8 +1013,8 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
 #pragma unroll
                 for (int c = 0; c < C::COLS; c += 16) {
                     uint32_t r0[16], r1[16];
-                    tmem_ld_32x16(t + c, r0);
-                    if (PL == 3) tmem_ld_32x16(t + BN + c, r1);
+                    tc::tmem_ld_32x16(t + c, r0);
+                    if (PL == 3) tc::tmem_ld_32x16(t + BN + c, r1);
                     tc::tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {

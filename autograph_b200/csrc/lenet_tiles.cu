@@ -155,13 +155,6 @@ __device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a_tmem, uint32_t b_
         "r"(a_tmem), "r"(b_low), "r"(idesc), "r"(accumulate), "n"(kDescHigh)
         : "memory");
 }
-__device__ __forceinline__ void ld16(uint32_t t, uint32_t *r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(t)
-                 : "memory");
-}
 __device__ __forceinline__ void st2(uint32_t t, const uint32_t *r) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(t), "r"(r[0]), "r"(r[1]) : "memory");
 }
@@ -367,8 +360,8 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                     tc::tc_fence_after();
                     uint32_t r[32], now[4];
                     uint32_t *o = Q == 0 || (Q == 3 && h == 1) ? now : held[2 * (Q - 1) + h];
-                    ld16(from, r);
-                    ld16(from + 32, r + 16);
+                    tc::tmem_ld_32x16(from, r);
+                    tc::tmem_ld_32x16(from + 32, r + 16);
                     tc::tmem_ld_wait();
                     tc::tc_fence_before();
                     __syncwarp();
@@ -403,7 +396,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
                     tc::tc_fence_after();
                     uint32_t r[48], o[6];
 #pragma unroll
-                    for (int i = 0; i < 48; i += 16) ld16(acc + i, r + i);
+                    for (int i = 0; i < 48; i += 16) tc::tmem_ld_32x16(acc + i, r + i);
                     tc::tmem_ld_wait();
                     tc::tc_fence_before();
                     __syncwarp();
@@ -455,8 +448,8 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
             {
                 const bf16 *bias = (const bf16 *)a.w.bias[0];
                 uint32_t r[32], o[16];
-                ld16(t + 32 * set, r);
-                ld16(t + 32 * set + 16, r + 16);
+                tc::tmem_ld_32x16(t + 32 * set, r);
+                tc::tmem_ld_32x16(t + 32 * set + 16, r + 16);
                 tc::tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 16; ++i)
@@ -493,7 +486,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
             if (set == 0) {
                 const bf16 *bias = (const bf16 *)a.w.bias[2];
                 uint32_t r[16];
-                ld16(t, r);
+                tc::tmem_ld_32x16(t, r);
                 tc::tmem_ld_wait();
                 if (b < a.bs) {
                     uint32_t *y = reinterpret_cast<uint32_t *>(a.y + (int64_t)b * D3);

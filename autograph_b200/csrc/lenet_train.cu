@@ -865,23 +865,6 @@ static int launch_pass(ag_device *dev, const Args &a, int ctas) {
     return AG_OK;
 }
 
-// A launch whose CTAs may be placed before the previous kernel ends (both wait for it themselves): at 100
-// images the step is a chain of launches, each of which started 2 us after the last.
-static int launch_after(ag_device *dev, void (*kernel)(const Finish), int ctas, const Finish &f) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(256);
-    cfg.stream = dev->stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    AG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, f));
-    AG_CHECK_LAUNCH();
-    return AG_OK;
-}
-
 template <class T>
 static int step_typed(ag_device *dev, const Net &net, const void *x, const uint8_t *t, int bs, void *values,
                       void *grads, void *velocity, const Sgd &sgd, float *loss) {
@@ -937,8 +920,10 @@ static int step_typed(ag_device *dev, const Net &net, const void *x, const uint8
     f.conv_planes = a.planes;
     f.row_loss = a.row_loss;
     f.loss = loss;
-    AG_TRY(launch_after(dev, lenet_finish_kernel<T>, kTiles * f.splits + kConvBlocks + 1, f));
-    if (f.splits > 1) AG_TRY(launch_after(dev, lenet_reduce_kernel<T>, (int)ceil_div(kDense, 256), f));
+    // Dependent launches: at 100 images the step is a chain of launches, each of which started 2 us after the last.
+    AG_TRY(launch_dependent(dev, lenet_finish_kernel<T>, dim3((unsigned)(kTiles * f.splits + kConvBlocks + 1)), 256, 0, f));
+    if (f.splits > 1)
+        AG_TRY(launch_dependent(dev, lenet_reduce_kernel<T>, dim3((unsigned)ceil_div(kDense, 256)), 256, 0, f));
     return AG_OK;
 }
 

@@ -1,9 +1,7 @@
 // Device objects, memory, transfers and error reporting of the C ABI.
 #include <atomic>
-#include <cstring>
-
-#include <atomic>
 #include <chrono>
+#include <cstring>
 
 #include "common.cuh"
 #include "tc_ptx.cuh"
