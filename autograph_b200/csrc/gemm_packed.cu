@@ -14,8 +14,8 @@
 //
 // What bounds it: the f32 form issues 24 MMAs of 256 x 256 x 16 per 64 k from two 96 KiB stages,
 // the tensor pipe at the clock the power limit leaves; the copy pass moves (4 + 6) bytes per
-// operand element.  f32 4096^3: 654 us (210 TFLOP/s of f32 multiply-adds, 1.26 PFLOP/s of bf16)
-// against 2650 - 2900 us on the FP32 pipe; bf16 4095 x 4093 x 4097: 152 us.
+// operand element.  f32 4096^3: 593 us (232 TFLOP/s of f32 multiply-adds, 1.39 PFLOP/s of bf16)
+// in a burst, 690 us under the power cap, against 2650 - 2900 us on the FP32 pipe; bf16 4095 x 4093 x 4097: 152 us.
 #include <cuda.h>
 
 #include "gemm_packed.cuh"

@@ -19,9 +19,9 @@ One JSON line is printed by rank 0.  Besides the contract keys it carries
   e2e           the same step through Model.infer with pinned host buffers (copies inside the
                 timed region); e2e_pipelined: two batches in flight through
                 ag_model_infer_enqueue / _wait; e2e_pageable: the same from pageable host memory
-  infer_sharded_65536   configs[4a]: 65536 images split evenly over the ranks (strong scaling)
-  train_dp      configs[4b]: 100 images per GPU, gradient all-reduce, SGD update
-  gemm          the standalone dot sweep (configs[1]) in TFLOP/s, with `gemm_roofline`
+  infer_sharded_65536   65536 images split evenly over the ranks (strong scaling)
+  train_dp      100 images per GPU, gradient all-reduce, SGD update
+  gemm          the standalone dot sweep in TFLOP/s, with `gemm_roofline`
                 for the 4096^3 bf16 dot against the measured bf16 tensor peak
   cpu_baseline  the CPU oracle (a port of the reference's host path) on this box's cores,
                 timed after the GPU work, when rank 0 is the only process left
@@ -381,7 +381,7 @@ def run_gpu(args):
         "gpu_launches": int(launches),
     }
 
-    # configs[4a]: 65536 images sharded evenly by batch, no collective (strong scaling: the
+    # 65536 images sharded evenly by batch, no collective (strong scaling: the
     # total is fixed, each rank runs 65536 / world images in one launch).
     try:
         n_shard = 65536 // world
@@ -400,7 +400,7 @@ def run_gpu(args):
     except Exception as exc:
         line["infer_sharded_65536_error"] = repr(exc)
 
-    # configs[4b]: data-parallel training, 100 images per GPU, one sum-all-reduce of the
+    # Data-parallel training, 100 images per GPU, one sum-all-reduce of the
     # flat gradient bucket per step, 1/world folded into the update.  Runs on every rank.
     try:
         line["train_dp"] = train_data_parallel(torch, ag, dp, dev, rank, world, barrier,
@@ -451,7 +451,7 @@ def run_gpu(args):
 
 
 def train_data_parallel(torch, ag, dp, dev, rank, world, barrier, max_over_ranks):
-    """configs[4b]: forward / backward on 100 images per GPU, then the data-parallel tail two
+    """Forward / backward on 100 images per GPU, then the data-parallel tail two
     ways: the fused kernel (one-shot all-reduce over NVLink + 1/world + SGD update) and, for
     comparison, an NCCL all-reduce of the bucket followed by the update kernel."""
     comm = dp.Comm.from_torch_distributed(dev) if world > 1 else dp.Comm.single_process([dev])
@@ -587,7 +587,7 @@ def lenet5_roofline(torch, ag, dev, model, xs, K, peaks):
 
 
 def gemm_sweep(torch, ag, dev, peaks, sampler):
-    """square dot products, f32 (SIMT) and bf16 (tcgen05), NN / TN / NT."""
+    """Square dot products, f32 (as six bf16 products) and bf16 on tcgen05, NN / TN / NT."""
     results = []
     roof = None
     for dtype, name in [(torch.bfloat16, "bf16"), (torch.float32, "f32")]:
@@ -619,7 +619,8 @@ def gemm_sweep(torch, ag, dev, peaks, sampler):
                 if name == "bf16":
                     entry["frac_of_measured_bf16_peak"] = tf / peaks["bf16_tflops"]
                 else:
-                    entry["frac_of_fp32_pipe_peak_at_max_clock"] = tf / (148 * 128 * 2 * 1.965e-3)
+                    # the tensor cores do an f32 product as six bf16 products
+                    entry["frac_of_measured_bf16_peak_as_six_products"] = 6.0 * tf / peaks["bf16_tflops"]
                 results.append(entry)
                 if name == "bf16" and n == 4096 and layout == "nn":
                     roof = {"bound": "tensor", "kernel": "gemm_bf16_tc2_kernel (tcgen05, cta_group::2), 4096^3 nn",
@@ -634,7 +635,7 @@ def gemm_sweep(torch, ag, dev, peaks, sampler):
 
 
 def extras(torch, ag, dev, peaks, world):
-    """bf16 inference, the configs[2] training step, u8 input pipeline, the wide conv stack."""
+    """bf16 inference, the batch-100 training step, u8 input pipeline, the wide conv stack."""
     out = {}
     # bf16 LeNet5 inference, batch 1000
     mb = ag.Model(dev, ag.LENET5_SPEC, torch.bfloat16, seed=2000)
@@ -648,7 +649,7 @@ def extras(torch, ag, dev, peaks, world):
     mb.close()
     del xb
     m = ag.Model(dev, ag.LENET5_SPEC, torch.float32, seed=2000)
-    # training step, batch 100, host buffers, plain SGD lr 0.01
+    # Training step, batch 100, host buffers, plain SGD lr 0.01
     xt = torch.rand((100, 1, 28, 28)).pin_memory()
     tt = torch.randint(0, 10, (100,), dtype=torch.uint8).pin_memory()
     for i in range(5):
@@ -673,7 +674,7 @@ def extras(torch, ag, dev, peaks, world):
         "d2h_bytes_per_step": BATCH * 40, "timing": "host wall clock over blocking calls"}
     mi.close()
     if world == 1:
-        # the wider conv stack, bf16, batch 256: forward + backward + SGD update.
+        # The wider conv stack, bf16, batch 256: forward + backward + SGD update.
         # FLOPs of one step: 2 * MACs of (conv1, conv2, dense1, dense2), forward once and
         # backward twice (input and weight gradients; conv1 has no input gradient).
         mw = ag.Model(dev, ag.WIDE_STACK_SPEC, torch.bfloat16, seed=2000)

@@ -1,14 +1,14 @@
 """GPU: the benchmark configurations at their full sizes.
 
-  configs[1]  8192^3 dot, f32 and bf16, nn / tn / nt: 4096 sampled elements against an f64
+  dot         8192^3, f32 and bf16, nn / tn / nt: 4096 sampled elements against an f64
               product of the sampled rows and columns, plus row and column checksums
               (the reference's own dot tests compare whole matrices at small sizes,
               tests/integration_tests.rs:353-371; at this size the checks are the
               size-independent ones)
-  configs[3]  wide conv stack at batch 256: logits of 16 sampled rows against the oracle and
+  wide stack  batch 256: logits of 16 sampled rows against the oracle and
               every gradient against torch-CPU float64 autograd (an implementation that shares
               nothing with the oracle or the kernels)
-  configs[4a] 65536 images through LeNet5: every row's argmax and the logits against the oracle
+  LeNet5      65536 images: every row's argmax and the logits against the oracle
   autograd    a parameter used by two layers (two gradients arriving at one node)
 """
 import numpy as np
@@ -28,7 +28,7 @@ def _rel(got, ref):
                  max(np.abs(ref).max(), 1e-30))
 
 
-# ------------------------------------------------------------------ configs[1] at 8192^3
+# ------------------------------------------------------------------ dot at 8192^3
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("layout", ["nn", "tn", "nt"])
 def test_dot_8192(dev, dtype, layout):
@@ -68,7 +68,7 @@ def test_dot_8192(dev, dtype, layout):
     assert np.isfinite(row_got).all() and abs(row_got.sum() - row_ref.sum()) <= tol * row_bound.sum()
 
 
-# ------------------------------------------------------------------ configs[3] at batch 256
+# ------------------------------------------------------------------ wide stack at batch 256
 def test_wide_stack_bf16_batch_256(dev):
     import autograph_b200 as ag
     dtype = torch.bfloat16
@@ -94,7 +94,7 @@ def test_wide_stack_bf16_batch_256(dev):
     model.close()
 
 
-# ------------------------------------------------------------------ configs[4a]: 65536 images
+# ------------------------------------------------------------------ LeNet5: 65536 images
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_lenet5_inference_65536(dev, dtype):
     import autograph_b200 as ag
