@@ -183,6 +183,45 @@ def test_bias_add_and_grad(dev, golden, dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("shape,offset", [((1, 1, 3, 3), 0), ((2, 3, 2, 5), 1), ((2, 3, 5, 2), 0), ((5, 7, 11, 6), 1),
+                                          ((1, 2, 1301, 2777), 0),   # more windows than one round of the grid holds
+                                          ((1, 1, 1902, 2782), 2)])
+def test_windows_of_two_by_two(dev, dtype, shape, offset):
+    """Odd planes, starts off 16 bytes, in and out of place: exact, and the cells no window covers are kept."""
+    rng = np.random.default_rng(31)
+    x = _prep(rng.integers(-4, 5, shape).astype(np.float32) * 0.5, dtype)
+    flat = dev.empty((x.size + offset,), dtype)
+    flat[offset:].copy_(dev.tensor(x, dtype).reshape(-1))
+    xd = flat[offset:].reshape(shape)
+    want = oracle.max_pool2(x, (2, 2), None)
+    assert np.array_equal(_np(dev.max_pool2(xd)), want)
+    dy = _prep(rng.standard_normal(want.shape), dtype)
+    want = oracle.max_pool2_backward(x, dy, (2, 2), None)
+    assert np.array_equal(_np(dev.max_pool2_backward_from_input(xd, dev.tensor(dy, dtype))), want)
+    assert np.array_equal(_np(dev.max_pool2_backward(xd, dev.tensor(dy, dtype))), want)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("shape,offset", [((1, 1, 2), 0), ((3, 2, 2, 2), 1), ((2, 3, 7), 0), ((9, 5, 511), 1), ((4, 3, 512), 0),
+                                          ((2, 2, 1023), 1), ((70, 33, 1025), 0), ((2, 1500, 6), 0), ((1, 1, 70001), 3)])
+def test_bias_grad_of_planes(dev, dtype, shape, offset):
+    """Planes that start and end anywhere in a 16-byte vector, one unit of loads or several, one launch or two.
+    An f32 sum of n values of size one, added in at most n / 32 + 32 steps per lane and tree, is off by less than
+    (n / 32 + 32) * 2^-24 * sum |x|."""
+    rng = np.random.default_rng(32)
+    x = _prep(rng.standard_normal(shape), dtype)
+    flat = dev.empty((x.size + offset,), dtype)
+    flat[offset:].copy_(dev.tensor(x, dtype).reshape(-1))
+    axes = tuple(i for i in range(len(shape)) if i != 1)
+    got = _np(dev.bias_grad(flat[offset:].reshape(shape)))
+    want, size = x.astype(np.float64).sum(axis=axes), np.abs(x).sum(axis=axes)
+    bound = (x.size / shape[1] / 32 + 32) * 2.0 ** -24 * size
+    if dtype == torch.bfloat16:
+        bound += 2.0 ** -8 * (np.abs(want) + bound)
+    assert (np.abs(got - want) <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_sgd(dev, dtype):
     rng = np.random.default_rng(5)
     n = 46920
