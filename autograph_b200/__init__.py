@@ -8,7 +8,7 @@ LeNet5-style model object) so that tests and benchmarks read like the
 reference's own.  PyTorch is used only to hold device memory, streams and for
 ``torch.distributed``.
 
-The per-step calls go through a small CPython extension (``csrc/python/front.c``) that
+The per-step calls go through a small CPython extension (``csrc/python/front.cpp``) that
 reads the tensors and calls the library directly; the methods below are the same calls in
 Python and ctypes, which it hands anything but the plain case to.
 
@@ -26,6 +26,7 @@ from . import _capi
 from ._capi import AgError, lib, lib_path  # noqa: F401
 
 try:
+    import torch as _  # noqa: F401  the extension finds torch's libraries among those already loaded
     from . import _front
     _DeviceBase, _ModelBase = _front.DeviceBase, _front.ModelBase
 except ImportError:   # not built yet (the build imports this package): creating a Device fails
@@ -78,7 +79,7 @@ def _bind_front():
     if not _front_bound:
         handle = lib()
         _front.bind({n: ctypes.cast(getattr(handle, n), ctypes.c_void_p).value for n in _front.FUNCTIONS},
-                    _torch(), _capi.check)
+                    _capi.check)
         for name in _front.METHODS:
             _front.set_fallback(name, getattr(_PyDevice, name, None) or getattr(_PyModel, name))
         _front_bound = True

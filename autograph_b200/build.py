@@ -1,5 +1,5 @@
 """Builds libautograph_b200.so (the C-ABI library) with nvcc for sm_100a, and the CPython extension
-that calls it from the Python front end with the C compiler.
+that calls it from the Python front end with the C++ compiler.
 
 Usage: ``python -m autograph_b200.build [--force] [--verbose]``.
 Objects go to ``autograph_b200/_build``; the shared library is written next to
@@ -81,13 +81,19 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
 
 def build_front(force: bool = False) -> Path:
-    """The native half of the Python front end (csrc/python/front.c), a CPython extension next to
-    the library."""
-    src = CSRC / "python" / "front.c"
+    """The native half of the Python front end (csrc/python/front.cpp), a CPython extension next to
+    the library.  It reads tensors through torch's C++ interface; the libraries that it names are those
+    that `import torch` has loaded."""
+    import importlib.util
+    src = CSRC / "python" / "front.cpp"
     out = HERE / ("_front" + sysconfig.get_config_var("EXT_SUFFIX"))
     stamp = BUILD / "front.stamp"
-    cmd = [os.environ.get("CC", "gcc"), "-O2", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden",
-           "-I" + sysconfig.get_paths()["include"], str(src), "-o", str(out)]
+    torch_dir = Path(importlib.util.find_spec("torch").origin).parent
+    cuda = Path(NVCC).resolve().parent.parent
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden",
+           "-I" + sysconfig.get_paths()["include"], "-isystem", str(torch_dir / "include"),
+           "-isystem", str(torch_dir / "include" / "torch" / "csrc" / "api" / "include"), "-isystem", str(cuda / "include"),
+           str(src), "-o", str(out), "-L" + str(torch_dir / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
     header = HERE.parent / "include" / "autograph_b200.h"
     key = hashlib.sha256(src.read_bytes() + header.read_bytes() + " ".join(cmd).encode()).hexdigest()
     if force or not out.exists() or not stamp.exists() or stamp.read_text() != key:
