@@ -198,7 +198,20 @@ inline bool is_label_dtype(ag_dtype t) { return t == AG_U8 || t == AG_U16 || t =
 
 // ---- element conversion (device) ------------------------------------------
 __device__ __forceinline__ float to_f32(float x) { return x; }
-__device__ __forceinline__ float to_f32(__nv_bfloat16 x) { return __bfloat162float(x); }
+// A shift of the bits.
+__device__ __forceinline__ float to_f32(__nv_bfloat16 x) { return __uint_as_float((uint32_t)__bfloat16_as_ushort(x) << 16); }
+// An operand's element, or zero outside of it: a load under a predicate, so that several can be in flight
+// (256 x 200 x 10, transposed: f32 11.5 us with a branch around each, 10.7 so; bf16 26.2 and 23.9).
+__device__ __forceinline__ float load_or_zero(const float *p, bool ok) {
+    float v = 0.f;
+    if (ok) v = __ldg(p);
+    return v;
+}
+__device__ __forceinline__ float load_or_zero(const __nv_bfloat16 *p, bool ok) {
+    uint32_t v = 0;
+    if (ok) v = __ldg(reinterpret_cast<const unsigned short *>(p));
+    return __uint_as_float(v << 16);
+}
 template <class T>
 __device__ __forceinline__ T from_f32(float x);
 template <>

@@ -56,8 +56,8 @@ __device__ __forceinline__ float im2col_at(const T *x, const ConvGeom &g, int po
     g.div_fw.divmod(f, fi, fj);
     int hx = (int)(hy * g.sh + fi * g.dh) - g.ph;
     int wx = (int)(wy * g.sw + fj * g.dw) - g.pw;
-    if ((unsigned)hx >= (unsigned)g.ih || (unsigned)wx >= (unsigned)g.iw) return 0.f;
-    return to_f32(x[((int64_t)(b * g.c + ci) * g.ih + hx) * g.iw + wx]);
+    return load_or_zero(x + ((int64_t)(b * g.c + ci) * g.ih + hx) * g.iw + wx,
+                        (unsigned)hx < (unsigned)g.ih && (unsigned)wx < (unsigned)g.iw);
 }
 
 // im2col(x) as a GEMM operand. POS_IS_K = false: mn = patch position (forward A
@@ -87,10 +87,9 @@ struct DyTransposedOperand {
     int mn_size, k_size;
     bool vec;
     __device__ __forceinline__ float at(int mn, int k) const {
-        if (mn >= mn_size || k >= k_size) return 0.f;
         uint32_t b, r;
         div_ohw.divmod((uint32_t)k, b, r);
-        return to_f32(dy[((int64_t)b * oc + mn) * ohw + r]);
+        return load_or_zero(dy + ((int64_t)b * oc + mn) * ohw + r, mn < mn_size && k < k_size);
     }
     __device__ __forceinline__ bool in_range4(int, int) const { return false; }
     __device__ __forceinline__ void load4(int, int, float (&)[4]) const {}
@@ -139,10 +138,9 @@ struct WeightTransposedOperand {
     int mn_size, k_size;
     bool vec;
     __device__ __forceinline__ float at(int mn, int k) const {
-        if (mn >= mn_size || k >= k_size) return 0.f;
         uint32_t co, f;
         div_ff.divmod((uint32_t)k, co, f);
-        return to_f32(w[((int64_t)co * ic + mn) * ff + f]);
+        return load_or_zero(w + ((int64_t)co * ic + mn) * ff + f, mn < mn_size && k < k_size);
     }
     __device__ __forceinline__ bool in_range4(int, int) const { return false; }
     __device__ __forceinline__ void load4(int, int, float (&)[4]) const {}

@@ -16,8 +16,7 @@
 namespace ag {
 namespace dense_small {
 
-// One layer of the chain's code on 8 rows per CTA: layers with at most 16 outputs, and batches
-// large enough to fill the GPU at 8 rows per CTA.
+// One layer of the chain's code on 8 rows per CTA: batches large enough to fill the GPU at 8 rows per CTA.
 template <class T>
 __global__ void __launch_bounds__(1024)
     dense_rows_kernel(const T *__restrict__ x, T *__restrict__ y, int M, const ChainStep st) {
@@ -32,6 +31,51 @@ __global__ void __launch_bounds__(1024)
     }
     __syncthreads();
     chain_layer<T>(st, reinterpret_cast<const T *>(st.w), xs, nullptr, red, m0, rows, true, y);
+}
+
+// A layer with at most 16 outputs (narrow_step) on its own: narrow_layer's sums, four lanes per output that add
+// k = q, q + 4, ..., with the weights and R rows of x in shared memory.  Read from L2 16 at a time and on 8 rows
+// per CTA, 256 x 512 x 10 took 7.8 us (32 CTAs, eight trips to L2 one after another), now 4.0; 4096 x 84 x 10 6.1 and 3.7.
+template <class T>
+__global__ void __launch_bounds__(256)
+    dense_narrow_kernel(const T *__restrict__ x, T *__restrict__ y, int M, int R, const ChainStep st) {
+    extern __shared__ __align__(16) float smem[];
+    float *ws = smem, *xs = smem + st.K * st.N;   // [K][N], [R][K]
+    const T *w = reinterpret_cast<const T *>(st.w), *bias = reinterpret_cast<const T *>(st.bias);
+    const int m0 = blockIdx.x * R, rows = min(R, M - m0);
+    const T *xr = x + (int64_t)m0 * st.K;
+    const int n_w = st.K * st.N, n_x = rows * st.K;
+    for (int i0 = threadIdx.x; i0 < n_w + n_x; i0 += 8 * 256) {
+        T v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int i = i0 + j * 256;
+            if (i < n_w) v[j] = __ldg(w + i);
+            else if (i < n_w + n_x) v[j] = __ldg(xr + (i - n_w));
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (i0 + j * 256 < n_w + n_x) smem[i0 + j * 256] = to_f32(v[j]);
+    }
+    __syncthreads();
+    const int total = rows * st.N * 4, padded = (total + 31) & ~31;   // whole warps take part in the shuffles
+    for (int it = threadIdx.x; it < padded; it += 256) {
+        const bool live = it < total;
+        const int q = it & 3, o = live ? it >> 2 : 0, r = o / st.N, c = o - r * st.N;
+        float p = 0.f;
+        if (live) {
+            const float *wp = ws + c, *xp = xs + r * st.K;
+#pragma unroll 8
+            for (int k = q; k < st.K; k += 4) p = fmaf(xp[k], wp[k * st.N], p);
+        }
+        p += __shfl_xor_sync(0xffffffffu, p, 1);
+        p += __shfl_xor_sync(0xffffffffu, p, 2);
+        if (!live || q != 0) continue;
+        float v = to_f32(from_f32<T>(p));
+        if (bias != nullptr) v = to_f32(from_f32<T>(__fadd_rn(v, to_f32(bias[c]))));
+        if (st.relu) v = (v >= 0.f) ? v : 0.f;
+        y[(int64_t)(m0 + r) * st.N + c] = from_f32<T>(v);
+    }
 }
 
 // R rows x 32 columns per CTA, a warp per k slice.  Latency bound (a CTA streams kchunk weights
@@ -122,10 +166,16 @@ int forward(ag_device *dev, const T *x, int m, int k, const T *w, int n, const T
     // Rows x columns against k: with many outputs the 8-row form's wider tiles win, with a long k the
     // spread form's larger number of loads in flight (f32 100 x 256 x 128: 7.9 us on 8 rows per CTA,
     // 4.2 us spread; 256^3 13.1 and 10.1; 384 x 145 x 135 5.9 and 6.8; bf16 256^3 13.1 and 13.9).
-    const bool narrow = narrow_step(st);
-    if (narrow || (int64_t)m * st.np > (sizeof(T) == 4 ? 256 : 128) * (int64_t)k) {
-        const int threads = narrow ? (ROWS * n * 4 < 512 ? (ROWS * n * 4 + 31) / 32 * 32 : 512) : st.np * st.slices;
-        const size_t smem = ((size_t)k * ROWS + (narrow ? 0 : (size_t)st.slices * ROWS * st.np)) * sizeof(float);
+    if (narrow_step(st)) {
+        // as many rows per CTA, up to four, as leave every SM one; 512 inputs and 16 outputs take 40 KB
+        const int r = ceil_div(m, 4) >= dev->sm_count ? 4 : ceil_div(m, 2) >= dev->sm_count ? 2 : 1;
+        dense_narrow_kernel<T><<<(unsigned)ceil_div(m, r), 256, sizeof(float) * (size_t)k * (n + r), dev->stream>>>(x, y, m, r, st);
+        AG_CHECK_LAUNCH();
+        return AG_OK;
+    }
+    if ((int64_t)m * st.np > (sizeof(T) == 4 ? 256 : 128) * (int64_t)k) {
+        const int threads = st.np * st.slices;
+        const size_t smem = ((size_t)k * ROWS + (size_t)st.slices * ROWS * st.np) * sizeof(float);
         static bool configured_on[64] = {};
         if (smem > 48 * 1024 && !configured_on[dev->ordinal & 63]) {
             AG_CUDA_TRY(cudaFuncSetAttribute(dense_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -77,8 +77,7 @@ struct StridedOperand {
     int mn_size, k_size;
     bool vec;
     __device__ __forceinline__ float at(int mn, int k) const {
-        if (mn >= mn_size || k >= k_size) return 0.f;
-        return to_f32(p[(int64_t)mn * smn + (int64_t)k * sk]);
+        return load_or_zero(p + (int64_t)mn * smn + (int64_t)k * sk, mn < mn_size && k < k_size);
     }
     __device__ __forceinline__ bool in_range4(int mn, int k) const {
         return FAST_K ? (mn < mn_size && k + 3 < k_size) : (mn + 3 < mn_size && k < k_size);

@@ -160,3 +160,18 @@ def test_errors_like_reference(dev):
         dev.gemm(1.0, a, dev.empty((5, 3), torch.float32), 0.0, dev.empty((4, 4), torch.float32))
     with pytest.raises(ag.AgError, match="unimplemented"):
         dev.dot(dev.empty((2, 2), torch.float64), dev.empty((2, 2), torch.float64))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (3, 512, 16), (5, 511, 10), (149, 84, 10), (600, 7, 3), (4096, 84, 10)])
+def test_dense_with_few_outputs(dev, dtype, m, k, n):
+    """One, two and four rows per CTA with ragged ends, against float64: k products and additions of f32 are within
+    (k + 2) * 2^-24 of the sum of magnitudes, and bf16 rounds twice more."""
+    gen = torch.Generator(device=dev.torch_device).manual_seed(m + n)
+    x, w, b = (torch.rand(s, generator=gen, device=dev.torch_device).sub_(0.5).to(dtype) for s in ((m, k), (k, n), (n,)))
+    got = dev.dense_forward(x, w, bias=b, relu=True).double()
+    want = (x.double() @ w.double() + b.double()).clamp(min=0)
+    bound = (k + 2) * 2.0 ** -24 * (x.double().abs() @ w.double().abs() + b.double().abs())
+    if dtype == torch.bfloat16:
+        bound += 2.0 ** -7 * (want.abs() + b.double().abs() + bound)
+    assert ((got - want).abs() <= bound).all()
