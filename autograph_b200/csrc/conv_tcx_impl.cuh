@@ -38,6 +38,8 @@ static ConvMap conv_map(int64_t channels, int64_t sh, int64_t sw, int64_t gh, in
 template <class T>
 __global__ void repack_kernel(const T *w, T *out, int total, int channels, int cp, int s_row, int s_c,
                               FastDiv div_k, FastDiv div_cp) {
+    let_dependents_launch();
+    dependency_wait();
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;
     if (i >= (uint32_t)total) return;
     uint32_t row, k, tap, c;
@@ -61,9 +63,7 @@ static int patches_times_filters(ag_device *dev, const T *src, const ConvMap &ma
         staging(dev, (size_t)total * sizeof(T), &ws) != AG_OK)
         return gemm<T>(dev, M, N, K, ConvRows<T>{src, map, M}, FilterRows<T>{w, s_row, s_c, map.channels, map.div_cp}, E);
     T *packed = (T *)ws;
-    repack_kernel<T><<<(unsigned)ceil_div(total, 256), 256, 0, dev->stream>>>(
-        w, packed, total, map.channels, map.cp, s_row, s_c, FastDiv((uint32_t)K), map.div_cp);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, repack_kernel<T>, dim3((unsigned)ceil_div(total, 256)), 256, 0, w, packed, total, map.channels, map.cp, s_row, s_c, FastDiv((uint32_t)K), map.div_cp)));
     return gemm<T>(dev, M, N, K, ConvRows<T>{src, map, M}, strided<kVecK>((const T *)packed, K, 1, N), E);
 }
 
@@ -97,6 +97,8 @@ template <class T>
 __global__ void __launch_bounds__(256)
     taps_to_image_kernel(const float *col, T *dx, ConvMap g, int grid_hw, int64_t positions,
                          int total, FastDiv div_hw, FastDiv div_w, FastDiv div_c) {
+    let_dependents_launch();
+    dependency_wait();
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;
     if (i >= (uint32_t)total) return;
     uint32_t plane, r, y, x, b, c;
@@ -151,10 +153,7 @@ int conv_backward_input(ag_device *dev, const T *w, int64_t oc, int64_t ic, cons
                            ConvRows<T>{dy + b * oc * oh * ow, conv_map(oc, oh, ow, oh, ow, &point, false), (int)positions},
                            strided<kByRow>(w, 1, taps_n, taps_n), StridedOut<float>{col, 1, positions, 1.f, 0.f}));
             const int total = (int)(n * ic * ih * iw);
-            taps_to_image_kernel<T><<<(unsigned)ceil_div(total, 256), 256, 0, dev->stream>>>(
-                col, dx + b * ic * ih * iw, map, (int)(oh * ow), positions, total, FastDiv((uint32_t)(ih * iw)),
-                FastDiv((uint32_t)iw), FastDiv((uint32_t)ic));
-            AG_CHECK_LAUNCH();
+            AG_TRY((launch_dependent(dev, taps_to_image_kernel<T>, dim3((unsigned)ceil_div(total, 256)), 256, 0, col, dx + b * ic * ih * iw, map, (int)(oh * ow), positions, total, FastDiv((uint32_t)(ih * iw)), FastDiv((uint32_t)iw), FastDiv((uint32_t)ic))));
         }
         return AG_OK;
     }

@@ -269,6 +269,8 @@ __device__ __forceinline__ void store_tile(const Op &op, float *S, int tid,
 template <class Cfg, class AOp, class BOp, class Epi>
 __global__ void __launch_bounds__(Cfg::THREADS, Cfg::MIN_BLOCKS)
     gemm_simt_kernel(int M, int N, int K, int k_chunk, AOp A, BOp B, Epi E) {
+    let_dependents_launch();
+    dependency_wait();
     constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, TM = Cfg::TM, TN = Cfg::TN;
     constexpr int THREADS = Cfg::THREADS;
     constexpr int PA = BM + Cfg::PAD, PB = BN + Cfg::PAD;
@@ -450,6 +452,8 @@ __device__ __forceinline__ void small_k_slot(int tid, int &mn, int &kb) {
 template <class AOp, class BOp, class Epi>
 __global__ void __launch_bounds__(256)
     gemm_small_k_kernel(int M, int N, int K, AOp A, BOp B, Epi E) {
+    let_dependents_launch();
+    dependency_wait();
     __shared__ __align__(16) float As[kSmallK][kSmallPitch];
     __shared__ __align__(16) float Bs[kSmallK][kSmallPitch];
     const int tid = threadIdx.x;
@@ -525,6 +529,8 @@ __global__ void __launch_bounds__(256)
 template <class Epi>
 __global__ void splitk_reduce_kernel(const float *ws, int64_t plane, int splits, int M, int N,
                                      Epi E) {
+    let_dependents_launch();
+    dependency_wait();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= plane) return;
     float s = 0.f;
@@ -539,6 +545,8 @@ __global__ void splitk_reduce_kernel(const float *ws, int64_t plane, int splits,
 template <class Epi>
 __global__ void __launch_bounds__(256)
     splitk_reduce_small_kernel(const float *ws, int64_t plane, int splits, int M, int N, Epi E) {
+    let_dependents_launch();
+    dependency_wait();
     __shared__ float part[8][32];
     const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
     const int64_t i = (int64_t)blockIdx.x * 32 + lane;

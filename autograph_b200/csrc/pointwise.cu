@@ -55,6 +55,8 @@ static bool aligned16(const T *p) {
 template <class T, class F>
 __global__ void map2_kernel(const T *a, const T *b, T *out,
                             int64_t n, bool vec, F f) {
+    let_dependents_launch();
+    dependency_wait();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     constexpr int V = Vec16<T>::N;
@@ -85,9 +87,7 @@ static int map2(ag_device *dev, const T *a, const T *b, T *out, int64_t n, F f) 
     const bool vec = aligned16(a) && aligned16(out) && (b == nullptr || aligned16(b));
     const int threads = 256;
     const int64_t items = vec ? ceil_div(n, Vec16<T>::N) : n;
-    map2_kernel<T, F><<<grid_for(items, threads, dev->sm_count), threads, 0, dev->stream>>>(
-        a, b, out, n, vec, f);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, map2_kernel<T, F>, dim3(grid_for(items, threads, dev->sm_count)), threads, 0, a, b, out, n, vec, f)));
     return AG_OK;
 }
 
@@ -137,6 +137,8 @@ __global__ void max_pool2_kernel(const T *__restrict__ x, T *__restrict__ y, int
 template <class T>
 __global__ void max_pool2_2x2_kernel(const T *__restrict__ x, T *__restrict__ y, int64_t planes,
                                      int ih, int iw, int oh, int ow) {
+    let_dependents_launch();
+    dependency_wait();
     constexpr int V = Vec16<T>::N;  // inputs per vector
     const int vec_per_row = iw / V;
     const int64_t total = planes * oh * vec_per_row;
@@ -199,6 +201,8 @@ __global__ void max_pool2_backward_kernel(T *__restrict__ dx, const T *__restric
 template <class T>
 __global__ void max_pool2_backward_2x2_kernel(const T *src, T *dx, const T *__restrict__ dy,
                                               int64_t planes, int ih, int iw, int oh, int ow) {
+    let_dependents_launch();
+    dependency_wait();
     constexpr int V = Vec16<T>::N;
     const int vec_per_row = iw / V;
     const int64_t total = planes * oh * vec_per_row;
@@ -273,6 +277,8 @@ __device__ __forceinline__ void store_cell(float *p, uint32_t a) { *p = __uint_a
 // RELU: the window is taken over relu(x) (x >= 0 ? x : 0), i.e. Relu followed by the pool.
 template <class T, bool RELU, bool PAIR>
 __global__ void __launch_bounds__(256) max_pool2_2x2_window_kernel(const T *__restrict__ x, T *__restrict__ y, const PoolMap m) {
+    let_dependents_launch();
+    dependency_wait();
     const uint32_t step = gridDim.x * 256u;
     for (uint32_t i0 = blockIdx.x * 256u + threadIdx.x; i0 < m.total; i0 += kPoolWindows * step) {
         uint32_t v[kPoolWindows][4];
@@ -337,6 +343,8 @@ __device__ __forceinline__ void store_row(T *p, uint32_t a, uint32_t b, bool row
 template <class T, bool RELU, bool PAIR>
 __global__ void __launch_bounds__(256) max_pool2_backward_2x2_window_kernel(const T *src, T *dx, const T *__restrict__ dy,
                                                                             const PoolMap m, int oh, int ow) {
+    let_dependents_launch();
+    dependency_wait();
     const uint32_t step = gridDim.x * 256u, lane = threadIdx.x % 32;
     // whole warps: i0 - lane is the warp's first window
     for (uint32_t i0 = blockIdx.x * 256u + threadIdx.x; i0 - lane < m.total; i0 += kPoolWindows * step) {
@@ -421,8 +429,7 @@ static int for_pool_planes(ag_device *dev, int64_t planes, int64_t ih, int64_t i
             const int64_t n = std::min(at_once, planes - p), band = std::min(rows, gh - y);
             const PoolMap m{(int)(y + band == gh ? ih - 2 * y : 2 * band), (int)iw, (int)band, (int)gw,
                             (uint32_t)(n * band * gw), FastDiv((uint32_t)gw), FastDiv((uint32_t)band)};
-            launch(p, y, m, grid_for(ceil_div((int64_t)m.total, kPoolWindows), 256, dev->sm_count));
-            AG_CHECK_LAUNCH();
+            AG_TRY(launch(p, y, m, dim3(grid_for(ceil_div((int64_t)m.total, kPoolWindows), 256, dev->sm_count))));
         }
     return AG_OK;
 }
@@ -435,11 +442,11 @@ static bool pair_aligned(const T *p) {
 template <class T, bool RELU>
 static int pool_windows(ag_device *dev, const T *x, T *y, int64_t planes, int64_t ih, int64_t iw, int64_t oh, int64_t ow) {
     const bool pair = (iw & 1) == 0 && pair_aligned(x);
-    return for_pool_planes(dev, planes, ih, iw, oh, ow, [&](int64_t p, int64_t y0, const PoolMap &m, unsigned grid) {
+    return for_pool_planes(dev, planes, ih, iw, oh, ow, [&](int64_t p, int64_t y0, const PoolMap &m, dim3 grid) {
         const T *src = x + (p * ih + 2 * y0) * iw;
         T *dst = y + (p * oh + y0) * ow;
-        if (pair) max_pool2_2x2_window_kernel<T, RELU, true><<<grid, 256, 0, dev->stream>>>(src, dst, m);
-        else max_pool2_2x2_window_kernel<T, RELU, false><<<grid, 256, 0, dev->stream>>>(src, dst, m);
+        return launch_dependent(dev, pair ? max_pool2_2x2_window_kernel<T, RELU, true> : max_pool2_2x2_window_kernel<T, RELU, false>, grid,
+                                256, 0, src, dst, m);
     });
 }
 
@@ -448,11 +455,13 @@ static int pool_windows_backward(ag_device *dev, const T *x, T *dx, const T *dy,
                                  int64_t ow) {
     // pairs: every cell is in a window
     const bool pair = (iw & 1) == 0 && (ih & 1) == 0 && pair_aligned(x) && pair_aligned(dx);
-    return for_pool_planes(dev, planes, ih, iw, (ih + 1) / 2, (iw + 1) / 2, [&](int64_t p, int64_t y0, const PoolMap &m, unsigned grid) {
+    return for_pool_planes(dev, planes, ih, iw, (ih + 1) / 2, (iw + 1) / 2, [&](int64_t p, int64_t y0, const PoolMap &m, dim3 grid) {
         const T *src = x + (p * ih + 2 * y0) * iw, *g = dy + (p * oh + y0) * ow;
         T *dst = dx + (p * ih + 2 * y0) * iw;
-        if (pair) max_pool2_backward_2x2_window_kernel<T, RELU, true><<<grid, 256, 0, dev->stream>>>(src, dst, g, m, (int)oh, (int)ow);
-        else max_pool2_backward_2x2_window_kernel<T, RELU, false><<<grid, 256, 0, dev->stream>>>(src, dst, g, m, (int)oh, (int)ow);
+        return launch_dependent(dev,
+                                pair ? max_pool2_backward_2x2_window_kernel<T, RELU, true>
+                                     : max_pool2_backward_2x2_window_kernel<T, RELU, false>,
+                                grid, 256, 0, src, dst, g, m, (int)oh, (int)ow);
     });
 }
 
@@ -668,6 +677,8 @@ template <class T>
 __global__ void __launch_bounds__(256)
     bias_grad_planes_kernel(const T *__restrict__ x, float *__restrict__ partial, int64_t cols, int64_t inner, int64_t units,
                             int64_t units_per_chunk, int units_per_row, int *__restrict__ arrivals, T *__restrict__ y, float beta) {
+    let_dependents_launch();
+    dependency_wait();
     constexpr int V = Vec16<T>::N;
     __shared__ float part[8];
     __shared__ bool last;
@@ -761,9 +772,7 @@ static int bias_grad_planes(ag_device *dev, const T *x, int64_t rows, int64_t co
     AG_TRY(workspace(dev, sizeof(float) * (size_t)chunks * (size_t)cols, &ws));
     // one launch when every column has a counter
     int *arrivals = cols < kTileCounters ? dev->tile_counters : nullptr;
-    bias_grad_planes_kernel<T><<<dim3((unsigned)cols, (unsigned)chunks), 256, 0, dev->stream>>>(
-        x, (float *)ws, cols, inner, units, per_chunk, (int)per_row, arrivals, y, beta);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, bias_grad_planes_kernel<T>, dim3((unsigned)cols, (unsigned)chunks), 256, 0, x, (float *)ws, cols, inner, units, per_chunk, (int)per_row, arrivals, y, beta)));
     if (arrivals != nullptr) return AG_OK;
     bias_grad_final_kernel<T><<<(unsigned)ceil_div(cols, 32), dim3(32, 8), 0, dev->stream>>>((const float *)ws, y, cols, (int)chunks,
                                                                                              beta);
@@ -878,8 +887,8 @@ static int pool_forward(ag_device *dev, const T *x, T *y, int64_t planes, int ih
     const int64_t plane_bytes = (int64_t)ih * iw * (int64_t)sizeof(T);
     if (h == 2 && w == 2 && sh == 2 && sw == 2 && iw % V == 0 && aligned16(x)) {
         const int64_t items = planes * oh * (iw / V);
-        max_pool2_2x2_kernel<T><<<grid_for(items, threads, dev->sm_count), threads, 0,
-                                  dev->stream>>>(x, y, planes, ih, iw, oh, ow);
+        return launch_dependent(dev, max_pool2_2x2_kernel<T>, dim3(grid_for(items, threads, dev->sm_count)), threads, 0, x, y, planes, ih,
+                                iw, oh, ow);
     } else if (h == 2 && w == 2 && sh == 2 && sw == 2) {
         return pool_windows<T, false>(dev, x, y, planes, ih, iw, oh, ow);
     } else if (plane_bytes <= 40 * 1024 && planes >= dev->sm_count) {
@@ -1005,11 +1014,8 @@ static int pool_backward(ag_device *dev, ag_dtype dtype, const void *x, void *dx
         (reinterpret_cast<uintptr_t>(dx) & 15) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
         ((ih & 1) == 0 || x == dx)) {  // out of place, a last row no window covers must be copied
         const unsigned grid2 = grid_for(planes * oh * (iw / vlen), threads, dev->sm_count);
-        AG_DISPATCH_FLOAT(dtype, T,
-            max_pool2_backward_2x2_kernel<T><<<grid2, threads, 0, dev->stream>>>(
-                (const T *)x, (T *)dx, (const T *)dy, planes, (int)ih, (int)iw, oh, ow););
-        AG_CHECK_LAUNCH();
-        return AG_OK;
+        AG_DISPATCH_FLOAT(dtype, T, return launch_dependent(dev, max_pool2_backward_2x2_kernel<T>, dim3(grid2), threads, 0, (const T *)x,
+                                                            (T *)dx, (const T *)dy, planes, (int)ih, (int)iw, oh, ow););
     }
     if (h == 2 && w == 2 && sh == 2 && sw == 2)
         AG_DISPATCH_FLOAT(dtype, T, return (pool_windows_backward<T, false>(dev, (const T *)x, (T *)dx, (const T *)dy, planes, ih, iw,
