@@ -93,15 +93,17 @@ namespace ag {
 // Programmatic dependent launch.  A kernel launched with launch_dependent may be placed on SMs that its
 // predecessor in the stream has left and set itself up there; after dependency_wait everything the
 // predecessor wrote is visible.  Every thread that touches global memory comes through that wait first.
+// A kernel that allocates tensor memory does so before it lets dependents launch: one that came first could hold the
+// columns it still needs, and wait for it.
 // The operators' kernels are small enough for that to count: a kernel of 2 us in a stream of them took 4 us, and a
 // convolution stage called operator by operator (16 -> 32 3x3, 64 x 32 x 32 f32, eleven launches) 128 us, now 116.
 __device__ __forceinline__ void let_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class... P, class... A>
-int launch_dependent(ag_device *dev, void (*kernel)(P...), dim3 grid, int threads, size_t smem, const A &...args) {
+int launch_dependent(ag_device *dev, void (*kernel)(P...), dim3 grid, dim3 threads, size_t smem, const A &...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3((unsigned)threads);
+    cfg.blockDim = threads;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = dev->stream;
     cudaLaunchAttribute attr;
@@ -251,5 +253,10 @@ struct FastDiv {
 };
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+// Dynamic shared memory of a persistent kernel that wants an SM per CTA.  Launched dependent, its CTAs go to the SMs
+// that its predecessor leaves first, two or three to one if they fit, and the others stay idle (the first layer's
+// convolution of the wide stack 58 us, so 130): more than half of an SM's memory keeps them apart.
+constexpr int kOneCtaPerSm = 116 * 1024;
 
 }  // namespace ag

@@ -42,6 +42,8 @@ __global__ void __launch_bounds__(256, 2)
     conv2_direct_kernel(const T *__restrict__ x, const T *__restrict__ w,
                         const T *__restrict__ bias, T *__restrict__ y, const Params p,
                         T *__restrict__ pre_y) {
+    let_dependents_launch();
+    dependency_wait();
     extern __shared__ __align__(16) float smem[];
     const int img_elems = p.ic * p.ih * p.iw;
     const int taps = p.ic * FH * FW;
@@ -157,6 +159,8 @@ template <class T, int FH, int FW>
 __global__ void __launch_bounds__(256, 2)
     conv2_direct_banded_kernel(const T *__restrict__ x, const T *__restrict__ w,
                                const T *__restrict__ bias, T *__restrict__ y, const Params p) {
+    let_dependents_launch();
+    dependency_wait();
     extern __shared__ __align__(16) float smem[];
     const int img_elems = p.ic * p.ih * p.iw;
     const int taps = p.ic * FH * FW;
@@ -225,8 +229,7 @@ static int launch_banded(ag_device *dev, const T *x, const T *w, const T *bias, 
     if (smem > 48 * 1024)
         AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem));
-    kernel<<<(unsigned)p.bs, 256, smem, dev->stream>>>(x, w, bias, y, p);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, kernel, dim3((unsigned)p.bs), 256, smem, x, w, bias, y, p)));
     return AG_OK;
 }
 
@@ -277,8 +280,7 @@ static int launch(ag_device *dev, const T *x, const T *w, const T *bias, T *y, c
     if (threads > 256) threads = 256;
     if (threads < 64) threads = 64;
     const unsigned grid = (unsigned)ceil_div(p.bs, p.group);
-    kernel<<<grid, threads, smem, dev->stream>>>(x, w, bias, y, p, pre_y);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, kernel, dim3((unsigned)grid), threads, smem, x, w, bias, y, p, pre_y)));
     return AG_OK;
 }
 

@@ -27,6 +27,8 @@ template <class T, int FH, int FW>
 __global__ void __launch_bounds__(1024)
     conv2_wgrad_kernel(const T *__restrict__ x, const T *__restrict__ dy, float *__restrict__ partial,
                        const WgradParams p) {
+    let_dependents_launch();
+    dependency_wait();
     extern __shared__ __align__(16) float smem[];
     const int oh = p.ih - FH + 1, ow = p.iw - FW + 1;
     const int x_elems = p.ic * p.ih * p.iw, dy_elems = p.oc * oh * ow;
@@ -102,6 +104,8 @@ template <class T>
 __global__ void __launch_bounds__(256)
     conv2_wgrad_reduce_kernel(const float *__restrict__ partial, int planes, int len, float beta,
                               T *__restrict__ dw) {
+    let_dependents_launch();
+    dependency_wait();
     __shared__ float part[8][32];
     const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
     const int i = blockIdx.x * 32 + lane;
@@ -169,11 +173,8 @@ static int launch_wgrad(ag_device *dev, const T *x, const T *dy, const WgradPara
     void *ws = nullptr;
     AG_TRY(workspace(dev, sizeof(float) * (size_t)ctas * (size_t)len, &ws));
     const int threads = ((p.items * p.slices + 31) / 32) * 32;
-    kernel<<<ctas, threads, smem, dev->stream>>>(x, dy, (float *)ws, p);
-    AG_CHECK_LAUNCH();
-    conv2_wgrad_reduce_kernel<T><<<(unsigned)ceil_div(len, 32), 256, 0, dev->stream>>>(
-        (const float *)ws, ctas, len, beta, dw);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, kernel, dim3((unsigned)ctas), threads, smem, x, dy, (float *)ws, p)));
+    AG_TRY((launch_dependent(dev, conv2_wgrad_reduce_kernel<T>, dim3((unsigned)ceil_div(len, 32)), 256, 0, (const float *)ws, ctas, len, beta, dw)));
     return AG_OK;
 }
 

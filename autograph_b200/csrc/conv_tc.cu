@@ -128,13 +128,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     // one output-channel block per CTA keeps its bias resident; with several blocks the
     // epilogue reads the bias from global memory
     const bool bias_resident = p.n_blocks == 1;
-    if (bias_resident)
-        for (int i = threadIdx.x; i < BLOCK_N; i += NUM_THREADS)
-            s_bias[i] = (p.bias != nullptr && i < p.OC) ? __bfloat162float(p.bias[i]) : 0.f;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    let_dependents_launch();
+    dependency_wait();
+    if (bias_resident)
+        for (int i = threadIdx.x; i < BLOCK_N; i += NUM_THREADS)
+            s_bias[i] = (p.bias != nullptr && i < p.OC) ? __bfloat162float(p.bias[i]) : 0.f;
+    __syncthreads();
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
@@ -304,6 +307,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 __global__ void __launch_bounds__(256)
     nchw_to_nhwc_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ out, int C,
                         int HW, int Cp, int W, int Hp, int Wp, int pad_h, int pad_w) {
+    let_dependents_launch();
+    dependency_wait();
     const int px = blockIdx.x * 256 + threadIdx.x;
     if (px >= HW) return;
     const int c0 = blockIdx.y * 16;
@@ -335,6 +340,8 @@ constexpr int NCHW_PITCH = NCHW_PIX + 16;
 __global__ void __launch_bounds__(256)
     nhwc_to_nchw_kernel(const __nv_bfloat16 *__restrict__ in, __nv_bfloat16 *__restrict__ out, int C,
                         int HW, int Cp) {
+    let_dependents_launch();
+    dependency_wait();
     __shared__ __align__(16) unsigned short tile[16 * NCHW_PITCH];
     const int p0 = blockIdx.x * NCHW_PIX;
     const int c0 = blockIdx.y * 16;
@@ -377,6 +384,8 @@ __global__ void __launch_bounds__(256)
 __global__ void repack_filters_kernel(const __nv_bfloat16 *__restrict__ w,
                                       __nv_bfloat16 *__restrict__ wk, int OC, int IC, int taps,
                                       int Cp) {
+    let_dependents_launch();
+    dependency_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)OC * taps * Cp) return;
     const int c = (int)(i % Cp);
@@ -390,6 +399,8 @@ __global__ void repack_filters_kernel(const __nv_bfloat16 *__restrict__ w,
 __global__ void repack_filters_transposed_kernel(const __nv_bfloat16 *__restrict__ w,
                                                  __nv_bfloat16 *__restrict__ wk, int OC, int IC,
                                                  int taps, int OCp) {
+    let_dependents_launch();
+    dependency_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)IC * taps * OCp) return;
     const int oc = (int)(i % OCp);
@@ -422,10 +433,7 @@ static bool halo_enabled() {
 int to_nhwc(ag_device *dev, const __nv_bfloat16 *x, int64_t bs, int64_t c, int64_t hw, int64_t cp,
             __nv_bfloat16 *out) {
     // no border: the frame is the image, any width gives the same row index
-    nchw_to_nhwc_kernel<<<dim3((unsigned)ceil_div(hw, 256), (unsigned)(cp / 16), (unsigned)bs), 256,
-                          0, dev->stream>>>(x, out, (int)c, (int)hw, (int)cp, (int)hw, 1, (int)hw, 0,
-                                            0);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, nchw_to_nhwc_kernel, dim3((unsigned)ceil_div(hw, 256), (unsigned)(cp / 16), (unsigned)bs), 256, 0, x, out, (int)c, (int)hw, (int)cp, (int)hw, 1, (int)hw, 0, 0)));
     return AG_OK;
 }
 
@@ -434,10 +442,7 @@ int to_nhwc_framed(ag_device *dev, const __nv_bfloat16 *x, int64_t bs, int64_t c
     const int64_t hp = h + 2 * pad_h, wp = w + 2 * pad_w;
     if (pad_h || pad_w)
         AG_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)(bs * hp * wp * cp * 2), dev->stream));
-    nchw_to_nhwc_kernel<<<dim3((unsigned)ceil_div(h * w, 256), (unsigned)(cp / 16), (unsigned)bs),
-                          256, 0, dev->stream>>>(x, out, (int)c, (int)(h * w), (int)cp, (int)w,
-                                                 (int)hp, (int)wp, pad_h, pad_w);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, nchw_to_nhwc_kernel, dim3((unsigned)ceil_div(h * w, 256), (unsigned)(cp / 16), (unsigned)bs), 256, 0, x, out, (int)c, (int)(h * w), (int)cp, (int)w, (int)hp, (int)wp, pad_h, pad_w)));
     return AG_OK;
 }
 
@@ -489,8 +494,7 @@ static int launch(ag_device *dev, const CUtensorMap &tx, const CUtensorMap &tw, 
     }
     const int64_t tiles = (int64_t)p.B * p.tiles_y * p.tiles_x * p.n_blocks;
     const int grid = (int)(tiles < dev->sm_count ? tiles : dev->sm_count);
-    kernel<<<grid, NUM_THREADS, C::SMEM_BYTES, dev->stream>>>(tx, tw, p);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, kernel, dim3((unsigned)grid), NUM_THREADS, C::SMEM_BYTES, tx, tw, p)));
     return AG_OK;
 }
 
@@ -507,9 +511,7 @@ int64_t nhwc_filter_scratch_bytes(const NhwcConv &c) {
 
 int from_nhwc(ag_device *dev, const __nv_bfloat16 *in, int64_t bs, int64_t c, int64_t hw, int64_t cp,
               __nv_bfloat16 *out) {
-    nhwc_to_nchw_kernel<<<dim3((unsigned)ceil_div(hw, NCHW_PIX), (unsigned)ceil_div(c, 16), (unsigned)bs),
-                          256, 0, dev->stream>>>(in, out, (int)c, (int)hw, (int)cp);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, nhwc_to_nchw_kernel, dim3((unsigned)ceil_div(hw, NCHW_PIX), (unsigned)ceil_div(c, 16), (unsigned)bs), 256, 0, in, out, (int)c, (int)hw, (int)cp)));
     return AG_OK;
 }
 
@@ -531,13 +533,8 @@ int correlate_nhwc(ag_device *dev, const NhwcConv &c, const __nv_bfloat16 *act_n
     const int64_t wk_elems = c_out * taps * cp;
     const int64_t ocp = round_up(c_out, 64);
     const unsigned rgrid = (unsigned)ceil_div(wk_elems, 256);
-    if (c.transposed)
-        repack_filters_transposed_kernel<<<rgrid, 256, 0, dev->stream>>>(w, wk, (int)w_oc, (int)w_ic,
-                                                                         taps, (int)cp);
-    else
-        repack_filters_kernel<<<rgrid, 256, 0, dev->stream>>>(w, wk, (int)w_oc, (int)w_ic, taps,
-                                                              (int)cp);
-    AG_CHECK_LAUNCH();
+    AG_TRY(launch_dependent(dev, c.transposed ? repack_filters_transposed_kernel : repack_filters_kernel, dim3(rgrid), 256, 0, w, wk,
+                            (int)w_oc, (int)w_ic, taps, (int)cp));
     if (halo)
         return run_halo(dev, act_nhwc, wk, bs, cp, hp, wp, fh, fw, c_out, out_h, out_w, bias, relu,
                         out_nhwc);

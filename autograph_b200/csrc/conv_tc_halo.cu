@@ -99,8 +99,6 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    for (int i = threadIdx.x; i < BLOCK_N; i += H_THREADS)
-        s_bias[i] = (p.bias != nullptr && i < p.OC) ? __bfloat162float(p.bias[i]) : 0.f;
     if (warp == 1) {
         tmem_alloc(smem_u32(tmem_base_slot), TMEM_COLS);
         tmem_relinquish();
@@ -109,6 +107,11 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    let_dependents_launch();
+    dependency_wait();
+    for (int i = threadIdx.x; i < BLOCK_N; i += H_THREADS)
+        s_bias[i] = (p.bias != nullptr && i < p.OC) ? __bfloat162float(p.bias[i]) : 0.f;
+    __syncthreads();
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
@@ -267,6 +270,7 @@ template <int BLOCK_N>
 int launch_halo(ag_device *dev, const CUtensorMap &tx, const CUtensorMap &tw, const HaloParams &p,
                 int smem) {
     auto kernel = conv2_bf16_tc_halo_kernel<BLOCK_N>;
+    if (smem < kOneCtaPerSm) smem = kOneCtaPerSm;
     // the attribute belongs to the (kernel, GPU) pair: largest size set so far, per
     // instantiation and GPU
     static int configured_on[64] = {};
@@ -277,8 +281,7 @@ int launch_halo(ag_device *dev, const CUtensorMap &tx, const CUtensorMap &tw, co
     }
     const int tiles = (p.R + HB_M - 1) / HB_M;
     const int grid = tiles < dev->sm_count ? tiles : dev->sm_count;
-    kernel<<<grid, H_THREADS, smem, dev->stream>>>(tx, tw, p);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, kernel, dim3((unsigned)grid), H_THREADS, smem, tx, tw, p)));
     return AG_OK;
 }
 

@@ -100,6 +100,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    let_dependents_launch();
+    dependency_wait();
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
@@ -230,6 +232,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
 __global__ void wgrad_reduce_kernel(const float *__restrict__ partial, int splits, int64_t m_total,
                                     int taps, int Cp, int OC, int IC, float beta,
                                     __nv_bfloat16 *__restrict__ dw) {
+    let_dependents_launch();
+    dependency_wait();
     __shared__ float part[8][33];
     const int64_t i = (int64_t)blockIdx.x * 32 + threadIdx.x;
     const bool live = i < (int64_t)OC * taps * IC;
@@ -265,7 +269,7 @@ template <int NT>
 int launch_wgrad(ag_device *dev, const CUtensorMap &tdy, const CUtensorMap &tx, const WgParams &p,
                  int grid) {
     auto kernel = conv2_wgrad_bf16_tc_kernel<NT>;
-    const int smem = p.stages * p.stage_bytes + 1024 + 256;
+    const int need = p.stages * p.stage_bytes + 1024 + 256, smem = need < kOneCtaPerSm ? kOneCtaPerSm : need;
     // the attribute belongs to the (kernel, GPU) pair: largest size set so far, per
     // instantiation and GPU
     static int configured_on[64] = {};
@@ -274,8 +278,7 @@ int launch_wgrad(ag_device *dev, const CUtensorMap &tdy, const CUtensorMap &tx, 
         AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         configured = smem;
     }
-    kernel<<<grid, WG_THREADS, smem, dev->stream>>>(tdy, tx, p);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, kernel, dim3((unsigned)grid), WG_THREADS, smem, tdy, tx, p)));
     return AG_OK;
 }
 
@@ -391,9 +394,7 @@ int backward_weight_nhwc(ag_device *dev, const __nv_bfloat16 *xh, int64_t bs, in
     else
         AG_TRY(launch_wgrad<64>(dev, tdy, tx, p, grid));
     const int64_t outs = oc * p.taps * ic;
-    wgrad_reduce_kernel<<<(unsigned)ceil_div(outs, 32), dim3(32, 8), 0, dev->stream>>>(
-        p.partial, splits, m_total, p.taps, (int)cp, (int)oc, (int)ic, beta, dw);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, wgrad_reduce_kernel, dim3((unsigned)ceil_div(outs, 32)), dim3(32, 8), 0, p.partial, splits, m_total, p.taps, (int)cp, (int)oc, (int)ic, beta, dw)));
     return AG_OK;
 }
 

@@ -116,6 +116,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    let_dependents_launch();
+    dependency_wait();
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
@@ -421,8 +423,7 @@ static int launch(ag_device *dev, const CUtensorMap &ta, const CUtensorMap &tb, 
     }
     const int tiles = (int)(ceil_div(p.M, BLOCK_M) * ceil_div(p.N, BLOCK_N)) * p.splits;
     const int grid = tiles < dev->sm_count ? tiles : dev->sm_count;
-    kernel<<<grid, NUM_THREADS, SMEM_BYTES, dev->stream>>>(ta, tb, p);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, kernel, dim3((unsigned)grid), NUM_THREADS, SMEM_BYTES, ta, tb, p)));
     return AG_OK;
 }
 
@@ -495,15 +496,12 @@ int gemm_bf16(ag_device *dev, int m, int k, int n, float alpha, const __nv_bfloa
         if (epi) {
             using Epi = simt::BiasReluEpilogue<__nv_bfloat16>;
             Epi E{c, rsc, epi->bias, epi->relu};
-            simt::splitk_reduce_kernel<Epi><<<(unsigned)ceil_div(plane, 256), 256, 0, dev->stream>>>(
-                p.partial, plane, splits, m, n, E);
+            AG_TRY((launch_dependent(dev, simt::splitk_reduce_kernel<Epi>, dim3((unsigned)ceil_div(plane, 256)), 256, 0, p.partial, plane, splits, m, n, E)));
         } else {
             using Epi = simt::StridedEpilogue<__nv_bfloat16>;
             Epi E{c, rsc, 1, alpha, beta, false, n};
-            simt::splitk_reduce_kernel<Epi><<<(unsigned)ceil_div(plane, 256), 256, 0, dev->stream>>>(
-                p.partial, plane, splits, m, n, E);
+            AG_TRY((launch_dependent(dev, simt::splitk_reduce_kernel<Epi>, dim3((unsigned)ceil_div(plane, 256)), 256, 0, p.partial, plane, splits, m, n, E)));
         }
-        AG_CHECK_LAUNCH();
     }
     return AG_OK;
 }

@@ -69,6 +69,8 @@ template <int FH, int FW>
 __global__ void __launch_bounds__(256)
     im2col_rows_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ out, int ic, int ih, int iw, int oh,
                        int ow, int rows) {
+    let_dependents_launch();
+    dependency_wait();
     extern __shared__ __align__(16) unsigned short staged[];   // [ic][rows + FH - 1][iw]
     constexpr int taps = FH * FW, groups = 8;
     const int64_t b = blockIdx.y;
@@ -128,6 +130,8 @@ bool launch_im2col_rows(ag_device *dev, const __nv_bfloat16 *x, __nv_bfloat16 *o
 
 __global__ void relu_pool_kernel(const __nv_bfloat16 *__restrict__ pre, __nv_bfloat16 *__restrict__ y,
                                  uint32_t *__restrict__ codes, int ih, int iw, int ph, int pw, int cp, int64_t total) {
+    let_dependents_launch();
+    dependency_wait();
     const int groups = cp / 8;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -173,6 +177,8 @@ __global__ void relu_pool_backward_kernel(const __nv_bfloat16 *__restrict__ pre,
                                           const __nv_bfloat16 *__restrict__ dy, __nv_bfloat16 *__restrict__ out,
                                           int ih, int iw, int ph, int pw, int cp, int64_t row_pitch,
                                           int64_t image_pitch, int64_t total) {
+    let_dependents_launch();
+    dependency_wait();
     const int groups = cp / 8;
     const int wh = (ih + 1) / 2, ww = (iw + 1) / 2;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -230,6 +236,8 @@ __global__ void relu_pool_backward_kernel(const __nv_bfloat16 *__restrict__ pre,
 
 __global__ void zero_frame_kernel(__nv_bfloat16 *framed, int hp, int wp, int pad_h, int pad_w, int cp,
                                   int64_t cells_per_image, int64_t total) {
+    let_dependents_launch();
+    dependency_wait();
     const int groups = cp / 8;
     const int64_t band = (int64_t)pad_h * wp;   // cells of the top (and of the bottom) rows
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -308,9 +316,7 @@ int relu_pool(ag_device *dev, const __nv_bfloat16 *pre, int64_t bs, int64_t ih, 
     const int64_t ph = ih / 2, pw = iw / 2;
     const int64_t total = bs * ph * pw * (cp / 8);
     if (total == 0) return AG_OK;
-    relu_pool_kernel<<<grid_for(dev, total), 256, 0, dev->stream>>>(pre, y, codes, (int)ih, (int)iw, (int)ph,
-                                                                   (int)pw, (int)cp, total);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, relu_pool_kernel, dim3(grid_for(dev, total)), 256, 0, pre, y, codes, (int)ih, (int)iw, (int)ph, (int)pw, (int)cp, total)));
     return AG_OK;
 }
 
@@ -324,10 +330,7 @@ int relu_pool_backward(ag_device *dev, const __nv_bfloat16 *pre, const uint32_t 
     AG_REQUIRE(pre != nullptr || (ih % 2 == 0 && iw % 2 == 0), AG_ERR_INVALID, "relu_pool_backward: odd planes need pre");
     const int64_t total = bs * ((ih + 1) / 2) * ((iw + 1) / 2) * (cp / 8);
     if (total == 0) return AG_OK;
-    relu_pool_backward_kernel<<<grid_for(dev, total), 256, 0, dev->stream>>>(
-        pre, codes, dy, out, (int)ih, (int)iw, (int)(ih / 2), (int)(iw / 2), (int)cp, out_row_pitch,
-        out_image_pitch, total);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, relu_pool_backward_kernel, dim3(grid_for(dev, total)), 256, 0, pre, codes, dy, out, (int)ih, (int)iw, (int)(ih / 2), (int)(iw / 2), (int)cp, out_row_pitch, out_image_pitch, total)));
     return AG_OK;
 }
 
@@ -337,9 +340,7 @@ int zero_frame(ag_device *dev, __nv_bfloat16 *framed, int64_t bs, int64_t hp, in
     const int64_t cells = 2 * (int64_t)pad_h * wp + 2 * (int64_t)pad_w * (hp - 2 * pad_h);
     const int64_t total = bs * cells * (cp / 8);
     if (total <= 0) return AG_OK;
-    zero_frame_kernel<<<grid_for(dev, total), 256, 0, dev->stream>>>(framed, (int)hp, (int)wp, pad_h,
-                                                                    pad_w, (int)cp, cells, total);
-    AG_CHECK_LAUNCH();
+    AG_TRY((launch_dependent(dev, zero_frame_kernel, dim3(grid_for(dev, total)), 256, 0, framed, (int)hp, (int)wp, pad_h, pad_w, (int)cp, cells, total)));
     return AG_OK;
 }
 
