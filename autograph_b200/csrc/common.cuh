@@ -255,8 +255,8 @@ struct FastDiv {
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // Dynamic shared memory of a persistent kernel that wants an SM per CTA.  Launched dependent, its CTAs go to the SMs
-// that its predecessor leaves first, two or three to one if they fit, and the others stay idle (the first layer's
-// convolution of the wide stack 58 us, so 130): more than half of an SM's memory keeps them apart.
+// that its predecessor leaves first, two or three to one if they fit, and the others stay idle (the wide stack at 256
+// images bf16: inference 203 us, so 289, a training step 492 and 569): more than half of an SM's memory keeps them apart.
 constexpr int kOneCtaPerSm = 116 * 1024;
 
 }  // namespace ag
