@@ -83,6 +83,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     float *xa = reinterpret_cast<float *>(smem + pl.xa_off), *xb = reinterpret_cast<float *>(smem + pl.xb_off);
     const uint32_t bar_w = tc::smem_u32(smem + pl.bar_off);   // weight copy
     const uint32_t bar_tile0 = bar_w + 8;                      // [TILES] MMA completion
+    if (warp == 0) {   // tensor memory for the eight accumulators, before a dependent can take any
+        tc::tmem_alloc(tc::smem_u32(&s_tmem), TMEM_COLS);
+        tc::tmem_relinquish();
+    }
+    __syncthreads();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     AG_STAMP(0);
@@ -101,10 +106,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (pl.w_smem[l] >= 0)
                     tc::bulk_load(tc::smem_u32(smem + pl.w_smem[l]), pl.chain.s[l].w, (uint32_t)pl.w_bytes[l], bar_w);
         }
-    }
-    if (warp == 0) {   // tensor memory for the eight accumulators
-        tc::tmem_alloc(tc::smem_u32(&s_tmem), TMEM_COLS);
-        tc::tmem_relinquish();
     }
 
     // ---- images, conv1 filter bank; zeroed operand buffers; conv2 filter bank as B operands
