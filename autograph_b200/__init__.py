@@ -216,7 +216,17 @@ class _PyDevice:
         torch.cuda.current_stream(self.index).synchronize()
         return out
 
-    def _sync_in(self):
+    def _sync_in(self, *tensors, strided=False):
+        """Refuses operands whose addresses this GPU's kernels cannot use: host memory (unless it is page-locked, which
+        they can read; and then without a copy on the way, which would not be) and other GPUs'.  None stands for an
+        operand that is absent."""
+        for t in tensors:
+            if t is None or (t.is_cuda and t.device.index == self.index):
+                continue
+            if t.is_cuda:
+                raise AgError(_capi.AG_ERR_INVALID, f"tensor of shape {tuple(t.shape)} is on another GPU")
+            if not ((strided or t.is_contiguous()) and t.is_pinned()):
+                raise AgError(_capi.AG_ERR_INVALID, f"tensor of shape {tuple(t.shape)} must be in device memory")
         # Inputs were produced on torch's current stream; order this stream after it (nothing
         # to do when that stream is this device's own, which is the case unless the caller
         # changed torch's current stream after creating the device).
@@ -240,7 +250,7 @@ class _PyDevice:
             raise AgError(_capi.AG_ERR_SHAPE, f"a_cols != b_rows, {k} != {k2}")
         if n != n2:
             raise AgError(_capi.AG_ERR_SHAPE, f"b_cols != c_rows, {n} != {n2}")
-        self._sync_in()
+        self._sync_in(a, b, c, strided=True)
         self._check(lib().ag_gemm(
             self._h, _dtype_code(a.dtype), m, k, n, ctypes.c_float(alpha),
             _ptr(a), 0, a.stride(0), a.stride(1), _ptr(b), 0, b.stride(0), b.stride(1),
@@ -274,7 +284,7 @@ class _PyDevice:
         o = _conv_options((fh, fw), padding, stride, dilation)
         oh, ow = self.conv2_output_shape(ih, iw, (fh, fw), padding, stride, dilation)
         y = self._out((bs, oc, oh, ow), x.dtype)
-        self._sync_in()
+        self._sync_in(x, w, bias)
         self._check(lib().ag_conv2_forward(self._h, _dtype_code(x.dtype), _ptr(x.contiguous()), bs,
                                            ic, ih, iw, _ptr(w.contiguous()), oc, _ptr(bias),
                                            ctypes.byref(o), int(relu), _ptr(y)))
@@ -293,7 +303,7 @@ class _PyDevice:
             raise AgError(_capi.AG_ERR_SHAPE, "pool window does not fit the convolution output")
         y = self._out((bs, oc, (oh - pool[0]) // pool[0] + 1, (ow - pool[1]) // pool[1] + 1),
                        x.dtype)
-        self._sync_in()
+        self._sync_in(x, w, bias)
         self._check(lib().ag_conv2_relu_max_pool2_forward(
             self._h, _dtype_code(x.dtype), _ptr(x.contiguous()), bs, ic, ih, iw,
             _ptr(w.contiguous()), oc, _ptr(bias), ctypes.byref(o), int(relu), pool[0], pool[1],
@@ -312,7 +322,7 @@ class _PyDevice:
         oh, ow = self.conv2_output_shape(ih, iw, (fh, fw), padding, stride, dilation)
         pre = self._out((bs, oc, oh, ow), x.dtype)
         y = self._out((bs, oc, oh // 2, ow // 2), x.dtype)
-        self._sync_in()
+        self._sync_in(x, w, bias)
         self._check(lib().ag_conv2_relu_max_pool2_forward_keep(
             self._h, _dtype_code(x.dtype), _ptr(x.contiguous()), bs, ic, ih, iw,
             _ptr(w.contiguous()), oc, _ptr(bias), ctypes.byref(o), _ptr(pre), _ptr(y)))
@@ -325,7 +335,7 @@ class _PyDevice:
         if x.shape[1] != w.shape[0]:
             raise AgError(_capi.AG_ERR_SHAPE, f"a_cols != b_rows, {x.shape[1]} != {w.shape[0]}")
         y = self._out((x.shape[0], w.shape[1]), x.dtype)
-        self._sync_in()
+        self._sync_in(x, w, bias)
         self._check(lib().ag_dense_forward(self._h, _dtype_code(x.dtype), _ptr(x.contiguous()),
                                            x.shape[0], x.shape[1], _ptr(w.contiguous()),
                                            w.shape[1], _ptr(bias), int(relu), _ptr(y)))
@@ -341,7 +351,7 @@ class _PyDevice:
         bs = (ctypes.c_void_p * n)(*[(b.data_ptr() if b is not None else None) for b in biases])
         rl = (ctypes.c_int32 * n)(*[int(r) for r in relus])
         y = self._out((x.shape[0], weights[-1].shape[1]), x.dtype)
-        self._sync_in()
+        self._sync_in(x, *weights, *biases)
         self._check(lib().ag_dense_chain_forward(self._h, _dtype_code(x.dtype),
                                                  _ptr(x.contiguous()), x.shape[0], n, dims, ws, bs,
                                                  rl, _ptr(y)))
@@ -362,7 +372,7 @@ class _PyDevice:
                for w, r in zip(weights, relus)]
         pp = (ctypes.c_void_p * n)(*[_ptr(t) for t in pre])
         ap = (ctypes.c_void_p * n)(*[(_ptr(t) if t is not None else None) for t in act])
-        self._sync_in()
+        self._sync_in(x, *weights, *biases)
         self._check(lib().ag_dense_chain_forward_keep(self._h, _dtype_code(x.dtype),
                                                       _ptr(x.contiguous()), x.shape[0], n, dims, ws,
                                                       bs, rl, pp, ap))
@@ -384,7 +394,7 @@ class _PyDevice:
         if not relus[-1]:
             g[-1] = dy
         arr = lambda ts: (ctypes.c_void_p * n)(*[(_ptr(t) if t is not None else None) for t in ts])
-        self._sync_in()
+        self._sync_in(*ins, dy, *weights, *pre, *act)
         self._check(lib().ag_dense_chain_backward(
             self._h, _dtype_code(dt), x.shape[0], n, dims, arr(ins),
             arr([w.contiguous() for w in weights]), arr([pre[i] if relus[i] else None for i in range(n)]),
@@ -426,7 +436,7 @@ class _PyDevice:
     def scaled_cast_u8(self, x_u8, alpha, dtype):
         """≙ Tensor::scaled_cast for u8 input: alpha * x in `dtype` (f32 or bf16)."""
         y = self._out(tuple(x_u8.shape), dtype)
-        self._sync_in()
+        self._sync_in(x_u8)
         self._check(lib().ag_scaled_cast_u8(self._h, _dtype_code(dtype), ctypes.c_float(alpha),
                                             _ptr(x_u8.contiguous()), _ptr(y), x_u8.numel()))
         return y
@@ -459,7 +469,7 @@ class _PyDevice:
         rl = (ctypes.c_int32 * n)(*[int(r) for r in relus])
         out_dtype = weights[0].dtype
         y = self._out((bs, weights[-1].shape[1]), out_dtype)
-        self._sync_in()
+        self._sync_in(x, *(t for w, b, _, _ in convs for t in (w, b)), *weights, *biases)
         if u8_alpha is not None:
             self._check(lib().ag_conv_dense_chain_forward_u8(
                 self._h, _dtype_code(out_dtype), _ptr(x.contiguous()), ctypes.c_float(u8_alpha), bs,
@@ -477,7 +487,7 @@ class _PyDevice:
         ih, iw = input_hw
         o = _conv_options((fh, fw), padding, stride, dilation)
         dx = self._out((bs, ic, ih, iw), dy.dtype)
-        self._sync_in()
+        self._sync_in(w, dy)
         self._check(lib().ag_conv2_backward_input(self._h, _dtype_code(dy.dtype),
                                                   _ptr(w.contiguous()), oc, ic,
                                                   _ptr(dy.contiguous()), bs, ih, iw,
@@ -491,7 +501,7 @@ class _PyDevice:
         o = _conv_options(filter, padding, stride, dilation)
         if dw is None:
             dw = self._out((oc, ic, filter[0], filter[1]), x.dtype)
-        self._sync_in()
+        self._sync_in(x, dy, dw)
         self._check(lib().ag_conv2_backward_weight(self._h, _dtype_code(x.dtype),
                                                    _ptr(x.contiguous()), bs, ic, ih, iw,
                                                    _ptr(dy.contiguous()), oc, ctypes.byref(o),
@@ -503,7 +513,7 @@ class _PyDevice:
         o = _conv_options(filter, padding, stride, dilation)
         oh, ow = self.conv2_output_shape(ih, iw, filter, padding, stride, dilation)
         y = self._out((bs * oh * ow, c * filter[0] * filter[1]), x.dtype)
-        self._sync_in()
+        self._sync_in(x)
         self._check(lib().ag_im2col_conv2(self._h, _dtype_code(x.dtype), _ptr(x.contiguous()), bs,
                                           c, ih, iw, ctypes.byref(o), _ptr(y)))
         return y
@@ -517,7 +527,7 @@ class _PyDevice:
         ow = (gw - 1) * stride[1] + dilation[1] * (fw - 1) + 1 - 2 * padding[1]
         o = _conv_options(filter, padding, stride, dilation)
         y = self._out((bs, c, oh, ow), x.dtype)
-        self._sync_in()
+        self._sync_in(x)
         self._check(lib().ag_col2im_conv2(self._h, _dtype_code(x.dtype), _ptr(x.contiguous()), bs,
                                           c, gh, gw, ctypes.byref(o), _ptr(y)))
         return y
@@ -530,7 +540,7 @@ class _PyDevice:
             raise AgError(_capi.AG_ERR_SHAPE, "pool window does not fit input")
         oh, ow = (ih - size[0]) // strides[0] + 1, (iw - size[1]) // strides[1] + 1
         y = self._out((bs, c, oh, ow), x.dtype)
-        self._sync_in()
+        self._sync_in(x)
         self._check(lib().ag_max_pool2(self._h, _dtype_code(x.dtype), _ptr(x.contiguous()), bs, c,
                                        ih, iw, size[0], size[1], strides[0], strides[1], _ptr(y)))
         return y
@@ -542,7 +552,7 @@ class _PyDevice:
         if not dx.is_contiguous():
             raise AgError(_capi.AG_ERR_INVALID, "dx must be contiguous")
         bs, c, ih, iw = dx.shape
-        self._sync_in()
+        self._sync_in(dx, dy)
         self._check(lib().ag_max_pool2_backward(self._h, _dtype_code(dx.dtype), _ptr(dx), bs, c, ih,
                                                 iw, size[0], size[1], strides[0], strides[1],
                                                 _ptr(dy.contiguous())))
@@ -558,7 +568,7 @@ class _PyDevice:
         x = x.contiguous()
         dx = self._out(x.shape, x.dtype)
         bs, c, ih, iw = x.shape
-        self._sync_in()
+        self._sync_in(x, dy)
         self._check(lib().ag_max_pool2_backward_from_input(
             self._h, _dtype_code(x.dtype), _ptr(x), bs, c, ih, iw, size[0], size[1], strides[0],
             strides[1], _ptr(dy.contiguous()), _ptr(dx)))
@@ -569,7 +579,7 @@ class _PyDevice:
         x = x.contiguous()
         bs, c, ih, iw = x.shape
         y = self._out((bs, c, ih // 2, iw // 2), x.dtype)
-        self._sync_in()
+        self._sync_in(x)
         self._check(lib().ag_relu_max_pool2_forward(self._h, _dtype_code(x.dtype), _ptr(x), bs, c,
                                                     ih, iw, _ptr(y)))
         return y
@@ -579,7 +589,7 @@ class _PyDevice:
         x = x.contiguous()
         bs, c, ih, iw = x.shape
         dx = self._out(x.shape, x.dtype)
-        self._sync_in()
+        self._sync_in(x, dy)
         self._check(lib().ag_relu_max_pool2_backward(self._h, _dtype_code(x.dtype), _ptr(x), bs, c,
                                                      ih, iw, _ptr(dy.contiguous()), _ptr(dx)))
         return dx
@@ -587,14 +597,14 @@ class _PyDevice:
     def relu(self, x, inplace=False):
         x = x.contiguous()
         y = x if inplace else self._out(x.shape, x.dtype)
-        self._sync_in()
+        self._sync_in(x)
         self._check(lib().ag_relu(self._h, _dtype_code(x.dtype), _ptr(x), _ptr(y), x.numel()))
         return y
 
     def relu_backward(self, x, dy, inplace=False):
         x, dy = x.contiguous(), dy.contiguous()
         dx = dy if inplace else self._out(dy.shape, dy.dtype)
-        self._sync_in()
+        self._sync_in(x, dy)
         self._check(lib().ag_relu_backward(self._h, _dtype_code(x.dtype), _ptr(x), _ptr(dy),
                                            _ptr(dx), x.numel()))
         return dx
@@ -603,7 +613,7 @@ class _PyDevice:
     def scaled_add(self, y, alpha, x):
         """≙ ``y.scaled_add(alpha, &x)`` (in place on y)."""
         assert y.is_contiguous() and x.is_contiguous() and x.shape == y.shape
-        self._sync_in()
+        self._sync_in(y, x)
         self._check(lib().ag_scaled_add(self._h, _dtype_code(y.dtype), ctypes.c_float(alpha),
                                         _ptr(x), _ptr(y), y.numel()))
         return y
@@ -611,7 +621,7 @@ class _PyDevice:
     def bias_add(self, y, bias):
         rows, cols = y.shape[0], y.shape[1]
         inner = y[0, 0].numel() if y.dim() > 2 else 1
-        self._sync_in()
+        self._sync_in(y, bias)
         self._check(lib().ag_bias_add(self._h, _dtype_code(y.dtype), _ptr(y), _ptr(bias), rows,
                                       cols, inner))
         return y
@@ -621,7 +631,7 @@ class _PyDevice:
         inner = dy[0, 0].numel() if dy.dim() > 2 else 1
         if out is None:
             out = self._out((cols,), dy.dtype)
-        self._sync_in()
+        self._sync_in(dy, out)
         self._check(lib().ag_bias_grad(self._h, _dtype_code(dy.dtype), _ptr(dy.contiguous()), rows,
                                        cols, inner, ctypes.c_float(beta), _ptr(out)))
         return out
@@ -633,7 +643,7 @@ class _PyDevice:
             raise AgError(_capi.AG_ERR_SHAPE, f"Expected target with shape [{bs}], found "
                                               f"[{t.shape[0]}]")
         loss = ctypes.c_float()
-        self._sync_in()
+        self._sync_in(x, t)
         self._check(lib().ag_cross_entropy_loss(self._h, _dtype_code(x.dtype), _dtype_code(t.dtype),
                                                 _ptr(x.contiguous()), _ptr(t), bs, classes,
                                                 ctypes.byref(loss)))
@@ -645,7 +655,7 @@ class _PyDevice:
         x, t = x.contiguous(), t.contiguous()
         loss = torch.empty((1,), dtype=torch.float32, device=self.torch_device)
         dx = self._out(x.shape, x.dtype)
-        self._sync_in()
+        self._sync_in(x, t)
         self._check(lib().ag_cross_entropy_loss_device_grad(
             self._h, _dtype_code(x.dtype), _dtype_code(t.dtype), _ptr(x), _ptr(t), x.shape[0],
             x.shape[1], _ptr(loss), ctypes.c_float(dy), _ptr(dx)))
@@ -654,7 +664,7 @@ class _PyDevice:
     def cross_entropy_loss_backward(self, x, t, dy=1.0):
         bs, classes = x.shape
         dx = self._out(x.shape, x.dtype)
-        self._sync_in()
+        self._sync_in(x, t)
         self._check(lib().ag_cross_entropy_loss_backward(
             self._h, _dtype_code(x.dtype), _dtype_code(t.dtype), _ptr(x.contiguous()), _ptr(t), bs,
             classes, ctypes.c_float(dy), _ptr(dx)))
@@ -663,7 +673,7 @@ class _PyDevice:
     def accuracy(self, x, t) -> int:
         bs, classes = x.shape
         out = ctypes.c_uint64()
-        self._sync_in()
+        self._sync_in(x, t)
         self._check(lib().ag_accuracy(self._h, _dtype_code(x.dtype), _dtype_code(t.dtype),
                                       _ptr(x.contiguous()), _ptr(t), bs, classes,
                                       ctypes.byref(out)))
@@ -671,13 +681,13 @@ class _PyDevice:
 
     # -- optimizer ----------------------------------------------------------------------
     def sgd_update(self, w, g, lr):
-        self._sync_in()
+        self._sync_in(w, g)
         self._check(lib().ag_sgd_update(self._h, _dtype_code(w.dtype), _ptr(w), _ptr(g), w.numel(),
                                         ctypes.c_float(lr)))
         return w
 
     def sgd_update_momentum(self, w, g, v, lr, momentum):
-        self._sync_in()
+        self._sync_in(w, g, v)
         self._check(lib().ag_sgd_update_momentum(self._h, _dtype_code(w.dtype), _ptr(w), _ptr(g),
                                                  _ptr(v), w.numel(), ctypes.c_float(lr),
                                                  ctypes.c_float(momentum)))

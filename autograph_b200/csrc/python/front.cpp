@@ -104,7 +104,7 @@ static int parse(PyObject *const *args, Py_ssize_t nargs, PyObject *kwnames, con
 typedef struct {
     void *p;
     int64_t shape[4], stride[2];
-    int ndim, dtype, index;
+    int ndim, dtype;
 } View;
 
 static int tuple_ints(PyObject *t, int64_t *out, int most) {
@@ -118,9 +118,10 @@ static int tuple_ints(PyObject *t, int64_t *out, int most) {
     return (int)n;
 }
 
-/* Reads a tensor of `ndim` dimensions (0: any up to 4); strides only when asked for, otherwise
- * the tensor must be contiguous.  Device index: -1 for host memory. */
-static int view_of(PyObject *o, int ndim, int with_strides, View *v) {
+/* Reads a tensor of `ndim` dimensions (0: any up to 4) on the GPU `index`, or in host memory for index -1: its
+ * address goes to a kernel or a copy as it is.  Strides only when asked for, otherwise the tensor must be
+ * contiguous. */
+static int view_of(PyObject *o, int ndim, int with_strides, int index, View *v) {
     if (o == NULL || !THPVariable_CheckExact(o)) return 0;
     if (at::impl::torch_function_mode_enabled() || c10::impl::dispatch_mode_enabled()) return 0;
     const at::Tensor &t = THPVariable_Unpack(o);
@@ -143,7 +144,7 @@ static int view_of(PyObject *o, int ndim, int with_strides, View *v) {
             return 0;
         }
         const c10::Device device = t.device();
-        v->index = device.is_cpu() ? -1 : device.is_cuda() ? device.index() : -2;
+        if (index != (device.is_cpu() ? -1 : device.is_cuda() ? device.index() : -2)) return 0;
         v->p = t.data_ptr();   /* throws where there is no pointer to give (wrappers of function transforms) */
     } catch (const std::exception &) {
         return 0;
@@ -160,7 +161,11 @@ static int64_t count_of(const View *v) {
 /* The plain case of a device call: no guards, and the device's own stream is torch's current one. */
 static int plain(DeviceObject *d) {
     if (d->guarded || d->h == NULL) return 0;
-    return (uintptr_t)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)d->index).stream() == d->stream;
+    try {
+        return (uintptr_t)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)d->index).stream() == d->stream;
+    } catch (const std::exception &) {
+        return 0;
+    }
 }
 
 static PyObject *new_tensor(DeviceObject *d, int dtype, int ndim, const int64_t *shape, void **p) {
@@ -232,11 +237,11 @@ static int options_of(PyObject *padding, PyObject *stride, PyObject *dilation, i
 }
 
 /* bias: None or a contiguous vector */
-static int bias_of(PyObject *o, const void **p) {
+static int bias_of(PyObject *o, int index, const void **p) {
     *p = NULL;
     if (o == NULL || o == Py_None) return 1;
     View v;
-    if (!view_of(o, 1, 0, &v)) return 0;
+    if (!view_of(o, 1, 0, index, &v)) return 0;
     *p = v.p;
     return 1;
 }
@@ -258,8 +263,8 @@ ENTRY(dot) {
     DeviceObject *d = (DeviceObject *)self;
     PyObject *o[2];
     View a, b;
-    if (!parse(args, nargs, kwnames, names, 2, 2, o) || !plain(d) || !view_of(o[0], 2, 1, &a) ||
-        !view_of(o[1], 2, 1, &b) || a.dtype != b.dtype || a.dtype == AG_U8 || a.shape[1] != b.shape[0])
+    if (!parse(args, nargs, kwnames, names, 2, 2, o) || !plain(d) || !view_of(o[0], 2, 1, d->index, &a) ||
+        !view_of(o[1], 2, 1, d->index, &b) || a.dtype != b.dtype || a.dtype == AG_U8 || a.shape[1] != b.shape[0])
         FALL_BACK(M_DOT);
     void *c;
     const int64_t shape[2] = {a.shape[0], b.shape[1]};
@@ -275,8 +280,8 @@ ENTRY(gemm) {
     View a, b, c;
     float alpha, beta;
     if (!parse(args, nargs, kwnames, names, 5, 5, o) || !plain(d) || !float_of(o[0], 0, &alpha) ||
-        !float_of(o[3], 0, &beta) || !view_of(o[1], 2, 1, &a) || !view_of(o[2], 2, 1, &b) ||
-        !view_of(o[4], 2, 1, &c) || a.dtype != b.dtype || a.dtype != c.dtype || a.dtype == AG_U8 ||
+        !float_of(o[3], 0, &beta) || !view_of(o[1], 2, 1, d->index, &a) || !view_of(o[2], 2, 1, d->index, &b) ||
+        !view_of(o[4], 2, 1, d->index, &c) || a.dtype != b.dtype || a.dtype != c.dtype || a.dtype == AG_U8 ||
         a.shape[1] != b.shape[0] || a.shape[0] != c.shape[0] || b.shape[1] != c.shape[1])
         FALL_BACK(M_GEMM);
     return finish(run_gemm(d, alpha, &a, &b, beta, c.p, c.stride[0], c.stride[1]), Py_NewRef(o[4]));
@@ -289,9 +294,9 @@ ENTRY(dense_forward) {
     View x, w;
     const void *bias;
     int relu, st;
-    if (!parse(args, nargs, kwnames, names, 4, 2, o) || !plain(d) || !view_of(o[0], 2, 0, &x) ||
-        !view_of(o[1], 2, 0, &w) || x.dtype != w.dtype || x.dtype == AG_U8 || x.shape[1] != w.shape[0] ||
-        !bias_of(o[2], &bias) || !flag_of(o[3], &relu))
+    if (!parse(args, nargs, kwnames, names, 4, 2, o) || !plain(d) || !view_of(o[0], 2, 0, d->index, &x) ||
+        !view_of(o[1], 2, 0, d->index, &w) || x.dtype != w.dtype || x.dtype == AG_U8 || x.shape[1] != w.shape[0] ||
+        !bias_of(o[2], d->index, &bias) || !flag_of(o[3], &relu))
         FALL_BACK(M_DENSE);
     void *y;
     const int64_t shape[2] = {x.shape[0], w.shape[1]};
@@ -311,9 +316,9 @@ ENTRY(conv2_forward) {
     ag_conv2_options opt;
     int relu, st;
     int64_t oh, ow;
-    if (!parse(args, nargs, kwnames, names, 7, 2, o) || !plain(d) || !view_of(o[0], 4, 0, &x) ||
-        !view_of(o[1], 4, 0, &w) || x.dtype == AG_U8 || x.dtype != w.dtype || x.shape[1] != w.shape[1] ||
-        !bias_of(o[2], &bias) || !options_of(o[3], o[4], o[5], w.shape[2], w.shape[3], &opt) ||
+    if (!parse(args, nargs, kwnames, names, 7, 2, o) || !plain(d) || !view_of(o[0], 4, 0, d->index, &x) ||
+        !view_of(o[1], 4, 0, d->index, &w) || x.dtype == AG_U8 || x.dtype != w.dtype || x.shape[1] != w.shape[1] ||
+        !bias_of(o[2], d->index, &bias) || !options_of(o[3], o[4], o[5], w.shape[2], w.shape[3], &opt) ||
         !flag_of(o[6], &relu) || p_ag_conv2_output_shape(x.shape[2], x.shape[3], &opt, &oh, &ow) != AG_OK)
         FALL_BACK(M_CONV_FWD);
     void *y;
@@ -333,8 +338,8 @@ ENTRY(conv2_backward_input) {
     ag_conv2_options opt;
     int st;
     int32_t hw[2];
-    if (!parse(args, nargs, kwnames, names, 6, 3, o) || !plain(d) || !view_of(o[0], 4, 0, &w) ||
-        !view_of(o[1], 4, 0, &dy) || dy.dtype == AG_U8 || dy.dtype != w.dtype || !pair_of(o[2], hw, 0) ||
+    if (!parse(args, nargs, kwnames, names, 6, 3, o) || !plain(d) || !view_of(o[0], 4, 0, d->index, &w) ||
+        !view_of(o[1], 4, 0, d->index, &dy) || dy.dtype == AG_U8 || dy.dtype != w.dtype || !pair_of(o[2], hw, 0) ||
         !options_of(o[3], o[4], o[5], w.shape[2], w.shape[3], &opt))
         FALL_BACK(M_CONV_DX);
     void *dx;
@@ -355,8 +360,8 @@ ENTRY(conv2_backward_weight) {
     int st;
     int32_t f[2];
     float beta;
-    if (!parse(args, nargs, kwnames, names, 8, 3, o) || !plain(d) || !view_of(o[0], 4, 0, &x) ||
-        !view_of(o[1], 4, 0, &dy) || x.dtype == AG_U8 || x.dtype != dy.dtype || !pair_of(o[2], f, 0) ||
+    if (!parse(args, nargs, kwnames, names, 8, 3, o) || !plain(d) || !view_of(o[0], 4, 0, d->index, &x) ||
+        !view_of(o[1], 4, 0, d->index, &dy) || x.dtype == AG_U8 || x.dtype != dy.dtype || !pair_of(o[2], f, 0) ||
         !options_of(o[3], o[4], o[5], f[0], f[1], &opt) || !float_of(o[6], 0, &beta))
         FALL_BACK(M_CONV_DW);
     PyObject *out;
@@ -365,7 +370,7 @@ ENTRY(conv2_backward_weight) {
         out = new_tensor(d, x.dtype, 4, shape, &w.p);
         if (out == NULL) return NULL;
     } else {
-        if (!view_of(o[7], 4, 0, &w) || w.dtype != x.dtype) FALL_BACK(M_CONV_DW);
+        if (!view_of(o[7], 4, 0, d->index, &w) || w.dtype != x.dtype) FALL_BACK(M_CONV_DW);
         out = Py_NewRef(o[7]);
     }
     CALL(st, p_ag_conv2_backward_weight(d->h, (ag_dtype)x.dtype, x.p, x.shape[0], x.shape[1], x.shape[2],
@@ -392,7 +397,7 @@ ENTRY(max_pool2) {
     View x;
     int32_t h[2], s[2];
     int st;
-    if (!parse(args, nargs, kwnames, names, 3, 1, o) || !plain(d) || !view_of(o[0], 4, 0, &x) ||
+    if (!parse(args, nargs, kwnames, names, 3, 1, o) || !plain(d) || !view_of(o[0], 4, 0, d->index, &x) ||
         x.dtype == AG_U8 || !pool_of(o[1], o[2], &x, h, s))
         FALL_BACK(M_POOL);
     void *y;
@@ -412,8 +417,8 @@ ENTRY(max_pool2_backward_from_input) {
     View x, dy;
     int32_t h[2], s[2];
     int st;
-    if (!parse(args, nargs, kwnames, names, 4, 2, o) || !plain(d) || !view_of(o[0], 4, 0, &x) ||
-        !view_of(o[1], 4, 0, &dy) || x.dtype == AG_U8 || x.dtype != dy.dtype || !pool_of(o[2], o[3], &x, h, s))
+    if (!parse(args, nargs, kwnames, names, 4, 2, o) || !plain(d) || !view_of(o[0], 4, 0, d->index, &x) ||
+        !view_of(o[1], 4, 0, d->index, &dy) || x.dtype == AG_U8 || x.dtype != dy.dtype || !pool_of(o[2], o[3], &x, h, s))
         FALL_BACK(M_POOL_BWD);
     void *dx;
     PyObject *out = new_tensor(d, x.dtype, 4, x.shape, &dx);
@@ -429,7 +434,7 @@ ENTRY(relu) {
     PyObject *o[2];
     View x;
     int inplace, st;
-    if (!parse(args, nargs, kwnames, names, 2, 1, o) || !plain(d) || !view_of(o[0], 0, 0, &x) ||
+    if (!parse(args, nargs, kwnames, names, 2, 1, o) || !plain(d) || !view_of(o[0], 0, 0, d->index, &x) ||
         x.dtype == AG_U8 || !flag_of(o[1], &inplace))
         FALL_BACK(M_RELU);
     void *y = x.p;
@@ -445,8 +450,8 @@ ENTRY(relu_backward) {
     PyObject *o[3];
     View x, dy;
     int inplace, st;
-    if (!parse(args, nargs, kwnames, names, 3, 2, o) || !plain(d) || !view_of(o[0], 0, 0, &x) ||
-        !view_of(o[1], 0, 0, &dy) || x.dtype == AG_U8 || x.dtype != dy.dtype || count_of(&x) != count_of(&dy) ||
+    if (!parse(args, nargs, kwnames, names, 3, 2, o) || !plain(d) || !view_of(o[0], 0, 0, d->index, &x) ||
+        !view_of(o[1], 0, 0, d->index, &dy) || x.dtype == AG_U8 || x.dtype != dy.dtype || count_of(&x) != count_of(&dy) ||
         !flag_of(o[2], &inplace))
         FALL_BACK(M_RELU_BWD);
     void *dx = dy.p;
@@ -470,8 +475,8 @@ ENTRY(bias_add) {
     View y, b;
     int64_t inner;
     int st;
-    if (!parse(args, nargs, kwnames, names, 2, 2, o) || !plain(d) || !view_of(o[0], 0, 0, &y) ||
-        !view_of(o[1], 1, 0, &b) || y.dtype == AG_U8 || y.dtype != b.dtype || !rows_cols_inner(&y, &inner))
+    if (!parse(args, nargs, kwnames, names, 2, 2, o) || !plain(d) || !view_of(o[0], 0, 0, d->index, &y) ||
+        !view_of(o[1], 1, 0, d->index, &b) || y.dtype == AG_U8 || y.dtype != b.dtype || !rows_cols_inner(&y, &inner))
         FALL_BACK(M_BIAS_ADD);
     CALL(st, p_ag_bias_add(d->h, (ag_dtype)y.dtype, y.p, b.p, y.shape[0], y.shape[1], inner));
     return finish(st, Py_NewRef(o[0]));
@@ -485,7 +490,7 @@ ENTRY(bias_grad) {
     int64_t inner;
     float beta;
     int st;
-    if (!parse(args, nargs, kwnames, names, 3, 1, o) || !plain(d) || !view_of(o[0], 0, 0, &dy) ||
+    if (!parse(args, nargs, kwnames, names, 3, 1, o) || !plain(d) || !view_of(o[0], 0, 0, d->index, &dy) ||
         dy.dtype == AG_U8 || !float_of(o[1], 0, &beta) || !rows_cols_inner(&dy, &inner))
         FALL_BACK(M_BIAS_GRAD);
     PyObject *out;
@@ -493,7 +498,7 @@ ENTRY(bias_grad) {
         out = new_tensor(d, dy.dtype, 1, &dy.shape[1], &b.p);
         if (out == NULL) return NULL;
     } else {
-        if (!view_of(o[2], 1, 0, &b) || b.dtype != dy.dtype) FALL_BACK(M_BIAS_GRAD);
+        if (!view_of(o[2], 1, 0, d->index, &b) || b.dtype != dy.dtype) FALL_BACK(M_BIAS_GRAD);
         out = Py_NewRef(o[2]);
     }
     CALL(st, p_ag_bias_grad(d->h, (ag_dtype)dy.dtype, dy.p, dy.shape[0], dy.shape[1], inner, beta, b.p));
@@ -534,7 +539,7 @@ static PyTypeObject DeviceType = {PyVarObject_HEAD_INIT(NULL, 0)};
 /* A batch [bs, c, h, w] (or a vector / matrix) of the given type on the GPU `index`, or in host
  * memory for index -1. */
 static int batch_of(PyObject *t, int ndim, int dtype, int index, View *v) {
-    return view_of(t, ndim, 0, v) && v->dtype == dtype && v->index == index;
+    return view_of(t, ndim, 0, index, v) && v->dtype == dtype;
 }
 
 /* logits: given, or a new tensor; NULL without an exception when the given one does not fit */

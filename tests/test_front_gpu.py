@@ -64,6 +64,24 @@ def test_same_errors(plain):
         plain.dot(x)
 
 
+def test_host_tensors_are_refused(plain):
+    """One tensor in host memory, whichever argument: an error before anything is launched."""
+    for name, args, kw in _calls(plain, torch.float32):
+        for key in [*range(len(args)), *kw]:
+            a, w = list(args), dict(kw)
+            at = a if isinstance(key, int) else w
+            if not isinstance(at[key], torch.Tensor):
+                continue
+            at[key] = at[key].cpu()
+            with pytest.raises(ag.AgError, match="must be in device memory"):
+                getattr(plain, name)(*a, **w)
+
+
+def test_page_locked_operands_are_read(plain):
+    a, b = torch.randn(40, 24).pin_memory(), torch.randn(24, 33).pin_memory()
+    assert torch.equal(plain.dense_forward(a, b), plain.dense_forward(a.cuda(), b.cuda()))
+
+
 def test_another_current_stream_is_ordered(plain):
     """Inputs produced on another current stream: the call waits for that stream."""
     a = torch.zeros((512, 512), device=plain.torch_device)
