@@ -29,8 +29,8 @@ try:
     import torch as _  # noqa: F401  the extension finds torch's libraries among those already loaded
     from . import _front
     _DeviceBase, _ModelBase = _front.DeviceBase, _front.ModelBase
-except ImportError:   # not built yet (the build imports this package): creating a Device fails
-    _front = None
+except ImportError as e:   # not built yet (the build imports this package): creating a Device fails
+    _front, _front_error = None, e
 
     class _DeviceBase:
         pass
@@ -74,8 +74,8 @@ def _bind_front():
     """Gives the extension the library's functions and the Python form of every method."""
     global _front_bound
     if _front is None:
-        raise ImportError("autograph_b200._front is missing: build it with "
-                          "`python -m autograph_b200.build`")
+        raise ImportError(f"autograph_b200._front does not load ({_front_error}): build it with "
+                          "`python -m autograph_b200.build`") from _front_error
     if not _front_bound:
         handle = lib()
         _front.bind({n: ctypes.cast(getattr(handle, n), ctypes.c_void_p).value for n in _front.FUNCTIONS},

@@ -80,26 +80,35 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     return LIB
 
 
+def _front_recipe(torch_dir: Path) -> tuple[list[str], str]:
+    """Command that builds the extension, and a key for all it is built from.  torch's headers lay out what the
+    extension reads, so torch's version is part of it: an upgrade in place changes nothing in the command."""
+    src = CSRC / "python" / "front.cpp"
+    cuda = Path(NVCC).resolve().parent.parent
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden",
+           "-I" + sysconfig.get_paths()["include"], "-isystem", str(torch_dir / "include"),
+           "-isystem", str(torch_dir / "include" / "torch" / "csrc" / "api" / "include"), "-isystem", str(cuda / "include"),
+           str(src), "-o", str(_front_path()), "-L" + str(torch_dir / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10_cuda",
+           "-lc10"]
+    parts = [src, HERE.parent / "include" / "autograph_b200.h", torch_dir / "version.py"]
+    return cmd, hashlib.sha256(b"".join(p.read_bytes() for p in parts) + " ".join(cmd).encode()).hexdigest()
+
+
+def _front_path() -> Path:
+    return HERE / ("_front" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
 def build_front(force: bool = False) -> Path:
     """The native half of the Python front end (csrc/python/front.cpp), a CPython extension next to
     the library.  It reads tensors through torch's C++ interface; the libraries that it names are those
     that `import torch` has loaded."""
     import importlib.util
-    src = CSRC / "python" / "front.cpp"
-    out = HERE / ("_front" + sysconfig.get_config_var("EXT_SUFFIX"))
-    stamp = BUILD / "front.stamp"
-    torch_dir = Path(importlib.util.find_spec("torch").origin).parent
-    cuda = Path(NVCC).resolve().parent.parent
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden",
-           "-I" + sysconfig.get_paths()["include"], "-isystem", str(torch_dir / "include"),
-           "-isystem", str(torch_dir / "include" / "torch" / "csrc" / "api" / "include"), "-isystem", str(cuda / "include"),
-           str(src), "-o", str(out), "-L" + str(torch_dir / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
-    header = HERE.parent / "include" / "autograph_b200.h"
-    key = hashlib.sha256(src.read_bytes() + header.read_bytes() + " ".join(cmd).encode()).hexdigest()
+    out, stamp = _front_path(), BUILD / "front.stamp"
+    cmd, key = _front_recipe(Path(importlib.util.find_spec("torch").origin).parent)
     if force or not out.exists() or not stamp.exists() or stamp.read_text() != key:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
-            raise RuntimeError(f"{cmd[0]} failed for {src.name}:\n{res.stderr[-4000:]}")
+            raise RuntimeError(f"{cmd[0]} failed for front.cpp:\n{res.stderr[-4000:]}")
         stamp.write_text(key)
     return out
 
