@@ -18,25 +18,14 @@ fails; if there is no B200, creating a :class:`Device` fails.
 from __future__ import annotations
 
 import ctypes
+import importlib
+import threading
 from pathlib import Path
 
 import numpy as np
 
 from . import _capi
 from ._capi import AgError, lib, lib_path  # noqa: F401
-
-try:
-    import torch as _  # noqa: F401  the extension finds torch's libraries among those already loaded
-    from . import _front
-    _DeviceBase, _ModelBase = _front.DeviceBase, _front.ModelBase
-except ImportError as e:   # not built yet (the build imports this package): creating a Device fails
-    _front, _front_error = None, e
-
-    class _DeviceBase:
-        pass
-
-    class _ModelBase:
-        pass
 
 __all__ = ["AgError", "Device", "Model", "lib", "lib_path", "LENET5_SPEC", "WIDE_STACK_SPEC"]
 
@@ -67,21 +56,48 @@ def _ptr(t) -> ctypes.c_void_p:
     return ctypes.c_void_p(t.data_ptr() if t is not None else 0)
 
 
+_extension = _front_error = None
 _front_bound = False
+_front_lock = threading.Lock()
+
+
+def _front_bases():
+    """The extension's base classes of Device and Model.  It is imported with them: it needs torch's libraries loaded,
+    and hosts that call the library alone import this package without torch."""
+    global _extension, _front_error
+    try:
+        import torch  # noqa: F401
+        _extension = importlib.import_module("._front", __name__)
+        return [_extension.DeviceBase], [_extension.ModelBase]
+    except ImportError as e:   # not built, or not for this torch: creating a Device says so
+        _extension, _front_error = None, e
+        return [], []
+
+
+def __getattr__(name):
+    """Device and Model are made when they are first asked for."""
+    if name not in ("Device", "Model"):
+        raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+    with _front_lock:
+        if name not in globals():
+            for python, bases in zip((_PyDevice, _PyModel), _front_bases()):
+                cls = python.__name__.removeprefix("_Py")
+                globals()[cls] = type(cls, (*bases, python), {"__doc__": python.__doc__, "__module__": __name__})
+    return globals()[name]
 
 
 def _bind_front():
     """Gives the extension the library's functions and the Python form of every method."""
     global _front_bound
-    if _front is None:
+    if _extension is None:
         raise ImportError(f"autograph_b200._front does not load ({_front_error}): build it with "
                           "`python -m autograph_b200.build`") from _front_error
     if not _front_bound:
         handle = lib()
-        _front.bind({n: ctypes.cast(getattr(handle, n), ctypes.c_void_p).value for n in _front.FUNCTIONS},
-                    _capi.check)
-        for name in _front.METHODS:
-            _front.set_fallback(name, getattr(_PyDevice, name, None) or getattr(_PyModel, name))
+        _extension.bind({n: ctypes.cast(getattr(handle, n), ctypes.c_void_p).value for n in _extension.FUNCTIONS},
+                         _capi.check)
+        for name in _extension.METHODS:
+            _extension.set_fallback(name, getattr(_PyDevice, name, None) or getattr(_PyModel, name))
         _front_bound = True
 
 
@@ -694,10 +710,6 @@ class _PyDevice:
         return w, v
 
 
-class Device(_DeviceBase, _PyDevice):
-    __doc__ = _PyDevice.__doc__
-
-
 # Layer specs shared with the oracle's composition (kind, a, b, c, d, bias).
 LENET5_SPEC = [
     ("conv", 1, 6, (5, 5), False), ("relu",), ("pool", (2, 2)),
@@ -932,7 +944,3 @@ class _PyModel:
 
     def apply_update(self, lr):
         _capi.check(lib().ag_model_apply_update(self._h, ctypes.c_float(lr)))
-
-
-class Model(_ModelBase, _PyModel):
-    __doc__ = _PyModel.__doc__

@@ -1,5 +1,5 @@
-"""Builds libautograph_b200.so (the C-ABI library) with nvcc for sm_100a, and the CPython extension
-that calls it from the Python front end with the C++ compiler.
+"""Builds libautograph_b200.so (the C-ABI library) with nvcc for sm_100a, and, where there is torch, the CPython
+extension that calls it from the Python front end with the C++ compiler.  Hosts in C and Rust need the library alone.
 
 Usage: ``python -m autograph_b200.build [--force] [--verbose]``.
 Objects go to ``autograph_b200/_build``; the shared library is written next to
@@ -65,8 +65,6 @@ def _compile(src: Path, digest: str, force: bool, verbose: bool) -> Path:
 
 def build(force: bool = False, verbose: bool = False) -> Path:
     BUILD.mkdir(exist_ok=True)
-    if not os.environ.get("AG_LIB_OUT"):
-        build_front(force)
     digest = _headers_digest()
     srcs = sources()
     with ThreadPoolExecutor(max_workers=min(8, len(srcs))) as pool:
@@ -77,6 +75,8 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stderr[-4000:]}")
+    if not os.environ.get("AG_LIB_OUT") and build_front(force) is None:
+        sys.stderr.write("torch is not installed: built without the Python front end\n")
     return LIB
 
 
@@ -98,13 +98,16 @@ def _front_path() -> Path:
     return HERE / ("_front" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 
-def build_front(force: bool = False) -> Path:
+def build_front(force: bool = False) -> Path | None:
     """The native half of the Python front end (csrc/python/front.cpp), a CPython extension next to
     the library.  It reads tensors through torch's C++ interface; the libraries that it names are those
-    that `import torch` has loaded."""
+    that `import torch` has loaded.  None where there is no torch."""
     import importlib.util
+    spec = importlib.util.find_spec("torch")
+    if spec is None:
+        return None
     out, stamp = _front_path(), BUILD / "front.stamp"
-    cmd, key = _front_recipe(Path(importlib.util.find_spec("torch").origin).parent)
+    cmd, key = _front_recipe(Path(spec.origin).parent)
     if force or not out.exists() or not stamp.exists() or stamp.read_text() != key:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
