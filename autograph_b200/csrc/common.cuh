@@ -93,11 +93,25 @@ namespace ag {
 // Programmatic dependent launch.  A kernel launched with launch_dependent may be placed on SMs that its
 // predecessor in the stream has left and set itself up there; after dependency_wait everything the
 // predecessor wrote is visible.  Every thread that touches global memory comes through that wait first.
+// That holds for loads through the read-only path too (__ldg, const __restrict__), which most operators use: they
+// rely on no line of what the predecessor writes coming into an SM's L1 between its write and their wait, and
+// nothing loads such data earlier.
 // A kernel that allocates tensor memory does so before it lets dependents launch: one that came first could hold the
 // columns it still needs, and wait for it.
 // The operators' kernels are small enough for that to count: a kernel of 2 us in a stream of them took 4 us, and a
-// convolution stage called operator by operator (16 -> 32 3x3, 64 x 32 x 32 f32, eleven launches) 128 us, now 116.
-__device__ __forceinline__ void let_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// convolution stage called operator by operator (16 -> 32 3x3, 64 x 32 x 32 f32, eleven launches) 118 us, now 100.
+//
+// Grids of up to half of the SMs let their dependents launch at once: those find the other half free.  Larger ones
+// say nothing, and their dependents launch when the last of their CTAs ends.  Let go at their start, dependents, and
+// theirs, took what room there was on the SMs that came free first and left the others idle, most of all replayed
+// from a graph, where no launch holds them up (us at the start, at the end): f32 256^3 13.0, 10.1; bf16 16 x 64 x 31 x 31
+// -> 128 3x3 24.2, 15.7; training LeNet5's layers on 2000 images bf16 518, 348.  Up to 111 CTAs at the start is too many
+// (convolution 1 -> 6 5x5, 100 x 28 x 28 f32: 4.7, 3.6); none at all costs small chains (LeNet5's layers, 16 images: 24.8
+// for 22.8 us an inference).
+constexpr unsigned kEarlyCtas = 74;
+__device__ __forceinline__ void let_dependents_launch(unsigned most = kEarlyCtas) {
+    if (gridDim.x * gridDim.y * gridDim.z <= most) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class... P, class... A>
 int launch_dependent(ag_device *dev, void (*kernel)(P...), dim3 grid, dim3 threads, size_t smem, const A &...args) {
@@ -254,9 +268,10 @@ struct FastDiv {
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
-// Dynamic shared memory of a persistent kernel that wants an SM per CTA.  Launched dependent, its CTAs go to the SMs
-// that its predecessor leaves first, two or three to one if they fit, and the others stay idle (the wide stack at 256
-// images bf16: inference 203 us, so 289, a training step 492 and 569): more than half of an SM's memory keeps them apart.
+// Dynamic shared memory of a persistent kernel that wants an SM per CTA.  Launched while its predecessor still runs, its
+// CTAs go to the SMs that came free first, two or three to one if they fit, and the others stay idle (after kernels that
+// let dependents launch at their start, the wide stack at 256 images bf16: inference 203 us, so 289, a training step 492
+// and 569): more than half of an SM's memory keeps them apart.
 constexpr int kOneCtaPerSm = 116 * 1024;
 
 }  // namespace ag
