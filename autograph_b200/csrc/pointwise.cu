@@ -242,18 +242,22 @@ __global__ void max_pool2_backward_2x2_kernel(const T *src, T *dx, const T *__re
     }
 }
 
-// Windows of 2x2 with stride 2 over planes of any size.  A thread takes kPoolWindows windows a grid apart and
-// loads all their cells before it uses the first: one window per thread with 64-bit divisions kept too few
-// bytes in flight (bf16, 6528 planes of 36 x 36: forward 12.5 us, gradient 14.1; now 8.5 and 13.6), and odd widths
-// went through shared memory (8128 planes of 55 x 55: 40 and 55 us; now 16 and 47).  Times under ncu, from DRAM: the
-// bytes of the two take 3.4 and 6, 9.4 and 17 us.  PAIR: even widths, rows that keep pairs aligned.
+// Windows of 2x2 with stride 2 over planes of any size.  One window per thread with 64-bit divisions kept too few
+// bytes in flight (bf16, 6528 planes of 36 x 36: forward 11.8 us, gradient 13.2; now 6.5 and 8.9), and odd widths
+// went through shared memory (8128 planes of 55 x 55: 38.9 and 57.3; now 14.3 and 38.2).  From DRAM, replayed; the bytes
+// of the two take 3.4 and 6, 9.4 and 17 us.  Forward, a thread loads all cells of W windows before it uses the first:
+// as many as fill the loads in flight (16384 planes of 62 x 62 f32: 51.8 us with one, 47.3 with two, 53.1 with four;
+// bf16 39.2, 40.0, 41.8; 8128 of 55 x 55 bf16 14.3, 15.1, 14.2).  The gradient takes one: it stores as much as
+// it loads, and more windows a thread only cost warps (62 x 62 f32 88.9 us, with four 102; bf16 59.4, 89).  PAIR:
+// even widths, rows that keep pairs aligned.
 // Offsets are 32-bit: the host cuts the planes into launches of fewer than 2^32 cells.
-constexpr int kPoolWindows = 4;
 struct PoolMap {
     int ih, iw, gh, gw;      // plane, grid of windows
     uint32_t total;          // windows of this launch
     FastDiv div_gw, div_gh;
 };
+template <class T, bool PAIR>
+constexpr int pool_windows_per_thread() { return sizeof(T) == 4 ? 2 : PAIR ? 1 : 4; }
 __device__ __forceinline__ uint32_t raw_of(__nv_bfloat16 v) { return __bfloat16_as_ushort(v); }
 __device__ __forceinline__ uint32_t raw_of(float v) { return __float_as_uint(v); }
 template <class T>
@@ -279,12 +283,12 @@ template <class T, bool RELU, bool PAIR>
 __global__ void __launch_bounds__(256) max_pool2_2x2_window_kernel(const T *__restrict__ x, T *__restrict__ y, const PoolMap m) {
     let_dependents_launch();
     dependency_wait();
-    const uint32_t step = gridDim.x * 256u;
-    for (uint32_t i0 = blockIdx.x * 256u + threadIdx.x; i0 < m.total; i0 += kPoolWindows * step) {
-        uint32_t v[kPoolWindows][4];
+    constexpr int W = pool_windows_per_thread<T, PAIR>();
+    for (uint32_t i0 = blockIdx.x * (256u * W) + threadIdx.x; i0 < m.total; i0 += gridDim.x * (256u * W)) {
+        uint32_t v[W][4];
 #pragma unroll
-        for (int u = 0; u < kPoolWindows; ++u) {
-            const uint32_t i = i0 + (uint32_t)u * step;
+        for (int u = 0; u < W; ++u) {
+            const uint32_t i = i0 + (uint32_t)u * 256u;
             if (i >= m.total) break;
             uint32_t wx, wy, t, plane;
             m.div_gw.divmod(i, t, wx);
@@ -301,8 +305,8 @@ __global__ void __launch_bounds__(256) max_pool2_2x2_window_kernel(const T *__re
             }
         }
 #pragma unroll
-        for (int u = 0; u < kPoolWindows; ++u) {
-            const uint32_t i = i0 + (uint32_t)u * step;
+        for (int u = 0; u < W; ++u) {
+            const uint32_t i = i0 + (uint32_t)u * 256u;
             if (i >= m.total) break;
             float best = 0.f;  // window order (0,0),(0,1),(1,0),(1,1); the first maximum wins
 #pragma unroll
@@ -337,7 +341,7 @@ __device__ __forceinline__ void store_row(T *p, uint32_t a, uint32_t b, bool row
 // Gradient of the same: src holds the forward input, dx receives dy at the first maximum of every window and
 // zero elsewhere; cells that no window covers (the last row or column of an odd plane) keep src's value.  The
 // grid counts those cells' partial windows too (gw = ceil(iw / 2)).  src may be dx: a warp has read its
-// windows' cells before it writes them.  RELU (even planes): src is the input of a Relu whose output was
+// window's cells before it writes them.  RELU (even planes): src is the input of a Relu whose output was
 // pooled; the result is the gradient at that input (the pool's gradient gated by src >= 0, as Relu's
 // backward gates it).
 template <class T, bool RELU, bool PAIR>
@@ -345,74 +349,67 @@ __global__ void __launch_bounds__(256) max_pool2_backward_2x2_window_kernel(cons
                                                                             const PoolMap m, int oh, int ow) {
     let_dependents_launch();
     dependency_wait();
-    const uint32_t step = gridDim.x * 256u, lane = threadIdx.x % 32;
-    // whole warps: i0 - lane is the warp's first window
-    for (uint32_t i0 = blockIdx.x * 256u + threadIdx.x; i0 - lane < m.total; i0 += kPoolWindows * step) {
-        uint32_t v[kPoolWindows][4], off[kPoolWindows];   // cells as they lie in memory
-        float g[kPoolWindows];
-        bool second[kPoolWindows], below[kPoolWindows], left[kPoolWindows], right[kPoolWindows];
-#pragma unroll
-        for (int u = 0; u < kPoolWindows; ++u) {
-            const uint32_t i = i0 + (uint32_t)u * step;
-            if (i >= m.total) continue;
-            uint32_t wx, wy, t, plane;
+    const uint32_t lane = threadIdx.x % 32;
+    // whole warps: i - lane is the warp's first window
+    for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i - lane < m.total; i += gridDim.x * 256u) {
+        const bool mine = i < m.total;
+        uint32_t v[4] = {}, off = 0, wx = 0, wy = 0;   // cells as they lie in memory
+        bool second = true, below = true;
+        float g = 0.f;
+        if (mine) {
+            uint32_t t, plane;
             m.div_gw.divmod(i, t, wx);
             m.div_gh.divmod(t, plane, wy);
-            off[u] = (plane * (uint32_t)m.ih + 2 * wy) * (uint32_t)m.iw + 2 * wx;
-            const T *q = src + off[u], *q1 = q + m.iw;
+            off = (plane * (uint32_t)m.ih + 2 * wy) * (uint32_t)m.iw + 2 * wx;
+            const T *q = src + off, *q1 = q + m.iw;
             if (PAIR) {
-                g[u] = to_f32(dy[i]);
-                load_word(q, v[u][0], v[u][1]);
-                load_word(q1, v[u][2], v[u][3]);
+                g = to_f32(dy[i]);
+                load_word(q, v[0], v[1]);
+                load_word(q1, v[2], v[3]);
             } else {
-                second[u] = (int)(2 * wx) < m.iw - 1;
-                below[u] = (int)(2 * wy) < m.ih - 1;
-                left[u] = lane > 0 && wx > 0;
-                right[u] = lane < 31 && wx + 1 < (uint32_t)m.gw && i + 1 < m.total;
-                v[u][0] = raw_of(q[0]);
-                if (second[u]) v[u][1] = raw_of(q[1]);
-                if (below[u]) v[u][2] = raw_of(q1[0]);
-                if (second[u] && below[u]) {
-                    v[u][3] = raw_of(q1[1]);
-                    g[u] = to_f32(dy[(plane * (uint32_t)oh + wy) * (uint32_t)ow + wx]);
+                second = (int)(2 * wx) < m.iw - 1;
+                below = (int)(2 * wy) < m.ih - 1;
+                v[0] = raw_of(q[0]);
+                if (second) v[1] = raw_of(q[1]);
+                if (below) v[2] = raw_of(q1[0]);
+                if (second && below) {
+                    v[3] = raw_of(q1[1]);
+                    g = to_f32(dy[(plane * (uint32_t)oh + wy) * (uint32_t)ow + wx]);
                 }
             }
         }
+        if (second && below) {
+            float c[4];
+            bool pass[4] = {true, true, true, true};  // Relu lets the gradient pass
 #pragma unroll
-        for (int u = 0; u < kPoolWindows; ++u) {
-            const bool mine = i0 + (uint32_t)u * step < m.total;
-            if (PAIR ? mine : mine && second[u] && below[u]) {
-                float c[4];
-                bool pass[4] = {true, true, true, true};  // Relu lets the gradient pass
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    c[j] = value_of<T>(v[u][j]);
-                    if (RELU) {
-                        pass[j] = c[j] >= 0.f;
-                        c[j] = pass[j] ? c[j] : 0.f;
-                    }
+            for (int j = 0; j < 4; ++j) {
+                c[j] = value_of<T>(v[j]);
+                if (RELU) {
+                    pass[j] = c[j] >= 0.f;
+                    c[j] = pass[j] ? c[j] : 0.f;
                 }
-                float best = c[0];
-                int am = 0;
-#pragma unroll
-                for (int j = 1; j < 4; ++j)
-                    if (c[j] > best) {
-                        best = c[j];
-                        am = j;
-                    }
-                const uint32_t gv = raw_of(from_f32<T>(__fadd_rn(0.f, g[u])));   // one conversion, then bits
-#pragma unroll
-                for (int j = 0; j < 4; ++j) v[u][j] = am == j && pass[j] ? gv : 0u;
             }
-            T *d = dx + off[u];
-            if (PAIR) {
-                if (!mine) continue;
-                store_word(d, v[u][0], v[u][1]);
-                store_word(d + m.iw, v[u][2], v[u][3]);
-            } else {
-                store_row<T>(d, v[u][0], v[u][1], mine, second[u], left[u], right[u]);
-                store_row<T>(d + m.iw, v[u][2], v[u][3], mine && below[u], second[u], left[u], right[u]);
-            }
+            float best = c[0];
+            int am = 0;
+#pragma unroll
+            for (int j = 1; j < 4; ++j)
+                if (c[j] > best) {
+                    best = c[j];
+                    am = j;
+                }
+            const uint32_t gv = raw_of(from_f32<T>(__fadd_rn(0.f, g)));   // one conversion, then bits
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = am == j && pass[j] ? gv : 0u;
+        }
+        T *d = dx + off;
+        if (PAIR) {
+            if (!mine) continue;
+            store_word(d, v[0], v[1]);
+            store_word(d + m.iw, v[2], v[3]);
+        } else {
+            const bool left = lane > 0 && wx > 0, right = lane < 31 && wx + 1 < (uint32_t)m.gw && i + 1 < m.total;
+            store_row<T>(d, v[0], v[1], mine, second, left, right);
+            store_row<T>(d + m.iw, v[2], v[3], mine && below, second, left, right);
         }
     }
 }
@@ -420,7 +417,7 @@ __global__ void __launch_bounds__(256) max_pool2_backward_2x2_window_kernel(cons
 // Calls launch(first plane, first row of windows, map, grid) for as many planes at a time as 32-bit offsets hold;
 // a plane of more cells than that is cut along its rows.  gh x gw windows a plane.
 template <class F>
-static int for_pool_planes(ag_device *dev, int64_t planes, int64_t ih, int64_t iw, int64_t gh, int64_t gw, F launch) {
+static int for_pool_planes(ag_device *dev, int64_t planes, int64_t ih, int64_t iw, int64_t gh, int64_t gw, int per_thread, F launch) {
     constexpr int64_t kCells = (1ll << 32) - 1;
     const int64_t most = kCells / ((ih + 1) * (iw + 1));
     const int64_t at_once = most < 1 ? 1 : most, rows = most < 1 ? kCells / (2 * (iw + 1)) : gh;
@@ -429,7 +426,7 @@ static int for_pool_planes(ag_device *dev, int64_t planes, int64_t ih, int64_t i
             const int64_t n = std::min(at_once, planes - p), band = std::min(rows, gh - y);
             const PoolMap m{(int)(y + band == gh ? ih - 2 * y : 2 * band), (int)iw, (int)band, (int)gw,
                             (uint32_t)(n * band * gw), FastDiv((uint32_t)gw), FastDiv((uint32_t)band)};
-            AG_TRY(launch(p, y, m, dim3(grid_for(ceil_div((int64_t)m.total, kPoolWindows), 256, dev->sm_count))));
+            AG_TRY(launch(p, y, m, dim3(grid_for(ceil_div((int64_t)m.total, per_thread), 256, dev->sm_count))));
         }
     return AG_OK;
 }
@@ -439,14 +436,31 @@ static bool pair_aligned(const T *p) {
     return reinterpret_cast<uintptr_t>(p) % (2 * sizeof(T)) == 0;
 }
 
+// Relu + pool takes pairs alone (relu_pool_check): the other form is not compiled for it.
+template <class T, bool RELU, bool PAIR>
+static int pool_windows_as(ag_device *dev, const T *x, T *y, int64_t planes, int64_t ih, int64_t iw, int64_t oh, int64_t ow) {
+    return for_pool_planes(dev, planes, ih, iw, oh, ow, pool_windows_per_thread<T, PAIR>(),
+                           [&](int64_t p, int64_t y0, const PoolMap &m, dim3 grid) {
+        return launch_dependent(dev, max_pool2_2x2_window_kernel<T, RELU, PAIR>, grid, 256, 0, x + (p * ih + 2 * y0) * iw,
+                                y + (p * oh + y0) * ow, m);
+    });
+}
+
 template <class T, bool RELU>
 static int pool_windows(ag_device *dev, const T *x, T *y, int64_t planes, int64_t ih, int64_t iw, int64_t oh, int64_t ow) {
-    const bool pair = (iw & 1) == 0 && pair_aligned(x);
-    return for_pool_planes(dev, planes, ih, iw, oh, ow, [&](int64_t p, int64_t y0, const PoolMap &m, dim3 grid) {
-        const T *src = x + (p * ih + 2 * y0) * iw;
-        T *dst = y + (p * oh + y0) * ow;
-        return launch_dependent(dev, pair ? max_pool2_2x2_window_kernel<T, RELU, true> : max_pool2_2x2_window_kernel<T, RELU, false>, grid,
-                                256, 0, src, dst, m);
+    if constexpr (!RELU)
+        if ((iw & 1) != 0 || !pair_aligned(x)) return pool_windows_as<T, RELU, false>(dev, x, y, planes, ih, iw, oh, ow);
+    return pool_windows_as<T, RELU, true>(dev, x, y, planes, ih, iw, oh, ow);
+}
+
+template <class T, bool RELU, bool PAIR>
+static int pool_windows_backward_as(ag_device *dev, const T *x, T *dx, const T *dy, int64_t planes, int64_t ih, int64_t iw,
+                                    int64_t oh, int64_t ow) {
+    return for_pool_planes(dev, planes, ih, iw, (ih + 1) / 2, (iw + 1) / 2, 1,
+                           [&](int64_t p, int64_t y0, const PoolMap &m, dim3 grid) {
+        const int64_t at = (p * ih + 2 * y0) * iw;
+        return launch_dependent(dev, max_pool2_backward_2x2_window_kernel<T, RELU, PAIR>, grid, 256, 0, x + at, dx + at,
+                                dy + (p * oh + y0) * ow, m, (int)oh, (int)ow);
     });
 }
 
@@ -454,15 +468,10 @@ template <class T, bool RELU>
 static int pool_windows_backward(ag_device *dev, const T *x, T *dx, const T *dy, int64_t planes, int64_t ih, int64_t iw, int64_t oh,
                                  int64_t ow) {
     // pairs: every cell is in a window
-    const bool pair = (iw & 1) == 0 && (ih & 1) == 0 && pair_aligned(x) && pair_aligned(dx);
-    return for_pool_planes(dev, planes, ih, iw, (ih + 1) / 2, (iw + 1) / 2, [&](int64_t p, int64_t y0, const PoolMap &m, dim3 grid) {
-        const T *src = x + (p * ih + 2 * y0) * iw, *g = dy + (p * oh + y0) * ow;
-        T *dst = dx + (p * ih + 2 * y0) * iw;
-        return launch_dependent(dev,
-                                pair ? max_pool2_backward_2x2_window_kernel<T, RELU, true>
-                                     : max_pool2_backward_2x2_window_kernel<T, RELU, false>,
-                                grid, 256, 0, src, dst, g, m, (int)oh, (int)ow);
-    });
+    if constexpr (!RELU)
+        if ((iw & 1) != 0 || (ih & 1) != 0 || !pair_aligned(x) || !pair_aligned(dx))
+            return pool_windows_backward_as<T, RELU, false>(dev, x, dx, dy, planes, ih, iw, oh, ow);
+    return pool_windows_backward_as<T, RELU, true>(dev, x, dx, dy, planes, ih, iw, oh, ow);
 }
 
 // Any non-overlapping window, any width: a CTA stages a run of whole planes in
@@ -991,6 +1000,17 @@ int ag_max_pool2(ag_device *dev, ag_dtype dtype, const void *x, int64_t bs, int6
     AG_DISPATCH_FLOAT(dtype, T, return pool_forward<T>(dev, (const T *)x, (T *)y, bs * c, (int)ih, (int)iw, oh, ow, h, w, sh, sw););
 }
 
+// Gradients of 2x2 windows that run faster staged than a thread per window: planes so small that half of the windows
+// are partial, each with up to eight accesses of its own, and enough of them to fill the staged form's CTAs (us, windows
+// and staged, from L2: bf16 131072 planes of 7 x 7 14.9, 11.3; 262144 of 3 x 3 10.4, 4.6; 131072 of 9 x 9 22.4, 17.7;
+// 65536 of 11 x 11 15.5, 14.4 but from DRAM 16.5, 19.2; 16384 of 5 x 5 2.6, 2.9; 4096 of 9 x 9 2.2, 3.2;
+// f32 262144 of 3 x 3 6.9, 5.4; 65536 of 3 x 3 2.8, 3.3; 262144 of 5 x 5 14.0, 14.0, from DRAM 15.2, 18.0).
+static bool many_small_odd_planes(ag_dtype dtype, int64_t planes, int64_t ih, int64_t iw) {
+    const int64_t windows = planes * ((ih + 1) / 2) * ((iw + 1) / 2);
+    if (ih % 2 == 0 || iw % 2 == 0) return false;
+    return dtype == AG_F32 ? ih * iw <= 9 && windows >= 500000 : ih * iw <= 81 && windows >= 200000;
+}
+
 // dx = max_pool2_backward(copy of x, dy); x == dx is the in-place form of the reference.
 static int pool_backward(ag_device *dev, ag_dtype dtype, const void *x, void *dx, int64_t bs,
                          int64_t c, int64_t ih, int64_t iw, int32_t h, int32_t w, int32_t sh,
@@ -1017,7 +1037,7 @@ static int pool_backward(ag_device *dev, ag_dtype dtype, const void *x, void *dx
         AG_DISPATCH_FLOAT(dtype, T, return launch_dependent(dev, max_pool2_backward_2x2_kernel<T>, dim3(grid2), threads, 0, (const T *)x,
                                                             (T *)dx, (const T *)dy, planes, (int)ih, (int)iw, oh, ow););
     }
-    if (h == 2 && w == 2 && sh == 2 && sw == 2)
+    if (h == 2 && w == 2 && sh == 2 && sw == 2 && !many_small_odd_planes(dtype, planes, ih, iw))
         AG_DISPATCH_FLOAT(dtype, T, return (pool_windows_backward<T, false>(dev, (const T *)x, (T *)dx, (const T *)dy, planes, ih, iw,
                                                                             oh, ow)););
     const int64_t plane_bytes = ih * iw * (int64_t)dtype_size(dtype);

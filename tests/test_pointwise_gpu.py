@@ -201,6 +201,105 @@ def test_windows_of_two_by_two(dev, dtype, shape, offset):
     assert np.array_equal(_np(dev.max_pool2_backward(xd, dev.tensor(dy, dtype))), want)
 
 
+def _pool_2x2(x, dy=None, relu=False):
+    """Torch, window by window in order: the first maximum wins, a NaN never after the first cell.  Output, or the
+    gradient with the cells no window covers kept."""
+    oh, ow = x.shape[2] // 2, x.shape[3] // 2
+    cells = [x[:, :, i:2 * oh:2, j:2 * ow:2] for i in (0, 1) for j in (0, 1)]
+    gates = [c >= 0 for c in cells]
+    if relu:
+        cells = [torch.where(g, c, torch.zeros_like(c)) for c, g in zip(cells, gates)]
+    best, at = cells[0].clone(), torch.zeros(cells[0].shape, dtype=torch.uint8, device=x.device)
+    for k in (1, 2, 3):
+        at[cells[k] > best] = k
+        best = torch.where(cells[k] > best, cells[k], best)
+    if dy is None:
+        return best
+    dx = x.clone()
+    for k, gate in enumerate(gates):
+        won = (at == k) & gate if relu else at == k
+        dx[:, :, k // 2:2 * oh:2, k % 2:2 * ow:2] = torch.where(won, dy + 0, torch.zeros_like(dy))
+    return dx
+
+
+def _same(a, b):
+    """Equal, NaNs and signs of zeros included."""
+    return bool((((a == b) & (torch.signbit(a) == torch.signbit(b))) | (a.isnan() & b.isnan())).all())
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("shape", [(9, 16, 14, 14), (9, 16, 13, 13), (5, 3, 37, 62), (2, 3, 301, 203),
+                                   (300, 64, 7, 7), (195, 64, 7, 7), (700, 64, 9, 9), (700, 64, 9, 11), (2000, 64, 3, 3),
+                                   (600, 64, 3, 3)])
+def test_windows_of_two_by_two_with_special_values(dev, dtype, shape):
+    """NaN, infinities, both zeros and the largest values, at the sizes where a rule chooses the kernel."""
+    gen = torch.Generator(device=dev.torch_device).manual_seed(sum(shape))
+    big = torch.finfo(dtype).max
+    pick = torch.tensor([float("nan"), float("inf"), -float("inf"), 0.0, -0.0, big, -big, 1.0], dtype=dtype, device=dev.torch_device)
+
+    def values(s):
+        t = torch.randn(s, generator=gen, device=dev.torch_device).to(dtype)
+        special = pick[torch.randint(0, 8, s, generator=gen, device=dev.torch_device)]
+        return torch.where(torch.rand(s, generator=gen, device=dev.torch_device) < 0.4, special, t)
+
+    x, dy = values(shape), values((*shape[:2], shape[2] // 2, shape[3] // 2))
+    assert _same(dev.max_pool2(x), _pool_2x2(x))
+    want = _pool_2x2(x, dy)
+    assert _same(dev.max_pool2_backward_from_input(x, dy), want)
+    assert _same(dev.max_pool2_backward(x, dy), want)
+    if shape[2] % 2 == 0 and shape[3] % 2 == 0:
+        assert _same(dev.relu_max_pool2(x), _pool_2x2(x, relu=True))
+        assert _same(dev.relu_max_pool2_backward(x, dy), _pool_2x2(x, dy, relu=True))
+
+
+@pytest.mark.parametrize("shape", [(70001, 1, 250, 251), (1, 1, 65537, 65539), (1, 1, 65538, 65540)])
+def test_windows_of_two_by_two_beyond_2_32_cells(dev, shape):
+    """Sets of planes, and single planes, that take several launches."""
+    dev.set_guards(False)   # their checks would need another 20 GB
+    assert shape[0] * shape[2] * shape[3] > 2 ** 32
+    x = torch.empty(shape, dtype=torch.bfloat16, device=dev.torch_device).normal_()
+    y = dev.max_pool2(x)
+    dx = dev.max_pool2_backward_from_input(x, y)
+    for part in range(16):   # by planes, or by pairs of rows
+        if shape[0] > 1:
+            at = slice(part * shape[0] // 16, (part + 1) * shape[0] // 16)
+            xs, ys, dxs = x[at], y[at], dx[at]
+        else:
+            r0, r1 = (y.shape[2] * p // 16 for p in (part, part + 1))
+            rows = slice(2 * r0, 2 * r1 if part < 15 else shape[2])
+            xs, ys, dxs = x[:, :, rows], y[:, :, r0:r1], dx[:, :, rows]
+        assert torch.equal(ys, _pool_2x2(xs)) and torch.equal(dxs, _pool_2x2(xs, ys))
+    del x, y, dx, xs, ys, dxs
+    torch.cuda.empty_cache()
+    dev.set_guards(True)
+
+
+def test_gradient_of_two_by_two_windows_keeps_up(dev):
+    """16384 planes of 62 x 62 bf16 take less than 1.7 times as long as a copy that moves as many bytes (1.35 with a
+    window per thread, 2.0 with four)."""
+    dev.set_guards(False)
+    x = torch.randn((256, 64, 62, 62), device=dev.torch_device).bfloat16()
+    dy = torch.randn((256, 64, 31, 31), device=dev.torch_device).bfloat16()
+    n = x.numel() + dy.numel() // 2
+    a, b = torch.empty(n, dtype=x.dtype, device=dev.torch_device), torch.empty(n, dtype=x.dtype, device=dev.torch_device)
+
+    def us(f):
+        best = float("inf")
+        for _ in range(10):
+            t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda._sleep(500_000)   # the launches queue up behind it
+            t0.record(dev.stream)
+            for _ in range(10):
+                f()
+            t1.record(dev.stream)
+            t1.synchronize()
+            best = min(best, t0.elapsed_time(t1) * 100)
+        return best
+
+    assert us(lambda: dev.max_pool2_backward_from_input(x, dy)) < 1.7 * us(lambda: b.copy_(a))
+    dev.set_guards(True)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("shape,offset", [((1, 1, 2), 0), ((3, 2, 2, 2), 1), ((2, 3, 7), 0), ((9, 5, 511), 1), ((4, 3, 512), 0),
                                           ((2, 2, 1023), 1), ((70, 33, 1025), 0), ((2, 1500, 6), 0), ((1, 1, 70001), 3)])
