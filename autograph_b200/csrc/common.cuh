@@ -108,7 +108,10 @@ namespace ag {
 // -> 128 3x3 24.2, 15.7; training LeNet5's layers on 2000 images bf16 518, 348.  Up to 111 CTAs at the start is too many
 // (convolution 1 -> 6 5x5, 100 x 28 x 28 f32: 4.7, 3.6); none at all costs small chains (LeNet5's layers, 16 images: 24.8
 // for 22.8 us an inference).
-constexpr unsigned kEarlyCtas = 74;
+// kAlwaysEarly: kernels that are followed by ones of a CTA per SM, which cannot crowd and gain their set-up time -- the
+// layout, filter and gradient passes around the tensor-core convolutions, the gathered engine's products (a training step
+// of the wide stack, 256 images bf16: 491 us without, 482 with; 65536 x 512 x 16 f32 103.5 and 101.0).
+constexpr unsigned kEarlyCtas = 74, kAlwaysEarly = ~0u;
 __device__ __forceinline__ void let_dependents_launch(unsigned most = kEarlyCtas) {
     if (gridDim.x * gridDim.y * gridDim.z <= most) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 __global__ void __launch_bounds__(256)
     nchw_to_nhwc_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restrict__ out, int C,
                         int HW, int Cp, int W, int Hp, int Wp, int pad_h, int pad_w) {
-    let_dependents_launch();
+    let_dependents_launch(kAlwaysEarly);
     dependency_wait();
     const int px = blockIdx.x * 256 + threadIdx.x;
     if (px >= HW) return;
@@ -340,7 +340,7 @@ constexpr int NCHW_PITCH = NCHW_PIX + 16;
 __global__ void __launch_bounds__(256)
     nhwc_to_nchw_kernel(const __nv_bfloat16 *__restrict__ in, __nv_bfloat16 *__restrict__ out, int C,
                         int HW, int Cp) {
-    let_dependents_launch();
+    let_dependents_launch(kAlwaysEarly);
     dependency_wait();
     __shared__ __align__(16) unsigned short tile[16 * NCHW_PITCH];
     const int p0 = blockIdx.x * NCHW_PIX;
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(256)
 __global__ void repack_filters_kernel(const __nv_bfloat16 *__restrict__ w,
                                       __nv_bfloat16 *__restrict__ wk, int OC, int IC, int taps,
                                       int Cp) {
-    let_dependents_launch();
+    let_dependents_launch(kAlwaysEarly);
     dependency_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)OC * taps * Cp) return;
@@ -399,7 +399,7 @@ __global__ void repack_filters_kernel(const __nv_bfloat16 *__restrict__ w,
 __global__ void repack_filters_transposed_kernel(const __nv_bfloat16 *__restrict__ w,
                                                  __nv_bfloat16 *__restrict__ wk, int OC, int IC,
                                                  int taps, int OCp) {
-    let_dependents_launch();
+    let_dependents_launch(kAlwaysEarly);
     dependency_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)IC * taps * OCp) return;

@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
 __global__ void wgrad_reduce_kernel(const float *__restrict__ partial, int splits, int64_t m_total,
                                     int taps, int Cp, int OC, int IC, float beta,
                                     __nv_bfloat16 *__restrict__ dw) {
-    let_dependents_launch();
+    let_dependents_launch(kAlwaysEarly);
     dependency_wait();
     __shared__ float part[8][33];
     const int64_t i = (int64_t)blockIdx.x * 32 + threadIdx.x;

@@ -851,10 +851,10 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    // A CTA takes an SM here: dependents find room beside any grid that leaves one free (input gradient of 8 x 6 x 20 x 20
-    // -> 16 5x5, stride 2, f32: 10.7 us, at the end 11.5); beside a full one they crowd (stage of 16 -> 32 3x3, 64 x 32 x 32
-    // f32: 109 us, at the end 100).
-    let_dependents_launch(147);
+    // The k slices of a convolution (its weight gradient) on every SM let dependents launch at their end: 16 -> 32 3x3,
+    // 64 x 32 x 32 f32, 40.0 us at the start, 33.8 so; with an SM left free they gain as all others do (8 x 6 x 20 x 20
+    // -> 16 5x5, stride 2, f32: 12.1, at the end 12.9).
+    let_dependents_launch(Epi::kLastCtaAdds && p.splits > 1 ? 147u : kAlwaysEarly);
     dependency_wait();
 
     const int tiles = p.tiles_m * p.tiles_n;

@@ -177,7 +177,7 @@ __global__ void relu_pool_backward_kernel(const __nv_bfloat16 *__restrict__ pre,
                                           const __nv_bfloat16 *__restrict__ dy, __nv_bfloat16 *__restrict__ out,
                                           int ih, int iw, int ph, int pw, int cp, int64_t row_pitch,
                                           int64_t image_pitch, int64_t total) {
-    let_dependents_launch();
+    let_dependents_launch(kAlwaysEarly);
     dependency_wait();
     const int groups = cp / 8;
     const int wh = (ih + 1) / 2, ww = (iw + 1) / 2;
@@ -236,7 +236,7 @@ __global__ void relu_pool_backward_kernel(const __nv_bfloat16 *__restrict__ pre,
 
 __global__ void zero_frame_kernel(__nv_bfloat16 *framed, int hp, int wp, int pad_h, int pad_w, int cp,
                                   int64_t cells_per_image, int64_t total) {
-    let_dependents_launch();
+    let_dependents_launch(kAlwaysEarly);
     dependency_wait();
     const int groups = cp / 8;
     const int64_t band = (int64_t)pad_h * wp;   // cells of the top (and of the bottom) rows
