@@ -9,8 +9,9 @@
  * ints, torch.empty) a convolution, pool or bias gradient took the host 6.4 to 7.0 us a call, now 4.4 to 4.8.
  *
  * Anything but the plain case -- other argument types, views that need a copy, shapes that do not
- * match, another current stream, a torch mode that wants to see operations, output guards switched on -- goes to
- * the Python implementation of the method (set_fallback()), which also raises the errors. */
+ * match, another current stream, a torch mode that wants to see operations (a default device does not: outputs have
+ * theirs), output guards switched on -- goes to the Python implementation of the method (set_fallback()), which also
+ * raises the errors. */
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <stddef.h>
@@ -22,6 +23,7 @@
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/PyInterpreter.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../../include/autograph_b200.h"
@@ -38,7 +40,7 @@
 FUNCTIONS(DECLARE)
 #undef DECLARE
 
-static PyObject *py_check;
+static PyObject *py_check, *device_context;
 
 enum Method {
     M_DOT, M_GEMM, M_DENSE, M_CONV_FWD, M_CONV_DX, M_CONV_DW, M_POOL, M_POOL_BWD, M_RELU, M_RELU_BWD,
@@ -118,12 +120,25 @@ static int tuple_ints(PyObject *t, int64_t *out, int most) {
     return (int)n;
 }
 
+/* Whether a torch mode wants to see operations.  torch.set_default_device and `with torch.device(...)` are modes too, of
+ * a class that only adds a device where none is given. */
+static int watched(void) {
+    if (c10::impl::dispatch_mode_enabled()) return 1;
+    if (!at::impl::torch_function_mode_enabled()) return 0;
+    const int64_t n = at::impl::PythonTorchFunctionTLS::stack_len();
+    for (int64_t i = 0; i < n; ++i) {
+        PyObject *mode = at::impl::PythonTorchFunctionTLS::get_stack_at(i)->ptr(getPyInterpreter());
+        if ((PyObject *)Py_TYPE(mode) != device_context) return 1;
+    }
+    return 0;
+}
+
 /* Reads a tensor of `ndim` dimensions (0: any up to 4) on the GPU `index`, or in host memory for index -1: its
  * address goes to a kernel or a copy as it is.  Strides only when asked for, otherwise the tensor must be
  * contiguous. */
 static int view_of(PyObject *o, int ndim, int with_strides, int index, View *v) {
     if (o == NULL || !THPVariable_CheckExact(o)) return 0;
-    if (at::impl::torch_function_mode_enabled() || c10::impl::dispatch_mode_enabled()) return 0;
+    if (watched()) return 0;
     const at::Tensor &t = THPVariable_Unpack(o);
     const c10::TensorImpl *impl = t.unsafeGetTensorImpl();
     if (impl->layout() != c10::kStrided || impl->has_symbolic_sizes_strides() || !impl->has_storage()) return 0;
@@ -677,6 +692,10 @@ static PyObject *bind(PyObject *mod, PyObject *args) {
     FUNCTIONS(TAKE)
 #undef TAKE
     py_check = Py_NewRef(check);
+    PyObject *modes = PyImport_ImportModule("torch.utils._device");
+    device_context = modes ? PyObject_GetAttrString(modes, "DeviceContext") : NULL;
+    Py_XDECREF(modes);
+    PyErr_Clear();   /* without it every mode is one that watches */
     Py_RETURN_NONE;
 }
 

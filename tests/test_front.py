@@ -116,3 +116,61 @@ def test_extension_leaves_host_tensors_to_the_python_form():
             if name in _front.METHODS:
                 assert taken(lambda: getattr(d, name)(*args, **kw)) == "python", name
         """)
+
+
+def test_a_default_device_keeps_the_fast_path():
+    _in_process("""
+        assert infer() == "native"
+        with torch.device("cpu"):
+            assert infer() == "native"
+            with torch.device("meta"):
+                assert infer() == "native"
+        torch.set_default_device("meta")
+        assert infer() == "native"
+        torch.set_default_device(None)
+        """)
+
+
+def test_what_the_extension_leaves_to_the_python_form():
+    """Modes that watch operations, wrappers of function transforms, subclasses, and tensors that are not what the kernels
+    read; tensors that only carry a gradient or inference flag are plain."""
+    _in_process("""
+        from torch.overrides import TorchFunctionMode
+        from torch.utils._device import DeviceContext
+        from torch.utils._python_dispatch import TorchDispatchMode
+        class Watching(TorchFunctionMode):
+            def __torch_function__(self, f, types, args=(), kwargs=None):
+                return f(*args, **(kwargs or {}))
+        class Dispatching(TorchDispatchMode):
+            def __torch_dispatch__(self, f, types, args=(), kwargs=None):
+                return f(*args, **(kwargs or {}))
+        class Context(DeviceContext):
+            pass
+        for mode in (Watching(), Dispatching(), Context(torch.device("cpu"))):
+            with mode:
+                assert infer() == "python", mode
+                with torch.device("cpu"):
+                    assert infer() == "python", mode
+        with torch.device("cpu"), Watching():
+            assert infer() == "python"
+        assert infer() == "native"
+
+        def mapped(x):
+            assert infer(x=x) == "python"
+            return x + 0
+        torch.func.vmap(mapped)(torch.zeros(3, 2, 1, 4, 4))
+        torch.func.jvp(mapped, (x,), (x,))
+
+        class Sub(torch.Tensor):
+            pass
+        for other in (x.as_subclass(Sub), x.double(), x.to("meta"), x.transpose(2, 3).expand(2, 1, 4, 4)[:, :, ::2],
+                      x.to_sparse(), torch.zeros(2, 4, 4), [0.0], None):
+            assert infer(x=other) == "python", type(other)
+        for out2 in (torch.zeros(2, 9), torch.zeros(3, 10), torch.zeros(10, 2).t(), out.double(), None):
+            assert infer(out=out2) == "python"
+        with torch.inference_mode():
+            made = torch.zeros(2, 1, 4, 4)
+            assert infer(x=made) == "native"
+        assert infer(x=made) == "native"
+        assert infer(x=torch.nn.Parameter(x)) == "native" and infer(x=x.requires_grad_()) == "native"
+        """)

@@ -82,6 +82,18 @@ def test_page_locked_operands_are_read(plain):
     assert torch.equal(plain.dense_forward(a, b), plain.dense_forward(a.cuda(), b.cuda()))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_default_device_changes_nothing(plain, dtype):
+    """Outputs come on the device's GPU, whatever tensors are made on by default."""
+    for name, args, kw in _calls(plain, dtype):
+        if kw.get("inplace") or "out" in kw or "dw" in kw or name in ("gemm", "bias_add") or True in args:
+            continue   # called twice below
+        want = getattr(plain, name)(*args, **kw)
+        with torch.device("cpu"):
+            got = getattr(plain, name)(*args, **kw)
+        assert got.device == want.device and torch.equal(got, want), name
+
+
 def test_another_current_stream_is_ordered(plain):
     """Inputs produced on another current stream: the call waits for that stream."""
     a = torch.zeros((512, 512), device=plain.torch_device)
