@@ -161,8 +161,8 @@ __device__ __forceinline__ float load1_as(const __nv_bfloat16 *p) {
 // all barriers and reduction.  Here every output (row, column) belongs to four adjacent lanes;
 // lane q adds the products of k = q, q + 4, ... in k order and the four sums are added as
 // (p0 + p1) + (p2 + p3) by two shuffles -- no scratch, one barrier.  The order does not depend
-// on the CTA size, and every kernel that runs such a layer comes through here, so the bits are
-// the same everywhere.
+// on the CTA size.  narrow_last_layer and the layer on its own (dense_narrow_kernel) add and round
+// in this order too, so the bits are the same everywhere.
 __host__ __device__ __forceinline__ bool narrow_step(const ChainStep &st) {
     return !st.transposed && st.gate == nullptr && st.N <= 16 && st.K <= 1024;
 }

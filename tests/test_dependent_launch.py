@@ -111,8 +111,8 @@ def _replay_us(dev, calls, n=20):
 @pytest.mark.parametrize("call", ["product", "narrow", "convolution"])
 def test_early_launches_cost_nothing(plain, call):
     """A kernel that follows itself at once is no slower than one that a launch of torch's, which waits for all of
-    it, comes between: dependents that crowd on the first free SMs made these 13.0, 34.8 and 24.2 us of 10.1, 21.9
-    and 15.7, and the launch between takes one or two."""
+    it, comes between: dependents that crowd on the first free SMs made these 13.0, 34.8 and 24.2 us of 8.3, 21.6
+    and 14.9, and the launch between takes one or two."""
     dev = plain
     rnd = lambda *s, dt=torch.float32: torch.randn(s, device=dev.torch_device).to(dt)
     if call == "product":

@@ -175,3 +175,18 @@ def test_dense_with_few_outputs(dev, dtype, m, k, n):
     if dtype == torch.bfloat16:
         bound += 2.0 ** -7 * (want.abs() + b.double().abs() + bound)
     assert ((got - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m", [5, 300, 1000])   # one, two and four rows per CTA on their own
+@pytest.mark.parametrize("k,n", [(84, 10), (83, 16), (130, 3), (256, 10), (7, 1)])
+def test_dense_with_few_outputs_gives_the_bits_of_the_chain(dev, dtype, m, k, n):
+    """The layer alone, as a dot, and as the last one of a run."""
+    gen = torch.Generator(device=dev.torch_device).manual_seed(m + k + n)
+    x, w0, w1, b = (torch.rand(s, generator=gen, device=dev.torch_device).sub_(0.5).to(dtype)
+                    for s in ((m, 24), (24, k), (k, n), (n,)))
+    h = dev.dense_forward(x, w0, relu=True)
+    for bias, relu in ((b, False), (None, True)):
+        chain = dev.dense_chain_forward(x, [w0, w1], [None, bias], [True, relu])
+        assert torch.equal(dev.dense_forward(h, w1, bias=bias, relu=relu), chain)
+    assert torch.equal(dev.dot(h, w1).clamp(min=0), chain)

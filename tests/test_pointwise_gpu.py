@@ -321,6 +321,33 @@ def test_bias_grad_of_planes(dev, dtype, shape, offset):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+def test_bias_grad_of_planes_accumulates(dev, dtype):
+    """beta and a given output, where the last chunk of a channel finishes it and where a second launch does (1024
+    channels and more), with other numbers of chunks in between: a call leaves every counter as it found it.  The bound
+    is that of the sums above, and two roundings of f32 for beta."""
+    gen = torch.Generator(device=dev.torch_device).manual_seed(33)
+    rnd = lambda *s: torch.randn(s, generator=gen, device=dev.torch_device).to(dtype)
+    cases = [(rnd(*s), rnd(s[1]), beta) for s, beta in
+             (((9, 5, 511), 1.0), ((70, 33, 1025), 0.5), ((2, 1500, 6), -2.0), ((1, 1, 70001), 1.0), ((300, 1023, 9), 0.25),
+              ((40, 1024, 33), 1.0), ((5, 7, 2), 1.0))]
+    first = []
+    for again in range(3):
+        for i, (x, y, beta) in enumerate(cases):
+            out = y.clone()
+            assert dev.bias_grad(x, beta, out) is out
+            if again == 0:
+                first.append(out)
+            assert torch.equal(out, first[i])
+    for (x, y, beta), got in zip(cases, first):
+        want = x.double().sum(dim=(0, 2)) + beta * y.double()
+        size = x.double().abs().sum(dim=(0, 2)) + abs(beta) * y.double().abs()
+        bound = (x.numel() / x.shape[1] / 32 + 34) * 2.0 ** -24 * size
+        if dtype == torch.bfloat16:
+            bound += 2.0 ** -8 * (want.abs() + bound)
+        assert ((got.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 def test_sgd(dev, dtype):
     rng = np.random.default_rng(5)
     n = 46920
