@@ -104,8 +104,8 @@ namespace ag {
 // Grids of up to half of the SMs let their dependents launch at once: those find the other half free.  Larger ones
 // say nothing, and their dependents launch when the last of their CTAs ends.  Let go at their start, dependents, and
 // theirs, took what room there was on the SMs that came free first and left the others idle, most of all replayed
-// from a graph, where no launch holds them up (us at the start, at the end): f32 256^3 13.0, 10.1; bf16 16 x 64 x 31 x 31
-// -> 128 3x3 24.2, 15.7; training LeNet5's layers on 2000 images bf16 518, 348.  Up to 111 CTAs at the start is too many
+// from a graph, where no launch holds them up (us at the start, at the end): f32 256^3 13.0, 8.3; bf16 16 x 64 x 31 x 31
+// -> 128 3x3 24.2, 14.9; training LeNet5's layers on 2000 images bf16 518, 348.  Up to 111 CTAs at the start is too many
 // (convolution 1 -> 6 5x5, 100 x 28 x 28 f32: 4.7, 3.6); none at all costs small chains (LeNet5's layers, 16 images: 24.8
 // for 22.8 us an inference).
 // kAlwaysEarly: kernels that are followed by ones of a CTA per SM, which cannot crowd and gain their set-up time -- the

@@ -248,7 +248,7 @@ __global__ void max_pool2_backward_2x2_kernel(const T *src, T *dx, const T *__re
 // of the two take 3.4 and 6, 9.4 and 17 us.  Forward, a thread loads all cells of W windows before it uses the first:
 // as many as fill the loads in flight (16384 planes of 62 x 62 f32: 51.8 us with one, 47.3 with two, 53.1 with four;
 // bf16 39.2, 40.0, 41.8; 8128 of 55 x 55 bf16 14.3, 15.1, 14.2).  The gradient takes one: it stores as much as
-// it loads, and more windows a thread only cost warps (62 x 62 f32 88.9 us, with four 102; bf16 59.4, 89).  PAIR:
+// it loads, and more windows a thread only cost warps (62 x 62 f32 89 to 92 us, with four 102 to 104; bf16 59, 89).  PAIR:
 // even widths, rows that keep pairs aligned.
 // Offsets are 32-bit: the host cuts the planes into launches of fewer than 2^32 cells.
 struct PoolMap {
