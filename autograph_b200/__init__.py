@@ -232,23 +232,36 @@ class _PyDevice:
         torch.cuda.current_stream(self.index).synchronize()
         return out
 
-    def _sync_in(self, *tensors, strided=False):
-        """Refuses operands whose addresses this GPU's kernels cannot use: host memory (unless it is page-locked, which
-        they can read; and then without a copy on the way, which would not be) and other GPUs'.  None stands for an
-        operand that is absent."""
-        for t in tensors:
+    def _sync_in(self, *tensors, inout=(), strided=False):
+        """The operands as kernels read them: contiguous (unless the call passes strides on).  The caller holds them until
+        the launch, or the memory of one copy would be the next one's.  Tensors that are written as well stay as they are
+        and have to be contiguous.  None stands for an operand that is absent.
+
+        Refuses operands whose addresses this GPU's kernels cannot use: host memory (unless it is page-locked, which they
+        can read) and other GPUs'."""
+        if not strided:
+            tensors = [t if t is None else t.contiguous() for t in tensors]
+        for t in (*tensors, *inout):
             if t is None or (t.is_cuda and t.device.index == self.index):
                 continue
             if t.is_cuda:
                 raise AgError(_capi.AG_ERR_INVALID, f"tensor of shape {tuple(t.shape)} is on another GPU")
-            if not ((strided or t.is_contiguous()) and t.is_pinned()):
+            if not t.is_pinned():
                 raise AgError(_capi.AG_ERR_INVALID, f"tensor of shape {tuple(t.shape)} must be in device memory")
+        for t in inout:
+            if t is not None and not t.is_contiguous():
+                raise AgError(_capi.AG_ERR_INVALID, f"tensor of shape {tuple(t.shape)} is written and must be contiguous")
         # Inputs were produced on torch's current stream; order this stream after it (nothing
         # to do when that stream is this device's own, which is the case unless the caller
-        # changed torch's current stream after creating the device).
+        # changed torch's current stream after creating the device), and keep their memory from
+        # being handed out on that stream before this one has read it.
         cur = _torch().cuda.current_stream(self.index)
         if cur.cuda_stream != self._stream_ptr:
             self.stream.wait_stream(cur)
+            for t in (*tensors, *inout):
+                if t is not None and t.is_cuda:
+                    t.record_stream(self.stream)
+        return tensors
 
     # -- linalg ----------------------------------------------------------------
     def gemm(self, alpha, a, b, beta, c):
@@ -300,9 +313,9 @@ class _PyDevice:
         o = _conv_options((fh, fw), padding, stride, dilation)
         oh, ow = self.conv2_output_shape(ih, iw, (fh, fw), padding, stride, dilation)
         y = self._out((bs, oc, oh, ow), x.dtype)
-        self._sync_in(x, w, bias)
-        self._check(lib().ag_conv2_forward(self._h, _dtype_code(x.dtype), _ptr(x.contiguous()), bs,
-                                           ic, ih, iw, _ptr(w.contiguous()), oc, _ptr(bias),
+        x, w, bias = self._sync_in(x, w, bias)
+        self._check(lib().ag_conv2_forward(self._h, _dtype_code(x.dtype), _ptr(x), bs,
+                                           ic, ih, iw, _ptr(w), oc, _ptr(bias),
                                            ctypes.byref(o), int(relu), _ptr(y)))
         return y
 
@@ -319,10 +332,10 @@ class _PyDevice:
             raise AgError(_capi.AG_ERR_SHAPE, "pool window does not fit the convolution output")
         y = self._out((bs, oc, (oh - pool[0]) // pool[0] + 1, (ow - pool[1]) // pool[1] + 1),
                        x.dtype)
-        self._sync_in(x, w, bias)
+        x, w, bias = self._sync_in(x, w, bias)
         self._check(lib().ag_conv2_relu_max_pool2_forward(
-            self._h, _dtype_code(x.dtype), _ptr(x.contiguous()), bs, ic, ih, iw,
-            _ptr(w.contiguous()), oc, _ptr(bias), ctypes.byref(o), int(relu), pool[0], pool[1],
+            self._h, _dtype_code(x.dtype), _ptr(x), bs, ic, ih, iw,
+            _ptr(w), oc, _ptr(bias), ctypes.byref(o), int(relu), pool[0], pool[1],
             _ptr(y)))
         return y
 
@@ -338,10 +351,10 @@ class _PyDevice:
         oh, ow = self.conv2_output_shape(ih, iw, (fh, fw), padding, stride, dilation)
         pre = self._out((bs, oc, oh, ow), x.dtype)
         y = self._out((bs, oc, oh // 2, ow // 2), x.dtype)
-        self._sync_in(x, w, bias)
+        x, w, bias = self._sync_in(x, w, bias)
         self._check(lib().ag_conv2_relu_max_pool2_forward_keep(
-            self._h, _dtype_code(x.dtype), _ptr(x.contiguous()), bs, ic, ih, iw,
-            _ptr(w.contiguous()), oc, _ptr(bias), ctypes.byref(o), _ptr(pre), _ptr(y)))
+            self._h, _dtype_code(x.dtype), _ptr(x), bs, ic, ih, iw,
+            _ptr(w), oc, _ptr(bias), ctypes.byref(o), _ptr(pre), _ptr(y)))
         return pre, y
 
     def dense_forward(self, x, w, bias=None, relu=False):
@@ -351,9 +364,9 @@ class _PyDevice:
         if x.shape[1] != w.shape[0]:
             raise AgError(_capi.AG_ERR_SHAPE, f"a_cols != b_rows, {x.shape[1]} != {w.shape[0]}")
         y = self._out((x.shape[0], w.shape[1]), x.dtype)
-        self._sync_in(x, w, bias)
-        self._check(lib().ag_dense_forward(self._h, _dtype_code(x.dtype), _ptr(x.contiguous()),
-                                           x.shape[0], x.shape[1], _ptr(w.contiguous()),
+        x, w, bias = self._sync_in(x, w, bias)
+        self._check(lib().ag_dense_forward(self._h, _dtype_code(x.dtype), _ptr(x),
+                                           x.shape[0], x.shape[1], _ptr(w),
                                            w.shape[1], _ptr(bias), int(relu), _ptr(y)))
         return y
 
@@ -363,13 +376,14 @@ class _PyDevice:
         biases = biases or [None] * n
         relus = relus or [False] * n
         dims = (ctypes.c_int64 * (n + 1))(x.shape[1], *[w.shape[1] for w in weights])
-        ws = (ctypes.c_void_p * n)(*[w.contiguous().data_ptr() for w in weights])
+        x, *rest = self._sync_in(x, *weights, *biases)
+        weights, biases = rest[:n], rest[n:]
+        ws = (ctypes.c_void_p * n)(*[w.data_ptr() for w in weights])
         bs = (ctypes.c_void_p * n)(*[(b.data_ptr() if b is not None else None) for b in biases])
         rl = (ctypes.c_int32 * n)(*[int(r) for r in relus])
         y = self._out((x.shape[0], weights[-1].shape[1]), x.dtype)
-        self._sync_in(x, *weights, *biases)
         self._check(lib().ag_dense_chain_forward(self._h, _dtype_code(x.dtype),
-                                                 _ptr(x.contiguous()), x.shape[0], n, dims, ws, bs,
+                                                 _ptr(x), x.shape[0], n, dims, ws, bs,
                                                  rl, _ptr(y)))
         return y
 
@@ -380,7 +394,9 @@ class _PyDevice:
         biases = biases or [None] * n
         relus = relus or [False] * n
         dims = (ctypes.c_int64 * (n + 1))(x.shape[1], *[w.shape[1] for w in weights])
-        ws = (ctypes.c_void_p * n)(*[w.contiguous().data_ptr() for w in weights])
+        x, *rest = self._sync_in(x, *weights, *biases)
+        weights, biases = rest[:n], rest[n:]
+        ws = (ctypes.c_void_p * n)(*[w.data_ptr() for w in weights])
         bs = (ctypes.c_void_p * n)(*[(b.data_ptr() if b is not None else None) for b in biases])
         rl = (ctypes.c_int32 * n)(*[int(r) for r in relus])
         pre = [self._out((x.shape[0], w.shape[1]), x.dtype) for w in weights]
@@ -388,9 +404,8 @@ class _PyDevice:
                for w, r in zip(weights, relus)]
         pp = (ctypes.c_void_p * n)(*[_ptr(t) for t in pre])
         ap = (ctypes.c_void_p * n)(*[(_ptr(t) if t is not None else None) for t in act])
-        self._sync_in(x, *weights, *biases)
         self._check(lib().ag_dense_chain_forward_keep(self._h, _dtype_code(x.dtype),
-                                                      _ptr(x.contiguous()), x.shape[0], n, dims, ws,
+                                                      _ptr(x), x.shape[0], n, dims, ws,
                                                       bs, rl, pp, ap))
         return pre, act
 
@@ -401,19 +416,19 @@ class _PyDevice:
         has_bias = has_bias or [False] * n
         dt = x.dtype
         dims = (ctypes.c_int64 * (n + 1))(x.shape[1], *[w.shape[1] for w in weights])
-        ins = [x.contiguous()] + [(act[i] if relus[i] else pre[i]) for i in range(n - 1)]
+        x, dy, *rest = self._sync_in(x, dy, *weights, *pre, *act)
+        weights, pre, act = rest[:n], rest[n:2 * n], rest[2 * n:]
+        ins = [x] + [(act[i] if relus[i] else pre[i]) for i in range(n - 1)]
         g = [self._out(p.shape, dt) for p in pre]
         dw = [self._out(w.shape, dt) for w in weights]
         db = [self._out((w.shape[1],), dt) if b else None for w, b in zip(weights, has_bias)]
         dx = self._out(x.shape, dt) if want_dx else None
-        dy = dy.contiguous()
         if not relus[-1]:
             g[-1] = dy
         arr = lambda ts: (ctypes.c_void_p * n)(*[(_ptr(t) if t is not None else None) for t in ts])
-        self._sync_in(*ins, dy, *weights, *pre, *act)
         self._check(lib().ag_dense_chain_backward(
             self._h, _dtype_code(dt), x.shape[0], n, dims, arr(ins),
-            arr([w.contiguous() for w in weights]), arr([pre[i] if relus[i] else None for i in range(n)]),
+            arr(weights), arr([pre[i] if relus[i] else None for i in range(n)]),
             _ptr(dy), arr([g[i] if (i < n - 1 or relus[i]) else None for i in range(n)]),
             _ptr(dx) if dx is not None else None, arr(dw), arr(db)))
         return dx, dw, db, g
@@ -452,9 +467,9 @@ class _PyDevice:
     def scaled_cast_u8(self, x_u8, alpha, dtype):
         """≙ Tensor::scaled_cast for u8 input: alpha * x in `dtype` (f32 or bf16)."""
         y = self._out(tuple(x_u8.shape), dtype)
-        self._sync_in(x_u8)
+        x_u8, = self._sync_in(x_u8)
         self._check(lib().ag_scaled_cast_u8(self._h, _dtype_code(dtype), ctypes.c_float(alpha),
-                                            _ptr(x_u8.contiguous()), _ptr(y), x_u8.numel()))
+                                            _ptr(x_u8), _ptr(y), x_u8.numel()))
         return y
 
     def conv_dense_chain_forward(self, x, convs, weights, biases=None, relus=None, u8_alpha=None):
@@ -464,35 +479,32 @@ class _PyDevice:
         u8_alpha into the weights' dtype while staging it.  Raises AgError(AG_ERR_UNSUPPORTED)
         when the network does not fit the fused kernel."""
         bs, ic, ih, iw = x.shape
+        n = len(weights)
+        biases = biases or [None] * n
+        relus = relus or [False] * n
+        x, *rest = self._sync_in(x, *weights, *biases, *(t for w, b, _, _ in convs for t in (w, b)))
+        weights, biases, filters = rest[:n], rest[n:2 * n], rest[2 * n:]
         stages = (_capi.ConvStage * len(convs))()
-        keep = []
-        for st, (w, b, relu, pool) in zip(stages, convs):
-            w = w.contiguous()
-            keep.append(w)
+        for st, w, b, (_, _, relu, pool) in zip(stages, filters[::2], filters[1::2], convs):
             st.w = w.data_ptr()
             st.bias = b.data_ptr() if b is not None else None
             st.oc = w.shape[0]
             st.options = _conv_options(tuple(w.shape[2:]))
             st.relu = int(relu)
             st.pool[0], st.pool[1] = pool if pool else (0, 0)
-        n = len(weights)
-        biases = biases or [None] * n
-        relus = relus or [False] * n
-        weights = [w.contiguous() for w in weights]
         dims = (ctypes.c_int64 * (n + 1))(weights[0].shape[0], *[w.shape[1] for w in weights])
         ws = (ctypes.c_void_p * n)(*[w.data_ptr() for w in weights])
         bp = (ctypes.c_void_p * n)(*[(b.data_ptr() if b is not None else None) for b in biases])
         rl = (ctypes.c_int32 * n)(*[int(r) for r in relus])
         out_dtype = weights[0].dtype
         y = self._out((bs, weights[-1].shape[1]), out_dtype)
-        self._sync_in(x, *(t for w, b, _, _ in convs for t in (w, b)), *weights, *biases)
         if u8_alpha is not None:
             self._check(lib().ag_conv_dense_chain_forward_u8(
-                self._h, _dtype_code(out_dtype), _ptr(x.contiguous()), ctypes.c_float(u8_alpha), bs,
+                self._h, _dtype_code(out_dtype), _ptr(x), ctypes.c_float(u8_alpha), bs,
                 ic, ih, iw, len(convs), stages, n, dims, ws, bp, rl, _ptr(y)))
         else:
             self._check(lib().ag_conv_dense_chain_forward(
-                self._h, _dtype_code(x.dtype), _ptr(x.contiguous()), bs, ic, ih, iw, len(convs),
+                self._h, _dtype_code(x.dtype), _ptr(x), bs, ic, ih, iw, len(convs),
                 stages, n, dims, ws, bp, rl, _ptr(y)))
         return y
 
@@ -503,10 +515,10 @@ class _PyDevice:
         ih, iw = input_hw
         o = _conv_options((fh, fw), padding, stride, dilation)
         dx = self._out((bs, ic, ih, iw), dy.dtype)
-        self._sync_in(w, dy)
+        w, dy = self._sync_in(w, dy)
         self._check(lib().ag_conv2_backward_input(self._h, _dtype_code(dy.dtype),
-                                                  _ptr(w.contiguous()), oc, ic,
-                                                  _ptr(dy.contiguous()), bs, ih, iw,
+                                                  _ptr(w), oc, ic,
+                                                  _ptr(dy), bs, ih, iw,
                                                   ctypes.byref(o), _ptr(dx)))
         return dx
 
@@ -517,10 +529,10 @@ class _PyDevice:
         o = _conv_options(filter, padding, stride, dilation)
         if dw is None:
             dw = self._out((oc, ic, filter[0], filter[1]), x.dtype)
-        self._sync_in(x, dy, dw)
+        x, dy = self._sync_in(x, dy, inout=(dw,))
         self._check(lib().ag_conv2_backward_weight(self._h, _dtype_code(x.dtype),
-                                                   _ptr(x.contiguous()), bs, ic, ih, iw,
-                                                   _ptr(dy.contiguous()), oc, ctypes.byref(o),
+                                                   _ptr(x), bs, ic, ih, iw,
+                                                   _ptr(dy), oc, ctypes.byref(o),
                                                    ctypes.c_float(beta), _ptr(dw)))
         return dw
 
@@ -529,8 +541,8 @@ class _PyDevice:
         o = _conv_options(filter, padding, stride, dilation)
         oh, ow = self.conv2_output_shape(ih, iw, filter, padding, stride, dilation)
         y = self._out((bs * oh * ow, c * filter[0] * filter[1]), x.dtype)
-        self._sync_in(x)
-        self._check(lib().ag_im2col_conv2(self._h, _dtype_code(x.dtype), _ptr(x.contiguous()), bs,
+        x, = self._sync_in(x)
+        self._check(lib().ag_im2col_conv2(self._h, _dtype_code(x.dtype), _ptr(x), bs,
                                           c, ih, iw, ctypes.byref(o), _ptr(y)))
         return y
 
@@ -543,8 +555,8 @@ class _PyDevice:
         ow = (gw - 1) * stride[1] + dilation[1] * (fw - 1) + 1 - 2 * padding[1]
         o = _conv_options(filter, padding, stride, dilation)
         y = self._out((bs, c, oh, ow), x.dtype)
-        self._sync_in(x)
-        self._check(lib().ag_col2im_conv2(self._h, _dtype_code(x.dtype), _ptr(x.contiguous()), bs,
+        x, = self._sync_in(x)
+        self._check(lib().ag_col2im_conv2(self._h, _dtype_code(x.dtype), _ptr(x), bs,
                                           c, gh, gw, ctypes.byref(o), _ptr(y)))
         return y
 
@@ -556,8 +568,8 @@ class _PyDevice:
             raise AgError(_capi.AG_ERR_SHAPE, "pool window does not fit input")
         oh, ow = (ih - size[0]) // strides[0] + 1, (iw - size[1]) // strides[1] + 1
         y = self._out((bs, c, oh, ow), x.dtype)
-        self._sync_in(x)
-        self._check(lib().ag_max_pool2(self._h, _dtype_code(x.dtype), _ptr(x.contiguous()), bs, c,
+        x, = self._sync_in(x)
+        self._check(lib().ag_max_pool2(self._h, _dtype_code(x.dtype), _ptr(x), bs, c,
                                        ih, iw, size[0], size[1], strides[0], strides[1], _ptr(y)))
         return y
 
@@ -568,10 +580,10 @@ class _PyDevice:
         if not dx.is_contiguous():
             raise AgError(_capi.AG_ERR_INVALID, "dx must be contiguous")
         bs, c, ih, iw = dx.shape
-        self._sync_in(dx, dy)
+        dy, = self._sync_in(dy, inout=(dx,))
         self._check(lib().ag_max_pool2_backward(self._h, _dtype_code(dx.dtype), _ptr(dx), bs, c, ih,
                                                 iw, size[0], size[1], strides[0], strides[1],
-                                                _ptr(dy.contiguous())))
+                                                _ptr(dy)))
         return dx
 
     def max_pool2_backward(self, x, dy, size=(2, 2), strides=None):
@@ -584,10 +596,10 @@ class _PyDevice:
         x = x.contiguous()
         dx = self._out(x.shape, x.dtype)
         bs, c, ih, iw = x.shape
-        self._sync_in(x, dy)
+        x, dy = self._sync_in(x, dy)
         self._check(lib().ag_max_pool2_backward_from_input(
             self._h, _dtype_code(x.dtype), _ptr(x), bs, c, ih, iw, size[0], size[1], strides[0],
-            strides[1], _ptr(dy.contiguous()), _ptr(dx)))
+            strides[1], _ptr(dy), _ptr(dx)))
         return dx
 
     def relu_max_pool2(self, x):
@@ -595,7 +607,7 @@ class _PyDevice:
         x = x.contiguous()
         bs, c, ih, iw = x.shape
         y = self._out((bs, c, ih // 2, iw // 2), x.dtype)
-        self._sync_in(x)
+        x, = self._sync_in(x)
         self._check(lib().ag_relu_max_pool2_forward(self._h, _dtype_code(x.dtype), _ptr(x), bs, c,
                                                     ih, iw, _ptr(y)))
         return y
@@ -605,22 +617,22 @@ class _PyDevice:
         x = x.contiguous()
         bs, c, ih, iw = x.shape
         dx = self._out(x.shape, x.dtype)
-        self._sync_in(x, dy)
+        x, dy = self._sync_in(x, dy)
         self._check(lib().ag_relu_max_pool2_backward(self._h, _dtype_code(x.dtype), _ptr(x), bs, c,
-                                                     ih, iw, _ptr(dy.contiguous()), _ptr(dx)))
+                                                     ih, iw, _ptr(dy), _ptr(dx)))
         return dx
 
     def relu(self, x, inplace=False):
         x = x.contiguous()
         y = x if inplace else self._out(x.shape, x.dtype)
-        self._sync_in(x)
+        x, = self._sync_in(x)
         self._check(lib().ag_relu(self._h, _dtype_code(x.dtype), _ptr(x), _ptr(y), x.numel()))
         return y
 
     def relu_backward(self, x, dy, inplace=False):
         x, dy = x.contiguous(), dy.contiguous()
         dx = dy if inplace else self._out(dy.shape, dy.dtype)
-        self._sync_in(x, dy)
+        x, dy = self._sync_in(x, dy)
         self._check(lib().ag_relu_backward(self._h, _dtype_code(x.dtype), _ptr(x), _ptr(dy),
                                            _ptr(dx), x.numel()))
         return dx
@@ -629,7 +641,7 @@ class _PyDevice:
     def scaled_add(self, y, alpha, x):
         """≙ ``y.scaled_add(alpha, &x)`` (in place on y)."""
         assert y.is_contiguous() and x.is_contiguous() and x.shape == y.shape
-        self._sync_in(y, x)
+        x, = self._sync_in(x, inout=(y,))
         self._check(lib().ag_scaled_add(self._h, _dtype_code(y.dtype), ctypes.c_float(alpha),
                                         _ptr(x), _ptr(y), y.numel()))
         return y
@@ -637,7 +649,7 @@ class _PyDevice:
     def bias_add(self, y, bias):
         rows, cols = y.shape[0], y.shape[1]
         inner = y[0, 0].numel() if y.dim() > 2 else 1
-        self._sync_in(y, bias)
+        bias, = self._sync_in(bias, inout=(y,))
         self._check(lib().ag_bias_add(self._h, _dtype_code(y.dtype), _ptr(y), _ptr(bias), rows,
                                       cols, inner))
         return y
@@ -647,8 +659,8 @@ class _PyDevice:
         inner = dy[0, 0].numel() if dy.dim() > 2 else 1
         if out is None:
             out = self._out((cols,), dy.dtype)
-        self._sync_in(dy, out)
-        self._check(lib().ag_bias_grad(self._h, _dtype_code(dy.dtype), _ptr(dy.contiguous()), rows,
+        dy, = self._sync_in(dy, inout=(out,))
+        self._check(lib().ag_bias_grad(self._h, _dtype_code(dy.dtype), _ptr(dy), rows,
                                        cols, inner, ctypes.c_float(beta), _ptr(out)))
         return out
 
@@ -659,9 +671,9 @@ class _PyDevice:
             raise AgError(_capi.AG_ERR_SHAPE, f"Expected target with shape [{bs}], found "
                                               f"[{t.shape[0]}]")
         loss = ctypes.c_float()
-        self._sync_in(x, t)
+        x, t = self._sync_in(x, t)
         self._check(lib().ag_cross_entropy_loss(self._h, _dtype_code(x.dtype), _dtype_code(t.dtype),
-                                                _ptr(x.contiguous()), _ptr(t), bs, classes,
+                                                _ptr(x), _ptr(t), bs, classes,
                                                 ctypes.byref(loss)))
         return loss.value
 
@@ -671,7 +683,7 @@ class _PyDevice:
         x, t = x.contiguous(), t.contiguous()
         loss = torch.empty((1,), dtype=torch.float32, device=self.torch_device)
         dx = self._out(x.shape, x.dtype)
-        self._sync_in(x, t)
+        x, t = self._sync_in(x, t)
         self._check(lib().ag_cross_entropy_loss_device_grad(
             self._h, _dtype_code(x.dtype), _dtype_code(t.dtype), _ptr(x), _ptr(t), x.shape[0],
             x.shape[1], _ptr(loss), ctypes.c_float(dy), _ptr(dx)))
@@ -680,30 +692,30 @@ class _PyDevice:
     def cross_entropy_loss_backward(self, x, t, dy=1.0):
         bs, classes = x.shape
         dx = self._out(x.shape, x.dtype)
-        self._sync_in(x, t)
+        x, t = self._sync_in(x, t)
         self._check(lib().ag_cross_entropy_loss_backward(
-            self._h, _dtype_code(x.dtype), _dtype_code(t.dtype), _ptr(x.contiguous()), _ptr(t), bs,
+            self._h, _dtype_code(x.dtype), _dtype_code(t.dtype), _ptr(x), _ptr(t), bs,
             classes, ctypes.c_float(dy), _ptr(dx)))
         return dx
 
     def accuracy(self, x, t) -> int:
         bs, classes = x.shape
         out = ctypes.c_uint64()
-        self._sync_in(x, t)
+        x, t = self._sync_in(x, t)
         self._check(lib().ag_accuracy(self._h, _dtype_code(x.dtype), _dtype_code(t.dtype),
-                                      _ptr(x.contiguous()), _ptr(t), bs, classes,
+                                      _ptr(x), _ptr(t), bs, classes,
                                       ctypes.byref(out)))
         return out.value
 
     # -- optimizer ----------------------------------------------------------------------
     def sgd_update(self, w, g, lr):
-        self._sync_in(w, g)
+        g, = self._sync_in(g, inout=(w,))
         self._check(lib().ag_sgd_update(self._h, _dtype_code(w.dtype), _ptr(w), _ptr(g), w.numel(),
                                         ctypes.c_float(lr)))
         return w
 
     def sgd_update_momentum(self, w, g, v, lr, momentum):
-        self._sync_in(w, g, v)
+        g, = self._sync_in(g, inout=(w, v))
         self._check(lib().ag_sgd_update_momentum(self._h, _dtype_code(w.dtype), _ptr(w), _ptr(g),
                                                  _ptr(v), w.numel(), ctypes.c_float(lr),
                                                  ctypes.c_float(momentum)))

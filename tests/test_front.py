@@ -1,14 +1,17 @@
 """The front end without a GPU: which calls the extension takes itself, and what the Python forms refuse before
 anything is launched."""
+import ctypes
 import subprocess
 import sys
 import textwrap
+import weakref
 from pathlib import Path
 
 import pytest
 import torch
 
 import autograph_b200 as ag
+from autograph_b200 import _capi
 
 ROOT = Path(__file__).resolve().parent.parent
 
@@ -50,7 +53,7 @@ def no_launch(monkeypatch):
 
     monkeypatch.setattr(ag, "lib", Library)
     d = ag._PyDevice.__new__(ag._PyDevice)
-    d.index, d.torch_device, d._stream_ptr = 0, torch.device("cpu"), 0
+    d.index, d.torch_device, d._stream_ptr, d._h = 0, torch.device("cpu"), 0, None
     return d
 
 
@@ -70,6 +73,72 @@ def test_operators_refuse_tensors_of_another_gpu(no_launch):
             continue   # its intermediate outputs are the operator's own
         with pytest.raises(ag.AgError, match="on another GPU"):
             getattr(ag._PyDevice, name)(no_launch, *args, **kw)
+
+
+def test_python_forms_hold_copies_and_refuse_strided_outputs(no_launch, monkeypatch):
+    """Operands that are not contiguous reach the library as contiguous copies that are all alive during the call: freed
+    before it, the memory of one was the next one's.  Tensors that are written too are refused instead."""
+    copies, originals = [], set()
+
+    class Here(torch.Tensor):
+        is_cuda, device = True, torch.device("cuda", 0)
+
+        def contiguous(self):
+            if self.is_contiguous():
+                return self
+            t = super().contiguous()
+            copies.append(weakref.ref(t))
+            originals.add(self.data_ptr())
+            return t
+
+    def strided(shape, dt=torch.float32):
+        if len(shape) == 1:
+            return torch.zeros(2 * shape[0], dtype=dt)[::2].as_subclass(Here)
+        return torch.zeros(shape[::-1], dtype=dt).permute(*reversed(range(len(shape)))).as_subclass(Here)
+
+    def pointers(args):
+        for a in args:
+            if isinstance(a, ctypes.c_void_p):
+                yield a.value
+            elif isinstance(a, ctypes.Array) and a._type_ is ctypes.c_void_p:
+                yield from a
+            elif isinstance(a, ctypes.Array) and a._type_ is _capi.ConvStage:
+                yield from (p for st in a for p in (st.w, st.bias))
+
+    reached = []
+
+    class Library:
+        ag_conv2_output_shape = ag.lib().ag_conv2_output_shape
+
+        def __getattr__(self, name):
+            def call(*args):
+                assert copies and all(ref() is not None for ref in copies), f"{name}: a copy was freed"
+                assert not originals & set(pointers(args)), f"{name}: reads a strided tensor"
+                reached.append(name)
+                return 0
+            return call
+
+    library = Library()
+    monkeypatch.setattr(ag, "lib", lambda: library)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda index: type("Stream", (), {"cuda_stream": 0}))
+    written = {"gemm": None, "conv2_backward_weight": "dw", "max_pool2_backward_inplace": 0, "bias_add": 0, "bias_grad": "out",
+               "sgd_update": 0, "sgd_update_momentum": (0, 2)}
+    for name, args, kw in _operator_calls(strided):
+        if name in ("gemm", "dot", "scaled_add"):
+            continue   # strides are passed on; refused by an assertion
+        args, outs = list(args), written.get(name, ())
+        for key in outs if isinstance(outs, tuple) else (outs,):
+            at = kw if isinstance(key, str) else args
+            before, at[key] = at[key], torch.zeros(at[key].shape).as_subclass(Here)
+            with pytest.raises(ag.AgError, match="must be contiguous"):
+                at[key], plain = before, at[key]
+                getattr(ag._PyDevice, name)(no_launch, *args, **kw)
+            at[key] = plain
+        copies.clear()
+        originals.clear()
+        reached.clear()
+        getattr(ag._PyDevice, name)(no_launch, *args, **kw)
+        assert len(reached) == 1, name
 
 
 # In a process of its own: the library's functions are replaced by ones that count, and no device is needed for the

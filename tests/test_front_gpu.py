@@ -94,6 +94,37 @@ def test_a_default_device_changes_nothing(plain, dtype):
         assert got.device == want.device and torch.equal(got, want), name
 
 
+def _strided(t):
+    if t.dim() == 1:
+        return torch.stack((t, t + 1), 1)[:, 0]
+    back = tuple(reversed(range(t.dim())))
+    return t.permute(back).contiguous().permute(back)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_strided_operands(plain, dtype):
+    """Every operand strided at once, of equal sizes too: a copy freed early would be the next one's memory."""
+    sq = lambda k: torch.randn((64, 64), generator=torch.Generator("cuda").manual_seed(k), device="cuda").to(dtype)
+    calls = _calls(plain, dtype) + [("dense_forward", (sq(1), sq(2)), {}), ("dense_chain_forward", (sq(1), [sq(2), sq(3)]), {}),
+                                    ("relu_backward", (sq(1), sq(2)), {})]
+    for name, args, kw in calls:
+        if name in ("gemm", "bias_add") or kw.get("inplace") or "out" in kw or "dw" in kw or any(a is True for a in args):
+            continue
+        as_strided = lambda v: _strided(v) if isinstance(v, torch.Tensor) else [_strided(t) for t in v] if isinstance(v, list) else v
+        want = getattr(plain, name)(*args, **kw)
+        got = getattr(plain, name)(*map(as_strided, args), **{k: as_strided(v) for k, v in kw.items()})
+        assert torch.equal(got, want), name
+    other = torch.cuda.Stream()
+    a, b = sq(4), sq(5)
+    want = plain.dense_forward(a, b)
+    plain.wait()
+    with torch.cuda.stream(other):
+        got = [plain.dense_forward(_strided(a), _strided(b)) for _ in range(50)]
+    other.synchronize()
+    plain.wait()
+    assert all(torch.equal(g, want) for g in got)
+
+
 def test_another_current_stream_is_ordered(plain):
     """Inputs produced on another current stream: the call waits for that stream."""
     a = torch.zeros((512, 512), device=plain.torch_device)
