@@ -140,11 +140,11 @@ class _PyDevice:
                                                      ctypes.byref(handle)))
         self._h = handle
         _bind_front()
-        self._bind(handle.value, self._stream_ptr, index, self.torch_device)
+        self._bind(handle.value, self._stream_ptr, index)
 
     def close(self):
         if getattr(self, "_h", None):
-            self._bind(0, 0, self.index, self.torch_device)
+            self._bind(0, 0, self.index)
             lib().ag_device_destroy(self._h)
             self._h = None
 

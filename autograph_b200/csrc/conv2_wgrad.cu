@@ -174,7 +174,8 @@ static int launch_wgrad(ag_device *dev, const T *x, const T *dy, const WgradPara
     AG_TRY(workspace(dev, sizeof(float) * (size_t)ctas * (size_t)len, &ws));
     const int threads = ((p.items * p.slices + 31) / 32) * 32;
     AG_TRY((launch_dependent(dev, kernel, dim3((unsigned)ctas), threads, smem, x, dy, (float *)ws, p)));
-    AG_TRY((launch_dependent(dev, conv2_wgrad_reduce_kernel<T>, dim3((unsigned)ceil_div(len, 32)), 256, 0, (const float *)ws, ctas, len, beta, dw)));
+    AG_TRY((launch_dependent(dev, conv2_wgrad_reduce_kernel<T>, dim3((unsigned)ceil_div(len, 32)), 256, 0,
+                             (const float *)ws, ctas, len, beta, dw)));
     return AG_OK;
 }
 

@@ -433,7 +433,9 @@ static bool halo_enabled() {
 int to_nhwc(ag_device *dev, const __nv_bfloat16 *x, int64_t bs, int64_t c, int64_t hw, int64_t cp,
             __nv_bfloat16 *out) {
     // no border: the frame is the image, any width gives the same row index
-    AG_TRY((launch_dependent(dev, nchw_to_nhwc_kernel, dim3((unsigned)ceil_div(hw, 256), (unsigned)(cp / 16), (unsigned)bs), 256, 0, x, out, (int)c, (int)hw, (int)cp, (int)hw, 1, (int)hw, 0, 0)));
+    AG_TRY((launch_dependent(dev, nchw_to_nhwc_kernel,
+                             dim3((unsigned)ceil_div(hw, 256), (unsigned)(cp / 16), (unsigned)bs), 256, 0, x, out,
+                             (int)c, (int)hw, (int)cp, (int)hw, 1, (int)hw, 0, 0)));
     return AG_OK;
 }
 
@@ -442,7 +444,9 @@ int to_nhwc_framed(ag_device *dev, const __nv_bfloat16 *x, int64_t bs, int64_t c
     const int64_t hp = h + 2 * pad_h, wp = w + 2 * pad_w;
     if (pad_h || pad_w)
         AG_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)(bs * hp * wp * cp * 2), dev->stream));
-    AG_TRY((launch_dependent(dev, nchw_to_nhwc_kernel, dim3((unsigned)ceil_div(h * w, 256), (unsigned)(cp / 16), (unsigned)bs), 256, 0, x, out, (int)c, (int)(h * w), (int)cp, (int)w, (int)hp, (int)wp, pad_h, pad_w)));
+    AG_TRY((launch_dependent(dev, nchw_to_nhwc_kernel,
+                             dim3((unsigned)ceil_div(h * w, 256), (unsigned)(cp / 16), (unsigned)bs), 256, 0, x, out,
+                             (int)c, (int)(h * w), (int)cp, (int)w, (int)hp, (int)wp, pad_h, pad_w)));
     return AG_OK;
 }
 
@@ -511,7 +515,9 @@ int64_t nhwc_filter_scratch_bytes(const NhwcConv &c) {
 
 int from_nhwc(ag_device *dev, const __nv_bfloat16 *in, int64_t bs, int64_t c, int64_t hw, int64_t cp,
               __nv_bfloat16 *out) {
-    AG_TRY((launch_dependent(dev, nhwc_to_nchw_kernel, dim3((unsigned)ceil_div(hw, NCHW_PIX), (unsigned)ceil_div(c, 16), (unsigned)bs), 256, 0, in, out, (int)c, (int)hw, (int)cp)));
+    AG_TRY((launch_dependent(dev, nhwc_to_nchw_kernel,
+                             dim3((unsigned)ceil_div(hw, NCHW_PIX), (unsigned)ceil_div(c, 16), (unsigned)bs), 256, 0,
+                             in, out, (int)c, (int)hw, (int)cp)));
     return AG_OK;
 }
 
@@ -533,7 +539,8 @@ int correlate_nhwc(ag_device *dev, const NhwcConv &c, const __nv_bfloat16 *act_n
     const int64_t wk_elems = c_out * taps * cp;
     const int64_t ocp = round_up(c_out, 64);
     const unsigned rgrid = (unsigned)ceil_div(wk_elems, 256);
-    AG_TRY(launch_dependent(dev, c.transposed ? repack_filters_transposed_kernel : repack_filters_kernel, dim3(rgrid), 256, 0, w, wk,
+    AG_TRY(launch_dependent(dev, c.transposed ? repack_filters_transposed_kernel : repack_filters_kernel, dim3(rgrid),
+                            256, 0, w, wk,
                             (int)w_oc, (int)w_ic, taps, (int)cp));
     if (halo)
         return run_halo(dev, act_nhwc, wk, bs, cp, hp, wp, fh, fw, c_out, out_h, out_w, bias, relu,

@@ -63,7 +63,8 @@ static int patches_times_filters(ag_device *dev, const T *src, const ConvMap &ma
         staging(dev, (size_t)total * sizeof(T), &ws) != AG_OK)
         return gemm<T>(dev, M, N, K, ConvRows<T>{src, map, M}, FilterRows<T>{w, s_row, s_c, map.channels, map.div_cp}, E);
     T *packed = (T *)ws;
-    AG_TRY((launch_dependent(dev, repack_kernel<T>, dim3((unsigned)ceil_div(total, 256)), 256, 0, w, packed, total, map.channels, map.cp, s_row, s_c, FastDiv((uint32_t)K), map.div_cp)));
+    AG_TRY((launch_dependent(dev, repack_kernel<T>, dim3((unsigned)ceil_div(total, 256)), 256, 0, w, packed, total,
+                             map.channels, map.cp, s_row, s_c, FastDiv((uint32_t)K), map.div_cp)));
     return gemm<T>(dev, M, N, K, ConvRows<T>{src, map, M}, strided<kVecK>((const T *)packed, K, 1, N), E);
 }
 
@@ -153,7 +154,9 @@ int conv_backward_input(ag_device *dev, const T *w, int64_t oc, int64_t ic, cons
                            ConvRows<T>{dy + b * oc * oh * ow, conv_map(oc, oh, ow, oh, ow, &point, false), (int)positions},
                            strided<kByRow>(w, 1, taps_n, taps_n), StridedOut<float>{col, 1, positions, 1.f, 0.f}));
             const int total = (int)(n * ic * ih * iw);
-            AG_TRY((launch_dependent(dev, taps_to_image_kernel<T>, dim3((unsigned)ceil_div(total, 256)), 256, 0, col, dx + b * ic * ih * iw, map, (int)(oh * ow), positions, total, FastDiv((uint32_t)(ih * iw)), FastDiv((uint32_t)iw), FastDiv((uint32_t)ic))));
+            AG_TRY((launch_dependent(dev, taps_to_image_kernel<T>, dim3((unsigned)ceil_div(total, 256)), 256, 0, col,
+                                     dx + b * ic * ih * iw, map, (int)(oh * ow), positions, total,
+                                     FastDiv((uint32_t)(ih * iw)), FastDiv((uint32_t)iw), FastDiv((uint32_t)ic))));
         }
         return AG_OK;
     }

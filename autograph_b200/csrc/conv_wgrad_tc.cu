@@ -394,7 +394,8 @@ int backward_weight_nhwc(ag_device *dev, const __nv_bfloat16 *xh, int64_t bs, in
     else
         AG_TRY(launch_wgrad<64>(dev, tdy, tx, p, grid));
     const int64_t outs = oc * p.taps * ic;
-    AG_TRY((launch_dependent(dev, wgrad_reduce_kernel, dim3((unsigned)ceil_div(outs, 32)), dim3(32, 8), 0, p.partial, splits, m_total, p.taps, (int)cp, (int)oc, (int)ic, beta, dw)));
+    AG_TRY((launch_dependent(dev, wgrad_reduce_kernel, dim3((unsigned)ceil_div(outs, 32)), dim3(32, 8), 0, p.partial,
+                             splits, m_total, p.taps, (int)cp, (int)oc, (int)ic, beta, dw)));
     return AG_OK;
 }
 

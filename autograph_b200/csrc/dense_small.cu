@@ -156,7 +156,8 @@ bool fits_one_kernel(int64_t k, int64_t n) { return n > 0 && n <= 256 && k > 0 &
 template <class T, int R>
 static int launch_small(ag_device *dev, const T *x, T *y, int m, const ChainStep &st) {
     const size_t smem = ((size_t)st.K + (size_t)st.slices * 32) * R * sizeof(float);
-    AG_TRY((launch_dependent(dev, dense_small_kernel<T, R>, dim3((unsigned)ceil_div(m, R), (unsigned)(st.np / 32)), 32 * st.slices, smem, x, y, m, st)));
+    AG_TRY((launch_dependent(dev, dense_small_kernel<T, R>, dim3((unsigned)ceil_div(m, R), (unsigned)(st.np / 32)),
+                             32 * st.slices, smem, x, y, m, st)));
     return AG_OK;
 }
 
@@ -173,7 +174,8 @@ int forward(ag_device *dev, const T *x, int m, int k, const T *w, int n, const T
     if (narrow_step(st)) {
         // as many rows per CTA, up to four, as leave every SM one; 512 inputs and 16 outputs take 40 KB
         const int r = ceil_div(m, 4) >= dev->sm_count ? 4 : ceil_div(m, 2) >= dev->sm_count ? 2 : 1;
-        AG_TRY((launch_dependent(dev, dense_narrow_kernel<T>, dim3((unsigned)ceil_div(m, r)), 256, sizeof(float) * (size_t)k * (n + r), x, y, m, r, st)));
+        AG_TRY((launch_dependent(dev, dense_narrow_kernel<T>, dim3((unsigned)ceil_div(m, r)), 256,
+                                 sizeof(float) * (size_t)k * (n + r), x, y, m, r, st)));
         return AG_OK;
     }
     if ((int64_t)m * st.np > (sizeof(T) == 4 ? 256 : 128) * (int64_t)k) {
@@ -185,7 +187,8 @@ int forward(ag_device *dev, const T *x, int m, int k, const T *w, int n, const T
                                              80 * 1024));
             configured_on[dev->ordinal & 63] = true;
         }
-        AG_TRY((launch_dependent(dev, dense_rows_kernel<T>, dim3((unsigned)ceil_div(m, ROWS)), threads, smem, x, y, m, st)));
+        AG_TRY((launch_dependent(dev, dense_rows_kernel<T>, dim3((unsigned)ceil_div(m, ROWS)), threads, smem, x, y, m,
+                                 st)));
         return AG_OK;
     }
     // the most rows per CTA (weights read once for them) that still give every SM eight warps;

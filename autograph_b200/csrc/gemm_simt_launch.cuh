@@ -13,7 +13,8 @@ int launch_cfg(ag_device *dev, int M, int N, int K, int splits, int k_chunk, con
     dim3 grid((unsigned)ceil_div(M, Cfg::BM), (unsigned)ceil_div(N, Cfg::BN), (unsigned)splits);
     AG_REQUIRE(grid.y <= 65535u && grid.z <= 65535u, AG_ERR_LIMIT,
                "problem too large for one launch (n tiles %u, splits %u)", grid.y, grid.z);
-    AG_TRY((launch_dependent(dev, gemm_simt_kernel<Cfg, AOp, BOp, Epi>, grid, Cfg::THREADS, 0, M, N, K, k_chunk, A, B, E)));
+    AG_TRY((launch_dependent(dev, gemm_simt_kernel<Cfg, AOp, BOp, Epi>, grid, Cfg::THREADS, 0, M, N, K, k_chunk, A, B,
+                             E)));
     return AG_OK;
 }
 
@@ -95,10 +96,12 @@ int gemm(ag_device *dev, int M, int N, int K, const AOp &A, const BOp &B, const 
     PartialEpilogue P{(float *)ws, plane, N};
     AG_TRY(launch_any(dev, id, M, N, K, splits, k_chunk, A, B, P));
     if (splits >= 16 && plane <= 32 * 4 * (int64_t)dev->sm_count) {
-        AG_TRY((launch_dependent(dev, splitk_reduce_small_kernel<Epi>, dim3((unsigned)ceil_div(plane, 32)), 256, 0, (const float *)ws, plane, splits, M, N, E)));
+        AG_TRY((launch_dependent(dev, splitk_reduce_small_kernel<Epi>, dim3((unsigned)ceil_div(plane, 32)), 256, 0,
+                                 (const float *)ws, plane, splits, M, N, E)));
     } else {
         int threads = 256;
-        AG_TRY((launch_dependent(dev, splitk_reduce_kernel<Epi>, dim3((unsigned)ceil_div(plane, threads)), threads, 0, (const float *)ws, plane, splits, M, N, E)));
+        AG_TRY((launch_dependent(dev, splitk_reduce_kernel<Epi>, dim3((unsigned)ceil_div(plane, threads)), threads, 0,
+                                 (const float *)ws, plane, splits, M, N, E)));
     }
     return AG_OK;
 }

@@ -496,11 +496,13 @@ int gemm_bf16(ag_device *dev, int m, int k, int n, float alpha, const __nv_bfloa
         if (epi) {
             using Epi = simt::BiasReluEpilogue<__nv_bfloat16>;
             Epi E{c, rsc, epi->bias, epi->relu};
-            AG_TRY((launch_dependent(dev, simt::splitk_reduce_kernel<Epi>, dim3((unsigned)ceil_div(plane, 256)), 256, 0, p.partial, plane, splits, m, n, E)));
+            AG_TRY((launch_dependent(dev, simt::splitk_reduce_kernel<Epi>, dim3((unsigned)ceil_div(plane, 256)), 256, 0,
+                                     p.partial, plane, splits, m, n, E)));
         } else {
             using Epi = simt::StridedEpilogue<__nv_bfloat16>;
             Epi E{c, rsc, 1, alpha, beta, false, n};
-            AG_TRY((launch_dependent(dev, simt::splitk_reduce_kernel<Epi>, dim3((unsigned)ceil_div(plane, 256)), 256, 0, p.partial, plane, splits, m, n, E)));
+            AG_TRY((launch_dependent(dev, simt::splitk_reduce_kernel<Epi>, dim3((unsigned)ceil_div(plane, 256)), 256, 0,
+                                     p.partial, plane, splits, m, n, E)));
         }
     }
     return AG_OK;

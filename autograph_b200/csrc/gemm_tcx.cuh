@@ -1174,7 +1174,8 @@ int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
         if (C::PL == 1) break;
     }
     if (p.splits > 1 && p.arrivals == nullptr) {
-        AG_TRY(launch_dependent(dev, reduce_splits_kernel<Epi>, dim3((unsigned)ceil_div((int64_t)p.M * p.N, 256)), 256, 0,
+        AG_TRY(launch_dependent(dev, reduce_splits_kernel<Epi>, dim3((unsigned)ceil_div((int64_t)p.M * p.N, 256)), 256,
+                                0,
                                 (const float *)p.partial, p.splits, p.M, p.N, FastDiv((uint32_t)p.M), E));
     }
     return AG_OK;

@@ -921,7 +921,8 @@ static int step_typed(ag_device *dev, const Net &net, const void *x, const uint8
     f.row_loss = a.row_loss;
     f.loss = loss;
     // Dependent launches: at 100 images the step is a chain of launches, each of which started 2 us after the last.
-    AG_TRY(launch_dependent(dev, lenet_finish_kernel<T>, dim3((unsigned)(kTiles * f.splits + kConvBlocks + 1)), 256, 0, f));
+    AG_TRY(launch_dependent(dev, lenet_finish_kernel<T>, dim3((unsigned)(kTiles * f.splits + kConvBlocks + 1)), 256, 0,
+                            f));
     if (f.splits > 1)
         AG_TRY(launch_dependent(dev, lenet_reduce_kernel<T>, dim3((unsigned)ceil_div(kDense, 256)), 256, 0, f));
     return AG_OK;

@@ -316,7 +316,8 @@ int relu_pool(ag_device *dev, const __nv_bfloat16 *pre, int64_t bs, int64_t ih, 
     const int64_t ph = ih / 2, pw = iw / 2;
     const int64_t total = bs * ph * pw * (cp / 8);
     if (total == 0) return AG_OK;
-    AG_TRY((launch_dependent(dev, relu_pool_kernel, dim3(grid_for(dev, total)), 256, 0, pre, y, codes, (int)ih, (int)iw, (int)ph, (int)pw, (int)cp, total)));
+    AG_TRY((launch_dependent(dev, relu_pool_kernel, dim3(grid_for(dev, total)), 256, 0, pre, y, codes, (int)ih, (int)iw,
+                             (int)ph, (int)pw, (int)cp, total)));
     return AG_OK;
 }
 
@@ -330,7 +331,9 @@ int relu_pool_backward(ag_device *dev, const __nv_bfloat16 *pre, const uint32_t 
     AG_REQUIRE(pre != nullptr || (ih % 2 == 0 && iw % 2 == 0), AG_ERR_INVALID, "relu_pool_backward: odd planes need pre");
     const int64_t total = bs * ((ih + 1) / 2) * ((iw + 1) / 2) * (cp / 8);
     if (total == 0) return AG_OK;
-    AG_TRY((launch_dependent(dev, relu_pool_backward_kernel, dim3(grid_for(dev, total)), 256, 0, pre, codes, dy, out, (int)ih, (int)iw, (int)(ih / 2), (int)(iw / 2), (int)cp, out_row_pitch, out_image_pitch, total)));
+    AG_TRY((launch_dependent(dev, relu_pool_backward_kernel, dim3(grid_for(dev, total)), 256, 0, pre, codes, dy, out,
+                             (int)ih, (int)iw, (int)(ih / 2), (int)(iw / 2), (int)cp, out_row_pitch, out_image_pitch,
+                             total)));
     return AG_OK;
 }
 
@@ -340,7 +343,8 @@ int zero_frame(ag_device *dev, __nv_bfloat16 *framed, int64_t bs, int64_t hp, in
     const int64_t cells = 2 * (int64_t)pad_h * wp + 2 * (int64_t)pad_w * (hp - 2 * pad_h);
     const int64_t total = bs * cells * (cp / 8);
     if (total <= 0) return AG_OK;
-    AG_TRY((launch_dependent(dev, zero_frame_kernel, dim3(grid_for(dev, total)), 256, 0, framed, (int)hp, (int)wp, pad_h, pad_w, (int)cp, cells, total)));
+    AG_TRY((launch_dependent(dev, zero_frame_kernel, dim3(grid_for(dev, total)), 256, 0, framed, (int)hp, (int)wp,
+                             pad_h, pad_w, (int)cp, cells, total)));
     return AG_OK;
 }
 

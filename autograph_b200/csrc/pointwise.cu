@@ -87,7 +87,8 @@ static int map2(ag_device *dev, const T *a, const T *b, T *out, int64_t n, F f) 
     const bool vec = aligned16(a) && aligned16(out) && (b == nullptr || aligned16(b));
     const int threads = 256;
     const int64_t items = vec ? ceil_div(n, Vec16<T>::N) : n;
-    AG_TRY((launch_dependent(dev, map2_kernel<T, F>, dim3(grid_for(items, threads, dev->sm_count)), threads, 0, a, b, out, n, vec, f)));
+    AG_TRY((launch_dependent(dev, map2_kernel<T, F>,
+                             dim3(grid_for(items, threads, dev->sm_count)), threads, 0, a, b, out, n, vec, f)));
     return AG_OK;
 }
 
@@ -441,7 +442,8 @@ template <class T, bool RELU, bool PAIR>
 static int pool_windows_as(ag_device *dev, const T *x, T *y, int64_t planes, int64_t ih, int64_t iw, int64_t oh, int64_t ow) {
     return for_pool_planes(dev, planes, ih, iw, oh, ow, pool_windows_per_thread<T, PAIR>(),
                            [&](int64_t p, int64_t y0, const PoolMap &m, dim3 grid) {
-        return launch_dependent(dev, max_pool2_2x2_window_kernel<T, RELU, PAIR>, grid, 256, 0, x + (p * ih + 2 * y0) * iw,
+        return launch_dependent(dev, max_pool2_2x2_window_kernel<T, RELU, PAIR>, grid, 256, 0,
+                                x + (p * ih + 2 * y0) * iw,
                                 y + (p * oh + y0) * ow, m);
     });
 }
@@ -781,7 +783,8 @@ static int bias_grad_planes(ag_device *dev, const T *x, int64_t rows, int64_t co
     AG_TRY(workspace(dev, sizeof(float) * (size_t)chunks * (size_t)cols, &ws));
     // one launch when every column has a counter
     int *arrivals = cols < kTileCounters ? dev->tile_counters : nullptr;
-    AG_TRY((launch_dependent(dev, bias_grad_planes_kernel<T>, dim3((unsigned)cols, (unsigned)chunks), 256, 0, x, (float *)ws, cols, inner, units, per_chunk, (int)per_row, arrivals, y, beta)));
+    AG_TRY((launch_dependent(dev, bias_grad_planes_kernel<T>, dim3((unsigned)cols, (unsigned)chunks), 256, 0, x,
+                             (float *)ws, cols, inner, units, per_chunk, (int)per_row, arrivals, y, beta)));
     if (arrivals != nullptr) return AG_OK;
     bias_grad_final_kernel<T><<<(unsigned)ceil_div(cols, 32), dim3(32, 8), 0, dev->stream>>>((const float *)ws, y, cols, (int)chunks,
                                                                                              beta);
@@ -896,7 +899,8 @@ static int pool_forward(ag_device *dev, const T *x, T *y, int64_t planes, int ih
     const int64_t plane_bytes = (int64_t)ih * iw * (int64_t)sizeof(T);
     if (h == 2 && w == 2 && sh == 2 && sw == 2 && iw % V == 0 && aligned16(x)) {
         const int64_t items = planes * oh * (iw / V);
-        return launch_dependent(dev, max_pool2_2x2_kernel<T>, dim3(grid_for(items, threads, dev->sm_count)), threads, 0, x, y, planes, ih,
+        return launch_dependent(dev, max_pool2_2x2_kernel<T>,
+                                dim3(grid_for(items, threads, dev->sm_count)), threads, 0, x, y, planes, ih,
                                 iw, oh, ow);
     } else if (h == 2 && w == 2 && sh == 2 && sw == 2) {
         return pool_windows<T, false>(dev, x, y, planes, ih, iw, oh, ow);
@@ -1034,7 +1038,8 @@ static int pool_backward(ag_device *dev, ag_dtype dtype, const void *x, void *dx
         (reinterpret_cast<uintptr_t>(dx) & 15) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
         ((ih & 1) == 0 || x == dx)) {  // out of place, a last row no window covers must be copied
         const unsigned grid2 = grid_for(planes * oh * (iw / vlen), threads, dev->sm_count);
-        AG_DISPATCH_FLOAT(dtype, T, return launch_dependent(dev, max_pool2_backward_2x2_kernel<T>, dim3(grid2), threads, 0, (const T *)x,
+        AG_DISPATCH_FLOAT(dtype, T, return launch_dependent(dev, max_pool2_backward_2x2_kernel<T>, dim3(grid2), threads,
+                0, (const T *)x,
                                                             (T *)dx, (const T *)dy, planes, (int)ih, (int)iw, oh, ow););
     }
     if (h == 2 && w == 2 && sh == 2 && sw == 2 && !many_small_odd_planes(dtype, planes, ih, iw))

@@ -520,14 +520,12 @@ ENTRY(bias_grad) {
     return finish(st, out);
 }
 
-/* _bind(handle, stream, index, torch_device): handle 0 when the device is closed */
+/* _bind(handle, stream, index): handle 0 when the device is closed */
 static PyObject *device_bind(PyObject *self, PyObject *args) {
     DeviceObject *d = (DeviceObject *)self;
     unsigned long long h, stream;
     int index;
-    PyObject *dev;
-    if (!PyArg_ParseTuple(args, "KKiO", &h, &stream, &index, &dev)) return NULL;
-    (void)dev;
+    if (!PyArg_ParseTuple(args, "KKi", &h, &stream, &index)) return NULL;
     d->h = (ag_device *)(uintptr_t)h;
     d->stream = (uintptr_t)stream;
     d->index = index;

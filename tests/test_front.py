@@ -180,7 +180,7 @@ def test_extension_leaves_host_tensors_to_the_python_form():
     _in_process("""
         from test_front import _operator_calls
         d = _front.DeviceBase()
-        d._bind(1, 0, 0, None)
+        d._bind(1, 0, 0)
         for name, args, kw in _operator_calls(lambda s, dt=torch.float32: torch.zeros(s, dtype=dt)):
             if name in _front.METHODS:
                 assert taken(lambda: getattr(d, name)(*args, **kw)) == "python", name
