@@ -8,8 +8,10 @@
 // convolution and one Relu + pool kernel, the backward pass one kernel for the gradient at the
 // convolution's output (written straight into the zero frame the input-gradient kernel wants)
 // and the two gradient convolutions.  A first layer with few input channels (3 x 3 x 3 = 27 <= 64)
-// is run as a 1 x 1 convolution over its patches (the patch is the channel axis), which puts it on
-// the tensor cores too and makes its weight gradient a plain [oc][27] product.
+// on images (2 to 4 channels 3 x 3, 1 or 2 channels 5 x 5) is one kernel each way (image_stage.cuh) that keeps neither
+// patches nor the convolution's output; other geometries with so few values per patch, and odd planes whose uncovered
+// cells the backward pass needs, run as a 1 x 1 convolution over patches (the patch is the channel axis), which puts them
+// on the tensor cores too and makes the weight gradient a plain [oc][27] product.
 //
 // The values are those of the separate layers (Conv2 layer.rs:842-948, Relu layer.rs:1254-1298,
 // MaxPool2 layer.rs:1193-1216 and their backward edges): the same roundings at the same places,
@@ -22,6 +24,7 @@
 #include <vector>
 
 #include "../conv_tc.cuh"
+#include "../image_stage.cuh"
 #include "../nhwc_ops.cuh"
 #include "nn.hpp"
 
@@ -34,6 +37,8 @@ struct StageDesc {
     int64_t ph = 0, pw = 0;           // pooled
     int fh = 0, fw = 0;
     bool patches = false;             // few input channels: a 1 x 1 convolution over the patches
+    bool image = false;               // few input channels: the whole stage in one kernel
+    ::ag::image_stage::Shape image_shape(int64_t bs) const { return {bs, ic, ih, iw, oc, fh, fw}; }
     // the convolution as the kernels see it
     int64_t k_ic = 0, k_ih = 0, k_iw = 0;
     int k_fh = 0, k_fw = 0;
@@ -71,6 +76,7 @@ inline bool plan_stage(Conv2 &conv, const MaxPool2 &mp, ag_dtype dtype, int64_t 
     d->ocp = round_up_64(d->oc);
     if (d->ocp != d->oc) return false;   // whole 64-channel blocks only (also: the bias gradient is a column sum)
     d->patches = ic < 16 && ic * d->fh * d->fw <= 64 && !needs_dx;
+    d->image = d->patches && (!recording || (d->oh % 2 == 0 && d->ow % 2 == 0)) && ::ag::image_stage::takes(d->image_shape(bs));
     if (d->patches) {
         d->k_ic = ic * d->fh * d->fw; d->k_ih = d->oh; d->k_iw = d->ow;
         d->k_fh = d->k_fw = 1;
@@ -101,6 +107,7 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
     std::vector<Tensor> code;         // per stage: where each pool window's gradient goes
     std::vector<Tensor> dpre;         // per stage: gradient at the convolution's output (maybe framed)
     std::vector<char> have, framed;
+    Tensor sums;                      // an image stage's parameter gradients, by slices of the batch
 
     using bf16 = __nv_bfloat16;
     static const bf16 *cptr(const Tensor &t) { return reinterpret_cast<const bf16 *>(t.data()); }
@@ -149,6 +156,20 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
         Tensor pooled;
         for (size_t s = 0; s < st.size(); ++s) {
             const StageDesc &d = st[s];
+            Tensor y = make({bs, d.ph, d.pw, d.ocp});
+            Tensor codes = keep ? Tensor::uninit(*pool, {bs, d.ph, d.pw, d.ocp / 2}, AG_U8) : Tensor{};
+            if (d.image) {
+                check(::ag::image_stage::forward(dev, d.image_shape(bs), cptr(x), cptr(d.conv->weight.value),
+                                                 d.conv->has_bias ? cptr(d.conv->bias.value) : nullptr, ptr(y),
+                                                 keep ? (uint32_t *)codes.data() : nullptr));
+                if (keep) {
+                    code.push_back(codes);
+                    act.push_back(x);
+                    pre.push_back(Tensor{});
+                }
+                pooled = y;
+                continue;
+            }
             Tensor a;
             if (s == 0) {
                 if (d.patches) {
@@ -169,8 +190,6 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
             check(::ag::convtc::correlate_nhwc(
                 dev, c, cptr(a), ::ag::convtc::nhwc_wants_frame(c), cptr(wv), d.oc, d.k_ic,
                 d.conv->has_bias ? cptr(d.conv->bias.value) : nullptr, false, ptr(wk), ptr(p)));
-            Tensor y = make({bs, d.ph, d.pw, d.ocp});
-            Tensor codes = keep ? Tensor::uninit(*pool, {bs, d.ph, d.pw, d.ocp / 2}, AG_U8) : Tensor{};
             check(::ag::nhwc::relu_pool(dev, cptr(p), bs, d.oh, d.ow, d.ocp, ptr(y),
                                         keep ? (uint32_t *)codes.data() : nullptr));
             if (keep) {
@@ -215,7 +234,7 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
         return dx;
     }
 
-    // Makes dpre[s]; dy_out is the gradient at the run's output (NCHW).
+    // Makes dpre[s], or an image stage's sums; dy_out is the gradient at the run's output (NCHW).
     void ensure(size_t s, const Tensor &dy_out) {
         if (have[s]) return;
         ::ag::DeviceGuard guard(dev);
@@ -226,6 +245,13 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
             check(::ag::convtc::to_nhwc(dev, cptr(dy_out), bs, d.oc, d.ph * d.pw, d.ocp, ptr(dpool)));
         } else {
             dpool = input_gradient(s + 1, dy_out);
+        }
+        if (d.image) {
+            sums = Tensor::uninit(*pool, {::ag::image_stage::partial_floats(dev, d.image_shape(bs))}, AG_F32);
+            check(::ag::image_stage::backward(dev, d.image_shape(bs), cptr(act[s]), cptr(dpool),
+                                              (const uint32_t *)code[s].data(), (float *)sums.data()));
+            have[s] = 1;
+            return;
         }
         const bool fr = wants_dx(s) && ::ag::convtc::nhwc_wants_frame(backward_conv(d));
         framed[s] = fr ? 1 : 0;
@@ -248,6 +274,10 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
         ensure(s, dy_out);
         ::ag::DeviceGuard guard(dev);
         const StageDesc &d = st[s];
+        if (d.image) {
+            check(::ag::image_stage::weight_gradient(dev, d.image_shape(bs), (const float *)sums.data(), ptr(dw)));
+            return;
+        }
         const View v = interior(s);
         const ag_conv2_options ko = kernel_options(d);
         check(::ag::convtc::backward_weight_nhwc(dev, cptr(act[s]), bs, d.k_ic, d.k_ih, d.k_iw, v.p,
@@ -257,6 +287,11 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
     void bias_gradient(size_t s, const Tensor &dy_out, Tensor &db) {
         ensure(s, dy_out);
         const StageDesc &d = st[s];
+        if (d.image) {
+            ::ag::DeviceGuard guard(dev);
+            check(::ag::image_stage::bias_gradient(dev, d.image_shape(bs), (const float *)sums.data(), ptr(db)));
+            return;
+        }
         // column sums of the whole buffer: the frame, when there is one, holds zeros
         const int64_t rows = dpre[s].len() / d.ocp;
         check(ag_bias_grad(dev, AG_BF16, dpre[s].data(), rows, d.ocp, 1, 0.f, db.data()));

@@ -2,6 +2,7 @@
 // 16 bytes (8 channels of one pixel); consecutive threads take consecutive channel groups of a
 // pixel and then consecutive pixels, so every access of a warp is one contiguous run.
 #include "nhwc_ops.cuh"
+#include "pool_codes.cuh"
 
 namespace ag {
 namespace nhwc {
@@ -145,27 +146,13 @@ __global__ void relu_pool_kernel(const __nv_bfloat16 *__restrict__ pre, __nv_bfl
         const uint4 raw[4] = {*reinterpret_cast<const uint4 *>(p), *reinterpret_cast<const uint4 *>(p + cp),
                               *reinterpret_cast<const uint4 *>(p + (int64_t)iw * cp),
                               *reinterpret_cast<const uint4 *>(p + (int64_t)iw * cp + cp)};   // (0,0), (0,1), (1,0), (1,1)
-        // two channels per instruction: one at a time the arithmetic takes longer than the memory
         uint32_t code = 0, o[4];
-        const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            __nv_bfloat162 v[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const uint32_t w = (&raw[c].x)[j];
-                v[c] = __hmax2(*reinterpret_cast<const __nv_bfloat162 *>(&w), zero);   // Relu; a NaN gives 0
-            }
-            const __nv_bfloat162 m = __hmax2(__hmax2(v[0], v[1]), __hmax2(v[2], v[3]));
-            o[j] = *reinterpret_cast<const uint32_t *>(&m);
-            // the first cell that holds the maximum, and whether the Relu passes its gradient: it does
-            // for a positive maximum; a zero one is cell 0's, whose sign decides
-            const uint32_t e0 = __heq2_mask(v[0], m), e1 = __heq2_mask(v[1], m), e2 = __heq2_mask(v[2], m);
-            const uint32_t first = (&raw[0].x)[j];
-            const uint32_t pass = __hgt2_mask(m, zero) | __hge2_mask(*reinterpret_cast<const __nv_bfloat162 *>(&first), zero);
-            const uint32_t bit1 = ~e0 & ~e1, bit0 = ~e0 & (e1 | ~e2);
-            const uint32_t w = (bit0 & 0x00010001u) | (bit1 & 0x00020002u) | (pass & 0x00040004u);
-            code |= ((w | (w >> 12)) & 0xffu) << (8 * j);
+            const uint32_t cells[4] = {(&raw[0].x)[j], (&raw[1].x)[j], (&raw[2].x)[j], (&raw[3].x)[j]};
+            uint32_t c8;
+            o[j] = relu_pool_pair(cells, c8);
+            code |= c8 << (8 * j);
         }
         if (codes != nullptr) codes[i] = code;
         reinterpret_cast<uint4 *>(y)[i] = make_uint4(o[0], o[1], o[2], o[3]);

@@ -260,6 +260,41 @@ def test_channels_last_stage_runs(dev, case):
     model.close()
 
 
+@pytest.mark.parametrize("ic,f,oc,bs,h,w,bias", [
+    (3, 3, 64, 5, 34, 34, True),       # a last tile of 128 (and of 64) windows that is not full
+    (2, 3, 128, 3, 50, 30, False),     # two blocks of output channels
+    (4, 3, 192, 2, 48, 52, True),
+    (1, 5, 64, 8, 28, 28, True),
+    (2, 5, 256, 9, 26, 30, True),
+    (3, 3, 64, 90, 66, 66, True),      # several tiles per CTA, stages that are used again
+    (3, 3, 64, 4, 41, 35, True),       # odd planes, pixels in odd rows: inference alone takes the kernel
+])
+def test_stage_on_images(dev, ic, f, oc, bs, h, w, bias):
+    """Conv2 -> Relu -> MaxPool2 on images of few channels (image_stage.cu) against the oracle.  Pixels and filters are
+    small integers: the convolution is exact in bf16 and windows have many equal cells, so no gate can turn on a rounding.
+    What is left is the rounding of the logits and of the gradient that arrives (2^-9 each way)."""
+    import autograph_b200 as ag
+    ph, pw = (h - f + 1) // 2, (w - f + 1) // 2
+    spec = [("conv", ic, oc, (f, f), bias), ("relu",), ("pool", (2, 2)), ("flatten",), ("dense", oc * ph * pw, 10, True)]
+    P = _params(spec, 7400, True)
+    rng = np.random.default_rng(7401)
+    P[0] = rng.integers(-1, 2, P[0].shape).astype(np.float32)
+    if bias:
+        P[1] = rng.integers(-3, 4, P[1].shape).astype(np.float32)
+    x = rng.integers(-2, 3, (bs, ic, h, w)).astype(np.float32)
+    t = rng.integers(0, 10, bs).astype(np.uint8)
+    model = ag.Model(dev, spec, torch.bfloat16, seed=1)
+    model.set_parameters(P)
+    xh = torch.from_numpy(x).to(torch.bfloat16).pin_memory()
+    logits = model.infer(xh).float().numpy()
+    assert _rel(logits, models.forward(spec, P, x, acc="f64", bf16=True)) <= 2 ** -8
+    model.train_step(xh, torch.from_numpy(t).pin_memory(), 0.01)
+    _, grads, _, _ = models.train_step(spec, P, x, t.astype(np.uint32), 0.01, acc="f64", bf16=True)
+    for i, g in enumerate(grads):
+        assert _rel(model.get_gradient(i), g.ravel()) <= 2 ** -6, i
+    model.close()
+
+
 def test_wide_stack_full_batch_properties(dev):
     """Config 3 at its full batch 256: rows are independent, so the first 8 rows of the
     batch-256 forward equal the batch-8 forward."""
