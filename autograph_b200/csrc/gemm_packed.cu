@@ -199,7 +199,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (PL == 3 && threadIdx.x < tcx::kMarks / 4) marks[threadIdx.x] = 0;
-    __syncthreads();
+    // Both CTAs of the pair are here before either allocates: an allocation of a pair needs the other one.  With a
+    // barrier of the CTA alone, and a load of a microsecond before it, one in some hundred launches of 74 pairs left a
+    // CTA without an address (0xffffffe0).
+    cluster_sync();
     // Tensor memory in two 256-column steps; after the first the pair compares addresses (as in
     // gemm_tc2.cu) and stops before anything could block on them if they differ.
     if (warp == 1) tmem_alloc2(smem_u32(&tmem_slot[0]), 256);

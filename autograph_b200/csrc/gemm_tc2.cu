@@ -151,7 +151,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    __syncthreads();
+    // both CTAs are here before either allocates: an allocation of a pair needs the other one (see gemm_packed.cu)
+    cluster_sync();
     // ---- tensor memory, step 1: 256 columns; the pair must agree on the address ----
     if (warp == 1) tmem_alloc2(smem_u32(&tmem_slot[0]), 256);
     tc_fence_before();

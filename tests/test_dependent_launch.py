@@ -30,6 +30,22 @@ def test_tensor_memory_comes_before_dependents():
     assert seen >= 5
 
 
+def test_pairs_meet_before_they_allocate():
+    """Tensor memory of a pair of CTAs is allocated by both: a barrier of the cluster comes before the first allocation,
+    with no barrier of one CTA alone between the two."""
+    seen = 0
+    for path in sorted(CSRC.glob("*.cu")):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for body in re.split(r"\b__global__\b", text)[1:]:
+            alloc = body.split("\n}\n")[0].find("tmem_alloc2(")
+            if alloc < 0:
+                continue
+            seen += 1
+            barriers = re.findall(r"cluster_sync\(\)|__syncthreads\(\)", body[:alloc])
+            assert barriers and barriers[-1] == "cluster_sync()", path.name
+    assert seen == 2
+
+
 @pytest.fixture
 def plain(dev):
     """The device without output guards, whose fills would come between the kernels."""
