@@ -229,6 +229,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_acc[2] = {tmem_slot[0], tmem_slot[1]};
+    // The copy pass, this and the sum of slices each set up while their predecessor ends (us plain and so: f32 1024^3 34.9
+    // and 27.2, 2048^3 92 and 86, 256 x 25088 x 512 78 and 71; bf16 4313 x 791 x 1252 43.1 and 37.7).
+    let_dependents_launch();
+    dependency_wait();
 
     if (warp == 0) {
         if (elect_one()) {
@@ -452,6 +456,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 // C from the f32 sums of the slices, added in slice order.
 template <class T>
 __global__ void __launch_bounds__(256) reduce_kernel(const __grid_constant__ Params<T> p, FastDiv div_m) {
+    let_dependents_launch();
+    dependency_wait();
     const int64_t plane = (int64_t)p.M * p.N;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < plane; i += (int64_t)gridDim.x * 256) {
         float s = 0.f;
@@ -478,6 +484,8 @@ struct PackJob {
 // that a warp makes 128 bytes of, and loads that need no alignment.  DRAM bound.
 template <class T>
 __global__ void __launch_bounds__(256) pack_kernel(const PackJob<T> j0, const PackJob<T> j1) {
+    let_dependents_launch(kAlwaysEarly);
+    dependency_wait();
     const PackJob<T> &j = blockIdx.y == 0 ? j0 : j1;
     const uint32_t words = (uint32_t)j.pitch / 2;
     const uint32_t total = words * (uint32_t)j.outer;
@@ -530,8 +538,7 @@ static int launch(ag_device *dev, const CUtensorMap &ta, const CUtensorMap &tb, 
         const int left = p.num_work - p.work0, n = left < most ? left : most;
         p.work1 = p.work0 + n;
         const int pairs = n < dev->sm_count / 2 ? n : dev->sm_count / 2;
-        kernel<<<2 * pairs, THREADS, Cfg<PL>::SMEM, dev->stream>>>(ta, tb, tt, p);
-        AG_CHECK_LAUNCH();
+        AG_TRY(launch_dependent(dev, kernel, dim3(2 * pairs), THREADS, Cfg<PL>::SMEM, ta, tb, tt, p));
     }
     return AG_OK;
 }
@@ -643,8 +650,7 @@ int gemm(ag_device *dev, int M, int N, int K, const T *p, int64_t p_row, int64_t
     if (a.splits > 1) a.partial = (float *)((char *)ws + a_bytes + b_bytes);
 
     const int64_t blocks = ceil_div(words, 1024), cap = (int64_t)dev->sm_count * 8;
-    pack_kernel<T><<<dim3((unsigned)(blocks < cap ? blocks : cap), 2), 256, 0, dev->stream>>>(ja, jb);
-    AG_CHECK_LAUNCH();
+    AG_TRY(launch_dependent(dev, pack_kernel<T>, dim3((unsigned)(blocks < cap ? blocks : cap), 2), 256, 0, ja, jb));
 
     CUtensorMap ta, tb, tt;
     AG_TRY(packed_map(&ta, ja.dst, ja.inner, ja.outer, ja.pitch, PL, a_mn ? 64 : 128));
@@ -660,8 +666,7 @@ int gemm(ag_device *dev, int M, int N, int K, const T *p, int64_t p_row, int64_t
         AG_TRY((launch<PL, false, false>(dev, ta, tb, tt, a)));
     if (a.splits > 1) {
         const int64_t n = ceil_div((int64_t)M * N, 256);
-        reduce_kernel<T><<<(unsigned)(n < cap ? n : cap), 256, 0, dev->stream>>>(a, FastDiv((uint32_t)M));
-        AG_CHECK_LAUNCH();
+        AG_TRY(launch_dependent(dev, reduce_kernel<T>, dim3((unsigned)(n < cap ? n : cap)), 256, 0, a, FastDiv((uint32_t)M)));
     }
     return AG_OK;
 }

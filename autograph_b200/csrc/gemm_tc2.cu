@@ -185,6 +185,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_acc[2] = {tmem_slot[0], tmem_slot[1]};
+    // Set up, tensor memory and all, while the predecessor ends (products in a row, us plain and so: 1024^3 12.3 and 8.8,
+    // 2048^3 20.5 and 17.8, 4096^3 86.6 and 85.4; 1264 x 3008 x 304 16.5 and 14.1).
+    let_dependents_launch();
+    dependency_wait();
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer (both CTAs)
@@ -479,13 +483,9 @@ static int launch_pair(ag_device *dev, const CUtensorMap &ta, const CUtensorMap 
                                          pair::SMEM_BYTES));
         if (dev->ordinal < 64) attr_done[dev->ordinal] = true;
     }
-    const int tiles = (int)(ceil_div(p.M, pair::TILE_M) * ceil_div(p.N, pair::TILE_N));
-    (void)tiles;
     int pairs = dev->sm_count / 2;
     if (p.num_work < pairs) pairs = p.num_work;
-    kernel<<<2 * pairs, pair::NUM_THREADS, pair::SMEM_BYTES, dev->stream>>>(ta, tb, tb_tail, p);
-    AG_CHECK_LAUNCH();
-    return AG_OK;
+    return launch_dependent(dev, kernel, dim3(2 * pairs), pair::NUM_THREADS, pair::SMEM_BYTES, ta, tb, tb_tail, p);
 }
 
 bool gemm_bf16_pair_enabled() {

@@ -21,13 +21,13 @@ def test_tensor_memory_comes_before_dependents():
     seen = 0
     for file, name, body in _kernels():
         trigger = re.search(r"let_dependents_launch\(|griddepcontrol\.launch_dependents", body)
-        alloc = body.find("tmem_alloc(")
+        alloc = max(body.find("tmem_alloc("), body.rfind("tmem_alloc2("))
         if trigger is None or alloc < 0:
             continue
         seen += 1
         assert alloc < trigger.start(), f"{file}: {name} lets dependents launch before it allocates tensor memory"
         assert "__syncthreads()" in body[alloc:trigger.start()], f"{file}: {name}: no barrier between the two"
-    assert seen >= 5
+    assert seen >= 9
 
 
 def test_pairs_meet_before_they_allocate():
