@@ -67,15 +67,16 @@ static int dense_forward_simt(ag_device *dev, const T *x, int bs, int inputs, co
 using namespace ag;
 
 // Aligned bf16 products that the TMA kernels are better at than the gathered engine, whose k slices and smaller tiles fill
-// the chip where those have a handful of tiles.  m x k x n, us with TMA and gathered: 160 x 416 x 432 12.4 and 8.2, 208 x
-// 1328 x 144 16.6 and 8.6, 1408 x 608 x 192 12.4 and 9.6, 176 x 560 x 1648 12.4 and 8.8, 6928 x 64 x 432 10.4 and 12.7, 384 x
-// 2864 x 336 16.5 and 11.4, 176 x 3680 x 1088 26 and 16, 960 x 224 x 2608 11.0 and 19.2, 496 x 4832 x 416 20.8 and 21.3.
-// Over 320 drawn products of 4e7 to 3e9 multiply-adds these lines are 0.6 % above always taking the faster one.
+// the chip where those have a handful of tiles.  m x k x n, us with TMA and gathered: 352 x 1328 x 256 13.4 and 8.7, 176 x
+// 480 x 848 10.2 and 7.5, 2640 x 192 x 160 8.0 and 6.8, 1200 x 256 x 432 6.1 and 8.2, 656 x 208 x 1328 6.5 and 7.4, 912 x
+// 320 x 464 6.6 and 9.2; few tiles with a long k 192 x 3760 x 496 16.8 and 11.1, 240 x 1456 x 560 15.8 and 10.6, 336 x
+// 1216 x 1408 9.6 and 16.7, 176 x 8128 x 624 16.0 and 21.5, 720 x 4528 x 272 15.9 and 23.7.  Over 160 drawn products of
+// 5e6 to 2e9 multiply-adds these lines are 0.9 % above always taking the faster one.
 static bool tma_worth(int64_t m, int64_t k, int64_t n) {
     const double macs = (double)m * (double)n * (double)k;
     if (!tcx::gemm_worth(AG_BF16, m, k, n)) return true;
-    if (k >= 1024 && ag::ceil_div(m, 128) * ag::ceil_div(n, 128) <= 32) return macs >= 1e9;
-    return macs >= (k < 160 ? 1.5e8 : 2.5e8);
+    if (k >= 1024 && ag::ceil_div(m, 128) * ag::ceil_div(n, 128) <= 16) return macs >= 6e8;
+    return macs >= 9e7;
 }
 
 extern "C" int ag_dense_forward(ag_device *dev, ag_dtype dtype, const void *x, int64_t bs,

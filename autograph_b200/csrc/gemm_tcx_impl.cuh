@@ -37,13 +37,16 @@ static int run(ag_device *dev, int M, int N, int K, const T *p, int64_t p_row, i
 }
 
 template <class T>
+constexpr ag_dtype kDtype = sizeof(T) == 4 ? AG_F32 : AG_BF16;
+
+template <class T>
 int gemm_strided(ag_device *dev, int m, int k, int n, float alpha, const T *a, int64_t rsa,
                  int64_t csa, const T *b, int64_t rsb, int64_t csb, float beta, T *c, int64_t rsc,
                  int64_t csc) {
     // A warp of the epilogue writes 32 consecutive tile rows: they run along C's contiguous index,
     // so a row-major C is computed as C^T = B^T . A^T.
     const bool a_ok = rsa == 1 || csa == 1, b_ok = rsb == 1 || csb == 1;
-    if (a_ok && b_ok && packed_worth(m, k, n)) {
+    if (a_ok && b_ok && packed_worth(kDtype<T>, m, k, n)) {
         if (csc == 1 && packed::reserve<T>(dev, n, m, k, rsb, csa))
             return packed::gemm<T>(dev, n, m, k, b, csb, rsb, a, rsa, csa, alpha, beta, c, rsc, nullptr, false);
         if (csc != 1 && rsc == 1 && packed::reserve<T>(dev, m, n, k, csa, rsb))
@@ -57,7 +60,7 @@ int gemm_strided(ag_device *dev, int m, int k, int n, float alpha, const T *a, i
 template <class T>
 int dense(ag_device *dev, const T *x, int bs, int inputs, const T *w, int outputs, const T *bias,
           bool relu, T *y) {
-    if (packed_worth(bs, inputs, outputs) && packed::reserve<T>(dev, outputs, bs, inputs, outputs, 1))
+    if (packed_worth(kDtype<T>, bs, inputs, outputs) && packed::reserve<T>(dev, outputs, bs, inputs, outputs, 1))
         return packed::gemm<T>(dev, outputs, bs, inputs, w, 1, outputs, x, inputs, 1, 1.f, 0.f, y, outputs,
                                bias, relu);
     const DenseOut<T> E{y, outputs, bias, relu};

@@ -12,7 +12,7 @@ namespace tcx {
 bool gemm_worth(ag_dtype dtype, int64_t m, int64_t k, int64_t n);
 
 // True when such a product is large enough to copy its operands into aligned bf16 planes first.
-bool packed_worth(int64_t m, int64_t k, int64_t n);
+bool packed_worth(ag_dtype dtype, int64_t m, int64_t k, int64_t n);
 
 // C = alpha * A.B + beta * C on strided views.
 template <class T>
