@@ -79,6 +79,18 @@ static bool tma_worth(int64_t m, int64_t k, int64_t n) {
     return macs >= 9e7;
 }
 
+// Products a^T . b with few columns (the weight gradient of a layer with few outputs), few_columns against the SIMT tiles,
+// m x k x n, us here and there (replayed): bf16 512 x 256 x 10 5.1 and 10.7, 512 x 100 x 16 3.1 and 5.4, 4096 x 256 x 2 3.5
+// and 27, 128 x 32 x 10 2.4 and 3.2, 128 x 1000 x 10 15.0 and 14.9, 128 x 2000 x 10 28 and 15; f32 512 x 256 x 10 4.7 and 5.9,
+// 4096 x 256 x 10 4.9 and 11.9, 512 x 1000 x 10 13.5 and 7.8.  Beyond a CTA per SM a CTA's 32 columns are too few for what it
+// stages: bf16 25088 x 32 x 10 8.4 and 5.4, x 100 10.8 and 12.8, f32 25088 x 100 x 10 10.0 and 8.4, x 256 x 2 7.4 and 15.
+// f32 with k up to 128 stays: there are fewer roundings in its sums (k = 32: 4.5e-8 and here 6.1e-8 in relative 2-norm; k =
+// 256: 6.9e-8 and 6.1e-8).
+static bool few_columns_worth(ag_dtype dtype, int64_t m, int64_t k, int64_t n, int sms) {
+    if (n > dense_small::kFewColumns || k > 512 || k < (dtype == AG_F32 ? 129 : 32)) return false;
+    return ag::ceil_div(m, 32) <= sms || (dtype == AG_F32 ? n <= 4 : k >= 100);
+}
+
 extern "C" int ag_dense_forward(ag_device *dev, ag_dtype dtype, const void *x, int64_t bs,
                                 int64_t inputs, const void *w, int64_t outputs, const void *bias,
                                 int fuse_relu, void *y) {
@@ -333,6 +345,14 @@ extern "C" int ag_gemm(ag_device *dev, ag_dtype dtype, int64_t m, int64_t k, int
             (int)n, nullptr, false, (__nv_bfloat16 *)c + off_c);
     }
     const bool tensor_core = tcx::gemm_worth(dtype, m, k, n);
+    if (!tensor_core && alpha == 1.f && beta == 0.f && rsa == 1 && csb == 1 && csc == 1 &&
+        few_columns_worth(dtype, m, k, n, dev->sm_count)) {
+        if (dtype == AG_F32)
+            return dense_small::few_columns<float>(dev, (int)m, (int)k, (int)n, (const float *)a + off_a, csa,
+                                                   (const float *)b + off_b, rsb, (float *)c + off_c, rsc);
+        return dense_small::few_columns<__nv_bfloat16>(dev, (int)m, (int)k, (int)n, (const __nv_bfloat16 *)a + off_a, csa,
+                                                       (const __nv_bfloat16 *)b + off_b, rsb, (__nv_bfloat16 *)c + off_c, rsc);
+    }
     if (dtype == AG_F32) {
         if (tensor_core)
             return tcx::gemm_strided<float>(dev, (int)m, (int)k, (int)n, alpha,

@@ -190,3 +190,28 @@ def test_dense_with_few_outputs_gives_the_bits_of_the_chain(dev, dtype, m, k, n)
         chain = dev.dense_chain_forward(x, [w0, w1], [None, bias], [True, relu])
         assert torch.equal(dev.dense_forward(h, w1, bias=bias, relu=relu), chain)
     assert torch.equal(dev.dot(h, w1).clamp(min=0), chain)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m,k,n", [(1, 129, 1), (31, 512, 16), (33, 511, 5), (64, 130, 8), (70, 256, 9), (512, 256, 10),
+                                   (100, 300, 13), (5000, 150, 3), (129, 513, 12)])
+def test_products_with_few_columns(dev, dtype, m, k, n):
+    """a^T . b with up to 16 columns, rows of either operand and of the result further apart than they are long, against
+    float64: the sums' roundings, at most k / 16 + 16 in a row of 2^-24 of the sum of magnitudes each, and bf16's store."""
+    rng = torch.Generator().manual_seed(m * 1000 + k + n)
+    a = torch.empty((k, m + 3)).uniform_(-1, 1, generator=rng).to(dtype).cuda(dev.torch_device)
+    b = torch.empty((k, n + 2)).uniform_(-1, 1, generator=rng).to(dtype).cuda(dev.torch_device)
+    c = torch.full((m, n + 1), 7.0, dtype=dtype, device=dev.torch_device)
+    av, bv, cv = a[:, 1:m + 1], b[:, 2:], c[:, :n]
+    from autograph_b200 import _capi, lib
+    code = _capi.AG_F32 if dtype == torch.float32 else _capi.AG_BF16
+    _capi.check(lib().ag_gemm(dev._h, code, m, k, n, 1.0, av.data_ptr(), 0, 1, m + 3, bv.data_ptr(), 0, n + 2, 1, 0.0,
+                              cv.data_ptr(), 0, n + 1, 1))
+    dev.wait()
+    a64, b64 = av.double(), bv.double()
+    bound = (k / 16 + 16) * 2.0 ** -24 * (a64.abs().t() @ b64.abs())
+    ref = a64.t() @ b64
+    if dtype == torch.bfloat16:
+        bound = bound + 2.0 ** -8 * ref.abs()
+    assert bool(((cv.double() - ref).abs() <= bound).all())
+    assert bool((c[:, n] == 7.0).all())
