@@ -156,7 +156,8 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
         Tensor pooled;
         for (size_t s = 0; s < st.size(); ++s) {
             const StageDesc &d = st[s];
-            Tensor y = make({bs, d.ph, d.pw, d.ocp});
+            const bool to_nchw = pools_to_nchw(s);
+            Tensor y = make(to_nchw ? Shape{bs, d.oc, d.ph, d.pw} : Shape{bs, d.ph, d.pw, d.ocp});
             Tensor codes = keep ? Tensor::uninit(*pool, {bs, d.ph, d.pw, d.ocp / 2}, AG_U8) : Tensor{};
             if (d.image) {
                 check(::ag::image_stage::forward(dev, d.image_shape(bs), cptr(x), cptr(d.conv->weight.value),
@@ -190,8 +191,9 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
             check(::ag::convtc::correlate_nhwc(
                 dev, c, cptr(a), ::ag::convtc::nhwc_wants_frame(c), cptr(wv), d.oc, d.k_ic,
                 d.conv->has_bias ? cptr(d.conv->bias.value) : nullptr, false, ptr(wk), ptr(p)));
-            check(::ag::nhwc::relu_pool(dev, cptr(p), bs, d.oh, d.ow, d.ocp, ptr(y),
-                                        keep ? (uint32_t *)codes.data() : nullptr));
+            uint32_t *code_ptr = keep ? (uint32_t *)codes.data() : nullptr;
+            check(to_nchw ? ::ag::nhwc::relu_pool_nchw(dev, cptr(p), bs, d.oh, d.ow, d.ocp, ptr(y), code_ptr)
+                          : ::ag::nhwc::relu_pool(dev, cptr(p), bs, d.oh, d.ow, d.ocp, ptr(y), code_ptr));
             if (keep) {
                 code.push_back(codes);
                 act.push_back(a);
@@ -201,12 +203,20 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
             pooled = y;
         }
         const StageDesc &l = st.back();
-        Tensor out = make({bs, l.oc, l.ph, l.pw});
-        check(::ag::convtc::from_nhwc(dev, cptr(pooled), bs, l.oc, l.ph * l.pw, l.ocp, ptr(out)));
+        Tensor out = pooled;
+        if (!pools_to_nchw(st.size() - 1)) {
+            out = make({bs, l.oc, l.ph, l.pw});
+            check(::ag::convtc::from_nhwc(dev, cptr(pooled), bs, l.oc, l.ph * l.pw, l.ocp, ptr(out)));
+        }
         dpre.resize(st.size());
         have.assign(st.size(), 0);
         framed.assign(st.size(), 0);
         return out;
+    }
+
+    // The run's output is NCHW: the last stage's pool writes it so, and its gradient is read so (but by an image stage).
+    bool pools_to_nchw(size_t s) const {
+        return s + 1 == st.size() && !st[s].image && st[s].ph * st[s].pw <= ::ag::nhwc::kMostWindows;
     }
 
     bool wants_dx(size_t s) const { return s > 0 || input_grad; }
@@ -239,6 +249,18 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
         if (have[s]) return;
         ::ag::DeviceGuard guard(dev);
         const StageDesc &d = st[s];
+        const bool fr = !d.image && wants_dx(s) && ::ag::convtc::nhwc_wants_frame(backward_conv(d));
+        framed[s] = fr ? 1 : 0;
+        const int fy = fr ? d.k_fh - 1 : 0, fx = fr ? d.k_fw - 1 : 0;
+        const int64_t hp = d.oh + 2 * fy, wp = d.ow + 2 * fx;
+        if (pools_to_nchw(s) && (reinterpret_cast<uintptr_t>(dy_out.data()) & 15) == 0) {
+            dpre[s] = make({bs, hp, wp, d.ocp});
+            check(::ag::nhwc::relu_pool_backward_nchw(dev, pre[s].defined() ? cptr(pre[s]) : nullptr,
+                                                     (const uint32_t *)code[s].data(), cptr(dy_out), bs, d.oh, d.ow, d.ocp, fy,
+                                                     fx, ptr(dpre[s])));
+            have[s] = 1;
+            return;
+        }
         Tensor dpool;
         if (s + 1 == st.size()) {
             dpool = make({bs, d.ph, d.pw, d.ocp});
@@ -253,16 +275,8 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
             have[s] = 1;
             return;
         }
-        const bool fr = wants_dx(s) && ::ag::convtc::nhwc_wants_frame(backward_conv(d));
-        framed[s] = fr ? 1 : 0;
-        if (fr) {
-            const int fy = d.k_fh - 1, fx = d.k_fw - 1;
-            const int64_t hp = d.oh + 2 * fy, wp = d.ow + 2 * fx;
-            dpre[s] = make({bs, hp, wp, d.ocp});
-            check(::ag::nhwc::zero_frame(dev, ptr(dpre[s]), bs, hp, wp, fy, fx, d.ocp));
-        } else {
-            dpre[s] = make({bs, d.oh, d.ow, d.ocp});
-        }
+        dpre[s] = make({bs, hp, wp, d.ocp});
+        if (fr) check(::ag::nhwc::zero_frame(dev, ptr(dpre[s]), bs, hp, wp, fy, fx, d.ocp));
         const View v = interior(s);
         check(::ag::nhwc::relu_pool_backward(dev, pre[s].defined() ? cptr(pre[s]) : nullptr, (const uint32_t *)code[s].data(),
                                             cptr(dpool), bs, d.oh, d.ow, d.ocp, v.p,

@@ -33,6 +33,15 @@ int relu_pool_backward(ag_device *dev, const __nv_bfloat16 *pre, const uint32_t 
                        int64_t ih, int64_t iw, int64_t cp, __nv_bfloat16 *out, int64_t out_row_pitch,
                        int64_t out_image_pitch);
 
+// The same two for the last stage of a run, whose pooled side is NCHW (dense, 16-byte aligned), without a copy between the
+// layouts; the backward one also zeroes a frame of pad_h rows and pad_w columns around the gradient, whose interior `out`
+// points to.  For planes of up to kMostWindows windows and channels in multiples of 64.
+constexpr int64_t kMostWindows = 1024;
+int relu_pool_nchw(ag_device *dev, const __nv_bfloat16 *pre, int64_t bs, int64_t ih, int64_t iw, int64_t c, __nv_bfloat16 *y,
+                   uint32_t *codes);
+int relu_pool_backward_nchw(ag_device *dev, const __nv_bfloat16 *pre, const uint32_t *codes, const __nv_bfloat16 *dy,
+                            int64_t bs, int64_t ih, int64_t iw, int64_t c, int pad_h, int pad_w, __nv_bfloat16 *framed);
+
 // Zeroes the frame of pad_h rows / pad_w columns around the interior of [bs][hp][wp][cp].
 int zero_frame(ag_device *dev, __nv_bfloat16 *framed, int64_t bs, int64_t hp, int64_t wp, int pad_h,
                int pad_w, int64_t cp);
