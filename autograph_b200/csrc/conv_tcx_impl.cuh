@@ -32,6 +32,115 @@ static ConvMap conv_map(int64_t channels, int64_t sh, int64_t sw, int64_t gh, in
     return g;
 }
 
+// Eight values as pieces of the planes, `plane` pieces apart.
+__device__ __forceinline__ void store_pieces(const Vec8<float> &x, uint4 *dst, int64_t plane) {
+    uint32_t h[4], m[4], l[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        uint32_t hb[2], mb[2], lb[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) split3(x.v[2 * e + u], hb[u], mb[u], lb[u]);
+        h[e] = upper_halves(hb[0], hb[1]);
+        m[e] = upper_halves(mb[0], mb[1]);
+        l[e] = upper_halves(lb[0], lb[1]);
+    }
+    dst[0] = make_uint4(h[0], h[1], h[2], h[3]);
+    dst[plane] = make_uint4(m[0], m[1], m[2], m[3]);
+    dst[2 * plane] = make_uint4(l[0], l[1], l[2], l[3]);
+}
+__device__ __forceinline__ void store_pieces(const Vec8<__nv_bfloat16> &x, uint4 *dst, int64_t) {
+    dst[0] = make_uint4(__byte_perm(x.v[0], x.v[1], 0x5410), __byte_perm(x.v[2], x.v[3], 0x5410),
+                        __byte_perm(x.v[4], x.v[5], 0x5410), __byte_perm(x.v[6], x.v[7], 0x5410));
+}
+
+// src[outer][channel * s_c][inner] into pieces of eight channels: a tensor [image][channels][hw] (inner = hw, s_c = hw) into
+// [image][hw][groups], or a filter bank (rows, channels, taps) into [row][tap][groups].  A thread makes one piece; a warp
+// reads neighbouring inner indices, which are whole lines of a tensor.
+template <class T>
+struct SplitJob {
+    const T *src;
+    uint4 *dst;
+    int64_t plane;           // pieces per plane
+    int64_t s_outer;
+    int channels, inner, s_c, groups;
+    uint32_t total;          // outer x groups x inner
+    FastDiv div_inner, div_groups;
+};
+template <class T>
+__global__ void __launch_bounds__(256) split_kernel(const SplitJob<T> j0, const SplitJob<T> j1) {
+    let_dependents_launch(kAlwaysEarly);
+    dependency_wait();
+    const SplitJob<T> &j = blockIdx.y == 0 ? j0 : j1;
+    for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < j.total; i += gridDim.x * 256u) {
+        uint32_t t, in, outer, group;
+        j.div_inner.divmod(i, t, in);
+        j.div_groups.divmod(t, outer, group);
+        const int c0 = (int)group * 8;
+        const T *q = j.src + outer * j.s_outer + (int64_t)c0 * j.s_c + in;
+        Vec8<T> x;
+#pragma unroll
+        for (int e = 0; e < 8; ++e, q += j.s_c) fetch(x.v[e], q, c0 + e < j.channels);
+        store_pieces(x, j.dst + ((int64_t)outer * j.inner + in) * j.groups + group, j.plane);
+    }
+}
+
+template <class T>
+static SplitJob<T> split_job(const T *src, int64_t outer, int64_t s_outer, int64_t channels, int64_t s_c, int64_t inner) {
+    SplitJob<T> j;
+    j.src = src;
+    j.dst = nullptr;
+    j.s_outer = s_outer;
+    j.channels = (int)channels;
+    j.inner = (int)inner;
+    j.s_c = (int)s_c;
+    j.groups = (int)ceil_div(channels, 8);
+    j.plane = outer * inner * j.groups;
+    j.total = (uint32_t)j.plane;
+    j.div_inner = FastDiv((uint32_t)inner);
+    j.div_groups = FastDiv((uint32_t)j.groups);
+    return j;
+}
+template <class T>
+static int64_t split_bytes(const SplitJob<T> &j) { return j.plane * Planes<T>::N * 16; }
+
+// Both tensors, to scratch; false without room for it.
+template <class T>
+static bool split_scratch(ag_device *dev, SplitJob<T> *a, SplitJob<T> *b) {
+    void *ws = nullptr;
+    if (staging(dev, (size_t)(split_bytes(*a) + split_bytes(*b)), &ws) != AG_OK) return false;
+    a->dst = (uint4 *)ws;
+    b->dst = (uint4 *)((char *)ws + split_bytes(*a));
+    return true;
+}
+template <class T>
+static int launch_split(ag_device *dev, const SplitJob<T> &a, const SplitJob<T> &b) {
+    const int64_t blocks = ceil_div(a.total > b.total ? a.total : b.total, 256), cap = (int64_t)dev->sm_count * 16;
+    return launch_dependent(dev, split_kernel<T>, dim3((unsigned)(blocks < cap ? blocks : cap), 2), 256, 0, a, b);
+}
+
+// Whether tensors are split once, ahead of the product of `positions` rows, the map's patches and n columns (the weight
+// gradient's likewise).  Against gathering, us split and gathered, images x channels x side -> filters: f32 forward 172 x
+// 32 x 16 -> 128 5x5 58 and 81, 16 x 64 x 37 -> 128 3x3 46 and 61, 52 x 32 x 37 -> 6 3x3 29 and 33, weight gradient 46 x 32 x
+// 27 -> 96 5x5 59 and 80, input gradient 34 x 16 x 47 -> 128 5x5 186 and 276; bf16 forward 48 x 16 x 47 -> 128 5x5 / 2 25 and
+// 42, weight gradient 171 x 64 x 42 -> 16 3x3 148 and 176, input gradient 34 x 16 x 47 -> 128 5x5 117 and 187.  The pass and
+// its launch want a long patch and some work: f32 64 x 16 x 32 -> 32 3x3 (144 values) forward 27 and 24, 13 x 6 x 39 -> 32
+// 16 and 12, 11 x 32 x 40 -> 6 3x3 14 and 12, input gradient 5 x 32 x 42 -> 96 20.7 and 18.3; the weight gradient's second
+// tensor wants more of it (37 x 6 x 52 -> 128 5x5, 200 values, 119 and 89).  Planes beyond what stays in L2 are read again
+// per tap from memory: f32 171 x 64 x 42 -> 16 (116 MB) 237 and 211.  Over 70 drawn convolutions the affected passes take
+// 0.94 (f32 forward), 0.94, 0.86 and (bf16) 0.93, 0.97, 0.87 of their time.
+template <class T>
+static bool split_worth(const ConvMap &g, int64_t bytes, int64_t positions, int64_t n, int least_patch) {
+    const int64_t patch = (int64_t)g.ff * g.cp;
+    return patch >= least_patch && bytes <= 80000000 && positions * patch * (n < 32 ? 32 : n) >= 300000000;
+}
+
+// The map that counts positions instead of elements.
+static ConvMap of_positions(const ConvMap &g) {
+    ConvMap p = g;
+    p.channels = 1;
+    return p;
+}
+
 // A filter bank in the order of ConvRows' k: out[row][tap * cp + c] = w[row * s_row + c * s_c + tap],
 // zero for the padding channels.  Without it every 64-k step of every tile would fetch filters at a
 // stride of the tap count, one sector per element.
@@ -51,9 +160,17 @@ __global__ void repack_kernel(const T *w, T *out, int total, int channels, int c
 // A product with the patch matrix of `map` (rows = positions, k = taps x channels) and the filter
 // bank w[row * s_row + channel * s_c + tap].
 template <class T>
-static int patches_times_filters(ag_device *dev, const T *src, const ConvMap &map, int M, const T *w, int N,
+static int patches_times_filters(ag_device *dev, const T *src, int64_t images, const ConvMap &map, int M, const T *w, int N,
                                  int s_row, int s_c, const NchwOut<T> &E) {
     const int K = map.ff * map.cp, total = N * K;
+    const int64_t hw = (int64_t)map.sh * map.sw;
+    SplitJob<T> x = split_job(src, images, map.channels * hw, (int64_t)map.channels, hw, hw);
+    SplitJob<T> f = split_job(w, (int64_t)N, (int64_t)s_row, (int64_t)map.channels, (int64_t)s_c, (int64_t)map.ff);
+    if (split_worth<T>(map, split_bytes(x), M, N, 200) && split_scratch(dev, &x, &f)) {
+        AG_TRY(launch_split<T>(dev, x, f));
+        return gemm<T>(dev, M, N, K, SplitRows<T>{{x.dst, x.plane}, of_positions(map), x.div_groups, x.groups, {src, map, M}},
+                       SplitFilters<T>{{f.dst, f.plane}, K / 8, {w, s_row, s_c, map.channels, map.div_cp}}, E);
+    }
     // One wave of tiles and up to 18 k steps of an input gradient, whose neighbouring rows are neighbouring
     // filters: read in place at the copy's device time, without its launch (forward, 5 x 64 x 22 x 22 -> 128:
     // 27 us in place, 19 copied; input gradient 21.7 and 21.5; 50 steps of 128 channels 5x5 190 and 87).
@@ -88,7 +205,7 @@ int conv_forward(ag_device *dev, const T *x, int64_t bs, int64_t ic, int64_t ih,
         const int patch = (int)ic * ff;
         return gemm<T>(dev, M, N, patch, FewRows<T>{x, map, M, patch}, strided<kByRow>(w, patch, 1, N), E);
     }
-    return patches_times_filters<T>(dev, x, map, M, w, N, (int)ic * ff, ff, E);
+    return patches_times_filters<T>(dev, x, bs, map, M, w, N, (int)ic * ff, ff, E);
 }
 
 constexpr int64_t kTapSums = 1ll << 28;   // f32 values
@@ -161,7 +278,7 @@ int conv_backward_input(ag_device *dev, const T *w, int64_t oc, int64_t ic, cons
         return AG_OK;
     }
     NchwOut<T> E{dx, nullptr, N, (int)(ih * iw), FastDiv((uint32_t)(ih * iw)), false};
-    return patches_times_filters<T>(dev, dy, map, M, w, N, ff, (int)ic * ff, E);
+    return patches_times_filters<T>(dev, dy, bs, map, M, w, N, ff, (int)ic * ff, E);
 }
 
 template <class T>
@@ -176,6 +293,14 @@ int conv_backward_weight(ag_device *dev, const T *x, int64_t bs, int64_t ic, int
                        StridedOut<T>{dw, 1, patch, 1.f, beta});
     }
     const int M = map.ff * map.cp;
+    SplitJob<T> jx = split_job(x, bs, ic * ih * iw, ic, ih * iw, ih * iw);
+    SplitJob<T> jy = split_job(dy, bs, oc * hw, oc, (int64_t)hw, (int64_t)hw);
+    if (split_worth<T>(map, split_bytes(jx) + split_bytes(jy), K, N, 288) && split_scratch(dev, &jx, &jy)) {
+        AG_TRY(launch_split<T>(dev, jx, jy));
+        return gemm<T>(dev, M, N, K, SplitCols<T>{{jx.dst, jx.plane}, of_positions(map), jx.div_groups, jx.groups, {x, map, M}},
+                       SplitChannels<T>{{jy.dst, jy.plane}, jy.groups, {dy, N, hw, FastDiv((uint32_t)hw)}},
+                       FilterOut<T>{dw, map.channels, map.ff, map.div_cp, map.cp, beta});
+    }
     return gemm<T>(dev, M, N, K, ConvCols<T>{x, map, M}, ChannelRows<T>{dy, N, hw, FastDiv((uint32_t)hw)},
                    FilterOut<T>{dw, map.channels, map.ff, map.div_cp, map.cp, beta});
 }

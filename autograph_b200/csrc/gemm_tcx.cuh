@@ -32,6 +32,8 @@
 // memory each, about 2600 cycles; the producers convert 16 k elements in the same time.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "tc_ptx.cuh"
 
@@ -143,7 +145,11 @@ enum Walk {
               // 32 neighbouring rows; K-major tile
     kByK,     // contiguous along k, no alignment: a thread keeps one k and fetches 8 rows one by one,
               // a warp 32 neighbouring k; MN-major tile
+    kPiecesByRow,   // pieces of 16 bytes along k: as kVecK, with a state per row
+    kPiecesByK,     // pieces of 16 bytes along the rows: eight threads a k (64 rows), MN-major tile
 };
+constexpr bool by_rows(Walk w) { return w == kByRow || w == kPiecesByRow; }   // states belong to rows
+constexpr bool mn_major(Walk w) { return w == kByK || w == kPiecesByK; }
 // Concept:
 //   static constexpr Walk kWalk
 //   static constexpr int kTable      ints of shared memory prepared by init()
@@ -506,6 +512,113 @@ struct ChannelRows {
     }
 };
 
+// The same on tensors that have been split once, [plane][image][position][cp] bf16 with the channels padded to eight (zeros):
+// eight channels of a position are one 16-byte piece per plane, which cp.async brings to the tile, where the forms above
+// fetch eight times and split again for every tap that meets the position.
+//   int piece(State &, table, row, k, k_end)   index of the piece at (row, k), or -1 for zeros
+// `from` is the form it stands for, which an output that is not finite is computed with.
+constexpr bool in_pieces(Walk w) { return w == kPiecesByRow || w == kPiecesByK; }
+struct Pieces {
+    const uint4 *p;
+    int64_t plane;                       // pieces per plane
+};
+template <class T>
+struct SplitRows {                       // as ConvRows
+    static constexpr Walk kWalk = kPiecesByRow;
+    static constexpr int kTable = 32;
+    Pieces src;
+    ConvMap g;                           // of one channel: bases and offsets count positions
+    FastDiv div_groups;
+    int groups;                          // of eight channels
+    ConvRows<T> from;
+    struct State {
+        int base;
+        uint32_t mask;
+    };
+    __device__ __forceinline__ void init(int *table, int tid, int threads) const {
+        for (int t = tid; t < g.ff; t += threads) table[t] = g.tap_offset(t);
+    }
+    __device__ __forceinline__ void begin(State &s, const int *, int row, int end) const {
+        s.base = 0;
+        s.mask = 0;
+        if (row < end) g.position(row, s.base, s.mask);
+    }
+    __device__ __forceinline__ int piece(const State &s, const int *table, int, int k, int k_end) const {
+        uint32_t tap, c;
+        div_groups.divmod((uint32_t)k / 8, tap, c);
+        return k < k_end && ((s.mask >> tap) & 1u) ? (s.base + table[tap]) * groups + (int)c : -1;
+    }
+    __device__ __forceinline__ float at(int row, int k) const { return from.at(row, k); }
+};
+template <class T>
+struct SplitCols {                       // as ConvCols
+    static constexpr Walk kWalk = kPiecesByK;
+    static constexpr int kTable = 32;
+    Pieces src;
+    ConvMap g;
+    FastDiv div_groups;
+    int groups;
+    ConvCols<T> from;
+    struct State {
+        int base;
+        uint32_t mask;
+    };
+    __device__ __forceinline__ void init(int *table, int tid, int threads) const {
+        for (int t = tid; t < g.ff; t += threads) table[t] = g.tap_offset(t);
+    }
+    __device__ __forceinline__ void begin(State &s, const int *, int k, int end) const {
+        s.base = 0;
+        s.mask = 0;
+        if (k < end) g.position(k, s.base, s.mask);
+    }
+    __device__ __forceinline__ int piece(const State &s, const int *table, int row, int, int) const {
+        uint32_t tap, c;
+        div_groups.divmod((uint32_t)row / 8, tap, c);
+        return (s.mask >> tap) & 1u ? (s.base + table[tap]) * groups + (int)c : -1;
+    }
+    __device__ __forceinline__ float at(int row, int k) const { return from.at(row, k); }
+};
+template <class T>
+struct SplitChannels {                   // as ChannelRows
+    static constexpr Walk kWalk = kPiecesByK;
+    static constexpr int kTable = 0;
+    Pieces src;
+    int groups;
+    ChannelRows<T> from;
+    struct State { int base; };
+    __device__ __forceinline__ void init(int *, int, int) const {}
+    __device__ __forceinline__ void begin(State &s, const int *, int k, int end) const { s.base = k < end ? k * groups : -1; }
+    __device__ __forceinline__ int piece(const State &s, const int *, int row, int, int) const {
+        return s.base < 0 ? -1 : s.base + row / 8;
+    }
+    __device__ __forceinline__ float at(int row, int k) const { return from.at(row, k); }
+};
+template <class T>
+struct SplitFilters {                    // as FilterRows: [plane][row][(tap, padded channel)]
+    static constexpr Walk kWalk = kPiecesByRow;
+    static constexpr int kTable = 0;
+    Pieces src;
+    int pitch;                           // pieces per row
+    FilterRows<T> from;
+    struct State { int base; };
+    __device__ __forceinline__ void init(int *, int, int) const {}
+    __device__ __forceinline__ void begin(State &s, const int *, int row, int) const { s.base = row * pitch; }
+    __device__ __forceinline__ int piece(const State &s, const int *, int, int k, int k_end) const {
+        return k < k_end ? s.base + k / 8 : -1;
+    }
+    __device__ __forceinline__ float at(int row, int k) const { return from.at(row, k); }
+};
+
+// 16 bytes of global memory, or zeros, to shared memory, asynchronously.
+__device__ __forceinline__ void copy_piece(uint32_t dst, const uint4 *src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+template <int PL>
+__device__ __forceinline__ void copy_pieces(uint32_t dst, uint32_t plane_bytes, const Pieces &src, int at) {
+#pragma unroll
+    for (int i = 0; i < PL; ++i) copy_piece(dst + i * plane_bytes, src.p + (at < 0 ? 0 : i * src.plane + at), at >= 0);
+}
+
 // ---------------------------------------------------------------- epilogues
 // Concept: State begin(int row, int col); void store(State &, int col, float acc), which stores at the
 // state's position and moves it to the next column: with a 64-bit address per element from
@@ -642,27 +755,37 @@ struct Params {
 // the 128-byte swizzle.
 template <Walk WALK, int R, int PRODUCERS>
 struct Slots {
-    int a, b;      // kByRow: row, chunk; kVecK: row, chunk; kByK: k, group of 8 rows
+    static constexpr bool kEight = WALK == kVecK || WALK == kPiecesByRow || WALK == kPiecesByK;   // eight threads a row or k
+    static constexpr int kAtoms = R >= 64 ? R / 64 : 1;
+    // States of an operand that a thread walks with, and the one of its i-th chunk.
+    static constexpr int kChunks = R * 8 / PRODUCERS < 1 ? 1 : R * 8 / PRODUCERS;
+    static constexpr int kStates = WALK == kPiecesByRow ? kChunks : WALK == kPiecesByK ? (kChunks + kAtoms - 1) / kAtoms : 1;
+    static constexpr __device__ __forceinline__ int state(int i) {
+        return WALK == kPiecesByRow ? i : WALK == kPiecesByK ? i / kAtoms : 0;
+    }
+    int a, b;      // kByRow: row, chunk; kVecK, kPiecesByRow: row, chunk; kByK, kPiecesByK: k, group of 8 rows
     bool mine;
     __device__ __forceinline__ explicit Slots(int tid) {
-        a = WALK == kByRow ? (tid & (R - 1)) : WALK == kVecK ? (tid >> 3) : (tid & 63);
-        b = WALK == kByRow ? tid / R : WALK == kVecK ? (tid & 7) : (tid >> 6);
+        a = WALK == kByRow ? (tid & (R - 1)) : kEight ? (tid >> 3) : (tid & 63);
+        b = WALK == kByRow ? tid / R : kEight ? (tid & 7) : (tid >> 6);
         // One value per warp, and known to be: what follows from it (tap, channel, the table's entry,
         // the bounds) is computed once per warp.  With 256 producers, who hold four chunks of each operand,
         // the same costs spills (9 x 64 x 44 x 44 -> 128 5x5 f32 72 -> 83 us).
-        if (WALK != kVecK && PRODUCERS > 256) b = __shfl_sync(0xffffffffu, b, 0);
+        if (!kEight && PRODUCERS > 256) b = __shfl_sync(0xffffffffu, b, 0);
         mine = R * 8 >= PRODUCERS || tid < R * 8;
     }
     __device__ __forceinline__ int row(int i) const {
-        return WALK == kByRow ? a : WALK == kVecK ? a + i * (PRODUCERS / 8) : (b + i * (PRODUCERS / 64)) * 8;
+        return WALK == kByRow ? a : WALK == kPiecesByK ? (b + i % kAtoms * 8) * 8
+             : WALK == kByK ? (b + i * (PRODUCERS / 64)) * 8 : a + i * (PRODUCERS / 8);
     }
     __device__ __forceinline__ int k(int i) const {
-        return WALK == kByRow ? (b + i * (PRODUCERS / R)) * 8 : WALK == kVecK ? b * 8 : a;
+        return WALK == kByRow ? (b + i * (PRODUCERS / R)) * 8 : WALK == kPiecesByK ? a + i / kAtoms * (PRODUCERS / 8)
+             : WALK == kByK ? a : b * 8;
     }
     __device__ __forceinline__ uint32_t offset(int i) const {
-        if (WALK == kByK) {
-            const int g = b + i * (PRODUCERS / 64);
-            return (g >> 3) * 8192 + a * 128 + (((g & 7) ^ (a & 7)) << 4);
+        if (mn_major(WALK)) {
+            const int g = row(i) >> 3, kk = k(i);
+            return (g >> 3) * 8192 + kk * 128 + (((g & 7) ^ (kk & 7)) << 4);
         }
         const int r = row(i), ch = k(i) >> 3;
         return r * ROW_BYTES + ((ch ^ (r & 7)) << 4);
@@ -774,7 +897,7 @@ __device__ __noinline__ void redo_marked(const AOp &A, const BOp &B, const Epi &
             const int col0 = (tile / p.tiles_m) * C::BN + e / 4 * C::COLS + block / C::EPI_WARPS * 32;
             if ((mark >> e & 1u) == 0 || row0 >= p.M || col0 >= p.N || turn++ % WARPS != warp) continue;
             float acc[4][8];
-            redo_block<AOp::kWalk == kByRow, BOp::kWalk == kByRow>(A, B, row0, p.M, col0, p.N, k_begin, k_end, buf, acc);
+            redo_block<by_rows(AOp::kWalk), by_rows(BOp::kWalk)>(A, B, row0, p.M, col0, p.N, k_begin, k_end, buf, acc);
             const int row = row0 + lane / 4 * 4, col = col0 + lane % 4 * 8;
             for (int r = 0; r < 4; ++r) {
                 if (row + r >= p.M || col >= p.N) break;
@@ -866,30 +989,84 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
         constexpr int B_PER = BN * 8 / PRODUCERS < 1 ? 1 : BN * 8 / PRODUCERS;
         int stage = 0;
         uint32_t phase = 0;
+        int in_flight = 0, oldest = 0;   // pieces: steps whose copies are under way, and the stage of the first
+        const auto hand_over = [&](auto left) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(decltype(left)::value) : "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(tc::smem_u32(&full_bar[oldest]));
+            if (++oldest == STAGES) oldest = 0;
+        };
         for (int w = work0; w < num_work; w += gridDim.x) {
             const int tile = w % tiles, z = w / tiles;
             const int m0 = (tile % p.tiles_m) * BM, n0 = (tile / p.tiles_m) * BN;
             const int k_begin = z * p.k_split, k_end = min(p.K, k_begin + p.k_split);
-            const Slots<AOp::kWalk, BM, PRODUCERS> la(tid);
-            const Slots<BOp::kWalk, BN, PRODUCERS> lb(tid);
-            typename AOp::State sa;
-            typename BOp::State sb;
-            if (AOp::kWalk == kByRow) A.begin(sa, table_a, m0 + la.row(0), p.M);
-            if (BOp::kWalk == kByRow) B.begin(sb, table_b, n0 + lb.row(0), p.N);
+            using LA = Slots<AOp::kWalk, BM, PRODUCERS>;
+            using LB = Slots<BOp::kWalk, BN, PRODUCERS>;
+            const LA la(tid);
+            const LB lb(tid);
+            typename AOp::State sa[LA::kStates];
+            typename BOp::State sb[LB::kStates];
+#pragma unroll
+            for (int i = 0; i < LA::kStates; ++i)
+                if (by_rows(AOp::kWalk)) A.begin(sa[i], table_a, m0 + la.row(i), p.M);
+#pragma unroll
+            for (int i = 0; i < LB::kStates; ++i)
+                if (by_rows(BOp::kWalk)) B.begin(sb[i], table_b, n0 + lb.row(i), p.N);
             bool ok = true;
+            if constexpr (in_pieces(AOp::kWalk) && in_pieces(BOp::kWalk)) {
+                // A step is handed over when the copies of up to STAGES - 2 after it are under way, so that the tensor
+                // cores have one while the next is waited for.
+                constexpr int kAhead = STAGES > 2 ? STAGES - 2 : 0;
+                for (int k0 = k_begin; k0 < k_end; k0 += BK) {
+                    const int k_stop = k0 + BK <= k_end ? BK : (k_end - k0 + 15) & ~15;
+                    if (!tc::mbar_wait(tc::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag)) {
+                        if (lane == 0) atomicExch(p.status, 181);
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t a_base = tc::smem_u32(smem + stage * C::STAGE);
+                    const uint32_t b_base = a_base + PL * C::A_PLANE;
+#pragma unroll
+                    for (int i = 0; i < LA::kStates; ++i)
+                        if (mn_major(AOp::kWalk)) A.begin(sa[i], table_a, k0 + la.k(i * LA::kAtoms), k_end);
+#pragma unroll
+                    for (int i = 0; i < A_PER; ++i)
+                        if (m0 + la.row(i) < p.M && la.k(i) < k_stop)
+                            copy_pieces<PL>(a_base + la.offset(i), C::A_PLANE, A.src,
+                                            A.piece(sa[LA::state(i)], table_a, m0 + la.row(i), k0 + la.k(i), k_end));
+#pragma unroll
+                    for (int i = 0; i < LB::kStates; ++i)
+                        if (mn_major(BOp::kWalk)) B.begin(sb[i], table_b, k0 + lb.k(i * LB::kAtoms), k_end);
+#pragma unroll
+                    for (int i = 0; i < B_PER; ++i)
+                        if (lb.mine && n0 + lb.row(i) < p.N && lb.k(i) < k_stop)
+                            copy_pieces<PL>(b_base + lb.offset(i), C::B_PLANE, B.src,
+                                            B.piece(sb[LB::state(i)], table_b, n0 + lb.row(i), k0 + lb.k(i), k_end));
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+                    if (++in_flight > kAhead) {
+                        --in_flight;
+                        hand_over(std::integral_constant<int, kAhead>());
+                    }
+                    if (++stage == STAGES) {
+                        stage = 0;
+                        phase ^= 1;
+                    }
+                }
+            } else {
             for (int k0 = k_begin; k0 < k_end; k0 += BK) {
                 Vec8<T> va[A_PER], vb[B_PER];
                 const int k_stop = k0 + BK <= k_end ? BK : (k_end - k0 + 15) & ~15;   // what the MMAs will read
-                if (AOp::kWalk == kByK) A.begin(sa, table_a, k0 + la.k(0), k_end);
+                if (AOp::kWalk == kByK) A.begin(sa[0], table_a, k0 + la.k(0), k_end);
 #pragma unroll
                 for (int i = 0; i < A_PER; ++i)
                     if (m0 + la.row(i) < p.M && la.k(i) < k_stop)
-                        A.load(sa, table_a, m0 + la.row(i), k0 + la.k(i), k_end, va[i]);
-                if (BOp::kWalk == kByK) B.begin(sb, table_b, k0 + lb.k(0), k_end);
+                        A.load(sa[0], table_a, m0 + la.row(i), k0 + la.k(i), k_end, va[i]);
+                if (BOp::kWalk == kByK) B.begin(sb[0], table_b, k0 + lb.k(0), k_end);
 #pragma unroll
                 for (int i = 0; i < B_PER; ++i)
                     if (lb.mine && n0 + lb.row(i) < p.N && lb.k(i) < k_stop)
-                        B.load(sb, table_b, n0 + lb.row(i), k0 + lb.k(i), k_end, vb[i]);
+                        B.load(sb[0], table_b, n0 + lb.row(i), k0 + lb.k(i), k_end, vb[i]);
                 if (!tc::mbar_wait(tc::smem_u32(&empty_bar[stage]), phase ^ 1, abort_flag)) {
                     if (lane == 0) atomicExch(p.status, 181);
                     ok = false;
@@ -911,12 +1088,18 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
                     phase ^= 1;
                 }
             }
+            }
             if (!ok) break;
+        }
+        if constexpr (in_pieces(AOp::kWalk) && in_pieces(BOp::kWalk)) {
+            // the last steps, one after another (after a wait that expired there is nobody to hand them to)
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            for (; in_flight > 0; --in_flight) hand_over(std::integral_constant<int, 0>());
         }
     } else if (warp == MMA_WARP) {
         // ------------------------------------------------------------------ MMA issue
         if (tc::elect_one()) {
-            constexpr bool A_MN = AOp::kWalk == kByK, B_MN = BOp::kWalk == kByK;
+            constexpr bool A_MN = mn_major(AOp::kWalk), B_MN = mn_major(BOp::kWalk);
             constexpr uint32_t idesc1 = tc::make_idesc(A_MN, B_MN, BM, BN);
             constexpr uint32_t idesc2 = tc::make_idesc(A_MN, B_MN, BM, PL == 3 ? 2 * BN : BN);
             // 16 k further on, and the stride between 64-row atoms
@@ -1189,7 +1372,7 @@ int gemm(ag_device *dev, int M, int N, int K, const AOp &A, const BOp &B, const 
     p.M = M;
     p.N = N;
     p.K = K;
-    if constexpr (BOp::kWalk != kByK) {
+    if constexpr (!mn_major(BOp::kWalk)) {
         if (N <= 32) return launch<T, 32>(dev, A, B, E, p);
     }
     const int64_t tiles = ceil_div(M, BM) * ceil_div(N, 128);

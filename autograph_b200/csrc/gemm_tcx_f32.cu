@@ -37,17 +37,18 @@ bool gemm_worth(ag_dtype dtype, int64_t m, int64_t k, int64_t n) {
 }
 
 // Against the gathered engine, m x k x n, us packed and gathered: f32 940 x 589 x 1039 28 and 21, 2401 x 352 x 875 30 and
-// 21, 1584 x 902 x 444 26 and 29, 607 x 1199 x 1072 28 and 37, 391 x 843 x 2387 32 and 45, 808 x 3023 x 420 31 and 47; bf16
-// 873 x 969 x 1119 22 and 17, 215 x 4559 x 725 21 and 17, 535 x 1481 x 1347 20 and 24, 3821 x 2459 x 153 25 and 35.  The
-// copy pass wants some 5e8 multiply-adds, counted by how much of its 256 x 256 tiles the output fills (528 columns are
-// 69 % of three tiles), and more of them when k is short, because a tile is then mostly its epilogue; bf16, whose
-// gathered tiles take half the time, wants more.  Over 90 drawn products of 1e8 to 3e9 multiply-adds these lines are 0.9 %
-// (f32) and 0.7 % (bf16) above always taking the faster engine; 873 x 969 x 1119 is on the wrong side of both.
+// 21, 1037 x 438 x 1885 33 and 27, 1584 x 902 x 444 26 and 29, 607 x 1199 x 1072 28 and 37, 391 x 843 x 2387 32 and 45, 808
+// x 3023 x 420 31 and 47; bf16 873 x 969 x 1119 22 and 17, 215 x 4559 x 725 21 and 17, 535 x 1481 x 1347 20 and 24, 3821 x
+// 2459 x 153 25 and 35.  The copy pass wants some 5e8 multiply-adds, counted by how much of its 256 x 256 tiles the output
+// fills (528 columns are 69 % of three tiles), and more of them when k is short, because a tile is then mostly its
+// epilogue; bf16, whose gathered tiles take half the time, wants more.  Over 90 drawn products of 1e8 to 3e9 multiply-adds
+// these lines are 1.0 % (f32) and 0.7 % (bf16) above always taking the faster engine; 873 x 969 x 1119 is on the wrong side
+// of both.
 bool packed_worth(ag_dtype dtype, int64_t m, int64_t k, int64_t n) {
     const double fill = ((double)m / (256.0 * ceil_div(m, 256))) * ((double)n / (256.0 * ceil_div(n, 256)));
     const double macs = (double)m * (double)n * (double)k * fill;
     const bool f32 = dtype == AG_F32;
-    return m >= 128 && n >= 128 && k >= 64 && macs >= (f32 ? 4.5e8 : 6e8) && macs * (double)k >= (f32 ? 2.5e11 : 8e11);
+    return m >= 128 && n >= 128 && k >= 64 && macs >= (f32 ? 4.5e8 : 6e8) && macs * (double)k >= (f32 ? 3e11 : 8e11);
 }
 
 // The filters are also counted with their channels padded to eight, in an int (repack_kernel).

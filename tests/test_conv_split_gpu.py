@@ -1,0 +1,67 @@
+"""GPU: convolutions whose tensors are split into channels-last bf16 planes ahead of the product (split_worth in
+csrc/conv_tcx_impl.cuh): every direction against float64, and sums that are not finite."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+# bs, ic, h, w, oc, filter, padding, stride, dilation: 3e8 multiply-adds in every direction
+CASES = [
+    (27, 40, 31, 28, 48, (3, 3), (1, 1), (1, 1), (1, 1)),    # channels in eights that are no sixteens
+    (14, 45, 33, 30, 70, (3, 3), (0, 1), (1, 1), (1, 1)),    # channels and columns padded, 128-column tiles with a rest
+    (33, 36, 29, 41, 33, (3, 5), (1, 2), (2, 1), (1, 1)),   # strides, columns beyond 32
+    (36, 64, 27, 25, 20, (3, 3), (2, 2), (1, 1), (2, 2)),    # dilation: masks of taps, fewer columns than a tile
+    (60, 32, 9, 9, 96, (5, 5), (2, 2), (1, 1), (1, 1)),     # few tiles: slices of k
+    (6, 72, 50, 22, 130, (5, 3), (4, 0), (1, 2), (1, 1)),   # taps that leave the image on most sides
+]
+
+
+def _reference(x, w, dy, p, s, d):
+    x, w, dy = x.double(), w.double(), dy.double()
+    kw = dict(padding=p, stride=s, dilation=d)
+    y = F.conv2d(x, w, **kw)
+    dx = torch.nn.grad.conv2d_input(x.shape, w, dy, **kw)
+    dw = torch.nn.grad.conv2d_weight(x, w.shape, dy, **kw)
+    return y, dw, dx
+
+
+def _inputs(dev, case, dtype):
+    bs, ic, h, w, oc, f, p, s, d = case
+    gen = torch.Generator(device=dev.torch_device).manual_seed(ic * oc)
+    rnd = lambda *shape: torch.randn(shape, generator=gen, device=dev.torch_device).to(dtype)
+    out = [(n + 2 * p[i] - d[i] * (f[i] - 1) - 1) // s[i] + 1 for i, n in enumerate((h, w))]
+    return rnd(bs, ic, h, w), rnd(oc, ic, *f), rnd(bs, oc, *out), dict(padding=p, stride=s, dilation=d)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("case", CASES)
+def test_split_convolutions(dev, case, dtype):
+    x, w, dy, opt = _inputs(dev, case, dtype)
+    got = (dev.conv2_forward(x, w, **opt), dev.conv2_backward_weight(x, dy, tuple(w.shape[2:]), **opt),
+           dev.conv2_backward_input(w, dy, tuple(x.shape[2:]), **opt))
+    ref = _reference(x, w, dy, opt["padding"], opt["stride"], opt["dilation"])
+    size = _reference(x.abs(), w.abs(), dy.abs(), opt["padding"], opt["stride"], opt["dilation"])
+    dev.wait()
+    for g, r, m in zip(got, ref, size):
+        # an f32 rounding per 64 products and slice, on sums that grow as a walk: 2^-20 of the sum of magnitudes is a
+        # hundred of them in a row; bf16's store on top
+        bound = 2.0 ** -20 * m + (2.0 ** -8 * r.abs() if dtype == torch.bfloat16 else 0.0)
+        assert bool(((g.double() - r).abs() <= bound).all())
+
+
+def test_split_convolutions_with_infinities(dev):
+    """An infinity and a NaN of the input reach the outputs that they reach in float64.  Their blocks of 32 x 32 are computed
+    again with FMAs one after another, so the others there have other roundings, within the same bound."""
+    x, w, dy, opt = _inputs(dev, CASES[1], torch.float32)
+    clean = x.clone()
+    x[2, 7, 11, 13], x[5, 44, 0, 29] = float("inf"), float("nan")
+    got = dev.conv2_forward(x, w, **opt), dev.conv2_backward_weight(x, dy, (3, 3), **opt)
+    ref = _reference(x, w, dy, opt["padding"], opt["stride"], opt["dilation"])
+    size = _reference(clean.abs(), w.abs(), dy.abs(), opt["padding"], opt["stride"], opt["dilation"])
+    dev.wait()
+    for g, r, m in zip(got, ref, size):
+        assert torch.equal(g.isnan(), r.isnan()) and torch.equal(g.isinf(), r.isinf())
+        assert bool((g[r.isinf()].sign() == r[r.isinf()].sign()).all())
+        ok = r.isfinite()
+        assert bool(((g.double() - r).abs()[ok] <= 2.0 ** -20 * m[ok]).all())
