@@ -1,0 +1,28 @@
+// f32 convolutions with stride 1 on the tensor cores, filters resident, one box of pixels per tile (conv_halo_f32.cu).
+#pragma once
+
+#include "common.cuh"
+
+namespace ag {
+namespace halo32 {
+
+// y[b][n][oy][ox] = sum over (c, fi, fj) of src[b][c][oy + fi - pad_h][ox + fj - pad_w] * w[n * s_row + c * s_c + tap], tap =
+// fi * fw + fj, or that counted from the end (reversed: the input gradient's order).
+struct Problem {
+    const float *src, *w;
+    int64_t bs, channels, h, wd;   // source
+    int64_t n, oh, ow;
+    int fh, fw, pad_h, pad_w;
+    int64_t s_row, s_c;
+    bool reversed;
+};
+
+// Up to 64 channels and columns whose filters fit shared memory beside two boxes; where it is the faster engine.
+bool takes(ag_device *dev, const Problem &p);
+
+// With the optional bias and relu of the separate operators.  *taken is false, and nothing was launched, where there is no
+// room for the planes.
+int run(ag_device *dev, const Problem &p, const float *bias, bool relu, float *y, bool *taken);
+
+}  // namespace halo32
+}  // namespace ag

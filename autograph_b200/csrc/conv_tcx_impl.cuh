@@ -1,6 +1,7 @@
 // Convolutions on the gathered-operand tensor-core engine, for one element type.
 #pragma once
 
+#include "conv_halo_f32.cuh"
 #include "gemm_tcx_impl.cuh"
 
 namespace ag {
@@ -131,6 +132,9 @@ static int launch_split(ag_device *dev, const SplitJob<T> &a, const SplitJob<T> 
 template <class T>
 static bool split_worth(const ConvMap &g, int64_t bytes, int64_t positions, int64_t n, int least_patch) {
     const int64_t patch = (int64_t)g.ff * g.cp;
+    // few columns are little work per element: with a stride, which makes few patches of them, not enough (136 x 64 x 24 ->
+    // 6 / 2 f32 36 and 31)
+    if (sizeof(T) == 4 && n < 32 && positions * patch * 48 < 8 * bytes) return false;
     return patch >= least_patch && bytes <= 80000000 && positions * patch * (n < 32 ? 32 : n) >= 300000000;
 }
 
@@ -155,6 +159,20 @@ __global__ void repack_kernel(const T *w, T *out, int total, int channels, int c
     div_k.divmod(i, row, k);
     div_cp.divmod(k, tap, c);
     out[i] = (int)c < channels ? w[(int)row * s_row + (int)c * s_c + (int)tap] : from_f32<T>(0.f);
+}
+
+// f32 convolutions with stride and dilation 1 on the engine with resident filters; AG_ERR_UNSUPPORTED (nothing launched,
+// no message) where that is not the one to take them.
+template <class T>
+static int by_halo(ag_device *dev, const ag_conv2_options *o, const halo32::Problem &p, const T *bias, bool relu, T *y) {
+    if constexpr (sizeof(T) == 4) {
+        bool taken = false;
+        if (o->stride[0] == 1 && o->stride[1] == 1 && o->dilation[0] == 1 && o->dilation[1] == 1 && halo32::takes(dev, p)) {
+            AG_TRY(halo32::run(dev, p, bias, relu, y, &taken));
+            if (taken) return AG_OK;
+        }
+    }
+    return AG_ERR_UNSUPPORTED;
 }
 
 // A product with the patch matrix of `map` (rows = positions, k = taps x channels) and the filter
@@ -199,6 +217,12 @@ int conv_forward(ag_device *dev, const T *x, int64_t bs, int64_t ic, int64_t ih,
                  const T *w, int64_t oc, const T *bias, const ag_conv2_options *o, int64_t oh,
                  int64_t ow, bool relu, T *y) {
     const int M = (int)(bs * oh * ow), N = (int)oc, ff = o->filter[0] * o->filter[1];
+    if constexpr (sizeof(T) == 4) {
+        const halo32::Problem p{x, w, bs, ic, ih, iw, oc, oh, ow, o->filter[0], o->filter[1], o->padding[0], o->padding[1],
+                                ic * ff, ff, false};
+        const int status = by_halo<T>(dev, o, p, bias, relu, y);
+        if (status != AG_ERR_UNSUPPORTED) return status;
+    }
     NchwOut<T> E{y, bias, N, (int)(oh * ow), FastDiv((uint32_t)(oh * ow)), relu};
     const ConvMap map = conv_map(ic, ih, iw, oh, ow, o, false);
     if (few_channels(map)) {
@@ -247,6 +271,12 @@ int conv_backward_input(ag_device *dev, const T *w, int64_t oc, int64_t ic, cons
                         T *dx) {
     const int ff = o->filter[0] * o->filter[1];
     const int M = (int)(bs * ih * iw), N = (int)ic;
+    if constexpr (sizeof(T) == 4) {
+        const halo32::Problem p{dy, w, bs, oc, oh, ow, ic, ih, iw, o->filter[0], o->filter[1], o->filter[0] - 1 - o->padding[0],
+                                o->filter[1] - 1 - o->padding[1], ff, ic * ff, true};
+        const int status = by_halo<T>(dev, o, p, nullptr, false, dx);
+        if (status != AG_ERR_UNSUPPORTED) return status;
+    }
     const ConvMap map = conv_map(oc, oh, ow, ih, iw, o, true);
     // With few input channels a tile of the patch form is mostly empty columns, and it gathers dy
     // once per tap.  The other order multiplies dy by the filters of every (channel, tap) and adds

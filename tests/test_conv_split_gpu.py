@@ -1,5 +1,6 @@
 """GPU: convolutions whose tensors are split into channels-last bf16 planes ahead of the product (split_worth in
-csrc/conv_tcx_impl.cuh): every direction against float64, and sums that are not finite."""
+csrc/conv_tcx_impl.cuh; csrc/conv_halo_f32.cu, whose filters stay in shared memory): every direction against float64, and sums
+that are not finite."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -14,6 +15,18 @@ CASES = [
     (36, 64, 27, 25, 20, (3, 3), (2, 2), (1, 1), (2, 2)),    # dilation: masks of taps, fewer columns than a tile
     (60, 32, 9, 9, 96, (5, 5), (2, 2), (1, 1), (1, 1)),     # few tiles: slices of k
     (6, 72, 50, 22, 130, (5, 3), (4, 0), (1, 2), (1, 1)),   # taps that leave the image on most sides
+]
+# The same for the engine with resident filters, f32, 8e7 multiply-adds forward and in the input gradient: pixel rows of 32, 64
+# and 128 bytes both ways, 16, 32 and 64 columns with a rest, padding none, "same" and full, k groups with a rest
+RESIDENT = [
+    (64, 16, 32, 32, 32, (3, 3), (1, 1), (1, 1), (1, 1)),
+    (90, 12, 29, 23, 20, (3, 3), (0, 0), (1, 1), (1, 1)),
+    (30, 30, 41, 35, 62, (3, 3), (2, 2), (1, 1), (1, 1)),
+    (40, 60, 30, 27, 15, (3, 3), (1, 0), (1, 1), (1, 1)),
+    (70, 16, 26, 31, 6, (5, 5), (2, 2), (1, 1), (1, 1)),
+    (150, 6, 33, 34, 33, (3, 3), (1, 1), (1, 1), (1, 1)),
+    (50, 33, 25, 26, 13, (1, 5), (0, 2), (1, 1), (1, 1)),
+    (1500, 20, 12, 11, 40, (2, 3), (1, 1), (1, 1), (1, 1)),   # several images per tile, tiles in every accumulator
 ]
 
 
@@ -34,10 +47,12 @@ def _inputs(dev, case, dtype):
     return rnd(bs, ic, h, w), rnd(oc, ic, *f), rnd(bs, oc, *out), dict(padding=p, stride=s, dilation=d)
 
 
-@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("case", CASES)
+@pytest.mark.parametrize("case,dtype", [(c, t) for c in CASES for t in (torch.float32, torch.bfloat16)] +
+                         [(c, torch.float32) for c in RESIDENT])
 def test_split_convolutions(dev, case, dtype):
     x, w, dy, opt = _inputs(dev, case, dtype)
+    bias = torch.randn(w.shape[0], generator=torch.Generator().manual_seed(1)).to(dtype).to(x.device)
+    biased = dev.conv2_forward(x, w, bias, relu=True, **opt)
     got = (dev.conv2_forward(x, w, **opt), dev.conv2_backward_weight(x, dy, tuple(w.shape[2:]), **opt),
            dev.conv2_backward_input(w, dy, tuple(x.shape[2:]), **opt))
     ref = _reference(x, w, dy, opt["padding"], opt["stride"], opt["dilation"])
@@ -48,14 +63,16 @@ def test_split_convolutions(dev, case, dtype):
         # hundred of them in a row; bf16's store on top
         bound = 2.0 ** -20 * m + (2.0 ** -8 * r.abs() if dtype == torch.bfloat16 else 0.0)
         assert bool(((g.double() - r).abs() <= bound).all())
+    assert torch.equal(biased, (got[0] + bias[:, None, None]).clamp(min=0))
 
 
-def test_split_convolutions_with_infinities(dev):
+@pytest.mark.parametrize("case", [CASES[1], RESIDENT[1]])
+def test_split_convolutions_with_infinities(dev, case):
     """An infinity and a NaN of the input reach the outputs that they reach in float64.  Their blocks of 32 x 32 are computed
     again with FMAs one after another, so the others there have other roundings, within the same bound."""
-    x, w, dy, opt = _inputs(dev, CASES[1], torch.float32)
+    x, w, dy, opt = _inputs(dev, case, torch.float32)
     clean = x.clone()
-    x[2, 7, 11, 13], x[5, 44, 0, 29] = float("inf"), float("nan")
+    x[2, 7, 11, 13], x[5, -1, 0, 22] = float("inf"), float("nan")
     got = dev.conv2_forward(x, w, **opt), dev.conv2_backward_weight(x, dy, (3, 3), **opt)
     ref = _reference(x, w, dy, opt["padding"], opt["stride"], opt["dilation"])
     size = _reference(clean.abs(), w.abs(), dy.abs(), opt["padding"], opt["stride"], opt["dilation"])
