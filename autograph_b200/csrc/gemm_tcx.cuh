@@ -35,7 +35,7 @@
 #include <type_traits>
 
 #include "common.cuh"
-#include "tc_ptx.cuh"
+#include "pair_ptx.cuh"
 
 namespace ag {
 namespace tcx {
@@ -734,6 +734,9 @@ struct Cfg {
     static constexpr int ACC_COLS = PL == 3 ? 2 * BN : BN;       // f32: leading block + corrections
     static constexpr int TMEM = 2 * ACC_COLS < 64 ? 64 : 2 * ACC_COLS;
     static constexpr int SMEM = STAGES * STAGE + 1024 + 256 + 2 * kFewPatch * (int)sizeof(int) + (PL == 3 ? kMarks : 0);
+    // A slice's sums lie behind redo_block's buffers.
+    static constexpr int SUMS = PL == 3 ? (THREADS / 32 * kRedoFloats * 4 + 1023) / 1024 * 1024 : 0;
+    static_assert(SUMS + BN * BM * 4 <= STAGES * STAGE, "a slice's sums fit the stages");
     static_assert(SMEM <= 227 * 1024, "shared memory");
     static_assert(TMEM <= 512 && (TMEM & (TMEM - 1)) == 0, "tensor memory columns");
     static_assert(COLS % 32 == 0 && EPI_WARPS <= 8, "blocks of 32 columns, a mark bit per epilogue warp");
@@ -747,6 +750,7 @@ struct Params {
     int work0, work1;                       // this launch's share of the tiles x slices
     float *partial;                         // splits > 1: [splits][N][M] f32 sums
     int *arrivals;                          // not null: the CTA of a tile that finishes last adds its slices
+    int cluster;                            // the CTAs of a tile's slices are a cluster, which adds them
     int *status;
 };
 
@@ -880,14 +884,21 @@ __device__ __forceinline__ void reduce_tile(const Params &p, const Epi &E, int m
     }
 }
 
+// First work item of a CTA; item w is slice w / tiles of tile w % tiles, and the slices of a tile are neighbouring CTAs
+// where they are a cluster.
+__device__ __forceinline__ int first_item(const Params &p) {
+    if (p.cluster) return (int)(blockIdx.x % (unsigned)p.splits) * p.tiles_m * p.tiles_n + (int)(blockIdx.x / (unsigned)p.splits);
+    return p.work0 + (int)blockIdx.x;
+}
+
 // The marked blocks of this CTA's tiles, dealt to its warps.
 template <class C, class AOp, class BOp, class Epi>
 __device__ __noinline__ void redo_marked(const AOp &A, const BOp &B, const Epi &E, const Params &p,
-                                         const unsigned *marks, float *buf) {
+                                         const unsigned *marks, float *buf, float *sums) {
     constexpr int WARPS = C::THREADS / 32, BLOCKS = C::EPI_WARPS * C::COLS / 32;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, tiles = p.tiles_m * p.tiles_n;
     int turn = 0;
-    for (int w = p.work0 + blockIdx.x, i = 0; w < p.work1; w += gridDim.x, ++i) {
+    for (int w = first_item(p), i = 0; w < p.work1; w += gridDim.x, ++i) {
         const unsigned mark = marks[i / 4] >> (i % 4 * 8) & 255u;
         const int tile = w % tiles, z = w / tiles;
         const int k_begin = z * p.k_split, k_end = min(p.K, k_begin + p.k_split);
@@ -906,7 +917,9 @@ __device__ __noinline__ void redo_marked(const AOp &A, const BOp &B, const Epi &
                 for (int c = 0; c < 8; ++c) {
                     if (col + c >= p.N) break;
                     const float v = r == 0 ? acc[0][c] : r == 1 ? acc[1][c] : r == 2 ? acc[2][c] : acc[3][c];
-                    if (p.splits > 1)
+                    if (Epi::kLastCtaAdds && p.cluster)
+                        sums[(col + c) % C::BN * BM + (row + r) % BM] = v;
+                    else if (p.splits > 1)
                         p.partial[((int64_t)z * p.N + col + c) * p.M + row + r] = v;
                     else
                         E.store(st, col + c, v);
@@ -937,6 +950,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
 
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     constexpr int MMA_WARP = PRODUCERS / 32 + C::EPI_WARPS;
+    float *sums = reinterpret_cast<float *>(smem + C::SUMS);   // [column][row] of a slice, in stages that are not used any more
 
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -981,7 +995,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
     dependency_wait();
 
     const int tiles = p.tiles_m * p.tiles_n;
-    const int num_work = p.work1, work0 = p.work0 + blockIdx.x;
+    const int num_work = p.work1, work0 = first_item(p);
 
     if (warp < PRODUCERS / 32) {
         // ------------------------------------------------------------------ producers
@@ -1235,6 +1249,11 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
                 }
             }
             if (redo_it) {
+            } else if (Epi::kLastCtaAdds && p.cluster) {
+                // the stages have been read: this CTA's products are done
+                float *q = sums + col_base * BM + quarter * 32 + lane;
+#pragma unroll
+                for (int j = 0; j < C::COLS; ++j) q[j * BM] = sum[j];
             } else if (in && p.splits > 1) {
                 float *q = p.partial + ((int64_t)z * p.N + col0) * p.M + row;
 #pragma unroll
@@ -1261,8 +1280,30 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
         tc::tmem_dealloc(tmem, C::TMEM);
     }
     if (PL == 3 && *redo && !*abort_flag) {
-        redo_marked<C, AOp, BOp, Epi>(A, B, E, p, marks, reinterpret_cast<float *>(smem) + warp * kRedoFloats);
+        redo_marked<C, AOp, BOp, Epi>(A, B, E, p, marks, reinterpret_cast<float *>(smem) + warp * kRedoFloats, sums);
         __syncthreads();
+    }
+    if (Epi::kLastCtaAdds && p.cluster) {
+        // Every CTA adds a share of the columns over the slices, in slice order as reduce_splits_kernel does.
+        tc::pair::cluster_sync();
+        const int tile = work0 % tiles, rank = work0 / tiles;
+        const int m0 = (tile % p.tiles_m) * BM, n0 = (tile / p.tiles_m) * BN, row = tid % BM;
+        const int share = (min(BN, p.N - n0) + p.splits - 1) / p.splits;
+        const int first = rank * share, last = min(min(BN, p.N - n0), first + share);
+        if (tid < C::THREADS / BM * BM && m0 + row < p.M)
+            for (int col = first + tid / BM; col < last; col += C::THREADS / BM) {
+                const uint32_t at = tc::smem_u32(sums + col * BM + row);
+                float v[8], sum = 0.f;
+#pragma unroll
+                for (int z = 0; z < 8; ++z) v[z] = z < p.splits ? __uint_as_float(tc::pair::ld_shared_cluster(tc::pair::map_to_cta(at, z))) : 0.f;
+#pragma unroll
+                for (int z = 0; z < 8; ++z)
+                    if (z < p.splits) sum += v[z];
+                typename Epi::State st = E.begin(m0 + row, n0 + col);
+                E.store(st, n0 + col, sum);
+            }
+        tc::pair::cluster_sync();   // the others have read this CTA's sums
+        return;
     }
     if (Epi::kLastCtaAdds && p.arrivals != nullptr) {
         // every CTA has had one slice of one tile (grid = tiles * splits)
@@ -1310,6 +1351,48 @@ __global__ void __launch_bounds__(256)
 }
 
 // --------------------------------------------------------------------- host
+constexpr int kMostCluster = 8;   // what every GPU takes
+
+// One more than the clusters of `size` CTAs that run at a time.
+template <class... P>
+int cluster_room(void (*kernel)(P...), int threads, int smem, int size, int *room) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)size);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)size;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    AG_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
+    *room = n + 1;
+    return AG_OK;
+}
+
+// launch_dependent with clusters of `size` CTAs.
+template <class... P, class... A>
+int launch_clusters(ag_device *dev, void (*kernel)(P...), int grid, int threads, int smem, int size, const A &...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = dev->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)size;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    AG_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
+    AG_CHECK_LAUNCH();
+    return AG_OK;
+}
+
 template <class T, int BN, class AOp, class BOp, class Epi>
 int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
     using C = Cfg<T, BN>;
@@ -1329,7 +1412,27 @@ int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
     p.status = dev->status_dev;
     p.partial = nullptr;
     p.arrivals = nullptr;
-    if (p.splits > 1) {
+    auto kernel = gemm_tcx_kernel<T, BN, AOp, BOp, Epi>;
+    static bool configured_on[64] = {};
+    bool &configured = configured_on[dev->ordinal & 63];
+    if (!configured) {
+        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+        configured = true;
+    }
+    // Convolutions of up to eight short slices: the CTAs of a tile are a cluster and add them through its shared memory, if
+    // all clusters find room at once (a GPC holds two of eight CTAs).  Against the tile's last CTA, us, images x channels x
+    // side -> filters: 9 x 16 x 10 -> 64 5x5 f32 forward 14.5 and 18.0, weight gradient 11.6 and 15.0, 24 x 64 x 13 -> 128 5x5
+    // bf16 forward 18.8 and 21.1, weight gradient 23.6 and 28.0.  Long slices are slower so (6 x 64 x 43 -> 128 5x5 f32 weight
+    // gradient, 35 steps each, 72 and 60), and so are products in a row, whose second launch overlaps the next one (464 x 256
+    // x 112 bf16 8.6 and 7.2).
+    p.cluster = 0;
+    if (Epi::kLastCtaAdds && p.splits > 1 && p.splits <= kMostCluster && per <= 16) {
+        static int room_on[64][kMostCluster + 1] = {};   // clusters + 1
+        int &room = room_on[dev->ordinal & 63][p.splits];
+        if (room == 0) AG_TRY(cluster_room(kernel, C::THREADS, C::SMEM, p.splits, &room));
+        p.cluster = tiles < room;
+    }
+    if (p.splits > 1 && !p.cluster) {
         void *ws = nullptr;
         AG_TRY(engine_scratch(dev, sizeof(float) * (size_t)p.splits * p.M * p.N, &ws));
         p.partial = (float *)ws;
@@ -1341,12 +1444,10 @@ int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
             (int64_t)p.splits * (p.M < BM ? p.M : BM) * (p.N < BN ? p.N : BN) <= 65536)
             p.arrivals = dev->tile_counters;
     }
-    auto kernel = gemm_tcx_kernel<T, BN, AOp, BOp, Epi>;
-    static bool configured_on[64] = {};
-    bool &configured = configured_on[dev->ordinal & 63];
-    if (!configured) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-        configured = true;
+    if (p.cluster) {
+        p.work0 = 0;
+        p.work1 = (int)(tiles * p.splits);
+        return launch_clusters(dev, kernel, p.work1, C::THREADS, C::SMEM, p.splits, A, B, E, p);
     }
     const int64_t work = tiles * p.splits, most = (int64_t)kMarks * dev->sm_count;
     for (int64_t w = 0; w < work; w += most) {   // one launch, but for f32 outputs of 2.4e9 values and more

@@ -82,3 +82,27 @@ def test_split_convolutions_with_infinities(dev, case):
         assert bool((g[r.isinf()].sign() == r[r.isinf()].sign()).all())
         ok = r.isfinite()
         assert bool(((g.double() - r).abs()[ok] <= 2.0 ** -20 * m[ok]).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("case", [
+    (9, 16, 10, 11, 64, (5, 5), (0, 0), (1, 1), (1, 1)),     # a few slices of one wave of tiles
+    (24, 64, 13, 13, 100, (5, 5), (2, 2), (1, 1), (1, 1)),   # columns with a rest, shares of them that differ
+    (50, 64, 12, 13, 33, (3, 3), (0, 0), (2, 2), (1, 1)),    # a last tile of 33 - 32 columns' share, strides
+    (4, 40, 20, 24, 17, (3, 3), (1, 1), (1, 1), (1, 1)),
+])
+def test_slices_added_by_clusters(dev, case, dtype):
+    """Convolutions whose k slices are added through the shared memory of a cluster, and one with a NaN in a slice."""
+    x, w, dy, opt = _inputs(dev, case, dtype)
+    for bad in (False, True):
+        if bad:
+            x[1, 3, 4, 5] = float("nan")
+        got = dev.conv2_forward(x, w, **opt), dev.conv2_backward_weight(x, dy, tuple(w.shape[2:]), **opt)
+        ref = _reference(x, w, dy, opt["padding"], opt["stride"], opt["dilation"])
+        size = _reference(x.abs().nan_to_num(), w.abs(), dy.abs(), opt["padding"], opt["stride"], opt["dilation"])
+        dev.wait()
+        for g, r, m in zip(got, ref, size):
+            ok = r.isfinite()
+            assert torch.equal(g.isnan(), r.isnan())
+            bound = 2.0 ** -20 * m + (2.0 ** -8 * r.abs() if dtype == torch.bfloat16 else 0.0)
+            assert bool(((g.double() - r).abs()[ok] <= bound[ok]).all())
