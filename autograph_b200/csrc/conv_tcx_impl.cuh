@@ -166,11 +166,8 @@ __global__ void repack_kernel(const T *w, T *out, int total, int channels, int c
 template <class T>
 static int by_halo(ag_device *dev, const ag_conv2_options *o, const halo32::Problem &p, const T *bias, bool relu, T *y) {
     if constexpr (sizeof(T) == 4) {
-        bool taken = false;
-        if (o->stride[0] == 1 && o->stride[1] == 1 && o->dilation[0] == 1 && o->dilation[1] == 1 && halo32::takes(dev, p)) {
-            AG_TRY(halo32::run(dev, p, bias, relu, y, &taken));
-            if (taken) return AG_OK;
-        }
+        if (o->stride[0] == 1 && o->stride[1] == 1 && o->dilation[0] == 1 && o->dilation[1] == 1 && halo32::takes(dev, p))
+            return halo32::run(dev, p, bias, relu, y);
     }
     return AG_ERR_UNSUPPORTED;
 }
@@ -315,6 +312,14 @@ template <class T>
 int conv_backward_weight(ag_device *dev, const T *x, int64_t bs, int64_t ic, int64_t ih, int64_t iw,
                          const T *dy, int64_t oc, const ag_conv2_options *o, int64_t oh, int64_t ow,
                          float beta, T *dw) {
+    if constexpr (sizeof(T) == 4) {
+        const halo32::Wgrad p{x, dy, bs, ic, ih, iw, oc, oh, ow, o->filter[0], o->filter[1], o->padding[0], o->padding[1]};
+        if (o->stride[0] == 1 && o->stride[1] == 1 && o->dilation[0] == 1 && o->dilation[1] == 1 && halo32::takes_wgrad(p)) {
+            bool taken = false;
+            AG_TRY(halo32::run_wgrad(dev, p, beta, dw, &taken));
+            if (taken) return AG_OK;
+        }
+    }
     const ConvMap map = conv_map(ic, ih, iw, oh, ow, o, false);
     const int N = (int)oc, K = (int)(bs * oh * ow), hw = (int)(oh * ow);
     if (few_channels(map)) {

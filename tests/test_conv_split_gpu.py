@@ -27,6 +27,11 @@ RESIDENT = [
     (150, 6, 33, 34, 33, (3, 3), (1, 1), (1, 1), (1, 1)),
     (50, 33, 25, 26, 13, (1, 5), (0, 2), (1, 1), (1, 1)),
     (1500, 20, 12, 11, 40, (2, 3), (1, 1), (1, 1), (1, 1)),   # several images per tile, tiles in every accumulator
+    (1500, 20, 12, 11, 30, (2, 3), (1, 1), (1, 1), (1, 1)),
+    (200, 40, 24, 23, 31, (3, 3), (1, 1), (1, 1), (1, 1)),    # weight gradients: two products a filter row, one accumulator of each
+    (41, 3, 20, 21, 10, (3, 3), (0, 1), (1, 1), (1, 1)),
+    (17, 33, 9, 57, 16, (1, 7), (0, 3), (1, 1), (1, 1)),      # four of them
+    (9, 1, 40, 31, 5, (5, 4), (4, 3), (1, 1), (1, 1)),        # padding of all but a pixel
 ]
 
 
