@@ -6,15 +6,18 @@
 // is the output pixel.  With both tensors rewritten channels-last, a chunk of 64
 // pixels (a TH x TW rectangle of one image) of dy is a [64 pixels][64 channels]
 // TMA box -- an MN-major operand tile for tcgen05.mma -- and the matching chunk
-// of x for tap (fi, fj) is the same box shifted by the tap; pixels outside the
+// of x for tap (fi, fj) is the same rectangle shifted by the tap; pixels outside the
 // image read as zero, which is both the padding and the ragged edge.
 //
 // A CTA owns one filter row (FW taps), one block of 128 output channels, one
 // block of input channels and a contiguous range of pixel chunks: every stage of
-// its ring holds one dy tile and FW shifted x tiles, the FW accumulators live in
-// TMEM for the whole range, and the f32 partial result goes to a scratch plane
-// [split][oc][tap][ci].  A second kernel adds the planes in split order (so the
-// result is reproducible), applies beta and writes dw in its [oc][ci][fi][fj]
+// its ring holds one dy tile and one box of x, FW - 1 pixels wider, in which the
+// taps' tiles start one pixel apart (the swizzle is a function of the absolute
+// shared-memory address).  With a box per tap a stage of 3 x 3 filters was 40 KB for 64 pixels of 64 channels, which the L2
+// fed at 11 TB/s; it is 25 KB: 256 x 64 x 31 x 31 -> 128 40.0 us and 35.5.  The FW accumulators live in TMEM for the whole
+// range, and the f32 partial result goes to a scratch plane
+// [split][tap][ci][oc], in which a warp's 32 output channels are one line (as [oc][tap][ci], 32 lines a store: 35.5 us and
+// 31.0).  A second kernel adds the planes in split order (so the result is reproducible), applies beta and writes dw in its [oc][ci][fi][fj]
 // layout.  Warp roles and the bounded waits are those of the GEMM kernel.
 #include "conv_tc.cuh"
 #include "tc_ptx.cuh"
@@ -43,8 +46,8 @@ struct WgParams {
     int m_blocks, n_blocks;
     int pad_h, pad_w;
     int Cp, taps;
-    int stages, stage_bytes;
-    float *partial;            // [splits][m_blocks * 128][taps][Cp]
+    int stages, stage_bytes, x_atom_bytes, load_bytes;   // x_atom_bytes: a box of 64 channels, a multiple of 1024
+    float *partial;            // [splits][taps][Cp][m_blocks * 128]
     int *status;
 };
 
@@ -120,18 +123,17 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
                     break;
                 }
                 const uint32_t bar = smem_u32(&full_bar[stage]);
-                mbar_arrive_expect_tx(bar, (uint32_t)p.stage_bytes);
+                mbar_arrive_expect_tx(bar, (uint32_t)p.load_bytes);
                 const uint32_t a_dst = smem_u32(smem + stage * p.stage_bytes);
                 const uint32_t b_dst = a_dst + WG_A_BYTES;
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
                     tma_load_4d(a_dst + i * WG_ATOM_BYTES, &tmap_dy, bar, m_blk * WG_BLOCK_M + i * 64,
                                 ox0, oy0, b);
-                for (int g = 0; g < p.FW; ++g)
 #pragma unroll
-                    for (int j = 0; j < ATOMS_N; ++j)
-                        tma_load_4d(b_dst + (g * ATOMS_N + j) * WG_ATOM_BYTES, &tmap_x, bar,
-                                    n_blk * NT + j * 64, ox0 + g - p.pad_w, oy0 + group - p.pad_h, b);
+                for (int j = 0; j < ATOMS_N; ++j)
+                    tma_load_4d(b_dst + j * p.x_atom_bytes, &tmap_x, bar, n_blk * NT + j * 64, ox0 - p.pad_w,
+                                oy0 + group - p.pad_h, b);
                 if (++stage == p.stages) {
                     stage = 0;
                     phase ^= 1;
@@ -142,11 +144,11 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
         if (elect_one()) {
-            // The x tiles of the taps of a filter row lie one after the other in the stage and
-            // their accumulators one after the other in TMEM, so several taps are ONE operand
-            // of up to 256 columns: one tcgen05.mma per k step covers them all, which moves
-            // far fewer operand bytes per flop than one 64-column instruction per tap.
-            const int taps_per_mma = min(p.FW, 256 / NT);
+            // Up to four taps of a filter row are ONE operand, blocks of 64 channels that start one
+            // pixel apart: one tcgen05.mma per k step covers them all, which moves far fewer
+            // operand bytes per flop than one 64-column instruction per tap.
+            const int pitch = p.TW + p.FW - 1;   // pixels of a row of x's box
+            const uint32_t x_groups = p.TW == 8 ? (uint32_t)pitch * 128 : 1024u;   // from eight pixels to the next
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -159,21 +161,20 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
                 tc_fence_after();
                 const uint32_t a_base = smem_u32(smem + stage * p.stage_bytes);
                 const uint32_t b_base = a_base + WG_A_BYTES;
-                for (int g0 = 0; g0 < p.FW; g0 += taps_per_mma) {
-                    const int n_cols = min(taps_per_mma, p.FW - g0) * NT;
-                    const uint32_t idesc = make_idesc(true, true, WG_BLOCK_M, n_cols);
 #pragma unroll
-                    for (int k = 0; k < WG_CHUNK / WG_UMMA_K; ++k) {
-                        // 16 pixel rows of 128 bytes per k step
-                        const uint64_t a_desc =
-                            make_smem_desc(a_base + k * WG_UMMA_K * 128, WG_ATOM_BYTES, 1024);
-                        const uint64_t b_desc =
-                            make_smem_desc(b_base + g0 * ATOMS_N * WG_ATOM_BYTES + k * WG_UMMA_K * 128,
-                                           WG_ATOM_BYTES, 1024);
-                        umma_bf16(tmem_base + (uint32_t)(g0 * NT), a_desc, b_desc, idesc,
-                                  (c > c_begin || k > 0) ? 1u : 0u);
+                for (int j = 0; j < ATOMS_N; ++j)
+                    for (int g0 = 0; g0 < p.FW; g0 += 4) {
+                        const uint32_t idesc = make_idesc(true, true, WG_BLOCK_M, min(4, p.FW - g0) * 64);
+#pragma unroll
+                        for (int k = 0; k < WG_CHUNK / WG_UMMA_K; ++k) {
+                            // 16 pixel rows of 128 bytes per k step
+                            const int at = k * WG_UMMA_K, pixel = (at >> p.tw_shift) * pitch + (at & (p.TW - 1)) + g0;
+                            const uint64_t a_desc = make_smem_desc(a_base + at * 128, WG_ATOM_BYTES, 1024);
+                            const uint64_t b_desc = make_smem_desc(b_base + j * p.x_atom_bytes + pixel * 128, 128, x_groups);
+                            umma_bf16(tmem_base + (uint32_t)((j * p.FW + g0) * 64), a_desc, b_desc, idesc,
+                                      (c > c_begin || k > 0) ? 1u : 0u);
+                        }
                     }
-                }
                 umma_commit(smem_u32(&empty_bar[stage]));
                 if (++stage == p.stages) {
                     stage = 0;
@@ -190,21 +191,18 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
             tc_fence_after();
             const int row = m_blk * WG_BLOCK_M + quarter * 32 + lane;  // output channel
             const int64_t m_total = (int64_t)p.m_blocks * WG_BLOCK_M;
-            float *base = p.partial + (((int64_t)split * m_total + row) * p.taps) * p.Cp +
-                          (int64_t)n_blk * NT;
+            float *base = p.partial + ((int64_t)split * p.taps * p.Cp + n_blk * NT) * m_total + row;
             for (int g = 0; g < p.FW; ++g) {
-                float *dst = base + (int64_t)(group * p.FW + g) * p.Cp;
+                float *dst = base + (int64_t)(group * p.FW + g) * p.Cp * m_total;
 #pragma unroll 1
                 for (int chunk = 0; chunk < NT / 32; ++chunk) {
                     uint32_t v[32];
                     tmem_ld_32x32(tmem_base + ((uint32_t)(quarter * 32) << 16) +
-                                      (uint32_t)(g * NT + chunk * 32),
+                                      (uint32_t)((chunk / 2 * p.FW + g) * 64 + chunk % 2 * 32),
                                   v);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        reinterpret_cast<uint4 *>(dst + chunk * 32)[j] =
-                            make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    for (int j = 0; j < 32; ++j, dst += m_total) *dst = __uint_as_float(v[j]);
                 }
             }
         } else if (lane == 0) {
@@ -225,23 +223,21 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     }
 }
 
-// dw[oc][ci][tap] = beta * dw + sum over splits (in order) of partial[s][oc][tap][ci]
-// Block of 32 x 8 threads: 32 consecutive outputs, the split planes dealt round-robin to the 8
+// dw[oc][ci][tap] = beta * dw + sum over splits (in order) of partial[s][tap][ci][oc]
+// Block of 32 x 8 threads: 32 consecutive output channels of one (tap, ci), the split planes dealt round-robin to the 8
 // rows (every load of a warp is 128 contiguous bytes of one plane); the 8 row sums are added in
-// row order, so the result does not depend on scheduling.
+// row order, so the result does not depend on scheduling.  Threads that found their (oc, tap, ci) by 64-bit divisions spent most
+// of their instructions on them: 49 planes of 128 x 9 x 64, cold, 11.8 us and 9.9; a call on 9 x 6 x 63 x 63 -> 32 25.6 and 20.1.
 __global__ void wgrad_reduce_kernel(const float *__restrict__ partial, int splits, int64_t m_total,
                                     int taps, int Cp, int OC, int IC, float beta,
                                     __nv_bfloat16 *__restrict__ dw) {
     let_dependents_launch(kAlwaysEarly);
     dependency_wait();
     __shared__ float part[8][33];
-    const int64_t i = (int64_t)blockIdx.x * 32 + threadIdx.x;
-    const bool live = i < (int64_t)OC * taps * IC;
-    const int ci = live ? (int)(i % IC) : 0;
-    const int tap = live ? (int)((i / IC) % taps) : 0;
-    const int oc = live ? (int)(i / ((int64_t)IC * taps)) : 0;
+    const int tap = (int)blockIdx.x / IC, ci = (int)blockIdx.x - tap * IC, oc = blockIdx.y * 32 + threadIdx.x;
+    const bool live = oc < OC;
     const int64_t plane = m_total * taps * Cp;
-    const float *src = partial + ((int64_t)oc * taps + tap) * Cp + ci;
+    const float *src = partial + ((int64_t)tap * Cp + ci) * m_total + oc;
     float s = 0.f;
     if (live)
         for (int z = threadIdx.y; z < splits; z += 48) {   // six loads in flight (one at a time: 7.3 us for 148 planes)
@@ -358,7 +354,10 @@ int backward_weight_nhwc(ag_device *dev, const __nv_bfloat16 *xh, int64_t bs, in
     p.pad_w = o->padding[1];
     p.Cp = (int)cp;
     p.taps = fh * fw;
-    p.stage_bytes = WG_A_BYTES + fw * nt * 128;
+    const int x_box = (p.TW + fw - 1) * th * 128;
+    p.x_atom_bytes = (int)round_up64(x_box, 1024);
+    p.stage_bytes = WG_A_BYTES + nt / 64 * p.x_atom_bytes;
+    p.load_bytes = WG_A_BYTES + nt / 64 * x_box;
     p.stages = (200 * 1024) / p.stage_bytes;
     if (p.stages > WG_MAX_STAGES) p.stages = WG_MAX_STAGES;
     AG_REQUIRE(p.stages >= 2, AG_ERR_LIMIT, "filter too wide for the tensor-core weight gradient");
@@ -385,7 +384,7 @@ int backward_weight_nhwc(ag_device *dev, const __nv_bfloat16 *xh, int64_t bs, in
     {
         const uint64_t dims[4] = {(uint64_t)cp, (uint64_t)iw, (uint64_t)ih, (uint64_t)bs};
         const uint64_t strides[3] = {(uint64_t)cp, (uint64_t)(iw * cp), (uint64_t)(ih * iw * cp)};
-        const uint32_t box[4] = {64, (uint32_t)p.TW, (uint32_t)th, 1};
+        const uint32_t box[4] = {64, (uint32_t)(p.TW + fw - 1), (uint32_t)th, 1};
         AG_TRY(make_tmap_bf16(&tx, xh, 4, dims, strides, box));
     }
     const int grid = splits * base;
@@ -393,8 +392,7 @@ int backward_weight_nhwc(ag_device *dev, const __nv_bfloat16 *xh, int64_t bs, in
         AG_TRY(launch_wgrad<128>(dev, tdy, tx, p, grid));
     else
         AG_TRY(launch_wgrad<64>(dev, tdy, tx, p, grid));
-    const int64_t outs = oc * p.taps * ic;
-    AG_TRY((launch_dependent(dev, wgrad_reduce_kernel, dim3((unsigned)ceil_div(outs, 32)), dim3(32, 8), 0, p.partial,
+    AG_TRY((launch_dependent(dev, wgrad_reduce_kernel, dim3((unsigned)(p.taps * ic), (unsigned)ceil_div(oc, 32)), dim3(32, 8), 0, p.partial,
                              splits, m_total, p.taps, (int)cp, (int)oc, (int)ic, beta, dw)));
     return AG_OK;
 }

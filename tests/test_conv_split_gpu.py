@@ -69,6 +69,10 @@ def test_split_convolutions(dev, case, dtype):
         bound = 2.0 ** -20 * m + (2.0 ** -8 * r.abs() if dtype == torch.bfloat16 else 0.0)
         assert bool(((g.double() - r).abs() <= bound).all())
     assert torch.equal(biased, (got[0] + bias[:, None, None]).clamp(min=0))
+    if dtype == torch.float32:
+        added = dev.conv2_backward_weight(x, dy, tuple(w.shape[2:]), beta=1.0, dw=torch.ones_like(got[1]), **opt)
+        dev.wait()
+        assert torch.equal(added, got[1] + 1)
 
 
 @pytest.mark.parametrize("case", [CASES[1], RESIDENT[1]])

@@ -104,3 +104,18 @@ def test_conv_tc_weight_gradient(dev, shape):
                                     (f, f), **kw).float().cpu().numpy()
     assert np.abs(got - ref64).max() / np.abs(ref64).max() <= 1e-2
     dev.wait()
+
+
+@pytest.mark.parametrize("fh,fw", [(1, 1), (3, 2), (2, 3), (3, 4), (1, 5), (2, 8)])
+@pytest.mark.parametrize("ic,ow", [(40, 8), (64, 15), (100, 29), (128, 16), (64, 64), (130, 7)])
+def test_conv_tc_weight_gradient_boxes(dev, ic, ow, fh, fw):
+    """Every width of a pixel chunk (8 to 64) by every number of taps that share its box, one and two blocks of 64 channels: exact on
+    small integers."""
+    rng = np.random.default_rng(ic + ow + 16 * fw)
+    kw = dict(padding=(fh - 1, fw // 2))
+    oh, bs = 11, -(-4200 // (11 * ow))
+    x = _ints(rng, (bs, ic, oh - fh + 1, ow + fw - 1 - 2 * (fw // 2)), -2, 2)
+    dy = _ints(rng, (bs, 48, oh, ow), -2, 2)
+    got = dev.conv2_backward_weight(dev.tensor(x, torch.bfloat16), dev.tensor(dy, torch.bfloat16), (fh, fw), **kw)
+    ref = torch.nn.grad.conv2d_weight(torch.from_numpy(x).double(), (48, ic, fh, fw), torch.from_numpy(dy).double(), **kw)
+    assert torch.equal(got.double().cpu(), ref.to(torch.bfloat16).double())
