@@ -886,8 +886,9 @@ __device__ __forceinline__ void reduce_tile(const Params &p, const Epi &E, int m
 
 // First work item of a CTA; item w is slice w / tiles of tile w % tiles, and the slices of a tile are neighbouring CTAs
 // where they are a cluster.
+template <class Epi>
 __device__ __forceinline__ int first_item(const Params &p) {
-    if (p.cluster) return (int)(blockIdx.x % (unsigned)p.splits) * p.tiles_m * p.tiles_n + (int)(blockIdx.x / (unsigned)p.splits);
+    if (Epi::kLastCtaAdds && p.cluster) return (int)(blockIdx.x % (unsigned)p.splits) * p.tiles_m * p.tiles_n + (int)(blockIdx.x / (unsigned)p.splits);
     return p.work0 + (int)blockIdx.x;
 }
 
@@ -898,7 +899,7 @@ __device__ __noinline__ void redo_marked(const AOp &A, const BOp &B, const Epi &
     constexpr int WARPS = C::THREADS / 32, BLOCKS = C::EPI_WARPS * C::COLS / 32;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, tiles = p.tiles_m * p.tiles_n;
     int turn = 0;
-    for (int w = first_item(p), i = 0; w < p.work1; w += gridDim.x, ++i) {
+    for (int w = first_item<Epi>(p), i = 0; w < p.work1; w += gridDim.x, ++i) {
         const unsigned mark = marks[i / 4] >> (i % 4 * 8) & 255u;
         const int tile = w % tiles, z = w / tiles;
         const int k_begin = z * p.k_split, k_end = min(p.K, k_begin + p.k_split);
@@ -995,7 +996,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
     dependency_wait();
 
     const int tiles = p.tiles_m * p.tiles_n;
-    const int num_work = p.work1, work0 = first_item(p);
+    const int num_work = p.work1, work0 = first_item<Epi>(p);
 
     if (warp < PRODUCERS / 32) {
         // ------------------------------------------------------------------ producers
