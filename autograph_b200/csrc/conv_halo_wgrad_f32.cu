@@ -29,7 +29,7 @@ constexpr int kMostSums = 6;   // accumulators of 16 columns that a warp's regis
 
 struct WgradParams {
     Source x, dy;
-    int tiles, wp, fh, products;          // products: blocks of taps of a filter row
+    int tiles, wp, fh, fw, products;      // products: blocks of taps of a filter row
     int x_rows, dy_rows, stages;          // of a box
     float *partial;                       // [CTA][product][filter row, last first][n][128]
     int *status;
@@ -178,6 +178,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         // 32 rows and 16 columns of every accumulator
         const int quarter = warp % 4, part = (warp - 2) / 4;
         const bool mine = part * 16 < N;
+        // taps of a product's rows; those beyond the filter are neither read nor stored
+        const int first = quarter * 64 / RB, tap = (quarter * 32 + lane) * 2 / RB;
         float sum[kMostSums][16];
 #pragma unroll
         for (int i = 0; i < kMostSums; ++i)
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (mine)
 #pragma unroll
                     for (int i = 0; i < kMostSums; ++i)
-                        if (i < accs) {
+                        if (i < accs && i / p.fh * BLOCKS + first < p.fw) {
                             const uint32_t at = t + (i + i / p.fh * p.fh) * N;   // a product's two blocks of fh * N
                             uint32_t r0[16], r1[16];
                             tmem_ld_32x16(at, r0);
@@ -219,7 +221,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             float *q = p.partial + ((int64_t)blockIdx.x * accs * N + part * 16) * 128 + quarter * 32 + lane;
 #pragma unroll
             for (int i = 0; i < kMostSums; ++i)
-                if (i < accs)
+                if (i < accs && i / p.fh * BLOCKS + tap < p.fw)
 #pragma unroll
                     for (int j = 0; j < 16; ++j) q[(i * N + j) * 128] = sum[i][j];
         }
@@ -382,6 +384,7 @@ int run_wgrad(ag_device *dev, const Wgrad &p, float beta, float *dw, bool *taken
     a.tiles = (int)l.tiles;
     a.wp = (int)l.wp;
     a.fh = p.fh;
+    a.fw = p.fw;
     a.products = l.products;
     a.x_rows = l.x_rows;
     a.dy_rows = l.dy_rows;
