@@ -410,7 +410,8 @@ int ag_conv2_backward_input(ag_device *dev, ag_dtype dtype, const void *w, int64
         return convtc::backward_input(dev, (const __nv_bfloat16 *)w, oc, ic,
                                       (const __nv_bfloat16 *)dy, bs, ih, iw, opt,
                                       (__nv_bfloat16 *)dx);
-    if (direct::eligible_backward_input(bs, ic, ih, iw, oc, opt)) {
+    if (direct::eligible_backward_input(bs, ic, ih, iw, oc, opt) &&
+        !tcx::input_by_rows(dev, dtype, oc, ic, bs, ih, iw, opt, g.oh, g.ow)) {
         if (dtype == AG_F32)
             return direct::backward_input<float>(dev, (const float *)w, oc, ic, (const float *)dy,
                                                  bs, ih, iw, opt, (float *)dx);
@@ -448,7 +449,8 @@ int ag_conv2_backward_weight(ag_device *dev, ag_dtype dtype, const void *x, int6
         return convtc::backward_weight(dev, (const __nv_bfloat16 *)x, bs, ic, ih, iw,
                                        (const __nv_bfloat16 *)dy, oc, opt, beta,
                                        (__nv_bfloat16 *)dw);
-    if (direct::eligible_backward_weight(bs, ic, ih, iw, oc, opt)) {
+    if (direct::eligible_backward_weight(bs, ic, ih, iw, oc, opt) &&
+        !tcx::weight_by_rows(dtype, bs, ic, ih, iw, oc, opt, g.oh, g.ow)) {
         if (dtype == AG_F32)
             return direct::backward_weight<float>(dev, (const float *)x, bs, ic, ih, iw,
                                                   (const float *)dy, oc, opt, beta, (float *)dw);

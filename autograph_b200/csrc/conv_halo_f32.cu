@@ -374,13 +374,14 @@ int launch(ag_device *dev, const Plan &l, const Params &a) {
 // 40 -> 64 13.2 and 14.4, 10 x 32 x 42 -> 64's input gradient 19.2 and 21.5).  Channels are padded to 16 and columns to 16, 32 or 64: up to
 // 4 channels gain where there is much work (189 x 3 x 20 -> 64 18.5 and 21.2, 246 x 3 x 55 -> 64 146 and 111), 94 x 6 x 31
 // -> 64 5 x 5 43 and 46.  Many channels into few columns are faster as products with every tap: 189 x 3 x 20 -> 64's input
-// gradient 22.7 and 30.8, 232 x 1 x 60 -> 32's 101 and 138, but 8 x 1 x 61 -> 32's 14.6 and 11.6.
+// gradient 22.7 and 30.8, 232 x 1 x 60 -> 32's 101 and 138, 658 x 3 x 27 -> 20 5 x 5's 178 and 222, but 8 x 1 x 61 -> 32's 14.6 and 11.6.
 bool takes(ag_device *dev, const Problem &p) {
     Plan l;
     if (!make_plan(dev, p, &l)) return false;
     const int64_t taps = p.fh * p.fw, work = p.bs * p.oh * p.ow * taps * p.channels * (p.n < 16 ? 16 : p.n);
     if (p.channels < 12 && taps > 9 && p.n > 32) return false;
-    if ((p.channels > 32 && p.n * taps <= 128) || (p.channels > 16 && p.n <= 2 && work > (taps > 9 ? 100000000 : 300000000)))
+    if ((p.channels > 32 && p.n * taps <= 128) || (p.channels > 16 && p.n <= 2 && work > (taps > 9 ? 100000000 : 300000000)) ||
+        (p.channels > 16 && p.n <= 4 && taps > 9 && work > 300000000))
         return false;
     if (2 * p.oh * p.ow < l.hp * l.wp) return false;   // rows of the frame that are outputs
     if (p.channels <= 4) return taps <= 9 && work >= 200000000;

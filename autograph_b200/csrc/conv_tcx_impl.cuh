@@ -161,12 +161,26 @@ __global__ void repack_kernel(const T *w, T *out, int total, int channels, int c
     out[i] = (int)c < channels ? w[(int)row * s_row + (int)c * s_c + (int)tap] : from_f32<T>(0.f);
 }
 
+inline bool plain(const ag_conv2_options *o) {
+    return o->stride[0] == 1 && o->stride[1] == 1 && o->dilation[0] == 1 && o->dilation[1] == 1;
+}
+inline halo32::Problem input_rows(const float *w, int64_t oc, int64_t ic, const float *dy, int64_t bs, int64_t ih, int64_t iw,
+                                  const ag_conv2_options *o, int64_t oh, int64_t ow) {
+    const int fh = o->filter[0], fw = o->filter[1];
+    return halo32::Problem{dy, w, bs, oc, oh, ow, ic, ih, iw, fh, fw, fh - 1 - o->padding[0], fw - 1 - o->padding[1],
+                           (int64_t)fh * fw, ic * fh * fw, true};
+}
+inline halo32::Wgrad weight_rows(const float *x, int64_t bs, int64_t ic, int64_t ih, int64_t iw, const float *dy, int64_t oc,
+                                 const ag_conv2_options *o, int64_t oh, int64_t ow) {
+    return halo32::Wgrad{x, dy, bs, ic, ih, iw, oc, oh, ow, o->filter[0], o->filter[1], o->padding[0], o->padding[1]};
+}
+
 // f32 convolutions with stride and dilation 1 on the engine with resident filters; AG_ERR_UNSUPPORTED (nothing launched,
 // no message) where that is not the one to take them.
 template <class T>
 static int by_halo(ag_device *dev, const ag_conv2_options *o, const halo32::Problem &p, const T *bias, bool relu, T *y) {
     if constexpr (sizeof(T) == 4) {
-        if (o->stride[0] == 1 && o->stride[1] == 1 && o->dilation[0] == 1 && o->dilation[1] == 1 && halo32::takes(dev, p))
+        if (plain(o) && halo32::takes(dev, p))
             return halo32::run(dev, p, bias, relu, y);
     }
     return AG_ERR_UNSUPPORTED;
@@ -269,8 +283,7 @@ int conv_backward_input(ag_device *dev, const T *w, int64_t oc, int64_t ic, cons
     const int ff = o->filter[0] * o->filter[1];
     const int M = (int)(bs * ih * iw), N = (int)ic;
     if constexpr (sizeof(T) == 4) {
-        const halo32::Problem p{dy, w, bs, oc, oh, ow, ic, ih, iw, o->filter[0], o->filter[1], o->filter[0] - 1 - o->padding[0],
-                                o->filter[1] - 1 - o->padding[1], ff, ic * ff, true};
+        const halo32::Problem p = input_rows((const float *)w, oc, ic, (const float *)dy, bs, ih, iw, o, oh, ow);
         const int status = by_halo<T>(dev, o, p, nullptr, false, dx);
         if (status != AG_ERR_UNSUPPORTED) return status;
     }
@@ -313,8 +326,8 @@ int conv_backward_weight(ag_device *dev, const T *x, int64_t bs, int64_t ic, int
                          const T *dy, int64_t oc, const ag_conv2_options *o, int64_t oh, int64_t ow,
                          float beta, T *dw) {
     if constexpr (sizeof(T) == 4) {
-        const halo32::Wgrad p{x, dy, bs, ic, ih, iw, oc, oh, ow, o->filter[0], o->filter[1], o->padding[0], o->padding[1]};
-        if (o->stride[0] == 1 && o->stride[1] == 1 && o->dilation[0] == 1 && o->dilation[1] == 1 && halo32::takes_wgrad(p)) {
+        const halo32::Wgrad p = weight_rows((const float *)x, bs, ic, ih, iw, (const float *)dy, oc, o, oh, ow);
+        if (plain(o) && halo32::takes_wgrad(p)) {
             bool taken = false;
             AG_TRY(halo32::run_wgrad(dev, p, beta, dw, &taken));
             if (taken) return AG_OK;

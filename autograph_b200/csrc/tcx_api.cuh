@@ -31,6 +31,12 @@ bool conv_worth(ag_dtype dtype, int64_t patch, int64_t cols, int64_t positions, 
 bool conv_input_worth(int64_t patch, int64_t cols, int64_t positions, const ag_conv2_options *o);
 bool conv_weight_worth(ag_dtype dtype, int64_t patch, int64_t oc, int64_t positions,
                        const ag_conv2_options *o);
+// f32 gradients that the kernels on pixel rows (conv_halo_f32.cuh) take and are faster at than the direct kernels.
+bool input_by_rows(ag_device *dev, ag_dtype dtype, int64_t oc, int64_t ic, int64_t bs, int64_t ih, int64_t iw,
+                   const ag_conv2_options *o, int64_t oh, int64_t ow);
+bool weight_by_rows(ag_dtype dtype, int64_t bs, int64_t ic, int64_t ih, int64_t iw, int64_t oc, const ag_conv2_options *o,
+                    int64_t oh, int64_t ow);
+
 template <class T>
 int conv_forward(ag_device *dev, const T *x, int64_t bs, int64_t ic, int64_t ih, int64_t iw,
                  const T *w, int64_t oc, const T *bias, const ag_conv2_options *o, int64_t oh,

@@ -32,6 +32,8 @@ RESIDENT = [
     (41, 3, 20, 21, 10, (3, 3), (0, 1), (1, 1), (1, 1)),
     (17, 33, 9, 57, 16, (1, 7), (0, 3), (1, 1), (1, 1)),      # four of them
     (9, 1, 40, 31, 5, (5, 4), (4, 3), (1, 1), (1, 1)),        # padding of all but a pixel
+    (33, 16, 20, 22, 6, (3, 3), (0, 0), (1, 1), (1, 1)),      # where the direct kernels could be
+    (60, 12, 24, 26, 16, (5, 5), (0, 0), (1, 1), (1, 1)),
 ]
 
 
