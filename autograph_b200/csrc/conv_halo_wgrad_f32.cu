@@ -354,7 +354,7 @@ int launch_wgrad(ag_device *dev, const WgradPlan &l, int grid, const WgradParams
 }  // namespace
 
 // Against the gathered engine, us there and here, images x channels x side -> columns, 3 x 3 unless said: 64 x 16 x 32 -> 32 34.2 and
-// 22.5, 163 x 32 x 40 -> 16 117 and 42, 144 x 64 x 56 -> 6 438 and 124, 136 x 16 x 53 -> 32 149 and 78, 231 x 6 x 57 -> 6 5 x 5 248
+// 21.7, 163 x 32 x 40 -> 16 117 and 42, 144 x 64 x 56 -> 6 438 and 124, 136 x 16 x 53 -> 32 149 and 78, 231 x 6 x 57 -> 6 5 x 5 248
 // and 100, 53 x 3 x 48 -> 16 28 and 20, 87 x 1 x 17 -> 6 14.3 and 11.3, 4 x 64 x 39 -> 16 16.2 and 15.7.
 // It pads channels and columns and has two launches: 17 x 16 x 22 -> 32 5 x 5 13.7 and 18.0, 5 x 64 x 47 -> 32 21.9 and 25.4 (61 x 64
 // x 31 -> 32 57 and 45), 136 x 1 x 57 -> 32 5 x 5 70 and 123, 14 x 64 x 10 -> 6 9.9 and 12.7.  With 64 columns a tile's sums are 96
