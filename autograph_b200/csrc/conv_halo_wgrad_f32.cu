@@ -1,4 +1,4 @@
-// Weight gradients of f32 convolutions with stride 1 and up to 64 channels both ways on tcgen05 (three bf16 planes per operand
+// Weight gradients of f32 convolutions with stride 1 from up to 64 channels into up to 32 on tcgen05 (three bf16 planes per operand
 // and sums of 64 k read out and added in registers, as in gemm_tcx.cuh).
 //
 //   dw[n][c][fi][fj] = sum over rows r of x[r + fj][c] * dy[r - fi * Wp][n]
