@@ -4,6 +4,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -276,5 +277,22 @@ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 // let dependents launch at their start, the wide stack at 256 images bf16: inference 203 us, so 289, a training step 492
 // and 569): more than half of an SM's memory keeps them apart.
 constexpr int kOneCtaPerSm = 116 * 1024;
+
+// What lets a kernel have more than 48 KB of dynamic shared memory is an attribute of the (kernel, GPU) pair, while calls are
+// serialised per ag_device: devices of one GPU in several threads share it.  So every kernel gets one constant that no
+// call exceeds.  A size per call, or the largest so far, can be lowered by another thread between a call's set and its
+// launch, which then fails.
+constexpr int kMostSmem = 226 * 1024;   // beside up to 1 KB of static shared memory
+struct SmemAllowed {
+    std::atomic<uint64_t> gpus{0};   // a bit per ordinal; beyond 64 of them the attribute is set on every call
+};
+template <class K>
+int allow_smem(ag_device *dev, K kernel, SmemAllowed &done) {
+    const uint64_t bit = dev->ordinal < 64 ? 1ull << dev->ordinal : 0;
+    if (done.gpus.load(std::memory_order_acquire) & bit) return AG_OK;
+    AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem));
+    done.gpus.fetch_or(bit, std::memory_order_release);
+    return AG_OK;
+}
 
 }  // namespace ag

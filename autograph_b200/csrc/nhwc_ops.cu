@@ -440,7 +440,10 @@ static int channels_per_cta(ag_device *dev, int64_t bs, int64_t c) {
 template <class K, class... A>
 static int launch_nchw(ag_device *dev, K kernel, int cg, int64_t bs, int64_t c, int64_t windows, const A &...args) {
     const int smem = (int)(cg * windows * 2);
-    if (smem > 48 * 1024) AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (cg == 64) {   // the others stay below 48 KB
+        static SmemAllowed allowed;
+        AG_TRY(allow_smem(dev, kernel, allowed));
+    }
     return launch_dependent(dev, kernel, dim3((unsigned)(c / cg), (unsigned)bs), 256, (size_t)smem, args...);
 }
 
