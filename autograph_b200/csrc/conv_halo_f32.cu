@@ -341,7 +341,7 @@ bool make_plan(ag_device *dev, const Problem &p, Plan *l) {
     if (halo > 256) return false;
     l->halo_rows = (int)halo;
     const int weights = (p.fh * p.fw * 3 * l->bn * l->rb + 1023) / 1024 * 1024, box = (int)halo * l->rb * 3;
-    l->stages = (226 * 1024 - 1024 - kControl - weights) / box;
+    l->stages = (kMostSmem - 1024 - kControl - weights) / box;
     if (l->stages < 2) return false;
     if (l->stages > kStages) l->stages = kStages;
     l->smem = weights + l->stages * box + 1024 + kControl;
@@ -353,12 +353,8 @@ template <int RB, int BN>
 int launch(ag_device *dev, const Plan &l, const Params &a) {
     auto kernel = conv_halo_f32_kernel<RB, BN>;
     const int smem = l.smem < kOneCtaPerSm ? kOneCtaPerSm : l.smem;
-    static int configured_on[64] = {};
-    int &configured = configured_on[dev->ordinal & 63];
-    if (smem > configured) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        configured = smem;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem(dev, kernel, allowed));
     const int grid = l.tiles < dev->sm_count ? (int)l.tiles : dev->sm_count;
     return launch_dependent(dev, kernel, dim3((unsigned)grid), kThreads, smem, a);
 }

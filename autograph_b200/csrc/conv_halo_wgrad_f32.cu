@@ -330,7 +330,7 @@ bool make_wgrad_plan(const Wgrad &p, WgradPlan *l) {
     if (l->wp * (l->rn >> 4) >= (1 << 14)) return false;   // a descriptor's stride
     l->dy_rows = (int)ceil_div(128 + (p.fh - 1) * l->wp, 32) * 32;
     const int64_t stage = 3 * ((int64_t)l->x_rows * l->rb + (int64_t)l->dy_rows * l->rn);
-    l->stages = (int)((226 * 1024 - 1024 - kControl) / stage);
+    l->stages = (int)((kMostSmem - 1024 - kControl) / stage);
     if (l->stages < 2) return false;
     if (l->stages > kStages) l->stages = kStages;
     l->smem = l->stages * (int)stage + 1024 + kControl;
@@ -342,12 +342,8 @@ template <int RB, int RN>
 int launch_wgrad(ag_device *dev, const WgradPlan &l, int grid, const WgradParams &a) {
     auto kernel = conv_halo_wgrad_kernel<RB, RN>;
     const int smem = l.smem < kOneCtaPerSm ? kOneCtaPerSm : l.smem;
-    static int configured_on[64] = {};
-    int &configured = configured_on[dev->ordinal & 63];
-    if (smem > configured) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        configured = smem;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem(dev, kernel, allowed));
     return launch_dependent(dev, kernel, dim3((unsigned)grid), kThreads, smem, a);
 }
 

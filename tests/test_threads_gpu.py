@@ -48,3 +48,26 @@ def test_pools_to_nchw_of_several_sizes(dev, monkeypatch):
     for d in devices:
         d.wait()
     assert not raised, raised
+
+
+def test_convolutions_on_pixel_rows_of_several_sizes(dev):
+    """The first calls of the kernels on pixel rows, 16 channels into 32, in two threads: boxes of 224 rows and of 160, filters
+    of 27 KB and of 9 KB, whose shared memory differs."""
+    import autograph_b200 as ag
+    cases = []
+    for hw, f in ((32, (3, 3)), (24, (1, 3))):
+        x = torch.randn((64, 16, hw, hw), device=dev.torch_device)
+        w = torch.randn((32, 16, *f), device=dev.torch_device)
+        dy = torch.randn((64, 32, hw, hw), device=dev.torch_device)
+        cases.append((ag.Device(0), x, w, dy, dict(padding=(f[0] // 2, f[1] // 2))))
+    torch.cuda.synchronize()
+
+    def call(d, x, w, dy, opt):
+        d.conv2_forward(x, w, **opt)
+        d.conv2_backward_weight(x, dy, tuple(w.shape[2:]), **opt)
+        d.conv2_backward_input(w, dy, tuple(x.shape[2:]), **opt)
+
+    raised = _in_threads([lambda c=c: call(*c) for c in cases], 200)
+    for d, *_ in cases:
+        d.wait()
+    assert not raised, raised
