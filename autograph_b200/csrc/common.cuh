@@ -282,15 +282,15 @@ constexpr int kOneCtaPerSm = 116 * 1024;
 // serialised per ag_device: devices of one GPU in several threads share it.  So every kernel gets one constant that no
 // call exceeds.  A size per call, or the largest so far, can be lowered by another thread between a call's set and its
 // launch, which then fails.
-constexpr int kMostSmem = 226 * 1024;   // beside up to 1 KB of static shared memory
+constexpr int kMostSmem = 226 * 1024;   // of 227, beside up to 1 KB of static shared memory
 struct SmemAllowed {
     std::atomic<uint64_t> gpus{0};   // a bit per ordinal; beyond 64 of them the attribute is set on every call
 };
-template <class K>
+template <int MOST = kMostSmem, class K>
 int allow_smem(ag_device *dev, K kernel, SmemAllowed &done) {
     const uint64_t bit = dev->ordinal < 64 ? 1ull << dev->ordinal : 0;
     if (done.gpus.load(std::memory_order_acquire) & bit) return AG_OK;
-    AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem));
+    AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST));
     done.gpus.fetch_or(bit, std::memory_order_release);
     return AG_OK;
 }

@@ -226,9 +226,10 @@ template <class T, int FH, int FW>
 static int launch_banded(ag_device *dev, const T *x, const T *w, const T *bias, T *y,
                          const Params &p, size_t smem) {
     auto kernel = conv2_direct_banded_kernel<T, FH, FW>;
-    if (smem > 48 * 1024)
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
+    if (smem > 48 * 1024) {
+        static SmemAllowed allowed;
+        AG_TRY(allow_smem(dev, kernel, allowed));
+    }
     AG_TRY((launch_dependent(dev, kernel, dim3((unsigned)p.bs), 256, smem, x, w, bias, y, p)));
     return AG_OK;
 }
@@ -272,9 +273,10 @@ template <class T, int FH, int FW, bool BWD>
 static int launch(ag_device *dev, const T *x, const T *w, const T *bias, T *y, const Params &p,
                   size_t smem, int items_per_img, T *pre_y = nullptr) {
     auto kernel = conv2_direct_kernel<T, FH, FW, BWD>;
-    if (smem > 48 * 1024)
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
+    if (smem > 48 * 1024) {
+        static SmemAllowed allowed;
+        AG_TRY(allow_smem(dev, kernel, allowed));
+    }
     int threads = ((p.group * items_per_img * p.split + 31) / 32) * 32;
     if (p.fine) threads *= (p.pool || p.keep_pre) ? 4 : 8;
     if (threads > 256) threads = 256;

@@ -165,9 +165,10 @@ template <class T, int FH, int FW>
 static int launch_wgrad(ag_device *dev, const T *x, const T *dy, const WgradParams &p, size_t smem,
                         float beta, T *dw) {
     auto kernel = conv2_wgrad_kernel<T, FH, FW>;
-    if (smem > 48 * 1024)
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
+    if (smem > 48 * 1024) {
+        static SmemAllowed allowed;
+        AG_TRY(allow_smem(dev, kernel, allowed));
+    }
     const int len = p.items * FW;
     const int ctas = (int)ceil_div(p.bs, p.group);
     void *ws = nullptr;

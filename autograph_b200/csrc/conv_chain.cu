@@ -236,9 +236,10 @@ bool eligible(int64_t bs, int64_t ic, int64_t ih, int64_t iw, int n_conv,
 template <class T, int F>
 static int launch(ag_device *dev, const T *x, T *y, const Plan &pl, size_t smem) {
     auto kernel = conv_chain_kernel<T, F>;
-    if (smem > 48 * 1024)
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
+    if (smem > 48 * 1024) {
+        static SmemAllowed allowed;
+        AG_TRY(allow_smem(dev, kernel, allowed));
+    }
     kernel<<<(unsigned)ceil_div(pl.bs, pl.group), 512, smem, dev->stream>>>(x, y, pl);
     AG_CHECK_LAUNCH();
     return AG_OK;
@@ -260,11 +261,8 @@ static int launch_lenet(ag_device *dev, const T *x, const uint8_t *x8, float alp
     lp.status = dev->status_dev;
     if (flat_out == nullptr) lp.done = take_signal(dev);
     auto kernel = lenet::lenet_chain_kernel<T>;
-    static bool attr_set[64] = {};
-    if (dev->ordinal >= 64 || !attr_set[dev->ordinal]) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsmem));
-        if (dev->ordinal < 64) attr_set[dev->ordinal] = true;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem<227 * 1024 - 64>(dev, kernel, allowed));   // the plans' budget
     // launched so that it may overlap the tail of a preceding launch of the same kernel
     // (the kernel itself waits for its predecessor before it reads or writes memory)
     cudaLaunchConfig_t cfg = {};
@@ -365,12 +363,8 @@ int forward(ag_device *dev, const T *x, const uint8_t *x8, float alpha, int64_t 
             int64_t group = ceil_div(bs, (int64_t)dev->sm_count);
             tp.group = (int)(group < 1 ? 1 : (group > lenet::kGroup ? lenet::kGroup : group));
             tp.status = dev->status_dev;
-            static bool attr_set = false;
-            if (!attr_set) {
-                AG_CUDA_TRY(cudaFuncSetAttribute(lenet_tc::lenet_chain_tc_kernel,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem));
-                attr_set = true;
-            }
+            static SmemAllowed allowed;
+            AG_TRY(allow_smem<227 * 1024 - 64>(dev, lenet_tc::lenet_chain_tc_kernel, allowed));
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)ceil_div(bs, (int64_t)tp.group));
             cfg.blockDim = dim3(lenet::kThreads);

@@ -488,14 +488,8 @@ template <int BLOCK_N>
 static int launch(ag_device *dev, const CUtensorMap &tx, const CUtensorMap &tw, const Params &p) {
     using C = Cfg<BLOCK_N>;
     auto kernel = conv2_bf16_tc_kernel<BLOCK_N>;
-    // the attribute belongs to the (kernel, GPU) pair: remembered per instantiation and GPU
-    static bool configured_on[64] = {};
-    bool &configured = configured_on[dev->ordinal & 63];
-    if (!configured) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         C::SMEM_BYTES));
-        configured = true;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem<C::SMEM_BYTES>(dev, kernel, allowed));
     const int64_t tiles = (int64_t)p.B * p.tiles_y * p.tiles_x * p.n_blocks;
     const int grid = (int)(tiles < dev->sm_count ? tiles : dev->sm_count);
     AG_TRY((launch_dependent(dev, kernel, dim3((unsigned)grid), NUM_THREADS, C::SMEM_BYTES, tx, tw, p)));

@@ -271,14 +271,8 @@ int launch_halo(ag_device *dev, const CUtensorMap &tx, const CUtensorMap &tw, co
                 int smem) {
     auto kernel = conv2_bf16_tc_halo_kernel<BLOCK_N>;
     if (smem < kOneCtaPerSm) smem = kOneCtaPerSm;
-    // the attribute belongs to the (kernel, GPU) pair: largest size set so far, per
-    // instantiation and GPU
-    static int configured_on[64] = {};
-    int &configured = configured_on[dev->ordinal & 63];
-    if (smem > configured) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        configured = smem;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem(dev, kernel, allowed));
     const int tiles = (p.R + HB_M - 1) / HB_M;
     const int grid = tiles < dev->sm_count ? tiles : dev->sm_count;
     AG_TRY((launch_dependent(dev, kernel, dim3((unsigned)grid), H_THREADS, smem, tx, tw, p)));

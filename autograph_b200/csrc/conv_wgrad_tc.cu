@@ -266,14 +266,8 @@ int launch_wgrad(ag_device *dev, const CUtensorMap &tdy, const CUtensorMap &tx, 
                  int grid) {
     auto kernel = conv2_wgrad_bf16_tc_kernel<NT>;
     const int need = p.stages * p.stage_bytes + 1024 + 256, smem = need < kOneCtaPerSm ? kOneCtaPerSm : need;
-    // the attribute belongs to the (kernel, GPU) pair: largest size set so far, per
-    // instantiation and GPU
-    static int configured_on[64] = {};
-    int &configured = configured_on[dev->ordinal & 63];
-    if (smem > configured) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        configured = smem;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem(dev, kernel, allowed));
     AG_TRY((launch_dependent(dev, kernel, dim3((unsigned)grid), WG_THREADS, smem, tdy, tx, p)));
     return AG_OK;
 }

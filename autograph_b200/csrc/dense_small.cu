@@ -181,11 +181,9 @@ int forward(ag_device *dev, const T *x, int m, int k, const T *w, int n, const T
     if ((int64_t)m * st.np > (sizeof(T) == 4 ? 256 : 128) * (int64_t)k) {
         const int threads = st.np * st.slices;
         const size_t smem = ((size_t)k * ROWS + (size_t)st.slices * ROWS * st.np) * sizeof(float);
-        static bool configured_on[64] = {};
-        if (smem > 48 * 1024 && !configured_on[dev->ordinal & 63]) {
-            AG_CUDA_TRY(cudaFuncSetAttribute(dense_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             80 * 1024));
-            configured_on[dev->ordinal & 63] = true;
+        if (smem > 48 * 1024) {
+            static SmemAllowed allowed;
+            AG_TRY(allow_smem(dev, dense_rows_kernel<T>, allowed));
         }
         AG_TRY((launch_dependent(dev, dense_rows_kernel<T>, dim3((unsigned)ceil_div(m, ROWS)), threads, smem, x, y, m,
                                  st)));
@@ -235,9 +233,10 @@ int chain_forward(ag_device *dev, const T *x, int m, int n_layers, const ChainLa
     const size_t smem = plan_chain(&p, m, n_layers, layers) * sizeof(float);
     const int threads = p.threads;
     auto kernel = dense_chain_kernel<T>;
-    if (smem > 48 * 1024)
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
+    if (smem > 48 * 1024) {
+        static SmemAllowed allowed;
+        AG_TRY(allow_smem(dev, kernel, allowed));
+    }
     kernel<<<(unsigned)ceil_div(m, ROWS), threads, smem, dev->stream>>>(x, y, p);
     AG_CHECK_LAUNCH();
     return AG_OK;
@@ -289,9 +288,10 @@ int chain_backward_input(ag_device *dev, const T *dy, int m, int n_steps, const 
     ChainParams p;
     const size_t smem = plan_chain(&p, m, n_steps, steps) * sizeof(float);
     auto kernel = dense_chain_backward_kernel<T>;
-    if (smem > 48 * 1024)
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
+    if (smem > 48 * 1024) {
+        static SmemAllowed allowed;
+        AG_TRY(allow_smem(dev, kernel, allowed));
+    }
     kernel<<<(unsigned)ceil_div(m, ROWS), p.threads, smem, dev->stream>>>(dy, gate_last, g_last, y, p);
     AG_CHECK_LAUNCH();
     return AG_OK;

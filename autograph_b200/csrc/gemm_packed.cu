@@ -526,13 +526,8 @@ template <int PL, bool A_MN, bool B_MN, class T>
 static int launch(ag_device *dev, const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &tt,
                   Params<T> p) {
     auto kernel = gemm_packed_kernel<PL, A_MN, B_MN, T>;
-    static bool configured_on[64] = {};
-    bool &configured = configured_on[dev->ordinal & 63];
-    if (!configured) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Cfg<PL>::SMEM));
-        configured = true;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem<Cfg<PL>::SMEM>(dev, kernel, allowed));
     const int most = tcx::kMarks * (dev->sm_count / 2);   // one launch for up to 5e9 outputs
     for (p.work0 = 0; p.work0 < p.num_work; p.work0 = p.work1) {
         const int left = p.num_work - p.work0, n = left < most ? left : most;

@@ -413,14 +413,8 @@ bool gemm_bf16_eligible(int64_t m, int64_t k, int64_t n, const __nv_bfloat16 *a,
 template <bool A_MN, bool B_MN>
 static int launch(ag_device *dev, const CUtensorMap &ta, const CUtensorMap &tb, const Params &p) {
     auto kernel = gemm_bf16_tc_kernel<A_MN, B_MN>;
-    // the attribute belongs to the (kernel, GPU) pair: remembered per instantiation and GPU
-    static bool configured_on[64] = {};
-    bool &configured = configured_on[dev->ordinal & 63];
-    if (!configured) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SMEM_BYTES));
-        configured = true;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem<SMEM_BYTES>(dev, kernel, allowed));
     const int tiles = (int)(ceil_div(p.M, BLOCK_M) * ceil_div(p.N, BLOCK_N)) * p.splits;
     const int grid = tiles < dev->sm_count ? tiles : dev->sm_count;
     AG_TRY((launch_dependent(dev, kernel, dim3((unsigned)grid), NUM_THREADS, SMEM_BYTES, ta, tb, p)));

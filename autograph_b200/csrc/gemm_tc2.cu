@@ -477,12 +477,8 @@ template <bool A_MN, bool B_MN>
 static int launch_pair(ag_device *dev, const CUtensorMap &ta, const CUtensorMap &tb,
                        const CUtensorMap &tb_tail, const pair::Params &p) {
     auto kernel = pair::gemm_bf16_tc2_kernel<A_MN, B_MN>;
-    static bool attr_done[64] = {};   // per GPU: the attribute belongs to the GPU's copy of the kernel
-    if (dev->ordinal >= 64 || !attr_done[dev->ordinal]) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         pair::SMEM_BYTES));
-        if (dev->ordinal < 64) attr_done[dev->ordinal] = true;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem<pair::SMEM_BYTES>(dev, kernel, allowed));
     int pairs = dev->sm_count / 2;
     if (p.num_work < pairs) pairs = p.num_work;
     return launch_dependent(dev, kernel, dim3(2 * pairs), pair::NUM_THREADS, pair::SMEM_BYTES, ta, tb, tb_tail, p);

@@ -1414,12 +1414,8 @@ int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
     p.partial = nullptr;
     p.arrivals = nullptr;
     auto kernel = gemm_tcx_kernel<T, BN, AOp, BOp, Epi>;
-    static bool configured_on[64] = {};
-    bool &configured = configured_on[dev->ordinal & 63];
-    if (!configured) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-        configured = true;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem<C::SMEM>(dev, kernel, allowed));
     // Convolutions of up to eight short slices: the CTAs of a tile are a cluster and add them through its shared memory, if
     // all clusters find room at once (a GPC holds two of eight CTAs).  Against the tile's last CTA, us, images x channels x
     // side -> filters: 9 x 16 x 10 -> 64 5x5 f32 forward 14.5 and 18.0, weight gradient 11.6 and 15.0, 24 x 64 x 13 -> 128 5x5

@@ -566,12 +566,8 @@ int run_forward(ag_device *dev, const Shape &s, const __nv_bfloat16 *x, const __
     const Params p = make_params(dev, s, x, F_TILE);
     constexpr int most = F_STAGES * f_stage_bytes<P>() + kMostChannels * P::KP * 2;
     constexpr int smem = most < kOneCtaPerSm ? kOneCtaPerSm : most;
-    static bool configured_on[64] = {};
-    bool &configured = configured_on[dev->ordinal & 63];
-    if (!configured) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(image_stage_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        configured = true;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem<smem>(dev, image_stage_kernel<P>, allowed));
     const int grid = p.tiles < dev->sm_count ? p.tiles : dev->sm_count;
     return launch_dependent(dev, image_stage_kernel<P>, dim3((unsigned)grid), F_THREADS, smem, p, w, bias, y, codes);
 }
@@ -589,12 +585,8 @@ int run_backward(ag_device *dev, const Shape &s, const __nv_bfloat16 *x, const _
     const Params p = make_params(dev, s, x, B_TILE);
     constexpr int smem = C::STAGES * C::STAGE + 1024;
     static_assert(smem >= kOneCtaPerSm && smem <= 226 * 1024, "one CTA per SM");
-    static bool configured_on[64] = {};
-    bool &configured = configured_on[dev->ordinal & 63];
-    if (!configured) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(image_stage_backward_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        configured = true;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem<smem>(dev, image_stage_backward_kernel<P>, allowed));
     const int blocks = (int)(s.oc / 64), grid = splits_of(dev, s) * blocks;
     return launch_dependent(dev, image_stage_backward_kernel<P>, dim3((unsigned)grid), B_THREADS, smem, p, dy, codes, blocks,
                             partial);

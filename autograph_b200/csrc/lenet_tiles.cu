@@ -667,11 +667,8 @@ int forward(ag_device *dev, const void *x, int64_t bs, const Weights &w, void *y
     const int threads = tiles > kBlob / 2 ? tiles : kBlob / 2;
     pack_kernel<<<(unsigned)ceil_div(threads, 256), 256, 0, dev->stream>>>(w, (unsigned char *)ws, a.bad, tiles);
     AG_CHECK_LAUNCH();
-    static bool configured[64] = {};
-    if (dev->ordinal >= 64 || !configured[dev->ordinal]) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-        if (dev->ordinal < 64) configured[dev->ordinal] = true;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem<kSmem>(dev, tile_kernel, allowed));
     tile_kernel<<<(unsigned)(tiles < dev->sm_count ? tiles : dev->sm_count), kThreads, kSmem, dev->stream>>>(a);
     AG_CHECK_LAUNCH();
     return AG_OK;

@@ -854,12 +854,8 @@ template <class T, int G>
 static int launch_pass(ag_device *dev, const Args &a, int ctas) {
     auto kernel = lenet_train_kernel<T, G>;
     constexpr int bytes = Smem<T, G>::floats * 4;
-    static bool configured_on[64] = {};
-    bool &configured = configured_on[dev->ordinal & 63];
-    if (!configured) {
-        AG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        configured = true;
-    }
+    static SmemAllowed allowed;
+    AG_TRY(allow_smem<bytes>(dev, kernel, allowed));
     kernel<<<ctas, kThreads, bytes, dev->stream>>>(a);
     AG_CHECK_LAUNCH();
     return AG_OK;
