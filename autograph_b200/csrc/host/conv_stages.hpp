@@ -271,7 +271,7 @@ class StageRun : public std::enable_shared_from_this<StageRun> {
         if (d.image) {
             sums = Tensor::uninit(*pool, {::ag::image_stage::partial_floats(dev, d.image_shape(bs))}, AG_F32);
             check(::ag::image_stage::backward(dev, d.image_shape(bs), cptr(act[s]), cptr(dpool),
-                                              (const uint32_t *)code[s].data(), (float *)sums.data()));
+                                              (const uint32_t *)code[s].data(), d.conv->has_bias, (float *)sums.data()));
             have[s] = 1;
             return;
         }

@@ -12,12 +12,15 @@
 //   patches, which overlap, from those registers.  Operands lie in 16-byte rows without swizzle,
 //   [8 values of k][window][8]: a warp's stores are 512 consecutive bytes.
 //
-// Backward.  dw[oc][k] and, against a k value that is 1 everywhere, db[oc]: the reduction runs over windows and cells.
+// Backward.  dw[oc][k] and db[oc]: the reduction runs over windows and cells.
 // The operand of a cell is the pooled gradient where the code names that cell and zero elsewhere, written by the
 // producers to [window][64 channels] rows (MN-major); the patches are the same rows as in the forward pass, read
 // MN-major.  Two cells share an instruction: rows 0 - 63 of A are cell 2j's channels, rows 64 - 127 cell 2j + 1's, the
 // columns of B the patches of both; the two diagonal blocks of the accumulator are wanted, and the instruction
-// costs what one of half its rows does.  Every CTA leaves its sums; a second kernel adds them in order.
+// costs what one of half its rows does.  The bias gradient is added in registers by the producers: as a product with a
+// k value of 1 it was a sum of all of a CTA's windows in one accumulator, which adds with truncation (1024 images of 64 x
+// 64, 831 additions: more than 4e-6 of a value short, and the more the more images).  Every CTA leaves its sums; a second
+// kernel adds them in order.
 //
 // Measured at 256 x 3 x 64 x 64 -> 64, each kernel alone with cold caches: forward 23 us (patches, convolution and Relu +
 // pool as kernels of their own 38 + 57 + 23), backward 27 + 6 (pool gradient 30, weight gradient and its sum 47); a training
@@ -39,7 +42,7 @@ template <int IC_, int F_>
 struct Geo {
     static constexpr int IC = IC_, F = F_;
     static constexpr int K = IC * F * F;
-    static constexpr int KP = (K + 1 + 15) / 16 * 16;   // with room for the value that is 1
+    static constexpr int KP = (K + 1 + 15) / 16 * 16;   // a sum's column K is the bias gradient
     static constexpr int G = KP / 8;
     static constexpr int ROWS = F + 1, WORDS = (F + 1) / 2;
     static_assert(F % 2 == 1, "pairs of pixels");
@@ -74,8 +77,7 @@ struct Geo {
         auto word = [&](int k) { return v[k / (F * F)][dy + k / F % F][(dx + k % F) / 2]; };
         const int s0 = (dx + k % F) % 2 ? 0x32 : 0x10, s1 = (dx + (k + 1) % F) % 2 ? 0x7600 : 0x5400;
         if (k + 1 < K) return __byte_perm(word(k), word(k + 1), s0 | s1);
-        if (k < K) return __byte_perm(word(k), 0x3f80u, s0 | 0x5400);   // bf16 1
-        return k == K ? 0x3f80u : 0u;
+        return k < K ? __byte_perm(word(k), 0u, s0 | 0x5400) : 0u;
     }
     // The four patches: cell c's group g of this window at dst + (c * G + g) * pitch.
     __device__ __forceinline__ void store(uint8_t *dst, int pitch) const {
@@ -342,7 +344,8 @@ __device__ __forceinline__ uint32_t pair_mask(uint32_t lo, uint32_t hi, int j) {
     return m;
 }
 
-template <class P>
+// BIAS: with the bias gradient.
+template <class P, bool BIAS>
 __global__ void __launch_bounds__(B_THREADS, 1)
     image_stage_backward_kernel(const Params p, const __nv_bfloat16 *__restrict__ dy, const uint32_t *__restrict__ codes,
                                 int blocks, float *__restrict__ partial) {
@@ -350,6 +353,7 @@ __global__ void __launch_bounds__(B_THREADS, 1)
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ uint64_t full_bar[C::STAGES], empty_bar[C::STAGES], done_bar;
+    __shared__ float s_db[B_GRAD][64];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_word;
     volatile int *abort_flag = &abort_word;
@@ -381,6 +385,7 @@ __global__ void __launch_bounds__(B_THREADS, 1)
         const int row = warp * 4 + lane / 8, group = lane % 8;   // and row + 32
         uint4 g[2][2];
         uint32_t c[2][2];
+        float db[8] = {};   // of the group's channels
         auto fetch = [&](int buf, int tile) {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
@@ -424,6 +429,14 @@ __global__ void __launch_bounds__(B_THREADS, 1)
                             make_uint4(v.x & pair_mask(lo, hi, 0), v.y & pair_mask(lo, hi, 1), v.z & pair_mask(lo, hi, 2),
                                        v.w & pair_mask(lo, hi, 3));
                     }
+                    if (!BIAS) continue;
+                    const uint32_t passed = (c[buf][i] >> 2) & 0x11111111u, lo = passed << 7, hi = passed << 3;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t pair = (&v.x)[j] & pair_mask(lo, hi, j);
+                        db[2 * j] += __uint_as_float(pair << 16);
+                        db[2 * j + 1] += __uint_as_float(pair & 0xffff0000u);
+                    }
                 }
                 publish(smem_u32(&full_bar[stage]));
                 fetch(buf, tile + 2 * splits);
@@ -434,17 +447,31 @@ __global__ void __launch_bounds__(B_THREADS, 1)
                 tile += splits;
             }
         }
+        if (BIAS) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {   // lanes 8 apart have the same channels
+                db[e] += __shfl_xor_sync(0xffffffffu, db[e], 8);
+                db[e] += __shfl_xor_sync(0xffffffffu, db[e], 16);
+                if (lane < 8) s_db[warp][group * 8 + e] = db[e];
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(B_GRAD * 32) : "memory");   // the producers of gradients
+        }
         // the sums: rows 0 - 63 and columns below KP are the even cells', the others the odd ones'
         if (ok && warp < 4) {
             if (mbar_wait(smem_u32(&done_bar), 0, abort_flag)) {
                 tc_fence_after();
                 const int cell = warp / 2, oc = n0 + warp % 2 * 32 + lane;
+                float bias_sum = 0.f;   // in the even cells' sums
+                if (BIAS && cell == 0)
+#pragma unroll
+                    for (int i = 0; i < B_GRAD; ++i) bias_sum += s_db[i][warp % 2 * 32 + lane];
                 float *dst = partial + ((int64_t)(2 * split + cell) * p.oc + oc) * P::KP;
 #pragma unroll
                 for (int k = 0; k < P::KP; k += 16) {
                     uint32_t r[16];
                     tmem_ld_32x16(tmem + ((uint32_t)(warp * 32) << 16) + cell * P::KP + k, r);
                     tmem_ld_wait();
+                    if (k <= P::K && P::K < k + 16) r[P::K % 16] = __float_as_uint(bias_sum);
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                         reinterpret_cast<uint4 *>(dst + k)[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
@@ -578,7 +605,7 @@ int splits_of(ag_device *dev, const Shape &s) {
     return (int)(tiles < room ? tiles : room);
 }
 
-template <class P>
+template <class P, bool BIAS>
 int run_backward(ag_device *dev, const Shape &s, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, const uint32_t *codes,
                  float *partial) {
     using C = BCfg<P>;
@@ -586,10 +613,10 @@ int run_backward(ag_device *dev, const Shape &s, const __nv_bfloat16 *x, const _
     constexpr int smem = C::STAGES * C::STAGE + 1024;
     static_assert(smem >= kOneCtaPerSm && smem <= 226 * 1024, "one CTA per SM");
     static SmemAllowed allowed;
-    AG_TRY(allow_smem<smem>(dev, image_stage_backward_kernel<P>, allowed));
+    AG_TRY(allow_smem<smem>(dev, image_stage_backward_kernel<P, BIAS>, allowed));
     const int blocks = (int)(s.oc / 64), grid = splits_of(dev, s) * blocks;
-    return launch_dependent(dev, image_stage_backward_kernel<P>, dim3((unsigned)grid), B_THREADS, smem, p, dy, codes, blocks,
-                            partial);
+    return launch_dependent(dev, image_stage_backward_kernel<P, BIAS>, dim3((unsigned)grid), B_THREADS, smem, p, dy, codes,
+                            blocks, partial);
 }
 
 // `call` with the geometry's type, or -1.
@@ -629,11 +656,14 @@ int forward(ag_device *dev, const Shape &s, const __nv_bfloat16 *x, const __nv_b
 
 int64_t partial_floats(ag_device *dev, const Shape &s) { return 2ll * splits_of(dev, s) * s.oc * padded_k(s); }
 
-int backward(ag_device *dev, const Shape &s, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, const uint32_t *codes,
+int backward(ag_device *dev, const Shape &s, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, const uint32_t *codes, bool bias,
              float *partial) {
     AG_REQUIRE(takes(s) && (s.ih - s.fh + 1) % 2 == 0 && (s.iw - s.fw + 1) % 2 == 0, AG_ERR_UNSUPPORTED,
                "image stage: shape not taken");
-    return with_geometry(s, [&](auto g) { return run_backward<decltype(g)>(dev, s, x, dy, codes, partial); });
+    return with_geometry(s, [&](auto g) {
+        return bias ? run_backward<decltype(g), true>(dev, s, x, dy, codes, partial)
+                    : run_backward<decltype(g), false>(dev, s, x, dy, codes, partial);
+    });
 }
 
 int weight_gradient(ag_device *dev, const Shape &s, const float *partial, __nv_bfloat16 *dw) {

@@ -19,10 +19,10 @@ bool takes(const Shape &s);
 int forward(ag_device *dev, const Shape &s, const __nv_bfloat16 *x, const __nv_bfloat16 *w, const __nv_bfloat16 *bias,
             __nv_bfloat16 *y, uint32_t *codes);
 
-// The gradients of w and bias given dy [bs][ph][pw][oc] and the forward pass's codes, in two steps: f32 sums of
+// The gradients of w and (bias) of the bias given dy [bs][ph][pw][oc] and the forward pass's codes, in two steps: f32 sums of
 // slices of the batch (partial_floats of them), and their sum.  For even planes (the pool covers all cells).
 int64_t partial_floats(ag_device *dev, const Shape &s);
-int backward(ag_device *dev, const Shape &s, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, const uint32_t *codes,
+int backward(ag_device *dev, const Shape &s, const __nv_bfloat16 *x, const __nv_bfloat16 *dy, const uint32_t *codes, bool bias,
              float *partial);
 int weight_gradient(ag_device *dev, const Shape &s, const float *partial, __nv_bfloat16 *dw);
 int bias_gradient(ag_device *dev, const Shape &s, const float *partial, __nv_bfloat16 *db);

@@ -295,6 +295,45 @@ def test_stage_on_images(dev, ic, f, oc, bs, h, w, bias):
     model.close()
 
 
+@pytest.mark.parametrize("ic,f,oc", [(3, 3, 64), (4, 3, 64), (1, 5, 128), (2, 5, 64)])
+def test_bias_gradient_of_a_stage_on_images_is_a_sum_in_f32(dev, ic, f, oc):
+    """The bias gradient of a stage on images is the sum of a million gradients of one sign, 1024 images of 961 windows.  With
+    filters of zero every window passes its gradient, which the dense layer below makes: its first class is the target,
+    its second has all of the probability, so every image's gradient is the second class's weights / 1024.  They are chosen
+    for sums that lie 4e-6 above the middle of two bf16 values: one in f32 (a chain of some 210 in a thread, 32 threads and 148
+    CTAs, roundings of 2^-24 that walk) is rounded up, truncated additions, more than that short, are rounded down."""
+    import autograph_b200 as ag
+    bs, pooled = 1024, 31
+    size, windows = 2 * pooled + f - 1, pooled * pooled
+    spec = [("conv", ic, oc, (f, f), True), ("relu",), ("pool", (2, 2)), ("flatten",), ("dense", oc * windows, 2, False)]
+    rng = np.random.default_rng(7500 + oc)
+    w = oracle.round_bf16(rng.uniform(0.5, 1, (oc, windows)).astype(np.float32)) * 2.0 ** -rng.integers(0, 12, (oc, windows))
+    w = w.astype(np.float32)
+    w[:, -8:] = 0
+    want = np.empty(oc)
+    for c in range(oc):
+        total = w[c].astype(np.float64).sum()
+        ulp = 2.0 ** (np.floor(np.log2(total)) - 7)
+        low = np.floor(total / ulp) * ulp + ulp
+        ulp = 2.0 ** (np.floor(np.log2(low)) - 7)   # low may be the next power of two
+        rest = (low + ulp / 2) * (1 + 4e-6) - total
+        for i in range(8):   # bf16 pieces of what is missing, each rounded down
+            m, e = np.frexp(rest)
+            w[c, windows - 8 + i] = np.ldexp(np.floor(m * 256) / 256, e)
+            rest -= float(w[c, windows - 8 + i])
+        assert rest < 1e-12 * total and np.array_equal(w[c], oracle.round_bf16(w[c]))
+        want[c] = low + ulp
+    P = _params(spec, 7501, True)
+    P[0], P[1] = np.zeros_like(P[0]), np.ones_like(P[1])
+    P[2] = np.stack([np.zeros(oc * windows, np.float32), w.ravel()], axis=1)
+    model = ag.Model(dev, spec, torch.bfloat16, seed=1)
+    model.set_parameters(P)
+    x = torch.from_numpy(rng.integers(-2, 3, (bs, ic, size, size)).astype(np.float32)).to(torch.bfloat16)
+    model.train_step(x.pin_memory(), torch.zeros(bs, dtype=torch.uint8).pin_memory(), 0.01)
+    assert model.get_gradient(1).tolist() == want.tolist()
+    model.close()
+
+
 def test_wide_stack_full_batch_properties(dev):
     """Config 3 at its full batch 256: rows are independent, so the first 8 rows of the
     batch-256 forward equal the batch-8 forward."""
