@@ -72,10 +72,16 @@ using namespace ag;
 // 320 x 464 6.6 and 9.2; few tiles with a long k 192 x 3760 x 496 16.8 and 11.1, 240 x 1456 x 560 15.8 and 10.6, 336 x
 // 1216 x 1408 9.6 and 16.7, 176 x 8128 x 624 16.0 and 21.5, 720 x 4528 x 272 15.9 and 23.7.  Over 160 drawn products of
 // 5e6 to 2e9 multiply-adds these lines are 0.9 % above always taking the faster one.
-static bool tma_worth(int64_t m, int64_t k, int64_t n) {
+// One of their accumulators takes a whole slice of k, and the additions into it truncate (k = 4000, positive operands: 9e-6
+// short); the gathered engine reads one out after 1024 k.  So products with longer slices come here only from 1e9 (beyond
+// 32 tiles 2.5e8) multiply-adds on, though they would be faster here before that (256 x 4000 x 896 18.1 and 20.2, 512 x
+// 2048 x 640 11.9 and 15.5, 256 x 1536 x 2048 10.1 and 18.9; in slices of 1024 k 20.0, 17.8 and 16.6).
+static bool tma_worth(int64_t m, int64_t k, int64_t n, int sms) {
     const double macs = (double)m * (double)n * (double)k;
     if (!tcx::gemm_worth(AG_BF16, m, k, n)) return true;
-    if (k >= 1024 && ag::ceil_div(m, 128) * ag::ceil_div(n, 128) <= 16) return macs >= 6e8;
+    const int64_t tiles = ag::ceil_div(m, 128) * ag::ceil_div(n, 128);
+    if (tc::k_slices(sms, m, k, n).kb_per_split > 16) return macs >= (tiles <= 32 ? 1e9 : 2.5e8);
+    if (k >= 1024 && tiles <= 16) return macs >= 6e8;
     return macs >= 9e7;
 }
 
@@ -120,7 +126,7 @@ extern "C" int ag_dense_forward(ag_device *dev, ag_dtype dtype, const void *x, i
                                          fuse_relu != 0, (float *)y);
     const __nv_bfloat16 *px = (const __nv_bfloat16 *)x, *pw = (const __nv_bfloat16 *)w;
     __nv_bfloat16 *py = (__nv_bfloat16 *)y;
-    if (tma_worth(bs, inputs, outputs) &&
+    if (tma_worth(bs, inputs, outputs, dev->sm_count) &&
         tc::gemm_bf16_eligible(bs, inputs, outputs, px, inputs, 1, pw, outputs, 1, py, outputs, 1)) {
         // Large products go to the tensor cores with bias and relu in the kernel's epilogue
         // (a bias that is not 16-byte aligned is added by a separate pass).
@@ -367,7 +373,7 @@ extern "C" int ag_gemm(ag_device *dev, ag_dtype dtype, int64_t m, int64_t k, int
     const __nv_bfloat16 *pa = (const __nv_bfloat16 *)a + off_a;
     const __nv_bfloat16 *pb = (const __nv_bfloat16 *)b + off_b;
     __nv_bfloat16 *pc = (__nv_bfloat16 *)c + off_c;
-    if (tma_worth(m, k, n) && tc::gemm_bf16_eligible(m, k, n, pa, rsa, csa, pb, rsb, csb, pc, rsc, csc))
+    if (tma_worth(m, k, n, dev->sm_count) && tc::gemm_bf16_eligible(m, k, n, pa, rsa, csa, pb, rsb, csb, pc, rsc, csc))
         return tc::gemm_bf16(dev, (int)m, (int)k, (int)n, alpha, pa, rsa, csa, pb, rsb, csb, beta,
                              pc, rsc, csc);
     if (tensor_core)

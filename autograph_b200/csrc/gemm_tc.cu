@@ -421,6 +421,22 @@ static int launch(ag_device *dev, const CUtensorMap &ta, const CUtensorMap &tb, 
     return AG_OK;
 }
 
+// Few output tiles and a long k (a Dense layer with tens of thousands of inputs at a
+// small batch): slices of k become work items so that the whole GPU is used.  A shorter k is
+// worth the reduction's second launch only for a handful of tiles (200 x 3000 x 400 on four
+// tiles: 28 -> 15.5 us; 512 x 1024 x 512 on eight: 11.3 us whole, 13.2 us in slices).
+KSlices k_slices(int sm_count, int64_t m, int64_t k, int64_t n) {
+    const int64_t out_tiles = ceil_div(m, BLOCK_M) * ceil_div(n, BLOCK_N), total_kb = ceil_div(k, BLOCK_K);
+    int64_t splits = 1;
+    if (out_tiles * (total_kb >= 64 ? 4 : 32) <= sm_count && total_kb >= 16) {
+        splits = sm_count / out_tiles;
+        if (splits > total_kb / 4) splits = total_kb / 4;  // at least four k blocks per slice
+        if (splits < 1) splits = 1;
+    }
+    const int64_t kb_per_split = ceil_div(total_kb, splits);
+    return {(int)ceil_div(total_kb, kb_per_split), (int)kb_per_split};
+}
+
 int gemm_bf16(ag_device *dev, int m, int k, int n, float alpha, const __nv_bfloat16 *a,
               int64_t rsa, int64_t csa, const __nv_bfloat16 *b, int64_t rsb, int64_t csb,
               float beta, __nv_bfloat16 *c, int64_t rsc, int64_t csc, const Epilogue *epi) {
@@ -429,20 +445,7 @@ int gemm_bf16(ag_device *dev, int m, int k, int n, float alpha, const __nv_bfloa
     if (epi) AG_REQUIRE(alpha == 1.f && beta == 0.f, AG_ERR_INVALID, "fused epilogue needs alpha 1, beta 0");
     if (epi && epi->bias)
         AG_REQUIRE((reinterpret_cast<uintptr_t>(epi->bias) & 15) == 0, AG_ERR_INVALID, "bias not 16-byte aligned");
-    // Few output tiles and a long k (a Dense layer with tens of thousands of inputs at a
-    // small batch): slices of k become work items so that the whole GPU is used.  A shorter k is
-    // worth the reduction's second launch only for a handful of tiles (200 x 3000 x 400 on four
-    // tiles: 28 -> 15.5 us; 512 x 1024 x 512 on eight: 11.3 us whole, 13.2 us in slices).
-    const int out_tiles = (int)(ceil_div(m, BLOCK_M) * ceil_div(n, BLOCK_N));
-    const int total_kb = (int)ceil_div(k, BLOCK_K);
-    int splits = 1, kb_per_split = total_kb;
-    if (out_tiles * (total_kb >= 64 ? 4 : 32) <= dev->sm_count && total_kb >= 16) {
-        splits = dev->sm_count / out_tiles;
-        if (splits > total_kb / 4) splits = total_kb / 4;  // at least four k blocks per slice
-        if (splits < 1) splits = 1;
-        kb_per_split = (int)ceil_div(total_kb, splits);
-        splits = (int)ceil_div(total_kb, kb_per_split);
-    }
+    const auto [splits, kb_per_split] = k_slices(dev->sm_count, m, k, n);
     if (splits == 1 && gemm_bf16_pair_enabled() && m >= 256 && n >= 256)
         return gemm_bf16_pair(dev, m, k, n, alpha, a, rsa, csa, b, rsb, csb, beta, c, rsc, csc, epi);
     const bool a_mn = !(csa == 1 && rsa % 8 == 0 && rsa >= k);  // else contiguous along m

@@ -21,6 +21,12 @@ struct Epilogue {
     bool relu;
 };
 
+// The slices of k that gemm_bf16 makes work items of, in 64-wide blocks of k.  One accumulator takes a whole slice.
+struct KSlices {
+    int splits, kb_per_split;
+};
+KSlices k_slices(int sm_count, int64_t m, int64_t k, int64_t n);
+
 int gemm_bf16(ag_device *dev, int m, int k, int n, float alpha, const __nv_bfloat16 *a,
               int64_t rsa, int64_t csa, const __nv_bfloat16 *b, int64_t rsb, int64_t csb,
               float beta, __nv_bfloat16 *c, int64_t rsc, int64_t csc,

@@ -144,3 +144,22 @@ def test_dense_epilogue_fused_on_the_tensor_cores(dev, shape, with_bias, relu):
     if relu:
         ref = np.maximum(ref, 0)
     assert np.abs(y.float().cpu().numpy() - ref).max() <= 1e-2 * max(np.abs(ref).max(), 1e-6)
+
+
+@pytest.mark.parametrize("m,k,n", [(256, 4000, 896), (512, 2048, 640), (512, 3000, 512), (256, 8192, 384), (384, 1088, 1024)])
+def test_long_sums_are_not_cut_short(dev, m, k, n):
+    """tcgen05.mma adds with truncation, so a long sum of positive products in one accumulator comes out short.  Against
+    float64 rounded to bf16 the mean error, over outputs of several powers of two, is what more of them rounded down leave: at
+    most 64 additions (k = 1024) that lose half a unit in the last place, 2^-24 of a value."""
+    gen = torch.Generator(device=dev.torch_device).manual_seed(m + k + n)
+
+    def positive(rows, cols):
+        scale = torch.rand((rows, 1), generator=gen, device=dev.torch_device).mul_(3).exp2_()
+        return torch.rand((rows, cols), generator=gen, device=dev.torch_device).add_(1).mul_(scale).to(torch.bfloat16)
+
+    a, b = positive(m, k), positive(n, k).t().contiguous()
+    got = dev.dot(a, b).double()
+    exact = a.double() @ b.double()
+    dev.wait()
+    short = ((got - exact.to(torch.bfloat16).double()) / exact).mean().item()
+    assert abs(short) <= 64 * 2.0 ** -24, short
