@@ -411,49 +411,45 @@ int chain_weight_grads(ag_device *dev, int m, int n, WgradProblem *problems) {
     return AG_OK;
 }
 
-// C[m][n] = sum over k of A[k][m] . B[k][n], n <= NP: the weight gradient of a layer with few outputs.  A lane owns a
+// C[m][n] = sum over k of A[k][m] . B[k][n], k <= kFewK, n <= NP: the weight gradient of a layer with few outputs.  A lane owns a
 // column of A and all of B's, so A is read once, coalesced, and B comes from shared memory for the whole warp; the sixteen
 // warps take every sixteenth k and their sums are added in warp order.
-constexpr int kColWarps = 16, kColChunk = 512;
+constexpr int kColWarps = 16;
 template <class T, int NP>
 __global__ void __launch_bounds__(kColWarps * 32)
     few_columns_kernel(const T *__restrict__ a, int64_t lda, const T *__restrict__ b, int64_t ldb, T *__restrict__ c,
                        int64_t ldc, int M, int K, int N) {
     let_dependents_launch();
     dependency_wait();
-    constexpr int kFloats = kColWarps * NP * 33 > kColChunk * NP ? kColWarps * NP * 33 : kColChunk * NP;
-    __shared__ __align__(16) float buf[kFloats];   // [chunk][NP] of B, then [warp][NP][33] sums
+    constexpr int kFloats = kColWarps * NP * 33 > kFewK * NP ? kColWarps * NP * 33 : kFewK * NP;
+    __shared__ __align__(16) float buf[kFloats];   // [k][NP] of B, then [warp][NP][33] sums
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, m = blockIdx.x * 32 + lane;
     float acc[NP];
 #pragma unroll
     for (int j = 0; j < NP; ++j) acc[j] = 0.f;
-    for (int kc = 0; kc < K; kc += kColChunk) {
-        const int n_k = min(kColChunk, K - kc);
-        if (kc > 0) __syncthreads();
-        for (int i = threadIdx.x; i < n_k * NP; i += kColWarps * 32) {
-            const int k = i / NP, j = i % NP;
-            buf[i] = load_or_zero(b + (int64_t)(kc + k) * ldb + j, j < N);
+    for (int i = threadIdx.x; i < K * NP; i += kColWarps * 32) {
+        const int k = i / NP, j = i % NP;
+        buf[i] = load_or_zero(b + (int64_t)k * ldb + j, j < N);
+    }
+    __syncthreads();
+    for (int k0 = warp; k0 < K; k0 += 8 * kColWarps) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int k = k0 + u * kColWarps;
+            v[u] = load_or_zero(a + (int64_t)k * lda + m, k < K && m < M);
         }
-        __syncthreads();
-        for (int k0 = warp; k0 < n_k; k0 += 8 * kColWarps) {
-            float v[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int k = k0 + u * kColWarps;
-                v[u] = load_or_zero(a + (int64_t)(kc + k) * lda + m, k < n_k && m < M);
-            }
+        for (int u = 0; u < 8; ++u) {
+            const int k = k0 + u * kColWarps;
+            if (k >= K) break;   // what shared memory holds there may be anything
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int k = k0 + u * kColWarps;
-                if (k >= n_k) break;   // what shared memory holds there may be anything
-#pragma unroll
-                for (int j = 0; j < NP; j += 4) {
-                    const float4 w = *reinterpret_cast<const float4 *>(buf + k * NP + j);
-                    acc[j] = fmaf(v[u], w.x, acc[j]);
-                    acc[j + 1] = fmaf(v[u], w.y, acc[j + 1]);
-                    acc[j + 2] = fmaf(v[u], w.z, acc[j + 2]);
-                    acc[j + 3] = fmaf(v[u], w.w, acc[j + 3]);
-                }
+            for (int j = 0; j < NP; j += 4) {
+                const float4 w = *reinterpret_cast<const float4 *>(buf + k * NP + j);
+                acc[j] = fmaf(v[u], w.x, acc[j]);
+                acc[j + 1] = fmaf(v[u], w.y, acc[j + 1]);
+                acc[j + 2] = fmaf(v[u], w.z, acc[j + 2]);
+                acc[j + 3] = fmaf(v[u], w.w, acc[j + 3]);
             }
         }
     }
@@ -473,6 +469,7 @@ __global__ void __launch_bounds__(kColWarps * 32)
 
 template <class T>
 int few_columns(ag_device *dev, int m, int k, int n, const T *a, int64_t lda, const T *b, int64_t ldb, T *c, int64_t ldc) {
+    AG_REQUIRE(k <= kFewK && n <= kFewColumns, AG_ERR_LIMIT, "product has too many columns or too long a k");
     const dim3 grid((unsigned)ceil_div(m, 32));
     auto kernel = n <= 4 ? few_columns_kernel<T, 4> : n <= 8 ? few_columns_kernel<T, 8>
                 : n <= 12 ? few_columns_kernel<T, 12> : few_columns_kernel<T, 16>;

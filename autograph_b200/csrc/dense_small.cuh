@@ -22,8 +22,8 @@ template <class T>
 int forward(ag_device *dev, const T *x, int m, int k, const T *w, int n, const T *bias, bool relu,
             T *y);
 
-// c[m,n] = a^T . b, a [k,m], b [k,n], c [m,n], rows lda, ldb, ldc apart; n <= 16.
-constexpr int kFewColumns = 16;
+// c[m,n] = a^T . b, a [k,m], b [k,n], c [m,n], rows lda, ldb, ldc apart; k <= kFewK, n <= kFewColumns.
+constexpr int kFewK = 512, kFewColumns = 16;
 template <class T>
 int few_columns(ag_device *dev, int m, int k, int n, const T *a, int64_t lda, const T *b, int64_t ldb, T *c, int64_t ldc);
 

@@ -93,7 +93,7 @@ static bool tma_worth(int64_t m, int64_t k, int64_t n, int sms) {
 // f32 with k up to 128 stays: there are fewer roundings in its sums (k = 32: 4.5e-8 and here 6.1e-8 in relative 2-norm; k =
 // 256: 6.9e-8 and 6.1e-8).
 static bool few_columns_worth(ag_dtype dtype, int64_t m, int64_t k, int64_t n, int sms) {
-    if (n > dense_small::kFewColumns || k > 512 || k < (dtype == AG_F32 ? 129 : 32)) return false;
+    if (n > dense_small::kFewColumns || k > dense_small::kFewK || k < (dtype == AG_F32 ? 129 : 32)) return false;
     return ag::ceil_div(m, 32) <= sms || (dtype == AG_F32 ? n <= 4 : k >= 100);
 }
 

@@ -215,3 +215,25 @@ def test_products_with_few_columns(dev, dtype, m, k, n):
         bound = bound + 2.0 ** -8 * ref.abs()
     assert bool(((cv.double() - ref).abs() <= bound).all())
     assert bool((c[:, n] == 7.0).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m,k,n", [(33, 511, 5), (512, 256, 10), (31, 512, 12)])
+def test_products_with_few_columns_and_values_that_are_not_finite(dev, dtype, m, k, n):
+    """One launch, and infinities and NaNs reach the outputs that they reach in float64 and no others: column 0 of b is zero, and
+    what a warp's last group of eight k has beyond k multiplies nothing."""
+    import autograph_b200 as ag
+    rng = torch.Generator().manual_seed(m * 1000 + k + n)
+    a = torch.empty((k, m)).uniform_(-1, 1, generator=rng).to(dtype).cuda(dev.torch_device)
+    b = torch.empty((k, n)).uniform_(-1, 1, generator=rng).to(dtype).cuda(dev.torch_device)
+    b[:, 0] = 0
+    a[7, 3], a[k - 1, 20], a[k // 2, 11] = float("inf"), float("-inf"), float("nan")
+    b[k - 2, n - 1] = float("inf")
+    launches = ag.kernel_launch_count()
+    c = dev.dot(a.t(), b).double()
+    assert ag.kernel_launch_count() - launches == 1
+    ref = a.double().t() @ b.double()
+    dev.wait()
+    assert torch.equal(c.isnan(), ref.isnan()) and torch.equal(c.isposinf(), ref.isposinf()) and torch.equal(c.isneginf(), ref.isneginf())
+    ok = ref.isfinite()
+    assert bool(((c - ref).abs()[ok] <= (2.0 ** -8 if dtype == torch.bfloat16 else 1e-5) * (1 + ref.abs()[ok])).all())
