@@ -231,6 +231,11 @@ STAGE_SPECS = {
         ("conv", 3, 16, (5, 5), True), ("relu",), ("pool", (2, 2)),
         ("conv", 16, 64, (3, 3), True), ("relu",), ("pool", (2, 2)),
         ("flatten",), ("dense", 64 * 13 * 13, 32, False), ("relu",), ("dense", 32, 10, True)]),
+    # the last pool and its gradient with sixteen channels a block, odd planes
+    "sixteen_channels_a_block": (40, 26, [
+        ("conv", 3, 16, (3, 3), True), ("relu",), ("pool", (2, 2)),
+        ("conv", 16, 64, (2, 2), True), ("relu",), ("pool", (2, 2)),
+        ("flatten",), ("dense", 64 * 5 * 5, 32, False), ("relu",), ("dense", 32, 10, True)]),
     # a run of two stages: patches first layer with bias, odd second plane (17 x 17 -> 8 x 8)
     "two_stages_bias_odd": (16, 40, [
         ("conv", 3, 64, (3, 3), True), ("relu",), ("pool", (2, 2)),
@@ -293,6 +298,104 @@ def test_stage_on_images(dev, ic, f, oc, bs, h, w, bias):
     for i, g in enumerate(grads):
         assert _rel(model.get_gradient(i), g.ravel()) <= 2 ** -6, i
     model.close()
+
+
+def test_last_pool_writes_the_same_with_any_channels_a_block(dev):
+    """The pool that writes NCHW takes 64, 16 or 8 channels of an image per block, by the batch: rows are independent, so a small
+    batch's are the large one's."""
+    import autograph_b200 as ag
+    model = ag.Model(dev, [("conv", 16, 64, (3, 3), True), ("relu",), ("pool", (2, 2)), ("flatten",),
+                           ("dense", 64 * 12 * 12, 64 * 12, False)], torch.bfloat16, seed=5)
+    gen = torch.Generator(device=dev.torch_device).manual_seed(5)
+    x = torch.randn((300, 16, 27, 27), generator=gen, device=dev.torch_device).to(torch.bfloat16)
+    rows = {}
+    for bs in (300, 40, 8):
+        out = dev.empty((bs, 64 * 12), torch.bfloat16)
+        rows[bs] = model.forward_device(x[:bs].contiguous(), out)[:8].clone()
+    dev.wait()
+    # the dense layer's products of these batches may be other engines': a rounding of the logits
+    scale = rows[300].float().abs().max()
+    for bs in (40, 8):
+        assert bool(((rows[bs].float() - rows[300].float()).abs() <= 2.0 ** -8 * scale).all())
+    model.close()
+
+
+@pytest.mark.parametrize("h,w", [(34, 34), (33, 41)])
+def test_stage_on_images_with_pixels_that_are_not_finite(dev, h, w):
+    """A convolution of an infinity or a NaN that is NaN or negative is 0 after the Relu, a positive infinity wins its window.
+    Every pooled value around the pixels, ten at a time through a dense layer that picks them."""
+    import autograph_b200 as ag
+    ph, pw, oc = (h - 2) // 2, (w - 2) // 2, 64
+    rng = np.random.default_rng(7600)
+    x = rng.integers(-2, 3, (8, 3, h, w)).astype(np.float32)
+    x[1, 0, 5, 6], x[2, 2, 7, 8] = -np.inf, np.nan
+    weight = rng.integers(1, 3, (oc, 3, 3, 3)).astype(np.float32)
+    weight[::2] = rng.integers(-2, 1, weight[::2].shape)
+    bias = rng.integers(-3, 4, oc).astype(np.float32)
+
+    def pooled(x):
+        y = torch.nn.functional.conv2d(*(torch.from_numpy(v).double() for v in (x, weight, bias)))
+        return torch.nn.functional.max_pool2d(torch.where(y >= 0, y, torch.zeros_like(y)), 2).reshape(len(x), -1)
+
+    spec = [("conv", 3, oc, (3, 3), True), ("relu",), ("pool", (2, 2)), ("flatten",), ("dense", oc * ph * pw, 10, False)]
+    model = ag.Model(dev, spec, torch.bfloat16, seed=1)
+
+    def logits(x, dense):
+        model.set_parameters([weight, bias, dense])
+        return model.infer(torch.from_numpy(x).to(torch.bfloat16).pin_memory()).double()
+
+    # with filters of both signs +inf meets either: the image's sum is infinite, and not NaN
+    hot = x.copy()
+    hot[0, 1, 10, 11], hot[1, 0, 5, 6], hot[2, 2, 7, 8] = np.inf, 1, 1
+    assert bool(pooled(hot)[0].isposinf().any()) and not bool(pooled(hot).isnan().any())
+    ones = np.ones((oc * ph * pw, 10), np.float32)
+    got = logits(hot, ones)
+    assert bool(got[0].isposinf().all()) and bool(got[1:].isfinite().all())
+    # -inf with negative filters: the same for image 1
+    assert bool(logits(x, ones)[1].isposinf().all())
+    cold = x.copy()
+    cold[1] = x[2]   # images of a NaN
+    around = [(c * ph + y) * pw + z for c in range(0, oc, 7) for y in (2, 3) for z in (3, 4)]
+    for i in range(0, len(around), 10):
+        pick = np.zeros((oc * ph * pw, 10), np.float32)
+        for j, at in enumerate(around[i:i + 10]):
+            pick[at, j] = 1
+        got = logits(cold, pick)
+        assert torch.equal(got[:, :len(around[i:i + 10])], pooled(cold)[:, around[i:i + 10]])
+    model.close()
+
+
+def test_stage_on_images_with_gradients_that_are_not_finite(dev):
+    """A pixel of -inf under positive filters is 0 after the Relu and passes no gradient, but 0 times it is NaN: the weight
+    gradients of its channel, and no others.  Gradients of NaN reach the filters and biases whose windows pass them."""
+    import autograph_b200 as ag
+    bs, oc, pooled = 8, 64, 16
+    spec = [("conv", 3, oc, (3, 3), True), ("relu",), ("pool", (2, 2)), ("flatten",), ("dense", oc * pooled ** 2, 10, True)]
+    P = _params(spec, 7700, True)
+    rng = np.random.default_rng(7701)
+    P[0] = rng.integers(1, 3, P[0].shape).astype(np.float32)
+    P[1] = np.where(np.arange(oc) < 32, -1000, 3).astype(np.float32)   # the first half passes nothing
+    x = rng.integers(0, 3, (bs, 3, 34, 34)).astype(np.float32)
+    t = rng.integers(0, 10, bs).astype(np.uint8)
+
+    def gradients(x, P):
+        model = ag.Model(dev, spec, torch.bfloat16, seed=1)
+        model.set_parameters(P)
+        model.train_step(torch.from_numpy(x).to(torch.bfloat16).pin_memory(), torch.from_numpy(t).pin_memory(), 0.01)
+        dw, db = model.get_gradient(0).reshape(oc, 3, 9), model.get_gradient(1)
+        model.close()
+        return dw, db
+
+    bad = x.copy()
+    bad[3, 1, 12, 15] = -np.inf
+    dw, db = gradients(bad, P)
+    assert np.isnan(dw[:, 1]).all()
+    assert np.isfinite(dw[:, (0, 2)]).all() and np.isfinite(db).all()
+    assert (dw[:32][:, (0, 2)] == 0).all() and (db[:32] == 0).all() and (db[32:] != 0).all()
+    P[-1][4] = np.nan   # a bias of the logits
+    dw, db = gradients(x, P)
+    assert (dw[:32] == 0).all() and (db[:32] == 0).all()
+    assert np.isnan(dw[32:]).all() and np.isnan(db[32:]).all()
 
 
 @pytest.mark.parametrize("ic,f,oc", [(3, 3, 64), (4, 3, 64), (1, 5, 128), (2, 5, 64)])
