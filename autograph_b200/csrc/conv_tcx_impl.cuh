@@ -127,15 +127,27 @@ static int launch_split(ag_device *dev, const SplitJob<T> &a, const SplitJob<T> 
 // its launch want a long patch and some work: f32 64 x 16 x 32 -> 32 3x3 (144 values) forward 27 and 24, 13 x 6 x 39 -> 32
 // 16 and 12, 11 x 32 x 40 -> 6 3x3 14 and 12, input gradient 5 x 32 x 42 -> 96 20.7 and 18.3; the weight gradient's second
 // tensor wants more of it (37 x 6 x 52 -> 128 5x5, 200 values, 119 and 89).  Planes beyond what stays in L2 are read again
-// per tap from memory: f32 171 x 64 x 42 -> 16 (116 MB) 237 and 211.  Over 70 drawn convolutions the affected passes take
-// 0.94 (f32 forward), 0.94, 0.86 and (bf16) 0.93, 0.97, 0.87 of their time.
+// per tap from memory: f32 171 x 64 x 42 -> 16 (116 MB) 237 and 211.
+// A pass costs some 4 us per 10 MB of planes, and an element that is not gathered saves 4e-7 us (bf16 2e-7) per 128 columns, so the
+// elements that would be gathered are held against the bytes of the planes.  Few reads of each, with a stride or a filter of
+// few taps, make no gain but in f32 tiles of more than 80 columns or with a long patch (forward 153 x 64 x 30 -> 6 3x3 / 2 f32 45
+// and 32, 107 x 32 x 47 -> 64 3x3 / 2 42 and 35, its weight gradient 58 and 50, 15 x 96 x 63 x 50 -> 36 1x3 37 and 31, bf16 215 x 91
+// x 10 x 32 -> 62 3x1 / 2x1 23 and 18; from 32 channels into 96 3x3 / 2 85 and 94), nor do channels that are mostly padding (42 x 6 x
+// 57 -> 32 5x5 56 and 52) or a short patch and little work (input gradient 49 x 45 x 25 x 30 -> 11 5x3 / 2x1 24 and 22).  With a
+// dilation the pieces of a row of taps lie apart (80 x 18 x 58 x 60 -> 31 5x3 dilated 97 and 70).  Over 627 passes of 500 drawn
+// convolutions, a third of them with strides of two and a third dilated, the time is 0.866 of gathering, 0.864 if each took the
+// faster form, the worst 1.10; by patch, planes and work alone it was 0.874 and 1.40.
 template <class T>
-static bool split_worth(const ConvMap &g, int64_t bytes, int64_t positions, int64_t n, int least_patch) {
-    const int64_t patch = (int64_t)g.ff * g.cp;
-    // few columns are little work per element: with a stride, which makes few patches of them, not enough (136 x 64 x 24 ->
-    // 6 / 2 f32 36 and 31)
-    if (sizeof(T) == 4 && n < 32 && positions * patch * 48 < 8 * bytes) return false;
-    return patch >= least_patch && bytes <= 80000000 && positions * patch * (n < 32 ? 32 : n) >= 300000000;
+static bool split_worth(const ConvMap &g, int64_t bytes, int tensors, int64_t positions, int64_t n, int least_patch) {
+    const bool f32 = sizeof(T) == 4, wide = n > 80;
+    const int64_t patch = (int64_t)g.ff * g.cp, work = positions * patch * (n < 32 ? 32 : n);
+    if (patch < least_patch || bytes > 80000000 || work < 300000000) return false;
+    if (!wide && patch < 270 && work < 500000000) return false;
+    if (f32 && !wide && tensors == 1 && g.ff * g.channels < 200) return false;
+    double least = wide ? (f32 ? 0.33 : 0.9) : !f32 ? (tensors == 1 ? 1.75 : 2) : patch < 600 || tensors == 2 ? 1 : 0.6;
+    if (g.dil_w > 1 && g.cp <= 64) least *= 2;
+    if (tensors == 1 && bytes > 60000000 && least < 1) least = 1;
+    return (double)(positions * patch * ceil_div(n, 128) * tensors) >= least * (double)bytes;
 }
 
 // The map that counts positions instead of elements.
@@ -195,7 +207,7 @@ static int patches_times_filters(ag_device *dev, const T *src, int64_t images, c
     const int64_t hw = (int64_t)map.sh * map.sw;
     SplitJob<T> x = split_job(src, images, map.channels * hw, (int64_t)map.channels, hw, hw);
     SplitJob<T> f = split_job(w, (int64_t)N, (int64_t)s_row, (int64_t)map.channels, (int64_t)s_c, (int64_t)map.ff);
-    if (split_worth<T>(map, split_bytes(x), M, N, 200) && split_scratch(dev, &x, &f)) {
+    if (split_worth<T>(map, split_bytes(x), 1, M, N, 200) && split_scratch(dev, &x, &f)) {
         AG_TRY(launch_split<T>(dev, x, f));
         return gemm<T>(dev, M, N, K, SplitRows<T>{{x.dst, x.plane}, of_positions(map), x.div_groups, x.groups, {src, map, M}},
                        SplitFilters<T>{{f.dst, f.plane}, K / 8, {w, s_row, s_c, map.channels, map.div_cp}}, E);
@@ -343,7 +355,7 @@ int conv_backward_weight(ag_device *dev, const T *x, int64_t bs, int64_t ic, int
     const int M = map.ff * map.cp;
     SplitJob<T> jx = split_job(x, bs, ic * ih * iw, ic, ih * iw, ih * iw);
     SplitJob<T> jy = split_job(dy, bs, oc * hw, oc, (int64_t)hw, (int64_t)hw);
-    if (split_worth<T>(map, split_bytes(jx) + split_bytes(jy), K, N, 288) && split_scratch(dev, &jx, &jy)) {
+    if (split_worth<T>(map, split_bytes(jx) + split_bytes(jy), 2, K, N, 288) && split_scratch(dev, &jx, &jy)) {
         AG_TRY(launch_split<T>(dev, jx, jy));
         return gemm<T>(dev, M, N, K, SplitCols<T>{{jx.dst, jx.plane}, of_positions(map), jx.div_groups, jx.groups, {x, map, M}},
                        SplitChannels<T>{{jy.dst, jy.plane}, jy.groups, {dy, N, hw, FastDiv((uint32_t)hw)}},
