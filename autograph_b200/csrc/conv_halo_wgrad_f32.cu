@@ -363,14 +363,17 @@ int launch_wgrad(ag_device *dev, const WgradPlan &l, int grid, const WgradParams
 // It pads channels and columns and has two launches: 17 x 16 x 22 -> 32 5 x 5 13.7 and 18.0, 5 x 64 x 47 -> 32 21.9 and 25.4 (61 x 64
 // x 31 -> 32 57 and 45), 136 x 1 x 57 -> 32 5 x 5 70 and 123, 14 x 64 x 10 -> 6 9.9 and 12.7.  With 64 columns a tile's sums are 96
 // registers a thread and its boxes leave two stages: 72 x 16 x 57 -> 64 100 and 97, 130 x 6 x 42 -> 64 48 and 78, so
-// there are none.  Over 170 drawn convolutions the gradients that come here take 0.62 of their time and none more than it.
+// there are none.  One channel with 5 x 5 filters is a sixteenth of its rows and slower here (121 x 1 x 43 -> 16 42.9 and 45.2), and
+// so are few positions of many channels (50 x 64 x 12 -> 16 13.9 and 15.3).  Over 331 drawn gradients those that come here take
+// 0.69 of their time, all but one (278 x 3 x 17 x 45 -> 6 5 x 1, 35.7 and 39.6) at most 1.02.
 // Errors against float64 are 0.35 to 0.86 of the gathered engine's over 106 drawn gradients.
 bool takes_wgrad(const Wgrad &p) {
     WgradPlan l;
     if (!make_wgrad_plan(p, &l)) return false;
     const int64_t positions = p.bs * p.oh * p.ow;
     if (2 * p.oh * p.ow < l.hp * l.wp) return false;   // rows of the frame that are outputs
-    if (p.n <= 16) return positions >= 4000;
+    if (p.channels == 1 && p.fh * p.fw >= 25) return false;
+    if (p.n <= 16) return positions >= (p.channels > 32 ? 6000 : 4000);
     return p.channels > 4 && positions >= (p.channels > 32 || p.fh * p.fw > 9 ? 40000 : 10000);
 }
 
