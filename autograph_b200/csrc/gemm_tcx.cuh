@@ -884,11 +884,20 @@ __device__ __forceinline__ void reduce_tile(const Params &p, const Epi &E, int m
     }
 }
 
+// Whether CTAs of this kernel add slices themselves.  Operands of few channels have three steps of k at most, which are never
+// sliced: the code for it cost their bf16 kernels spills (47 x 3 x 15 x 21 -> 121 1x3 7.0 us, 6.5 without).
+template <class AOp>
+constexpr bool kShortK = false;
+template <class T>
+constexpr bool kShortK<FewRows<T>> = true;
+template <class AOp, class Epi>
+constexpr bool kAddsSlices = Epi::kLastCtaAdds && !kShortK<AOp>;
+
 // First work item of a CTA; item w is slice w / tiles of tile w % tiles, and the slices of a tile are neighbouring CTAs
 // where they are a cluster.
-template <class Epi>
+template <bool ADDS>
 __device__ __forceinline__ int first_item(const Params &p) {
-    if (Epi::kLastCtaAdds && p.cluster) return (int)(blockIdx.x % (unsigned)p.splits) * p.tiles_m * p.tiles_n + (int)(blockIdx.x / (unsigned)p.splits);
+    if (ADDS && p.cluster) return (int)(blockIdx.x % (unsigned)p.splits) * p.tiles_m * p.tiles_n + (int)(blockIdx.x / (unsigned)p.splits);
     return p.work0 + (int)blockIdx.x;
 }
 
@@ -899,7 +908,8 @@ __device__ __noinline__ void redo_marked(const AOp &A, const BOp &B, const Epi &
     constexpr int WARPS = C::THREADS / 32, BLOCKS = C::EPI_WARPS * C::COLS / 32;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, tiles = p.tiles_m * p.tiles_n;
     int turn = 0;
-    for (int w = first_item<Epi>(p), i = 0; w < p.work1; w += gridDim.x, ++i) {
+    constexpr bool ADDS = kAddsSlices<AOp, Epi>;
+    for (int w = first_item<ADDS>(p), i = 0; w < p.work1; w += gridDim.x, ++i) {
         const unsigned mark = marks[i / 4] >> (i % 4 * 8) & 255u;
         const int tile = w % tiles, z = w / tiles;
         const int k_begin = z * p.k_split, k_end = min(p.K, k_begin + p.k_split);
@@ -918,7 +928,7 @@ __device__ __noinline__ void redo_marked(const AOp &A, const BOp &B, const Epi &
                 for (int c = 0; c < 8; ++c) {
                     if (col + c >= p.N) break;
                     const float v = r == 0 ? acc[0][c] : r == 1 ? acc[1][c] : r == 2 ? acc[2][c] : acc[3][c];
-                    if (Epi::kLastCtaAdds && p.cluster)
+                    if (ADDS && p.cluster)
                         sums[(col + c) % C::BN * BM + (row + r) % BM] = v;
                     else if (p.splits > 1)
                         p.partial[((int64_t)z * p.N + col + c) * p.M + row + r] = v;
@@ -936,6 +946,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
                     const __grid_constant__ Epi E, const __grid_constant__ Params p) {
     using C = Cfg<T, BN>;
     constexpr int PL = C::PL, STAGES = C::STAGES, PRODUCERS = C::PRODUCERS;
+    constexpr bool ADDS = kAddsSlices<AOp, Epi>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                                 ~uintptr_t(1023));
@@ -992,11 +1003,11 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
     // The k slices of a convolution (its weight gradient) on every SM let dependents launch at their end: 16 -> 32 3x3,
     // 64 x 32 x 32 f32, 40.0 us at the start, 33.8 so; with an SM left free they gain as all others do (8 x 6 x 20 x 20
     // -> 16 5x5, stride 2, f32: 12.1, at the end 12.9).
-    let_dependents_launch(Epi::kLastCtaAdds && p.splits > 1 ? 147u : kAlwaysEarly);
+    let_dependents_launch(ADDS && p.splits > 1 ? 147u : kAlwaysEarly);
     dependency_wait();
 
     const int tiles = p.tiles_m * p.tiles_n;
-    const int num_work = p.work1, work0 = first_item<Epi>(p);
+    const int num_work = p.work1, work0 = first_item<ADDS>(p);
 
     if (warp < PRODUCERS / 32) {
         // ------------------------------------------------------------------ producers
@@ -1250,7 +1261,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
                 }
             }
             if (redo_it) {
-            } else if (Epi::kLastCtaAdds && p.cluster) {
+            } else if (ADDS && p.cluster) {
                 // the stages have been read: this CTA's products are done
                 float *q = sums + col_base * BM + quarter * 32 + lane;
 #pragma unroll
@@ -1284,7 +1295,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
         redo_marked<C, AOp, BOp, Epi>(A, B, E, p, marks, reinterpret_cast<float *>(smem) + warp * kRedoFloats, sums);
         __syncthreads();
     }
-    if (Epi::kLastCtaAdds && p.cluster) {
+    if (ADDS && p.cluster) {
         // Every CTA adds a share of the columns over the slices, in slice order as reduce_splits_kernel does.
         tc::pair::cluster_sync();
         const int tile = work0 % tiles, rank = work0 / tiles;
@@ -1306,7 +1317,7 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
         tc::pair::cluster_sync();   // the others have read this CTA's sums
         return;
     }
-    if (Epi::kLastCtaAdds && p.arrivals != nullptr) {
+    if (ADDS && p.arrivals != nullptr) {
         // every CTA has had one slice of one tile (grid = tiles * splits)
         const int tile = blockIdx.x % tiles;
         int *last = table_a;
@@ -1423,7 +1434,7 @@ int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
     // gradient, 35 steps each, 72 and 60), and so are products in a row, whose second launch overlaps the next one (464 x 256
     // x 112 bf16 8.6 and 7.2).
     p.cluster = 0;
-    if (Epi::kLastCtaAdds && p.splits > 1 && p.splits <= kMostCluster && per <= 16) {
+    if (kAddsSlices<AOp, Epi> && p.splits > 1 && p.splits <= kMostCluster && per <= 16) {
         static int room_on[64][kMostCluster + 1] = {};   // clusters + 1
         int &room = room_on[dev->ordinal & 63][p.splits];
         if (room == 0) AG_TRY(cluster_room(kernel, C::THREADS, C::SMEM, p.splits, &room));
@@ -1437,7 +1448,7 @@ int launch(ag_device *dev, const AOp &A, const BOp &B, const Epi &E, Params p) {
         // than the separate kernel (512^3 f32 13.8 us against 9.9), whose launch costs 4 us on the host; a pass
         // over a small convolution's edges is ten launches that the device waits for, a product by itself
         // is not.  More slices would be a chain of round trips (37 slices: 24 us against 13).
-        if (Epi::kLastCtaAdds && p.splits <= 8 && tiles <= kTileCounters &&
+        if (kAddsSlices<AOp, Epi> && p.splits <= 8 && tiles <= kTileCounters &&
             (int64_t)p.splits * (p.M < BM ? p.M : BM) * (p.N < BN ? p.N : BN) <= 65536)
             p.arrivals = dev->tile_counters;
     }
