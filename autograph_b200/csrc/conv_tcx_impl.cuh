@@ -130,23 +130,25 @@ static int launch_split(ag_device *dev, const SplitJob<T> &a, const SplitJob<T> 
 // per tap from memory: f32 171 x 64 x 42 -> 16 (116 MB) 237 and 211.
 // A pass costs some 4 us per 10 MB of planes, and an element that is not gathered saves 4e-7 us (bf16 2e-7) per 128 columns, so the
 // elements that would be gathered are held against the bytes of the planes.  Few reads of each, with a stride or a filter of
-// few taps, make no gain but in f32 tiles of more than 80 columns or with a long patch (forward 153 x 64 x 30 -> 6 3x3 / 2 f32 45
-// and 32, 107 x 32 x 47 -> 64 3x3 / 2 42 and 35, its weight gradient 58 and 50, 15 x 96 x 63 x 50 -> 36 1x3 37 and 31, bf16 215 x 91
-// x 10 x 32 -> 62 3x1 / 2x1 23 and 18; from 32 channels into 96 3x3 / 2 85 and 94), nor do channels that are mostly padding (42 x 6 x
-// 57 -> 32 5x5 56 and 52) or a short patch and little work (input gradient 49 x 45 x 25 x 30 -> 11 5x3 / 2x1 24 and 22).  With a
-// dilation the pieces of a row of taps lie apart (80 x 18 x 58 x 60 -> 31 5x3 dilated 97 and 70).  Over 627 passes of 500 drawn
-// convolutions, a third of them with strides of two and a third dilated, the time is 0.866 of gathering, 0.864 if each took the
-// faster form, the worst 1.10; by patch, planes and work alone it was 0.874 and 1.40.
+// few taps, make no gain but with many columns or a long patch (forward 153 x 64 x 30 -> 6 3x3 / 2 f32 45 and 32, 107 x 32 x 47 ->
+// 64 3x3 / 2 42 and 35, its weight gradient 58 and 50, 15 x 96 x 63 x 50 -> 36 1x3 37 and 31, bf16 215 x 91 x 10 x 32 -> 62 3x1 / 2x1
+// 23 and 18; from 32 channels into 96 3x3 / 2 85 and 94, 19 x 47 x 42 x 51 -> 68 2x5 / 2x1 40 and 49), nor do channels that are mostly
+// padding (42 x 6 x 57 -> 32 5x5 56 and 52), a short patch and little work (input gradient 49 x 45 x 25 x 30 -> 11 5x3 / 2x1 24 and
+// 22).  Planes of 60 MB and more leave the L2 (40 x 72 x 57 x 57 -> 10 3x3 75 and 66).  With a dilation the pieces of a row of taps
+// lie apart, most of all short ones (80 x 18 x 58 x 60 -> 31 5x3 dilated 97 and 70).  Over 617 passes of 500 drawn convolutions,
+// a third of them with strides of two and a third dilated, the time is 0.861 of gathering, 0.858 if each took the faster form;
+// by patch, planes and work alone it was 0.867.  Passes that take more than 1.03 of gathering's time: 20 (to 1.26) and 50 (1.51).
 template <class T>
 static bool split_worth(const ConvMap &g, int64_t bytes, int tensors, int64_t positions, int64_t n, int least_patch) {
     const bool f32 = sizeof(T) == 4, wide = n > 80;
     const int64_t patch = (int64_t)g.ff * g.cp, work = positions * patch * (n < 32 ? 32 : n);
     if (patch < least_patch || bytes > 80000000 || work < 300000000) return false;
-    if (!wide && patch < 270 && work < 500000000) return false;
-    if (f32 && !wide && tensors == 1 && g.ff * g.channels < 200) return false;
-    double least = wide ? (f32 ? 0.33 : 0.9) : !f32 ? (tensors == 1 ? 1.75 : 2) : patch < 600 || tensors == 2 ? 1 : 0.6;
-    if (g.dil_w > 1 && g.cp <= 64) least *= 2;
-    if (tensors == 1 && bytes > 60000000 && least < 1) least = 1;
+    const bool padding = f32 && tensors == 1 && g.ff * g.channels < 200 && !(g.gradient && g.st_w > 1);
+    if (n >= 32 && !wide && ((patch < 270 && work < 500000000) || padding)) return false;
+    double least = f32 ? (wide ? 0.3 : tensors == 2 ? (n > 32 ? 0.8 : 1) : n > 32 ? 0.6 : patch < 600 ? 1 : 0.8)
+                       : n >= (tensors == 1 ? 64 : 81) ? 0.9 : tensors == 1 ? 1.75 : n > 40 ? 2 : 3.5;
+    if (g.dil_w > 1 && g.cp <= 24) least *= 2;
+    if (tensors == 1 && bytes > 60000000 && least < 1.4) least = 1.4;
     return (double)(positions * patch * ceil_div(n, 128) * tensors) >= least * (double)bytes;
 }
 

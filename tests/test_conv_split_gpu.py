@@ -27,7 +27,7 @@ RESIDENT = {
     (90, 12, 29, 23, 20, (3, 3), (0, 0), (1, 1), (1, 1)): "rrr",
     (30, 30, 41, 35, 62, (3, 3), (2, 2), (1, 1), (1, 1)): "rss",
     (40, 60, 30, 27, 15, (3, 3), (1, 0), (1, 1), (1, 1)): "rrr",
-    (70, 16, 26, 31, 6, (5, 5), (2, 2), (1, 1), (1, 1)): "sr.",
+    (70, 16, 26, 31, 6, (5, 5), (2, 2), (1, 1), (1, 1)): "srs",
     (150, 6, 33, 34, 33, (3, 3), (1, 1), (1, 1), (1, 1)): "r..",
     (50, 33, 25, 26, 13, (1, 5), (0, 2), (1, 1), (1, 1)): ".rr",
     (1500, 20, 12, 11, 40, (2, 3), (1, 1), (1, 1), (1, 1)): "r..",   # several images per tile, tiles in every accumulator
@@ -49,7 +49,7 @@ GATHERED = {
     (50, 64, 12, 12, 16, (3, 3), (0, 0), (1, 1), (1, 1)): "...",
 }
 # bf16 runs here where the convolutions on TMA boxes do not take it.
-ALL = [(c, torch.float32, e) for c, e in zip(CASES, ("sss", "sss", "sss", ".s.", "sss", "sss", "sss"))] + [(c, torch.float32, e) for c, e in RESIDENT.items()]
+ALL = [(c, torch.float32, e) for c, e in zip(CASES, ("sss", "sss", "sss", "ss.", "sss", "sss", "sss"))] + [(c, torch.float32, e) for c, e in RESIDENT.items()]
 ALL += [(c, torch.bfloat16, e) for c, e in zip(CASES, ("...", "...", "sss", "ss.", "...", "sss", "sss"))]
 ALL += [(c, torch.float32, e) for c, e in GATHERED.items()]
 
