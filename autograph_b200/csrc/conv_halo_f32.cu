@@ -10,8 +10,10 @@
 // and bottom rows of every image, are computed and dropped.
 //
 // The gathered engine fetches and splits every element once per tap (16 channels 3 x 3: 92 KB per tile from L1 and L2, and
-// most of its instructions); here it is once per box, 1.5 times over all of a 32 x 32 image.  A pass that wrote the rows for TMA
-// to load was half of the operator's time.  What bounds it: products of 32 to 128 columns, of which each takes some 45 cycles.
+// most of its instructions); here it is once per box, whose rows are rounded up to 32: 224 rows for a tile of 128 of a 32 x 32
+// image in its frame, so 1.75 times over all.  A pass that wrote the rows for TMA to load was half of the operator's time.
+// What bounds it is latency: at 64 x 16 x 32 x 32 -> 32, four tiles an SM, the tensor pipe is active 12 % (input gradient 9 %) and
+// warps wait for loads of pixels (long scoreboard, 2.5 and 4.7 per issue) and, in the epilogue, for the other ones (barrier 2.5).
 //
 // Warps: 1 issues, 2 - 9 split the filters and then read accumulators, in two sets that take turns at tiles, each with two
 // accumulators (leading block and corrections) of its own, 0 and 10 - 15 load and split rows.

@@ -27,7 +27,8 @@ bool input_by_rows(ag_device *dev, ag_dtype dtype, int64_t oc, int64_t ic, int64
 bool weight_by_rows(ag_dtype dtype, int64_t bs, int64_t ic, int64_t ih, int64_t iw, int64_t oc, const ag_conv2_options *o,
                     int64_t oh, int64_t ow) {
     return dtype == AG_F32 && plain(o) && oc >= 6 && ic * oc >= 64 && (ic >= 12 || ih * iw >= 400) &&
-           conv_weight_worth(dtype, ic * o->filter[0] * o->filter[1], oc, bs * oh * ow, o) && bs * oc * oh * ow < (1ll << 31) && halo32::takes_wgrad(weight_rows(nullptr, bs, ic, ih, iw, nullptr, oc, o, oh, ow));
+           conv_weight_worth(dtype, ic * o->filter[0] * o->filter[1], oc, bs * oh * ow, o) && bs * oc * oh * ow < (1ll << 31) &&
+           halo32::takes_wgrad(weight_rows(nullptr, bs, ic, ih, iw, nullptr, oc, o, oh, ow));
 }
 
 }  // namespace tcx

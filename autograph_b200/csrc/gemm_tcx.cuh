@@ -1307,7 +1307,8 @@ __global__ void __launch_bounds__(Cfg<T, BN>::THREADS, 1)
                 const uint32_t at = tc::smem_u32(sums + col * BM + row);
                 float v[8], sum = 0.f;
 #pragma unroll
-                for (int z = 0; z < 8; ++z) v[z] = z < p.splits ? __uint_as_float(tc::pair::ld_shared_cluster(tc::pair::map_to_cta(at, z))) : 0.f;
+                for (int z = 0; z < 8; ++z)
+                    v[z] = z < p.splits ? __uint_as_float(tc::pair::ld_shared_cluster(tc::pair::map_to_cta(at, z))) : 0.f;
 #pragma unroll
                 for (int z = 0; z < 8; ++z)
                     if (z < p.splits) sum += v[z];

@@ -11,7 +11,8 @@ struct Shape {
     int fh, fw;   // padding 0, stride 1, dilation 1
 };
 
-// True for 3 x 3 filters on 2 to 4 channels and 5 x 5 on 1 or 2, and 64, 128, 192 or 256 output channels.
+// True for 3 x 3 filters on 2 to 4 channels and 5 x 5 on 1 or 2, and 64, 128, 192 or 256 output channels.  The geometries that are
+// compiled; others, one channel of 3 x 3 among them, keep the form with patches in memory.
 bool takes(const Shape &s);
 
 // y [bs][ph][pw][oc] = max over 2 x 2 windows of relu(conv2(x, w) + bias), x NCHW, an odd last row or column left out
